@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "ptx.cuh"
 
 namespace toner {
@@ -118,7 +120,7 @@ struct GemmSmem {
   static constexpr int kStages = (192 * 1024) / kStageBytes;
   static constexpr int kTileBytes = kStages * kStageBytes;
   static constexpr int kBarBytes = 256;
-  static constexpr int kEpiBytes = 8 * 32 * 33 * 4;  // one padded 32 x 32 FP32 staging block per epilogue warp
+  static constexpr int kEpiBytes = 8 * 32 * 32 * 4;  // one 32 x 32 FP32 staging block per epilogue warp
   static constexpr int kTotal = kTileBytes + kBarBytes + kEpiBytes + 1024;  // 1024: alignment slack
   static constexpr int kTmemCols = kWide ? 512 : 2 * BN;
 };
@@ -165,11 +167,18 @@ struct EpilogueTile {
   __half* S0b;
   __half* S1b;
   float alpha, beta;
-  bool use_c;
+  bool use_c, stats;
 };
 
-constexpr int kEpiStride = 33;                      // floats per staged row: 32 + 1 keeps both access patterns conflict-free
-constexpr int kEpiWarpBytes = 32 * kEpiStride * 4;  // one 32 x 32 block per epilogue warp
+constexpr int kEpiWarpFloats = 32 * 32;  // one 32 x 32 staging block per epilogue warp
+
+// Staged block: 32 rows of eight 16-byte chunks, the chunk index exchanged by the row, so that all three access patterns
+// are free of bank conflicts: a lane writing the chunks of its own row, eight lanes reading one row, and (for the mirrored
+// half) eight lanes reading one column of every fourth row.
+__device__ __forceinline__ int stage_at(int row, int chunk) { return row * 32 + (((chunk ^ row ^ (row >> 2)) & 7) << 2); }
+__device__ __forceinline__ float stage_get(const float* stage, int row, int col) {
+  return stage[stage_at(row, col >> 2) + (col & 3)];
+}
 
 __device__ __forceinline__ uint16_t to_bits16(float v, int bf16) {
   const __half h = __float2half_rn(v);
@@ -187,15 +196,12 @@ __device__ __forceinline__ uint2 pack4_16(float a, float b, float c, float d, in
 }
 
 // FP16 hi/lo split of four consecutive values: hi = rn(x), lo = rn(x - hi).
-__device__ __forceinline__ void store_split4(__half* hi, long long plane, float x0, float x1, float x2, float x3) {
-  const __half2 h0 = __floats2half2_rn(x0, x1), h1 = __floats2half2_rn(x2, x3);
+__device__ __forceinline__ void split4(float4 x, uint2& hi, uint2& lo) {
+  const __half2 h0 = __floats2half2_rn(x.x, x.y), h1 = __floats2half2_rn(x.z, x.w);
   const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-  const __half2 l0 = __floats2half2_rn(x0 - f0.x, x1 - f0.y), l1 = __floats2half2_rn(x2 - f1.x, x3 - f1.y);
-  uint2 u, w;
-  u.x = *reinterpret_cast<const uint32_t*>(&h0); u.y = *reinterpret_cast<const uint32_t*>(&h1);
-  w.x = *reinterpret_cast<const uint32_t*>(&l0); w.y = *reinterpret_cast<const uint32_t*>(&l1);
-  *reinterpret_cast<uint2*>(hi) = u;
-  *reinterpret_cast<uint2*>(hi + plane) = w;
+  const __half2 l0 = __floats2half2_rn(x.x - f0.x, x.y - f0.y), l1 = __floats2half2_rn(x.z - f1.x, x.w - f1.y);
+  hi.x = *reinterpret_cast<const uint32_t*>(&h0); hi.y = *reinterpret_cast<const uint32_t*>(&h1);
+  lo.x = *reinterpret_cast<const uint32_t*>(&l0); lo.y = *reinterpret_cast<const uint32_t*>(&l1);
 }
 __device__ __forceinline__ void store_split1(__half* hi, long long plane, float x) {
   const __half h = __float2half_rn(x);
@@ -203,107 +209,207 @@ __device__ __forceinline__ void store_split1(__half* hi, long long plane, float 
   hi[plane] = __float2half_rn(x - __half2float(h));
 }
 
-// The epilogue writes the result in 32 x 32 blocks staged in shared memory (thread t's row of the
-// accumulator at stage[t * kEpiStride ...]), so that the loops below are rolled -- the code stays a few
-// KB and resident in the instruction cache -- and every global access of a warp is made of contiguous runs.
+// The epilogue writes the result in 32 x 32 blocks staged in shared memory, so that every global access of a warp is made
+// of contiguous runs: lane = (row within a group of four, four consecutive columns), one warp access covers four rows x
+// 128 bytes, and the mirrored half of a symmetric result is written the same way with rows and columns exchanged.
 
-// Interior block: wholly inside the matrix, 16-byte aligned rows, no element needing diagonal treatment
-// (for a symmetric result the block lies strictly above the diagonal, so all of it is mirrored and counts
-// twice in the sum of squares).  Lane = (row within a group of four, four consecutive columns): one warp
-// access covers four rows x 128 bytes.  The mirrored half is written the same way with rows and columns
-// exchanged.  The values read from C are fetched four row-groups at a time before any store, so that the
-// loads overlap (C and D may be the same matrix; every element is read before it is written).
-__device__ __forceinline__ void epilogue_block_vec(const GemmParams& p, const EpilogueTile& e, float* stage, int row_first,
-                                                   int c0, int lane, float& ssq, float& mabs, float& maff, float& mres) {
-  const int q = lane & 7, sub = lane >> 3;
-  const int col = c0 + 4 * q;
-  const bool mirror = p.tri && p.mirror;
-  const float s0 = p.s0_scale, s1 = p.s1_scale * p.s1_aff_b;  // no diagonal element in an interior block
-  float s = 0.f, m = 0.f;
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    float4 cv[4];
-    if (e.use_c) {
+struct EpilogueSums {
+  float ssq = 0.f, mabs = 0.f, maff = 0.f, mres = 0.f;
+};
+
+// C of four row groups (four rows each) of a block, all loads in flight at once; zero outside the matrix.
+__device__ __forceinline__ void epilogue_load_c(const GemmParams& p, const EpilogueTile& e, int row0, int c0, int lane,
+                                                float4 (&cv)[4]) {
+  const int row = row0 + (lane >> 3), col = c0 + 4 * (lane & 7);
+  const float* src = e.Cb + (long long)row * (int)p.ldc + col;
+  const long long step = 4LL * (int)p.ldc;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int row = row_first + 16 * half + 4 * u + sub;
-        cv[u] = *reinterpret_cast<const float4*>(e.Cb + (long long)row * p.ldc + col);
-      }
-    }
+  for (int u = 0; u < 4; ++u, src += step) {
+    cv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row + 4 * u < p.M && col < p.N) cv[u] = *reinterpret_cast<const float4*>(src);
+  }
+}
+
+// Every requested output of four row groups (row, row + 4, row + 8, row + 12; four consecutive columns each).  The
+// outputs are the outer loop: the tests for which of them exist are then made once per sixteen elements of a lane.
+// dg: position of the diagonal element within row group u is dg + 4 u (outside 0..3: none).
+__device__ __forceinline__ void epilogue_emit(const GemmParams& p, const EpilogueTile& e, int row, int col, const float4 (&v)[4],
+                                              const bool (&ok)[4], bool with_d, bool whole, int dg) {
+  if (with_d) {
+    float* dst = e.Db + (long long)row * (int)p.ldd + col;
+    const long long step = 4LL * (int)p.ldd;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = 16 * half + 4 * u + sub;
-      const int row = row_first + i;
-      float* src = stage + i * kEpiStride + 4 * q;
-      float v0 = e.alpha * src[0], v1 = e.alpha * src[1], v2 = e.alpha * src[2], v3 = e.alpha * src[3];
-      if (e.use_c) {
-        v0 = fmaf(e.beta, cv[u].x, v0); v1 = fmaf(e.beta, cv[u].y, v1);
-        v2 = fmaf(e.beta, cv[u].z, v2); v3 = fmaf(e.beta, cv[u].w, v3);
+    for (int u = 0; u < 4; ++u, dst += step)
+      if (ok[u]) *reinterpret_cast<float4*>(dst) = v[u];
+  }
+  if (e.Hb) {
+    uint16_t* dst = e.Hb + (long long)row * (int)p.ld16 + col;
+    const long long step = 4LL * (int)p.ld16;
+#pragma unroll
+    for (int u = 0; u < 4; ++u, dst += step)
+      if (ok[u]) *reinterpret_cast<uint2*>(dst) = pack4_16(v[u].x, v[u].y, v[u].z, v[u].w, p.d16_fmt);
+  }
+  const long long sstep = 4LL * (int)p.s_ld;
+  if (e.S0b) {
+    __half* dst = e.S0b + (long long)row * (int)p.s_ld + col;
+    const float s0 = p.s0_scale;
+#pragma unroll
+    for (int u = 0; u < 4; ++u, dst += sstep) {
+      uint2 hi, lo;
+      split4(make_float4(s0 * v[u].x, s0 * v[u].y, s0 * v[u].z, s0 * v[u].w), hi, lo);
+      if (ok[u]) {
+        *reinterpret_cast<uint2*>(dst) = hi;
+        *reinterpret_cast<uint2*>(dst + p.s_plane) = lo;
       }
-      if (e.Db) *reinterpret_cast<float4*>(e.Db + (long long)row * p.ldd + col) = make_float4(v0, v1, v2, v3);
-      if (e.Hb) *reinterpret_cast<uint2*>(e.Hb + (long long)row * p.ld16 + col) = pack4_16(v0, v1, v2, v3, p.d16_fmt);
-      if (e.S0b) store_split4(e.S0b + (long long)row * p.s_ld + col, p.s_plane, s0 * v0, s0 * v1, s0 * v2, s0 * v3);
-      if (e.S1b) store_split4(e.S1b + (long long)row * p.s_ld + col, p.s_plane, s1 * v0, s1 * v1, s1 * v2, s1 * v3);
-      if (mirror) {
-        src[0] = v0; src[1] = v1; src[2] = v2; src[3] = v3;
-      }
-      s = fmaf(v0, v0, s); s = fmaf(v1, v1, s); s = fmaf(v2, v2, s); s = fmaf(v3, v3, s);
-      m = fmaxf(fmaxf(fmaxf(m, fabsf(v0)), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3)));
     }
   }
-  ssq += p.tri ? 2.f * s : s;
-  mabs = fmaxf(mabs, m);
-  maff = fmaxf(maff, fabsf(p.aff_b) * m);  // off the diagonal the affine map is a plain scaling
-  // and the distance from the identity is |d|; fmaxf drops NaN, the sum of squares does not
-  mres = fmaxf(mres, isfinite(s) ? m : INFINITY);
-  if (mirror) {
-    __syncwarp();
-    const int tcol = row_first + 4 * q;  // source rows 4q .. 4q+3 become four consecutive target columns
-    const float* src = stage + (4 * q) * kEpiStride;
-#pragma unroll 2
-    for (int it = 0; it < 8; ++it) {
-      const int j = 4 * it + sub;  // source column = target row
-      const float v0 = src[j], v1 = src[kEpiStride + j], v2 = src[2 * kEpiStride + j], v3 = src[3 * kEpiStride + j];
-      const long long trow = c0 + j;
-      if (e.Db && !p.upper_d) *reinterpret_cast<float4*>(e.Db + trow * p.ldd + tcol) = make_float4(v0, v1, v2, v3);
-      if (e.Hb) *reinterpret_cast<uint2*>(e.Hb + trow * p.ld16 + tcol) = pack4_16(v0, v1, v2, v3, p.d16_fmt);
-      if (e.S0b) store_split4(e.S0b + trow * p.s_ld + tcol, p.s_plane, s0 * v0, s0 * v1, s0 * v2, s0 * v3);
-      if (e.S1b) store_split4(e.S1b + trow * p.s_ld + tcol, p.s_plane, s1 * v0, s1 * v1, s1 * v2, s1 * v3);
+  if (e.S1b) {
+    __half* dst = e.S1b + (long long)row * (int)p.s_ld + col;
+    const float s1 = p.s1_scale * p.s1_aff_b, sd = whole ? p.s1_scale * p.s1_aff_a : 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u, dst += sstep) {
+      const int d = dg + 4 * u;
+      uint2 hi, lo;
+      split4(make_float4(fmaf(s1, v[u].x, d == 0 ? sd : 0.f), fmaf(s1, v[u].y, d == 1 ? sd : 0.f),
+                         fmaf(s1, v[u].z, d == 2 ? sd : 0.f), fmaf(s1, v[u].w, d == 3 ? sd : 0.f)), hi, lo);
+      if (ok[u]) {
+        *reinterpret_cast<uint2*>(dst) = hi;
+        *reinterpret_cast<uint2*>(dst + p.s_plane) = lo;
+      }
+    }
+  }
+}
+
+// One block with 16-byte accesses: interior, at the matrix edge (N a multiple of four), or a diagonal block of a mirrored
+// symmetric result, which is written whole from its upper half.  One rolled loop over half blocks -- two for the block
+// itself, two for its mirror image (or, of a diagonal block, for all of it) -- so that the code stays small: an epilogue of
+// a short product runs once per SM from a cold instruction cache, and with two epilogue warps per scheduler the number of
+// instructions is what it costs (800 per block made it 3650 cycles, whatever was stored).
+// With kAhead the caller has loaded C of the block's first half; C of the next half (or of the next block, next_c0) is
+// fetched as soon as the registers are free, i.e. before the stores, so that its latency hides behind them.
+template <bool kAhead>
+__device__ __forceinline__ void epilogue_block_vec(const GemmParams& p, const EpilogueTile& e, float* stage, int row_first,
+                                                   int c0, int lane, bool holds_diag, float4 (&cv)[4], int next_c0,
+                                                   EpilogueSums& t) {
+  const int q = lane & 7, sub = lane >> 3;
+  const bool mirror = p.tri && p.mirror;
+  const bool whole = mirror && holds_diag;
+  const int halves = mirror ? 4 : 2;
+#pragma unroll 1
+  for (int h = 0; h < halves; ++h) {
+    const bool image = h >= 2;
+    const int i0 = 16 * (h & 1) + sub;
+    float4 v[4];
+    if (!image) {
+      if (!kAhead && e.use_c) epilogue_load_c(p, e, row_first + 16 * h, c0, lane, cv);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        v[u] = *reinterpret_cast<const float4*>(stage + stage_at(i0 + 4 * u, q));
+        v[u].x *= e.alpha; v[u].y *= e.alpha; v[u].z *= e.alpha; v[u].w *= e.alpha;
+      }
+      if (e.use_c) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          v[u].x = fmaf(e.beta, cv[u].x, v[u].x); v[u].y = fmaf(e.beta, cv[u].y, v[u].y);
+          v[u].z = fmaf(e.beta, cv[u].z, v[u].z); v[u].w = fmaf(e.beta, cv[u].w, v[u].w);
+        }
+        const int c = h ? next_c0 : c0;
+        if (kAhead && c >= 0) epilogue_load_c(p, e, h ? row_first : row_first + 16, c, lane, cv);
+      }
+      if (mirror) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(stage + stage_at(i0 + 4 * u, q)) = v[u];
+      }
+    } else {
+      if (h == 2) __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + 4 * u;
+        float x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {   // of a diagonal block, only the elements left of the diagonal are exchanged
+          const bool swap = !whole || 4 * q + k < i;
+          x[k] = stage_get(stage, swap ? 4 * q + k : i, swap ? i : 4 * q + k);
+        }
+        v[u] = make_float4(x[0], x[1], x[2], x[3]);
+      }
+    }
+    const int row = (image && !whole ? c0 : row_first) + i0, col = (image && !whole ? row_first : c0) + 4 * q;
+    bool ok[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ok[u] = row + 4 * u < p.M && col < p.N;
+    if (whole == image || !whole) epilogue_emit(p, e, row, col, v, ok, e.Db && !(image && !whole && p.upper_d), whole, row - col);
+    if (e.stats && whole == image) {   // (outside the matrix the results are zero: operands and C are read as zero there)
+      float s = 0.f, m = 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s = fmaf(x[k], x[k], s);
+          if (whole && row + 4 * u == col + k) {   // the diagonal element's distance from the identity is its own
+            if (ok[u]) {
+              t.mabs = fmaxf(t.mabs, fabsf(x[k]));
+              t.maff = fmaxf(t.maff, fabsf(fmaf(p.aff_b, x[k], p.aff_a)));
+              t.mres = fmaxf(t.mres, fabsf(1.f - x[k]));
+            }
+          } else {
+            m = fmaxf(m, fabsf(x[k]));
+          }
+        }
+      }
+      t.ssq += (p.tri && !whole) ? 2.f * s : s;    // a block above the diagonal counts for its mirror image as well
+      t.mabs = fmaxf(t.mabs, m);
+      t.maff = fmaxf(t.maff, fabsf(p.aff_b) * m);  // off the diagonal the affine map is a plain scaling
+      // and the distance from the identity is |d|; fmaxf drops NaN, the sum of squares does not
+      t.mres = fmaxf(t.mres, isfinite(s) ? m : INFINITY);
     }
   }
   __syncwarp();
 }
 
-// Any other block (matrix edge, diagonal block of a symmetric result, packed or unaligned output): one
-// element per lane with full masking, lane = column, so rows -- also rows of a packed triangle -- are
-// still written as contiguous runs; the mirrored half with lane = source row.
+// Any other block (packed or unaligned output): one element per lane with full masking, lane = column, so rows -- also
+// rows of a packed triangle -- are still written as contiguous runs; the mirrored half with lane = source row.  C is
+// fetched eight rows at a time.
 __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const EpilogueTile& e, float* stage, int row_first,
-                                                      int c0, int lane, float& ssq, float& mabs, float& maff, float& mres) {
+                                                      int c0, int lane, EpilogueSums& t) {
   const int col = c0 + lane;
   const bool col_ok = col < p.N;
   const bool mirror = p.tri && p.mirror;
   const int rows = min(32, p.M - row_first);
 #pragma unroll 1
-  for (int i = 0; i < rows; ++i) {
-    const int row = row_first + i;
-    float v = 0.f;
-    if (col_ok && !(p.tri && col < row)) {
-      v = e.alpha * stage[i * kEpiStride + lane];
-      const long long co = p.packed ? packed_off(row, col, p.N) : (long long)row * p.ldc + col;
-      const long long dof = p.packed ? packed_off(row, col, p.N) : (long long)row * p.ldd + col;
-      if (e.use_c) v = fmaf(e.beta, e.Cb[co], v);
-      if (e.Db) e.Db[dof] = v;
-      if (e.Hb) e.Hb[(long long)row * p.ld16 + col] = to_bits16(v, p.d16_fmt);
-      const float dg = (col == row) ? 1.f : 0.f;
-      if (e.S0b) store_split1(e.S0b + (long long)row * p.s_ld + col, p.s_plane, p.s0_scale * v);
-      if (e.S1b) store_split1(e.S1b + (long long)row * p.s_ld + col, p.s_plane, p.s1_scale * fmaf(p.s1_aff_b, v, p.s1_aff_a * dg));
-      mres = isfinite(v) ? fmaxf(mres, fabsf(dg - v)) : INFINITY;  // a non-finite result must not pass as converged
-      const float w = (p.tri && col > row) ? 2.f : 1.f;
-      ssq = fmaf(w * v, v, ssq);
-      mabs = fmaxf(mabs, fabsf(v));
-      maff = fmaxf(maff, fabsf(fmaf(p.aff_b, v, col == row ? p.aff_a : 0.f)));
+  for (int i0 = 0; i0 < rows; i0 += 8) {
+    float cv[8];
+    if (e.use_c) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int row = row_first + i0 + u;
+        cv[u] = 0.f;
+        if (row < p.M && col_ok && !(p.tri && col < row))
+          cv[u] = e.Cb[p.packed ? packed_off(row, col, p.N) : (long long)row * p.ldc + col];
+      }
     }
-    if (mirror) stage[i * kEpiStride + lane] = v;  // final value; zero where masked
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int i = i0 + u, row = row_first + i;
+      float* const at = stage + stage_at(i, lane >> 2) + (lane & 3);
+      float v = 0.f;
+      if (row < p.M && col_ok && !(p.tri && col < row)) {
+        v = e.alpha * *at;
+        if (e.use_c) v = fmaf(e.beta, cv[u], v);
+        if (e.Db) e.Db[p.packed ? packed_off(row, col, p.N) : (long long)row * p.ldd + col] = v;
+        if (e.Hb) e.Hb[(long long)row * p.ld16 + col] = to_bits16(v, p.d16_fmt);
+        const float dg = (col == row) ? 1.f : 0.f;
+        if (e.S0b) store_split1(e.S0b + (long long)row * p.s_ld + col, p.s_plane, p.s0_scale * v);
+        if (e.S1b) store_split1(e.S1b + (long long)row * p.s_ld + col, p.s_plane, p.s1_scale * fmaf(p.s1_aff_b, v, p.s1_aff_a * dg));
+        t.mres = isfinite(v) ? fmaxf(t.mres, fabsf(dg - v)) : INFINITY;  // a non-finite result must not pass as converged
+        const float w = (p.tri && col > row) ? 2.f : 1.f;
+        t.ssq = fmaf(w * v, v, t.ssq);
+        t.mabs = fmaxf(t.mabs, fabsf(v));
+        t.maff = fmaxf(t.maff, fabsf(fmaf(p.aff_b, v, col == row ? p.aff_a : 0.f)));
+      }
+      if (mirror) *at = v;  // final value; zero where masked
+    }
   }
   if (mirror) {
     __syncwarp();
@@ -314,7 +420,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
       for (int j = 0; j < cols; ++j) {
         const int c = c0 + j;
         if (c > row) {
-          const float v = stage[lane * kEpiStride + j];
+          const float v = stage_get(stage, lane, j);
           if (e.Db && !p.upper_d) e.Db[(long long)c * p.ldd + row] = v;
           if (e.Hb) e.Hb[(long long)c * p.ld16 + row] = to_bits16(v, p.d16_fmt);
           if (e.S0b) store_split1(e.S0b + (long long)c * p.s_ld + row, p.s_plane, p.s0_scale * v);
@@ -640,7 +746,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     constexpr int NCH = BN / 64;  // 32-column chunks per warp
     const int lane_group = warp & 3;
     const int half = (warp - 4) >> 2;
-    float* const stage = reinterpret_cast<float*>(smem + S::kTileBytes + S::kBarBytes) + (warp - 4) * (32 * kEpiStride);
+    float* const stage = reinterpret_cast<float*>(smem + S::kTileBytes + S::kBarBytes) + (warp - 4) * kEpiWarpFloats;
     constexpr bool chained = kChained;
     // Running sums of the accumulation chains (chained products only), added with round-to-nearest: the
     // tensor core itself adds into its accumulator by truncation.
@@ -684,6 +790,36 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         return tmem_base + ((uint32_t)(lane_group * 32) << 16) + (uint32_t)((kWide ? 0 : buf * BN) + half * (BN / 2));
       };
 
+      EpilogueTile e;
+      e.alpha = p.alpha;
+      e.beta = p.beta;
+      if (p.alpha_a) e.alpha *= __ldg(p.alpha_a + b);
+      if (p.alpha_b) e.alpha *= __ldg(p.alpha_b + (long long)b * p.alpha_b_step);
+      if (p.beta_v) e.beta *= __ldg(p.beta_v + b);
+      e.use_c = (p.C != nullptr) && (e.beta != 0.f);
+      e.stats = p.sumsq || p.maxabs || p.maxaff || p.maxres;
+      e.Cb = p.C ? p.C + (long long)b * p.c_bs : nullptr;
+      e.Db = p.D ? p.D + (long long)b * p.d_bs : nullptr;
+      e.Hb = p.D16 ? reinterpret_cast<uint16_t*>(p.D16) + (long long)b * p.d16_bs : nullptr;
+      e.S0b = p.S0 ? p.S0 + (long long)b * p.s_bs : nullptr;
+      e.S1b = p.S1 ? p.S1 + (long long)b * p.s_bs : nullptr;
+      // the blocks this warp writes: a contiguous run of its NCH 32-column blocks (warp-uniform)
+      int cc_first = 0, cc_end = NCH;
+      while (cc_first < NCH && !needed(col_first + cc_first * 32)) ++cc_first;
+      while (cc_end > cc_first && !needed(col_first + (cc_end - 1) * 32)) --cc_end;
+      const bool rows_inside = row_first + 32 <= p.M;
+      // warp-uniform choice of the 16-byte path; a symmetric result that is not mirrored keeps its lower triangle untouched,
+      // and diagonal elements that need their own treatment are looked after where a diagonal block is written whole
+      auto vectorised = [&](int c0) {
+        const bool holds_diag = c0 <= row_first + 31 && c0 + 31 >= row_first;
+        const bool plain_diag = holds_diag && (p.tri ? !p.mirror : (p.maxaff || p.maxres || p.S1));
+        return p.vec_ok && ((rows_inside && c0 + 32 <= p.N) || p.N % 4 == 0) && !plain_diag;
+      };
+      // C of the first block is fetched while the accumulator is still being formed
+      float4 cv[4];
+      if (!chained && e.use_c && cc_first < cc_end && vectorised(col_first + cc_first * 32))
+        epilogue_load_c(p, e, row_first, col_first + cc_first * 32, lane, cv);
+
       if (chained) {
 #pragma unroll
         for (int j = 0; j < NCH * 32; ++j) racc[j] = 0.f;
@@ -720,86 +856,67 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
 
       // ---- write the tile: one rolled loop over the warp's 32 x 32 blocks, staged through shared memory
       const long long o0 = p.prof ? clock64() : 0;
-      EpilogueTile e;
-      e.alpha = p.alpha;
-      e.beta = p.beta;
-      if (p.alpha_a) e.alpha *= __ldg(p.alpha_a + b);
-      if (p.alpha_b) e.alpha *= __ldg(p.alpha_b + (long long)b * p.alpha_b_step);
-      if (p.beta_v) e.beta *= __ldg(p.beta_v + b);
-      e.use_c = (p.C != nullptr) && (e.beta != 0.f);
-      e.Cb = p.C ? p.C + (long long)b * p.c_bs : nullptr;
-      e.Db = p.D ? p.D + (long long)b * p.d_bs : nullptr;
-      e.Hb = p.D16 ? reinterpret_cast<uint16_t*>(p.D16) + (long long)b * p.d16_bs : nullptr;
-      e.S0b = p.S0 ? p.S0 + (long long)b * p.s_bs : nullptr;
-      e.S1b = p.S1 ? p.S1 + (long long)b * p.s_bs : nullptr;
-      float ssq = 0.f, mabs = 0.f, maff = 0.f, mres = 0.f;
-      const bool rows_inside = row_first + 32 <= p.M;
+      EpilogueSums sums;
       const uint32_t taddr = tmem_of(kWide ? 0 : (int)(gchunk & 1u));
-      float* const mine = stage + lane * kEpiStride;
 #pragma unroll 1
-      for (int cc = 0; cc < NCH; ++cc) {
+      for (int cc = cc_first; cc < cc_end; ++cc) {
         const int c0 = col_first + cc * 32;
-        if (!needed(c0)) continue;
-        if (chained) {
-          switch (cc) {  // the running sums live in registers: static indices only
-            case 0:
+        auto put = [&](int j, float x0, float x1, float x2, float x3) {
+          *reinterpret_cast<float4*>(stage + stage_at(lane, j)) = make_float4(x0, x1, x2, x3);
+        };
+        if constexpr (chained) {
+          // the running sums live in registers: static indices only
+          auto put_sums = [&](auto first) {
+            constexpr int o = decltype(first)::value;
 #pragma unroll
-              for (int j = 0; j < 32; ++j) mine[j] = racc[j];
-              break;
-            case 1:
-#pragma unroll
-              for (int j = 0; j < 32; ++j) mine[j] = racc[32 + j];
-              break;
-            case 2:
-              if (NCH > 2) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) mine[j] = racc[(NCH > 2 ? 64 : 0) + j];
-              }
-              break;
-            default:
-              if (NCH > 2) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) mine[j] = racc[(NCH > 2 ? 96 : 0) + j];
-              }
-              break;
-          }
+            for (int j = 0; j < 8; ++j) put(j, racc[o + 4 * j], racc[o + 4 * j + 1], racc[o + 4 * j + 2], racc[o + 4 * j + 3]);
+          };
+          if (cc == 0) put_sums(std::integral_constant<int, 0>());
+          if (cc == 1) put_sums(std::integral_constant<int, chained ? 32 : 0>());
+          if (cc == 2) put_sums(std::integral_constant<int, (chained && NCH > 2) ? 64 : 0>());
+          if (cc == 3) put_sums(std::integral_constant<int, (chained && NCH > 2) ? 96 : 0>());
         } else {
           uint32_t raw[32];
           ptx::tmem_ld32(taddr + (uint32_t)(cc * 32), raw);
           ptx::tmem_ld_wait();
+          // every block has been read: the MMA warp may have the accumulator back (a wide tile: this warp read columns of
+          // half `half` only, and that half's barrier counts its four lane groups of both CTAs)
+          if (cc == cc_end - 1) release(kWide ? half : (int)(gchunk & 1u));
 #pragma unroll
-          for (int j = 0; j < 32; ++j) mine[j] = __uint_as_float(raw[j]);
+          for (int j = 0; j < 8; ++j)
+            put(j, __uint_as_float(raw[4 * j]), __uint_as_float(raw[4 * j + 1]), __uint_as_float(raw[4 * j + 2]),
+                __uint_as_float(raw[4 * j + 3]));
         }
         __syncwarp();
-        // warp-uniform choice: interior blocks take the vector path
-        const bool holds_diag = (c0 <= row_first + 31) && (c0 + 31 >= row_first);
-        if (rows_inside && (c0 + 32 <= p.N) && p.vec_ok && !(holds_diag && (p.tri || p.maxaff || p.maxres || p.S1))) {
-          epilogue_block_vec(p, e, stage, row_first, c0, lane, ssq, mabs, maff, mres);
+        if (vectorised(c0)) {
+          const int next = (cc + 1 < cc_end && vectorised(c0 + 32)) ? c0 + 32 : -1;
+          epilogue_block_vec<!kChained>(p, e, stage, row_first, c0, lane, c0 <= row_first + 31 && c0 + 31 >= row_first, cv,
+                                           next, sums);
         } else {
-          epilogue_block_scalar(p, e, stage, row_first, c0, lane, ssq, mabs, maff, mres);
+          epilogue_block_scalar(p, e, stage, row_first, c0, lane, sums);
+          if (!chained && e.use_c && cc + 1 < cc_end && vectorised(c0 + 32))
+            epilogue_load_c(p, e, row_first, c0 + 32, lane, cv);
         }
       }
       if (!chained) {
-        // wide tile: this warp read columns of half `half` only, and that half's barrier counts its four lane groups
-        // of both CTAs
-        release(kWide ? half : (int)(gchunk & 1u));
+        if (cc_first >= cc_end) release(kWide ? half : (int)(gchunk & 1u));   // nothing of this tile is this warp's to read
         ++gchunk;
       }
       if (p.prof) prof_out += clock64() - o0;
 
-      if (p.sumsq || p.maxabs || p.maxaff || p.maxres) {
+      if (e.stats) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-          ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
-          mabs = fmaxf(mabs, __shfl_xor_sync(0xffffffffu, mabs, o));
-          maff = fmaxf(maff, __shfl_xor_sync(0xffffffffu, maff, o));
-          mres = fmaxf(mres, __shfl_xor_sync(0xffffffffu, mres, o));
+          sums.ssq += __shfl_xor_sync(0xffffffffu, sums.ssq, o);
+          sums.mabs = fmaxf(sums.mabs, __shfl_xor_sync(0xffffffffu, sums.mabs, o));
+          sums.maff = fmaxf(sums.maff, __shfl_xor_sync(0xffffffffu, sums.maff, o));
+          sums.mres = fmaxf(sums.mres, __shfl_xor_sync(0xffffffffu, sums.mres, o));
         }
         if (lane == 0) {
-          if (p.sumsq) atomicAdd(p.sumsq + b, ssq);  // order of these additions is not fixed
-          if (p.maxabs) atomicMax(p.maxabs + b, __float_as_uint(mabs));
-          if (p.maxaff) atomicMax(p.maxaff + b, __float_as_uint(maff));
-          if (p.maxres) atomicMax(p.maxres + b, __float_as_uint(mres));
+          if (p.sumsq) atomicAdd(p.sumsq + b, sums.ssq);  // order of these additions is not fixed
+          if (p.maxabs) atomicMax(p.maxabs + b, __float_as_uint(sums.mabs));
+          if (p.maxaff) atomicMax(p.maxaff + b, __float_as_uint(sums.maff));
+          if (p.maxres) atomicMax(p.maxres + b, __float_as_uint(sums.mres));
         }
       }
     }
