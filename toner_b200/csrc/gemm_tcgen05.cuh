@@ -70,7 +70,8 @@ struct GemmParams {
   int packed;   // C and D are packed upper triangles (row r starts at r*N - r(r-1)/2 - r ... see packed_off)
   int mirror;   // tri: also store the transposed element
   int upper_d;  // tri + mirror: the FP32 result D is not mirrored (its lower triangle is never read)
-  int vec_ok;   // leading dimensions and batch strides allow 16-byte vector access
+  int tma_ok;   // C and every output can be moved by TMA (16-byte bases and strides): *_map below are valid
+  int s_lo_z;   // the lo plane of an operand-plane output is s_lo_z batches behind the hi plane in s0_map / s1_map
   float* sumsq;           // per batch: sum of d^2 over the full (mirrored) result
   unsigned int* maxabs;   // per batch: max |d| as FP32 bits
   unsigned int* maxaff;   // per batch: max |aff_a * [r==c] + aff_b * d| as FP32 bits
@@ -85,6 +86,8 @@ struct GemmParams {
   float s0_scale, s1_scale, s1_aff_a, s1_aff_b;
   int* status;  // set non-zero if a bounded wait ran out
   unsigned long long* prof;  // optional: eight cycle counters summed over CTAs (see toner_gemm_phase_cycles)
+  // 32 x 32 boxes of C and of the outputs, (columns, rows, batch): FP32 with 128-byte, 16-bit with 64-byte swizzle
+  CUtensorMap c_map, d_map, h_map, s0_map, s1_map;
 };
 
 __host__ __device__ inline long long packed_off(long long r, long long c, long long n) {
@@ -110,6 +113,8 @@ __host__ __device__ inline int gemm_tiles_per_batch(int M, int N, int BN, int tr
 // fills all 512 columns of tensor memory, so there is no second buffer: the epilogue of a tile overlaps the next
 // tile's MMAs only half by half.  It pays where the accumulation is long (K in the thousands of k-blocks, as in
 // the statistic X^T X, or three plane passes of a wide matrix).
+constexpr int kEpiBlockBytes = 32 * 32 * 4;  // one staged 32 x 32 block of the epilogue
+
 template <int BN, bool kPair = false>
 struct GemmSmem {
   static constexpr bool kWide = kPair && BN == 512;
@@ -117,11 +122,14 @@ struct GemmSmem {
   static constexpr int kBRows = kPair ? BN / 2 : BN;   // rows of B this CTA loads per stage
   static constexpr int kBBytes = kBRows * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = (192 * 1024) / kStageBytes;
+  // Four stages keep the main loop fed as well as six did (BF16 4096^3 x 4 on pair tiles: 436 us with either; three stages
+  // of the 48 KB tiles); the rest of shared memory is the epilogue's, which needs several blocks per warp in flight.
+  static constexpr int kStages = kStageBytes > 32 * 1024 ? 3 : 4;
   static constexpr int kTileBytes = kStages * kStageBytes;
+  static constexpr int kEpiBufs = kStageBytes > 32 * 1024 ? 2 : 3;          // 4 KB blocks per epilogue warp
+  static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
   static constexpr int kBarBytes = 256;
-  static constexpr int kEpiBytes = 8 * 32 * 32 * 4;  // one 32 x 32 FP32 staging block per epilogue warp
-  static constexpr int kTotal = kTileBytes + kBarBytes + kEpiBytes + 1024;  // 1024: alignment slack
+  static constexpr int kTotal = kTileBytes + kEpiBytes + kBarBytes + 1024;  // 1024: alignment slack
   static constexpr int kTmemCols = kWide ? 512 : 2 * BN;
 };
 
@@ -170,207 +178,207 @@ struct EpilogueTile {
   bool use_c, stats;
 };
 
-constexpr int kEpiWarpFloats = 32 * 32;  // one 32 x 32 staging block per epilogue warp
-
-// Staged block: 32 rows of eight 16-byte chunks, the chunk index exchanged by the row, so that all three access patterns
-// are free of bank conflicts: a lane writing the chunks of its own row, eight lanes reading one row, and (for the mirrored
-// half) eight lanes reading one column of every fourth row.
-__device__ __forceinline__ int stage_at(int row, int chunk) { return row * 32 + (((chunk ^ row ^ (row >> 2)) & 7) << 2); }
-__device__ __forceinline__ float stage_get(const float* stage, int row, int col) {
-  return stage[stage_at(row, col >> 2) + (col & 3)];
-}
-
 __device__ __forceinline__ uint16_t to_bits16(float v, int bf16) {
   const __half h = __float2half_rn(v);
   const __nv_bfloat16 g = __float2bfloat16_rn(v);
   return bf16 ? *reinterpret_cast<const uint16_t*>(&g) : *reinterpret_cast<const uint16_t*>(&h);
 }
 
-__device__ __forceinline__ uint2 pack4_16(float a, float b, float c, float d, int bf16) {
-  const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, d);
-  const __nv_bfloat162 g0 = __floats2bfloat162_rn(a, b), g1 = __floats2bfloat162_rn(c, d);
-  uint2 u;
-  u.x = bf16 ? *reinterpret_cast<const uint32_t*>(&g0) : *reinterpret_cast<const uint32_t*>(&h0);
-  u.y = bf16 ? *reinterpret_cast<const uint32_t*>(&g1) : *reinterpret_cast<const uint32_t*>(&h1);
-  return u;
+__device__ __forceinline__ uint32_t pack2_16(float a, float b, int bf16) {
+  const __half2 h = __floats2half2_rn(a, b);
+  const __nv_bfloat162 g = __floats2bfloat162_rn(a, b);
+  return bf16 ? *reinterpret_cast<const uint32_t*>(&g) : *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// FP16 hi/lo split of four consecutive values: hi = rn(x), lo = rn(x - hi).
-__device__ __forceinline__ void split4(float4 x, uint2& hi, uint2& lo) {
-  const __half2 h0 = __floats2half2_rn(x.x, x.y), h1 = __floats2half2_rn(x.z, x.w);
-  const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-  const __half2 l0 = __floats2half2_rn(x.x - f0.x, x.y - f0.y), l1 = __floats2half2_rn(x.z - f1.x, x.w - f1.y);
-  hi.x = *reinterpret_cast<const uint32_t*>(&h0); hi.y = *reinterpret_cast<const uint32_t*>(&h1);
-  lo.x = *reinterpret_cast<const uint32_t*>(&l0); lo.y = *reinterpret_cast<const uint32_t*>(&l1);
-}
 __device__ __forceinline__ void store_split1(__half* hi, long long plane, float x) {
   const __half h = __float2half_rn(x);
   hi[0] = h;
   hi[plane] = __float2half_rn(x - __half2float(h));
 }
 
-// The epilogue writes the result in 32 x 32 blocks staged in shared memory, so that every global access of a warp is made
-// of contiguous runs: lane = (row within a group of four, four consecutive columns), one warp access covers four rows x
-// 128 bytes, and the mirrored half of a symmetric result is written the same way with rows and columns exchanged.
-
+// The epilogue works in 32 x 32 blocks.  A thread has one row of the block in registers (that is how tensor memory is
+// read), writes it to a shared-memory block in the layout of a swizzled TMA box -- row by row, or exchanged for the mirrored
+// half of a symmetric result -- and one lane stores the box.  No address arithmetic per element, no masks (TMA clips at
+// the matrix edge), and the stores run behind the next block.  With two epilogue warps per scheduler it is the number of
+// instructions a block takes that bounds short products: staging rows in shared memory, reading them back and storing
+// them with 16-byte accesses took about 500 per block and output, 2100 cycles for one FP32 output.
+//
+// Offsets inside a staged block (base 1024-byte aligned), conflict-free for a lane = row writer:
+//   FP32 box, 128-byte rows: 16-byte chunk index ^= row & 7;    16-bit box, 64-byte rows: chunk index ^= (row >> 1) & 3.
 struct EpilogueSums {
   float ssq = 0.f, mabs = 0.f, maff = 0.f, mres = 0.f;
 };
 
-// C of four row groups (four rows each) of a block, all loads in flight at once; zero outside the matrix.
-__device__ __forceinline__ void epilogue_load_c(const GemmParams& p, const EpilogueTile& e, int row0, int c0, int lane,
-                                                float4 (&cv)[4]) {
-  const int row = row0 + (lane >> 3), col = c0 + 4 * (lane & 7);
-  const float* src = e.Cb + (long long)row * (int)p.ldc + col;
-  const long long step = 4LL * (int)p.ldc;
+__device__ __forceinline__ void stage_rows_f32(uint32_t buf, int lane, const float (&v)[32]) {
+  const uint32_t at = buf + lane * 128 + ((lane & 7) << 4);
 #pragma unroll
-  for (int u = 0; u < 4; ++u, src += step) {
-    cv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row + 4 * u < p.M && col < p.N) cv[u] = *reinterpret_cast<const float4*>(src);
+  for (int j = 0; j < 8; ++j)
+    ptx::sts128(at ^ (j << 4), __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]),
+                __float_as_uint(v[4 * j + 3]));
+}
+__device__ __forceinline__ void stage_cols_f32(uint32_t buf, int lane, const float (&v)[32]) {
+  const uint32_t at = buf + ((lane >> 2) << 4) + (lane & 3) * 4;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) ptx::sts32((at ^ ((j & 7) << 4)) + j * 128, __float_as_uint(v[j]));
+}
+__device__ __forceinline__ void load_row_f32(uint32_t buf, int lane, float4 (&r)[8]) {
+  const uint32_t at = buf + lane * 128 + ((lane & 7) << 4);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = ptx::lds128(at ^ (j << 4));
+}
+// w[k]: the 16-bit elements 2k (low half) and 2k + 1 of this lane's row
+__device__ __forceinline__ void stage_rows_16(uint32_t buf, int lane, const uint32_t (&w)[16]) {
+  const uint32_t at = buf + lane * 64 + (((lane >> 1) & 3) << 4);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) ptx::sts128(at ^ (c << 4), w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+}
+__device__ __forceinline__ void stage_cols_16(uint32_t buf, int lane, const uint32_t (&w)[16]) {
+  const uint32_t at = buf + ((lane >> 3) << 4) + (lane & 7) * 2;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    ptx::sts16((at ^ ((k & 3) << 4)) + k * 128, w[k]);
+    ptx::sts16_hi((at ^ ((k & 3) << 4)) + k * 128 + 64, w[k]);
   }
 }
 
-// Every requested output of four row groups (row, row + 4, row + 8, row + 12; four consecutive columns each).  The
-// outputs are the outer loop: the tests for which of them exist are then made once per sixteen elements of a lane.
-// dg: position of the diagonal element within row group u is dg + 4 u (outside 0..3: none).
-__device__ __forceinline__ void epilogue_emit(const GemmParams& p, const EpilogueTile& e, int row, int col, const float4 (&v)[4],
-                                              const bool (&ok)[4], bool with_d, bool whole, int dg) {
-  if (with_d) {
-    float* dst = e.Db + (long long)row * (int)p.ldd + col;
-    const long long step = 4LL * (int)p.ldd;
-#pragma unroll
-    for (int u = 0; u < 4; ++u, dst += step)
-      if (ok[u]) *reinterpret_cast<float4*>(dst) = v[u];
+// A warp's ring of kBufs staged blocks.  Every acquired block ends in exactly one bulk group, committed in the order of
+// acquisition, so "all but the kBufs - 1 newest groups have been read" frees the block acquired kBufs acquisitions ago.
+template <int kBufs>
+struct EpilogueRing {
+  uint32_t base;
+  int next = 0;
+  __device__ __forceinline__ uint32_t acquire(int lane) {
+    if (lane == 0) ptx::bulk_wait_read<kBufs - 1>();
+    __syncwarp();
+    const uint32_t buf = base + next * kEpiBlockBytes;
+    next = next + 1 == kBufs ? 0 : next + 1;
+    return buf;
   }
-  if (e.Hb) {
-    uint16_t* dst = e.Hb + (long long)row * (int)p.ld16 + col;
-    const long long step = 4LL * (int)p.ld16;
+};
+
+// One block of the result: v holds alpha * accumulator of this lane's row on entry.  `held`: a block of the ring that is
+// already this block's own (C arrived in it), 0 if none.  `whole`: a diagonal block of a mirrored symmetric result; it is
+// made symmetric from its upper half and written once.
+template <int kBufs>
+__device__ __forceinline__ void epilogue_block(const GemmParams& p, const EpilogueTile& e, EpilogueRing<kBufs>& ring, float (&v)[32],
+                                               uint32_t held, int b, int row_first, int c0, int lane, bool whole,
+                                               EpilogueSums& t) {
+  auto take = [&]() {
+    const uint32_t buf = held ? held : ring.acquire(lane);
+    held = 0;
+    return buf;
+  };
+  auto send = [&](auto&& stores) {   // what the lanes staged becomes visible to the copy engine, then one lane stores it
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      stores();
+      ptx::bulk_commit();
+    }
+  };
+  if (whole) {
+    if (!held) held = ring.acquire(lane);
+    stage_cols_f32(held, lane, v);
+    __syncwarp();
+    float4 r[8];
+    load_row_f32(held, lane, r);
 #pragma unroll
-    for (int u = 0; u < 4; ++u, dst += step)
-      if (ok[u]) *reinterpret_cast<uint2*>(dst) = pack4_16(v[u].x, v[u].y, v[u].z, v[u].w, p.d16_fmt);
+    for (int j = 0; j < 8; ++j) {
+      if (4 * j < lane) v[4 * j] = r[j].x;
+      if (4 * j + 1 < lane) v[4 * j + 1] = r[j].y;
+      if (4 * j + 2 < lane) v[4 * j + 2] = r[j].z;
+      if (4 * j + 3 < lane) v[4 * j + 3] = r[j].w;
+    }
+    __syncwarp();
   }
-  const long long sstep = 4LL * (int)p.s_ld;
-  if (e.S0b) {
-    __half* dst = e.S0b + (long long)row * (int)p.s_ld + col;
-    const float s0 = p.s0_scale;
+  const bool image = p.tri && p.mirror && !whole;   // the block below the diagonal is this lane's row as a column
+  if (e.stats) {   // (outside the matrix the results are zero: operands and C are read as zero there)
+    float s = 0.f, m = 0.f;
+    const bool diag = c0 == row_first && row_first + lane < p.M && row_first + lane < p.N;
 #pragma unroll
-    for (int u = 0; u < 4; ++u, dst += sstep) {
-      uint2 hi, lo;
-      split4(make_float4(s0 * v[u].x, s0 * v[u].y, s0 * v[u].z, s0 * v[u].w), hi, lo);
-      if (ok[u]) {
-        *reinterpret_cast<uint2*>(dst) = hi;
-        *reinterpret_cast<uint2*>(dst + p.s_plane) = lo;
+    for (int j = 0; j < 32; ++j) {
+      s = fmaf(v[j], v[j], s);
+      if (diag && j == lane) {   // the diagonal element's distance from the identity and its affine image are its own
+        t.mabs = fmaxf(t.mabs, fabsf(v[j]));
+        t.maff = fmaxf(t.maff, fabsf(fmaf(p.aff_b, v[j], p.aff_a)));
+        t.mres = fmaxf(t.mres, fabsf(1.f - v[j]));
+      } else {
+        m = fmaxf(m, fabsf(v[j]));
       }
     }
+    t.ssq += (p.tri && !whole) ? 2.f * s : s;    // a block above the diagonal counts for its mirror image as well
+    t.mabs = fmaxf(t.mabs, m);
+    t.maff = fmaxf(t.maff, fabsf(p.aff_b) * m);  // off the diagonal the affine map is a plain scaling
+    // and the distance from the identity is |d|; fmaxf drops NaN, the sum of squares does not
+    t.mres = fmaxf(t.mres, isfinite(s) ? m : INFINITY);
   }
-  if (e.S1b) {
-    __half* dst = e.S1b + (long long)row * (int)p.s_ld + col;
-    const float s1 = p.s1_scale * p.s1_aff_b, sd = whole ? p.s1_scale * p.s1_aff_a : 0.f;
-#pragma unroll
-    for (int u = 0; u < 4; ++u, dst += sstep) {
-      const int d = dg + 4 * u;
-      uint2 hi, lo;
-      split4(make_float4(fmaf(s1, v[u].x, d == 0 ? sd : 0.f), fmaf(s1, v[u].y, d == 1 ? sd : 0.f),
-                         fmaf(s1, v[u].z, d == 2 ? sd : 0.f), fmaf(s1, v[u].w, d == 3 ? sd : 0.f)), hi, lo);
-      if (ok[u]) {
-        *reinterpret_cast<uint2*>(dst) = hi;
-        *reinterpret_cast<uint2*>(dst + p.s_plane) = lo;
-      }
+  if (p.D) {
+    const uint32_t buf = take();
+    stage_rows_f32(buf, lane, v);
+    send([&]() { ptx::tma_store_3d(&p.d_map, buf, c0, row_first, b); });
+    if (image && !p.upper_d) {
+      const uint32_t tb = take();
+      stage_cols_f32(tb, lane, v);
+      send([&]() { ptx::tma_store_3d(&p.d_map, tb, row_first, c0, b); });
     }
   }
+  if (p.D16) {
+    uint32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) w[k] = pack2_16(v[2 * k], v[2 * k + 1], p.d16_fmt);
+    const uint32_t buf = take();
+    stage_rows_16(buf, lane, w);
+    if (image) stage_cols_16(buf + kEpiBlockBytes / 2, lane, w);
+    send([&]() {
+      ptx::tma_store_3d(&p.h_map, buf, c0, row_first, b);
+      if (image) ptx::tma_store_3d(&p.h_map, buf + kEpiBlockBytes / 2, row_first, c0, b);
+    });
+  }
+  // FP16 hi/lo planes of s * v (+ d on the diagonal): hi = rn(x), lo = rn(x - hi)
+  auto planes = [&](const CUtensorMap* map, float s, float d) {
+    uint32_t hi[16], lo[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float x = s * v[2 * k], y = s * v[2 * k + 1];
+      if (d != 0.f) {
+        if (2 * k == lane) x = fmaf(s, v[2 * k], d);
+        if (2 * k + 1 == lane) y = fmaf(s, v[2 * k + 1], d);
+      }
+      const __half2 h = __floats2half2_rn(x, y);
+      const float2 f = __half22float2(h);
+      const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+      hi[k] = *reinterpret_cast<const uint32_t*>(&h);
+      lo[k] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+    const uint32_t buf = take();
+    stage_rows_16(buf, lane, hi);
+    stage_rows_16(buf + kEpiBlockBytes / 2, lane, lo);
+    send([&]() {
+      ptx::tma_store_3d(map, buf, c0, row_first, b);
+      ptx::tma_store_3d(map, buf + kEpiBlockBytes / 2, c0, row_first, b + p.s_lo_z);
+    });
+    if (image) {
+      const uint32_t tb = take();
+      stage_cols_16(tb, lane, hi);
+      stage_cols_16(tb + kEpiBlockBytes / 2, lane, lo);
+      send([&]() {
+        ptx::tma_store_3d(map, tb, row_first, c0, b);
+        ptx::tma_store_3d(map, tb + kEpiBlockBytes / 2, row_first, c0, b + p.s_lo_z);
+      });
+    }
+  };
+  if (p.S0) planes(&p.s0_map, p.s0_scale, 0.f);
+  if (p.S1) planes(&p.s1_map, p.s1_scale * p.s1_aff_b, c0 == row_first ? p.s1_scale * p.s1_aff_a : 0.f);
 }
 
-// One block with 16-byte accesses: interior, at the matrix edge (N a multiple of four), or a diagonal block of a mirrored
-// symmetric result, which is written whole from its upper half.  One rolled loop over half blocks -- two for the block
-// itself, two for its mirror image (or, of a diagonal block, for all of it) -- so that the code stays small: an epilogue of
-// a short product runs once per SM from a cold instruction cache, and with two epilogue warps per scheduler the number of
-// instructions is what it costs (800 per block made it 3650 cycles, whatever was stored).
-// With kAhead the caller has loaded C of the block's first half; C of the next half (or of the next block, next_c0) is
-// fetched as soon as the registers are free, i.e. before the stores, so that its latency hides behind them.
-template <bool kAhead>
-__device__ __forceinline__ void epilogue_block_vec(const GemmParams& p, const EpilogueTile& e, float* stage, int row_first,
-                                                   int c0, int lane, bool holds_diag, float4 (&cv)[4], int next_c0,
-                                                   EpilogueSums& t) {
-  const int q = lane & 7, sub = lane >> 3;
-  const bool mirror = p.tri && p.mirror;
-  const bool whole = mirror && holds_diag;
-  const int halves = mirror ? 4 : 2;
-#pragma unroll 1
-  for (int h = 0; h < halves; ++h) {
-    const bool image = h >= 2;
-    const int i0 = 16 * (h & 1) + sub;
-    float4 v[4];
-    if (!image) {
-      if (!kAhead && e.use_c) epilogue_load_c(p, e, row_first + 16 * h, c0, lane, cv);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        v[u] = *reinterpret_cast<const float4*>(stage + stage_at(i0 + 4 * u, q));
-        v[u].x *= e.alpha; v[u].y *= e.alpha; v[u].z *= e.alpha; v[u].w *= e.alpha;
-      }
-      if (e.use_c) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          v[u].x = fmaf(e.beta, cv[u].x, v[u].x); v[u].y = fmaf(e.beta, cv[u].y, v[u].y);
-          v[u].z = fmaf(e.beta, cv[u].z, v[u].z); v[u].w = fmaf(e.beta, cv[u].w, v[u].w);
-        }
-        const int c = h ? next_c0 : c0;
-        if (kAhead && c >= 0) epilogue_load_c(p, e, h ? row_first : row_first + 16, c, lane, cv);
-      }
-      if (mirror) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(stage + stage_at(i0 + 4 * u, q)) = v[u];
-      }
-    } else {
-      if (h == 2) __syncwarp();
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + 4 * u;
-        float x[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {   // of a diagonal block, only the elements left of the diagonal are exchanged
-          const bool swap = !whole || 4 * q + k < i;
-          x[k] = stage_get(stage, swap ? 4 * q + k : i, swap ? i : 4 * q + k);
-        }
-        v[u] = make_float4(x[0], x[1], x[2], x[3]);
-      }
-    }
-    const int row = (image && !whole ? c0 : row_first) + i0, col = (image && !whole ? row_first : c0) + 4 * q;
-    bool ok[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) ok[u] = row + 4 * u < p.M && col < p.N;
-    if (whole == image || !whole) epilogue_emit(p, e, row, col, v, ok, e.Db && !(image && !whole && p.upper_d), whole, row - col);
-    if (e.stats && whole == image) {   // (outside the matrix the results are zero: operands and C are read as zero there)
-      float s = 0.f, m = 0.f;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          s = fmaf(x[k], x[k], s);
-          if (whole && row + 4 * u == col + k) {   // the diagonal element's distance from the identity is its own
-            if (ok[u]) {
-              t.mabs = fmaxf(t.mabs, fabsf(x[k]));
-              t.maff = fmaxf(t.maff, fabsf(fmaf(p.aff_b, x[k], p.aff_a)));
-              t.mres = fmaxf(t.mres, fabsf(1.f - x[k]));
-            }
-          } else {
-            m = fmaxf(m, fabsf(x[k]));
-          }
-        }
-      }
-      t.ssq += (p.tri && !whole) ? 2.f * s : s;    // a block above the diagonal counts for its mirror image as well
-      t.mabs = fmaxf(t.mabs, m);
-      t.maff = fmaxf(t.maff, fabsf(p.aff_b) * m);  // off the diagonal the affine map is a plain scaling
-      // and the distance from the identity is |d|; fmaxf drops NaN, the sum of squares does not
-      t.mres = fmaxf(t.mres, isfinite(s) ? m : INFINITY);
-    }
-  }
-  __syncwarp();
-}
+// Element of a block staged by stage_rows_f32.
+__device__ __forceinline__ int stage_at(int row, int col) { return row * 32 + (((col >> 2) ^ (row & 7)) << 2) + (col & 3); }
 
-// Any other block (packed or unaligned output): one element per lane with full masking, lane = column, so rows -- also
-// rows of a packed triangle -- are still written as contiguous runs; the mirrored half with lane = source row.  C is
-// fetched eight rows at a time.
+// Any other block (packed or unaligned output; a diagonal block of a symmetric result that is not mirrored), from its rows
+// staged in FP32: one element per lane with full masking, lane = column, so rows -- also rows of a packed triangle -- are
+// still written as contiguous runs; the mirrored half with lane = source row.  C is fetched eight rows at a time.
+// v = acc here, not yet scaled.
+
 __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const EpilogueTile& e, float* stage, int row_first,
                                                       int c0, int lane, EpilogueSums& t) {
   const int col = c0 + lane;
@@ -392,7 +400,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int i = i0 + u, row = row_first + i;
-      float* const at = stage + stage_at(i, lane >> 2) + (lane & 3);
+      float* const at = stage + stage_at(i, lane);
       float v = 0.f;
       if (row < p.M && col_ok && !(p.tri && col < row)) {
         v = e.alpha * *at;
@@ -420,7 +428,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
       for (int j = 0; j < cols; ++j) {
         const int c = c0 + j;
         if (c > row) {
-          const float v = stage_get(stage, lane, j);
+          const float v = stage[stage_at(lane, j)];
           if (e.Db && !p.upper_d) e.Db[(long long)c * p.ldd + row] = v;
           if (e.Hb) e.Hb[(long long)c * p.ld16 + row] = to_bits16(v, p.d16_fmt);
           if (e.S0b) store_split1(e.S0b + (long long)c * p.s_ld + row, p.s_plane, p.s0_scale * v);
@@ -452,14 +460,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* const smem = smem_raw + (base - raw);
-  // barrier block after the tiles
-  const uint32_t bars = base + S::kTileBytes;
+  // barrier block after the tiles and the epilogue's blocks
+  const uint32_t bars = base + S::kTileBytes + S::kEpiBytes;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (S::kStages + s); };
   auto tfull_bar = [&](int s) { return bars + 8u * (2 * S::kStages + s); };
   auto tempty_bar = [&](int s) { return bars + 8u * (2 * S::kStages + 2 + s); };
-  volatile uint32_t* const tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + S::kTileBytes + 8 * (2 * S::kStages + 4));
-  volatile int* const abort_flag = reinterpret_cast<volatile int*>(smem + S::kTileBytes + 8 * (2 * S::kStages + 4) + 8);
+  auto c_bar = [&](int w) { return bars + 8u * (2 * S::kStages + 4 + w); };   // C blocks of epilogue warp w
+  constexpr int kAfterBars = S::kTileBytes + S::kEpiBytes + 8 * (2 * S::kStages + 12);
+  static_assert(8 * (2 * S::kStages + 12) + 16 <= S::kBarBytes, "barrier block");
+  volatile uint32_t* const tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kAfterBars);
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(smem + kAfterBars + 8);
   // A role that gives up stops its own CTA and, in a pair, the peer as well: both CTAs' roles poll their CTA's flag
   // between waits, so neither keeps issuing copies or MMAs for two more seconds.  The peer's shared memory is valid
   // until the closing cluster barrier, which every thread of both CTAs reaches.
@@ -522,6 +533,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       // one arrival per epilogue warp (of both CTAs of a pair); per half of a wide tile: the four warps that read it
       ptx::mbar_init(tempty_bar(s), kWide ? 8 : (kPair ? 16 : 8));
     }
+    for (int w = 0; w < 8; ++w) ptx::mbar_init(c_bar(w), 1);
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -746,7 +758,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     constexpr int NCH = BN / 64;  // 32-column chunks per warp
     const int lane_group = warp & 3;
     const int half = (warp - 4) >> 2;
-    float* const stage = reinterpret_cast<float*>(smem + S::kTileBytes + S::kBarBytes) + (warp - 4) * kEpiWarpFloats;
+    const int ew = warp - 4;
+    EpilogueRing<S::kEpiBufs> ring{base + S::kTileBytes + ew * S::kEpiBufs * kEpiBlockBytes};
+    uint32_t c_buf = 0, c_phase = 0;   // block of the ring C is arriving in (0: none), parity of its barrier
     constexpr bool chained = kChained;
     // Running sums of the accumulation chains (chained products only), added with round-to-nearest: the
     // tensor core itself adds into its accumulator by truncation.
@@ -760,8 +774,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN;  // this CTA's 128 rows of the tile
       const int row_first = m0 + lane_group * 32;
       const int col_first = n0 + half * (BN / 2);
-      // 32-column blocks this warp never needs: beyond N, or wholly below the diagonal (warp-uniform)
-      auto needed = [&](int c0) { return (c0 < p.N) && !(p.tri && c0 + 31 < row_first); };
+      // 32-column blocks this warp never needs: outside the matrix, or wholly below the diagonal (warp-uniform)
+      auto needed = [&](int c0) { return c0 < p.N && row_first < p.M && !(p.tri && c0 + 31 < row_first); };
       auto wait_chain = [&](int buf) {
         const long long w0 = p.prof ? clock64() : 0;
         // every lane observes the barrier itself, so each one is ordered after the MMAs' TMEM writes
@@ -798,27 +812,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       if (p.beta_v) e.beta *= __ldg(p.beta_v + b);
       e.use_c = (p.C != nullptr) && (e.beta != 0.f);
       e.stats = p.sumsq || p.maxabs || p.maxaff || p.maxres;
-      e.Cb = p.C ? p.C + (long long)b * p.c_bs : nullptr;
-      e.Db = p.D ? p.D + (long long)b * p.d_bs : nullptr;
-      e.Hb = p.D16 ? reinterpret_cast<uint16_t*>(p.D16) + (long long)b * p.d16_bs : nullptr;
-      e.S0b = p.S0 ? p.S0 + (long long)b * p.s_bs : nullptr;
-      e.S1b = p.S1 ? p.S1 + (long long)b * p.s_bs : nullptr;
       // the blocks this warp writes: a contiguous run of its NCH 32-column blocks (warp-uniform)
       int cc_first = 0, cc_end = NCH;
       while (cc_first < NCH && !needed(col_first + cc_first * 32)) ++cc_first;
       while (cc_end > cc_first && !needed(col_first + (cc_end - 1) * 32)) --cc_end;
-      const bool rows_inside = row_first + 32 <= p.M;
-      // warp-uniform choice of the 16-byte path; a symmetric result that is not mirrored keeps its lower triangle untouched,
-      // and diagonal elements that need their own treatment are looked after where a diagonal block is written whole
-      auto vectorised = [&](int c0) {
-        const bool holds_diag = c0 <= row_first + 31 && c0 + 31 >= row_first;
-        const bool plain_diag = holds_diag && (p.tri ? !p.mirror : (p.maxaff || p.maxres || p.S1));
-        return p.vec_ok && ((rows_inside && c0 + 32 <= p.N) || p.N % 4 == 0) && !plain_diag;
+      // Boxes move by TMA unless an address or stride rules it out; a symmetric result that is not mirrored keeps its lower
+      // triangle untouched, which a box across the diagonal would not.
+      auto boxed = [&](int c0) { return p.tma_ok && !(p.tri && !p.mirror && c0 <= row_first + 31); };
+      // C of a block is fetched into the ring as soon as the block before it has been staged -- of the tile's first block,
+      // while the accumulator is still being formed.
+      auto fetch_c = [&](int cc) {
+        if (!e.use_c || cc >= cc_end || !boxed(col_first + cc * 32)) return;
+        c_buf = ring.acquire(lane);
+        if (lane == 0) {
+          ptx::mbar_expect_tx(c_bar(ew), kEpiBlockBytes);
+          ptx::tma_load_3d(c_buf, &p.c_map, c_bar(ew), col_first + cc * 32, row_first, b);
+        }
       };
-      // C of the first block is fetched while the accumulator is still being formed
-      float4 cv[4];
-      if (!chained && e.use_c && cc_first < cc_end && vectorised(col_first + cc_first * 32))
-        epilogue_load_c(p, e, row_first, col_first + cc_first * 32, lane, cv);
+      fetch_c(cc_first);
 
       if (chained) {
 #pragma unroll
@@ -854,27 +865,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         break;
       }
 
-      // ---- write the tile: one rolled loop over the warp's 32 x 32 blocks, staged through shared memory
+      // ---- write the tile: one rolled loop over the warp's 32 x 32 blocks
       const long long o0 = p.prof ? clock64() : 0;
       EpilogueSums sums;
       const uint32_t taddr = tmem_of(kWide ? 0 : (int)(gchunk & 1u));
 #pragma unroll 1
       for (int cc = cc_first; cc < cc_end; ++cc) {
         const int c0 = col_first + cc * 32;
-        auto put = [&](int j, float x0, float x1, float x2, float x3) {
-          *reinterpret_cast<float4*>(stage + stage_at(lane, j)) = make_float4(x0, x1, x2, x3);
-        };
+        float v[32];
         if constexpr (chained) {
           // the running sums live in registers: static indices only
-          auto put_sums = [&](auto first) {
-            constexpr int o = decltype(first)::value;
+          auto take_sums = [&](auto first) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) put(j, racc[o + 4 * j], racc[o + 4 * j + 1], racc[o + 4 * j + 2], racc[o + 4 * j + 3]);
+            for (int j = 0; j < 32; ++j) v[j] = racc[decltype(first)::value + j];
           };
-          if (cc == 0) put_sums(std::integral_constant<int, 0>());
-          if (cc == 1) put_sums(std::integral_constant<int, chained ? 32 : 0>());
-          if (cc == 2) put_sums(std::integral_constant<int, (chained && NCH > 2) ? 64 : 0>());
-          if (cc == 3) put_sums(std::integral_constant<int, (chained && NCH > 2) ? 96 : 0>());
+          if (cc == 0) take_sums(std::integral_constant<int, 0>());
+          if (cc == 1) take_sums(std::integral_constant<int, chained ? 32 : 0>());
+          if (cc == 2) take_sums(std::integral_constant<int, (chained && NCH > 2) ? 64 : 0>());
+          if (cc == 3) take_sums(std::integral_constant<int, (chained && NCH > 2) ? 96 : 0>());
         } else {
           uint32_t raw[32];
           ptx::tmem_ld32(taddr + (uint32_t)(cc * 32), raw);
@@ -883,21 +891,52 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           // half `half` only, and that half's barrier counts its four lane groups of both CTAs)
           if (cc == cc_end - 1) release(kWide ? half : (int)(gchunk & 1u));
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            put(j, __uint_as_float(raw[4 * j]), __uint_as_float(raw[4 * j + 1]), __uint_as_float(raw[4 * j + 2]),
-                __uint_as_float(raw[4 * j + 3]));
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
         }
-        __syncwarp();
-        if (vectorised(c0)) {
-          const int next = (cc + 1 < cc_end && vectorised(c0 + 32)) ? c0 + 32 : -1;
-          epilogue_block_vec<!kChained>(p, e, stage, row_first, c0, lane, c0 <= row_first + 31 && c0 + 31 >= row_first, cv,
-                                           next, sums);
+        if (boxed(c0)) {
+          const uint32_t held = c_buf;
+          if (held) {
+            const bool got = __all_sync(0xffffffffu, ptx::mbar_wait(c_bar(ew), c_phase, kWaitCycles) ? 1 : 0);
+            if (!got || *abort_flag) {
+              if (lane == 0) {
+                report(p.status, kTimeoutEpilogue);
+                raise_abort();
+              }
+              alive = false;
+              break;
+            }
+            c_buf = 0;
+            c_phase ^= 1u;
+            float4 r[8];
+            load_row_f32(held, lane, r);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              v[4 * j] = fmaf(e.beta, r[j].x, e.alpha * v[4 * j]);
+              v[4 * j + 1] = fmaf(e.beta, r[j].y, e.alpha * v[4 * j + 1]);
+              v[4 * j + 2] = fmaf(e.beta, r[j].z, e.alpha * v[4 * j + 2]);
+              v[4 * j + 3] = fmaf(e.beta, r[j].w, e.alpha * v[4 * j + 3]);
+            }
+            __syncwarp();   // every lane has its row of C: the block is free for the result
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] *= e.alpha;
+          }
+          epilogue_block<S::kEpiBufs>(p, e, ring, v, held, b, row_first, c0, lane, p.tri && p.mirror && c0 == row_first, sums);
         } else {
-          epilogue_block_scalar(p, e, stage, row_first, c0, lane, sums);
-          if (!chained && e.use_c && cc + 1 < cc_end && vectorised(c0 + 32))
-            epilogue_load_c(p, e, row_first, c0 + 32, lane, cv);
+          const uint32_t buf = ring.acquire(lane);
+          stage_rows_f32(buf, lane, v);
+          __syncwarp();
+          e.Cb = p.C ? p.C + (long long)b * p.c_bs : nullptr;
+          e.Db = p.D ? p.D + (long long)b * p.d_bs : nullptr;
+          e.Hb = p.D16 ? reinterpret_cast<uint16_t*>(p.D16) + (long long)b * p.d16_bs : nullptr;
+          e.S0b = p.S0 ? p.S0 + (long long)b * p.s_bs : nullptr;
+          e.S1b = p.S1 ? p.S1 + (long long)b * p.s_bs : nullptr;
+          epilogue_block_scalar(p, e, reinterpret_cast<float*>(smem + (buf - base)), row_first, c0, lane, sums);
+          if (lane == 0) ptx::bulk_commit();   // (nothing in flight: the ring counts one group per block)
         }
+        fetch_c(cc + 1);
       }
+      if (!alive) break;
       if (!chained) {
         if (cc_first >= cc_end) release(kWide ? half : (int)(gchunk & 1u));   // nothing of this tile is this warp's to read
         ++gchunk;
@@ -919,6 +958,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           if (p.maxres) atomicMax(p.maxres + b, __float_as_uint(sums.mres));
         }
       }
+    }
+    if (lane == 0) {
+      if (c_buf) ptx::mbar_wait(c_bar(ew), c_phase, kDrainCycles);   // (gave up with a block of C on its way)
+      ptx::bulk_wait_all();   // the stores have read shared memory and are written before the CTA ends
     }
     if (p.prof && leader && warp == 4 && lane == 0) {
       atomicAdd(p.prof + 4, (unsigned long long)prof_wait);

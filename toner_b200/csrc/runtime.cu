@@ -106,6 +106,21 @@ static int encode_one(CUtensorMap* out, const void* base, int rows, int cols, lo
   return 0;
 }
 
+// Map of the 32 x 32 boxes in which the GEMM's epilogue moves C and the results (elt: 4 = FP32, 2 = 16-bit).  False where
+// the addresses or strides are not what TMA takes; the epilogue then goes element by element.
+static bool encode_box(CUtensorMap* out, const void* base, int rows, int cols, long long ld, long long bs, int nz, int elt) {
+  const long long zs = nz > 1 ? bs : (long long)rows * ld;
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) || (ld * elt) % 16 || (zs * elt) % 16 || ld < cols || zs <= 0) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)nz};
+  const cuuint64_t strides[2] = {(cuuint64_t)(ld * elt), (cuuint64_t)(zs * elt)};
+  const cuuint32_t box[3] = {32u, 32u, 1u};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  return g_encode(out, elt == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base),
+                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  elt == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cudaStream_t stream, const CUtensorMap** out) {
   const int count = op.list ? batch : 1;
   const int brows = op.mn_major ? 64 : box_rows;
@@ -240,15 +255,17 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   p.packed = d.packed ? 1 : 0;
   p.mirror = d.mirror ? 1 : 0;
   p.upper_d = (d.upper_d && d.tri && d.mirror) ? 1 : 0;
-  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-  p.vec_ok = !d.packed && (!d.c || (d.ldc % 4 == 0 && d.c_bs % 4 == 0 && al16(d.c))) &&
-             (!d.d || (d.ldd % 4 == 0 && d.d_bs % 4 == 0 && al16(d.d))) &&
-             (!d.d16 || (d.ld16 % 4 == 0 && d.d16_bs % 4 == 0 && (reinterpret_cast<uintptr_t>(d.d16) & 7u) == 0));
-  if (d.split0 || d.split1) {
-    const bool ok = d.split_ld % 4 == 0 && d.split_bs % 4 == 0 && d.split_plane % 4 == 0 &&
-                    (!d.split0 || (reinterpret_cast<uintptr_t>(d.split0) & 7u) == 0) &&
-                    (!d.split1 || (reinterpret_cast<uintptr_t>(d.split1) & 7u) == 0);
-    p.vec_ok = p.vec_ok && ok;
+  p.tma_ok = !d.packed;
+  if (p.tma_ok && d.c) p.tma_ok = encode_box(&p.c_map, d.c, d.m, d.n, d.ldc, d.c_bs, d.batch, 4);
+  if (p.tma_ok && d.d) p.tma_ok = encode_box(&p.d_map, d.d, d.m, d.n, d.ldd, d.d_bs, d.batch, 4);
+  if (p.tma_ok && d.d16) p.tma_ok = encode_box(&p.h_map, d.d16, d.m, d.n, d.ld16, d.d16_bs, d.batch, 2);
+  if (p.tma_ok && (d.split0 || d.split1)) {
+    // the lo plane is reached through the batch coordinate: a whole number of batch strides behind the hi plane
+    const long long step = d.batch > 1 ? d.split_bs : d.split_plane;
+    p.tma_ok = step > 0 && d.split_plane > 0 && d.split_plane % step == 0 && d.split_plane / step < (1 << 30);
+    p.s_lo_z = p.tma_ok ? (int)(d.split_plane / step) : 0;
+    if (p.tma_ok && d.split0) p.tma_ok = encode_box(&p.s0_map, d.split0, d.m, d.n, d.split_ld, step, p.s_lo_z + d.batch, 2);
+    if (p.tma_ok && d.split1) p.tma_ok = encode_box(&p.s1_map, d.split1, d.m, d.n, d.split_ld, step, p.s_lo_z + d.batch, 2);
   }
   p.S0 = static_cast<__half*>(d.split0); p.S1 = static_cast<__half*>(d.split1);
   p.s_ld = d.split_ld; p.s_bs = d.split_bs; p.s_plane = d.split_plane;
