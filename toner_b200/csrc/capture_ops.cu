@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(32 * kCaptureWarps) capture_rows_kernel(const 
                                                                           const long long* __restrict__ at,
                                                                           const long long* __restrict__ idx, int rows, int P,
                                                                           float eps) {
+  ptx::pdl_begin();
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * kCaptureWarps + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -148,9 +149,7 @@ extern "C" int toner_capture(const toner_capture_job* jobs_device, const toner_c
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const dim3 grid((unsigned)((rows + kCaptureWarps - 1) / kCaptureWarps), (unsigned)n_jobs);
-  capture_rows_kernel<<<grid, 32 * kCaptureWarps, 0, stream>>>(jobs_device, reinterpret_cast<const long long*>(at),
-                                                             reinterpret_cast<const long long*>(idx), (int)rows, positions, eps);
-  count_launch();
+  TONER_LAUNCH(capture_rows_kernel, grid, 32 * kCaptureWarps, stream, jobs_device, reinterpret_cast<const long long*>(at), reinterpret_cast<const long long*>(idx), (int)rows, positions, eps);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }

@@ -215,6 +215,7 @@ static int default_iterations(double l0, int p) {
 
 // ------------------------------------------------------------------ elementwise helpers
 __global__ void __launch_bounds__(256) trace_kernel(const float* __restrict__ c, int n, float* __restrict__ trace) {
+  ptx::pdl_begin();
   const int b = blockIdx.x;
   const float* C = c + (long long)b * n * n;
   float s = 0.f;
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(256) trace_kernel(const float* __restrict__ c,
 // 32x32 tile pairs so that C and C^T are both read along rows.
 __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, float* __restrict__ a, int n, float damping,
                                                    const float* __restrict__ trace) {
+  ptx::pdl_begin();
   const int ti = blockIdx.y, tj = blockIdx.x;
   if (ti > tj) return;
   __shared__ float up[32][33], lo[32][33];
@@ -276,9 +278,10 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
                                                           const float* __restrict__ sumsq, float a, float b, float s_m,
                                                           float s_t, __half* __restrict__ m_planes,
                                                           __half* __restrict__ t_planes, __half* __restrict__ x_planes,
-                                                          const float* __restrict__ defl_v = nullptr,
-                                                          const float* __restrict__ defl_coef = nullptr, int defl_r = 0,
-                                                          int vstride = 0) {
+                                                          const float* __restrict__ defl_v,
+                                                          const float* __restrict__ defl_coef, int defl_r,
+                                                          int vstride) {
+  ptx::pdl_begin();
   const int bi = blockIdx.y;
   float cf[8];
   bool any = false;
@@ -348,6 +351,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
 
 // v_0: a fixed pattern of +-1 / sqrt(n)
 __global__ void power_start_kernel(float* __restrict__ v, int n) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float s = rsqrtf((float)n);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -357,6 +361,7 @@ __global__ void power_start_kernel(float* __restrict__ v, int n) {
 // y = A v, one warp per row, FP64 accumulation
 __global__ void __launch_bounds__(256) gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
                                                    float* __restrict__ y, int n) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= n) return;
@@ -380,6 +385,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const float* __restrict__ a, 
 // The residual is summed term by term: the shortcut ||y||^2 - lambda^2 cancels catastrophically.
 __global__ void __launch_bounds__(256) power_norm_kernel(float* __restrict__ v, const float* __restrict__ y, int n,
                                                          float* __restrict__ lam, float* __restrict__ res) {
+  ptx::pdl_begin();
   const int b = blockIdx.x;
   float* V = v + (long long)b * n;
   const float* Y = y + (long long)b * n;
@@ -436,6 +442,7 @@ __global__ void __launch_bounds__(256) power_norm_kernel(float* __restrict__ v, 
 // sigma = lambda_1 - c if the pair converged and stands well above the rest, else 0;  corr = lambda_1^{-1/p} - c^{-1/p}
 __global__ void deflate_decide_kernel(const float* __restrict__ lam, const float* __restrict__ res, int k, int n,
                                       float damping, int p, float* __restrict__ neg_sigma, float* __restrict__ corr) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   const float l1 = lam[b];
@@ -449,6 +456,7 @@ __global__ void deflate_decide_kernel(const float* __restrict__ lam, const float
 // A_b += coef[b] v_b v_b^T  (skipped where coef is zero)
 __global__ void __launch_bounds__(256) rank1_update_kernel(float* __restrict__ a, const float* __restrict__ v,
                                                            const float* __restrict__ coef, int n) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float cf = coef[b];
   if (cf == 0.f) return;
@@ -486,6 +494,7 @@ constexpr int kBlockGemvRows = 32;
 template <int R>
 __global__ void __launch_bounds__(256) block_gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
                                                          float* __restrict__ y, int n, int r, int vstride) {
+  ptx::pdl_begin();
   __shared__ float4 sv[R][64];
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -647,6 +656,7 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
 // start vectors: the caller's vectors (warm), or r different fixed +-1 patterns (cold, and for a slot that holds
 // nothing yet because the rank grew since the last call), orthonormalised
 __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v, int n, int r, int vstride, int cold) {
+  ptx::pdl_begin();
   __shared__ double red[8];
   __shared__ double part[8 * kPairs], gram[kPairs];
   __shared__ double L[kMaxDeflate][kMaxDeflate];
@@ -683,6 +693,7 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
 // over the two blocks of vectors; every reduction is taken for all pairs at once.
 __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float* __restrict__ y, int n, int r, int vstride,
                                                    int last, float* __restrict__ theta, float* __restrict__ res) {
+  ptx::pdl_begin();
   constexpr int R = kMaxDeflate;
   __shared__ double part[8 * R * R], sums[R * R];
   __shared__ double H[R][R], Q[R][R], lam[R], L[R][R];
@@ -817,6 +828,7 @@ __global__ void block_decide_kernel(const float* __restrict__ theta, const float
                                     float damping, int p, float* __restrict__ coef, float* __restrict__ corr,
                                     int* __restrict__ count, float* __restrict__ rest_top, int* __restrict__ rest_idx,
                                     float* __restrict__ rest_trace) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   const double tr = (double)n * (1.0 + (double)damping);  // A has unit mean diagonal plus the damping
@@ -860,6 +872,7 @@ __global__ void block_decide_kernel(const float* __restrict__ theta, const float
 constexpr float kRitzGrow = 1.4f;
 __global__ void ritz_norm_kernel(float* __restrict__ bound2, const float* __restrict__ rest_top,
                                  const float* __restrict__ rest_trace, int k) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   const float cap = rest_trace[b];      // ||A'||_F <= trace(A') for a positive matrix: costs no pass over A'
@@ -873,6 +886,7 @@ __global__ void ritz_norm_kernel(float* __restrict__ bound2, const float* __rest
 __global__ void __launch_bounds__(256) pick_vector_kernel(const float* __restrict__ first, const float* __restrict__ v,
                                                           const int* __restrict__ idx, float* __restrict__ out, int n,
                                                           int vstride) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const int j = idx[b];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -885,6 +899,7 @@ __global__ void __launch_bounds__(256) pick_vector_kernel(const float* __restric
 // product v_r v_c has the same bits at (r, c) and (c, r) and the terms are added in the same order)
 __global__ void __launch_bounds__(256) rankr_update_kernel(float* __restrict__ a, const float* __restrict__ v,
                                                            const float* __restrict__ coef, int n, int r, int vstride) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   float cf[kMaxDeflate];
   bool any = false;
@@ -919,6 +934,7 @@ __global__ void __launch_bounds__(256) rankr_update_kernel(float* __restrict__ a
 // bound^2 <- bound^2 * t^2 with t the smallest of the three, 3 % above it for the single-pass products' rounding.
 __global__ void tighten_bound_kernel(float* __restrict__ bound2, const float* __restrict__ ss2, const float* __restrict__ ss4,
                                      const float* __restrict__ ss8, int k) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   float t = 1.f;
@@ -939,7 +955,8 @@ __global__ void tighten_bound_kernel(float* __restrict__ bound2, const float* __
 // the incoming v, 1 - v.y / v.v (0 where v is zero: nothing is known).
 // Vector j = blockIdx.y of statistic b sits at (b * vs + j) * n; its quotient goes to e[j * e_stride + b].
 __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v, const float* __restrict__ y, int n,
-                                                          float* __restrict__ e, int vs = 1, long long e_stride = 0) {
+                                                          float* __restrict__ e, int vs, long long e_stride) {
+  ptx::pdl_begin();
   const int b = blockIdx.x;
   float* V = v + ((long long)b * vs + blockIdx.y) * n;
   const float* Y = y + ((long long)b * vs + blockIdx.y) * n;
@@ -980,6 +997,7 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
 // schedule was built for: the caller's estimate of the spectrum's lower end was too high for this statistic.
 __global__ void verify_kernel(const float* __restrict__ e_est, const float* __restrict__ e_top, float e_allowed,
                               int* __restrict__ status, float* __restrict__ e_out, int k) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   float e = e_est[b];
@@ -991,6 +1009,7 @@ __global__ void verify_kernel(const float* __restrict__ e_est, const float* __re
 // lmin[b] = theta^(-power): the smallest eigenvalue of A from the largest eigenvalue theta (a Rayleigh quotient, so a
 // lower estimate) of its computed inverse root A^(-1/power).
 __global__ void lmin_from_root_kernel(const float* __restrict__ theta, float power, float* __restrict__ lmin, int k) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   const float t = theta[b];
@@ -1006,6 +1025,7 @@ __global__ void lmin_from_root_kernel(const float* __restrict__ theta, float pow
 __global__ void finish_kernel(const unsigned int* __restrict__ resid, const float* __restrict__ sumsq_a,
                               float* root_scale_lo, int* status, float* norm_out, int k, int p, float tol, float damping,
                               float lower_used, unsigned int* __restrict__ root_max_bits, float root_bound) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
   root_max_bits[b] = __float_as_uint(root_bound);
@@ -1221,49 +1241,35 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
 
     const float* C = ema + (long long)k0 * nn;
     const int t32 = (n + 31) / 32;
-    trace_kernel<<<kc, 256, 0, stream>>>(C, n, trace);
-    count_launch();
-    damp_kernel<<<dim3(t32, t32, kc), 256, 0, stream>>>(C, A32, n, damping, trace);
-    count_launch();
+    TONER_LAUNCH(trace_kernel, kc, 256, stream, C, n, trace);
+    TONER_LAUNCH(damp_kernel, dim3(t32, t32, kc), 256, stream, C, A32, n, damping, trace);
     if (defl_r > 0) {
       // dominant directions: block power iteration with Rayleigh-Ritz on the caller's vectors (eight sweeps from fixed
       // vectors -- the first three or four only find the subspace --, four from last call's), then deflate those that
       // converged and stand above the rest
-      block_start_kernel<<<kc, 256, 0, stream>>>(dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0);
-      count_launch();
+      TONER_LAUNCH(block_start_kernel, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0);
       const int sweeps = defl_cold ? 8 : 4;
       for (int sw = 0; sw < sweeps; ++sw) {
         const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
-        if (defl_r <= 2) block_gemv_kernel<2><<<bg, 256, 0, stream>>>(A32, dv, py, n, defl_r, kMaxDeflate);
-        else if (defl_r <= 4) block_gemv_kernel<4><<<bg, 256, 0, stream>>>(A32, dv, py, n, defl_r, kMaxDeflate);
-        else if (defl_r <= 6) block_gemv_kernel<6><<<bg, 256, 0, stream>>>(A32, dv, py, n, defl_r, kMaxDeflate);
-        else block_gemv_kernel<8><<<bg, 256, 0, stream>>>(A32, dv, py, n, defl_r, kMaxDeflate);
-        count_launch();
-        ritz_kernel<<<kc, 256, 0, stream>>>(dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
-        count_launch();
+        if (defl_r <= 2) TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+        else if (defl_r <= 4) TONER_LAUNCH(block_gemv_kernel<4>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+        else if (defl_r <= 6) TONER_LAUNCH(block_gemv_kernel<6>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+        else TONER_LAUNCH(block_gemv_kernel<8>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+        TONER_LAUNCH(ritz_kernel, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
       }
-      block_decide_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(th8, res8, kc, n, defl_r, damping, p, coef8, corr8,
-                                                               deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx,
-                                                               rest_trace);
-      count_launch();
+      TONER_LAUNCH(block_decide_kernel, (kc + 127) / 128, 128, stream, th8, res8, kc, n, defl_r, damping, p, coef8, corr8, deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx, rest_trace);
       if (!ritz_norm) {   // (with the norm estimate the deflation is applied where the operand planes are formed)
-        rankr_update_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(A32, dv, coef8, n, defl_r, kMaxDeflate);
-        count_launch();
+        TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, dv, coef8, n, defl_r, kMaxDeflate);
       }
     } else {
       // dominant direction: six power-iteration steps, then deflate where they converged
-      power_start_kernel<<<dim3(8, kc), 256, 0, stream>>>(pv, n);
-      count_launch();
+      TONER_LAUNCH(power_start_kernel, dim3(8, kc), 256, stream, pv, n);
       for (int pi = 0; pi < kPowerSteps; ++pi) {
-        gemv_kernel<<<dim3((n + 7) / 8, kc), 256, 0, stream>>>(A32, pv, py, n);
-        count_launch();
-        power_norm_kernel<<<kc, 256, 0, stream>>>(pv, py, n, lam, pres);
-        count_launch();
+        TONER_LAUNCH(gemv_kernel, dim3((n + 7) / 8, kc), 256, stream, A32, pv, py, n);
+        TONER_LAUNCH(power_norm_kernel, kc, 256, stream, pv, py, n, lam, pres);
       }
-      deflate_decide_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(lam, pres, kc, n, damping, p, neg_sigma, corr);
-      count_launch();
-      rank1_update_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(A32, pv, neg_sigma, n);
-      count_launch();
+      TONER_LAUNCH(deflate_decide_kernel, (kc + 127) / 128, 128, stream, lam, pres, kc, n, damping, p, neg_sigma, corr);
+      TONER_LAUNCH(rank1_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, pv, neg_sigma, n);
     }
     TONER_CUDA(cudaGetLastError());
     if (!ritz_norm) {
@@ -1274,17 +1280,11 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
     if (ritz_norm) {
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
-      ritz_norm_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(sumsq_a, rest_top, rest_trace, kc);
-      count_launch();
-      init_planes_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b,
-                                                                  s_m, s_t, Mb[0], Tb[0], Xb[1], dv, coef8, defl_r,
-                                                                  kMaxDeflate);
-      count_launch();
+      TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Tb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate);
       TONER_CUDA(cudaGetLastError());
     } else {
-    init_planes_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m,
-                                                                s_t, Mb[0], nullptr, nullptr);
-    count_launch();
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, nullptr, 0, 0);
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -1325,11 +1325,8 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       if (rc1) return rc1;
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
-      tighten_bound_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(sumsq_a, ss2, ss4, ss8, kc);
-      count_launch();
-      init_planes_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b,
-                                                                  s_m, s_t, Mb[0], Tb[0], Xb[1]);
-      count_launch();
+      TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Tb[0], Xb[1], nullptr, nullptr, 0, 0);
       TONER_CUDA(cudaGetLastError());
     }
     }
@@ -1381,10 +1378,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         x_bound = std::min(x_bound * sched[it].a, x_cap);
         if (last) {
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          finish_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(resid, sumsq_a, scale_lo, status ? status + k0 : nullptr,
-                                                            norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping,
-                                                            lower_used, max_r, (float)root_bound);
-          count_launch();
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping, lower_used, max_r, (float)root_bound);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  Horner steps
           // W_j = c_j R + R W_{j+1} (W_m = c_m R) build q(R) = c_0 I + W_1; the terms linear in M enter in FP32 as
@@ -1416,9 +1410,8 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
           rc = sym_product(Xcur, s_x, Mb[1], s_f, o, kPromoteX);
           if (rc) return rc;
           // put the deflated direction back: A^{-1/p} = A'^{-1/p} + (lambda_1^{-1/p} - c^{-1/p}) v v^T
-          if (defl_r > 0) rankr_update_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(R, dv, corr8, n, defl_r, kMaxDeflate);
-          else rank1_update_kernel<<<dim3(ew_blocks, kc), 256, 0, stream>>>(R, pv, corr, n);
-          count_launch();
+          if (defl_r > 0) TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, R, dv, corr8, n, defl_r, kMaxDeflate);
+          else TONER_LAUNCH(rank1_update_kernel, dim3(ew_blocks, kc), 256, stream, R, pv, corr, n);
           TONER_CUDA(cudaGetLastError());
           rc = sumsq_det(R, kc, n, n, n, nn, partials, fro_tmp, stream);
           if (rc) return rc;
@@ -1527,29 +1520,20 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
           // and lag the same way; they belong to the top of A', so the same four steps from the largest Ritz vector
           // that stayed in A' find them.  (An eigenvalue beyond a / b, where T changes sign, makes M grow instead and
           // fails the convergence test.)  Both starting vectors go through M in one pass per step.
-          pick_vector_kernel<<<dim3(8, kc), 256, 0, stream>>>(vt, dv, rest_idx, pv, n, kMaxDeflate);
-          count_launch();
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate);
           const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
           for (int sw = 0; sw < 4; ++sw) {
-            block_gemv_kernel<2><<<bg, 256, 0, stream>>>(A32, pv, py, n, 2, 2);
-            count_launch();
-            power_shift_kernel<<<dim3(kc, 2), 256, 0, stream>>>(pv, py, n, e_est, 2, (long long)(e_top - e_est));
-            count_launch();
+            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, pv, py, n, 2, 2);
+            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est));
           }
         } else {
           TONER_CUDA(cudaMemcpyAsync(pv, vt, sizeof(float) * (size_t)kc * n, cudaMemcpyDeviceToDevice, stream));
           for (int sw = 0; sw < 4; ++sw) {
-            gemv_kernel<<<dim3((n + 7) / 8, kc), 256, 0, stream>>>(A32, pv, py, n);
-            count_launch();
-            power_shift_kernel<<<kc, 256, 0, stream>>>(pv, py, n, e_est);
-            count_launch();
+            TONER_LAUNCH(gemv_kernel, dim3((n + 7) / 8, kc), 256, stream, A32, pv, py, n);
+            TONER_LAUNCH(power_shift_kernel, kc, 256, stream, pv, py, n, e_est, 1, 0);
           }
         }
-        verify_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(e_est, ritz_norm ? e_top : nullptr,
-                                                          (float)(1.15 * (1.0 - l_last) + 1e-3),
-                                                          status ? status + k0 : nullptr,
-                                                          resid_out ? resid_out + k0 : nullptr, kc);
-        count_launch();
+        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm ? e_top : nullptr, (float)(1.15 * (1.0 - l_last) + 1e-3), status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc);
         TONER_CUDA(cudaGetLastError());
       }
       const int sweeps = track_sweeps & 63;
@@ -1558,18 +1542,14 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         // highest inverse power just computed, where it stands out however small it is next to lambda_max(A).
         const float* top = (q > 1 ? root_hi : root_lo) + (long long)k0 * nn;
         if (track_sweeps & 256) {
-          power_start_kernel<<<dim3(8, kc), 256, 0, stream>>>(vt, n);
-          count_launch();
+          TONER_LAUNCH(power_start_kernel, dim3(8, kc), 256, stream, vt, n);
         }
         for (int sw = 0; sw < sweeps; ++sw) {
-          gemv_kernel<<<dim3((n + 7) / 8, kc), 256, 0, stream>>>(top, vt, py, n);
-          count_launch();
-          power_norm_kernel<<<kc, 256, 0, stream>>>(vt, py, n, theta, pres);
-          count_launch();
+          TONER_LAUNCH(gemv_kernel, dim3((n + 7) / 8, kc), 256, stream, top, vt, py, n);
+          TONER_LAUNCH(power_norm_kernel, kc, 256, stream, vt, py, n, theta, pres);
         }
         if (lmin_out) {
-          lmin_from_root_kernel<<<(kc + 127) / 128, 128, 0, stream>>>(theta, (float)p / (float)q, lmin_out + k0, kc);
-          count_launch();
+          TONER_LAUNCH(lmin_from_root_kernel, (kc + 127) / 128, 128, stream, theta, (float)p / (float)q, lmin_out + k0, kc);
         }
         TONER_CUDA(cudaGetLastError());
       }

@@ -40,10 +40,10 @@ constexpr long long kSettleCycles = 200000LL;    // after an abort: a CTA of a p
 enum GemmStatus : int { kOk = 0, kTimeoutProducer = 101, kTimeoutMma = 102, kTimeoutEpilogue = 103, kTimeoutSelftest = 199 };
 
 struct GemmParams {
-  // operands: arrays of 3-D tensor maps (inner, outer, z) in global memory
-  const CUtensorMap* a_maps;
+  // operands: one 3-D tensor map (inner, outer, z) each, or an array in global memory with one map per batch
+  CUtensorMap a_map, b_map;
+  const CUtensorMap* a_maps;   // non-null: separately allocated matrices
   const CUtensorMap* b_maps;
-  int a_map_stride, b_map_stride;  // map index   = batch * map_stride
   int a_z_stride, b_z_stride;      // z coordinate = batch * z_stride + seg_z[seg]
   int a_mn, b_mn;                  // 1: stored MN-major (outer index is k), 0: K-major (outer index is m / n)
   int a_seg_z[kMaxSegs], b_seg_z[kMaxSegs];
@@ -551,6 +551,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   else __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  ptx::pdl_begin();   // everything above runs beside the previous kernel
 
   if (warp < 4) {
   ptx::reg_dec<48>();
@@ -564,10 +565,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       for (int t = unit; t < total_tiles && ok; t += units) {
         int b, tm, tn;
         tile_coord(p, BN, TM, t, tiles_per_batch, tiles_n, b, tm, tn);
-        const CUtensorMap* amap = p.a_maps + (long long)b * p.a_map_stride;
-        const CUtensorMap* bmap = p.b_maps + (long long)b * p.b_map_stride;
-        ptx::fence_tensormap_acquire(amap);
-        ptx::fence_tensormap_acquire(bmap);
+        const CUtensorMap* amap = &p.a_map;
+        const CUtensorMap* bmap = &p.b_map;
+        if (p.a_maps) {
+          amap = p.a_maps + b;
+          ptx::fence_tensormap_acquire(amap);
+        }
+        if (p.b_maps) {
+          bmap = p.b_maps + b;
+          ptx::fence_tensormap_acquire(bmap);
+        }
         // a pair splits the tile's rows (A) and its columns (B) between its two CTAs
         // (of a wide tile each CTA holds 128 columns of either 256-column half: n0 is its share of the first half)
         const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN + (int)cta_rank * (kWide ? BNI / 2 : S::kBRows);

@@ -91,6 +91,7 @@ Context* context() {
 
 static int encode_one(CUtensorMap* out, const void* base, int rows, int cols, long long ld, long long z_stride, int nz,
                       int box_rows) {
+  if (base == nullptr) return fail(kErrArg, "null operand pointer");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return fail(kErrArg, "operand base must be 16-byte aligned");
   if (ld % 8 != 0 || ld < cols) return fail(kErrArg, "operand leading dimension must be a multiple of 8 elements and >= cols");
   if (nz > 1 && z_stride % 8 != 0) return fail(kErrArg, "operand z stride must be a multiple of 8 elements");
@@ -122,17 +123,13 @@ static bool encode_box(CUtensorMap* out, const void* base, int rows, int cols, l
 }
 
 int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cudaStream_t stream, const CUtensorMap** out) {
-  const int count = op.list ? batch : 1;
+  const int count = batch;
   const int brows = op.mn_major ? 64 : box_rows;
   std::string key;
   key.reserve(64 + 8 * count);
   auto put = [&key](const void* p, size_t n) { key.append(reinterpret_cast<const char*>(p), n); };
   put(&op.rows, 4); put(&op.cols, 4); put(&op.ld, 8); put(&op.z_stride, 8); put(&op.nz, 4); put(&brows, 4);
-  if (op.list) {
-    for (int i = 0; i < batch; ++i) put(&op.list[i], sizeof(void*));
-  } else {
-    put(&op.base, sizeof(void*));
-  }
+  for (int i = 0; i < batch; ++i) put(&op.list[i], sizeof(void*));
   std::lock_guard<std::mutex> lock(g_mutex);
   auto* cache = static_cast<MapCache*>(ctx->map_cache);
   auto it = cache->find(key);
@@ -163,9 +160,8 @@ int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cud
   }
   const int slot = ctx->arena_used;
   for (int i = 0; i < count; ++i) {
-    const void* base = op.list ? op.list[i] : op.base;
-    if (base == nullptr) return fail(kErrArg, "null operand pointer");
-    int rc = encode_one(ctx->arena_host + slot + i, base, op.rows, op.cols, op.ld, op.z_stride, op.list ? 1 : op.nz, brows);
+    if (op.list[i] == nullptr) return fail(kErrArg, "null operand pointer");
+    int rc = encode_one(ctx->arena_host + slot + i, op.list[i], op.rows, op.cols, op.ld, op.z_stride, 1, brows);
     if (rc) return rc;
   }
   MapEntry e;
@@ -225,12 +221,15 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
 
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  int rc = get_maps(ctx, d.a, d.batch, kBM, stream, &p.a_maps);
+  // a pair's CTA loads B in boxes of 128 rows; MN-major operands always come in 64 x 64 boxes
+  auto operand_map = [&](const toner_operand& op, int box_rows, CUtensorMap* map, const CUtensorMap** maps) {
+    if (op.list) return get_maps(ctx, op, d.batch, box_rows, stream, maps);
+    return encode_one(map, op.base, op.rows, op.cols, op.ld, op.z_stride, op.nz, op.mn_major ? 64 : box_rows);
+  };
+  int rc = operand_map(d.a, kBM, &p.a_map, &p.a_maps);
   if (rc) return rc;
-  rc = get_maps(ctx, d.b, d.batch, pair ? 128 : bn, stream, &p.b_maps);  // a pair's CTA loads B in boxes of 128 rows
+  rc = operand_map(d.b, pair ? 128 : bn, &p.b_map, &p.b_maps);
   if (rc) return rc;
-  p.a_map_stride = d.a.list ? 1 : 0;
-  p.b_map_stride = d.b.list ? 1 : 0;
   p.a_z_stride = d.a.list ? 0 : d.a.z_step;
   p.b_z_stride = d.b.list ? 0 : d.b.z_step;
   p.a_mn = d.a.mn_major ? 1 : 0;
@@ -281,34 +280,19 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   const bool chained = p.promote > 0;
   if (pair) {
     const int pairs = (int)(total < ctx->gemm_sms / 2 ? total : ctx->gemm_sms / 2);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = bn == 512 ? GemmSmem<512, true>::kTotal : GemmSmem<256, true>::kTotal;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (bn == 512) TONER_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<512, false, true>, p));
-    else if (chained) TONER_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<256, true, true>, p));
-    else TONER_CUDA(cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<256, false, true>, p));
-    count_launch();
+    if (bn == 512) TONER_CUDA(launch(gemm_tcgen05_kernel<512, false, true>, 2 * pairs, kGemmThreads, GemmSmem<512, true>::kTotal, stream, 2, p));
+    else if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<256, true, true>, 2 * pairs, kGemmThreads, GemmSmem<256, true>::kTotal, stream, 2, p));
+    else TONER_CUDA(launch(gemm_tcgen05_kernel<256, false, true>, 2 * pairs, kGemmThreads, GemmSmem<256, true>::kTotal, stream, 2, p));
     return 0;
   }
   const int grid = (int)(total < ctx->gemm_sms ? total : ctx->gemm_sms);
   if (bn == 256) {
-    if (chained) gemm_tcgen05_kernel<256, true><<<grid, kGemmThreads, GemmSmem<256>::kTotal, stream>>>(p);
-    else gemm_tcgen05_kernel<256, false><<<grid, kGemmThreads, GemmSmem<256>::kTotal, stream>>>(p);
+    if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<256, true>, grid, kGemmThreads, GemmSmem<256>::kTotal, stream, 0, p));
+    else TONER_CUDA(launch(gemm_tcgen05_kernel<256, false>, grid, kGemmThreads, GemmSmem<256>::kTotal, stream, 0, p));
   } else {
-    if (chained) gemm_tcgen05_kernel<128, true><<<grid, kGemmThreads, GemmSmem<128>::kTotal, stream>>>(p);
-    else gemm_tcgen05_kernel<128, false><<<grid, kGemmThreads, GemmSmem<128>::kTotal, stream>>>(p);
+    if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<128, true>, grid, kGemmThreads, GemmSmem<128>::kTotal, stream, 0, p));
+    else TONER_CUDA(launch(gemm_tcgen05_kernel<128, false>, grid, kGemmThreads, GemmSmem<128>::kTotal, stream, 0, p));
   }
-  count_launch();
-  TONER_CUDA(cudaGetLastError());
   return 0;
 }
 

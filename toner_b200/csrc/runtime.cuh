@@ -47,11 +47,35 @@ struct Context {
 // Number of kernels this library has launched (all devices, all streams).
 void count_launch(int n = 1);
 
+// Launch with programmatic stream serialisation: the kernel's blocks may be scheduled while the previous kernel of the
+// stream drains; each kernel orders itself with ptx::pdl_begin().  Launch latency and prologue (barriers, tensor memory,
+// descriptors) of a chain of short products then hide behind one another.  `cluster`: blocks per cluster (0: none).
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster > 0 ? cluster : 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  count_launch();
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#define TONER_LAUNCH(kernel, grid, threads, stream, ...) TONER_CUDA(launch(kernel, dim3(grid), threads, 0, stream, 0, __VA_ARGS__))
+
 // Context of the current device (created on first use).  Returns nullptr and sets the error on failure.
 Context* context();
 
-// Device pointer to `count` consecutive tensor maps describing `op` (one per batch when op.list is
-// given, else one).  box_rows is the outer box extent for K-major operands (tile rows); MN-major
+// Device pointer to `batch` consecutive tensor maps describing the separately allocated matrices of op.list (an operand
+// that is one stack needs no map in memory: its map travels with the launch).  box_rows is the outer box extent for K-major operands (tile rows); MN-major
 // operands always use 64 x 64 boxes.
 int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cudaStream_t stream, const CUtensorMap** out);
 

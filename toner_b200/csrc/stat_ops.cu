@@ -15,6 +15,7 @@ namespace toner {
 // elements are all loaded before the first is stored.
 __global__ void __launch_bounds__(256) unpack_ema_kernel(const float* __restrict__ packed, float* __restrict__ ema, int n,
                                                          int tiles, float beta, float gamma) {
+  ptx::pdl_begin();
   // tile (ti, tj), ti <= tj, from the running index: row ti holds tiles - ti of them
   // (rows 0 .. ti-1 hold ti * tiles - ti (ti - 1) / 2 tiles: solve for ti, then correct the rounding)
   const int idx = blockIdx.x;
@@ -66,6 +67,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const T* __restrict__ x, long long batch_stride, long long row_stride,
                                                           const int* __restrict__ positions, int count, int n, int rows_total,
                                                           __nv_bfloat16* __restrict__ dst) {
+  ptx::pdl_begin();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows_total) return;
   const int b = row / count, j = row - b * count;
@@ -90,6 +92,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const T* __restrict__ 
 __global__ void __launch_bounds__(256) maxabs_kernel(const float* __restrict__ x, const float* const* __restrict__ x_list,
                                                      int rows, int cols, long long ld, long long bs, float aff_a,
                                                      float aff_b, unsigned int* __restrict__ out) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float* X = x_list ? x_list[b] : x + (long long)b * bs;
   float m = 0.f;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ 
                                                       int batch, int rows, int cols, long long ld, long long bs,
                                                       float aff_a, float aff_b, const unsigned int* __restrict__ maxabs,
                                                       __half* __restrict__ planes, float* __restrict__ inv_scale) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float* X = x_list ? x_list[b] : x + (long long)b * bs;
   const float s = split_scale(maxabs[b]);
@@ -180,6 +184,7 @@ constexpr int kSumsqBlocks = 296;  // two per SM on a 148-SM part; fixed so that
 
 __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restrict__ x, int rows, int cols, long long ld,
                                                             long long bs, float* __restrict__ partial) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float* X = x + (long long)b * bs;
   const long long total = (long long)rows * cols;
@@ -229,6 +234,7 @@ __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restr
 }
 
 __global__ void sumsq_final_kernel(const float* __restrict__ partial, int blocks, int batch, float* __restrict__ out) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
   float t = 0.f;
@@ -240,10 +246,8 @@ size_t sumsq_scratch_bytes(int batch) { return (size_t)batch * kSumsqBlocks * si
 
 int sumsq_det(const float* x, int batch, int rows, int cols, long long ld, long long bs, float* scratch, float* out,
               cudaStream_t stream) {
-  sumsq_partial_kernel<<<dim3(kSumsqBlocks, batch), 256, 0, stream>>>(x, rows, cols, ld, bs, scratch);
-  count_launch();
-  sumsq_final_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(scratch, kSumsqBlocks, batch, out);
-  count_launch();
+  TONER_LAUNCH(sumsq_partial_kernel, dim3(kSumsqBlocks, batch), 256, stream, x, rows, cols, ld, bs, scratch);
+  TONER_LAUNCH(sumsq_final_kernel, (batch + 127) / 128, 128, stream, scratch, kSumsqBlocks, batch, out);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -297,14 +301,11 @@ int split16(const float* x, const float* const* x_list, int batch, int rows, int
     if (!scratch) return fail(kErrArg, "split16: maxabs or scratch is required");
     unsigned int* m = static_cast<unsigned int*>(scratch);
     TONER_CUDA(cudaMemsetAsync(m, 0, sizeof(unsigned int) * batch, stream));
-    maxabs_kernel<<<dim3(bx, batch), 256, 0, stream>>>(x, x_list, rows, cols, ld, bs, aff_a, aff_b, m);
-    count_launch();
+    TONER_LAUNCH(maxabs_kernel, dim3(bx, batch), 256, stream, x, x_list, rows, cols, ld, bs, aff_a, aff_b, m);
     TONER_CUDA(cudaGetLastError());
     maxabs = m;
   }
-  split16_kernel<<<dim3(bx, batch), 256, 0, stream>>>(x, x_list, batch, rows, cols, ld, bs, aff_a, aff_b, maxabs,
-                                                     static_cast<__half*>(planes), inv_scale);
-  count_launch();
+  TONER_LAUNCH(split16_kernel, dim3(bx, batch), 256, stream, x, x_list, batch, rows, cols, ld, bs, aff_a, aff_b, maxabs, static_cast<__half*>(planes), inv_scale);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -373,12 +374,9 @@ int toner_gather_rows(const void* x, int32_t x_is_fp32, int32_t batch, int32_t s
   const int blocks = (int)((rows + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (x_is_fp32)
-    gather_rows_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), batch_stride, row_stride, positions, count, n,
-                                                     (int)rows, static_cast<__nv_bfloat16*>(dst));
+    TONER_LAUNCH(gather_rows_kernel<float>, blocks, 256, s, static_cast<const float*>(x), batch_stride, row_stride, positions, count, n, (int)rows, static_cast<__nv_bfloat16*>(dst));
   else
-    gather_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), batch_stride, row_stride,
-                                                             positions, count, n, (int)rows, static_cast<__nv_bfloat16*>(dst));
-  count_launch();
+    TONER_LAUNCH(gather_rows_kernel<__nv_bfloat16>, blocks, 256, s, static_cast<const __nv_bfloat16*>(x), batch_stride, row_stride, positions, count, n, (int)rows, static_cast<__nv_bfloat16*>(dst));
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -406,8 +404,7 @@ int toner_unpack_ema(const float* packed, float* ema, int32_t k, int32_t n, floa
   if (!packed || !ema || k <= 0 || n <= 0) return fail(kErrArg, "unpack_ema: bad arguments");
   const int t = (n + 31) / 32;
   if (k > 65535) return fail(kErrArg, "unpack_ema: k too large");
-  unpack_ema_kernel<<<dim3(t * (t + 1) / 2, 1, k), 256, 0, static_cast<cudaStream_t>(stream)>>>(packed, ema, n, t, beta, gamma);
-  count_launch();
+  TONER_LAUNCH(unpack_ema_kernel, dim3(t * (t + 1) / 2, 1, k), 256, static_cast<cudaStream_t>(stream), packed, ema, n, t, beta, gamma);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }

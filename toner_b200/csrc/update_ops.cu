@@ -18,6 +18,7 @@ static int ew_grid(long long elems4, int num_sms) {
 __global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__ u, const float* __restrict__ sumsq,
                                                        float eps, long long per, float* __restrict__ x,
                                                        __nv_bfloat16* __restrict__ xb) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float f = 1.f / (sqrtf(sumsq[b]) + eps);
   const float4* U = reinterpret_cast<const float4*>(u + (long long)b * per);
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__
 __global__ void __launch_bounds__(256) muont_momentum_kernel(const float* const* __restrict__ grads, float* __restrict__ m,
                                                              float* __restrict__ u, long long per, float mu, int nesterov,
                                                              unsigned int* __restrict__ maxabs) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float4* G = reinterpret_cast<const float4*>(grads[b]);
   float4* M = reinterpret_cast<float4*>(m + (long long)b * per);
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(256) muont_momentum_kernel(const float* const*
 // c1[b] = lr wd n / ||R||_F^2 ,  c2[b] = lr scale sqrt(n) / ||R||_F   with ||R||_F^2 = fro2[first + b*step]
 __global__ void muont_coeff_kernel(const float* __restrict__ fro2, int first, int step, int count, int n, float lr, float wd,
                                    float scale, float* __restrict__ c1, float* __restrict__ c2) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= count) return;
   const float f2 = fro2[first + b * step];
@@ -81,6 +84,7 @@ __global__ void muont_coeff_kernel(const float* __restrict__ fro2, int first, in
 }
 
 __global__ void mul_vec_kernel2(float* a, const float* b, int k) {
+  ptx::pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < k) a[i] *= b[i];
 }
@@ -89,6 +93,7 @@ __global__ void mul_vec_kernel2(float* a, const float* b, int k) {
 // m <- b1 m + (1-b1) g
 __global__ void __launch_bounds__(256) adamt_m_kernel(const float* const* __restrict__ grads, float* __restrict__ m,
                                                       long long per, float b1) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float4* G = reinterpret_cast<const float4*>(grads[b]);
   float4* M = reinterpret_cast<float4*>(m + (long long)b * per);
@@ -106,6 +111,7 @@ __global__ void __launch_bounds__(256) adamt_m_kernel(const float* const* __rest
 __global__ void __launch_bounds__(256) adamt_ratio_kernel(const float* __restrict__ t, float* __restrict__ v,
                                                           float* __restrict__ num, long long per, float b2, float bc2,
                                                           float eps, unsigned int* __restrict__ maxabs) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float4* T = reinterpret_cast<const float4*>(t + (long long)b * per);
   float4* V = reinterpret_cast<float4*>(v + (long long)b * per);
@@ -132,6 +138,7 @@ __global__ void __launch_bounds__(256) adamt_ratio_kernel(const float* __restric
 __global__ void adamt_coeff_kernel(const float* __restrict__ fro2, int first, int step, int count, int n, float lr, float wd,
                                    const float* __restrict__ ss_before, const float* __restrict__ ss_after,
                                    float* __restrict__ c1, float* __restrict__ c2) {
+  ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= count) return;
   c1[b] = lr * wd * (float)n / fmaxf(fro2[first + b * step], 1e-60f);
@@ -142,6 +149,7 @@ __global__ void adamt_coeff_kernel(const float* __restrict__ fro2, int first, in
 // W_b += delta_b for separately allocated weights
 __global__ void __launch_bounds__(256) apply_delta_kernel(float* const* __restrict__ weights, const float* __restrict__ delta,
                                                           long long per) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   float4* W = reinterpret_cast<float4*>(weights[b]);
   const float4* D = reinterpret_cast<const float4*>(delta + (long long)b * per);
@@ -157,6 +165,7 @@ __global__ void __launch_bounds__(256) apply_delta_kernel(float* const* __restri
 // W_b <- ws * W_b + ds * delta_b (decoupled weight decay and a scaled change in one pass)
 __global__ void __launch_bounds__(256) apply_scaled_kernel(float* const* __restrict__ weights, const float* __restrict__ delta,
                                                            long long per, float ws, float ds) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   float4* W = reinterpret_cast<float4*>(weights[b]);
   const float4* D = reinterpret_cast<const float4*>(delta + (long long)b * per);
@@ -172,6 +181,7 @@ __global__ void __launch_bounds__(256) apply_scaled_kernel(float* const* __restr
 
 __global__ void __launch_bounds__(256) scale_stack_kernel(const float* __restrict__ x, const float* __restrict__ coeff,
                                                           float* __restrict__ out, long long per) {
+  ptx::pdl_begin();
   const int b = blockIdx.y;
   const float c = coeff[b];
   const float4* X = reinterpret_cast<const float4*>(x + (long long)b * per);
@@ -187,6 +197,7 @@ __global__ void __launch_bounds__(256) scale_stack_kernel(const float* __restric
 // out = a x + b y
 __global__ void __launch_bounds__(256) axpby_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                     float* __restrict__ out, long long n, float a, float b) {
+  ptx::pdl_begin();
   const long long n4 = n / 4;
   const float4* X = reinterpret_cast<const float4*>(x);
   const float4* Y = reinterpret_cast<const float4*>(y);
@@ -211,8 +222,7 @@ int toner_axpby(const float* x, const float* y, float* out, int64_t n, float a, 
   if (!x || !y || !out || n <= 0) return fail(kErrArg, "axpby: bad arguments");
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15u)
     return fail(kErrArg, "axpby: pointers must be 16-byte aligned");
-  axpby_kernel<<<ew_grid(n / 4 + 1, ctx->num_sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, out, n, a, b);
-  count_launch();
+  TONER_LAUNCH(axpby_kernel, ew_grid(n / 4 + 1, ctx->num_sms), 256, static_cast<cudaStream_t>(stream), x, y, out, n, a, b);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -221,8 +231,7 @@ int toner_scale_stack(const float* x, const float* coeff, float* out, int32_t co
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   if (!x || !coeff || !out || count <= 0 || per <= 0 || per % 4) return fail(kErrArg, "scale_stack: bad arguments");
-  scale_stack_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, coeff, out, per);
-  count_launch();
+  TONER_LAUNCH(scale_stack_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), x, coeff, out, per);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -261,8 +270,7 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
 
   int rc = sumsq_det(u, batch, m, n, n, mn, partial, ss, stream);
   if (rc) return rc;
-  ns_scale_kernel<<<dim3(ew_grid(mn / 4, ctx->num_sms), batch), 256, 0, stream>>>(u, ss, eps, mn, x_out, xb[0]);
-  count_launch();
+  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid(mn / 4, ctx->num_sms), batch), 256, stream, u, ss, eps, mn, x_out, xb[0]);
   TONER_CUDA(cudaGetLastError());
 
   const float ca = 3.4445f, cb = -4.7750f, cc = 2.0315f;  // src/toner/linalg.py:9
@@ -349,8 +357,7 @@ int toner_muont_momentum(const float* const* grad_ptrs, float* m, float* u, int3
   if (int rc = check_stack("muont_momentum", per)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (maxabs) TONER_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(uint32_t) * count, stream));
-  muont_momentum_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, stream>>>(grad_ptrs, m, u, per, mu, nesterov, maxabs);
-  count_launch();
+  TONER_LAUNCH(muont_momentum_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, stream, grad_ptrs, m, u, per, mu, nesterov, maxabs);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -359,8 +366,7 @@ int toner_muont_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
                        float scale, float* c1, float* c2, void* stream) {
   if (!context()) return kErrCuda;
   if (!fro2 || !c1 || !c2 || count <= 0) return fail(kErrArg, "muont_coeffs: bad arguments");
-  muont_coeff_kernel<<<(count + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(fro2, first, step, count, n, lr, wd, scale, c1, c2);
-  count_launch();
+  TONER_LAUNCH(muont_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, scale, c1, c2);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -368,8 +374,7 @@ int toner_muont_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
 int toner_scale_vec(float* a, const float* b, int32_t count, void* stream) {
   if (!context()) return kErrCuda;
   if (!a || !b || count <= 0) return fail(kErrArg, "scale_vec: bad arguments");
-  mul_vec_kernel2<<<(count + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(a, b, count);
-  count_launch();
+  TONER_LAUNCH(mul_vec_kernel2, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), a, b, count);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -379,8 +384,7 @@ int toner_adamt_first_moment(const float* const* grad_ptrs, float* m, int32_t co
   if (!ctx) return kErrCuda;
   if (!grad_ptrs || !m || count <= 0) return fail(kErrArg, "adamt_first_moment: bad arguments");
   if (int rc = check_stack("adamt_first_moment", per)) return rc;
-  adamt_m_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, static_cast<cudaStream_t>(stream)>>>(grad_ptrs, m, per, beta1);
-  count_launch();
+  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), grad_ptrs, m, per, beta1);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -393,8 +397,7 @@ int toner_adamt_ratio(const float* t, float* v, float* num, int32_t count, int64
   if (int rc = check_stack("adamt_ratio", per)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (maxabs) TONER_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(uint32_t) * count, stream));
-  adamt_ratio_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, stream>>>(t, v, num, per, beta2, bc2, eps, maxabs);
-  count_launch();
+  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, stream, t, v, num, per, beta2, bc2, eps, maxabs);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -403,8 +406,7 @@ int toner_adamt_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
                        const float* ss_before, const float* ss_after, float* c1, float* c2, void* stream) {
   if (!context()) return kErrCuda;
   if (!fro2 || !ss_before || !ss_after || !c1 || !c2 || count <= 0) return fail(kErrArg, "adamt_coeffs: bad arguments");
-  adamt_coeff_kernel<<<(count + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(fro2, first, step, count, n, lr, wd, ss_before, ss_after, c1, c2);
-  count_launch();
+  TONER_LAUNCH(adamt_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, ss_before, ss_after, c1, c2);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -414,8 +416,7 @@ int toner_apply_delta(float* const* weight_ptrs, const float* delta, int32_t cou
   if (!ctx) return kErrCuda;
   if (!weight_ptrs || !delta || count <= 0) return fail(kErrArg, "apply_delta: bad arguments");
   if (int rc = check_stack("apply_delta", per)) return rc;
-  apply_delta_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, static_cast<cudaStream_t>(stream)>>>(weight_ptrs, delta, per);
-  count_launch();
+  TONER_LAUNCH(apply_delta_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), weight_ptrs, delta, per);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -426,9 +427,7 @@ int toner_apply_scaled(float* const* weight_ptrs, const float* delta, int32_t co
   if (!ctx) return kErrCuda;
   if (!weight_ptrs || !delta || count <= 0) return fail(kErrArg, "apply_scaled: bad arguments");
   if (int rc = check_stack("apply_scaled", per)) return rc;
-  apply_scaled_kernel<<<dim3(ew_grid(per / 4, ctx->num_sms), count), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      weight_ptrs, delta, per, weight_scale, delta_scale);
-  count_launch();
+  TONER_LAUNCH(apply_scaled_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream),  weight_ptrs, delta, per, weight_scale, delta_scale);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
