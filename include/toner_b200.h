@@ -97,8 +97,9 @@ typedef struct toner_gemm_desc {
   uint32_t* maxabs;         /*   max |d| as FP32 bits, */
   uint32_t* maxaff;         /*   max |aff_a*[r==c] + aff_b*d| as FP32 bits */
   float aff_a, aff_b;
-  int32_t tile_n;           /* 0 = choose; else 128 or 256 (128-row tiles), 512 = 256 x 256 tiles on CTA pairs,
-                               1024 = 256 x 512 tiles on CTA pairs (no chained accumulation) */
+  int32_t tile_n;           /* 0 = choose; else 64, 128 or 256 (128-row tiles), -128 = 256 x 128 tiles on CTA pairs,
+                               512 = 256 x 256 tiles on CTA pairs, 1024 = 256 x 512 tiles on CTA pairs (no chained
+                               accumulation) */
   int32_t promote;          /* > 0: k-blocks (64 deep) per tensor-core accumulation chain; chains are summed in
                                FP32 registers with round-to-nearest (the tensor core truncates).  0: one chain */
   int32_t raster;           /* tile columns per rasterisation group for full schedules (0: default 8) */
@@ -118,6 +119,9 @@ typedef struct toner_gemm_desc {
   int32_t upper_d;          /* with tri + mirror: write the FP32 result d on and above the diagonal only (the 16-bit copy
                                and the operand planes are still mirrored) -- for a result whose FP32 form is read back
                                as the upper-triangle `c` of another symmetric product and nowhere else */
+  void* split_ws;           /* optional scratch: a product with few tiles and a long accumulation may then divide each tile's
+                               accumulation among several CTAs and add the parts (in a fixed order) there */
+  int64_t split_ws_bytes;
 } toner_gemm_desc;
 
 int toner_gemm(const toner_gemm_desc* desc, void* stream);
@@ -142,6 +146,14 @@ int toner_gemm_phase_cycles(int enable, void* stream, unsigned long long* out8);
 int toner_syrk_upper(const void* const* x_list, const void* x_base, int64_t x_batch_stride, int32_t k,
                      int32_t rows, int32_t n, int64_t ld, float* out, int32_t mode, float beta, float gamma,
                      void* stream);
+
+/* The same with scratch: few statistics over many rows (one 2048-wide statistic is 36 tiles of 256 x 256) then have each
+ * tile's rows divided among several CTAs.  toner_syrk_workspace_bytes gives the scratch that helps (0: none does);
+ * `workspace` may be NULL.  The parts are added in a fixed order: the same call gives the same bits. */
+size_t toner_syrk_workspace_bytes(int32_t k, int32_t rows, int32_t n);
+int toner_syrk_upper_ws(const void* const* x_list, const void* x_base, int64_t x_batch_stride, int32_t k, int32_t rows,
+                        int32_t n, int64_t ld, float* out, int32_t mode, float beta, float gamma, void* workspace,
+                        size_t workspace_bytes, void* stream);
 
 /* Sampled-row capture: dst[(b*count + j), :] = BF16(x[b, positions[j], :]) for a (batch, seq, n) activation tensor
  * (BF16, or FP32 when x_is_fp32: rounded to BF16 as autocast would), `positions` a DEVICE array of `count` token

@@ -26,7 +26,7 @@ def _close(got, want, k):
 
 
 @pytest.mark.parametrize("n", [8, 24, 40, 128, 136, 264, 520, 776])
-@pytest.mark.parametrize("tile_n", [0, 128, 512])
+@pytest.mark.parametrize("tile_n", [0, 64, 128, -128, 512])
 def test_symmetric_with_c(ops, n, tile_n):
     batch, k = 2, 72
     a = _rnd((batch, n, k), n, torch.bfloat16)
@@ -49,7 +49,7 @@ def test_symmetric_with_c(ops, n, tile_n):
 
 
 @pytest.mark.parametrize("m,n", [(8, 8), (40, 264), (136, 8), (200, 520), (392, 264)])
-@pytest.mark.parametrize("tile_n", [0, 128, 256, 512, 1024])
+@pytest.mark.parametrize("tile_n", [0, 64, 128, -128, 256, 512, 1024])
 def test_full_result_with_c_in_place(ops, m, n, tile_n):
     batch, k = 2, 136
     a, b = _rnd((batch, m, k), m, torch.bfloat16), _rnd((batch, n, k), n, torch.bfloat16)
@@ -75,3 +75,30 @@ def test_packed_triangle_accumulates(ops, n):
     iu = torch.triu_indices(n, n)
     want = 2.0 * (x.double().mT @ x.double())[:, iu[0], iu[1]]
     _close(out, want, k)
+
+
+@pytest.mark.parametrize("k,rows,n", [(1, 4097, 8), (1, 20001, 136), (2, 9000, 264), (1, 2500, 768), (3, 33000, 520)])
+@pytest.mark.parametrize("mode", ["packed", "ema"])
+def test_rows_divided_among_ctas(ops, k, rows, n, mode):
+    """Few tiles, many rows: each tile's rows are divided among several CTAs (one chain, and chains of 4096 rows)."""
+    from toner_b200 import _lib
+    assert _lib.load().toner_syrk_workspace_bytes(k, rows, n) > 0
+    x = _rnd((k, rows, n), rows + n, torch.bfloat16)
+    want = x.double().mT @ x.double()
+    got = []
+    for _ in range(2):
+        if mode == "ema":
+            out = torch.ones(k, n, n, device="cuda")
+            ops.syrk_upper(x, out, ops.EMA_FULL, 0.5, 1.0 / rows)
+            ref = 0.5 + want / rows
+        else:
+            out = torch.full((k, n * (n + 1) // 2), float("nan"), device="cuda")
+            ops.syrk_upper(x, out, ops.PACKED)
+            iu = torch.triu_indices(n, n)
+            ref = want[:, iu[0], iu[1]]
+        got.append(out)
+    ops.assert_healthy()
+    assert torch.equal(got[0], got[1])           # whichever part comes last, the parts are added in one order
+    # the tensor core truncates: up to 1.2e-7 of the sum per 64 rows, over chains of at most 64 such blocks
+    err = (got[0].double() - ref).abs().max().item() / ref.abs().max().item()
+    assert err < 1.5e-5, err

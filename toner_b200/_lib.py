@@ -55,6 +55,7 @@ class GemmDesc(C.Structure):
         ("split0_scale", C.c_float), ("split1_scale", C.c_float), ("split1_aff_a", C.c_float), ("split1_aff_b", C.c_float),
         ("maxres", C.c_void_p),
         ("upper_d", C.c_int32),
+        ("split_ws", C.c_void_p), ("split_ws_bytes", C.c_int64),
     ]
 
 
@@ -72,6 +73,8 @@ SIGNATURES = {
     "toner_selftest_bounded_wait": (C.c_int, [C.c_longlong, _vp]),
     "toner_gemm_phase_cycles": (C.c_int, [C.c_int, _vp, C.POINTER(C.c_uint64)]),
     "toner_syrk_upper": (C.c_int, [C.POINTER(_vp), _vp, _i64, _i32, _i32, _i32, _i64, _vp, _i32, _f32, _f32, _vp]),
+    "toner_syrk_workspace_bytes": (C.c_size_t, [_i32, _i32, _i32]),
+    "toner_syrk_upper_ws": (C.c_int, [C.POINTER(_vp), _vp, _i64, _i32, _i32, _i32, _i64, _vp, _i32, _f32, _f32, _vp, _sz, _vp]),
     "toner_unpack_ema": (C.c_int, [_vp, _vp, _i32, _i32, _f32, _f32, _vp]),
     "toner_inv_roots_workspace_bytes": (C.c_size_t, [_i32, _i32]),
     "toner_inv_roots_iterations": (C.c_int, [_i32, _f32, _i32]),

@@ -53,6 +53,12 @@ struct GemmParams {
   int tri;  // 1: M == N, only tiles meeting the upper triangle are computed
   int promote;  // > 0: k-blocks per tensor-core accumulation chain; chains are summed in FP32 registers
   int promote_all;  // 0: only the first segment is chained (split products); 1: every segment
+  // splits > 1: the accumulation of every tile is divided among that many units.  Each epilogue warp leaves its part of the
+  // partial sums in split_part and counts itself in at split_count (zeroed before the launch); the last of a tile's warps
+  // adds the parts in the order of the splits -- whoever comes last, so the result is reproducible -- and writes the result.
+  int splits;
+  float* split_part;
+  unsigned int* split_count;
   int raster;   // tile columns per rasterisation group (full schedules): keeps a group's B panels in L2
   // epilogue: d = alpha * acc + beta * C ; alpha, beta optionally scaled per batch from device arrays
   float alpha, beta;
@@ -124,7 +130,7 @@ struct GemmSmem {
   static constexpr int kStageBytes = kABytes + kBBytes;
   // Four stages keep the main loop fed as well as six did (BF16 4096^3 x 4 on pair tiles: 436 us with either; three stages
   // of the 48 KB tiles); the rest of shared memory is the epilogue's, which needs several blocks per warp in flight.
-  static constexpr int kStages = kStageBytes > 32 * 1024 ? 3 : 4;
+  static constexpr int kStages = kStageBytes > 32 * 1024 ? 3 : (kStageBytes < 32 * 1024 ? 5 : 4);
   static constexpr int kTileBytes = kStages * kStageBytes;
   static constexpr int kEpiBufs = kStageBytes > 32 * 1024 ? 2 : 3;          // 4 KB blocks per epilogue warp
   static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
@@ -447,7 +453,8 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 template <int BN, bool kChained, bool kPair = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair>;
-  static_assert(BN == 128 || BN == 256 || (BN == 512 && kPair && !kChained), "tile widths: 128, 256, or 512 on a pair");
+  static_assert((BN == 64 && !kPair) || BN == 128 || BN == 256 || (BN == 512 && kPair && !kChained),
+                "tile widths: 64 (single CTAs), 128, 256, or 512 (pairs)");
   constexpr bool kWide = S::kWide;
   constexpr int BNI = kWide ? 256 : BN;                // columns of one MMA instruction
   constexpr int NJ = BN / BNI;                         // MMAs per k-step (column halves of a wide tile)
@@ -498,11 +505,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   // two long chains give them that time; the short chains of the first segment follow.
   const bool rest_first = p.promote > 0 && !p.promote_all && p.segs > 1;
   auto chunk_range = [&](int ch, int& kb_begin, int& kb_end) {  // k-block indices in processing order
-    if (p.promote <= 0) {
-      kb_begin = 0;
-      kb_end = num_kb;
-      return;
-    }
     if (rest_first) {
       const int rest = p.segs - 1;
       if (ch < rest) {
@@ -522,6 +524,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     const bool chained = (seg == 0) || p.promote_all;
     kb_begin = seg * kb_per_seg + (chained ? c * p.promote : 0);
     kb_end = chained ? min(kb_begin + p.promote, (seg + 1) * kb_per_seg) : (seg + 1) * kb_per_seg;
+  };
+  // Work unit u: split u % splits of tile u / splits, i.e. accumulation chains [ch_lo, ch_hi) -- where there is one chain, a
+  // part of it -- and k-blocks [kb_lo, kb_hi) in processing order.
+  const int total_units = total_tiles * p.splits;
+  struct Unit {
+    int tile, split, ch_lo, ch_hi, kb_lo, kb_hi;
+  };
+  auto unit_of = [&](int u) {
+    Unit w;
+    w.tile = u / p.splits;
+    w.split = u - w.tile * p.splits;
+    if (p.promote > 0) {
+      w.ch_lo = chunks_per_tile * w.split / p.splits;
+      w.ch_hi = chunks_per_tile * (w.split + 1) / p.splits;
+      int unused;
+      chunk_range(w.ch_lo, w.kb_lo, unused);
+      chunk_range(w.ch_hi - 1, unused, w.kb_hi);
+    } else {
+      w.ch_lo = 0;
+      w.ch_hi = 1;
+      w.kb_lo = (int)((long long)num_kb * w.split / p.splits);
+      w.kb_hi = (int)((long long)num_kb * (w.split + 1) / p.splits);
+    }
+    return w;
   };
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::kStages; ++s) {
@@ -562,9 +588,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       uint32_t phase = 0;
       bool ok = true;
       long long prof_wait = 0;
-      for (int t = unit; t < total_tiles && ok; t += units) {
+      for (int u = unit; u < total_units && ok; u += units) {
+        const Unit w = unit_of(u);
         int b, tm, tn;
-        tile_coord(p, BN, TM, t, tiles_per_batch, tiles_n, b, tm, tn);
+        tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
         const CUtensorMap* amap = &p.a_map;
         const CUtensorMap* bmap = &p.b_map;
         if (p.a_maps) {
@@ -578,11 +605,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         // a pair splits the tile's rows (A) and its columns (B) between its two CTAs
         // (of a wide tile each CTA holds 128 columns of either 256-column half: n0 is its share of the first half)
         const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN + (int)cta_rank * (kWide ? BNI / 2 : S::kBRows);
-        for (int si = 0; si < p.segs && ok; ++si) {
+        for (int kb = w.kb_lo; kb < w.kb_hi && ok;) {
+          const int si = kb / kb_per_seg, seg_end = min(w.kb_hi, (si + 1) * kb_per_seg);
           const int seg = rest_first ? (si + 1 == p.segs ? 0 : si + 1) : si;
           const int za = b * p.a_z_stride + p.a_seg_z[seg];
           const int zb = b * p.b_z_stride + p.b_seg_z[seg];
-          for (int k0 = 0; k0 < p.K; k0 += kBK) {
+          for (; kb < seg_end; ++kb) {
+            const int k0 = (kb - si * kb_per_seg) * kBK;
             const long long w0 = p.prof ? clock64() : 0;
             const bool got = ptx::mbar_wait(empty_bar(stage), phase ^ 1u, kWaitCycles);
             if (p.prof) prof_wait += clock64() - w0;
@@ -678,10 +707,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       bool ok = true;
       long long prof_acc = 0, prof_ops = 0;
       const long long prof_t0 = p.prof ? clock64() : 0;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        for (int ch = 0; ch < chunks_per_tile && ok; ++ch, ++gchunk) {
-          int kb_begin, kb_end;
-          chunk_range(ch, kb_begin, kb_end);
+      for (int u = unit; u < total_units && ok; u += units) {
+        const Unit w = unit_of(u);
+        for (int ch = w.ch_lo; ch < w.ch_hi && ok; ++ch, ++gchunk) {
+          int kb_begin = w.kb_lo, kb_end = w.kb_hi;
+          if (p.promote > 0) chunk_range(ch, kb_begin, kb_end);
           // The wide tile has one accumulator of two halves, each with its own "drained" barrier (tempty 0 / 1): the
           // MMAs of the first k-block's first half start as soon as that half has been read out.
           const int buf = kWide ? 0 : (int)(gchunk & 1u);
@@ -775,9 +805,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     uint32_t gchunk = 0;
     bool alive = true;
     long long prof_wait = 0, prof_out = 0, prof_sum = 0;
-    for (int t = unit; t < total_tiles && alive; t += units) {
+    for (int u = unit; u < total_units && alive; u += units) {
+      const Unit w = unit_of(u);
       int b, tm, tn;
-      tile_coord(p, BN, TM, t, tiles_per_batch, tiles_n, b, tm, tn);
+      tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
       const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN;  // this CTA's 128 rows of the tile
       const int row_first = m0 + lane_group * 32;
       const int col_first = n0 + half * (BN / 2);
@@ -836,12 +867,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           ptx::tma_load_3d(c_buf, &p.c_map, c_bar(ew), col_first + cc * 32, row_first, b);
         }
       };
-      fetch_c(cc_first);
+      if (p.splits == 1) fetch_c(cc_first);
 
       if (chained) {
 #pragma unroll
         for (int j = 0; j < NCH * 32; ++j) racc[j] = 0.f;
-        for (int ch = 0; ch < chunks_per_tile; ++ch, ++gchunk) {
+        for (int ch = w.ch_lo; ch < w.ch_hi; ++ch, ++gchunk) {
           const int buf = gchunk & 1u;
           if (!wait_chain(buf)) {
             alive = false;
@@ -876,10 +907,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       const long long o0 = p.prof ? clock64() : 0;
       EpilogueSums sums;
       const uint32_t taddr = tmem_of(kWide ? 0 : (int)(gchunk & 1u));
-#pragma unroll 1
-      for (int cc = cc_first; cc < cc_end; ++cc) {
-        const int c0 = col_first + cc * 32;
-        float v[32];
+      // this unit's sums of block cc, one row per lane
+      auto take_block = [&](int cc, float (&v)[32]) {
         if constexpr (chained) {
           // the running sums live in registers: static indices only
           auto take_sums = [&](auto first) {
@@ -887,7 +916,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
             for (int j = 0; j < 32; ++j) v[j] = racc[decltype(first)::value + j];
           };
           if (cc == 0) take_sums(std::integral_constant<int, 0>());
-          if (cc == 1) take_sums(std::integral_constant<int, chained ? 32 : 0>());
+          if (cc == 1) take_sums(std::integral_constant<int, (chained && NCH > 1) ? 32 : 0>());
           if (cc == 2) take_sums(std::integral_constant<int, (chained && NCH > 2) ? 64 : 0>());
           if (cc == 3) take_sums(std::integral_constant<int, (chained && NCH > 2) ? 96 : 0>());
         } else {
@@ -900,6 +929,71 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
         }
+      };
+      // partial sums of (tile, split, warp, block): 32 floats of each lane, 16 bytes of all lanes side by side
+      auto part_at = [&](int split, int cc) {
+        const long long slot = ((long long)w.tile * p.splits + split) * (kPair ? 16 : 8) + (int)cta_rank * 8 + ew;
+        return reinterpret_cast<float4*>(p.split_part) + (slot * NCH + cc) * 256 + lane;
+      };
+      auto add_parts = [&](int cc, float* v) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        for (int split = 0; split < p.splits; ++split) {
+          const float4* src = part_at(split, cc);
+          constexpr int kAhead = chained ? 4 : 8;   // loads in flight (a chained kernel has its sums in registers as well)
+#pragma unroll
+          for (int j0 = 0; j0 < 8; j0 += kAhead) {
+            float4 r[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) r[j] = __ldcg(src + 32 * (j0 + j));
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+              float* t = v + 4 * (j0 + j);
+              t[0] += r[j].x; t[1] += r[j].y; t[2] += r[j].z; t[3] += r[j].w;
+            }
+          }
+        }
+      };
+      bool mine = true;   // this warp writes the result
+      if (p.splits > 1) {
+        auto leave_part = [&](int cc, const float* v) {
+          float4* dst = part_at(w.split, cc);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) __stcg(dst + 32 * j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+        };
+        if constexpr (chained) {
+#pragma unroll
+          for (int cc = 0; cc < NCH; ++cc)
+            if (cc >= cc_first && cc < cc_end) leave_part(cc, racc + 32 * cc);
+        } else {
+#pragma unroll 1
+          for (int cc = cc_first; cc < cc_end; ++cc) {
+            float v[32];
+            take_block(cc, v);
+            leave_part(cc, v);
+          }
+        }
+        __threadfence();
+        __syncwarp();
+        unsigned int before = 0;
+        if (lane == 0) before = atomicAdd(p.split_count + (long long)w.tile * (kPair ? 16 : 8) + (int)cta_rank * 8 + ew, 1u);
+        mine = __shfl_sync(0xffffffffu, before, 0) == (unsigned)(p.splits - 1);
+        __threadfence();
+        if (mine) {
+          fetch_c(cc_first);
+          if constexpr (chained) {   // the running sums have been handed over: their registers take the totals
+#pragma unroll
+            for (int cc = 0; cc < NCH; ++cc)
+              if (cc >= cc_first && cc < cc_end) add_parts(cc, racc + 32 * cc);
+          }
+        }
+      }
+#pragma unroll 1
+      for (int cc = cc_first; cc < cc_end && mine; ++cc) {
+        const int c0 = col_first + cc * 32;
+        float v[32];
+        if (chained || p.splits == 1) take_block(cc, v);
+        else add_parts(cc, v);
         if (boxed(c0)) {
           const uint32_t held = c_buf;
           if (held) {

@@ -78,13 +78,25 @@ Context* context() {
     return nullptr;
   }
   c.map_cache = new MapCache();
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<256>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<256>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<128>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<128>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<256, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<256, true>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<256, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<256, true>::kTotal);
-  cudaFuncSetAttribute(gemm_tcgen05_kernel<512, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<512, true>::kTotal);
+  bool ok = true;
+  auto allow = [&ok](auto kernel, int bytes) {
+    ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+  };
+  allow(gemm_tcgen05_kernel<64, false>, GemmSmem<64>::kTotal);
+  allow(gemm_tcgen05_kernel<64, true>, GemmSmem<64>::kTotal);
+  allow(gemm_tcgen05_kernel<128, false>, GemmSmem<128>::kTotal);
+  allow(gemm_tcgen05_kernel<128, true>, GemmSmem<128>::kTotal);
+  allow(gemm_tcgen05_kernel<256, false>, GemmSmem<256>::kTotal);
+  allow(gemm_tcgen05_kernel<256, true>, GemmSmem<256>::kTotal);
+  allow(gemm_tcgen05_kernel<128, false, true>, GemmSmem<128, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, true, true>, GemmSmem<128, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, false, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, true, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<512, false, true>, GemmSmem<512, true>::kTotal);
+  if (!ok) {
+    set_error("the GEMM kernels' shared memory was refused");
+    return nullptr;
+  }
   c.device = dev;
   return &c;
 }
@@ -177,6 +189,94 @@ int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cud
   return 0;
 }
 
+static long long gemm_tiles(const toner_gemm_desc& d, int bn, bool pair) {
+  return (long long)gemm_tiles_per_batch(d.m, d.n, bn, d.tri, pair ? 2 * kBM : kBM) * d.batch;
+}
+static size_t split_part_bytes(const toner_gemm_desc& d, int bn, bool pair, int splits) {
+  return (size_t)gemm_tiles(d, bn, pair) * splits * (pair ? 2 * kBM : kBM) * bn * sizeof(float);
+}
+static size_t split_count_bytes(const toner_gemm_desc& d, int bn, bool pair) {
+  return (size_t)gemm_tiles(d, bn, pair) * (pair ? 16 : 8) * sizeof(unsigned int);
+}
+
+struct TileChoice {
+  int bn;
+  bool pair;
+  int splits;
+  size_t ws_bytes;   // scratch the splits need
+};
+
+// Which tile, and among how many units a tile's accumulation is divided (only where the caller gave scratch for it).  An
+// estimate of the launch in SM cycles decides, from what was measured on the kernel:
+//   * the main loop is bound by shared memory (128 B per clock: operands written by TMA and read by the MMAs), 512 cycles
+//     per 64-deep k-block of 256 x 256 on a pair and of 128 x 128 on one CTA, 384 of 256 x 128 on a pair and of 128 x 64,
+//     768 of 128 x 256;
+//   * a 32 x 32 block of the epilogue takes a warp 900 cycles plus 450 per box moved, and its boxes take shared memory away
+//     from the main loop of the next tile;
+//   * tiles of one wave run side by side, and the epilogue of one tile beside the main loop of the next.
+// Small problems so get many small tiles (one 768 x 768 product: 128 x 64), a batch that just misses a wave of large tiles
+// gets 256 x 128, everything large gets 256 x 256.
+static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
+  struct Config {
+    int bn;
+    bool pair;
+    double per_kb;
+  };
+  static const Config configs[] = {{256, true, 512}, {128, true, 384}, {256, false, 768}, {128, false, 512}, {64, false, 384}};
+  const bool mirror = d.tri && d.mirror;
+  const double boxes = (d.c ? 1.2 : 0.0) + (d.d ? (mirror && !d.upper_d ? 2.0 : 1.0) : 0.0) + (d.d16 ? (mirror ? 1.6 : 1.0) : 0.0) +
+                       ((d.split0 ? 1.3 : 0.0) + (d.split1 ? 1.3 : 0.0)) * (mirror ? 2.0 : 1.0);
+  const double block = 900.0 + 450.0 * boxes, block_smem = 64.0 * boxes;
+  const double kb = (double)((d.k + kBK - 1) / kBK) * d.segs;
+  const int chains = d.promote > 0 ? ((d.k + kBK - 1) / kBK + d.promote - 1) / d.promote : (int)(kb / 4);
+  TileChoice best = {256, true, 1, 0};
+  double best_cost = 0.0;
+  for (const Config& c : configs) {
+    const long long tiles = gemm_tiles(d, c.bn, c.pair);
+    const int workers = c.pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
+    const int blocks = c.bn / 64;   // per epilogue warp
+    const double main = kb * c.per_kb, epi = blocks * block;
+    const double waves = (double)((tiles + workers - 1) / workers);
+    const double busy = main + blocks * 8 * block_smem;
+    double cost = main + epi + (waves - 1) * (busy > epi ? busy : epi);
+    int splits = 1;
+    if (d.split_ws && d.segs == 1) {
+      for (int s = 2; s <= 32 && s <= chains && tiles * s <= workers; ++s) {
+        const size_t need = split_part_bytes(d, c.bn, c.pair, s) + split_count_bytes(d, c.bn, c.pair);
+        if (need > (size_t)d.split_ws_bytes) break;
+        const double parts = 4000.0 + blocks * (800.0 + 400.0 * s);   // writing and adding the parts, the extra memset
+        if (main / s + parts + epi < cost) {
+          cost = main / s + parts + epi;
+          splits = s;
+        }
+      }
+    }
+    if (best_cost == 0.0 || cost < best_cost) {
+      best_cost = cost;
+      best = {c.bn, c.pair, splits, splits > 1 ? split_part_bytes(d, c.bn, c.pair, splits) + split_count_bytes(d, c.bn, c.pair) : 0};
+    }
+  }
+  if (best.bn == 256 && best.pair && best.splits == 1) {
+    // The wide tile: long accumulations only (its epilogue is not hidden behind the next tile), enough tiles for
+    // several waves, and a width for which the 512-column steps do not overshoot the triangle by much.
+    const long long twide = gemm_tiles(d, 512, true), tpair = gemm_tiles(d, 256, true);
+    const long long depth = (long long)d.k * d.segs;
+    if (ctx->gemm_wide_k > 0 && d.promote <= 0 && depth >= ctx->gemm_wide_k && twide >= 4LL * (ctx->gemm_sms / 2) &&
+        2 * twide * 100 <= tpair * 106)
+      best.bn = 512;
+  }
+  return best;
+}
+
+size_t gemm_split_bytes(const toner_gemm_desc& desc) {
+  Context* ctx = context();
+  if (!ctx) return 0;
+  toner_gemm_desc d = desc;
+  d.split_ws = ctx;                       // any address: the choice only asks whether there is one
+  d.split_ws_bytes = (int64_t)256 << 20;  // scratch a caller is asked for at most
+  return choose_tile(ctx, d).ws_bytes;
+}
+
 int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   Context* ctx = context();
   if (!ctx) return kErrCuda;
@@ -188,47 +288,38 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   if (d.packed && (d.split0 || d.split1)) return fail(kErrArg, "gemm: operand planes cannot be packed");
   if (d.fmt != 0 && d.fmt != 1) return fail(kErrArg, "gemm: fmt must be 0 (FP16) or 1 (BF16)");
 
-  // Tile choice: 256 x 256 tiles on CTA pairs when they fill the machine (fewest operand bytes per flop), else
-  // 128 x 256, else 128 x 128 (most tiles for small problems).  tile_n forces one: 128, 256, or 512 for the pair.
-  int bn = d.tile_n;
+  int bn = d.tile_n, splits = 1;
   bool pair = false;
   if (bn == 0) {
-    const long long tpair = (long long)gemm_tiles_per_batch(d.m, d.n, 256, d.tri, 256) * d.batch;
-    const long long t256 = (long long)gemm_tiles_per_batch(d.m, d.n, 256, d.tri) * d.batch;
-    if (tpair >= ctx->gemm_sms / 2) {
-      bn = 256;
-      pair = true;
-      // The wide tile: long accumulations only (its epilogue is not hidden behind the next tile), enough tiles for
-      // several waves, and a width for which the 512-column steps do not overshoot the triangle by much.
-      const long long twide = (long long)gemm_tiles_per_batch(d.m, d.n, 512, d.tri, 256) * d.batch;
-      const long long depth = (long long)d.k * d.segs;
-      if (ctx->gemm_wide_k > 0 && d.promote <= 0 && depth >= ctx->gemm_wide_k && twide >= 4LL * (ctx->gemm_sms / 2) &&
-          2 * twide * 100 <= tpair * 106)
-        bn = 512;
-    } else {
-      bn = (t256 >= ctx->gemm_sms) ? 256 : 128;
-    }
+    const TileChoice t = choose_tile(ctx, d);
+    bn = t.bn;
+    pair = t.pair;
+    splits = t.splits;
   } else if (bn == 512) {
     bn = 256;
+    pair = true;
+  } else if (bn == -128) {
+    bn = 128;
     pair = true;
   } else if (bn == 1024) {
     if (d.promote > 0) return fail(kErrArg, "gemm: the wide tile has no chained accumulation");
     bn = 512;
     pair = true;
   }
-  if (bn != 128 && bn != 256 && !(bn == 512 && pair))
-    return fail(kErrArg, "gemm: tile_n must be 0, 128, 256, 512 (256 x 256 on a CTA pair) or 1024 (256 x 512 on a pair)");
+  if (!(bn == 64 && !pair) && bn != 128 && bn != 256 && !(bn == 512 && pair))
+    return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
+                         "(256 x 512 on a pair)");
 
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  // a pair's CTA loads B in boxes of 128 rows; MN-major operands always come in 64 x 64 boxes
+  // a pair's CTA loads half a tile's rows of B, at most 128 at a time; MN-major operands always come in 64 x 64 boxes
   auto operand_map = [&](const toner_operand& op, int box_rows, CUtensorMap* map, const CUtensorMap** maps) {
     if (op.list) return get_maps(ctx, op, d.batch, box_rows, stream, maps);
     return encode_one(map, op.base, op.rows, op.cols, op.ld, op.z_stride, op.nz, op.mn_major ? 64 : box_rows);
   };
   int rc = operand_map(d.a, kBM, &p.a_map, &p.a_maps);
   if (rc) return rc;
-  rc = operand_map(d.b, pair ? 128 : bn, &p.b_map, &p.b_maps);
+  rc = operand_map(d.b, pair ? (bn == 128 ? 64 : 128) : bn, &p.b_map, &p.b_maps);
   if (rc) return rc;
   p.a_z_stride = d.a.list ? 0 : d.a.z_step;
   p.b_z_stride = d.b.list ? 0 : d.b.z_step;
@@ -272,27 +363,35 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   p.maxres = d.maxres;
   p.sumsq = d.sumsq; p.maxabs = d.maxabs; p.maxaff = d.maxaff;
   p.aff_a = d.aff_a; p.aff_b = d.aff_b;
+  p.splits = splits;
+  if (splits > 1) {
+    const size_t parts = split_part_bytes(d, bn, pair, splits), counts = split_count_bytes(d, bn, pair);
+    p.split_part = static_cast<float*>(d.split_ws);
+    p.split_count = reinterpret_cast<unsigned int*>(static_cast<char*>(d.split_ws) + parts);
+    TONER_CUDA(cudaMemsetAsync(p.split_count, 0, counts, stream));
+  }
   p.status = ctx->status_dev;
   p.prof = ctx->prof_dev;
 
-  const long long total = (long long)gemm_tiles_per_batch(d.m, d.n, bn, d.tri, pair ? 256 : kBM) * d.batch;
+  const long long total = gemm_tiles(d, bn, pair) * splits;
   if (total > 0x7fffffffLL) return fail(kErrArg, "gemm: too many tiles");
   const bool chained = p.promote > 0;
-  if (pair) {
-    const int pairs = (int)(total < ctx->gemm_sms / 2 ? total : ctx->gemm_sms / 2);
-    if (bn == 512) TONER_CUDA(launch(gemm_tcgen05_kernel<512, false, true>, 2 * pairs, kGemmThreads, GemmSmem<512, true>::kTotal, stream, 2, p));
-    else if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<256, true, true>, 2 * pairs, kGemmThreads, GemmSmem<256, true>::kTotal, stream, 2, p));
-    else TONER_CUDA(launch(gemm_tcgen05_kernel<256, false, true>, 2 * pairs, kGemmThreads, GemmSmem<256, true>::kTotal, stream, 2, p));
-    return 0;
-  }
-  const int grid = (int)(total < ctx->gemm_sms ? total : ctx->gemm_sms);
-  if (bn == 256) {
-    if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<256, true>, grid, kGemmThreads, GemmSmem<256>::kTotal, stream, 0, p));
-    else TONER_CUDA(launch(gemm_tcgen05_kernel<256, false>, grid, kGemmThreads, GemmSmem<256>::kTotal, stream, 0, p));
-  } else {
-    if (chained) TONER_CUDA(launch(gemm_tcgen05_kernel<128, true>, grid, kGemmThreads, GemmSmem<128>::kTotal, stream, 0, p));
-    else TONER_CUDA(launch(gemm_tcgen05_kernel<128, false>, grid, kGemmThreads, GemmSmem<128>::kTotal, stream, 0, p));
-  }
+  const int workers = pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
+  const int grid = (int)(total < workers ? total : workers) * (pair ? 2 : 1);
+#define TONER_GEMM(BN, CHAINED, PAIR)                                                                                       \
+  TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, PAIR>, grid, kGemmThreads, GemmSmem<BN, PAIR>::kTotal, stream, PAIR ? 2 : 0, p))
+  if (pair && bn == 512) TONER_GEMM(512, false, true);
+  else if (pair && bn == 256 && chained) TONER_GEMM(256, true, true);
+  else if (pair && bn == 256) TONER_GEMM(256, false, true);
+  else if (pair && chained) TONER_GEMM(128, true, true);
+  else if (pair) TONER_GEMM(128, false, true);
+  else if (bn == 256 && chained) TONER_GEMM(256, true, false);
+  else if (bn == 256) TONER_GEMM(256, false, false);
+  else if (bn == 128 && chained) TONER_GEMM(128, true, false);
+  else if (bn == 128) TONER_GEMM(128, false, false);
+  else if (chained) TONER_GEMM(64, true, false);
+  else TONER_GEMM(64, false, false);
+#undef TONER_GEMM
   return 0;
 }
 

@@ -80,6 +80,8 @@ Context* context();
 int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cudaStream_t stream, const CUtensorMap** out);
 
 int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream);
+// Scratch (split_ws) with which launch_gemm would divide the accumulation of this product among several units; 0: none.
+size_t gemm_split_bytes(const toner_gemm_desc& d);
 
 // FP16 hi/lo split of an FP32 stack (see toner_split16).
 int split16(const float* x, const float* const* x_list, int batch, int rows, int cols, long long ld, long long bs,

@@ -314,14 +314,43 @@ int split16(const float* x, const float* const* x_list, int batch, int rows, int
 
 extern "C" {
 
+// What X^T X asks of the GEMM whatever the result's form
+static toner_gemm_desc syrk_desc(int32_t k, int32_t rows, int32_t n) {
+  toner_gemm_desc d = {};
+  d.m = n; d.n = n; d.k = rows; d.batch = k;
+  d.segs = 1;
+  d.fmt = 1;
+  d.tri = 1;
+  // The tensor core adds into its accumulator by truncation; over tens of thousands of rows the all-positive
+  // sums of the diagonal would drift low by 1e-4.  Chains of 4096 rows, summed with rounding, bound it by 1.5e-5
+  // (two such chains also outlast the epilogue of the previous tile, so the tensor core never waits for it).
+  d.promote = rows > 4096 ? 64 : 0;
+  return d;
+}
+
+size_t toner_syrk_workspace_bytes(int32_t k, int32_t rows, int32_t n) {
+  if (k <= 0 || rows <= 0 || n <= 0) return 0;
+  toner_gemm_desc d = syrk_desc(k, rows, n);
+  d.d = reinterpret_cast<float*>(16);   // (the choice depends on which results there are, not where)
+  return toner::gemm_split_bytes(d);
+}
+
 int toner_syrk_upper(const void* const* x_list, const void* x_base, int64_t x_batch_stride, int32_t k, int32_t rows,
                      int32_t n, int64_t ld, float* out, int32_t mode, float beta, float gamma, void* stream) {
+  return toner_syrk_upper_ws(x_list, x_base, x_batch_stride, k, rows, n, ld, out, mode, beta, gamma, nullptr, 0, stream);
+}
+
+int toner_syrk_upper_ws(const void* const* x_list, const void* x_base, int64_t x_batch_stride, int32_t k, int32_t rows,
+                        int32_t n, int64_t ld, float* out, int32_t mode, float beta, float gamma, void* workspace,
+                        size_t workspace_bytes, void* stream) {
   using namespace toner;
   if ((!x_list && !x_base) || !out) return fail(kErrArg, "syrk: null pointer");
   if (k <= 0 || rows <= 0 || n <= 0) return fail(kErrArg, "syrk: sizes must be positive");
   if (n % 8 != 0 || ld % 8 != 0) return fail(kErrArg, "syrk: n and ld must be multiples of 8");
   if (mode < 0 || mode > 2) return fail(kErrArg, "syrk: mode must be 0 (PACKED), 1 (PACKED_ACC) or 2 (EMA_FULL)");
-  toner_gemm_desc d = {};
+  toner_gemm_desc d = syrk_desc(k, rows, n);
+  d.split_ws = workspace;
+  d.split_ws_bytes = (int64_t)workspace_bytes;
   toner_operand op = {};
   op.base = x_base;
   op.list = x_list;
@@ -334,14 +363,6 @@ int toner_syrk_upper(const void* const* x_list, const void* x_base, int64_t x_ba
   op.mn_major = 1;  // the buffer is (rows = k-index) x (n = m/n-index): X^T X reads it transposed on both sides
   d.a = op;
   d.b = op;
-  d.m = n; d.n = n; d.k = rows; d.batch = k;
-  d.segs = 1;
-  d.fmt = 1;
-  d.tri = 1;
-  // The tensor core adds into its accumulator by truncation; over tens of thousands of rows the all-positive
-  // sums of the diagonal would drift low by 1e-4.  Chains of 4096 rows, summed with rounding, bound it by 1.5e-5
-  // (two such chains also outlast the epilogue of the previous tile, so the tensor core never waits for it).
-  d.promote = rows > 4096 ? 64 : 0;
   const long long tri_elems = (long long)n * (n + 1) / 2;
   if (mode == 2) {
     d.mirror = 1;

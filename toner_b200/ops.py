@@ -195,6 +195,13 @@ def gemm(a: Operand, b: Operand, *, m: int, n: int, k: int, batch: int, fmt: int
     check(_lib.load().toner_gemm(C.byref(desc), _stream()), "toner_gemm")
 
 
+def _syrk_scratch(lib, k: int, rows: int, n: int, out: torch.Tensor):
+    """Scratch for few statistics over many rows, from the caching allocator: handed back when the call returns, and reused
+    only behind it on the same stream."""
+    need = lib.toner_syrk_workspace_bytes(k, rows, n)
+    return (torch.empty(need, device=out.device, dtype=torch.uint8) if need else None), need
+
+
 def syrk_upper(x, out: torch.Tensor, mode: int = PACKED, beta: float = 0.0, gamma: float = 1.0) -> None:
     """Upper-triangle X^T X of BF16 row buffers (toner_syrk_upper).
 
@@ -205,8 +212,9 @@ def syrk_upper(x, out: torch.Tensor, mode: int = PACKED, beta: float = 0.0, gamm
         if x.dtype != torch.bfloat16 or x.ndim != 3 or x.stride(2) != 1:
             raise ValueError("row buffers are (k, rows, n) BF16 with contiguous columns")
         k, rows, n = x.shape
-        check(lib.toner_syrk_upper(None, x.data_ptr(), x.stride(0), k, rows, n, x.stride(1), out.data_ptr(), mode,
-                                   beta, gamma, _stream()), "toner_syrk_upper")
+        ws, ws_bytes = _syrk_scratch(lib, k, rows, n, out)
+        check(lib.toner_syrk_upper_ws(None, x.data_ptr(), x.stride(0), k, rows, n, x.stride(1), out.data_ptr(), mode,
+                                      beta, gamma, _ptr(ws), ws_bytes, _stream()), "toner_syrk_upper")
         return
     xs = list(x)
     _need_cuda(*xs, out)
@@ -216,8 +224,9 @@ def syrk_upper(x, out: torch.Tensor, mode: int = PACKED, beta: float = 0.0, gamm
             raise ValueError("row buffers are equally shaped (rows, n) BF16 matrices with contiguous columns")
     arr = (C.c_void_p * len(xs))(*[t.data_ptr() for t in xs])
     rows, n = first.shape
-    check(lib.toner_syrk_upper(C.cast(arr, C.POINTER(C.c_void_p)), None, 0, len(xs), rows, n, first.stride(0),
-                               out.data_ptr(), mode, beta, gamma, _stream()), "toner_syrk_upper")
+    ws, ws_bytes = _syrk_scratch(lib, len(xs), rows, n, out)
+    check(lib.toner_syrk_upper_ws(C.cast(arr, C.POINTER(C.c_void_p)), None, 0, len(xs), rows, n, first.stride(0),
+                                  out.data_ptr(), mode, beta, gamma, _ptr(ws), ws_bytes, _stream()), "toner_syrk_upper")
 
 
 def gather_rows(x: torch.Tensor, positions: torch.Tensor, dst: torch.Tensor) -> None:
