@@ -305,6 +305,11 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
                             int32_t track_sweeps, float* deflate, int32_t deflate_rank, int32_t* deflated_out,
                             void* workspace, size_t workspace_bytes, void* stream);
 
+/* What a host reads after that call, written to HOST memory the device can address (pinned) by one kernel: status, norms,
+ * lmin, deflated (k words each, in this order), then the status word of toner_status_snapshot: 4 k + 1 words. */
+int toner_factor_report(const int32_t* status, const float* norms, const float* lmin, const int32_t* deflated, int32_t k,
+                        int32_t* host_out, void* stream);
+
 /* ------------------------------------------------------------------ Newton-Schulz polar iteration
  * x = u / (||u||_F + eps); `steps` times  A = x x^T (on the short side),  x <- a x + (b A + c A A) x  with
  * (a, b, c) = (3.4445, -4.7750, 2.0315); every product takes BF16-rounded operands and accumulates /
@@ -385,6 +390,41 @@ int toner_apply_delta(float* const* weight_ptrs, const float* delta, int32_t cou
  * and p.add_(o, alpha = -lr sqrt(max(1, rows / cols))) in one pass (src/toner/fast/muon.py:118-119,160-164). */
 int toner_apply_scaled(float* const* weight_ptrs, const float* delta, int32_t count, int64_t per, float weight_scale,
                        float delta_scale, void* stream);
+
+/* ------------------------------------------------------------------ whole stages of an update
+ * A stack of `count` equally shaped (rows, cols) weights whose statistics are entries first, first + step, ... of a set of
+ * `factors` factors, with the scratch its update needs: what the fused entry points below sequence (the reference's compiled
+ * update bodies, src/toner/fast/engine.py:17-63).  Device pointers; NULL inner_planes: the inner factor is the identity. */
+typedef struct toner_matrix_group {
+  const float* const* grads;   /* device table of gradients */
+  float* const* weights;       /* device table of weights (read only here) */
+  float* m; float* v;          /* first / second moment stacks (v: AdamT) */
+  float* work; float* work2;   /* FP32 stacks (work2: AdamT) */
+  void* planes; float* inv;    /* FP16 hi/lo planes (2, count, rows, cols), count inverse scales */
+  uint32_t* maxabs;            /* 3 * count accumulators */
+  float* c1; float* c2;        /* count coefficients each */
+  float* ss; float* ss_scratch;/* AdamT: 2 * count sums of squares, toner_sumsq_scratch_bytes(count) */
+  const void* inner_planes; const float* inner_inv;   /* factor planes (2, factors, cols, cols) and inverse scales */
+  const void* outer_planes; const float* outer_inv;
+  const float* outer_fro2;     /* squared Frobenius norms of the outer factors */
+  int32_t count, rows, cols, factors, first, step;
+} toner_matrix_group;
+
+/* m <- mu m + g, work <- (g + mu m  or  m) R_inner: what the polar iteration starts from */
+int toner_muont_input(const toner_matrix_group* group, float mu, int32_t nesterov, void* stream);
+/* delta = -(c1 W R + c2 P) R with P in `work`, c1 = lr wd cols / ||R||_F^2, c2 = lr scale sqrt(cols) / ||R||_F; polar_maxabs
+ * (optional, used without weight decay): max |P| per matrix as FP32 bits */
+int toner_muont_delta(const toner_matrix_group* group, const uint32_t* polar_maxabs, float lr, float weight_decay, float scale,
+                      float* delta, void* stream);
+/* moments, ratio and shaped decay of AdamT: delta = -(c1 W R) R - lr ||U||_F U R / ||U R||_F */
+int toner_adamt_delta(const toner_matrix_group* group, float lr, float weight_decay, float beta1, float beta2, float bc1, float bc2,
+                      float eps, float* delta, void* stream);
+
+/* Lists of `count` separately allocated matrices of `numel` FP32 elements (a multiple of 4, 16-byte aligned), HOST arrays of
+ * device pointers:  *host_flag (HOST memory the device can address) <- 1 if any element is NaN or Inf, else untouched;
+ * dst[i] <- beta dst[i] + gamma src[i] (beta == 0: dst is not read). */
+int toner_list_finite(const float* const* ptrs, int32_t count, int64_t numel, int32_t* host_flag, void* stream);
+int toner_list_axpby(const float* const* src, float* const* dst, int32_t count, int64_t numel, float beta, float gamma, void* stream);
 
 #ifdef __cplusplus
 }

@@ -59,6 +59,18 @@ class GemmDesc(C.Structure):
     ]
 
 
+class MatrixGroup(C.Structure):
+    _fields_ = [
+        ("grads", C.c_void_p), ("weights", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p),
+        ("work", C.c_void_p), ("work2", C.c_void_p), ("planes", C.c_void_p), ("inv", C.c_void_p), ("maxabs", C.c_void_p),
+        ("c1", C.c_void_p), ("c2", C.c_void_p), ("ss", C.c_void_p), ("ss_scratch", C.c_void_p),
+        ("inner_planes", C.c_void_p), ("inner_inv", C.c_void_p), ("outer_planes", C.c_void_p), ("outer_inv", C.c_void_p),
+        ("outer_fro2", C.c_void_p),
+        ("count", C.c_int32), ("rows", C.c_int32), ("cols", C.c_int32), ("factors", C.c_int32), ("first", C.c_int32),
+        ("step", C.c_int32),
+    ]
+
+
 # name -> (restype, argtypes).  Every symbol include/toner_b200.h declares is listed here.
 _vp, _i32, _i64, _f32, _sz = C.c_void_p, C.c_int32, C.c_int64, C.c_float, C.c_size_t
 SIGNATURES = {
@@ -86,6 +98,7 @@ SIGNATURES = {
     "toner_inv_roots_ex": (C.c_int, [_vp, _i32, _i32, _f32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "toner_inv_roots_tracked": (C.c_int, [_vp, _i32, _i32, _f32, _i32, _i32, _i32, _f32, _i32, _vp, _vp, _vp, _vp, _vp, _vp,
                                           _vp, _vp, _i32, _vp, _i32, _vp, _vp, _sz, _vp]),
+    "toner_factor_report": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _vp, _vp]),
     "toner_ns_polar_workspace_bytes": (C.c_size_t, [_i32, _i32, _i32]),
     "toner_ns_polar": (C.c_int, [_vp, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _sz, _vp]),
     "toner_sumsq_scratch_bytes": (C.c_size_t, [_i32]),
@@ -104,6 +117,11 @@ SIGNATURES = {
     "toner_scale_stack": (C.c_int, [_vp, _vp, _vp, _i32, _i64, _vp]),
     "toner_apply_delta": (C.c_int, [_vp, _vp, _i32, _i64, _vp]),
     "toner_apply_scaled": (C.c_int, [_vp, _vp, _i32, _i64, _f32, _f32, _vp]),
+    "toner_muont_input": (C.c_int, [C.POINTER(MatrixGroup), _f32, _i32, _vp]),
+    "toner_muont_delta": (C.c_int, [C.POINTER(MatrixGroup), _vp, _f32, _f32, _f32, _vp, _vp]),
+    "toner_adamt_delta": (C.c_int, [C.POINTER(MatrixGroup), _f32, _f32, _f32, _f32, _f32, _f32, _f32, _vp, _vp]),
+    "toner_list_finite": (C.c_int, [C.POINTER(_vp), _i32, _i64, _vp, _vp]),
+    "toner_list_axpby": (C.c_int, [C.POINTER(_vp), C.POINTER(_vp), _i32, _i64, _f32, _f32, _vp]),
     "toner_split16": (C.c_int, [_vp, _vp, _i32, _i32, _i32, _i64, _i64, _f32, _f32, _vp, _vp, _vp, _vp, _vp]),
 }
 

@@ -16,12 +16,14 @@ The two right-multiplications of the MuonT update are fused the way the referenc
 
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
-from . import ops
+from . import _lib, ops
 
 
 class Scratch:
@@ -88,11 +90,15 @@ class FactorSet:
         self.fro2_lo = torch.empty(k, device=device, dtype=torch.float32)
         self.fro2_hi = torch.empty(k, device=device, dtype=torch.float32) if self.q > 1 else None
         self.status = torch.zeros(k, device=device, dtype=torch.int32)
-        self.status_host = torch.zeros(k, dtype=torch.int32).pin_memory()
+        # What finish() reads, written by one kernel into pinned memory: status, norms, lmin, deflated (k words each) and
+        # the status word of the kernels' bounded waits.
+        self._host = torch.zeros(4 * k + 1, dtype=torch.int32).pin_memory()
+        self._host_np = self._host.numpy()
+        self.status_host = self._host[:k]
         # ||A'||_F of every statistic as the last factorisation saw it: next step's spectrum bound comes from it
         # (the statistics are EMAs and move by a few percent per step)
         self.norms = torch.zeros(k, device=device, dtype=torch.float32)
-        self.norms_host = torch.zeros(k, dtype=torch.float32).pin_memory()
+        self.norms_host = self._host[k:2 * k].view(torch.float32)
         self.lower = 0.0
         # Tracking of each statistic's smallest eigenvalue (toner_inv_roots_tracked): with it the next step's Newton
         # schedule starts from an estimate of the actual spectrum (verified after the chain) instead of the bound
@@ -100,14 +106,14 @@ class FactorSet:
         self.tracking = True
         self.track = torch.zeros(k, n, device=device, dtype=torch.float32)
         self.lmin = torch.zeros(k, device=device, dtype=torch.float32)
-        self.lmin_host = torch.zeros(k, dtype=torch.float32).pin_memory()
+        self.lmin_host = self._host[2 * k:3 * k].view(torch.float32)
         self.track_restart = True        # the vectors hold nothing yet (or the statistics were replaced)
         # Dominant directions (outlier features): eight vector slots per statistic, found by block power iteration and
         # deflated where they stand out.  The block is two vectors wider than the number of directions that looked like
         # outliers last time (a block wider than the group of outliers is what makes close outliers converge).
         self.deflate = torch.zeros(k, 8, n, device=device, dtype=torch.float32)
         self.deflated = torch.zeros(k, device=device, dtype=torch.int32)
-        self.deflated_host = torch.zeros(k, dtype=torch.int32).pin_memory()
+        self.deflated_host = self._host[3 * k:4 * k]
         self.deflate_rank = 4
         self.block_deflation = True      # False: the engine's own single-vector deflation (one dominant direction)
         self.ritz_norm = True            # the norm from the block iteration once it has followed the statistic for two steps
@@ -117,7 +123,6 @@ class FactorSet:
         self.estimate_backoff = 0        # steps left during which only certified bounds are used (after a bound failed)
         self.bound_failures = 0
         self.status_event: Optional[torch.cuda.Event] = None
-        self.health = ops.Health()
         self._root_bounds = None
         self.lo_planes = torch.empty(2, k, n, n, device=device, dtype=torch.float16)
         self.lo_inv = torch.empty(k, device=device, dtype=torch.float32)
@@ -129,7 +134,6 @@ class FactorSet:
         per = ops.inv_roots_workspace_bytes(1, n)
         if k == 0:            # a rank that owns no statistic of this width (weighted ownership): nothing to factor
             self.workspace = None
-            self.iterations = self.finish_order = 0
             self.fallbacks = self.repairs = 0
             return
         if chunk is None:
@@ -138,10 +142,22 @@ class FactorSet:
             budget = min(32 << 30, torch.cuda.get_device_properties(device).total_memory // 5)
             chunk = max(1, min(k, budget // per))
         self.workspace = self.scratch.bytes_like("inv_roots", ops.inv_roots_workspace_bytes(chunk, n), device)
-        self.iterations = ops.inv_roots_iterations(n, self.damping, self.p)
-        self.finish_order = ops.inv_roots_finish_order(n, self.damping, self.p)
+        self._lower_used = 0.0           # the bound the last call's schedule was built for
         self.fallbacks = 0
         self.repairs = 0
+
+    @property
+    def iterations(self) -> int:
+        """Newton steps of the last factorisation (before the first: of the bound that always holds)."""
+        if self.k == 0:
+            return 0
+        return (ops.inv_roots_iterations_for(self._lower_used, self.p) if self._lower_used > 0
+                else ops.inv_roots_iterations(self.n, self.damping, self.p))
+
+    @property
+    def finish_order(self) -> int:
+        """Degree of the last factorisation's finishing polynomial."""
+        return ops.inv_roots_finish_order(self.n, self.damping, self.p, self._lower_used) if self.k else 0
 
     # -- which stored root serves a given strength
     def _is_hi(self, strength: float) -> bool:
@@ -175,7 +191,7 @@ class FactorSet:
         # lower bound is an estimate as well, so that both are verified after the chain.
         ritz = (blocked and self.ritz_norm and self.lower_is_estimate and not self.track_restart
                 and self._warm_calls >= 2
-                and int((self.deflated_host & 255).max()) < min(self._rank_used, self.deflate_rank))
+                and int((self._host_np[3 * self.k:4 * self.k] & 255).max()) < min(self._rank_used, self.deflate_rank))
         self._warm_calls = 0 if (self.track_restart or not blocked) else self._warm_calls + 1
         self._rank_used = self.deflate_rank if blocked else 0
         self.ritz_in_flight = bool(ritz)
@@ -191,15 +207,9 @@ class FactorSet:
                       ritz_norm=ritz)
         self.track_restart = False
         self._estimate_in_flight = self.lower_is_estimate
-        self.iterations = (ops.inv_roots_iterations_for(self.lower, self.p) if self.lower > 0
-                           else ops.inv_roots_iterations(self.n, self.damping, self.p))
-        self.finish_order = ops.inv_roots_finish_order(self.n, self.damping, self.p, self.lower)
+        self._lower_used = self.lower
         self._split()
-        self.status_host.copy_(self.status, non_blocking=True)
-        self.norms_host.copy_(self.norms, non_blocking=True)
-        self.lmin_host.copy_(self.lmin, non_blocking=True)
-        self.deflated_host.copy_(self.deflated, non_blocking=True)
-        self.health.arm("the factor computation")
+        ops.factor_report(self.status, self.norms, self.lmin, self.deflated, self._host)
         self.status_event = torch.cuda.Event()
         self.status_event.record(torch.cuda.current_stream())
 
@@ -229,18 +239,21 @@ class FactorSet:
             return 0
         self.status_event.synchronize()
         self.status_event = None
-        self.health.check()   # a product of the factor engine that gave up a wait: raise before the factors are used
-        codes = self.status_host.tolist()
-        bad = [i for i, s in enumerate(codes) if s != 0]
+        k, host = self.k, self._host_np
+        if host[4 * k]:       # a product of the factor engine that gave up a wait: raise before the factors are used
+            ops.raise_gave_up(int(host[4 * k]), "the factor computation")
+        codes = host[:k].tolist()
+        bad = [i for i, s in enumerate(codes) if s != 0] if any(codes) else []
         # Next step's bound.  Certified: damping / norm of the widest statistic, with room for one step of EMA drift.
         # Estimated (tracking): the smallest eigenvalue found in this step's roots over the norm, halved -- the
         # estimate errs high by up to a quarter, the statistic moves by a few percent per step -- and used only where it
         # buys a step.  A flagged statistic (not converged, or below the bound used) sends the next step back to the
         # bound that always holds; an estimate that failed its verification is not tried again for eight steps.
-        top = float(self.norms_host.max())
+        norms, lmin = host[k:2 * k].view(np.float32), host[2 * k:3 * k].view(np.float32)
+        top = float(norms.max())
         worst = self.damping / (self.n * (1.0 + self.damping))
         if self.tracking and self.block_deflation:
-            candidates = int((self.deflated_host >> 8).max())
+            candidates = int((host[3 * k:4 * k] >> 8).max())
             self.deflate_rank = max(2, min(8, candidates + 2))
         self.lower, self.lower_is_estimate = 0.0, False
         if getattr(self, "_estimate_in_flight", False) and any(c in (1, 4) for c in codes):
@@ -256,7 +269,8 @@ class FactorSet:
             if worst < hint < 1.0:
                 self.lower = hint
             if self.tracking and not self.estimate_backoff and not bad:
-                ratio = float((self.lmin_host / self.norms_host).min())
+                with np.errstate(all="ignore"):
+                    ratio = float((lmin / norms).min())
                 guess = min(0.5 * ratio, 0.8)
                 if math.isfinite(guess) and guess > 1.5 * max(self.lower, worst):
                     self.lower, self.lower_is_estimate = guess, True
@@ -309,6 +323,7 @@ class MatrixGroup:
         self.m = torch.zeros(shape, device=self.device, dtype=torch.float32)
         self.v = torch.zeros(shape, device=self.device, dtype=torch.float32) if kind == "adamt" else None
         self.weight_ptrs = ops.pointer_table(self.weights)
+        self._c: Optional[_lib.MatrixGroup] = None   # the group as the C ABI takes it; addresses set in c_group()
         self._grad_key: Optional[Tuple[int, ...]] = None
         self._grad_ptrs: Optional[torch.Tensor] = None
 
@@ -323,26 +338,7 @@ class MatrixGroup:
         return self._grad_ptrs
 
 
-def _product(a_planes, a_inv, group: MatrixGroup, which: str, d, coarse: bool = False, **kw) -> None:
-    """d[b] = A[b] @ R[first + b*step], R the inner or outer factor (symmetric).  FP32-accurate from the FP16 hi/lo
-    planes (three plane products in one accumulator); ``coarse`` multiplies the hi planes only (relative error
-    about 5e-4), for terms that enter the result with a small coefficient."""
-    f = group.factors
-    r_planes, r_inv = f.planes(which)
-    count, m, n = group.count, group.out_features, group.in_features
-    if coarse:
-        a = ops.operand(a_planes, seg_z=(0, 0, 0))
-        b = ops.operand(r_planes, seg_z=(group.first, group.first, group.first), z_step=group.step)
-        segs = 1
-    else:
-        a = ops.operand(a_planes, seg_z=(0, 0, count))
-        b = ops.operand(r_planes, seg_z=(group.first, f.k + group.first, group.first), z_step=group.step)
-        segs = 3
-    ops.gemm(a, b, m=m, n=n, k=n, batch=count, fmt=0, segs=segs, d=d, alpha_a=a_inv,
-             alpha_b=r_inv[group.first:], alpha_b_step=group.step, promote=0, **kw)
-
-
-def _muont_buffers(group: MatrixGroup, scratch: Scratch, work: Optional[torch.Tensor] = None):
+def _buffers(group: MatrixGroup, scratch: Scratch, work: Optional[torch.Tensor] = None) -> Dict[str, torch.Tensor]:
     """Scratch of one matrix group's update.  `work` (count, out, in) replaces the shared FP32 work stack: several groups
     of one shape can then keep their stacks side by side and go through Newton-Schulz as one batch."""
     dev = group.device
@@ -353,23 +349,41 @@ def _muont_buffers(group: MatrixGroup, scratch: Scratch, work: Optional[torch.Te
     return dict(work=work if work is not None else scratch.get("work", shape, torch.float32, dev),
                 planes=scratch.get("planes", (2,) + shape, torch.float16, dev),
                 inv=scratch.get("inv", (count,), torch.float32, dev),
-                maxabs=scratch.get("maxabs", (count,), torch.int32, dev),
+                maxabs=scratch.get("maxabs", (3 * count,), torch.int32, dev),
                 c1=scratch.get("c1", (count,), torch.float32, dev),
                 c2=scratch.get("c2", (count,), torch.float32, dev))
+
+
+def _c_group(group: MatrixGroup, buf: Dict[str, torch.Tensor], grads: Optional[Sequence[torch.Tensor]]) -> _lib.MatrixGroup:
+    """The group as the fused entry points take it (toner_matrix_group)."""
+    f, c = group.factors, group._c
+    if c is None:
+        c = group._c = _lib.MatrixGroup()
+        c.weights = group.weight_ptrs.data_ptr()
+        c.m = group.m.data_ptr()
+        c.v = None if group.v is None else group.v.data_ptr()
+        c.count, c.rows, c.cols = group.count, group.out_features, group.in_features
+        c.factors, c.first, c.step = f.k, group.first, group.step
+        for which in ("inner", "outer"):
+            planes, inv = f.planes(which)
+            setattr(c, which + "_planes", None if planes is None else planes.data_ptr())
+            setattr(c, which + "_inv", None if inv is None else inv.data_ptr())
+        c.outer_fro2 = f.fro2_outer.data_ptr() if f.outer_strength != 0 else None
+    if grads is not None:
+        c.grads = group.grad_ptrs(grads).data_ptr()
+    for name, t in buf.items():
+        setattr(c, name, t.data_ptr())
+    return c
 
 
 def muont_ns_input(group: MatrixGroup, grads: Sequence[torch.Tensor], scratch: Scratch, *, momentum: float,
                    nesterov: bool, work: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Stage 1 of the MuonT update: momentum, Nesterov direction and the inner preconditioning d R_in
     (src/toner/reference.py:197-204).  Returns the (count, out, in) stack the polar iteration starts from."""
-    f = group.factors
-    buf = _muont_buffers(group, scratch, work)
-    work, planes, inv, maxabs = buf["work"], buf["planes"], buf["inv"], buf["maxabs"]
-    ops.muont_momentum(group.grad_ptrs(grads), group.m, work, momentum, nesterov, maxabs)
-    if f.inner_strength != 0:
-        ops.split16(work, planes=planes, inv_scale=inv, maxabs=maxabs)
-        _product(planes, inv, group, "inner", work)
-    return work
+    buf = _buffers(group, scratch, work)
+    _lib.check(_lib.load().toner_muont_input(ctypes.byref(_c_group(group, buf, grads)), momentum, int(nesterov), ops._stream()),
+               "toner_muont_input")
+    return buf["work"]
 
 
 def muont_delta_from_polar(group: MatrixGroup, polar: torch.Tensor, delta: torch.Tensor, scratch: Scratch, *, lr: float,
@@ -378,31 +392,15 @@ def muont_delta_from_polar(group: MatrixGroup, polar: torch.Tensor, delta: torch
     """Stage 3: outer map, shape scale and shaped weight decay (src/toner/reference.py:206-215), fused as the
     reference's engine fuses them (src/toner/fast/engine.py:42-51):
     delta = -((lr wd n / ||R||^2) W R + (lr s sqrt(n) / ||R||) P) R.  `polar` may be the work stack itself."""
-    f = group.factors
-    count, m, n = group.count, group.out_features, group.in_features
-    buf = _muont_buffers(group, scratch, work)
-    work, planes, inv, maxabs, c1, c2 = (buf[k] for k in ("work", "planes", "inv", "maxabs", "c1", "c2"))
-    if polar.data_ptr() != work.data_ptr():
-        work.copy_(polar)
+    buf = _buffers(group, scratch, work)
+    if polar.data_ptr() != buf["work"].data_ptr():
+        buf["work"].copy_(polar)
         polar_maxabs = None
-    scale = max(1.0, m / n) ** 0.5
-    if f.outer_strength == 0:
+    if group.factors.outer_strength == 0:
         raise ValueError("outer_strength 0 is not supported by the CUDA path")
-    ops.muont_coeffs(f.fro2_outer, group.first, group.step, count, n, lr, weight_decay, scale, c1, c2)
-    if weight_decay != 0:
-        ops.split16_list(group.weight_ptrs, count, m, n, planes, inv, maxabs)
-        ops.scale_vec(inv, c1)
-        maxabs.zero_()
-        # V = c1 W R + c2 P.  The decay term is lr wd ||W|| against lr ||P||, about 1 % of V: the hi planes suffice
-        _product(planes, inv, group, "outer", work, coarse=True, c=work, beta=1.0, beta_v=c2, maxabs=maxabs)
-        ops.split16(work, planes=planes, inv_scale=inv, maxabs=maxabs)
-    else:
-        if polar_maxabs is None:
-            ops.split16(work, planes=planes, inv_scale=inv, scratch=maxabs)
-        else:
-            ops.split16(work, planes=planes, inv_scale=inv, maxabs=polar_maxabs)
-        ops.scale_vec(inv, c2)  # V = c2 P
-    _product(planes, inv, group, "outer", delta, alpha=-1.0)
+    scale = max(1.0, group.out_features / group.in_features) ** 0.5
+    _lib.check(_lib.load().toner_muont_delta(ctypes.byref(_c_group(group, buf, None)), ops._ptr(polar_maxabs), lr, weight_decay,
+                                             scale, delta.data_ptr(), ops._stream()), "toner_muont_delta")
 
 
 def muont_group_delta(group: MatrixGroup, grads: Sequence[torch.Tensor], delta: torch.Tensor, scratch: Scratch, *,
@@ -412,7 +410,7 @@ def muont_group_delta(group: MatrixGroup, grads: Sequence[torch.Tensor], delta: 
     dev = group.device
     count, m, n = group.count, group.out_features, group.in_features
     work = muont_ns_input(group, grads, scratch, momentum=momentum, nesterov=nesterov)
-    maxabs = _muont_buffers(group, scratch)["maxabs"]
+    maxabs = scratch.get("maxabs_polar", (count,), torch.int32, dev)
     ns_ws = scratch.bytes_like("ns", ops.ns_polar_workspace_bytes(count, m, n), dev)
     ops.ns_polar(work, ns_steps, ns_eps, out=work, maxabs=maxabs, workspace=ns_ws)
     muont_delta_from_polar(group, work, delta, scratch, lr=lr, weight_decay=weight_decay, polar_maxabs=maxabs)
@@ -447,42 +445,14 @@ def muont_groups_delta(groups: Sequence[MatrixGroup], grads: Sequence[Sequence[t
 def adamt_group_delta(group: MatrixGroup, grads: Sequence[torch.Tensor], delta: torch.Tensor, scratch: Scratch, *,
                       lr: float, weight_decay: float, betas: Tuple[float, float], eps: float, t: int) -> None:
     """Write the AdamT parameter change of every matrix of the group into ``delta``."""
-    f, dev = group.factors, group.device
-    count, m, n = group.count, group.out_features, group.in_features
-    shape = (count, m, n)
     b1, b2 = betas
-    bc1, bc2 = 1 - b1 ** t, 1 - b2 ** t
-    work = scratch.get("work", shape, torch.float32, dev)
-    work2 = scratch.get("work2", shape, torch.float32, dev)
-    planes = scratch.get("planes", (2,) + shape, torch.float16, dev)
-    inv = scratch.get("inv", (count,), torch.float32, dev)
-    maxabs = scratch.get("maxabs", (count,), torch.int32, dev)
-    c1 = scratch.get("c1", (count,), torch.float32, dev)
-    c2 = scratch.get("c2", (count,), torch.float32, dev)
-    ss0 = scratch.get("ss0", (count,), torch.float32, dev)
-    ss1 = scratch.get("ss1", (count,), torch.float32, dev)
-    ssq_ws = scratch.bytes_like("sumsq", ops.sumsq_scratch_bytes(count), dev)
-    gp = group.grad_ptrs(grads)
-    ops.adamt_first_moment(gp, group.m, b1)
-    ops.split16_list(gp, count, m, n, planes, inv, maxabs)
-    _product(planes, inv, group, "inner", work)                       # t = g R
-    ops.split16(group.m, planes=planes, inv_scale=inv, scratch=maxabs)
-    _product(planes, inv, group, "inner", work2, alpha=1.0 / bc1)     # (m / bc1) R
-    ops.adamt_ratio(work, group.v, work2, b2, bc2, eps, maxabs)       # U, in work2
-    ops.sumsq(work2, out=ss0, scratch=ssq_ws)
-    ops.split16(work2, planes=planes, inv_scale=inv, maxabs=maxabs)
-    _product(planes, inv, group, "inner", work)                       # U R
-    ops.sumsq(work, out=ss1, scratch=ssq_ws)
-    ops.adamt_coeffs(f.fro2_outer, group.first, group.step, count, n, lr, weight_decay, ss0, ss1, c1, c2)
-    if weight_decay != 0:
-        ops.split16_list(group.weight_ptrs, count, m, n, planes, inv, maxabs)
-        ops.scale_vec(inv, c1)
-        maxabs.zero_()
-        _product(planes, inv, group, "outer", work2, coarse=True, maxabs=maxabs)   # c1 W R (small term: hi planes)
-        ops.split16(work2, planes=planes, inv_scale=inv, maxabs=maxabs)
-        _product(planes, inv, group, "outer", delta, alpha=-1.0, c=work, beta=1.0, beta_v=c2)
-    else:
-        ops.scale_stack(work, c2, delta)                              # delta = c2 * U R
+    count, dev = group.count, group.device
+    buf = _buffers(group, scratch)
+    buf["work2"] = scratch.get("work2", tuple(group.m.shape), torch.float32, dev)
+    buf["ss"] = scratch.get("ss", (2 * count,), torch.float32, dev)
+    buf["ss_scratch"] = scratch.bytes_like("sumsq", ops.sumsq_scratch_bytes(count), dev)
+    _lib.check(_lib.load().toner_adamt_delta(ctypes.byref(_c_group(group, buf, grads)), lr, weight_decay, b1, b2, 1 - b1 ** t,
+                                             1 - b2 ** t, eps, delta.data_ptr(), ops._stream()), "toner_adamt_delta")
 
 
 def apply_group_delta(group: MatrixGroup, delta: torch.Tensor) -> None:

@@ -100,20 +100,29 @@ struct FinishPoly {
   double c[kMaxFinishOrder + 1] = {};  // q(r) = sum_j c[j] r^j
 };
 
-// Degree-m Chebyshev interpolant of (1 - r)^(-1/p) on [lo, hi] as monomial coefficients; returns its largest
-// relative error on the interval.
-static double finish_fit(int p, double lo, double hi, int m, double* c) {
-  const double kPi = 3.14159265358979323846;
-  double cheb[kMaxFinishOrder + 1];
-  for (int j = 0; j <= m; ++j) {
-    double acc = 0.0;
-    for (int k = 0; k <= m; ++k) {
-      const double th = kPi * (k + 0.5) / (m + 1);
-      const double r = lo + (hi - lo) * (std::cos(th) + 1.0) * 0.5;
-      acc += std::pow(1.0 - r, -1.0 / p) * std::cos(j * th);
-    }
-    cheb[j] = acc * (j == 0 ? 1.0 : 2.0) / (m + 1);
+// (1 - r)^(1/p) at the points where a fit is checked; a point is evaluated when a fit first gets that far.
+struct FitSamples {
+  static constexpr int kPoints = 257;
+  double g[kPoints];
+  int known = 0;
+  double at(int i, int p, double lo, double hi) {
+    for (; known <= i; ++known) g[known] = std::pow(1.0 - (lo + (hi - lo) * known / (kPoints - 1)), 1.0 / p);
+    return g[i];
   }
+};
+
+// Degree-m Chebyshev interpolant of (1 - r)^(-1/p) on [lo, hi] as monomial coefficients; whether its largest relative
+// error on the interval is below `tail`.
+static bool finish_fit(int p, double lo, double hi, int m, double tail, FitSamples& samples, double* c) {
+  const double kPi = 3.14159265358979323846;
+  double cheb[kMaxFinishOrder + 1] = {};
+  for (int k = 0; k <= m; ++k) {
+    const double th = kPi * (k + 0.5) / (m + 1);
+    const double r = lo + (hi - lo) * (std::cos(th) + 1.0) * 0.5;
+    const double f = std::pow(1.0 - r, -1.0 / p);
+    for (int j = 0; j <= m; ++j) cheb[j] += f * std::cos(j * th);
+  }
+  for (int j = 0; j <= m; ++j) cheb[j] *= (j == 0 ? 1.0 : 2.0) / (m + 1);
   // sum_j cheb[j] T_j(x) in powers of x (T_{j+1} = 2 x T_j - T_{j-1}) ...
   double t0[kMaxFinishOrder + 1] = {1.0}, t1[kMaxFinishOrder + 1] = {0.0, 1.0}, px[kMaxFinishOrder + 1] = {};
   px[0] = cheb[0];
@@ -134,15 +143,13 @@ static double finish_fit(int p, double lo, double hi, int m, double* c) {
     for (int i = m; i >= 1; --i) c[i] = c[i] * beta + c[i - 1] * alpha;
     c[0] = c[0] * beta + px[j];
   }
-  double worst = 0.0;
-  const int samples = 256;
-  for (int i = 0; i <= samples; ++i) {
-    const double r = lo + (hi - lo) * i / samples;
+  for (int i = 0; i < FitSamples::kPoints; ++i) {
+    const double r = lo + (hi - lo) * i / (FitSamples::kPoints - 1);
     double q = 0.0;
     for (int j = m; j >= 0; --j) q = q * r + c[j];
-    worst = std::fmax(worst, std::fabs(q * std::pow(1.0 - r, 1.0 / p) - 1.0));
+    if (!(std::fabs(q * samples.at(i, p, lo, hi) - 1.0) < tail)) return false;
   }
-  return worst;
+  return true;
 }
 
 // In powers of r the fit's coefficients grow as the interval approaches the singularity at r = 1 (sooner for small p):
@@ -167,8 +174,9 @@ static FinishPoly finish_poly(int p, double e) {
   FinishPoly f;
   if (!(e < kFinishRadius)) return f;
   const double hi = kFinishGrow * e + kFinishPad;
+  FitSamples samples;
   for (int m = 2; m <= kMaxFinishOrder; ++m) {
-    if (finish_fit(p, kFinishLow, hi, m, f.c) < kFinishTail) {
+    if (finish_fit(p, kFinishLow, hi, m, kFinishTail, samples, f.c)) {
       f.order = m;
       if (!finish_usable(f, hi)) f.order = 0;
       return f;
@@ -187,8 +195,6 @@ static FinishPoly finish_poly_or_best(int p, double e) {
   for (int j = 1; j <= kMaxFinishOrder; ++j) f.c[j] = f.c[j - 1] * (1.0 / p + j - 1) / j;
   return f;
 }
-static int finish_order(int p, double e) { return finish_poly_or_best(p, e).order; }
-
 static int default_iterations(double l0, int p) {
   // k steps of M, then the finishing step on X alone: the k with the fewest plane passes,
   // 3 (log2 p + 2) per step of M and order - 1 for the series, among those the series can finish
@@ -211,6 +217,40 @@ static int default_iterations(double l0, int p) {
     }
   }
   return best ? best : 64;
+}
+
+// Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
+// Working it out takes tens of microseconds of host time and is asked for several times per factorisation (the call itself,
+// the step count and the degree it states), so a thread keeps the last few.
+struct Schedule {
+  double l0 = 0.0;
+  int p = 0, asked = 0;   // asked: the caller's step count, 0 = the one with the fewest plane passes
+  int iters = 0;
+  std::vector<NewtonStep> steps;
+  double l_last = 0.0;    // lower bound of the spectrum of the last M, i.e. after iters - 1 updates
+  FinishPoly fin;
+};
+
+static const Schedule& schedule_for(double l0, int p, int iters) {
+  constexpr int kKept = 8;
+  static thread_local Schedule kept[kKept];
+  static thread_local int oldest = 0;
+  if (iters < 0) iters = 0;
+  for (const Schedule& s : kept)
+    if (s.p == p && s.l0 == l0 && s.asked == iters) return s;
+  Schedule& s = kept[oldest];
+  oldest = (oldest + 1) % kKept;
+  s.p = 0;   // (not a match until it is complete)
+  s.l0 = l0;
+  s.asked = iters;
+  s.iters = iters > 0 ? iters : default_iterations(l0, p);
+  if (s.iters >= 2) {
+    s.steps = newton_schedule(l0, p, s.iters, nullptr);
+    newton_schedule(l0, p, s.iters - 1, &s.l_last);
+    s.fin = finish_poly_or_best(p, 1.0 - s.l_last);
+  }
+  s.p = p;
+  return s;
 }
 
 // ------------------------------------------------------------------ elementwise helpers
@@ -614,21 +654,27 @@ __device__ __forceinline__ void block_sum_many(double (&acc)[K], double* part, d
 constexpr int kPairs = kMaxDeflate * (kMaxDeflate + 1) / 2;  // entries of a symmetric r x r matrix, r = 8
 __device__ __forceinline__ int pair_index(int i, int j) { return i * (i + 1) / 2 + j; }  // j <= i
 
-// Cholesky-QR of the r vectors held in Y (r x n, vector-major): G = Y Y^T = L L^T (FP64, one thread), V = L^-1 Y.
-// `gram` holds G's lower triangle (pair_index order) on entry.  A vector that is (numerically) a combination of the
-// earlier ones comes out as zero; its slot is seeded afresh by the next call.
+// Cholesky-QR of the r vectors held in Y (r x n, vector-major): G = Y Y^T = L L^T (FP64), V = L^-1 Y.  `gram` holds G's
+// lower triangle (pair_index order) on entry.  A vector that is (numerically) a combination of the earlier ones comes out as
+// zero; its slot is seeded afresh by the next call.  L's columns are formed one after the other by the lanes of one warp (row
+// i of a column by lane i); the diagonal of `L` holds its reciprocal (zero for a dropped vector).
 __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, const double* gram, double (*L)[kMaxDeflate]) {
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < r; ++i) {
-      for (int j = 0; j <= i; ++j) {
-        double sum = gram[pair_index(i, j)];
-        for (int k = 0; k < j; ++k) sum -= L[i][k] * L[j][k];
-        if (i == j) {
-          L[i][i] = (sum > 1e-24 * gram[pair_index(i, i)] && sum > 0.0) ? sqrt(sum) : 0.0;
-        } else {
-          L[i][j] = L[j][j] > 0.0 ? sum / L[j][j] : 0.0;
-        }
-      }
+  if (threadIdx.x < 32) {
+    const int i = threadIdx.x;
+    double row[kMaxDeflate];
+#pragma unroll
+    for (int j = 0; j < kMaxDeflate; ++j) {
+      const bool on = i < r && j <= i && j < r;
+      double sum = on ? gram[pair_index(i, j)] : 0.0;
+#pragma unroll
+      for (int k = 0; k < kMaxDeflate; ++k)
+        if (k < j) sum -= row[k] * __shfl_sync(0xffffffffu, row[k], j);
+      // lane j holds the pivot
+      const double pivot = __shfl_sync(0xffffffffu, sum, j);
+      const double floor = j < r ? 1e-24 * gram[pair_index(j, j)] : 0.0;
+      const double inv = (j < r && pivot > floor && pivot > 0.0) ? rsqrt(pivot) : 0.0;
+      row[j] = i == j ? pivot * inv : sum * inv;
+      if (on) L[i][j] = i == j ? inv : row[j];
     }
   }
   __syncthreads();
@@ -641,7 +687,7 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
 #pragma unroll
         for (int i = 0; i < kMaxDeflate; ++i)
           if (i < j) sum -= L[j][i] * out[i];
-        out[j] = L[j][j] > 0.0 ? sum / L[j][j] : 0.0;
+        out[j] = sum * L[j][j];
       } else {
         out[j] = 0.0;
       }
@@ -651,6 +697,54 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
       if (j < r) V[(long long)j * n + c] = (float)out[j];
   }
   __syncthreads();
+}
+
+// Eigenpairs of the symmetric r x r matrix H (shared memory, FP64) by Jacobi rotations, H and Q of size kMaxDeflate with
+// zeros beyond r.  One warp: each of the seven rounds of a sweep rotates four disjoint pairs at once (round-robin order), eight
+// lanes a pair, one matrix index each.  A single thread doing the rotations one by one took 20 us of a 23 us launch at r = 4
+// and most of 160 us at r = 8.
+__device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) {
+  static_assert(kMaxDeflate == 8, "four pairs of eight lanes");
+  const int lane = threadIdx.x, pair = lane >> 3, k = lane & 7;
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    double off = 0.0, diag = 0.0;
+    for (int e = lane; e < 64; e += 32) {
+      const int i = e >> 3, j = e & 7;
+      const double h = H[i][j];
+      if (i == j) diag += h * h;
+      else if (j > i) off += h * h;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      diag += __shfl_xor_sync(0xffffffffu, diag, o);
+    }
+    if (!(off > 1e-30 * diag)) break;   // off-diagonal part below FP64 rounding of the diagonal: converged
+    for (int round = 0; round < 7; ++round) {
+      // seat 7 stays, the others rotate: pair 0 = (7, round), pair i = (round + i, round - i) mod 7
+      int a = pair == 0 ? 7 : (round + pair) % 7, b = pair == 0 ? round : (round + 7 - pair) % 7;
+      const int pp = min(a, b), qq = max(a, b);
+      const double apq = H[pp][qq];
+      double cs = 1.0, sn = 0.0;
+      if (apq != 0.0) {
+        const double tau = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
+        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+        cs = rsqrt(1.0 + t * t);
+        sn = t * cs;
+      }
+      __syncwarp();   // every pair has its rotation before any entry changes
+      const double hp = H[k][pp], hq = H[k][qq], qp = Q[k][pp], qv = Q[k][qq];   // columns pp, qq of H and Q
+      H[k][pp] = cs * hp - sn * hq;
+      H[k][qq] = sn * hp + cs * hq;
+      Q[k][pp] = cs * qp - sn * qv;
+      Q[k][qq] = sn * qp + cs * qv;
+      __syncwarp();
+      const double rp = H[pp][k], rq = H[qq][k];                                 // rows pp, qq of H
+      H[pp][k] = cs * rp - sn * rq;
+      H[qq][k] = sn * rp + cs * rq;
+      __syncwarp();
+    }
+  }
 }
 
 // start vectors: the caller's vectors (warm), or r different fixed +-1 patterns (cold, and for a slot that holds
@@ -687,10 +781,10 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
   cholesky_orthonormalise(V, V, n, r, gram, L);
 }
 
-// Rayleigh-Ritz on span(V) with Y = A V (V orthonormal): H = V Y^T, H = Q diag(theta) Q^T (Jacobi, FP64, one thread),
-// V <- Q^T V, Y <- Q^T Y (Ritz vectors, descending theta), res_j = ||Y_j - theta_j V_j|| / |theta_j|.  Unless this is
-// the last sweep, V is then replaced by the orthonormalised Y (one more step of the power iteration).  Three passes
-// over the two blocks of vectors; every reduction is taken for all pairs at once.
+// Rayleigh-Ritz on span(V) with Y = A V (V orthonormal): H = V Y^T, H = Q diag(theta) Q^T (Jacobi, FP64), V <- Q^T V,
+// Y <- Q^T Y (Ritz vectors, descending theta), res_j = ||Y_j - theta_j V_j|| / |theta_j|.  Unless this is the last sweep, V is
+// then replaced by the orthonormalised Y (one more step of the power iteration).  Three passes over the two blocks of
+// vectors; every reduction is taken for all pairs at once.
 __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float* __restrict__ y, int n, int r, int vstride,
                                                    int last, float* __restrict__ theta, float* __restrict__ res) {
   ptx::pdl_begin();
@@ -718,52 +812,30 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
     }
     block_sum_many<R * R>(acc, part, sums);
   }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < r; ++i)
-      for (int j = 0; j < r; ++j) {
-        H[i][j] = 0.5 * (sums[i * R + j] + sums[j * R + i]);
-        Q[i][j] = i == j ? 1.0 : 0.0;
-      }
-    for (int sweep = 0; sweep < 12; ++sweep) {
-      double off = 0.0;
-      for (int pp = 0; pp < r; ++pp)
-        for (int qq = pp + 1; qq < r; ++qq) off += H[pp][qq] * H[pp][qq];
-      double diag = 0.0;
-      for (int pp = 0; pp < r; ++pp) diag += H[pp][pp] * H[pp][pp];
-      if (!(off > 1e-30 * diag)) break;   // off-diagonal part below FP64 rounding of the diagonal: converged
-      for (int pp = 0; pp < r; ++pp)
-        for (int qq = pp + 1; qq < r; ++qq) {
-          const double apq = H[pp][qq];
-          if (apq == 0.0) continue;
-          const double tau = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
-          const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          const double cs = 1.0 / sqrt(1.0 + t * t), sn = t * cs;
-          for (int k = 0; k < r; ++k) {  // columns pp, qq of H and Q
-            const double hp = H[k][pp], hq = H[k][qq];
-            H[k][pp] = cs * hp - sn * hq;
-            H[k][qq] = sn * hp + cs * hq;
-            const double qp = Q[k][pp], qv = Q[k][qq];
-            Q[k][pp] = cs * qp - sn * qv;
-            Q[k][qq] = sn * qp + cs * qv;
-          }
-          for (int k = 0; k < r; ++k) {  // rows pp, qq of H
-            const double hp = H[pp][k], hq = H[qq][k];
-            H[pp][k] = cs * hp - sn * hq;
-            H[qq][k] = sn * hp + cs * hq;
-          }
-        }
+  if (threadIdx.x < 64) {
+    const int i = threadIdx.x >> 3, j = threadIdx.x & 7;
+    H[i][j] = (i < r && j < r) ? 0.5 * (sums[i * R + j] + sums[j * R + i]) : 0.0;
+    Q[i][j] = i == j ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    jacobi_warp(H, Q);
+    // descending order: lane i's place is the number of values before it; the columns of Q follow
+    const int i = threadIdx.x & 7;
+    const double mine = H[i][i];
+    int place = 0;
+    for (int j = 0; j < r; ++j) {
+      const double o = H[j][j];
+      if (o > mine || (o == mine && j < i)) ++place;
     }
-    for (int i = 0; i < r; ++i) lam[i] = H[i][i];
-    for (int i = 0; i < r; ++i) {  // selection sort, descending, columns of Q follow
-      int best = i;
-      for (int j = i + 1; j < r; ++j)
-        if (lam[j] > lam[best]) best = j;
-      if (best != i) {
-        const double t = lam[i]; lam[i] = lam[best]; lam[best] = t;
-        for (int k = 0; k < r; ++k) {
-          const double q = Q[k][i]; Q[k][i] = Q[k][best]; Q[k][best] = q;
-        }
-      }
+    double col[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) col[k] = Q[k][i];
+    __syncwarp();
+    if (threadIdx.x < r) {
+      lam[place] = mine;
+#pragma unroll
+      for (int k = 0; k < R; ++k) Q[k][place] = col[k];
     }
   }
   __syncthreads();
@@ -803,10 +875,12 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
       }
 #pragma unroll
       for (int i = 0; i < R; ++i) {
+        if (i < r) {
 #pragma unroll
-        for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += ny[i] * ny[j];
-        const double d = i < r ? ny[i] - lam[i] * nv[i] : 0.0;
-        acc[kPairs + i] += d * d;
+          for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += ny[i] * ny[j];
+          const double d = ny[i] - lam[i] * nv[i];
+          acc[kPairs + i] += d * d;
+        }
       }
     }
     block_sum_many<kPairs + R>(acc, part, sums);
@@ -1039,6 +1113,20 @@ __global__ void finish_kernel(const unsigned int* __restrict__ resid, const floa
   if (status) status[b] = st;
 }
 
+// What the host reads after a factorisation, written straight to its pinned memory: status, norms, lmin, deflated (k words
+// each) and the status word of the kernels' bounded waits.  One launch instead of five copies of a few bytes.
+__global__ void report_kernel(const int* __restrict__ status, const float* __restrict__ norms, const float* __restrict__ lmin,
+                              const int* __restrict__ deflated, const int* __restrict__ word, int* __restrict__ host, int k) {
+  ptx::pdl_begin();
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b == 0) host[4 * k] = *word;
+  if (b >= k) return;
+  host[b] = status[b];
+  host[k + b] = __float_as_int(norms[b]);
+  host[2 * k + b] = __float_as_int(lmin[b]);
+  host[3 * k + b] = deflated[b];
+}
+
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 static size_t per_statistic_bytes(int n) {
@@ -1070,43 +1158,47 @@ size_t toner_inv_roots_workspace_bytes(int32_t chunk, int32_t n) {
 
 int toner_inv_roots_iterations(int32_t n, float damping, int32_t p) {
   if (n <= 0 || !(damping > 0) || p < 1) return 0;
-  return toner::default_iterations((double)damping / ((double)n * (1.0 + damping)), p);
+  return toner::schedule_for((double)damping / ((double)n * (1.0 + damping)), p, 0).iters;
 }
 
 int toner_inv_roots_iterations_for(float lower, int32_t p) {
   if (!(lower > 0.f) || !(lower < 1.f) || p < 1) return 0;
-  return toner::default_iterations((double)lower, p);
+  return toner::schedule_for((double)lower, p, 0).iters;
 }
 
 int toner_inv_roots_finish_order_for(float lower, int32_t p, int32_t iters) {
   if (!(lower > 0.f) || !(lower < 1.f) || p < 1) return 0;
-  if (iters <= 0) iters = toner::default_iterations((double)lower, p);
-  if (iters < 2) return 0;
-  double l_last;
-  toner::newton_schedule((double)lower, p, iters - 1, &l_last);
-  return toner::finish_order(p, 1.0 - l_last);
+  const toner::Schedule& s = toner::schedule_for((double)lower, p, iters);
+  return s.iters < 2 ? 0 : s.fin.order;
 }
 
 int toner_inv_roots_schedule(float lower, int32_t p, int32_t iters, double* ab_out, int32_t ab_capacity, double* coef_out,
                              int32_t coef_capacity, int32_t* order_out, double* e_out) {
   if (!(lower > 0.f) || !(lower < 1.f) || p < 1) return 0;
-  if (iters <= 0) iters = toner::default_iterations((double)lower, p);
-  if (iters < 2) return 0;
-  const std::vector<toner::NewtonStep> sched = toner::newton_schedule((double)lower, p, iters, nullptr);
-  double l_last;
-  toner::newton_schedule((double)lower, p, iters - 1, &l_last);
-  const toner::FinishPoly fin = toner::finish_poly_or_best(p, 1.0 - l_last);
+  const toner::Schedule& s = toner::schedule_for((double)lower, p, iters);
+  if (s.iters < 2) return 0;
   if (ab_out) {
-    for (int k = 0; k < iters - 1 && 2 * k + 1 < ab_capacity; ++k) {
-      ab_out[2 * k] = sched[k].a;
-      ab_out[2 * k + 1] = sched[k].b;
+    for (int k = 0; k < s.iters - 1 && 2 * k + 1 < ab_capacity; ++k) {
+      ab_out[2 * k] = s.steps[k].a;
+      ab_out[2 * k + 1] = s.steps[k].b;
     }
   }
   if (coef_out)
-    for (int j = 0; j <= fin.order && j < coef_capacity; ++j) coef_out[j] = fin.c[j];
-  if (order_out) *order_out = fin.order;
-  if (e_out) *e_out = 1.0 - l_last;
-  return iters;
+    for (int j = 0; j <= s.fin.order && j < coef_capacity; ++j) coef_out[j] = s.fin.c[j];
+  if (order_out) *order_out = s.fin.order;
+  if (e_out) *e_out = 1.0 - s.l_last;
+  return s.iters;
+}
+
+int toner_factor_report(const int32_t* status, const float* norms, const float* lmin, const int32_t* deflated, int32_t k,
+                        int32_t* host_out, void* stream) {
+  using namespace toner;
+  Context* ctx = context();
+  if (!ctx) return kErrCuda;
+  if (!status || !norms || !lmin || !deflated || !host_out || k <= 0) return fail(kErrArg, "factor_report: bad arguments");
+  TONER_LAUNCH(report_kernel, (k + 127) / 128, 128, static_cast<cudaStream_t>(stream), status, norms, lmin, deflated, ctx->status_dev,
+               host_out, k);
+  return 0;
 }
 
 int toner_inv_roots(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
@@ -1158,12 +1250,12 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
                          "(both are verified together after the chain)");
   // > 0: certified bound, checked against damping / norm per statistic; < 0: estimate, verified after the chain
   const float lower_used = l0 > l_worst ? (estimated ? -(float)l0 : (float)l0) : 0.f;
-  if (iters <= 0) iters = default_iterations(l0, p);
+  const Schedule plan = schedule_for(l0, p, iters);
+  iters = plan.iters;
   if (iters < 2) return fail(kErrArg, "inv_roots: at least two iterations are required");
-  const std::vector<NewtonStep> sched = newton_schedule(l0, p, iters, nullptr);
-  double l_last;  // lower bound of the spectrum of the last M, i.e. after iters - 1 updates
-  newton_schedule(l0, p, iters - 1, &l_last);
-  const FinishPoly fin = finish_poly_or_best(p, 1.0 - l_last);
+  const std::vector<NewtonStep>& sched = plan.steps;
+  const double l_last = plan.l_last;
+  const FinishPoly& fin = plan.fin;
   const int order = fin.order;
   int log2p = 0;
   while ((1 << log2p) < p) ++log2p;

@@ -83,15 +83,34 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream);
 // Scratch (split_ws) with which launch_gemm would divide the accumulation of this product among several units; 0: none.
 size_t gemm_split_bytes(const toner_gemm_desc& d);
 
-// FP16 hi/lo split of an FP32 stack (see toner_split16).
+// FP16 hi/lo split of an FP32 stack (see toner_split16).  inv_mul: per-matrix factors of the inverse scales; hi_only: the lo
+// planes are not written; scratch_zeroed: the maximum accumulators in `scratch` are zero already.
 int split16(const float* x, const float* const* x_list, int batch, int rows, int cols, long long ld, long long bs,
             float aff_a, float aff_b, const uint32_t* maxabs, void* scratch, void* planes, float* inv_scale,
-            cudaStream_t stream);
+            cudaStream_t stream, const float* inv_mul = nullptr, bool hi_only = false, bool scratch_zeroed = false);
 
 // out[b] = sum of squares of matrix b, bitwise reproducible.  scratch: sumsq_scratch_bytes(batch).
 size_t sumsq_scratch_bytes(int batch);
+// (out == nullptr: only the kSumsqBlocks partial sums of each matrix are left in scratch)
+constexpr int kSumsqBlocks = 296;  // two per SM on a 148-SM part; fixed so that results do not depend on the device
 int sumsq_det(const float* x, int batch, int rows, int cols, long long ld, long long bs, float* scratch, float* out,
               cudaStream_t stream);
+
+// Sum of a matrix's partial sums, added one after the other in their order; called by one warp, every lane gets the total.
+// (The lanes fetch them together: the additions then run at register speed, not one load apart.)
+__device__ __forceinline__ float sumsq_total(const float* __restrict__ partial, int lane) {
+  constexpr int kRows = (kSumsqBlocks + 31) / 32;
+  float p[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) p[i] = (i * 32 + lane < kSumsqBlocks) ? partial[i * 32 + lane] : 0.f;
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+#pragma unroll 8
+    for (int l = 0; l < 32; ++l) t += __shfl_sync(0xffffffffu, p[i], l);
+  }
+  return t;
+}
 
 // Block-wide max of non-negative values into one FP32-bits accumulator: one atomic per block, and none when the
 // accumulator already holds as much (thousands of blocks share a few addresses; per-warp atomics serialise in L2).

@@ -129,12 +129,13 @@ __device__ __forceinline__ float split_scale(unsigned int maxabs_bits) {
 __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ x, const float* const* __restrict__ x_list,
                                                       int batch, int rows, int cols, long long ld, long long bs,
                                                       float aff_a, float aff_b, const unsigned int* __restrict__ maxabs,
+                                                      const float* __restrict__ inv_mul, int hi_only,
                                                       __half* __restrict__ planes, float* __restrict__ inv_scale) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
   const float* X = x_list ? x_list[b] : x + (long long)b * bs;
   const float s = split_scale(maxabs[b]);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && inv_scale) inv_scale[b] = 1.f / s;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && inv_scale) inv_scale[b] = inv_mul ? inv_mul[b] / s : 1.f / s;
   const long long per = (long long)rows * cols;
   __half* hi = planes + (long long)b * per;
   __half* lo = planes + ((long long)batch + b) * per;
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ 
         l[e] = __float2half_rn(w - __half2float(h[e]));
       }
       *reinterpret_cast<uint2*>(hi + (long long)r * cols + c) = *reinterpret_cast<uint2*>(h);
-      *reinterpret_cast<uint2*>(lo + (long long)r * cols + c) = *reinterpret_cast<uint2*>(l);
+      if (!hi_only) *reinterpret_cast<uint2*>(lo + (long long)r * cols + c) = *reinterpret_cast<uint2*>(l);
     };
     auto load4 = [&](long long i) {
       const int r = (int)(i / c4), c = (int)(i - (long long)r * c4) * 4;
@@ -173,14 +174,13 @@ __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ 
       const float w = (aff_b * X[(long long)r * ld + c] + (c == r ? aff_a : 0.f)) * s;
       const __half h = __float2half_rn(w);
       hi[i] = h;
-      lo[i] = __float2half_rn(w - __half2float(h));
+      if (!hi_only) lo[i] = __float2half_rn(w - __half2float(h));
     }
   }
 }
 
 // ------------------------------------------------------------------ deterministic sum of squares
 // Fixed grid, fixed reduction tree: the same input always gives the same bits (float atomics would not).
-constexpr int kSumsqBlocks = 296;  // two per SM on a 148-SM part; fixed so that results do not depend on the device
 
 __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restrict__ x, int rows, int cols, long long ld,
                                                             long long bs, float* __restrict__ partial) {
@@ -233,13 +233,10 @@ __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restr
   }
 }
 
-__global__ void sumsq_final_kernel(const float* __restrict__ partial, int blocks, int batch, float* __restrict__ out) {
+__global__ void __launch_bounds__(32) sumsq_final_kernel(const float* __restrict__ partial, float* __restrict__ out) {
   ptx::pdl_begin();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= batch) return;
-  float t = 0.f;
-  for (int i = 0; i < blocks; ++i) t += partial[(long long)b * blocks + i];
-  out[b] = t;
+  const float t = sumsq_total(partial + (long long)blockIdx.x * kSumsqBlocks, threadIdx.x);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 size_t sumsq_scratch_bytes(int batch) { return (size_t)batch * kSumsqBlocks * sizeof(float); }
@@ -247,9 +244,50 @@ size_t sumsq_scratch_bytes(int batch) { return (size_t)batch * kSumsqBlocks * si
 int sumsq_det(const float* x, int batch, int rows, int cols, long long ld, long long bs, float* scratch, float* out,
               cudaStream_t stream) {
   TONER_LAUNCH(sumsq_partial_kernel, dim3(kSumsqBlocks, batch), 256, stream, x, rows, cols, ld, bs, scratch);
-  TONER_LAUNCH(sumsq_final_kernel, (batch + 127) / 128, 128, stream, scratch, kSumsqBlocks, batch, out);
+  if (out) TONER_LAUNCH(sumsq_final_kernel, batch, 32, stream, scratch, out);
   TONER_CUDA(cudaGetLastError());
   return 0;
+}
+
+// ------------------------------------------------------------------ lists of separately allocated matrices
+// Pointers travel with the launch (no table in memory, no copy): up to kListMax matrices a kernel.
+constexpr int kListMax = 128;
+struct PointerList {
+  const float* src[kListMax];
+  float* dst[kListMax];
+};
+
+// *flag (host memory the device can address) <- 1 if any element of any matrix is NaN or Inf
+__global__ void __launch_bounds__(256) list_finite_kernel(const __grid_constant__ PointerList list, long long n4, int* flag) {
+  ptx::pdl_begin();
+  const float4* X = reinterpret_cast<const float4*>(list.src[blockIdx.y]);
+  bool bad = false;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  auto look = [&bad](const float4 v) { bad = bad || !(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w)); };
+  for (; i + 3 * step < n4; i += 4 * step) {   // four independent 16-byte loads in flight
+    const float4 a = X[i], b = X[i + step], c = X[i + 2 * step], d = X[i + 3 * step];
+    look(a); look(b); look(c); look(d);
+  }
+  for (; i < n4; i += step) look(X[i]);
+  if (__syncthreads_or(bad) && threadIdx.x == 0) *reinterpret_cast<volatile int*>(flag) = 1;
+}
+
+// dst <- beta dst + gamma src (beta == 0: dst is not read); dst may be src
+__global__ void __launch_bounds__(256) list_axpby_kernel(const __grid_constant__ PointerList list, long long n4, float beta,
+                                                         float gamma) {
+  ptx::pdl_begin();
+  const float4* X = reinterpret_cast<const float4*>(list.src[blockIdx.y]);
+  float4* D = reinterpret_cast<float4*>(list.dst[blockIdx.y]);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const float4 x = X[i];
+    float4 d = make_float4(gamma * x.x, gamma * x.y, gamma * x.z, gamma * x.w);
+    if (beta != 0.f) {
+      const float4 o = D[i];
+      d.x = fmaf(beta, o.x, d.x); d.y = fmaf(beta, o.y, d.y); d.z = fmaf(beta, o.z, d.z); d.w = fmaf(beta, o.w, d.w);
+    }
+    D[i] = d;
+  }
 }
 
 // ------------------------------------------------------------------ sum of squares without caller scratch
@@ -290,7 +328,7 @@ static int blocks_for(long long work, int per_block, int cap) {
 
 int split16(const float* x, const float* const* x_list, int batch, int rows, int cols, long long ld, long long bs,
             float aff_a, float aff_b, const uint32_t* maxabs, void* scratch, void* planes, float* inv_scale,
-            cudaStream_t stream) {
+            cudaStream_t stream, const float* inv_mul, bool hi_only, bool scratch_zeroed) {
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   if ((!x && !x_list) || !planes || batch <= 0 || rows <= 0 || cols <= 0) return fail(kErrArg, "split16: bad arguments");
@@ -300,12 +338,13 @@ int split16(const float* x, const float* const* x_list, int batch, int rows, int
   if (!maxabs) {
     if (!scratch) return fail(kErrArg, "split16: maxabs or scratch is required");
     unsigned int* m = static_cast<unsigned int*>(scratch);
-    TONER_CUDA(cudaMemsetAsync(m, 0, sizeof(unsigned int) * batch, stream));
+    if (!scratch_zeroed) TONER_CUDA(cudaMemsetAsync(m, 0, sizeof(unsigned int) * batch, stream));
     TONER_LAUNCH(maxabs_kernel, dim3(bx, batch), 256, stream, x, x_list, rows, cols, ld, bs, aff_a, aff_b, m);
     TONER_CUDA(cudaGetLastError());
     maxabs = m;
   }
-  TONER_LAUNCH(split16_kernel, dim3(bx, batch), 256, stream, x, x_list, batch, rows, cols, ld, bs, aff_a, aff_b, maxabs, static_cast<__half*>(planes), inv_scale);
+  TONER_LAUNCH(split16_kernel, dim3(bx, batch), 256, stream, x, x_list, batch, rows, cols, ld, bs, aff_a, aff_b, maxabs, inv_mul,
+               hi_only ? 1 : 0, static_cast<__half*>(planes), inv_scale);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -428,6 +467,39 @@ int toner_unpack_ema(const float* packed, float* ema, int32_t k, int32_t n, floa
   TONER_LAUNCH(unpack_ema_kernel, dim3(t * (t + 1) / 2, 1, k), 256, static_cast<cudaStream_t>(stream), packed, ema, n, t, beta, gamma);
   TONER_CUDA(cudaGetLastError());
   return 0;
+}
+
+static int list_call(const float* const* src, float* const* dst, int32_t count, int64_t numel, float beta, float gamma, int32_t* flag,
+                     void* stream_) {
+  using namespace toner;
+  Context* ctx = context();
+  if (!ctx) return kErrCuda;
+  if (!src || count <= 0 || numel <= 0 || numel % 4) return fail(kErrArg, "matrix list: the size must be a positive multiple of 4");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  for (int first = 0; first < count; first += kListMax) {
+    PointerList list;
+    const int here = count - first < kListMax ? count - first : kListMax;
+    for (int i = 0; i < here; ++i) {
+      list.src[i] = src[first + i];
+      list.dst[i] = dst ? dst[first + i] : nullptr;
+      if (!list.src[i] || (reinterpret_cast<uintptr_t>(list.src[i]) & 15u) || (reinterpret_cast<uintptr_t>(list.dst[i]) & 15u))
+        return fail(kErrArg, "matrix list: pointers must be set and 16-byte aligned");
+    }
+    const int bx = blocks_for(numel / 4, 256 * 4, 8 * ctx->num_sms / (here < 8 ? here : 8) + 1);
+    if (dst) TONER_LAUNCH(list_axpby_kernel, dim3(bx, here), 256, stream, list, numel / 4, beta, gamma);
+    else TONER_LAUNCH(list_finite_kernel, dim3(bx, here), 256, stream, list, numel / 4, flag);
+  }
+  return 0;
+}
+
+int toner_list_finite(const float* const* ptrs, int32_t count, int64_t numel, int32_t* host_flag, void* stream) {
+  if (!host_flag) return toner::fail(toner::kErrArg, "list_finite: null flag");
+  return list_call(ptrs, nullptr, count, numel, 0.f, 0.f, host_flag, stream);
+}
+
+int toner_list_axpby(const float* const* src, float* const* dst, int32_t count, int64_t numel, float beta, float gamma, void* stream) {
+  if (!dst) return toner::fail(toner::kErrArg, "list_axpby: null destination list");
+  return list_call(src, dst, count, numel, beta, gamma, nullptr, stream);
 }
 
 int toner_split16(const float* x, const float* const* x_list, int32_t batch, int32_t rows, int32_t cols, int64_t ld,

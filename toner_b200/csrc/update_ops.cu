@@ -14,13 +14,20 @@ static int ew_grid(long long elems4, int num_sms) {
 }
 
 // ------------------------------------------------------------------ Newton-Schulz helpers
-// x = u / (sqrt(sumsq[b]) + eps), written as FP32 and as BF16 (the operand the products read)
-__global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__ u, const float* __restrict__ sumsq,
+// x = u / (||u|| + eps), written as FP32 and as BF16 (the operand the products read); ||u||^2 as the partial sums that
+// sumsq_det left (each block adds them up itself: 1.2 KB from L2, against a launch of its own)
+__global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__ u, const float* __restrict__ partial,
                                                        float eps, long long per, float* __restrict__ x,
                                                        __nv_bfloat16* __restrict__ xb) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
-  const float f = 1.f / (sqrtf(sumsq[b]) + eps);
+  __shared__ float norm;
+  if (threadIdx.x < 32) {
+    const float t = sumsq_total(partial + (long long)b * kSumsqBlocks, threadIdx.x);
+    if (threadIdx.x == 0) norm = sqrtf(t);
+  }
+  __syncthreads();
+  const float f = 1.f / (norm + eps);
   const float4* U = reinterpret_cast<const float4*>(u + (long long)b * per);
   float4* X = reinterpret_cast<float4*>(x + (long long)b * per);
   uint2* XB = reinterpret_cast<uint2*>(xb + (long long)b * per);
@@ -73,37 +80,48 @@ __global__ void __launch_bounds__(256) muont_momentum_kernel(const float* const*
 }
 
 // c1[b] = lr wd n / ||R||_F^2 ,  c2[b] = lr scale sqrt(n) / ||R||_F   with ||R||_F^2 = fro2[first + b*step]
+// (and zero[2 * count] <- 0: the maximum accumulators of the passes that follow)
 __global__ void muont_coeff_kernel(const float* __restrict__ fro2, int first, int step, int count, int n, float lr, float wd,
-                                   float scale, float* __restrict__ c1, float* __restrict__ c2) {
+                                   float scale, float* __restrict__ c1, float* __restrict__ c2, unsigned int* __restrict__ zero) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= count) return;
+  if (zero) zero[b] = zero[count + b] = 0u;
   const float f2 = fro2[first + b * step];
   c1[b] = lr * wd * (float)n / fmaxf(f2, 1e-60f);
   c2[b] = lr * scale * sqrtf((float)n) / fmaxf(sqrtf(f2), 1e-30f);
 }
 
-__global__ void mul_vec_kernel2(float* a, const float* b, int k) {
+__global__ void mul_vec_kernel(float* a, const float* b, int k) {
   ptx::pdl_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < k) a[i] *= b[i];
 }
 
 // ------------------------------------------------------------------ AdamT elementwise
-// m <- b1 m + (1-b1) g
+// m <- b1 m + (1-b1) g ;  g_max[b] = max |g|, m_max[b] = max |m| (both or neither)
 __global__ void __launch_bounds__(256) adamt_m_kernel(const float* const* __restrict__ grads, float* __restrict__ m,
-                                                      long long per, float b1) {
+                                                      long long per, float b1, unsigned int* __restrict__ g_max,
+                                                      unsigned int* __restrict__ m_max) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
   const float4* G = reinterpret_cast<const float4*>(grads[b]);
   float4* M = reinterpret_cast<float4*>(m + (long long)b * per);
   const long long n4 = per / 4;
   const float w = 1.f - b1;
+  float gx = 0.f, mx = 0.f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     const float4 g = G[i];
     float4 mm = M[i];
     mm.x = mm.x * b1 + g.x * w; mm.y = mm.y * b1 + g.y * w; mm.z = mm.z * b1 + g.z * w; mm.w = mm.w * b1 + g.w * w;
     M[i] = mm;
+    gx = fmaxf(fmaxf(fmaxf(gx, fabsf(g.x)), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w)));
+    mx = fmaxf(fmaxf(fmaxf(mx, fabsf(mm.x)), fabsf(mm.y)), fmaxf(fabsf(mm.z), fabsf(mm.w)));
+  }
+  if (g_max) {
+    block_atomic_max(gx, g_max + b);
+    __syncthreads();
+    block_atomic_max(mx, m_max + b);
   }
 }
 
@@ -137,10 +155,11 @@ __global__ void __launch_bounds__(256) adamt_ratio_kernel(const float* __restric
 // c1[b] = lr wd n / ||R||_F^2 ;  c2[b] = -lr ||U||_F / max(||U R||_F, 1e-30)
 __global__ void adamt_coeff_kernel(const float* __restrict__ fro2, int first, int step, int count, int n, float lr, float wd,
                                    const float* __restrict__ ss_before, const float* __restrict__ ss_after,
-                                   float* __restrict__ c1, float* __restrict__ c2) {
+                                   float* __restrict__ c1, float* __restrict__ c2, unsigned int* __restrict__ zero) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= count) return;
+  if (zero) zero[b] = zero[count + b] = 0u;
   c1[b] = lr * wd * (float)n / fmaxf(fro2[first + b * step], 1e-60f);
   c2[b] = -lr * sqrtf(ss_before[b]) / fmaxf(sqrtf(ss_after[b]), 1e-30f);
 }
@@ -240,7 +259,7 @@ size_t toner_ns_polar_workspace_bytes(int32_t batch, int32_t m, int32_t n) {
   if (batch <= 0 || m <= 0 || n <= 0) return 0;
   const size_t a = (size_t)(m < n ? m : n);
   const size_t mn = (size_t)m * n;
-  return align_up(sumsq_scratch_bytes(batch), 256) + align_up((size_t)batch * 4, 256) +
+  return align_up(sumsq_scratch_bytes(batch), 256) +
          2 * align_up(mn * 2 * batch, 256) +                 // two BF16 copies of X (read one, write the other)
          align_up(a * a * 4 * batch, 256) +                  // Gram, FP32
          2 * align_up(a * a * 2 * batch, 256);               // Gram and polynomial, BF16
@@ -260,7 +279,6 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
   const long long mn = (long long)m * n, aa = (long long)a * a;
   char* w = static_cast<char*>(workspace);
   float* partial = reinterpret_cast<float*>(w); w += align_up(sumsq_scratch_bytes(batch), 256);
-  float* ss = reinterpret_cast<float*>(w); w += align_up((size_t)batch * 4, 256);
   __nv_bfloat16* xb[2];
   xb[0] = reinterpret_cast<__nv_bfloat16*>(w); w += align_up((size_t)mn * 2 * batch, 256);
   xb[1] = reinterpret_cast<__nv_bfloat16*>(w); w += align_up((size_t)mn * 2 * batch, 256);
@@ -268,9 +286,9 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
   __nv_bfloat16* gram_b = reinterpret_cast<__nv_bfloat16*>(w); w += align_up((size_t)aa * 2 * batch, 256);
   __nv_bfloat16* poly_b = reinterpret_cast<__nv_bfloat16*>(w);
 
-  int rc = sumsq_det(u, batch, m, n, n, mn, partial, ss, stream);
+  int rc = sumsq_det(u, batch, m, n, n, mn, partial, nullptr, stream);
   if (rc) return rc;
-  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid(mn / 4, ctx->num_sms), batch), 256, stream, u, ss, eps, mn, x_out, xb[0]);
+  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid(mn / 4, ctx->num_sms), batch), 256, stream, u, partial, eps, mn, x_out, xb[0]);
   TONER_CUDA(cudaGetLastError());
 
   const float ca = 3.4445f, cb = -4.7750f, cc = 2.0315f;  // src/toner/linalg.py:9
@@ -366,7 +384,7 @@ int toner_muont_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
                        float scale, float* c1, float* c2, void* stream) {
   if (!context()) return kErrCuda;
   if (!fro2 || !c1 || !c2 || count <= 0) return fail(kErrArg, "muont_coeffs: bad arguments");
-  TONER_LAUNCH(muont_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, scale, c1, c2);
+  TONER_LAUNCH(muont_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, scale, c1, c2, nullptr);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -374,7 +392,7 @@ int toner_muont_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
 int toner_scale_vec(float* a, const float* b, int32_t count, void* stream) {
   if (!context()) return kErrCuda;
   if (!a || !b || count <= 0) return fail(kErrArg, "scale_vec: bad arguments");
-  TONER_LAUNCH(mul_vec_kernel2, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), a, b, count);
+  TONER_LAUNCH(mul_vec_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), a, b, count);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -384,7 +402,7 @@ int toner_adamt_first_moment(const float* const* grad_ptrs, float* m, int32_t co
   if (!ctx) return kErrCuda;
   if (!grad_ptrs || !m || count <= 0) return fail(kErrArg, "adamt_first_moment: bad arguments");
   if (int rc = check_stack("adamt_first_moment", per)) return rc;
-  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), grad_ptrs, m, per, beta1);
+  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), grad_ptrs, m, per, beta1, nullptr, nullptr);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -406,7 +424,7 @@ int toner_adamt_coeffs(const float* fro2, int32_t first, int32_t step, int32_t c
                        const float* ss_before, const float* ss_after, float* c1, float* c2, void* stream) {
   if (!context()) return kErrCuda;
   if (!fro2 || !ss_before || !ss_after || !c1 || !c2 || count <= 0) return fail(kErrArg, "adamt_coeffs: bad arguments");
-  TONER_LAUNCH(adamt_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, ss_before, ss_after, c1, c2);
+  TONER_LAUNCH(adamt_coeff_kernel, (count + 127) / 128, 128, static_cast<cudaStream_t>(stream), fro2, first, step, count, n, lr, wd, ss_before, ss_after, c1, c2, nullptr);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -430,6 +448,124 @@ int toner_apply_scaled(float* const* weight_ptrs, const float* delta, int32_t co
   TONER_LAUNCH(apply_scaled_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream),  weight_ptrs, delta, per, weight_scale, delta_scale);
   TONER_CUDA(cudaGetLastError());
   return 0;
+}
+
+// ------------------------------------------------------------------ whole stages of an update
+// d[b] = alpha * A[b] R[first + b step]: FP32-accurate from hi/lo planes, or (coarse) the hi planes only
+static int right_product(const toner_matrix_group& g, bool outer, float* d, bool coarse, float alpha, const float* c,
+                         const float* beta_v, uint32_t* maxabs, cudaStream_t stream) {
+  const void* planes = outer ? g.outer_planes : g.inner_planes;
+  const float* inv = outer ? g.outer_inv : g.inner_inv;
+  toner_gemm_desc q = {};
+  q.a.base = g.planes;
+  q.a.rows = g.rows; q.a.cols = g.cols; q.a.ld = g.cols; q.a.z_stride = (int64_t)g.rows * g.cols; q.a.nz = 2 * g.count; q.a.z_step = 1;
+  q.b.base = planes;
+  q.b.rows = g.cols; q.b.cols = g.cols; q.b.ld = g.cols; q.b.z_stride = (int64_t)g.cols * g.cols; q.b.nz = 2 * g.factors;
+  q.b.z_step = g.step;
+  q.a.seg_z[2] = g.count;                         // Ah Ah Al
+  q.b.seg_z[0] = q.b.seg_z[2] = g.first;          // Rh Rl Rh
+  q.b.seg_z[1] = g.factors + g.first;
+  q.m = g.rows; q.n = g.cols; q.k = g.cols; q.batch = g.count;
+  q.segs = coarse ? 1 : 3;
+  q.fmt = 0;
+  q.alpha = alpha;
+  q.alpha_a = g.inv;
+  q.alpha_b = inv + g.first; q.alpha_b_step = g.step;
+  q.d = d; q.ldd = g.cols; q.d_bs = (int64_t)g.rows * g.cols;
+  if (c) {
+    q.c = c; q.ldc = g.cols; q.c_bs = (int64_t)g.rows * g.cols;
+    q.beta = 1.f;
+    q.beta_v = beta_v;
+  }
+  q.maxabs = maxabs;
+  return launch_gemm(q, stream);
+}
+
+static int check_group(const char* what, const toner_matrix_group* g) {
+  if (!context()) return kErrCuda;
+  if (!g || g->count <= 0 || g->rows <= 0 || g->cols <= 0 || g->factors <= 0 || !g->m || !g->work || !g->planes || !g->inv ||
+      !g->maxabs || !g->c1 || !g->c2)
+    return fail(kErrArg, std::string(what) + ": bad matrix group");
+  if (g->rows % 8 || g->cols % 8) return fail(kErrUnsupported, std::string(what) + ": matrix dimensions must be multiples of 8");
+  return 0;
+}
+
+static int split_stack(const toner_matrix_group& g, const float* x, const float* const* list, const uint32_t* maxabs, uint32_t* scratch,
+                       const float* inv_mul, bool hi_only, bool zeroed, cudaStream_t stream) {
+  return split16(x, list, g.count, g.rows, g.cols, g.cols, (long long)g.rows * g.cols, 0.f, 1.f, maxabs, scratch, g.planes, g.inv,
+                 stream, inv_mul, hi_only, zeroed);
+}
+
+int toner_muont_input(const toner_matrix_group* g, float mu, int32_t nesterov, void* stream_) {
+  if (int rc = check_group("muont_input", g)) return rc;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  int rc = toner_muont_momentum(g->grads, g->m, g->work, g->count, (int64_t)g->rows * g->cols, mu, nesterov, g->maxabs, stream);
+  if (rc || !g->inner_planes) return rc;
+  rc = split_stack(*g, g->work, nullptr, g->maxabs, nullptr, nullptr, false, false, stream);
+  if (rc) return rc;
+  return right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);
+}
+
+int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs, float lr, float weight_decay, float scale,
+                      float* delta, void* stream_) {
+  if (int rc = check_group("muont_delta", g)) return rc;
+  if (!delta || !g->outer_planes || !g->outer_fro2) return fail(kErrArg, "muont_delta: null pointer");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  uint32_t* const w_max = g->maxabs + g->count;       // cleared by the coefficient kernel, with the next
+  uint32_t* const v_max = g->maxabs + 2 * g->count;
+  TONER_LAUNCH(muont_coeff_kernel, (g->count + 127) / 128, 128, stream, g->outer_fro2, g->first, g->step, g->count, g->cols, lr,
+               weight_decay, scale, g->c1, g->c2, w_max);
+  int rc = 0;
+  if (weight_decay != 0.f) {
+    // V = c1 W R + c2 P.  The decay term is lr wd ||W|| against lr ||P||, about 1 % of V: the hi planes suffice, and only they
+    // are written
+    rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->weights), nullptr, w_max, g->c1, true, true, stream);
+    if (!rc) rc = right_product(*g, true, g->work, true, 1.f, g->work, g->c2, v_max, stream);
+    if (!rc) rc = split_stack(*g, g->work, nullptr, v_max, nullptr, nullptr, false, false, stream);
+  } else {   // V = c2 P
+    rc = split_stack(*g, g->work, nullptr, polar_maxabs, w_max, g->c2, false, true, stream);
+  }
+  if (rc) return rc;
+  return right_product(*g, true, delta, false, -1.f, nullptr, nullptr, nullptr, stream);
+}
+
+int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay, float beta1, float beta2, float bc1, float bc2,
+                      float eps, float* delta, void* stream_) {
+  if (int rc = check_group("adamt_delta", g)) return rc;
+  if (!delta || !g->v || !g->work2 || !g->ss || !g->ss_scratch || !g->inner_planes || !g->outer_fro2)
+    return fail(kErrArg, "adamt_delta: null pointer");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  Context* ctx = context();
+  const long long per = (long long)g->rows * g->cols;
+  float* const ss0 = g->ss;
+  float* const ss1 = g->ss + g->count;
+  uint32_t* const max0 = g->maxabs;
+  uint32_t* const max1 = g->maxabs + g->count;
+  uint32_t* const max2 = g->maxabs + 2 * g->count;
+  TONER_CUDA(cudaMemsetAsync(max0, 0, sizeof(uint32_t) * 3 * g->count, stream));
+  // one pass over the gradient: m <- b1 m + (1 - b1) g, max |g|, max |m|
+  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->grads, g->m, per, beta1, max0, max1);
+  int rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->grads), max0, nullptr, nullptr, false, false, stream);
+  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // t = g R
+  if (!rc) rc = split_stack(*g, g->m, nullptr, max1, nullptr, nullptr, false, false, stream);
+  if (!rc) rc = right_product(*g, false, g->work2, false, 1.f / bc1, nullptr, nullptr, nullptr, stream);         // (m / bc1) R
+  if (rc) return rc;
+  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->work, g->v, g->work2, per, beta2, bc2,
+               eps, max2);                                                                                       // U, in work2
+  rc = sumsq_det(g->work2, g->count, g->rows, g->cols, g->cols, per, g->ss_scratch, ss0, stream);
+  if (!rc) rc = split_stack(*g, g->work2, nullptr, max2, nullptr, nullptr, false, false, stream);
+  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // U R
+  if (!rc) rc = sumsq_det(g->work, g->count, g->rows, g->cols, g->cols, per, g->ss_scratch, ss1, stream);
+  if (rc) return rc;
+  TONER_LAUNCH(adamt_coeff_kernel, (g->count + 127) / 128, 128, stream, g->outer_fro2, g->first, g->step, g->count, g->cols, lr,
+               weight_decay, ss0, ss1, g->c1, g->c2, max0);
+  if (weight_decay == 0.f)                                                                                       // c2 U R
+    return toner_scale_stack(g->work, g->c2, delta, g->count, per, stream);
+  rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->weights), nullptr, max0, g->c1, true, true, stream);
+  if (!rc) rc = right_product(*g, true, g->work2, true, 1.f, nullptr, nullptr, max1, stream);                    // c1 W R
+  if (!rc) rc = split_stack(*g, g->work2, nullptr, max1, nullptr, nullptr, false, false, stream);
+  if (rc) return rc;
+  return right_product(*g, true, delta, false, -1.f, g->work, g->c2, nullptr, stream);
 }
 
 }  // extern "C"

@@ -58,6 +58,11 @@ def _check_matrix(p: Tensor) -> None:
         raise ValueError("toner_b200 needs matrix dimensions that are multiples of 8")
 
 
+def _plain(t: Tensor) -> bool:
+    """What the list kernels take: contiguous, aligned FP32 (a CUDA tensor of a multiple of four elements)."""
+    return t.dtype == torch.float32 and t.is_contiguous() and t.numel() % 4 == 0 and t.data_ptr() % 16 == 0
+
+
 class _Bucket:
     """Equally shaped parameters of one parameter group: one FactorSet entry and one stack row each."""
 
@@ -92,6 +97,7 @@ class _TonerGeneral(Optimizer):
         self._scratch = core.Scratch()
         self._buckets: Optional[Dict[Tuple, _Bucket]] = None
         self._bucket_of: Dict[Tensor, Tuple[_Bucket, int]] = {}
+        self._finite_flag: Optional[Tensor] = None  # pinned word the finiteness check of the statistics reports to
         self._health: Optional[ops.Health] = None   # the update kernels of the last step (created with the buckets)
 
     # ------------------------------------------------------------------ validation
@@ -169,7 +175,7 @@ class _TonerGeneral(Optimizer):
         error (src/toner/reference.py:51-81)."""
         self._ensure_built()
         owner = {p: g for g in self.param_groups for p in g["params"]}
-        finite = {}
+        distinct: Dict[int, Tensor] = {}
         for p, cov in second_moments.items():   # nothing is touched until every entry has passed
             if p not in owner:
                 raise ValueError("Received a statistic for a parameter not owned by this optimizer")
@@ -181,20 +187,44 @@ class _TonerGeneral(Optimizer):
                 raise ValueError("Input statistics must be finite floating-point matrices")
             if self.state[p].get("statistics_ready", False):
                 raise RuntimeError("Statistics already updated; aggregate microbatches before update_statistics()")
-            finite.setdefault(cov.data_ptr(), torch.isfinite(cov).all())     # one flag per distinct statistic
-        if finite and not bool(torch.stack(list(finite.values())).all()):    # one wait for all of them
+            distinct.setdefault(cov.data_ptr(), cov)
+        if distinct and not self._all_finite(distinct.values()):
             raise ValueError("Input statistics must be finite floating-point matrices")
+        updates: Dict[Tuple, Tuple[List[Tensor], List[Tensor]]] = {}
         for p, cov in second_moments.items():
             bucket, i = self._bucket_of[p]
             state, beta = self.state[p], owner[p]["statistic_momentum"]
-            if "input_ema" not in state:
-                bucket.factors.ema[i].zero_()
+            fresh = "input_ema" not in state
+            if fresh:
                 state["input_ema"] = bucket.factors.ema[i]
                 state["input_weight"] = 0.0
-            c = cov.to(torch.float32).contiguous()
-            ops.axpby(state["input_ema"], c, state["input_ema"], beta, 1 - beta)
+            src, dst = updates.setdefault((bucket.factors.n, 0.0 if fresh else beta, 1 - beta), ([], []))
+            src.append(cov if _plain(cov) else cov.to(torch.float32).contiguous())
+            dst.append(state["input_ema"])
             state["input_weight"] = beta * state["input_weight"] + (1 - beta)
             state["statistics_ready"] = True
+        for (_, keep, gain), (src, dst) in updates.items():    # one launch for all matrices of a width
+            ops.list_axpby(src, dst, keep, gain)
+
+    def _all_finite(self, matrices) -> bool:
+        """Whether every element of every matrix is finite: one launch per size and one wait."""
+        groups: Dict[int, List[Tensor]] = {}
+        ok = []
+        for cov in matrices:
+            if _plain(cov):
+                groups.setdefault(cov.numel(), []).append(cov)
+            else:
+                ok.append(torch.isfinite(cov).all())
+        if groups:
+            if self._finite_flag is None:
+                self._finite_flag = torch.zeros(1, dtype=torch.int32).pin_memory()
+            self._finite_flag[0] = 0
+            for same in groups.values():
+                ops.list_finite(same, self._finite_flag)
+            torch.cuda.current_stream().synchronize()
+            if int(self._finite_flag[0]):
+                return False
+        return not ok or bool(torch.stack(ok).all())
 
     def _check_step(self) -> None:
         self._validate_common()

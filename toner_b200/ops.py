@@ -87,9 +87,14 @@ class Health:
         code = int(self._host[0])
         if code:
             self._host.zero_()
-            device_status()   # clears the word on the device
-            raise _lib.TonerError(f"a CUDA kernel gave up a bounded wait (status {code}) during {self._what}: "
-                                  "its results are incomplete and were not applied")
+            raise_gave_up(code, self._what)
+
+
+def raise_gave_up(code: int, what: str) -> None:
+    """A kernel reported that a bounded wait ran out: clear the word on the device and raise."""
+    device_status()
+    raise _lib.TonerError(f"a CUDA kernel gave up a bounded wait (status {code}) during {what}: "
+                          "its results are incomplete and were not applied")
 
 
 def gemm_phase_cycles(enable: bool):
@@ -379,6 +384,13 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     return root_lo, root_hi, fro2_lo, status
 
 
+def factor_report(status: torch.Tensor, norms: torch.Tensor, lmin: torch.Tensor, deflated: torch.Tensor,
+                  host: torch.Tensor) -> None:
+    """Status, norms, lmin, deflated and the kernels' status word into pinned host memory (4 k + 1 words) in one launch."""
+    check(_lib.load().toner_factor_report(status.data_ptr(), norms.data_ptr(), lmin.data_ptr(), deflated.data_ptr(),
+                                          status.numel(), host.data_ptr(), _stream()), "toner_factor_report")
+
+
 def ns_polar_workspace_bytes(batch: int, m: int, n: int) -> int:
     return _lib.load().toner_ns_polar_workspace_bytes(batch, m, n)
 
@@ -498,6 +510,22 @@ def scale_stack(x: torch.Tensor, coeff: torch.Tensor, out: torch.Tensor) -> None
     """out[b] = coeff[b] * x[b] for (count, ...) FP32 stacks (toner_scale_stack)."""
     check(_lib.load().toner_scale_stack(x.data_ptr(), coeff.data_ptr(), out.data_ptr(), x.shape[0], x[0].numel(),
                                         _stream()), "toner_scale_stack")
+
+
+def _pointers(tensors: Sequence[torch.Tensor]):
+    return (C.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
+def list_finite(tensors: Sequence[torch.Tensor], flag: torch.Tensor) -> None:
+    """flag (pinned int32) <- 1 if an element of these equally sized, contiguous FP32 CUDA tensors is NaN or Inf."""
+    check(_lib.load().toner_list_finite(_pointers(tensors), len(tensors), tensors[0].numel(), flag.data_ptr(), _stream()),
+          "toner_list_finite")
+
+
+def list_axpby(src: Sequence[torch.Tensor], dst: Sequence[torch.Tensor], beta: float, gamma: float) -> None:
+    """dst[i] <- beta*dst[i] + gamma*src[i] over equally sized, contiguous FP32 CUDA tensors (toner_list_axpby)."""
+    check(_lib.load().toner_list_axpby(_pointers(src), _pointers(dst), len(src), src[0].numel(), beta, gamma, _stream()),
+          "toner_list_axpby")
 
 
 def axpby(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor, a: float, b: float) -> None:
