@@ -122,6 +122,9 @@ typedef struct toner_gemm_desc {
   void* split_ws;           /* optional scratch: a product with few tiles and a long accumulation may then divide each tile's
                                accumulation among several CTAs and add the parts (in a fixed order) there */
   int64_t split_ws_bytes;
+  int32_t interleave;       /* 1: a split product (segs = 3: Ah Bh, Ah Bl, Al Bh, one chain) may take its three plane products
+                               k-block by k-block, which saves a third of the operand traffic; the additions into the
+                               accumulator then come in that order instead of plane by plane */
 } toner_gemm_desc;
 
 int toner_gemm(const toner_gemm_desc* desc, void* stream);

@@ -75,6 +75,8 @@ static int chain_length(double lower) {
   return 0;
 }
 
+constexpr double kInterleaveLower = 5e-3;   // chain_length()'s first threshold
+
 // Products applied to X (and the final squarings) pass their error on linearly: one chain, about 1e-5.
 constexpr int kPromoteX = 0;
 
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 }
 
 // FP16 hi/lo planes of the two operands the iteration starts from, from A (FP32, damped and normalised):
-//   M_0 = A / ||A||_F  (scaled by s_m)      T_0 = a I - b M_0  (scaled by s_t)      X_1 = T_0
+//   M_0 = A / ||A||_F  (scaled by s_m)      T_0 = a I - b M_0  (scaled by s_t), which is also X_1
 // planes layout [2][batch][n][n], hi plane first.  With t_planes == nullptr only the hi plane of M_0 is written (all
 // that the single-pass squarings of the norm bound read).
 // With defl_v the input is A and the deflation A' = A + sum_j coef[j] v_j v_j^T is applied on the way (the terms of
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restrict__ a32, int n, int batch,
                                                           const float* __restrict__ sumsq, float a, float b, float s_m,
                                                           float s_t, __half* __restrict__ m_planes,
-                                                          __half* __restrict__ t_planes, __half* __restrict__ x_planes,
+                                                          __half* __restrict__ t_planes,
                                                           const float* __restrict__ defl_v,
                                                           const float* __restrict__ defl_coef, int defl_r,
                                                           int vstride) {
@@ -338,8 +340,6 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
   __half* ml = m_planes + ((long long)batch + bi) * nn;
   __half* th = t_planes + bi * nn;
   __half* tl = t_planes + ((long long)batch + bi) * nn;
-  __half* xh = x_planes + bi * nn;  // X_1 = T_0: a second copy, because T's buffer is rewritten by the first step
-  __half* xl = x_planes + ((long long)batch + bi) * nn;
   const int n4 = n / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nn / 4; i += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(i / n4), c = (int)(i - (long long)r * n4) * 4;
@@ -376,8 +376,6 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
     *reinterpret_cast<uint2*>(ml + i * 4) = *reinterpret_cast<uint2*>(l);
     *reinterpret_cast<uint2*>(th + i * 4) = *reinterpret_cast<uint2*>(g);
     *reinterpret_cast<uint2*>(tl + i * 4) = *reinterpret_cast<uint2*>(k);
-    *reinterpret_cast<uint2*>(xh + i * 4) = *reinterpret_cast<uint2*>(g);
-    *reinterpret_cast<uint2*>(xl + i * 4) = *reinterpret_cast<uint2*>(k);
   }
 }
 
@@ -1373,10 +1371,10 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Tb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate);
       TONER_CUDA(cudaGetLastError());
     } else {
-    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, nullptr, 0, 0);
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0);
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -1418,10 +1416,15 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
       TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Tb[0], Xb[1], nullptr, nullptr, 0, 0);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Xb[1], nullptr, nullptr, 0, 0);
       TONER_CUDA(cudaGetLastError());
     }
     }
+
+    // The plane products of a single-chain product are interleaved where the spectrum is not so wide that the M updates need
+    // the shortest chains: there, every rounding of the accumulation is magnified by the inverse of the smallest eigenvalue,
+    // and the order it was measured in (plane by plane) stays.
+    const bool interleave = l0 >= kInterleaveLower;
 
     // D = (A planes) * (B planes)^T / (sa * sb): symmetric result, FP32-accurate; outputs as requested
     struct Out {
@@ -1455,17 +1458,19 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)kc * nn;
       g.maxres = o.maxres;
       g.promote = promote;
+      g.interleave = interleave ? 1 : 0;
       return launch_gemm(g, stream);
     };
     int rc = 0;
-    const __half* Xcur = Xb[1];  // X_1 = T_0
+    // X_1 = T_0, read by both chains until the first product with X; the next T goes to T's own buffer
+    const __half* Xcur = Xb[1];
+    const __half* Tcur = Xb[1];
     float s_x = s_t;
     double x_bound = sched[0].a;
-    int xi = 0, mi = 0, ti = 0;
+    int xi = 0, mi = 0, ti = 1;   // ti: which T buffer was written last
 
     for (int it = 0; it < iters; ++it) {
       const bool last = (it == iters - 1);
-      const __half* Tcur = Tb[ti];
       if (it > 0) {
         x_bound = std::min(x_bound * sched[it].a, x_cap);
         if (last) {
@@ -1543,7 +1548,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       }
       {
         const float na = (float)sched[it + 1].a, nb = (float)sched[it + 1].b;
-        const int tn = (log2p == 0) ? (ti ^ 1) : ti;  // with p == 1 the product reads T itself
+        const int tn = (log2p == 0) ? (ti ^ 1) : 0;  // with p == 1 the product reads T itself
         Out o;
         o.s1 = Tb[tn];
         if (it == iters - 2) {
@@ -1564,6 +1569,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         if (rc) return rc;
         mi ^= 1;
         ti = tn;
+        Tcur = Tb[tn];
         s_t = o.s1_scale;
       }
     }

@@ -121,7 +121,7 @@ __host__ __device__ inline int gemm_tiles_per_batch(int M, int N, int BN, int tr
 // the statistic X^T X, or three plane passes of a wide matrix).
 constexpr int kEpiBlockBytes = 32 * 32 * 4;  // one staged 32 x 32 block of the epilogue
 
-template <int BN, bool kPair = false>
+template <int BN, bool kPair = false, bool kInter = false>
 struct GemmSmem {
   static constexpr bool kWide = kPair && BN == 512;
   static constexpr int kABytes = kBM * kBK * 2;
@@ -130,9 +130,10 @@ struct GemmSmem {
   static constexpr int kStageBytes = kABytes + kBBytes;
   // Four stages keep the main loop fed as well as six did (BF16 4096^3 x 4 on pair tiles: 436 us with either; three stages
   // of the 48 KB tiles); the rest of shared memory is the epilogue's, which needs several blocks per warp in flight.
-  static constexpr int kStages = kStageBytes > 32 * 1024 ? 3 : (kStageBytes < 32 * 1024 ? 5 : 4);
+  // (Interleaved plane products hold two stages until the three products of a k-block have been issued: six.)
+  static constexpr int kStages = kInter ? 6 : (kStageBytes > 32 * 1024 ? 3 : (kStageBytes < 32 * 1024 ? 5 : 4));
   static constexpr int kTileBytes = kStages * kStageBytes;
-  static constexpr int kEpiBufs = kStageBytes > 32 * 1024 ? 2 : 3;          // 4 KB blocks per epilogue warp
+  static constexpr int kEpiBufs = kInter ? 1 : (kStageBytes > 32 * 1024 ? 2 : 3);   // 4 KB blocks per epilogue warp
   static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
   static constexpr int kBarBytes = 256;
   static constexpr int kTotal = kTileBytes + kEpiBytes + kBarBytes + 1024;  // 1024: alignment slack
@@ -450,14 +451,20 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 // kPair: launched as clusters of two CTAs that share each 256 x BN tile (BN = 256): both load their halves of
 // the operands, the leader CTA's MMA thread issues cta_group::2 MMAs, each CTA's epilogue warps write the
 // 128 rows that sit in its own tensor memory.  The pair halves the operand traffic per flop of B.
-template <int BN, bool kChained, bool kPair = false>
+//
+// kInter: the split-precision product Ah Bh + Ah Bl + Al Bh with its three plane products interleaved k-block by k-block: a
+// stage with the hi planes of a k-block, a stage with the lo planes, three groups of MMAs over the two, so that each plane
+// comes from L2 once instead of one and a half times.  What bounds the main loop is that traffic: with all SMs running the
+// pair tiles take in 44 B per clock and SM whatever the tile (736 cycles per k-block of 256 x 256, 1100 of 256 x 512, against
+// 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.
+template <int BN, bool kChained, bool kPair = false, bool kInter = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
-  using S = GemmSmem<BN, kPair>;
+  using S = GemmSmem<BN, kPair, kInter>;
+  static_assert(!kInter || (kPair && BN == 256 && !kChained), "interleaved plane products: 256 x 256 on pairs");
   static_assert((BN == 64 && !kPair) || BN == 128 || BN == 256 || (BN == 512 && kPair && !kChained),
                 "tile widths: 64 (single CTAs), 128, 256, or 512 (pairs)");
   constexpr bool kWide = S::kWide;
   constexpr int BNI = kWide ? 256 : BN;                // columns of one MMA instruction
-  constexpr int NJ = BN / BNI;                         // MMAs per k-step (column halves of a wide tile)
   constexpr int TM = kPair ? 2 * kBM : kBM;            // rows of one scheduled tile
   const uint32_t cta_rank = kPair ? ptx::cluster_ctarank() : 0u;
   const bool leader = cta_rank == 0;
@@ -492,7 +499,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   const int tiles_per_batch = gemm_tiles_per_batch(p.M, p.N, BN, p.tri, TM);
   const int total_tiles = tiles_per_batch * p.batch;
   const int kb_per_seg = (p.K + kBK - 1) / kBK;
-  const int num_kb = kb_per_seg * p.segs;
+  const int num_kb = kInter ? kb_per_seg : kb_per_seg * p.segs;
   // Accumulation chains: with promote > 0 the MMA warp starts a fresh TMEM accumulator every `promote`
   // k-blocks of the FIRST segment and the epilogue warps sum the chains in registers.  Later segments
   // (the hi*lo cross terms of a split product, 2^-11 of the first) form one chain each: truncation
@@ -605,68 +612,77 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         // a pair splits the tile's rows (A) and its columns (B) between its two CTAs
         // (of a wide tile each CTA holds 128 columns of either 256-column half: n0 is its share of the first half)
         const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN + (int)cta_rank * (kWide ? BNI / 2 : S::kBRows);
-        for (int kb = w.kb_lo; kb < w.kb_hi && ok;) {
-          const int si = kb / kb_per_seg, seg_end = min(w.kb_hi, (si + 1) * kb_per_seg);
-          const int seg = rest_first ? (si + 1 == p.segs ? 0 : si + 1) : si;
-          const int za = b * p.a_z_stride + p.a_seg_z[seg];
-          const int zb = b * p.b_z_stride + p.b_seg_z[seg];
-          for (; kb < seg_end; ++kb) {
-            const int k0 = (kb - si * kb_per_seg) * kBK;
-            const long long w0 = p.prof ? clock64() : 0;
-            const bool got = ptx::mbar_wait(empty_bar(stage), phase ^ 1u, kWaitCycles);
-            if (p.prof) prof_wait += clock64() - w0;
-            if (!got || *abort_flag) {
-              report(p.status, kTimeoutProducer);
-              raise_abort();
-              ok = false;
-              break;
-            }
-            const uint32_t sa = base + stage * S::kStageBytes;
-            const uint32_t sb = sa + S::kABytes;
-            if constexpr (kPair) {
-              // Both CTAs' copies report to the leader's barrier, which expects the bytes of the whole pair.
-              const uint32_t lbar = ptx::mapa(full_bar(stage), 0);
-              if (leader) ptx::mbar_expect_tx(full_bar(stage), 2 * S::kStageBytes);
-              if (p.a_mn) {
+        // fill the next stage with k-block k0 of planes za / zb
+        auto fill = [&](int k0, int za, int zb) {
+          const long long w0 = p.prof ? clock64() : 0;
+          const bool got = ptx::mbar_wait(empty_bar(stage), phase ^ 1u, kWaitCycles);
+          if (p.prof) prof_wait += clock64() - w0;
+          if (!got || *abort_flag) {
+            report(p.status, kTimeoutProducer);
+            raise_abort();
+            ok = false;
+            return;
+          }
+          const uint32_t sa = base + stage * S::kStageBytes;
+          const uint32_t sb = sa + S::kABytes;
+          if constexpr (kPair) {
+            // Both CTAs' copies report to the leader's barrier, which expects the bytes of the whole pair.
+            const uint32_t lbar = ptx::mapa(full_bar(stage), 0);
+            if (leader) ptx::mbar_expect_tx(full_bar(stage), 2 * S::kStageBytes);
+            if (p.a_mn) {
 #pragma unroll
-                for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d_pair(sa + s * 8192, amap, lbar, m0 + s * 64, k0, za);
-              } else {
-                ptx::tma_load_3d_pair(sa, amap, lbar, k0, m0, za);
-              }
-              if constexpr (kWide) {
-                if (p.b_mn) {
-#pragma unroll
-                  for (int s = 0; s < 4; ++s)
-                    ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + (s >> 1) * BNI + (s & 1) * 64, k0, zb);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < 2; ++j) ptx::tma_load_3d_pair(sb + j * 16384, bmap, lbar, k0, n0 + j * BNI, zb);
-                }
-              } else if (p.b_mn) {
-#pragma unroll
-                for (int s = 0; s < S::kBRows / 64; ++s) ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + s * 64, k0, zb);
-              } else {
-                ptx::tma_load_3d_pair(sb, bmap, lbar, k0, n0, zb);
-              }
+              for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d_pair(sa + s * 8192, amap, lbar, m0 + s * 64, k0, za);
             } else {
-              ptx::mbar_expect_tx(full_bar(stage), S::kStageBytes);
-              if (p.a_mn) {
-#pragma unroll
-                for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d(sa + s * 8192, amap, full_bar(stage), m0 + s * 64, k0, za);
-              } else {
-                ptx::tma_load_3d(sa, amap, full_bar(stage), k0, m0, za);
-              }
+              ptx::tma_load_3d_pair(sa, amap, lbar, k0, m0, za);
+            }
+            if constexpr (kWide) {
               if (p.b_mn) {
 #pragma unroll
-                for (int s = 0; s < BN / 64; ++s) ptx::tma_load_3d(sb + s * 8192, bmap, full_bar(stage), n0 + s * 64, k0, zb);
+                for (int s = 0; s < 4; ++s)
+                  ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + (s >> 1) * BNI + (s & 1) * 64, k0, zb);
               } else {
-                ptx::tma_load_3d(sb, bmap, full_bar(stage), k0, n0, zb);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) ptx::tma_load_3d_pair(sb + j * 16384, bmap, lbar, k0, n0 + j * BNI, zb);
               }
+            } else if (p.b_mn) {
+#pragma unroll
+              for (int s = 0; s < S::kBRows / 64; ++s) ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + s * 64, k0, zb);
+            } else {
+              ptx::tma_load_3d_pair(sb, bmap, lbar, k0, n0, zb);
             }
-            if (++stage == S::kStages) {
-              stage = 0;
-              phase ^= 1u;
+          } else {
+            ptx::mbar_expect_tx(full_bar(stage), S::kStageBytes);
+            if (p.a_mn) {
+#pragma unroll
+              for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d(sa + s * 8192, amap, full_bar(stage), m0 + s * 64, k0, za);
+            } else {
+              ptx::tma_load_3d(sa, amap, full_bar(stage), k0, m0, za);
             }
+            if (p.b_mn) {
+#pragma unroll
+              for (int s = 0; s < BN / 64; ++s) ptx::tma_load_3d(sb + s * 8192, bmap, full_bar(stage), n0 + s * 64, k0, zb);
+            } else {
+              ptx::tma_load_3d(sb, bmap, full_bar(stage), k0, n0, zb);
+            }
+          }
+          if (++stage == S::kStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        };
+        if constexpr (kInter) {
+          const int za = b * p.a_z_stride, zb = b * p.b_z_stride;
+          for (int kb = w.kb_lo; kb < w.kb_hi && ok; ++kb) {
+            fill(kb * kBK, za + p.a_seg_z[0], zb + p.b_seg_z[0]);
+            if (ok) fill(kb * kBK, za + p.a_seg_z[2], zb + p.b_seg_z[1]);
+          }
+        } else {
+          for (int kb = w.kb_lo; kb < w.kb_hi && ok;) {
+            const int si = kb / kb_per_seg, seg_end = min(w.kb_hi, (si + 1) * kb_per_seg);
+            const int seg = rest_first ? (si + 1 == p.segs ? 0 : si + 1) : si;
+            const int za = b * p.a_z_stride + p.a_seg_z[seg];
+            const int zb = b * p.b_z_stride + p.b_seg_z[seg];
+            for (; kb < seg_end && ok; ++kb) fill((kb - si * kb_per_seg) * kBK, za, zb);
           }
         }
       }
@@ -731,43 +747,67 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           };
           if (!wait_drained(buf)) break;
           const uint32_t d_tmem = tmem_base + (uint32_t)(kWide ? 0 : buf * BN);
-          for (int kb = kb_begin; kb < kb_end; ++kb) {
+          // wait for the operands of a stage; its shared-memory address
+          auto operands = [&](int st, uint32_t ph) {
             const long long w1 = p.prof ? clock64() : 0;
-            const bool got_ops = ptx::mbar_wait(full_bar(stage), phase, kWaitCycles);
+            const bool got_ops = ptx::mbar_wait(full_bar(st), ph, kWaitCycles);
             if (p.prof) prof_ops += clock64() - w1;
             if (!got_ops || *abort_flag) {
               report(p.status, kTimeoutMma);
               raise_abort();
               ok = false;
-              break;
             }
             ptx::tc_fence_after();
-            const uint32_t sa = base + stage * S::kStageBytes;
+            return base + st * S::kStageBytes;
+          };
+          // the MMAs of one k-block (columns from 256 * j on), A from stage address sa, B from sb
+          auto multiply = [&](uint32_t sa, uint32_t sb, int j, uint32_t fresh) {
             const uint32_t a_lo = ((sa & 0x3FFFFu) >> 4) | a_lo_const;
-            const uint32_t b_lo = (((sa + S::kABytes) & 0x3FFFFu) >> 4) | b_lo_const;
-            const uint32_t fresh = (kb != kb_begin) ? 1u : 0u;
+            const uint32_t b_lo = (((sb + S::kABytes) & 0x3FFFFu) >> 4) | b_lo_const;
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-              if (kWide && j == 1 && kb == kb_begin && !wait_drained(1)) break;
-#pragma unroll
-              for (int k = 0; k < kBK / kUmmaK; ++k) {
-                const uint64_t da = ((uint64_t)desc_hi << 32) | (a_lo + k * a_step16);
-                const uint64_t db = ((uint64_t)desc_hi << 32) | (b_lo + j * ((BNI / 2) * kBK * 2 / 16) + k * b_step16);
-                if constexpr (kPair) ptx::mma_f16_pair(d_tmem + j * BNI, da, db, idesc, k != 0 ? 1u : fresh);
-                else ptx::mma_f16(d_tmem, da, db, idesc, k != 0 ? 1u : fresh);
-              }
+            for (int k = 0; k < kBK / kUmmaK; ++k) {
+              const uint64_t da = ((uint64_t)desc_hi << 32) | (a_lo + k * a_step16);
+              const uint64_t db = ((uint64_t)desc_hi << 32) | (b_lo + j * ((BNI / 2) * kBK * 2 / 16) + k * b_step16);
+              if constexpr (kPair) ptx::mma_f16_pair(d_tmem + j * BNI, da, db, idesc, k != 0 ? 1u : fresh);
+              else ptx::mma_f16(d_tmem, da, db, idesc, k != 0 ? 1u : fresh);
             }
-            if (!ok) break;
-            // frees the stage (in both CTAs of a pair) once these MMAs have read it
+          };
+          auto release_stage = [&](int st) {  // frees the stage (in both CTAs of a pair) once the MMAs so far have read it
             if constexpr (kPair) {
-              ptx::mma_commit_pair(empty_bar(stage));
-              ptx::mma_commit_pair(ptx::mapa(empty_bar(stage), 1));
+              ptx::mma_commit_pair(empty_bar(st));
+              ptx::mma_commit_pair(ptx::mapa(empty_bar(st), 1));
             } else {
-              ptx::mma_commit(empty_bar(stage));
+              ptx::mma_commit(empty_bar(st));
             }
+          };
+          auto advance = [&]() {
             if (++stage == S::kStages) {
               stage = 0;
               phase ^= 1u;
+            }
+          };
+          for (int kb = kb_begin; kb < kb_end; ++kb) {
+            const uint32_t fresh = (kb != kb_begin) ? 1u : 0u;
+            const int st = stage;
+            const uint32_t hi = operands(st, phase);
+            if (!ok) break;
+            multiply(hi, hi, 0, fresh);
+            if constexpr (kWide) {
+              if (kb == kb_begin && !wait_drained(1)) break;
+              multiply(hi, hi, 1, fresh);
+            }
+            advance();
+            if constexpr (kInter) {
+              const int st_lo = stage;
+              const uint32_t lo = operands(st_lo, phase);
+              if (!ok) break;
+              multiply(hi, lo, 0, 1u);
+              multiply(lo, hi, 0, 1u);
+              advance();
+              release_stage(st);
+              release_stage(st_lo);
+            } else {
+              release_stage(st);
             }
           }
           if (ok) {  // this chain's partial sum is complete

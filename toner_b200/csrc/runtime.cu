@@ -92,6 +92,7 @@ Context* context() {
   allow(gemm_tcgen05_kernel<128, true, true>, GemmSmem<128, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, false, true>, GemmSmem<256, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, true, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, false, true, true>, GemmSmem<256, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<512, false, true>, GemmSmem<512, true>::kTotal);
   if (!ok) {
     set_error("the GEMM kernels' shared memory was refused");
@@ -256,14 +257,16 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
       best = {c.bn, c.pair, splits, splits > 1 ? split_part_bytes(d, c.bn, c.pair, splits) + split_count_bytes(d, c.bn, c.pair) : 0};
     }
   }
-  if (best.bn == 256 && best.pair && best.splits == 1) {
-    // The wide tile: long accumulations only (its epilogue is not hidden behind the next tile), enough tiles for
-    // several waves, and a width for which the 512-column steps do not overshoot the triangle by much.
-    const long long twide = gemm_tiles(d, 512, true), tpair = gemm_tiles(d, 256, true);
-    const long long depth = (long long)d.k * d.segs;
-    if (ctx->gemm_wide_k > 0 && d.promote <= 0 && depth >= ctx->gemm_wide_k && twide >= 4LL * (ctx->gemm_sms / 2) &&
-        2 * twide * 100 <= tpair * 106)
-      best.bn = 512;
+  if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !d.c && kb >= ctx->gemm_wide_kb) {
+    // The wide tile takes in 48 KB per k-block for twice the work of 32 KB, but its epilogue is only half hidden and its
+    // waves are coarser.  Estimates of both, in k-blocks of the pair tile (measured wide / pair: 12 x 3072^3 x 3 planes
+    // symmetric 0.94, 2 x 4096^3 0.86, 12 x 768 x 3072 x 3072 0.89, 18 x 2048^3 0.99; one plane, or with C, above 1).
+    auto waves = [&](int bn) {
+      const long long t = gemm_tiles(d, bn, true), w = ctx->gemm_sms / 2;
+      return (double)((t + w - 1) / w);
+    };
+    const double epi = 8 * block * 0.6 / 736.0;
+    if (waves(512) * (kb * 1.5 + epi) < 0.97 * waves(256) * kb) best.bn = 512;
   }
   return best;
 }
@@ -310,6 +313,11 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
     return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
                          "(256 x 512 on a pair)");
 
+  // The three plane products interleaved: what the pair tiles are bound by is operand traffic, a third of which this saves.
+  const bool planes3 = d.segs == 3 && d.a.seg_z[0] == d.a.seg_z[1] && d.b.seg_z[0] == d.b.seg_z[2];
+  const bool inter = d.interleave && planes3 && d.promote <= 0 && splits == 1 && pair && bn >= 256 && d.tile_n == 0;
+  if (inter) bn = 256;
+
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
   // a pair's CTA loads half a tile's rows of B, at most 128 at a time; MN-major operands always come in 64 x 64 boxes
@@ -335,7 +343,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   p.tri = d.tri ? 1 : 0;
   p.promote = d.promote > 0 ? d.promote : 0;
   p.promote_all = d.promote_all ? 1 : 0;
-  p.raster = d.tri ? 0 : (d.raster > 0 ? d.raster : 8);
+  p.raster = d.tri ? 0 : (d.raster > 0 ? d.raster : (bn == 512 ? 4 : 8));   // (a group of 2048 columns)
   p.alpha = d.alpha; p.beta = d.beta;
   p.alpha_a = d.alpha_a; p.alpha_b = d.alpha_b; p.beta_v = d.beta_v;
   p.alpha_b_step = d.alpha_b_step > 0 ? d.alpha_b_step : 1;
@@ -378,6 +386,10 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   const bool chained = p.promote > 0;
   const int workers = pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
   const int grid = (int)(total < workers ? total : workers) * (pair ? 2 : 1);
+  if (inter) {
+    TONER_CUDA(launch(gemm_tcgen05_kernel<256, false, true, true>, grid, kGemmThreads, GemmSmem<256, true, true>::kTotal, stream, 2, p));
+    return 0;
+  }
 #define TONER_GEMM(BN, CHAINED, PAIR)                                                                                       \
   TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, PAIR>, grid, kGemmThreads, GemmSmem<BN, PAIR>::kTotal, stream, PAIR ? 2 : 0, p))
   if (pair && bn == 512) TONER_GEMM(512, false, true);
