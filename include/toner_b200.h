@@ -122,9 +122,10 @@ typedef struct toner_gemm_desc {
   void* split_ws;           /* optional scratch: a product with few tiles and a long accumulation may then divide each tile's
                                accumulation among several CTAs and add the parts (in a fixed order) there */
   int64_t split_ws_bytes;
-  int32_t interleave;       /* 1: a split product (segs = 3: Ah Bh, Ah Bl, Al Bh, one chain) may take its three plane products
-                               k-block by k-block, which saves a third of the operand traffic; the additions into the
-                               accumulator then come in that order instead of plane by plane */
+  int32_t interleave;       /* 1: a split product (segs = 3: Ah Bh, Ah Bl, Al Bh) may take its three plane products k-block by
+                               k-block, which saves a third of the operand traffic; the additions into the accumulator
+                               then come in that order instead of plane by plane (no less accurate: chains become
+                               shorter to make up for the cross products in them) */
 } toner_gemm_desc;
 
 int toner_gemm(const toner_gemm_desc* desc, void* stream);
@@ -273,7 +274,8 @@ int toner_inv_roots_ex(const float* ema, int32_t k, int32_t n, float damping, in
  *                  eigenvector of the smallest eigenvalue of A.  After the roots are computed the call advances it by
  *                  `track_sweeps` power-iteration steps on the highest inverse power (A^(-q/p)), where that eigenvalue
  *                  is the dominant one however small it is next to lambda_max(A); track_sweeps + 256 starts from a
- *                  fixed vector instead of the buffer's content (first call, or after the statistics were replaced).
+ *                  fixed vector instead of the buffer's content (first call, or after the statistics were replaced);
+ *                  track_sweeps + 512 keeps the plane-by-plane order of additions in every product (interleave = 0).
  *   lmin_out       (DEVICE, optional, k floats) the estimate of lambda_min(A_b) that comes with it: a Rayleigh quotient,
  *                  so it errs on the high side (by 5-25 % after 8 sweeps from scratch, less once tracking).
  *   lower, lower_is_estimate
@@ -411,6 +413,7 @@ typedef struct toner_matrix_group {
   const void* outer_planes; const float* outer_inv;
   const float* outer_fro2;     /* squared Frobenius norms of the outer factors */
   int32_t count, rows, cols, factors, first, step;
+  int32_t interleave;          /* 1: split products may take their plane products k-block by k-block (toner_gemm_desc) */
 } toner_matrix_group;
 
 /* m <- mu m + g, work <- (g + mu m  or  m) R_inner: what the polar iteration starts from */

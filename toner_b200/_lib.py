@@ -68,7 +68,7 @@ class MatrixGroup(C.Structure):
         ("inner_planes", C.c_void_p), ("inner_inv", C.c_void_p), ("outer_planes", C.c_void_p), ("outer_inv", C.c_void_p),
         ("outer_fro2", C.c_void_p),
         ("count", C.c_int32), ("rows", C.c_int32), ("cols", C.c_int32), ("factors", C.c_int32), ("first", C.c_int32),
-        ("step", C.c_int32),
+        ("step", C.c_int32), ("interleave", C.c_int32),
     ]
 
 

@@ -76,13 +76,14 @@ class FactorSet:
     of the outer factor."""
 
     def __init__(self, k: int, n: int, device: torch.device, strengths: Tuple[float, float], damping: float,
-                 scratch: Optional[Scratch] = None, chunk: Optional[int] = None) -> None:
+                 scratch: Optional[Scratch] = None, chunk: Optional[int] = None, interleave: bool = True) -> None:
         if n % 8:
             raise ValueError("statistic width must be a multiple of 8 (TMA row pitch of the 16-bit operands)")
         self.k, self.n, self.device, self.damping = k, n, device, float(damping)
         self.inner_strength, self.outer_strength = float(strengths[0]), float(strengths[1])
         self.p, self.q = root_orders(*strengths)
         self.scratch = scratch or Scratch()
+        self.interleave = interleave     # split products by k-block instead of by plane (toner_gemm_desc)
         self.ema = torch.zeros(k, n, n, device=device, dtype=torch.float32)
         self.weight = 0.0
         self.root_lo = torch.empty(k, n, n, device=device, dtype=torch.float32)
@@ -204,7 +205,7 @@ class FactorSet:
                       deflate=self.deflate if self.tracking and self.block_deflation else None,
                       deflate_rank=self.deflate_rank,
                       deflate_restart=self.track_restart, deflated=self.deflated if self.tracking else None,
-                      ritz_norm=ritz)
+                      ritz_norm=ritz, interleave=self.interleave)
         self.track_restart = False
         self._estimate_in_flight = self.lower_is_estimate
         self._lower_used = self.lower
@@ -281,7 +282,7 @@ class FactorSet:
         self.repairs += len(bad)
         idx = torch.tensor(bad, device=self.device)
         sub = self.ema.index_select(0, idx).contiguous()
-        lo, hi, fro2, st = ops.inv_roots(sub, self.damping, self.p, self.q)
+        lo, hi, fro2, st = ops.inv_roots(sub, self.damping, self.p, self.q, interleave=self.interleave)
         self.root_lo.index_copy_(0, idx, lo)
         if self.q > 1:
             self.root_hi.index_copy_(0, idx, hi)
@@ -364,6 +365,7 @@ def _c_group(group: MatrixGroup, buf: Dict[str, torch.Tensor], grads: Optional[S
         c.v = None if group.v is None else group.v.data_ptr()
         c.count, c.rows, c.cols = group.count, group.out_features, group.in_features
         c.factors, c.first, c.step = f.k, group.first, group.step
+        c.interleave = int(f.interleave)
         for which in ("inner", "outer"):
             planes, inv = f.planes(which)
             setattr(c, which + "_planes", None if planes is None else planes.data_ptr())

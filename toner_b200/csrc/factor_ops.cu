@@ -75,8 +75,6 @@ static int chain_length(double lower) {
   return 0;
 }
 
-constexpr double kInterleaveLower = 5e-3;   // chain_length()'s first threshold
-
 // Products applied to X (and the final squarings) pass their error on linearly: one chain, about 1e-5.
 constexpr int kPromoteX = 0;
 
@@ -1236,7 +1234,8 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
   const double l0 = (lower > 0.f && (double)lower > l_worst) ? (double)lower : l_worst;
   const bool estimated = lower_is_estimate != 0 && l0 > l_worst;
   if (estimated && !track) return fail(kErrArg, "inv_roots: an estimated bound needs the tracking vectors to verify it");
-  if (track_sweeps < 0 || (track_sweeps & ~(63 | 256))) return fail(kErrArg, "inv_roots: track_sweeps is 0..63, plus 256 to start afresh");
+  if (track_sweeps < 0 || (track_sweeps & ~(63 | 256 | 512)))
+    return fail(kErrArg, "inv_roots: track_sweeps is 0..63, plus 256 to start afresh, plus 512 for plane-by-plane products");
   const int defl_r = deflate ? (deflate_rank & 15) : 0;      // directions the block iteration looks for (0: one, the old way)
   const bool defl_cold = deflate && (deflate_rank & 256);
   const bool ritz_norm = deflate && (deflate_rank & 512);   // norm from the block iteration instead of three squarings
@@ -1421,10 +1420,9 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
     }
     }
 
-    // The plane products of a single-chain product are interleaved where the spectrum is not so wide that the M updates need
-    // the shortest chains: there, every rounding of the accumulation is magnified by the inverse of the smallest eigenvalue,
-    // and the order it was measured in (plane by plane) stays.
-    const bool interleave = l0 >= kInterleaveLower;
+    // Plane products are interleaved (toner_gemm_desc::interleave) unless the caller asked for the plane-by-plane order of
+    // additions and the spectrum is wide enough for it to be seen (chain_length()'s first threshold).
+    const bool interleave = !(track_sweeps & 512) || l0 >= 5e-3;
 
     // D = (A planes) * (B planes)^T / (sa * sb): symmetric result, FP32-accurate; outputs as requested
     struct Out {

@@ -133,7 +133,8 @@ struct GemmSmem {
   // (Interleaved plane products hold two stages until the three products of a k-block have been issued: six.)
   static constexpr int kStages = kInter ? 6 : (kStageBytes > 32 * 1024 ? 3 : (kStageBytes < 32 * 1024 ? 5 : 4));
   static constexpr int kTileBytes = kStages * kStageBytes;
-  static constexpr int kEpiBufs = kInter ? 1 : (kStageBytes > 32 * 1024 ? 2 : 3);   // 4 KB blocks per epilogue warp
+  // 4 KB blocks per epilogue warp
+  static constexpr int kEpiBufs = kInter && kStageBytes == 32 * 1024 ? 1 : (kInter || kStageBytes > 32 * 1024 ? 2 : 3);
   static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
   static constexpr int kBarBytes = 256;
   static constexpr int kTotal = kTileBytes + kEpiBytes + kBarBytes + 1024;  // 1024: alignment slack
@@ -453,14 +454,21 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 // 128 rows that sit in its own tensor memory.  The pair halves the operand traffic per flop of B.
 //
 // kInter: the split-precision product Ah Bh + Ah Bl + Al Bh with its three plane products interleaved k-block by k-block: a
-// stage with the hi planes of a k-block, a stage with the lo planes, three groups of MMAs over the two, so that each plane
+// stage with the lo planes of a k-block, a stage with the hi planes, three groups of MMAs over the two, so that each plane
 // comes from L2 once instead of one and a half times.  What bounds the main loop is that traffic: with all SMs running the
 // pair tiles take in 44 B per clock and SM whatever the tile (736 cycles per k-block of 256 x 256, 1100 of 256 x 512, against
-// 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.
+// 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.  Measured
+// plane by plane / interleaved: 12 x 3072^3 symmetric 1002 / 736 us (1.53 PFLOP/s), 6 x 5632^3 symmetric 3096 / 2145 us.
+// The cross products of a k-block go into the accumulator before its hi product.  Truncation (one unit of the accumulator's
+// last place per addition, so in proportion to the sum so far): with H the sum a hi k-block adds, four additions of either
+// kind per k-block and N k-blocks, plane by plane loses (2 N^2 + 8 N^2) H units, interleaved about 6 N^2 H; of chains of c
+// k-blocks (hi only; the cross products in chains of their own) it loses 2 c + 1/2 a k-block, of c interleaved ones 6 c - 3.5.
+// The host therefore turns a chain of c into one of (c + 2) / 3, which loses no more.  (GemmParams::segs is 1 here: the
+// three products are one.)
 template <int BN, bool kChained, bool kPair = false, bool kInter = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair, kInter>;
-  static_assert(!kInter || (kPair && BN == 256 && !kChained), "interleaved plane products: 256 x 256 on pairs");
+  static_assert(!kInter || (kPair && BN <= 256), "interleaved plane products: 256 x 256 or 256 x 128 on pairs");
   static_assert((BN == 64 && !kPair) || BN == 128 || BN == 256 || (BN == 512 && kPair && !kChained),
                 "tile widths: 64 (single CTAs), 128, 256, or 512 (pairs)");
   constexpr bool kWide = S::kWide;
@@ -499,7 +507,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   const int tiles_per_batch = gemm_tiles_per_batch(p.M, p.N, BN, p.tri, TM);
   const int total_tiles = tiles_per_batch * p.batch;
   const int kb_per_seg = (p.K + kBK - 1) / kBK;
-  const int num_kb = kInter ? kb_per_seg : kb_per_seg * p.segs;
+  const int num_kb = kb_per_seg * p.segs;
   // Accumulation chains: with promote > 0 the MMA warp starts a fresh TMEM accumulator every `promote`
   // k-blocks of the FIRST segment and the epilogue warps sum the chains in registers.  Later segments
   // (the hi*lo cross terms of a split product, 2^-11 of the first) form one chain each: truncation
@@ -673,8 +681,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         if constexpr (kInter) {
           const int za = b * p.a_z_stride, zb = b * p.b_z_stride;
           for (int kb = w.kb_lo; kb < w.kb_hi && ok; ++kb) {
-            fill(kb * kBK, za + p.a_seg_z[0], zb + p.b_seg_z[0]);
-            if (ok) fill(kb * kBK, za + p.a_seg_z[2], zb + p.b_seg_z[1]);
+            fill(kb * kBK, za + p.a_seg_z[2], zb + p.b_seg_z[1]);
+            if (ok) fill(kb * kBK, za + p.a_seg_z[0], zb + p.b_seg_z[0]);
           }
         } else {
           for (int kb = w.kb_lo; kb < w.kb_hi && ok;) {
@@ -789,24 +797,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           for (int kb = kb_begin; kb < kb_end; ++kb) {
             const uint32_t fresh = (kb != kb_begin) ? 1u : 0u;
             const int st = stage;
-            const uint32_t hi = operands(st, phase);
+            const uint32_t first = operands(st, phase);
             if (!ok) break;
-            multiply(hi, hi, 0, fresh);
-            if constexpr (kWide) {
-              if (kb == kb_begin && !wait_drained(1)) break;
-              multiply(hi, hi, 1, fresh);
-            }
             advance();
             if constexpr (kInter) {
-              const int st_lo = stage;
-              const uint32_t lo = operands(st_lo, phase);
+              const int st_hi = stage;
+              const uint32_t hi = operands(st_hi, phase);
               if (!ok) break;
-              multiply(hi, lo, 0, 1u);
-              multiply(lo, hi, 0, 1u);
               advance();
+              multiply(hi, first, 0, fresh);   // Ah Bl
+              multiply(first, hi, 0, 1u);      // Al Bh
               release_stage(st);
-              release_stage(st_lo);
+              multiply(hi, hi, 0, 1u);
+              release_stage(st_hi);
             } else {
+              multiply(first, first, 0, fresh);
+              if constexpr (kWide) {
+                if (kb == kb_begin && !wait_drained(1)) break;
+                multiply(first, first, 1, fresh);
+              }
               release_stage(st);
             }
           }

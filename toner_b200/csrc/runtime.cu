@@ -92,7 +92,10 @@ Context* context() {
   allow(gemm_tcgen05_kernel<128, true, true>, GemmSmem<128, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, false, true>, GemmSmem<256, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, true, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, false, true, true>, GemmSmem<128, true, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, true, true, true>, GemmSmem<128, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, false, true, true>, GemmSmem<256, true, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, true, true, true>, GemmSmem<256, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<512, false, true>, GemmSmem<512, true>::kTotal);
   if (!ok) {
     set_error("the GEMM kernels' shared memory was refused");
@@ -207,11 +210,17 @@ struct TileChoice {
   size_t ws_bytes;   // scratch the splits need
 };
 
+// Whether a product's three plane products may be interleaved (toner_gemm_desc::interleave); only pair tiles do.
+static bool may_interleave(const toner_gemm_desc& d) {
+  return d.interleave && d.segs == 3 && !d.promote_all && d.a.seg_z[0] == d.a.seg_z[1] && d.b.seg_z[0] == d.b.seg_z[2];
+}
+
 // Which tile, and among how many units a tile's accumulation is divided (only where the caller gave scratch for it).  An
 // estimate of the launch in SM cycles decides, from what was measured on the kernel:
 //   * the main loop is bound by shared memory (128 B per clock: operands written by TMA and read by the MMAs), 512 cycles
 //     per 64-deep k-block of 256 x 256 on a pair and of 128 x 128 on one CTA, 384 of 256 x 128 on a pair and of 128 x 64,
 //     768 of 128 x 256;
+//   * interleaved plane products bring two thirds of the operands: 256 x 256 stays bound by its MMAs, 256 x 128 takes 320;
 //   * a 32 x 32 block of the epilogue takes a warp 900 cycles plus 450 per box moved, and its boxes take shared memory away
 //     from the main loop of the next tile;
 //   * tiles of one wave run side by side, and the epilogue of one tile beside the main loop of the next.
@@ -221,9 +230,10 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
   struct Config {
     int bn;
     bool pair;
-    double per_kb;
+    double per_kb, per_kb_inter;
   };
-  static const Config configs[] = {{256, true, 512}, {128, true, 384}, {256, false, 768}, {128, false, 512}, {64, false, 384}};
+  static const Config configs[] = {{256, true, 512, 512}, {128, true, 384, 320}, {256, false, 768, 768}, {128, false, 512, 512}, {64, false, 384, 384}};
+  const bool inter = may_interleave(d);
   const bool mirror = d.tri && d.mirror;
   const double boxes = (d.c ? 1.2 : 0.0) + (d.d ? (mirror && !d.upper_d ? 2.0 : 1.0) : 0.0) + (d.d16 ? (mirror ? 1.6 : 1.0) : 0.0) +
                        ((d.split0 ? 1.3 : 0.0) + (d.split1 ? 1.3 : 0.0)) * (mirror ? 2.0 : 1.0);
@@ -236,7 +246,7 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
     const long long tiles = gemm_tiles(d, c.bn, c.pair);
     const int workers = c.pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
     const int blocks = c.bn / 64;   // per epilogue warp
-    const double main = kb * c.per_kb, epi = blocks * block;
+    const double main = kb * (inter ? c.per_kb_inter : c.per_kb), epi = blocks * block;
     const double waves = (double)((tiles + workers - 1) / workers);
     const double busy = main + blocks * 8 * block_smem;
     double cost = main + epi + (waves - 1) * (busy > epi ? busy : epi);
@@ -257,7 +267,7 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
       best = {c.bn, c.pair, splits, splits > 1 ? split_part_bytes(d, c.bn, c.pair, splits) + split_count_bytes(d, c.bn, c.pair) : 0};
     }
   }
-  if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !d.c && kb >= ctx->gemm_wide_kb) {
+  if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !d.c && !inter && kb >= ctx->gemm_wide_kb) {
     // The wide tile takes in 48 KB per k-block for twice the work of 32 KB, but its epilogue is only half hidden and its
     // waves are coarser.  Estimates of both, in k-blocks of the pair tile (measured wide / pair: 12 x 3072^3 x 3 planes
     // symmetric 0.94, 2 x 4096^3 0.86, 12 x 768 x 3072 x 3072 0.89, 18 x 2048^3 0.99; one plane, or with C, above 1).
@@ -313,10 +323,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
     return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
                          "(256 x 512 on a pair)");
 
-  // The three plane products interleaved: what the pair tiles are bound by is operand traffic, a third of which this saves.
-  const bool planes3 = d.segs == 3 && d.a.seg_z[0] == d.a.seg_z[1] && d.b.seg_z[0] == d.b.seg_z[2];
-  const bool inter = d.interleave && planes3 && d.promote <= 0 && splits == 1 && pair && bn >= 256 && d.tile_n == 0;
-  if (inter) bn = 256;
+  const bool inter = pair && bn <= 256 && may_interleave(d);
 
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
@@ -337,11 +344,11 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
     p.a_seg_z[s] = d.a.list ? 0 : d.a.seg_z[s];
     p.b_seg_z[s] = d.b.list ? 0 : d.b.seg_z[s];
   }
-  p.segs = d.segs;
+  p.segs = inter ? 1 : d.segs;
   p.M = d.m; p.N = d.n; p.K = d.k; p.batch = d.batch;
   p.fmt = d.fmt;
   p.tri = d.tri ? 1 : 0;
-  p.promote = d.promote > 0 ? d.promote : 0;
+  p.promote = d.promote > 0 ? (inter ? (d.promote + 2) / 3 : d.promote) : 0;   // (see gemm_tcgen05_kernel)
   p.promote_all = d.promote_all ? 1 : 0;
   p.raster = d.tri ? 0 : (d.raster > 0 ? d.raster : (bn == 512 ? 4 : 8));   // (a group of 2048 columns)
   p.alpha = d.alpha; p.beta = d.beta;
@@ -386,10 +393,16 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   const bool chained = p.promote > 0;
   const int workers = pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
   const int grid = (int)(total < workers ? total : workers) * (pair ? 2 : 1);
+#define TONER_INTER(BN, CHAINED)                                                                                           \
+  TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, true, true>, grid, kGemmThreads, GemmSmem<BN, true, true>::kTotal, stream, 2, p))
   if (inter) {
-    TONER_CUDA(launch(gemm_tcgen05_kernel<256, false, true, true>, grid, kGemmThreads, GemmSmem<256, true, true>::kTotal, stream, 2, p));
+    if (bn == 256 && chained) TONER_INTER(256, true);
+    else if (bn == 256) TONER_INTER(256, false);
+    else if (chained) TONER_INTER(128, true);
+    else TONER_INTER(128, false);
     return 0;
   }
+#undef TONER_INTER
 #define TONER_GEMM(BN, CHAINED, PAIR)                                                                                       \
   TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, PAIR>, grid, kGemmThreads, GemmSmem<BN, PAIR>::kTotal, stream, PAIR ? 2 : 0, p))
   if (pair && bn == 512) TONER_GEMM(512, false, true);

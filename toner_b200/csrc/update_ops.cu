@@ -451,10 +451,9 @@ int toner_apply_scaled(float* const* weight_ptrs, const float* delta, int32_t co
 }
 
 // ------------------------------------------------------------------ whole stages of an update
-// d[b] = alpha * A[b] R[first + b step]: FP32-accurate from hi/lo planes (interleave: see toner_gemm_desc), or (coarse) the
-// hi planes only
+// d[b] = alpha * A[b] R[first + b step]: FP32-accurate from hi/lo planes, or (coarse) the hi planes only
 static int right_product(const toner_matrix_group& g, bool outer, float* d, bool coarse, float alpha, const float* c,
-                         const float* beta_v, uint32_t* maxabs, bool interleave, cudaStream_t stream) {
+                         const float* beta_v, uint32_t* maxabs, cudaStream_t stream) {
   const void* planes = outer ? g.outer_planes : g.inner_planes;
   const float* inv = outer ? g.outer_inv : g.inner_inv;
   toner_gemm_desc q = {};
@@ -479,7 +478,7 @@ static int right_product(const toner_matrix_group& g, bool outer, float* d, bool
     q.beta_v = beta_v;
   }
   q.maxabs = maxabs;
-  q.interleave = interleave ? 1 : 0;
+  q.interleave = g.interleave;
   return launch_gemm(q, stream);
 }
 
@@ -505,7 +504,7 @@ int toner_muont_input(const toner_matrix_group* g, float mu, int32_t nesterov, v
   if (rc || !g->inner_planes) return rc;
   rc = split_stack(*g, g->work, nullptr, g->maxabs, nullptr, nullptr, false, false, stream);
   if (rc) return rc;
-  return right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, true, stream);
+  return right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);
 }
 
 int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs, float lr, float weight_decay, float scale,
@@ -522,13 +521,13 @@ int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs,
     // V = c1 W R + c2 P.  The decay term is lr wd ||W|| against lr ||P||, about 1 % of V: the hi planes suffice, and only they
     // are written
     rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->weights), nullptr, w_max, g->c1, true, true, stream);
-    if (!rc) rc = right_product(*g, true, g->work, true, 1.f, g->work, g->c2, v_max, true, stream);
+    if (!rc) rc = right_product(*g, true, g->work, true, 1.f, g->work, g->c2, v_max, stream);
     if (!rc) rc = split_stack(*g, g->work, nullptr, v_max, nullptr, nullptr, false, false, stream);
   } else {   // V = c2 P
     rc = split_stack(*g, g->work, nullptr, polar_maxabs, w_max, g->c2, false, true, stream);
   }
   if (rc) return rc;
-  return right_product(*g, true, delta, false, -1.f, nullptr, nullptr, nullptr, true, stream);
+  return right_product(*g, true, delta, false, -1.f, nullptr, nullptr, nullptr, stream);
 }
 
 int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay, float beta1, float beta2, float bc1, float bc2,
@@ -548,15 +547,15 @@ int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay,
   // one pass over the gradient: m <- b1 m + (1 - b1) g, max |g|, max |m|
   TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->grads, g->m, per, beta1, max0, max1);
   int rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->grads), max0, nullptr, nullptr, false, false, stream);
-  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, false, stream);                // t = g R
+  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // t = g R
   if (!rc) rc = split_stack(*g, g->m, nullptr, max1, nullptr, nullptr, false, false, stream);
-  if (!rc) rc = right_product(*g, false, g->work2, false, 1.f / bc1, nullptr, nullptr, nullptr, false, stream);         // (m / bc1) R
+  if (!rc) rc = right_product(*g, false, g->work2, false, 1.f / bc1, nullptr, nullptr, nullptr, stream);         // (m / bc1) R
   if (rc) return rc;
   TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->work, g->v, g->work2, per, beta2, bc2,
                eps, max2);                                                                                       // U, in work2
   rc = sumsq_det(g->work2, g->count, g->rows, g->cols, g->cols, per, g->ss_scratch, ss0, stream);
   if (!rc) rc = split_stack(*g, g->work2, nullptr, max2, nullptr, nullptr, false, false, stream);
-  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, false, stream);                // U R
+  if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // U R
   if (!rc) rc = sumsq_det(g->work, g->count, g->rows, g->cols, g->cols, per, g->ss_scratch, ss1, stream);
   if (rc) return rc;
   TONER_LAUNCH(adamt_coeff_kernel, (g->count + 127) / 128, 128, stream, g->outer_fro2, g->first, g->step, g->count, g->cols, lr,
@@ -564,10 +563,10 @@ int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay,
   if (weight_decay == 0.f)                                                                                       // c2 U R
     return toner_scale_stack(g->work, g->c2, delta, g->count, per, stream);
   rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->weights), nullptr, max0, g->c1, true, true, stream);
-  if (!rc) rc = right_product(*g, true, g->work2, true, 1.f, nullptr, nullptr, max1, false, stream);                    // c1 W R
+  if (!rc) rc = right_product(*g, true, g->work2, true, 1.f, nullptr, nullptr, max1, stream);                    // c1 W R
   if (!rc) rc = split_stack(*g, g->work2, nullptr, max1, nullptr, nullptr, false, false, stream);
   if (rc) return rc;
-  return right_product(*g, true, delta, false, -1.f, g->work, g->c2, nullptr, false, stream);
+  return right_product(*g, true, delta, false, -1.f, g->work, g->c2, nullptr, stream);
 }
 
 }  // extern "C"

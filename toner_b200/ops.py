@@ -340,7 +340,7 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
               track: Optional[torch.Tensor] = None, lmin: Optional[torch.Tensor] = None,
               resid: Optional[torch.Tensor] = None, track_sweeps: int = 0, track_restart: bool = False,
               deflate: Optional[torch.Tensor] = None, deflate_rank: int = 1, deflate_restart: bool = False,
-              deflated: Optional[torch.Tensor] = None, ritz_norm: bool = False):
+              deflated: Optional[torch.Tensor] = None, ritz_norm: bool = False, interleave: bool = True):
     """A^(-1/p) and A^(-q/p) of the damped, trace-normalised statistics (toner_inv_roots_tracked).
 
     ``lower``: a lower bound of the normalised spectrum valid for every statistic (0: the bound that always
@@ -349,7 +349,8 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     ``resid`` (k,): tracking of the smallest eigenvalue between calls and a bound that is an estimate, verified after
     the chain; ``deflate`` (k, 8, n), ``deflate_rank``, ``deflate_restart``, ``deflated`` (k,) int32: several dominant
     directions found by block power iteration and deflated (see the header); ``ritz_norm``: take the norm from that
-    iteration's largest remaining Ritz value instead of three squarings (an estimate, verified with ``lower``).
+    iteration's largest remaining Ritz value instead of three squarings (an estimate, verified with ``lower``);
+    ``interleave`` = False: plane products one after the other (see the header).
     Returns (root_lo, root_hi or None, fro2_lo, status); nothing is synchronised."""
     _need_cuda(ema)
     if ema.ndim == 2:
@@ -373,7 +374,7 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
         workspace = torch.empty(inv_roots_workspace_bytes(chunk, n), device=dev, dtype=torch.uint8)
     if track is not None and (track.shape != (k, n) or track.dtype != torch.float32 or not track.is_contiguous()):
         raise ValueError("the tracking vectors are a contiguous FP32 (k, n) tensor")
-    sweeps = (int(track_sweeps) & 63) | (256 if track_restart else 0)
+    sweeps = (int(track_sweeps) & 63) | (256 if track_restart else 0) | (0 if interleave else 512)
     if deflate is not None and (deflate.shape != (k, 8, n) or deflate.dtype != torch.float32 or not deflate.is_contiguous()):
         raise ValueError("the deflation vectors are a contiguous FP32 (k, 8, n) tensor")
     rank = (int(deflate_rank) & 15) | (256 if deflate_restart else 0) | (512 if ritz_norm else 0)
