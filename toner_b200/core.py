@@ -189,10 +189,14 @@ class FactorSet:
         blocked = self.tracking and self.block_deflation
         # The largest Ritz value left in the statistic replaces the norm bound's three squarings when the vector it
         # belongs to is at least two calls old (a fresh slot's Rayleigh quotient sits near the MEAN eigenvalue) and the
-        # lower bound is an estimate as well, so that both are verified after the chain.
+        # lower bound is an estimate as well, so that both are verified after the chain.  It needs a vector that is not
+        # deflated: where the whole block looks like outliers and all but one are deflated, deflating the last as well (which
+        # takes the certified norm) narrows the spectrum by more than the norm estimate saves.
+        found = self._host_np[3 * self.k:4 * self.k]
+        deflated, block = int((found & 255).max()), min(self._rank_used, self.deflate_rank)
         ritz = (blocked and self.ritz_norm and self.lower_is_estimate and not self.track_restart
-                and self._warm_calls >= 2
-                and int((self._host_np[3 * self.k:4 * self.k] & 255).max()) < min(self._rank_used, self.deflate_rank))
+                and self._warm_calls >= 2 and deflated < block
+                and not (deflated == block - 1 and int((found >> 8).max()) >= block))
         self._warm_calls = 0 if (self.track_restart or not blocked) else self._warm_calls + 1
         self._rank_used = self.deflate_rank if blocked else 0
         self.ritz_in_flight = bool(ritz)

@@ -890,12 +890,13 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
 }
 
 // Which of the r Ritz pairs are deflated: in descending order, as long as each has converged and stands above eight
-// times the mean c of everything that would remain; all accepted directions are moved to that common c.
+// times the mean c of everything that would remain, at most `most` of them (one fewer than r where the norm is to come from
+// the largest one that stays); all accepted directions are moved to that common c.
 //   coef[b][j] = -(theta_j - c)  (0 where not deflated)      corr[b][j] = theta_j^(-1/p) - c^(-1/p)
 // rest_top[b] / rest_idx[b]: the largest Ritz value that stays in A' and its vector's index (0 / -1 when every vector of
 // the block was deflated: nothing is known about the remainder then).
 __global__ void block_decide_kernel(const float* __restrict__ theta, const float* __restrict__ res, int k, int n, int r,
-                                    float damping, int p, float* __restrict__ coef, float* __restrict__ corr,
+                                    float damping, int p, int most, float* __restrict__ coef, float* __restrict__ corr,
                                     int* __restrict__ count, float* __restrict__ rest_top, int* __restrict__ rest_idx,
                                     float* __restrict__ rest_trace) {
   ptx::pdl_begin();
@@ -904,7 +905,7 @@ __global__ void block_decide_kernel(const float* __restrict__ theta, const float
   const double tr = (double)n * (1.0 + (double)damping);  // A has unit mean diagonal plus the damping
   double sum = 0.0;
   int m = 0;
-  for (int j = 0; j < r && n - (j + 1) > 0; ++j) {
+  for (int j = 0; j < most && n - (j + 1) > 0; ++j) {
     const double t = theta[b * kMaxDeflate + j];
     const double e = res[b * kMaxDeflate + j];
     const double c = (tr - sum - t) / (double)(n - (m + 1));
@@ -1346,7 +1347,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         else TONER_LAUNCH(block_gemv_kernel<8>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
         TONER_LAUNCH(ritz_kernel, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
       }
-      TONER_LAUNCH(block_decide_kernel, (kc + 127) / 128, 128, stream, th8, res8, kc, n, defl_r, damping, p, coef8, corr8, deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx, rest_trace);
+      TONER_LAUNCH(block_decide_kernel, (kc + 127) / 128, 128, stream, th8, res8, kc, n, defl_r, damping, p, ritz_norm ? defl_r - 1 : defl_r, coef8, corr8, deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx, rest_trace);
       if (!ritz_norm) {   // (with the norm estimate the deflation is applied where the operand planes are formed)
         TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, dv, coef8, n, defl_r, kMaxDeflate);
       }
