@@ -107,7 +107,7 @@ typedef struct toner_gemm_desc {
                                it and form one chain each); 1: chain every segment */
   /* Optional FP16 hi/lo operand planes of the result, written by the same kernel so that the next
    * split-precision product needs no separate splitting pass:
-   *   split0: planes of split0_scale * d
+   *   split0: planes of split0_scale * (split0_aff_a * I + d)
    *   split1: planes of split1_scale * (split1_aff_a * [r==c] + split1_aff_b * d)
    * hi plane element (b, r, c) at split + b*split_bs + r*split_ld + c, lo plane split_plane elements further.
    * The scales are the caller's (powers of two chosen from a bound on |d|; FP16 overflows above 65504). */
@@ -122,6 +122,7 @@ typedef struct toner_gemm_desc {
   void* split_ws;           /* optional scratch: a product with few tiles and a long accumulation may then divide each tile's
                                accumulation among several CTAs and add the parts (in a fixed order) there */
   int64_t split_ws_bytes;
+  float split0_aff_a;       /* see split0 */
   int32_t interleave;       /* 1: a split product (segs = 3: Ah Bh, Ah Bl, Al Bh) may take its three plane products k-block by
                                k-block, which saves a third of the operand traffic; the additions into the accumulator
                                then come in that order instead of plane by plane (no less accurate: chains become

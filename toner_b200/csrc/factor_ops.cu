@@ -152,6 +152,40 @@ static bool finish_fit(int p, double lo, double hi, int m, double tail, FitSampl
   return true;
 }
 
+// q(r) of degree m >= 4 in floor(m / 2) + (m odd) products instead of Horner's m - 1: repeated division by
+// y = r^2 + beta r leaves q = (..(w y + l_1(r)) y + ..) y + l_k(r) with linear l_i, which cost no product (they enter it in
+// FP32).  beta is chosen so that the innermost quotient is affine in y itself: top y + top0 (m even), or r (top y + top0) +
+// by_r_const (m odd).  About as accurate as Horner's: what one product's single planes (11 bits) lose is relative to
+// |y| |w| = 0.015 here, |r| |w| = 0.007 there (p = 8, |r| = 0.3) -- 1e-6 of the result, against the chain's 2e-5.  With m = 7
+// on 32 statistics of width 2048 two products of six go, 360 us each.
+struct QuadraticSteps {
+  double beta = 0.0, top = 0.0, top0 = 0.0, by_r_const = 0.0;
+  bool by_r = false;
+  std::vector<std::pair<double, double>> lin;   // (linear, constant) of every division, the outermost first
+};
+static bool quadratic_steps(const FinishPoly& fin, QuadraticSteps& out) {
+  const int m = fin.order;
+  if (m < 4 || !(fin.c[m] > 0.0)) return false;
+  const double beta = fin.c[m - 1] / ((m / 2) * fin.c[m]);
+  if (!(beta > 0.0 && beta < 2.0)) return false;   // (a fit whose leading coefficients are no longer those of a series)
+  out.beta = beta;
+  double q[kMaxFinishOrder + 1];
+  for (int j = 0; j <= m; ++j) q[j] = fin.c[j];
+  int deg = m;
+  const int stop = (m & 1) ? 3 : 2;
+  while (deg > stop) {
+    for (int j = deg; j >= 2; --j) q[j - 1] -= beta * q[j];   // q[j] is now the quotient's coefficient of r^(j-2)
+    out.lin.emplace_back(q[1], q[0]);
+    for (int j = 0; j <= deg - 2; ++j) q[j] = q[j + 2];
+    deg -= 2;
+  }
+  out.by_r = (m & 1) != 0;
+  out.top = q[deg];
+  out.top0 = out.by_r ? q[1] : q[0];
+  out.by_r_const = out.by_r ? q[0] : 0.0;
+  return true;
+}
+
 // In powers of r the fit's coefficients grow as the interval approaches the singularity at r = 1 (sooner for small p):
 // sums with cancellation, which single-pass FP16 products would not survive and whose Horner intermediates
 // W_j = sum_{k >= j} c_k r^(k-j+1) would leave the range the operand planes are scaled for.  Such a fit is not used.
@@ -1421,7 +1455,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
     }
     }
 
-    // Plane products are interleaved (toner_gemm_desc::interleave) unless the caller asked for the plane-by-plane order of
+    // Plane products are interleaved (toner_gemm_desc::interleave), and the finish takes its short form, unless the caller asked for the plane-by-plane order of
     // additions and the spectrum is wide enough for it to be seen (chain_length()'s first threshold).
     const bool interleave = !(track_sweeps & 512) || l0 >= 5e-3;
 
@@ -1430,7 +1464,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       float* d = nullptr;           // FP32 result
       const float* alpha_a = nullptr;  // optional per-statistic factors of the result
       const float* alpha_b = nullptr;
-      __half* s0 = nullptr; float s0_scale = 0.f;
+      __half* s0 = nullptr; float s0_scale = 0.f, s0_a = 0.f;
       __half* s1 = nullptr; float s1_scale = 0.f, s1_a = 0.f, s1_b = 0.f;
       unsigned int* maxres = nullptr;
       const float* c = nullptr; float beta = 0.f;  // result = gain * product + beta * c (c symmetric, FP32)
@@ -1452,7 +1486,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       g.alpha_a = o.alpha_a;
       g.alpha_b = o.alpha_b;
       g.d = o.d; g.ldd = n; g.d_bs = nn;
-      g.split0 = o.s0; g.split0_scale = o.s0_scale;
+      g.split0 = o.s0; g.split0_scale = o.s0_scale; g.split0_aff_a = o.s0_a;
       g.split1 = o.s1; g.split1_scale = o.s1_scale; g.split1_aff_a = o.s1_a; g.split1_aff_b = o.s1_b;
       g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)kc * nn;
       g.maxres = o.maxres;
@@ -1476,28 +1510,73 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
           TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping, lower_used, max_r, (float)root_bound);
           TONER_CUDA(cudaGetLastError());
-          // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  Horner steps
-          // W_j = c_j R + R W_{j+1} (W_m = c_m R) build q(R) = c_0 I + W_1; the terms linear in M enter in FP32 as
-          // beta * c.
+          // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
+          // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
           const float s_w = plane_scale(1.0), s_f = plane_scale(2.0);
-          const __half* wcur = Tcur;
-          float s_cur = s_t;
-          double gain = fin.c[order];
-          for (int j = order - 1; j >= 1; --j) {
-            const double aj = fin.c[j];
-            Out w;
-            w.segs = 1;
-            w.gain = gain;
-            w.c = A32; w.beta = (float)-aj;
-            w.s1 = Mb[j & 1];
-            w.s1_scale = (j == 1) ? s_f : s_w;
-            w.s1_a = (float)(j == 1 ? fin.c[0] + aj : aj);
-            w.s1_b = 1.f;
-            rc = sym_product(Tcur, s_t, wcur, s_cur, w, 0);
+          QuadraticSteps fast;
+          if (interleave && quadratic_steps(fin, fast)) {
+            // Steps of Y = R^2 + beta R (see quadratic_steps): the product that makes Y writes its planes and those of W, an
+            // affine function of Y, at once.
+            __half* const Yp = Pb[1];
+            const float s_y = plane_scale(1.0 + std::fabs(fast.beta));
+            int left = (int)fast.lin.size() + (fast.by_r ? 1 : 0);   // products after this one; the last writes Mb[1]
+            auto target = [&]() { return Mb[(left & 1) ^ 1]; };
+            auto scale = [&](double bound) { return left == 0 ? s_f : plane_scale(std::max(1.0, bound)); };
+            double bound = std::fabs(fast.top) * (1.0 + std::fabs(fast.beta)) + std::fabs(fast.top0);
+            Out y;
+            y.segs = 1;
+            y.c = A32; y.beta = (float)-fast.beta;
+            y.s0 = Yp; y.s0_scale = s_y; y.s0_a = (float)fast.beta;
+            y.s1 = target(); y.s1_scale = scale(bound);
+            y.s1_a = (float)(fast.top * fast.beta + fast.top0); y.s1_b = (float)fast.top;
+            rc = sym_product(Tcur, s_t, Tcur, s_t, y, 0);
             if (rc) return rc;
-            wcur = w.s1;
-            s_cur = w.s1_scale;
-            gain = 1.0;
+            const __half* wcur = y.s1;
+            float s_cur = y.s1_scale;
+            auto step = [&](const __half* by, float s_by, double linear, double constant) {
+              --left;
+              bound = (1.0 + std::fabs(fast.beta)) * bound + std::fabs(linear) + std::fabs(constant);
+              Out w;
+              w.segs = 1;
+              if (linear != 0.0) {
+                w.c = A32; w.beta = (float)-linear;
+              }
+              w.s1 = target(); w.s1_scale = scale(bound);
+              w.s1_a = (float)(linear + constant); w.s1_b = 1.f;
+              const int err = sym_product(by, s_by, wcur, s_cur, w, 0);
+              wcur = w.s1;
+              s_cur = w.s1_scale;
+              return err;
+            };
+            if (fast.by_r) {
+              rc = step(Tcur, s_t, 0.0, fast.by_r_const);
+              if (rc) return rc;
+            }
+            for (auto it2 = fast.lin.rbegin(); it2 != fast.lin.rend(); ++it2) {
+              rc = step(Yp, s_y, it2->first, it2->second);
+              if (rc) return rc;
+            }
+          } else {
+            // Horner steps W_j = c_j R + R W_{j+1} (W_m = c_m R) build q(R) = c_0 I + W_1
+            const __half* wcur = Tcur;
+            float s_cur = s_t;
+            double gain = fin.c[order];
+            for (int j = order - 1; j >= 1; --j) {
+              const double aj = fin.c[j];
+              Out w;
+              w.segs = 1;
+              w.gain = gain;
+              w.c = A32; w.beta = (float)-aj;
+              w.s1 = Mb[j & 1];
+              w.s1_scale = (j == 1) ? s_f : s_w;
+              w.s1_a = (float)(j == 1 ? fin.c[0] + aj : aj);
+              w.s1_b = 1.f;
+              rc = sym_product(Tcur, s_t, wcur, s_cur, w, 0);
+              if (rc) return rc;
+              wcur = w.s1;
+              s_cur = w.s1_scale;
+              gain = 1.0;
+            }
           }
           float* R = root_lo + (long long)k0 * nn;
           Out o;

@@ -84,12 +84,12 @@ struct GemmParams {
   float aff_a, aff_b;
   unsigned int* maxres;   // per batch: max |[r==c] - d| as FP32 bits (distance of the result from the identity)
   // optional FP16 hi/lo operand planes of the result, ready to feed the next split-precision product:
-  //   S0: planes of s0_scale * d            S1: planes of s1_scale * (s1_aff_a * [r==c] + s1_aff_b * d)
+  //   S0: planes of s0_scale * (s0_aff_a * [r==c] + d)            S1: planes of s1_scale * (s1_aff_a * [r==c] + s1_aff_b * d)
   // hi plane at S + b * s_bs + r * s_ld + c, lo plane s_plane elements further
   __half* S0;
   __half* S1;
   long long s_ld, s_bs, s_plane;
-  float s0_scale, s1_scale, s1_aff_a, s1_aff_b;
+  float s0_scale, s0_aff_a, s1_scale, s1_aff_a, s1_aff_b;
   int* status;  // set non-zero if a bounded wait ran out
   unsigned long long* prof;  // optional: eight cycle counters summed over CTAs (see toner_gemm_phase_cycles)
   // 32 x 32 boxes of C and of the outputs, (columns, rows, batch): FP32 with 128-byte, 16-bit with 64-byte swizzle
@@ -375,7 +375,7 @@ __device__ __forceinline__ void epilogue_block(const GemmParams& p, const Epilog
       });
     }
   };
-  if (p.S0) planes(&p.s0_map, p.s0_scale, 0.f);
+  if (p.S0) planes(&p.s0_map, p.s0_scale, c0 == row_first ? p.s0_scale * p.s0_aff_a : 0.f);
   if (p.S1) planes(&p.s1_map, p.s1_scale * p.s1_aff_b, c0 == row_first ? p.s1_scale * p.s1_aff_a : 0.f);
 }
 
@@ -416,7 +416,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
         if (e.Db) e.Db[p.packed ? packed_off(row, col, p.N) : (long long)row * p.ldd + col] = v;
         if (e.Hb) e.Hb[(long long)row * p.ld16 + col] = to_bits16(v, p.d16_fmt);
         const float dg = (col == row) ? 1.f : 0.f;
-        if (e.S0b) store_split1(e.S0b + (long long)row * p.s_ld + col, p.s_plane, p.s0_scale * v);
+        if (e.S0b) store_split1(e.S0b + (long long)row * p.s_ld + col, p.s_plane, p.s0_scale * (v + p.s0_aff_a * dg));
         if (e.S1b) store_split1(e.S1b + (long long)row * p.s_ld + col, p.s_plane, p.s1_scale * fmaf(p.s1_aff_b, v, p.s1_aff_a * dg));
         t.mres = isfinite(v) ? fmaxf(t.mres, fabsf(dg - v)) : INFINITY;  // a non-finite result must not pass as converged
         const float w = (p.tri && col > row) ? 2.f : 1.f;
@@ -459,12 +459,10 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 // pair tiles take in 44 B per clock and SM whatever the tile (736 cycles per k-block of 256 x 256, 1100 of 256 x 512, against
 // 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.  Measured
 // plane by plane / interleaved: 12 x 3072^3 symmetric 1002 / 736 us (1.53 PFLOP/s), 6 x 5632^3 symmetric 3096 / 2145 us.
-// The cross products of a k-block go into the accumulator before its hi product.  Truncation (one unit of the accumulator's
-// last place per addition, so in proportion to the sum so far): with H the sum a hi k-block adds, four additions of either
-// kind per k-block and N k-blocks, plane by plane loses (2 N^2 + 8 N^2) H units, interleaved about 6 N^2 H; of chains of c
-// k-blocks (hi only; the cross products in chains of their own) it loses 2 c + 1/2 a k-block, of c interleaved ones 6 c - 3.5.
-// The host therefore turns a chain of c into one of (c + 2) / 3, which loses no more.  (GemmParams::segs is 1 here: the
-// three products are one.)
+// The cross products of a k-block go into the accumulator before its hi product.  In a chained product they now share the
+// chains, which the host shortens from c k-blocks to (2 c + 1) / 3 so that no error grows: against FP64 at 2048^3, chains
+// of 2 plane by plane 4.1e-7, of 1 interleaved 1.7e-7; of 8 2.4e-6, of 5 interleaved 1.9e-6 (random signs 1.5e-6 and 1.4e-6);
+// one chain 1.8e-5 and 1.5e-5.  (GemmParams::segs is 1 here: the three products are one.)
 template <int BN, bool kChained, bool kPair = false, bool kInter = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair, kInter>;

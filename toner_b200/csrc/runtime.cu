@@ -348,7 +348,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   p.M = d.m; p.N = d.n; p.K = d.k; p.batch = d.batch;
   p.fmt = d.fmt;
   p.tri = d.tri ? 1 : 0;
-  p.promote = d.promote > 0 ? (inter ? (d.promote + 2) / 3 : d.promote) : 0;   // (see gemm_tcgen05_kernel)
+  p.promote = d.promote > 0 ? (inter ? (2 * d.promote + 1) / 3 : d.promote) : 0;   // (see gemm_tcgen05_kernel)
   p.promote_all = d.promote_all ? 1 : 0;
   p.raster = d.tri ? 0 : (d.raster > 0 ? d.raster : (bn == 512 ? 4 : 8));   // (a group of 2048 columns)
   p.alpha = d.alpha; p.beta = d.beta;
@@ -374,7 +374,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   }
   p.S0 = static_cast<__half*>(d.split0); p.S1 = static_cast<__half*>(d.split1);
   p.s_ld = d.split_ld; p.s_bs = d.split_bs; p.s_plane = d.split_plane;
-  p.s0_scale = d.split0_scale; p.s1_scale = d.split1_scale; p.s1_aff_a = d.split1_aff_a; p.s1_aff_b = d.split1_aff_b;
+  p.s0_scale = d.split0_scale; p.s0_aff_a = d.split0_aff_a; p.s1_scale = d.split1_scale; p.s1_aff_a = d.split1_aff_a; p.s1_aff_b = d.split1_aff_b;
   p.maxres = d.maxres;
   p.sumsq = d.sumsq; p.maxabs = d.maxabs; p.maxaff = d.maxaff;
   p.aff_a = d.aff_a; p.aff_b = d.aff_b;
