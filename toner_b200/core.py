@@ -18,7 +18,7 @@ from __future__ import annotations
 
 import ctypes
 import math
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
 import torch
@@ -31,12 +31,21 @@ class Scratch:
 
     def __init__(self) -> None:
         self._buffers: Dict[Tuple, torch.Tensor] = {}
+        # The stream whose memory pool buffers come from, where another one is current (see Lanes: work on a lane begins after
+        # this stream's and is waited for by it, so the pool's order of reuse holds).
+        self.home: Optional[torch.cuda.Stream] = None
+
+    def _empty(self, shape, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+        if self.home is None:
+            return torch.empty(shape, dtype=dtype, device=device)
+        with torch.cuda.stream(self.home):
+            return torch.empty(shape, dtype=dtype, device=device)
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype, device: torch.device) -> torch.Tensor:
         key = (name, tuple(shape), dtype, str(device))
         buf = self._buffers.get(key)
         if buf is None:
-            buf = torch.empty(tuple(shape), dtype=dtype, device=device)
+            buf = self._empty(tuple(shape), dtype, device)
             self._buffers[key] = buf
         return buf
 
@@ -45,9 +54,47 @@ class Scratch:
         key = (name, "bytes", str(device))
         buf = self._buffers.get(key)
         if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            buf = self._empty(nbytes, torch.uint8, device)
             self._buffers[key] = buf
         return buf
+
+
+class Lanes:
+    """Independent pieces of work side by side on a few streams, lane 0 being the stream that is current.  A small group's
+    products leave a good part of their last wave empty and its vector kernels most of the SMs; another group's work fills
+    them.  Work that runs side by side shares no scratch, so the pieces' scratch (`scratch_bytes`, one number a piece) adds
+    up where it was the largest alone before: above 4 GiB more there is one lane -- and problems that large fill the GPU."""
+
+    def __init__(self, device: torch.device, scratch_bytes: Sequence[int], priority: int = 0) -> None:
+        lanes = min(3, len(scratch_bytes)) if sum(scratch_bytes) - max(scratch_bytes, default=0) <= 4 << 30 else 1
+        self.streams = [torch.cuda.Stream(device=device, priority=priority) for _ in range(lanes - 1)]
+        self.scratch = [Scratch() for _ in range(max(lanes, 1))]
+
+    def of(self, i: int) -> int:
+        """The lane of piece i."""
+        return i % len(self.scratch)
+
+    def run(self, jobs: Sequence[Tuple[int, Callable[[Scratch], None]]]) -> None:
+        """Every (i, job): job(scratch of i's lane), on that lane.  The current stream then waits for all of them."""
+        by_lane: Dict[int, list] = {}
+        for i, job in jobs:
+            by_lane.setdefault(self.of(i), []).append(job)
+        others = [lane for lane in by_lane if lane]
+        if others:
+            current = torch.cuda.current_stream()
+            ready = current.record_event()
+        try:
+            for lane in others:
+                self.scratch[lane].home = current
+                with torch.cuda.stream(self.streams[lane - 1]):
+                    self.streams[lane - 1].wait_event(ready)
+                    for job in by_lane[lane]:
+                        job(self.scratch[lane])
+            for job in by_lane.get(0, ()):
+                job(self.scratch[0])
+        finally:
+            for lane in others:
+                current.wait_stream(self.streams[lane - 1])
 
 
 def root_orders(strength_a: float, strength_b: float) -> Tuple[int, int]:

@@ -165,15 +165,18 @@ class FastTonerCore:
         self.check_every = int(getattr(args, "check_every", 0) or 0)
         self.check: Dict[str, Tuple[float, float, float]] = {}
         self.owner_of_layer = [r for r, c in enumerate(self.layer_counts) for _ in range(c)]
-        self.scratch = core.Scratch()
+        # factors of the two widths, and updates of the matrix shapes, side by side
+        self.factor_lanes = core.Lanes(device, [ops.inv_roots_workspace_bytes(c * self.per_layers, n) if self.per_layers else 0
+                                                for c, n in ((len(KINDS_D), hid), (1, mlp))], priority=-1)
         strengths = (float(args.inner_strength), float(args.outer_strength))
         damping = float(getattr(args, "damping", 1e-3))
         self.groups = {
             "d": StatGroup("d", [(i, k) for i in range(layers) for k in KINDS_D], hid, row_capacity,
                            [len(KINDS_D) * c for c in self.layer_counts], rank, world, device, strengths, damping,
-                           self.scratch),
+                           self.factor_lanes.scratch[0]),
             "f": StatGroup("f", [(i, "down") for i in range(layers)], mlp, row_capacity, list(self.layer_counts), rank,
-                           world, device, strengths, damping, self.scratch),
+                           world, device, strengths, damping,
+                           self.factor_lanes.scratch[self.factor_lanes.of(1)]),
         }
         self.weight = 0.0
         # matrices by role; the owned layers of a role form one MatrixGroup
@@ -239,6 +242,11 @@ class FastTonerCore:
                                         all_ptrs=ops.pointer_table(all_w))
                 part["roles"].append(role)
             self.parts.append(part)
+        merged: Dict[Tuple[int, ...], int] = {}
+        for info in self.roles.values():
+            merged[info["matrix"]] = merged.get(info["matrix"], 0) + self.per_layers
+        self.lanes = core.Lanes(device, [ops.ns_polar_workspace_bytes(c, *shape) if c and kind == "muont" else 0
+                                         for shape, c in merged.items()])
         self.t = 0
         self.steps = 0
         self.timing: Dict[str, float] = {}
@@ -392,8 +400,9 @@ class FastTonerCore:
         if self.pieces_done != self.row_pieces - 1:
             raise RuntimeError(f"{self.pieces_done + 1} of the step's {self.row_pieces} row pieces were captured")
         if self.world == 1 and self.row_pieces == 1:
-            for g in self.groups.values():
-                ops.syrk_upper(g.rows_buf, g.factors.ema, ops.EMA_FULL, b, gamma)   # SYRK with the EMA fused
+            self.factor_lanes.run([   # SYRK with the EMA fused
+                (i, lambda _, g=g: ops.syrk_upper(g.rows_buf, g.factors.ema, ops.EMA_FULL, b, gamma))
+                for i, g in enumerate(self.groups.values())])
         elif self.world == 1:
             for g in self.groups.values():
                 self._partial_grams(g, 0)
@@ -470,8 +479,7 @@ class FastTonerCore:
             if ready is None:
                 self._stats()
                 self._ev[1].record(self.side)
-                for g in self.groups.values():
-                    g.factors.compute()
+                self.factor_lanes.run([(i, lambda _, g=g: g.factors.compute()) for i, g in enumerate(self.groups.values())])
             else:
                 self._stats_as_rows_arrive(ready)
                 self._ev[1].record(self.side)
@@ -484,8 +492,6 @@ class FastTonerCore:
     # ------------------------------------------------------------------ updates (main stream)
     @torch.no_grad()
     def step(self) -> None:
-        a = self.args
-        lr, wd = self.param_groups[0]["lr"], self.param_groups[0]["weight_decay"]
         if self._ev_last is not None and self._ev_last[3].query():
             e = self._ev_last
             self.gpu_ms = {"stats": e[0].elapsed_time(e[1]), "roots": e[1].elapsed_time(e[2]),
@@ -513,22 +519,8 @@ class FastTonerCore:
             by_shape: Dict[Tuple[int, ...], List[str]] = {}
             for role in part["roles"]:
                 by_shape.setdefault(self.roles[role]["matrix"], []).append(role)
-            for shape, names in by_shape.items():
-                infos = [self.roles[r] for r in names]
-                if infos[0]["group"] is not None:
-                    grads = [[p.grad for p in info["group"].weights] for info in infos]
-                    if self.kind == "muont":
-                        core.muont_groups_delta([info["group"] for info in infos], grads, [info["delta"] for info in infos],
-                                                self.scratch, lr=lr, weight_decay=wd, momentum=float(a.momentum),
-                                                nesterov=bool(a.nesterov), ns_steps=int(a.ns_steps),
-                                                ns_eps=float(a.ns_eps))
-                    else:
-                        for info, gr in zip(infos, grads):
-                            core.adamt_group_delta(info["group"], gr, info["delta"], self.scratch, lr=lr, weight_decay=wd,
-                                                   betas=(float(a.beta1), float(a.beta2)), eps=float(a.eps), t=self.t)
-                if self.world == 1:
-                    for info in infos:
-                        ops.apply_delta(info["all_ptrs"], info["delta"])
+            self.lanes.run([(i, lambda scratch, names=names: self._update_shape(names, scratch))
+                            for i, names in enumerate(by_shape.values())])
             if self.world > 1:   # this part's changes travel while the next part is computed
                 if self.uneven:
                     works.append(dist.all_gather(part["gathered"], part["delta"], group=self.pg, async_op=True))
@@ -556,6 +548,25 @@ class FastTonerCore:
         self._ev_last = self._ev
         self.steps += 1
         self.timing.update(roots_host=t1 - t0, update_host=time.perf_counter() - t1)
+
+    def _update_shape(self, names: Sequence[str], scratch: core.Scratch) -> None:
+        """The update of the owned matrices of one shape."""
+        a = self.args
+        lr, wd = self.param_groups[0]["lr"], self.param_groups[0]["weight_decay"]
+        infos = [self.roles[r] for r in names]
+        if infos[0]["group"] is not None:
+            grads = [[p.grad for p in info["group"].weights] for info in infos]
+            if self.kind == "muont":
+                core.muont_groups_delta([info["group"] for info in infos], grads, [info["delta"] for info in infos],
+                                        scratch, lr=lr, weight_decay=wd, momentum=float(a.momentum),
+                                        nesterov=bool(a.nesterov), ns_steps=int(a.ns_steps), ns_eps=float(a.ns_eps))
+            else:
+                for info, gr in zip(infos, grads):
+                    core.adamt_group_delta(info["group"], gr, info["delta"], scratch, lr=lr, weight_decay=wd,
+                                           betas=(float(a.beta1), float(a.beta2)), eps=float(a.eps), t=self.t)
+        if self.world == 1:
+            for info in infos:
+                ops.apply_delta(info["all_ptrs"], info["delta"])
 
     def zero_grad(self, set_to_none: bool = True) -> None:
         for p in self.params:

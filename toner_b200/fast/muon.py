@@ -13,7 +13,7 @@ from typing import Dict, List, Tuple
 
 import torch
 
-from .. import ops
+from .. import core, ops
 
 
 class Muon(torch.optim.Optimizer):
@@ -36,6 +36,7 @@ class Muon(torch.optim.Optimizer):
                              and dist.get_world_size() > 1) else None
         self.precond = None   # optional (p, grad) -> preconditioned gradient, as in the reference
         self._stacks: Dict[Tuple[int, Tuple[int, int]], dict] = {}
+        self._lanes = None   # streams the shapes run on side by side (created at the first step)
 
     def _stack(self, gi: int, shape: Tuple[int, int], members: List[torch.nn.Parameter]) -> dict:
         """Momentum buffers of one shape live in one (count, rows, cols) stack; state[p]['momentum_buffer'] are views."""
@@ -59,7 +60,6 @@ class Muon(torch.optim.Optimizer):
         if closure is not None:
             raise ValueError("Muon.step() takes no closure")
         for gi, g in enumerate(self.param_groups):
-            mu, lr, wd = g["momentum"], g["lr"], g["weight_decay"]
             by_shape: Dict[Tuple[int, int], List[torch.nn.Parameter]] = {}
             for p in g["params"]:
                 if p.grad is None:
@@ -69,6 +69,12 @@ class Muon(torch.optim.Optimizer):
                 if p.grad.is_sparse:
                     raise RuntimeError("Muon does not support sparse gradients")
                 by_shape.setdefault(tuple(p.shape), []).append(p)
+            if not by_shape:
+                continue
+            if self._lanes is None:
+                self._lanes = core.Lanes(next(iter(by_shape.values()))[0].device,
+                                         [ops.ns_polar_workspace_bytes(len(ms), *shape) for shape, ms in by_shape.items()])
+            jobs = []
             for shape, members in by_shape.items():
                 st = self._stack(gi, shape, members)
                 grads = [p.grad if self.precond is None else self.precond(p, p.grad) for p in members]
@@ -76,20 +82,28 @@ class Muon(torch.optim.Optimizer):
                 key = tuple(x.data_ptr() for x in grads)
                 if st["grad_key"] != key:
                     st["grad_ptrs"], st["grad_key"] = ops.pointer_table(grads), key
-                ops.muont_momentum(st["grad_ptrs"], st["buf"], st["u"], mu, bool(g["nesterov"]), None)
-                u = st["u"] if g["nesterov"] else st["buf"]
-                if self.dist is None:
-                    o = ops.ns_polar(u, g["ns_steps"], g["eps"], out=st["u"])
-                else:   # rank r takes matrices r, r + W, ...; padded to equal shares for the all-gather
-                    world, rank = self.dist.get_world_size(), self.dist.get_rank()
-                    count = len(members)
-                    per = -(-count // world)
-                    mine = torch.zeros((per,) + shape, device=u.device)
-                    own = u[rank::world]
-                    mine[: own.shape[0]].copy_(own)
-                    ops.ns_polar(mine, g["ns_steps"], g["eps"], out=mine)
-                    gathered = torch.empty((world, per) + shape, device=u.device)
-                    self.dist.all_gather_into_tensor(gathered, mine)
-                    o = gathered.transpose(0, 1).reshape((per * world,) + shape)[:count].contiguous()
-                ops.apply_scaled(st["weights"], o, 1.0 - lr * wd, -lr * max(1.0, shape[0] / shape[1]) ** 0.5)
+                st["grads"] = grads      # (a converted copy lives until the next step's)
+                jobs.append(lambda scratch, st=st, shape=shape: self._step_shape(g, shape, st, scratch))
+            # (collectives keep one order on every rank)
+            self._lanes.run([(i if self.dist is None else 0, job) for i, job in enumerate(jobs)])
         return None
+
+    def _step_shape(self, g: dict, shape: Tuple[int, int], st: dict, scratch: core.Scratch) -> None:
+        mu, lr, wd = g["momentum"], g["lr"], g["weight_decay"]
+        ops.muont_momentum(st["grad_ptrs"], st["buf"], st["u"], mu, bool(g["nesterov"]), None)
+        u = st["u"] if g["nesterov"] else st["buf"]
+        count = st["buf"].shape[0]
+        if self.dist is None:
+            ws = scratch.bytes_like("ns", ops.ns_polar_workspace_bytes(count, *shape), u.device)
+            o = ops.ns_polar(u, g["ns_steps"], g["eps"], out=st["u"], workspace=ws)
+        else:   # rank r takes matrices r, r + W, ...; padded to equal shares for the all-gather
+            world, rank = self.dist.get_world_size(), self.dist.get_rank()
+            per = -(-count // world)
+            mine = torch.zeros((per,) + shape, device=u.device)
+            own = u[rank::world]
+            mine[: own.shape[0]].copy_(own)
+            ops.ns_polar(mine, g["ns_steps"], g["eps"], out=mine)
+            gathered = torch.empty((world, per) + shape, device=u.device)
+            self.dist.all_gather_into_tensor(gathered, mine)
+            o = gathered.transpose(0, 1).reshape((per * world,) + shape)[:count].contiguous()
+        ops.apply_scaled(st["weights"], o, 1.0 - lr * wd, -lr * max(1.0, shape[0] / shape[1]) ** 0.5)

@@ -67,8 +67,8 @@ class _Bucket:
     """Equally shaped parameters of one parameter group: one FactorSet entry and one stack row each."""
 
     def __init__(self, params: List[Tensor], strengths: Tuple[float, float], damping: float, kind: str,
-                 scratch: core.Scratch) -> None:
-        self.params = params
+                 lane: int, scratch: core.Scratch) -> None:
+        self.params, self.lane = params, lane
         n = params[0].shape[1]
         # AdamT divides by its second moments, which in the first steps turns the sign of a gradient element near zero into a
         # full step: there the factors keep the order of additions they have had (plane by plane), bit for bit.
@@ -96,7 +96,7 @@ class _TonerGeneral(Optimizer):
 
     def __init__(self, params, defaults) -> None:
         super().__init__(params, defaults)
-        self._scratch = core.Scratch()
+        self._lanes: Optional[core.Lanes] = None    # streams the buckets' work runs on side by side (created with them)
         self._buckets: Optional[Dict[Tuple, _Bucket]] = None
         self._bucket_of: Dict[Tensor, Tuple[_Bucket, int]] = {}
         self._finite_flag: Optional[Tensor] = None  # pinned word the finiteness check of the statistics reports to
@@ -123,15 +123,23 @@ class _TonerGeneral(Optimizer):
         self._buckets, self._bucket_of = {}, {}
         if self._health is None:
             self._health = ops.Health()
+        stacked: Dict[Tuple[int, Tuple[int, int]], List[Tensor]] = {}
         for gi, group in enumerate(self.param_groups):
-            by_shape: Dict[Tuple[int, int], List[Tensor]] = {}
+            core.root_orders(*self._strengths(group))
             for p in group["params"]:
                 if not p.is_contiguous():
                     raise ValueError("toner_b200 needs contiguous weights")
-                by_shape.setdefault(tuple(p.shape), []).append(p)
-            for shape, ps in by_shape.items():
-                core.root_orders(*self._strengths(group))
-                bucket = _Bucket(ps, self._strengths(group), group["damping"], self._kind, self._scratch)
+                stacked.setdefault((gi, tuple(p.shape)), []).append(p)
+        muont = self._kind == "muont"
+        self._lanes = core.Lanes(self.param_groups[0]["params"][0].device, [
+            ops.inv_roots_workspace_bytes(len(ps), shape[1]) + (ops.ns_polar_workspace_bytes(len(ps), *shape) if muont else 0)
+            for (_, shape), ps in stacked.items()])
+        for gi, group in enumerate(self.param_groups):
+            for (owner, shape), ps in stacked.items():
+                if owner != gi:
+                    continue
+                i = len(self._buckets)
+                bucket = _Bucket(ps, self._strengths(group), group["damping"], self._kind, i, self._lanes.scratch[self._lanes.of(i)])
                 self._buckets[(gi, shape)] = bucket
                 for i, p in enumerate(ps):
                     self._bucket_of[p] = (bucket, i)
@@ -260,8 +268,8 @@ class _TonerGeneral(Optimizer):
     def _factor_all(self, work) -> None:
         """Factors of every active bucket: enqueue all, then wait for their flags (and for the status of the previous
         step's update kernels, which finished before them)."""
-        for _, bucket in work:
-            bucket.factors.compute()
+        if work:
+            self._lanes.run([(bucket.lane, lambda _, f=bucket.factors: f.compute()) for _, bucket in work])
         for _, bucket in work:
             bucket.factors.finish()
         self._health.check()
@@ -325,15 +333,18 @@ class MuonT(_TonerGeneral):
         self._validate_muon()
         work = list(self._active_buckets())
         self._factor_all(work)
-        for group, bucket in work:
-            grads = [p.grad for p in bucket.params]
-            core.muont_group_delta(bucket.group, grads, bucket.delta, self._scratch, lr=group["lr"],
+
+        def update(group, bucket, scratch):
+            core.muont_group_delta(bucket.group, [p.grad for p in bucket.params], bucket.delta, scratch, lr=group["lr"],
                                    weight_decay=group["weight_decay"], momentum=group["momentum"],
                                    nesterov=group["nesterov"], ns_steps=group["ns_steps"], ns_eps=group["ns_eps"])
             core.apply_group_delta(bucket.group, bucket.delta)
-            for i, p in enumerate(bucket.params):
-                self.state[p]["momentum_buffer"] = bucket.group.m[i]
+
         if work:
+            self._lanes.run([(bucket.lane, lambda scratch, g=group, b=bucket: update(g, b, scratch)) for group, bucket in work])
+            for _, bucket in work:
+                for i, p in enumerate(bucket.params):
+                    self.state[p]["momentum_buffer"] = bucket.group.m[i]
             self._health.arm("the previous step's update")
         self._consume_statistics()
         return loss
@@ -388,20 +399,24 @@ class AdamT(_TonerGeneral):
         self._validate_adam()
         work = list(self._active_buckets())
         self._factor_all(work)
-        for group, bucket in work:
+
+        def update(group, bucket, scratch):
+            t = self.state[bucket.params[0]]["step"]
+            core.adamt_group_delta(bucket.group, [p.grad for p in bucket.params], bucket.delta, scratch, lr=group["lr"],
+                                   weight_decay=group["weight_decay"], betas=tuple(group["betas"]), eps=group["eps"], t=t)
+            core.apply_group_delta(bucket.group, bucket.delta)
+
+        for _, bucket in work:
             steps = {self.state[p].get("step", 0) for p in bucket.params}
             if len(steps) != 1:
                 raise RuntimeError("parameters stacked together must have taken the same number of steps")
             t = steps.pop() + 1
-            grads = [p.grad for p in bucket.params]
-            core.adamt_group_delta(bucket.group, grads, bucket.delta, self._scratch, lr=group["lr"],
-                                   weight_decay=group["weight_decay"], betas=tuple(group["betas"]), eps=group["eps"], t=t)
-            core.apply_group_delta(bucket.group, bucket.delta)
             for i, p in enumerate(bucket.params):
                 st = self.state[p]
                 st["step"] = t
                 st["exp_avg"], st["exp_avg_sq"] = bucket.group.m[i], bucket.group.v[i]
         if work:
+            self._lanes.run([(bucket.lane, lambda scratch, g=group, b=bucket: update(g, b, scratch)) for group, bucket in work])
             self._health.arm("the previous step's update")
         self._consume_statistics()
         return loss
