@@ -594,8 +594,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
 
   if (warp < 4) {
   ptx::reg_dec<48>();
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
+  if (warp == 0 || warp == 2) {
+    // ------------------------------------------------------------ TMA producers: warp 0 brings A, warp 2 brings B
+    // Issuing a copy holds its thread up until the copy engine takes it: one thread fills 32 KB stages every 496 cycles at
+    // best (copies alone, two of 16 KB each), two threads every 430 -- and beside the MMAs one thread needed 736.
+    const bool for_a = warp == 0;
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -634,14 +637,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           if constexpr (kPair) {
             // Both CTAs' copies report to the leader's barrier, which expects the bytes of the whole pair.
             const uint32_t lbar = ptx::mapa(full_bar(stage), 0);
-            if (leader) ptx::mbar_expect_tx(full_bar(stage), 2 * S::kStageBytes);
-            if (p.a_mn) {
+            if (for_a) {
+              if (leader) ptx::mbar_expect_tx(full_bar(stage), 2 * S::kStageBytes);
+              if (p.a_mn) {
 #pragma unroll
-              for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d_pair(sa + s * 8192, amap, lbar, m0 + s * 64, k0, za);
-            } else {
-              ptx::tma_load_3d_pair(sa, amap, lbar, k0, m0, za);
-            }
-            if constexpr (kWide) {
+                for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d_pair(sa + s * 8192, amap, lbar, m0 + s * 64, k0, za);
+              } else {
+                ptx::tma_load_3d_pair(sa, amap, lbar, k0, m0, za);
+              }
+            } else if constexpr (kWide) {
               if (p.b_mn) {
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
@@ -656,7 +660,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
             } else {
               ptx::tma_load_3d_pair(sb, bmap, lbar, k0, n0, zb);
             }
-          } else {
+          } else if (for_a) {
             ptx::mbar_expect_tx(full_bar(stage), S::kStageBytes);
             if (p.a_mn) {
 #pragma unroll
@@ -664,12 +668,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
             } else {
               ptx::tma_load_3d(sa, amap, full_bar(stage), k0, m0, za);
             }
-            if (p.b_mn) {
+          } else if (p.b_mn) {
 #pragma unroll
-              for (int s = 0; s < BN / 64; ++s) ptx::tma_load_3d(sb + s * 8192, bmap, full_bar(stage), n0 + s * 64, k0, zb);
-            } else {
-              ptx::tma_load_3d(sb, bmap, full_bar(stage), k0, n0, zb);
-            }
+            for (int s = 0; s < BN / 64; ++s) ptx::tma_load_3d(sb + s * 8192, bmap, full_bar(stage), n0 + s * 64, k0, zb);
+          } else {
+            ptx::tma_load_3d(sb, bmap, full_bar(stage), k0, n0, zb);
           }
           if (++stage == S::kStages) {
             stage = 0;
@@ -692,22 +695,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           }
         }
       }
-      if (p.prof && leader) atomicAdd(p.prof + 3, (unsigned long long)prof_wait);
+      if (p.prof && leader && for_a) atomicAdd(p.prof + 3, (unsigned long long)prof_wait);
       if (!ok || *abort_flag) {
         // Copies already issued must land before this CTA gives its shared memory back (the closing barrier waits
         // for threads, not for bulk copies).  Stage s was last filled in this round if s < stage, else in the round
         // before (a stage never filled is "complete" at once: its barrier has not left phase 0).  In a pair every
         // copy of both CTAs reports to the leader's barriers, so the leader waits for them; a barrier whose other
-        // half was never issued cannot complete, hence the bound.  Copies the leader cannot account for (the peer
-        // ran a few stages ahead of it) get a fixed settling time in both CTAs: a copy lands within microseconds.
+        // half was never issued cannot complete, hence the bound.  Copies this thread cannot account for (the peer or the
+        // other producer ran a few stages ahead of it) get a fixed settling time: a copy lands within microseconds.
         if (!kPair || leader) {
           for (int s = 0; s < S::kStages; ++s)
             ptx::mbar_wait(full_bar(s), (s < stage) ? phase : (phase ^ 1u), kDrainCycles);
         }
-        if constexpr (kPair) {
-          const long long t0 = clock64();
-          while (clock64() - t0 < kSettleCycles) {
-          }
+        const long long t0 = clock64();
+        while (clock64() - t0 < kSettleCycles) {
         }
       }
     }
