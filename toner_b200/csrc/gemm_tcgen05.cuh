@@ -249,17 +249,22 @@ __device__ __forceinline__ void stage_cols_16(uint32_t buf, int lane, const uint
   }
 }
 
-// A warp's ring of kBufs staged blocks.  Every acquired block ends in exactly one bulk group, committed in the order of
-// acquisition, so "all but the kBufs - 1 newest groups have been read" frees the block acquired kBufs acquisitions ago.
-template <int kBufs>
+// A warp's ring of staged blocks: `bufs` (at most three) of them.  Every acquired block ends in exactly one bulk group,
+// committed in the order of acquisition, so "all but the bufs - 1 newest groups have been read" frees the block acquired bufs
+// acquisitions ago.
 struct EpilogueRing {
   uint32_t base;
+  int bufs;
   int next = 0;
   __device__ __forceinline__ uint32_t acquire(int lane) {
-    if (lane == 0) ptx::bulk_wait_read<kBufs - 1>();
+    if (lane == 0) {
+      if (bufs == 3) ptx::bulk_wait_read<2>();
+      else if (bufs == 2) ptx::bulk_wait_read<1>();
+      else ptx::bulk_wait_read<0>();
+    }
     __syncwarp();
     const uint32_t buf = base + next * kEpiBlockBytes;
-    next = next + 1 == kBufs ? 0 : next + 1;
+    next = next + 1 == bufs ? 0 : next + 1;
     return buf;
   }
 };
@@ -267,8 +272,7 @@ struct EpilogueRing {
 // One block of the result: v holds alpha * accumulator of this lane's row on entry.  `held`: a block of the ring that is
 // already this block's own (C arrived in it), 0 if none.  `whole`: a diagonal block of a mirrored symmetric result; it is
 // made symmetric from its upper half and written once.
-template <int kBufs>
-__device__ __forceinline__ void epilogue_block(const GemmParams& p, const EpilogueTile& e, EpilogueRing<kBufs>& ring, float (&v)[32],
+__device__ __forceinline__ void epilogue_block(const GemmParams& p, const EpilogueTile& e, EpilogueRing& ring, float (&v)[32],
                                                uint32_t held, int b, int row_first, int c0, int lane, bool whole,
                                                EpilogueSums& t) {
   auto take = [&]() {
@@ -844,8 +848,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     const int lane_group = warp & 3;
     const int half = (warp - 4) >> 2;
     const int ew = warp - 4;
-    EpilogueRing<S::kEpiBufs> ring{base + S::kTileBytes + ew * S::kEpiBufs * kEpiBlockBytes};
-    uint32_t c_buf = 0, c_phase = 0;   // block of the ring C is arriving in (0: none), parity of its barrier
+    // With C the last of the warp's blocks is C's own, where there are several: the next block's C is then on its way while
+    // this block's results are staged (a 32 x 32 block of C, D and D16 took 4000 cycles with C fetched after them, 1500 of
+    // them the wait for it).  With one block only, C arrives where D will be staged.
+    const bool c_apart = S::kEpiBufs > 1 && p.C != nullptr;
+    const uint32_t warp_bufs = base + S::kTileBytes + ew * S::kEpiBufs * kEpiBlockBytes;
+    EpilogueRing ring{warp_bufs, c_apart ? S::kEpiBufs - 1 : S::kEpiBufs};
+    uint32_t c_buf = 0, c_phase = 0;   // block C is arriving in (0: none), parity of its barrier
     constexpr bool chained = kChained;
     // Running sums of the accumulation chains (chained products only), added with round-to-nearest: the
     // tensor core itself adds into its accumulator by truncation.
@@ -905,11 +914,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       // Boxes move by TMA unless an address or stride rules it out; a symmetric result that is not mirrored keeps its lower
       // triangle untouched, which a box across the diagonal would not.
       auto boxed = [&](int c0) { return p.tma_ok && !(p.tri && !p.mirror && c0 <= row_first + 31); };
-      // C of a block is fetched into the ring as soon as the block before it has been staged -- of the tile's first block,
-      // while the accumulator is still being formed.
+      // C of a block is fetched as soon as its place is free -- of the tile's first block, while the accumulator is still
+      // being formed.
       auto fetch_c = [&](int cc) {
         if (!e.use_c || cc >= cc_end || !boxed(col_first + cc * 32)) return;
-        c_buf = ring.acquire(lane);
+        c_buf = c_apart ? warp_bufs + (S::kEpiBufs - 1) * kEpiBlockBytes : ring.acquire(lane);
         if (lane == 0) {
           ptx::mbar_expect_tx(c_bar(ew), kEpiBlockBytes);
           ptx::tma_load_3d(c_buf, &p.c_map, c_bar(ew), col_first + cc * 32, row_first, b);
@@ -1043,7 +1052,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         if (chained || p.splits == 1) take_block(cc, v);
         else add_parts(cc, v);
         if (boxed(c0)) {
-          const uint32_t held = c_buf;
+          uint32_t held = c_buf;
           if (held) {
             const bool got = __all_sync(0xffffffffu, ptx::mbar_wait(c_bar(ew), c_phase, kWaitCycles) ? 1 : 0);
             if (!got || *abort_flag) {
@@ -1065,12 +1074,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
               v[4 * j + 2] = fmaf(e.beta, r[j].z, e.alpha * v[4 * j + 2]);
               v[4 * j + 3] = fmaf(e.beta, r[j].w, e.alpha * v[4 * j + 3]);
             }
-            __syncwarp();   // every lane has its row of C: the block is free for the result
+            __syncwarp();   // every lane has its row of C: the block is free
+            if (c_apart) {
+              held = 0;
+              fetch_c(cc + 1);
+            }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] *= e.alpha;
           }
-          epilogue_block<S::kEpiBufs>(p, e, ring, v, held, b, row_first, c0, lane, p.tri && p.mirror && c0 == row_first, sums);
+          epilogue_block(p, e, ring, v, held, b, row_first, c0, lane, p.tri && p.mirror && c0 == row_first, sums);
         } else {
           const uint32_t buf = ring.acquire(lane);
           stage_rows_f32(buf, lane, v);
@@ -1083,7 +1096,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           epilogue_block_scalar(p, e, reinterpret_cast<float*>(smem + (buf - base)), row_first, c0, lane, sums);
           if (lane == 0) ptx::bulk_commit();   // (nothing in flight: the ring counts one group per block)
         }
-        fetch_c(cc + 1);
+        if (!c_buf) fetch_c(cc + 1);
       }
       if (!alive) break;
       if (!chained) {

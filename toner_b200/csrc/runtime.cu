@@ -220,7 +220,7 @@ static bool may_interleave(const toner_gemm_desc& d) {
 //   * the main loop is bound by shared memory (128 B per clock: operands written by TMA and read by the MMAs), 512 cycles
 //     per 64-deep k-block of 256 x 256 on a pair and of 128 x 128 on one CTA, 384 of 256 x 128 on a pair and of 128 x 64,
 //     768 of 128 x 256;
-//   * interleaved plane products bring two thirds of the operands: 256 x 256 stays bound by its MMAs, 256 x 128 takes 320;
+//   * interleaved plane products bring two thirds of the operands: 256 x 256 stays bound by its MMAs, 256 x 128 takes 500;
 //   * a 32 x 32 block of the epilogue takes a warp 900 cycles plus 450 per box moved, and its boxes take shared memory away
 //     from the main loop of the next tile;
 //   * tiles of one wave run side by side, and the epilogue of one tile beside the main loop of the next.
@@ -232,7 +232,7 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
     bool pair;
     double per_kb, per_kb_inter;
   };
-  static const Config configs[] = {{256, true, 512, 512}, {128, true, 384, 320}, {256, false, 768, 768}, {128, false, 512, 512}, {64, false, 384, 384}};
+  static const Config configs[] = {{256, true, 512, 512}, {128, true, 384, 500}, {256, false, 768, 768}, {128, false, 512, 512}, {64, false, 384, 384}};
   const bool inter = may_interleave(d);
   const bool mirror = d.tri && d.mirror;
   const double boxes = (d.c ? 1.2 : 0.0) + (d.d ? (mirror && !d.upper_d ? 2.0 : 1.0) : 0.0) + (d.d16 ? (mirror ? 1.6 : 1.0) : 0.0) +
