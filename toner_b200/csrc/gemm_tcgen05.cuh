@@ -464,9 +464,11 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 // 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.  Measured
 // plane by plane / interleaved: 12 x 3072^3 symmetric 1002 / 736 us (1.53 PFLOP/s), 6 x 5632^3 symmetric 3096 / 2145 us.
 // The cross products of a k-block go into the accumulator before its hi product.  In a chained product they now share the
-// chains, which the host shortens from c k-blocks to (2 c + 1) / 3 so that no error grows: against FP64 at 2048^3, chains
-// of 2 plane by plane 4.1e-7, of 1 interleaved 1.7e-7; of 8 2.4e-6, of 5 interleaved 1.9e-6 (random signs 1.5e-6 and 1.4e-6);
-// one chain 1.8e-5 and 1.5e-5.  (GemmParams::segs is 1 here: the three products are one.)
+// chains, which the host therefore makes shorter than c k-blocks, except c = 2 (see the MMA loop), so that no error grows:
+// against FP64 at 2048^3, chains of 2 plane by plane and interleaved 4.1e-7; of 8 plane by plane 2.4e-6, of 5 interleaved
+// 1.9e-6 (random signs 3.4e-7, 1.5e-6 and 1.4e-6); one chain 1.8e-5 and 1.5e-5.  18 x 2048^3, chains of 2: 780k cycles plane
+// by plane, 655k interleaved (and 767k in chains of one k-block, the other way to lose no more).  (GemmParams::segs is 1
+// here: the three products are one.)
 template <int BN, bool kChained, bool kPair = false, bool kInter = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair, kInter>;
@@ -797,27 +799,52 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
               phase ^= 1u;
             }
           };
-          for (int kb = kb_begin; kb < kb_end; ++kb) {
-            const uint32_t fresh = (kb != kb_begin) ? 1u : 0u;
-            const int st = stage;
-            const uint32_t first = operands(st, phase);
-            if (!ok) break;
-            advance();
-            if constexpr (kInter) {
-              const int st_hi = stage;
-              const uint32_t hi = operands(st_hi, phase);
+          // one stage's operands, and its index for release_stage
+          auto next_operands = [&](int& st) {
+            st = stage;
+            const uint32_t at = operands(st, phase);
+            if (ok) advance();
+            return at;
+          };
+          if constexpr (kInter) {
+            // In chains of two, the cross products of both k-blocks go into the accumulator before the hi products of either:
+            // they are added while it is still 2^-11 of what it becomes.  (Otherwise one k-block after the other: holding
+            // four stages until the hi products have been issued cost one-chain products 5 %.)
+            const bool pairs = kChained && p.promote == 2;
+            for (int kb = kb_begin; kb < kb_end; kb += pairs ? 2 : 1) {
+              const bool two = pairs && kb + 1 < kb_end;
+              int s_lo, s_hi, s_lo1, s_hi1 = 0;
+              const uint32_t lo = next_operands(s_lo), hi = ok ? next_operands(s_hi) : 0u;
               if (!ok) break;
-              advance();
-              multiply(hi, first, 0, fresh);   // Ah Bl
-              multiply(first, hi, 0, 1u);      // Al Bh
-              release_stage(st);
+              multiply(hi, lo, 0, kb != kb_begin ? 1u : 0u);   // Ah Bl
+              multiply(lo, hi, 0, 1u);                         // Al Bh
+              release_stage(s_lo);
+              uint32_t hi1 = 0;
+              if (two) {
+                const uint32_t lo1 = next_operands(s_lo1);
+                hi1 = ok ? next_operands(s_hi1) : 0u;
+                if (!ok) break;
+                multiply(hi1, lo1, 0, 1u);
+                multiply(lo1, hi1, 0, 1u);
+                release_stage(s_lo1);
+              }
               multiply(hi, hi, 0, 1u);
-              release_stage(st_hi);
-            } else {
-              multiply(first, first, 0, fresh);
+              release_stage(s_hi);
+              if (two) {
+                multiply(hi1, hi1, 0, 1u);
+                release_stage(s_hi1);
+              }
+            }
+          } else {
+            for (int kb = kb_begin; kb < kb_end; ++kb) {
+              const uint32_t fresh = (kb != kb_begin) ? 1u : 0u;
+              int st;
+              const uint32_t at = next_operands(st);
+              if (!ok) break;
+              multiply(at, at, 0, fresh);
               if constexpr (kWide) {
                 if (kb == kb_begin && !wait_drained(1)) break;
-                multiply(first, first, 1, fresh);
+                multiply(at, at, 1, fresh);
               }
               release_stage(st);
             }

@@ -348,7 +348,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   p.M = d.m; p.N = d.n; p.K = d.k; p.batch = d.batch;
   p.fmt = d.fmt;
   p.tri = d.tri ? 1 : 0;
-  p.promote = d.promote > 0 ? (inter ? (2 * d.promote + 1) / 3 : d.promote) : 0;   // (see gemm_tcgen05_kernel)
+  p.promote = d.promote > 0 ? (inter && d.promote > 2 ? (2 * d.promote + 1) / 3 : d.promote) : 0;   // (see gemm_tcgen05_kernel)
   p.promote_all = d.promote_all ? 1 : 0;
   p.raster = d.tri ? 0 : (d.raster > 0 ? d.raster : (bn == 512 ? 4 : 8));   // (a group of 2048 columns)
   p.alpha = d.alpha; p.beta = d.beta;
