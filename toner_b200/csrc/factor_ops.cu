@@ -560,12 +560,15 @@ constexpr int kMaxDeflate = 8;  // (init_planes_kernel keeps that many coefficie
 // The products of four slices (32 per lane) are summed in FP32 before they join the FP64 sums: conversions and FP64
 // additions run at a fraction of the FP32 rate, and with one per eight products they, not the pass over A, set the
 // pace.  R (the number of vectors, rounded up to even) is a template argument so that absent vectors cost nothing.
+// With eight vectors the sums alone are 96 registers and few warps fit: the next slice, of A in registers and of the
+// vectors in the other half of shared memory, is fetched while this one is multiplied (12 statistics of width 3072, eight
+// vectors: 262 -> 158 us a pass; two vectors 94 -> 75, at HBM's rate 69).
 constexpr int kBlockGemvRows = 32;
 template <int R>
-__global__ void __launch_bounds__(256) block_gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
+__global__ void __launch_bounds__(256, R <= 4 ? 2 : 1) block_gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
                                                          float* __restrict__ y, int n, int r, int vstride) {
   ptx::pdl_begin();
-  __shared__ float4 sv[R][64];
+  __shared__ float4 sv[2][R][64];
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * kBlockGemvRows + warp * 4;
@@ -581,24 +584,15 @@ __global__ void __launch_bounds__(256) block_gemv_kernel(const float* __restrict
       part[i][j] = 0.f;
     }
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  int slice = 0;
-  for (int c0 = 0; c0 < n; c0 += 256, ++slice) {
-    __syncthreads();  // the previous slice has been read
-    for (int i = threadIdx.x; i < R * 64; i += 256) {
-      const int j = i >> 6, col = c0 + (i & 63) * 4;
-      sv[j][i & 63] = (j < r && col < n) ? *reinterpret_cast<const float4*>(V + (long long)j * n + col) : zero;
-    }
-    __syncthreads();
-    const int ca = c0 + lane * 4, cb = ca + 128;
-    // this lane's eight columns of every vector, read from shared memory once for the warp's four rows (read per
-    // row, the shared-memory traffic is R times the traffic of A and sets the pace from four vectors on)
-    float4 x0[R], x1[R];
+  constexpr int kShare = (R * 64 + 255) / 256;   // elements of a vector slice a thread brings in
+  float4 vn[kShare], p0[4], p1[4];
+  auto fetch = [&](int c0) {
 #pragma unroll
-    for (int j = 0; j < R; ++j) {
-      x0[j] = sv[j][lane];
-      x1[j] = sv[j][lane + 32];
+    for (int q = 0; q < kShare; ++q) {
+      const int i = threadIdx.x + 256 * q, j = i >> 6, col = c0 + (i & 63) * 4;
+      vn[q] = (j < r && col < n) ? *reinterpret_cast<const float4*>(V + (long long)j * n + col) : zero;
     }
-    float4 p0[4], p1[4];
+    const int ca = c0 + lane * 4, cb = ca + 128;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = row0 + i;
@@ -606,12 +600,33 @@ __global__ void __launch_bounds__(256) block_gemv_kernel(const float* __restrict
       p0[i] = (row < n && ca < n) ? *reinterpret_cast<const float4*>(Ar + ca) : zero;
       p1[i] = (row < n && cb < n) ? *reinterpret_cast<const float4*>(Ar + cb) : zero;
     }
+  };
+  fetch(0);
+  int slice = 0;
+  for (int c0 = 0; c0 < n; c0 += 256, ++slice) {
+    float4 (&now)[R][64] = sv[slice & 1];   // (last read two slices ago, before the barrier of the slice between)
+#pragma unroll
+    for (int q = 0; q < kShare; ++q) {
+      const int i = threadIdx.x + 256 * q;
+      if (i < R * 64) now[i >> 6][i & 63] = vn[q];
+    }
+    float4 a0[4], a1[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      a0[i] = p0[i];
+      a1[i] = p1[i];
+    }
+    __syncthreads();
+    if (c0 + 256 < n) fetch(c0 + 256);
+    // a lane's eight columns of a vector are read from shared memory once for the warp's four rows (read per row, the
+    // shared-memory traffic is R times the traffic of A and sets the pace from four vectors on)
 #pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const float s0 = fmaf(p0[i].x, x0[j].x, fmaf(p0[i].y, x0[j].y, fmaf(p0[i].z, x0[j].z, p0[i].w * x0[j].w)));
-        const float s1 = fmaf(p1[i].x, x1[j].x, fmaf(p1[i].y, x1[j].y, fmaf(p1[i].z, x1[j].z, p1[i].w * x1[j].w)));
+    for (int j = 0; j < R; ++j) {
+      const float4 x0 = now[j][lane], x1 = now[j][lane + 32];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float s0 = fmaf(a0[i].x, x0.x, fmaf(a0[i].y, x0.y, fmaf(a0[i].z, x0.z, a0[i].w * x0.w)));
+        const float s1 = fmaf(a1[i].x, x1.x, fmaf(a1[i].y, x1.y, fmaf(a1[i].z, x1.z, a1[i].w * x1.w)));
         part[i][j] += s0 + s1;
       }
     }
@@ -681,23 +696,24 @@ __device__ __forceinline__ void block_sum_many(double (&acc)[K], double* part, d
   __syncthreads();
 }
 
-constexpr int kPairs = kMaxDeflate * (kMaxDeflate + 1) / 2;  // entries of a symmetric r x r matrix, r = 8
-__device__ __forceinline__ int pair_index(int i, int j) { return i * (i + 1) / 2 + j; }  // j <= i
+// entry (i, j), j <= i, of a symmetric matrix's lower triangle
+__device__ __forceinline__ int pair_index(int i, int j) { return i * (i + 1) / 2 + j; }
 
 // Cholesky-QR of the r vectors held in Y (r x n, vector-major): G = Y Y^T = L L^T (FP64), V = L^-1 Y.  `gram` holds G's
 // lower triangle (pair_index order) on entry.  A vector that is (numerically) a combination of the earlier ones comes out as
 // zero; its slot is seeded afresh by the next call.  L's columns are formed one after the other by the lanes of one warp (row
 // i of a column by lane i); the diagonal of `L` holds its reciprocal (zero for a dropped vector).
+template <int R>
 __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, const double* gram, double (*L)[kMaxDeflate]) {
   if (threadIdx.x < 32) {
     const int i = threadIdx.x;
-    double row[kMaxDeflate];
+    double row[R];
 #pragma unroll
-    for (int j = 0; j < kMaxDeflate; ++j) {
+    for (int j = 0; j < R; ++j) {
       const bool on = i < r && j <= i && j < r;
       double sum = on ? gram[pair_index(i, j)] : 0.0;
 #pragma unroll
-      for (int k = 0; k < kMaxDeflate; ++k)
+      for (int k = 0; k < R; ++k)
         if (k < j) sum -= row[k] * __shfl_sync(0xffffffffu, row[k], j);
       // lane j holds the pivot
       const double pivot = __shfl_sync(0xffffffffu, sum, j);
@@ -709,13 +725,13 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
   }
   __syncthreads();
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    double out[kMaxDeflate];
+    double out[R];
 #pragma unroll
-    for (int j = 0; j < kMaxDeflate; ++j) {
+    for (int j = 0; j < R; ++j) {
       if (j < r) {
         double sum = (double)Y[(long long)j * n + c];
 #pragma unroll
-        for (int i = 0; i < kMaxDeflate; ++i)
+        for (int i = 0; i < R; ++i)
           if (i < j) sum -= L[j][i] * out[i];
         out[j] = sum * L[j][j];
       } else {
@@ -723,7 +739,7 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
       }
     }
 #pragma unroll
-    for (int j = 0; j < kMaxDeflate; ++j)
+    for (int j = 0; j < R; ++j)
       if (j < r) V[(long long)j * n + c] = (float)out[j];
   }
   __syncthreads();
@@ -782,6 +798,7 @@ __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) 
 __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v, int n, int r, int vstride, int cold) {
   ptx::pdl_begin();
   __shared__ double red[8];
+  constexpr int kPairs = R * (R + 1) / 2;
   __shared__ double part[8 * kPairs], gram[kPairs];
   __shared__ double L[kMaxDeflate][kMaxDeflate];
   const int b = blockIdx.x;
@@ -799,28 +816,30 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
 #pragma unroll
   for (int i = 0; i < kPairs; ++i) acc[i] = 0.0;
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    double x[kMaxDeflate];
+    double x[R];
 #pragma unroll
-    for (int i = 0; i < kMaxDeflate; ++i) x[i] = i < r ? (double)V[(long long)i * n + c] : 0.0;
+    for (int i = 0; i < R; ++i) x[i] = i < r ? (double)V[(long long)i * n + c] : 0.0;
 #pragma unroll
-    for (int i = 0; i < kMaxDeflate; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += x[i] * x[j];
   }
   block_sum_many<kPairs>(acc, part, gram);
-  cholesky_orthonormalise(V, V, n, r, gram, L);
+  cholesky_orthonormalise<R>(V, V, n, r, gram, L);
 }
 
 // Rayleigh-Ritz on span(V) with Y = A V (V orthonormal): H = V Y^T, H = Q diag(theta) Q^T (Jacobi, FP64), V <- Q^T V,
 // Y <- Q^T Y (Ritz vectors, descending theta), res_j = ||Y_j - theta_j V_j|| / |theta_j|.  Unless this is the last sweep, V is
 // then replaced by the orthonormalised Y (one more step of the power iteration).  Three passes over the two blocks of
-// vectors; every reduction is taken for all pairs at once.
+// vectors; every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
+// vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2; now 17.
+template <int R>
 __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float* __restrict__ y, int n, int r, int vstride,
                                                    int last, float* __restrict__ theta, float* __restrict__ res) {
   ptx::pdl_begin();
-  constexpr int R = kMaxDeflate;
-  __shared__ double part[8 * R * R], sums[R * R];
-  __shared__ double H[R][R], Q[R][R], lam[R], L[R][R];
+  constexpr int kPairs = R * (R + 1) / 2, kSums = R * R > kPairs + R ? R * R : kPairs + R, kMost = kMaxDeflate;
+  __shared__ double part[8 * kSums], sums[kSums];
+  __shared__ double H[kMost][kMost], Q[kMost][kMost], lam[kMost], L[kMost][kMost];
   const int b = blockIdx.x;
   float* V = v + (long long)b * vstride * n;
   float* Y = y + (long long)b * vstride * n;
@@ -858,14 +877,14 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
       const double o = H[j][j];
       if (o > mine || (o == mine && j < i)) ++place;
     }
-    double col[R];
+    double col[kMost];
 #pragma unroll
-    for (int k = 0; k < R; ++k) col[k] = Q[k][i];
+    for (int k = 0; k < kMost; ++k) col[k] = Q[k][i];
     __syncwarp();
     if (threadIdx.x < r) {
       lam[place] = mine;
 #pragma unroll
-      for (int k = 0; k < R; ++k) Q[k][place] = col[k];
+      for (int k = 0; k < kMost; ++k) Q[k][place] = col[k];
     }
   }
   __syncthreads();
@@ -917,10 +936,10 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
   }
   if (threadIdx.x < r) {
     const double l = lam[threadIdx.x];
-    theta[b * R + threadIdx.x] = (float)l;
-    res[b * R + threadIdx.x] = l > 0.0 ? (float)(sqrt(sums[kPairs + threadIdx.x]) / l) : INFINITY;
+    theta[b * kMost + threadIdx.x] = (float)l;
+    res[b * kMost + threadIdx.x] = l > 0.0 ? (float)(sqrt(sums[kPairs + threadIdx.x]) / l) : INFINITY;
   }
-  if (!last) cholesky_orthonormalise(Y, V, n, r, sums, L);
+  if (!last) cholesky_orthonormalise<R>(Y, V, n, r, sums, L);
 }
 
 // Which of the r Ritz pairs are deflated: in descending order, as long as each has converged and stands above eight
@@ -1371,16 +1390,22 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       // dominant directions: block power iteration with Rayleigh-Ritz on the caller's vectors (eight sweeps from fixed
       // vectors -- the first three or four only find the subspace --, four from last call's), then deflate those that
       // converged and stand above the rest
-      TONER_LAUNCH(block_start_kernel, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0);
       const int sweeps = defl_cold ? 8 : 4;
-      for (int sw = 0; sw < sweeps; ++sw) {
-        const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
-        if (defl_r <= 2) TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
-        else if (defl_r <= 4) TONER_LAUNCH(block_gemv_kernel<4>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
-        else if (defl_r <= 6) TONER_LAUNCH(block_gemv_kernel<6>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
-        else TONER_LAUNCH(block_gemv_kernel<8>, bg, 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
-        TONER_LAUNCH(ritz_kernel, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
-      }
+      auto iterate = [&](auto width) -> int {   // (R as a type: every kernel of the iteration is specialised for it)
+        constexpr int R = decltype(width)::value;
+        TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0);
+        for (int sw = 0; sw < sweeps; ++sw) {
+          TONER_LAUNCH(block_gemv_kernel<R>, dim3((n + kBlockGemvRows - 1) / kBlockGemvRows, kc), 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+          TONER_LAUNCH(ritz_kernel<R>, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
+        }
+        return 0;
+      };
+      int rcd;
+      if (defl_r <= 2) rcd = iterate(std::integral_constant<int, 2>());
+      else if (defl_r <= 4) rcd = iterate(std::integral_constant<int, 4>());
+      else if (defl_r <= 6) rcd = iterate(std::integral_constant<int, 6>());
+      else rcd = iterate(std::integral_constant<int, 8>());
+      if (rcd) return rcd;
       TONER_LAUNCH(block_decide_kernel, (kc + 127) / 128, 128, stream, th8, res8, kc, n, defl_r, damping, p, ritz_norm ? defl_r - 1 : defl_r, coef8, corr8, deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx, rest_trace);
       if (!ritz_norm) {   // (with the norm estimate the deflation is applied where the operand planes are formed)
         TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, dv, coef8, n, defl_r, kMaxDeflate);
