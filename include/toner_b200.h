@@ -311,6 +311,16 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
                             int32_t track_sweeps, float* deflate, int32_t deflate_rank, int32_t* deflated_out,
                             void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same, and the operand planes of the roots with it: FP16 hi/lo planes (2, k, n, n) and k inverse scales of A^(-1/p)
+ * (lo_planes, lo_inv) and A^(-q/p) (hi_planes, hi_inv; q > 1), as toner_split16 with maxabs = 1.01 damping^(-1/p) or
+ * 1.01 damping^(-q/p) writes them, without its passes over the roots.  NULL: not wanted. */
+int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
+                           float lower, int32_t lower_is_estimate, float* root_lo, float* root_hi, float* fro2_lo,
+                           int32_t* status, float* norm_out, float* track, float* lmin_out, float* resid_out,
+                           int32_t track_sweeps, float* deflate, int32_t deflate_rank, int32_t* deflated_out,
+                           void* lo_planes, float* lo_inv, void* hi_planes, float* hi_inv, void* workspace,
+                           size_t workspace_bytes, void* stream);
+
 /* What a host reads after that call, written to HOST memory the device can address (pinned) by one kernel: status, norms,
  * lmin, deflated (k words each, in this order), then the status word of toner_status_snapshot: 4 k + 1 words. */
 int toner_factor_report(const int32_t* status, const float* norms, const float* lmin, const int32_t* deflated, int32_t k,

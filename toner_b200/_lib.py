@@ -99,6 +99,8 @@ SIGNATURES = {
     "toner_inv_roots_ex": (C.c_int, [_vp, _i32, _i32, _f32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "toner_inv_roots_tracked": (C.c_int, [_vp, _i32, _i32, _f32, _i32, _i32, _i32, _f32, _i32, _vp, _vp, _vp, _vp, _vp, _vp,
                                           _vp, _vp, _i32, _vp, _i32, _vp, _vp, _sz, _vp]),
+    "toner_inv_roots_planes": (C.c_int, [_vp, _i32, _i32, _f32, _i32, _i32, _i32, _f32, _i32, _vp, _vp, _vp, _vp, _vp, _vp,
+                                         _vp, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "toner_factor_report": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _vp, _vp]),
     "toner_ns_polar_workspace_bytes": (C.c_size_t, [_i32, _i32, _i32]),
     "toner_ns_polar": (C.c_int, [_vp, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _sz, _vp]),

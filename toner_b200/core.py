@@ -256,11 +256,12 @@ class FactorSet:
                       deflate=self.deflate if self.tracking and self.block_deflation else None,
                       deflate_rank=self.deflate_rank,
                       deflate_restart=self.track_restart, deflated=self.deflated if self.tracking else None,
-                      ritz_norm=ritz, interleave=self.interleave)
+                      ritz_norm=ritz, interleave=self.interleave, lo_planes=self.lo_planes, lo_inv=self.lo_inv,
+                      hi_planes=self.hi_planes if self.q > 1 else None, hi_inv=self.hi_inv if self.q > 1 else None)
         self.track_restart = False
         self._estimate_in_flight = self.lower_is_estimate
         self._lower_used = self.lower
-        self._split()
+        self._norm_hi()
         ops.factor_report(self.status, self.norms, self.lmin, self.deflated, self._host)
         self.status_event = torch.cuda.Event()
         self.status_event.record(torch.cuda.current_stream())
@@ -270,9 +271,14 @@ class FactorSet:
         self.lower, self.lower_is_estimate, self.track_restart, self.estimate_backoff = 0.0, False, True, 0
         self._warm_calls = 0
 
+    def _norm_hi(self) -> None:
+        if self.q > 1 and self.outer_strength != 0 and self._is_hi(self.outer_strength):   # (only the outer factor's norm is used)
+            ops.sumsq(self.root_hi, out=self.fro2_hi,
+                      scratch=self.scratch.bytes_like("sumsq", ops.sumsq_scratch_bytes(self.k), self.device))
+
     def _split(self) -> None:
-        # Operand planes of the roots, scaled by a bound known without a pass over them: the statistic is factored
-        # with damping added, so no entry of A^-s exceeds damping^-s.
+        # Operand planes of the roots after a repair (otherwise the engine writes them), scaled by a bound known without a
+        # pass over them: the statistic is factored with damping added, so no entry of A^-s exceeds damping^-s.
         if self._root_bounds is None:
             bits = lambda s: torch.full((self.k,), 1.01 * self.damping ** -s, device=self.device,
                                         dtype=torch.float32).view(torch.int32)
@@ -280,9 +286,7 @@ class FactorSet:
         ops.split16(self.root_lo, planes=self.lo_planes, inv_scale=self.lo_inv, maxabs=self._root_bounds[0])
         if self.q > 1:
             ops.split16(self.root_hi, planes=self.hi_planes, inv_scale=self.hi_inv, maxabs=self._root_bounds[1])
-            if self.outer_strength != 0 and self._is_hi(self.outer_strength):   # (only the outer factor's norm is used)
-                ops.sumsq(self.root_hi, out=self.fro2_hi,
-                          scratch=self.scratch.bytes_like("sumsq", ops.sumsq_scratch_bytes(self.k), self.device))
+        self._norm_hi()
 
     def finish(self) -> int:
         """Wait for the convergence flags only; recompute flagged statistics by eigendecomposition (the

@@ -795,6 +795,7 @@ __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) 
 
 // start vectors: the caller's vectors (warm), or r different fixed +-1 patterns (cold, and for a slot that holds
 // nothing yet because the rank grew since the last call), orthonormalised
+template <int R>
 __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v, int n, int r, int vstride, int cold) {
   ptx::pdl_begin();
   __shared__ double red[8];
@@ -1053,6 +1054,87 @@ __global__ void __launch_bounds__(256) rankr_update_kernel(float* __restrict__ a
   }
 }
 
+// The last pass over the roots: R_b += sum_j coef[b][j] v_bj v_bj^T as above, the partial sums of its squares (the grid, the
+// order of the additions and so the bits are sumsq_det's), and its FP16 hi/lo planes scaled by s (a power of two; planes ==
+// nullptr: none), the lo plane lo_step matrices behind the hi plane.  One read and two writes of the stack where the three
+// passes took four reads and two writes.  inv[b] <- 1 / s, inv2[b] <- 1 / s2.
+__global__ void __launch_bounds__(256) root_finish_kernel(float* __restrict__ a, const float* __restrict__ v,
+                                                          const float* __restrict__ coef, int n, int r, int vstride, int cstride,
+                                                          float s, __half* __restrict__ planes, int lo_step,
+                                                          float* __restrict__ inv, float s2, float* __restrict__ inv2,
+                                                          float* __restrict__ partial) {
+  ptx::pdl_begin();
+  const int b = blockIdx.y;
+  float cf[kMaxDeflate];
+  bool any = false;
+#pragma unroll
+  for (int j = 0; j < kMaxDeflate; ++j) {
+    cf[j] = j < r ? coef[b * cstride + j] : 0.f;
+    any = any || cf[j] != 0.f;
+  }
+  const long long nn = (long long)n * n;
+  float4* A = reinterpret_cast<float4*>(a + b * nn);
+  const float* V = v + (long long)b * vstride * n;
+  uint2* hi = reinterpret_cast<uint2*>(planes + b * nn);
+  uint2* lo = reinterpret_cast<uint2*>(planes + ((long long)lo_step + b) * nn);
+  const unsigned n4 = n / 4, total4 = (unsigned)(nn / 4);   // (n <= 65536)
+  const unsigned per = (total4 + gridDim.x - 1) / gridDim.x;
+  const unsigned first = per * blockIdx.x, last = min(first + per, total4);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (inv) inv[b] = 1.f / s;
+    if (inv2) inv2[b] = 1.f / s2;
+  }
+  auto finished = [&](unsigned i, float4 x) {
+    if (any) {
+      const unsigned row = i / n4, c = (i - row * n4) * 4;
+#pragma unroll
+      for (int j = 0; j < kMaxDeflate; ++j) {
+        if (cf[j] != 0.f) {
+          const float vr = V[(long long)j * n + row];
+          const float4 vc = *reinterpret_cast<const float4*>(V + (long long)j * n + c);
+          x.x = fmaf(cf[j], vr * vc.x, x.x); x.y = fmaf(cf[j], vr * vc.y, x.y);
+          x.z = fmaf(cf[j], vr * vc.z, x.z); x.w = fmaf(cf[j], vr * vc.w, x.w);
+        }
+      }
+      A[i] = x;
+    }
+    if (planes) {
+      const __half2 h0 = __floats2half2_rn(s * x.x, s * x.y), h1 = __floats2half2_rn(s * x.z, s * x.w);
+      const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+      const __half2 l0 = __floats2half2_rn(s * x.x - f0.x, s * x.y - f0.y), l1 = __floats2half2_rn(s * x.z - f1.x, s * x.w - f1.y);
+      hi[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+      lo[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+    }
+    return x;
+  };
+  float s0 = 0.f, s1 = 0.f, s2q = 0.f, s3 = 0.f;
+  auto square = [&](const float4 x) {
+    s0 = fmaf(x.x, x.x, s0); s1 = fmaf(x.y, x.y, s1); s2q = fmaf(x.z, x.z, s2q); s3 = fmaf(x.w, x.w, s3);
+  };
+  unsigned i = first + threadIdx.x;
+  for (; i + 768 < last; i += 1024) {
+    const float4 x0 = A[i], x1 = A[i + 256], x2 = A[i + 512], x3 = A[i + 768];
+    square(finished(i, x0)); square(finished(i + 256, x1)); square(finished(i + 512, x2)); square(finished(i + 768, x3));
+  }
+  for (; i < last; i += 256) square(finished(i, A[i]));
+  float t = (s0 + s1) + (s2q + s3);
+  __shared__ float red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float sum = 0.f;
+    for (int w = 0; w < 8; ++w) sum += red[w];
+    partial[(long long)b * gridDim.x + blockIdx.x] = sum;
+  }
+}
+__global__ void __launch_bounds__(32) root_norm_kernel(const float* __restrict__ partial, float* __restrict__ out) {
+  ptx::pdl_begin();
+  const float t = sumsq_total(partial + (long long)blockIdx.x * kSumsqBlocks, threadIdx.x);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
+}
+
 // With P = A' / ||A'||_F:  lambda_max(P) <= ||P^(2^j)||_F^(1 / 2^j) = (sum lambda^(2^(j+1)))^(1 / 2^(j+1))  for every j, and
 // the bound tightens with j (for a flat spectrum it is n^(-1/2) times n^(1/4), n^(1/8), n^(1/16) for j = 1, 2, 3).
 // bound^2 <- bound^2 * t^2 with t the smallest of the three, 3 % above it for the single-pass products' rounding.
@@ -1148,11 +1230,10 @@ __global__ void lmin_from_root_kernel(const float* __restrict__ theta, float pow
 // pass over the result.
 __global__ void finish_kernel(const unsigned int* __restrict__ resid, const float* __restrict__ sumsq_a,
                               float* root_scale_lo, int* status, float* norm_out, int k, int p, float tol, float damping,
-                              float lower_used, unsigned int* __restrict__ root_max_bits, float root_bound) {
+                              float lower_used) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
-  root_max_bits[b] = __float_as_uint(root_bound);
   const float ub = sqrtf(fmaxf(sumsq_a[b], 1e-60f));
   root_scale_lo[b] = powf(ub, -1.f / p);
   if (norm_out) norm_out[b] = ub;
@@ -1195,6 +1276,12 @@ static size_t small_bytes(int chunk, int n) {
 // for |x| <= bound, and elements down to 2^-16 of the bound keep all 22 bits of the hi/lo pair.
 static float plane_scale(double bound) {
   return (float)std::ldexp(1.0, (int)std::floor(std::log2(16384.0 / bound)));
+}
+// The scale toner_split16 gives a matrix whose largest entry is `bound`.
+static float root_plane_scale(double bound) {
+  int e;
+  std::frexp((float)bound, &e);
+  return (float)std::ldexp(1.0, 14 - e);
 }
 
 }  // namespace toner
@@ -1270,12 +1357,25 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
                             int32_t* status, float* norm_out, float* track, float* lmin_out, float* resid_out,
                             int32_t track_sweeps, float* deflate, int32_t deflate_rank, int32_t* deflated_out,
                             void* workspace, size_t workspace_bytes, void* stream_) {
+  return toner_inv_roots_planes(ema, k, n, damping, p, q, iters, lower, lower_is_estimate, root_lo, root_hi, fro2_lo, status, norm_out,
+                                track, lmin_out, resid_out, track_sweeps, deflate, deflate_rank, deflated_out, nullptr, nullptr,
+                                nullptr, nullptr, workspace, workspace_bytes, stream_);
+}
+
+int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
+                           float lower, int32_t lower_is_estimate, float* root_lo, float* root_hi, float* fro2_lo,
+                           int32_t* status, float* norm_out, float* track, float* lmin_out, float* resid_out,
+                           int32_t track_sweeps, float* deflate, int32_t deflate_rank, int32_t* deflated_out,
+                           void* lo_planes, float* lo_inv, void* hi_planes, float* hi_inv,
+                           void* workspace, size_t workspace_bytes, void* stream_) {
   using namespace toner;
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!ema || !root_lo || !workspace) return fail(kErrArg, "inv_roots: null pointer");
   if (k <= 0 || n <= 0) return fail(kErrArg, "inv_roots: sizes must be positive");
+  if (!lo_planes != !lo_inv || !hi_planes != !hi_inv || (hi_planes && q == 1))
+    return fail(kErrArg, "inv_roots: planes come with their inverse scales, the second root's only where there is one");
   if (n % 8 != 0) return fail(kErrUnsupported, "inv_roots: n must be a multiple of 8");
   if (!(damping > 0.f)) return fail(kErrArg, "inv_roots: damping must be positive");
   if (p < 1 || p > 32 || (p & (p - 1))) return fail(kErrUnsupported, "inv_roots: root order p must be a power of two <= 32");
@@ -1359,7 +1459,6 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
     float* neg_sigma = small(7);
     float* corr = small(8);
     float* inv_r = small(9);
-    unsigned int* max_r = reinterpret_cast<unsigned int*>(small(10));
     float* ss2 = small(11);
     float* ss4 = small(12);
     float* ss8 = small(13);
@@ -1492,18 +1591,21 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       __half* s0 = nullptr; float s0_scale = 0.f, s0_a = 0.f;
       __half* s1 = nullptr; float s1_scale = 0.f, s1_a = 0.f, s1_b = 0.f;
       unsigned int* maxres = nullptr;
+      int lo_step = 0;              // s0: matrices between its hi and lo planes (0: the chunk's)
       const float* c = nullptr; float beta = 0.f;  // result = gain * product + beta * c (c symmetric, FP32)
       double gain = 1.0;
       int segs = 3;                                // 1: hi planes only (a single pass)
     };
-    auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote) -> int {
+    // (in_step: matrices between the hi and lo planes of the operands; 0: the chunk's)
+    auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote, int in_step = 0) -> int {
       toner_gemm_desc g = {};
       toner_operand op = {};
-      op.rows = n; op.cols = n; op.ld = n; op.z_stride = nn; op.nz = 2 * kc; op.z_step = 1;
+      const int lo = in_step ? in_step : kc;
+      op.rows = n; op.cols = n; op.ld = n; op.z_stride = nn; op.nz = lo + kc; op.z_step = 1;
       g.a = op; g.a.base = ap;
       g.b = op; g.b.base = bp;
-      g.a.seg_z[0] = 0; g.a.seg_z[1] = 0; g.a.seg_z[2] = kc;   // Ah Ah Al
-      g.b.seg_z[0] = 0; g.b.seg_z[1] = kc; g.b.seg_z[2] = 0;   // Bh Bl Bh
+      g.a.seg_z[0] = 0; g.a.seg_z[1] = 0; g.a.seg_z[2] = lo;   // Ah Ah Al
+      g.b.seg_z[0] = 0; g.b.seg_z[1] = lo; g.b.seg_z[2] = 0;   // Bh Bl Bh
       g.m = n; g.n = n; g.k = n; g.batch = kc; g.segs = o.segs; g.fmt = 0;
       g.tri = 1; g.mirror = 1;
       g.alpha = (float)(o.gain / ((double)sa * (double)sb));
@@ -1513,13 +1615,17 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
       g.d = o.d; g.ldd = n; g.d_bs = nn;
       g.split0 = o.s0; g.split0_scale = o.s0_scale; g.split0_aff_a = o.s0_a;
       g.split1 = o.s1; g.split1_scale = o.s1_scale; g.split1_aff_a = o.s1_a; g.split1_aff_b = o.s1_b;
-      g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)kc * nn;
+      g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)(o.lo_step ? o.lo_step : kc) * nn;
       g.maxres = o.maxres;
       g.promote = promote;
       g.interleave = interleave ? 1 : 0;
       return launch_gemm(g, stream);
     };
     int rc = 0;
+    __half* root_planes = nullptr;   // of A^{-1/p}, root_step matrices between hi and lo
+    int root_step = 0;
+    const float s_root = root_plane_scale(root_bound);
+    const float s_hi = root_plane_scale(1.01 * std::pow((double)damping, -(double)q / p));
     // X_1 = T_0, read by both chains until the first product with X; the next T goes to T's own buffer
     const __half* Xcur = Xb[1];
     const __half* Tcur = Xb[1];
@@ -1533,7 +1639,7 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         x_bound = std::min(x_bound * sched[it].a, x_cap);
         if (last) {
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping, lower_used, max_r, (float)root_bound);
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping, lower_used);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
@@ -1609,17 +1715,19 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
           o.alpha_a = scale_lo;
           rc = sym_product(Xcur, s_x, Mb[1], s_f, o, kPromoteX);
           if (rc) return rc;
-          // put the deflated direction back: A^{-1/p} = A'^{-1/p} + (lambda_1^{-1/p} - c^{-1/p}) v v^T
-          if (defl_r > 0) TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, R, dv, corr8, n, defl_r, kMaxDeflate);
-          else TONER_LAUNCH(rank1_update_kernel, dim3(ew_blocks, kc), 256, stream, R, pv, corr, n);
-          TONER_CUDA(cudaGetLastError());
-          rc = sumsq_det(R, kc, n, n, n, nn, partials, fro_tmp, stream);
-          if (rc) return rc;
-          if (q > 1) {  // operand planes of the finished root for the squarings below
-            rc = split16(R, nullptr, kc, n, n, n, nn, 0.f, 1.f, max_r, nullptr, Xb[xi], inv_r, stream);
-            if (rc) return rc;
+          // put the deflated directions back: A^{-1/p} = A'^{-1/p} + (lambda_1^{-1/p} - c^{-1/p}) v v^T; with that the root's
+          // norm and its operand planes, for the squarings below and for the caller
+          if (lo_planes) {
+            root_planes = static_cast<__half*>(lo_planes) + (long long)k0 * nn;
+            root_step = k;
+          } else if (q > 1) {
+            root_planes = Xb[xi];
           }
-          Xcur = Xb[xi];
+          TONER_LAUNCH(root_finish_kernel, dim3(kSumsqBlocks, kc), 256, stream, R, defl_r > 0 ? dv : pv, defl_r > 0 ? corr8 : corr, n,
+                       defl_r > 0 ? defl_r : 1, defl_r > 0 ? kMaxDeflate : 1, defl_r > 0 ? kMaxDeflate : 1, s_root, root_planes,
+                       root_step ? root_step : kc, lo_planes ? lo_inv + k0 : inv_r, s_hi, hi_inv ? hi_inv + k0 : nullptr, partials);
+          TONER_LAUNCH(root_norm_kernel, kc, 32, stream, partials, fro_tmp);
+          TONER_CUDA(cudaGetLastError());
           break;
         }
         Out o;
@@ -1679,7 +1787,8 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
     if (fro2_lo) TONER_CUDA(cudaMemcpyAsync(fro2_lo + k0, fro_tmp, sizeof(float) * kc, cudaMemcpyDeviceToDevice, stream));
 
     if (q > 1) {
-      // A^{-q/p} by repeated squaring of A^{-1/p} (its planes came with the last product)
+      // A^{-q/p} by repeated squaring of A^{-1/p}
+      Xcur = root_planes;
       int have = 1;
       double bound = root_bound;
       int pi = 0;
@@ -1690,16 +1799,20 @@ int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float dampin
         bound *= bound;
         Out o;
         if (first) {
-          o.alpha_a = inv_r;
-          o.alpha_b = inv_r;
+          o.alpha_a = o.alpha_b = lo_planes ? lo_inv + k0 : inv_r;
         }
         if (have == q) {
           o.d = root_hi + (long long)k0 * nn;
+          if (hi_planes) {
+            o.s0 = static_cast<__half*>(hi_planes) + (long long)k0 * nn;
+            o.s0_scale = s_hi;
+            o.lo_step = k;
+          }
         } else {
           o.s0 = Pb[pi];
           o.s0_scale = plane_scale(bound);
         }
-        rc = sym_product(Xcur, s_x, Xcur, s_x, o, kPromoteX);
+        rc = sym_product(Xcur, s_x, Xcur, s_x, o, kPromoteX, first ? root_step : 0);
         if (rc) return rc;
         Xcur = Pb[pi];
         s_x = o.s0_scale;

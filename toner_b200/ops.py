@@ -340,7 +340,9 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
               track: Optional[torch.Tensor] = None, lmin: Optional[torch.Tensor] = None,
               resid: Optional[torch.Tensor] = None, track_sweeps: int = 0, track_restart: bool = False,
               deflate: Optional[torch.Tensor] = None, deflate_rank: int = 1, deflate_restart: bool = False,
-              deflated: Optional[torch.Tensor] = None, ritz_norm: bool = False, interleave: bool = True):
+              deflated: Optional[torch.Tensor] = None, ritz_norm: bool = False, interleave: bool = True,
+              lo_planes: Optional[torch.Tensor] = None, lo_inv: Optional[torch.Tensor] = None,
+              hi_planes: Optional[torch.Tensor] = None, hi_inv: Optional[torch.Tensor] = None):
     """A^(-1/p) and A^(-q/p) of the damped, trace-normalised statistics (toner_inv_roots_tracked).
 
     ``lower``: a lower bound of the normalised spectrum valid for every statistic (0: the bound that always
@@ -350,7 +352,8 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     the chain; ``deflate`` (k, 8, n), ``deflate_rank``, ``deflate_restart``, ``deflated`` (k,) int32: several dominant
     directions found by block power iteration and deflated (see the header); ``ritz_norm``: take the norm from that
     iteration's largest remaining Ritz value instead of three squarings (an estimate, verified with ``lower``);
-    ``interleave`` = False: plane products one after the other (see the header).
+    ``interleave`` = False: plane products one after the other (see the header); ``lo_planes`` (2, k, n, n) FP16 with
+    ``lo_inv`` (k,), ``hi_planes`` with ``hi_inv``: the roots' operand planes (toner_inv_roots_planes).
     Returns (root_lo, root_hi or None, fro2_lo, status); nothing is synchronised."""
     _need_cuda(ema)
     if ema.ndim == 2:
@@ -378,12 +381,15 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     if deflate is not None and (deflate.shape != (k, 8, n) or deflate.dtype != torch.float32 or not deflate.is_contiguous()):
         raise ValueError("the deflation vectors are a contiguous FP32 (k, 8, n) tensor")
     rank = (int(deflate_rank) & 15) | (256 if deflate_restart else 0) | (512 if ritz_norm else 0)
-    check(_lib.load().toner_inv_roots_tracked(ema.data_ptr(), k, n, damping, p, q, iters, lower, int(lower_is_estimate),
-                                              root_lo.data_ptr(), _ptr(root_hi), fro2_lo.data_ptr(), status.data_ptr(),
-                                              _ptr(norms), _ptr(track), _ptr(lmin), _ptr(resid), sweeps,
-                                              _ptr(deflate), rank, _ptr(deflated),
-                                              workspace.data_ptr(), workspace.numel(), _stream()),
-          "toner_inv_roots_tracked")
+    for t in (lo_planes, hi_planes):
+        if t is not None and (t.shape != (2, k, n, n) or t.dtype != torch.float16 or not t.is_contiguous()):
+            raise ValueError("operand planes are a contiguous FP16 (2, k, n, n) tensor")
+    check(_lib.load().toner_inv_roots_planes(ema.data_ptr(), k, n, damping, p, q, iters, lower, int(lower_is_estimate),
+                                             root_lo.data_ptr(), _ptr(root_hi), fro2_lo.data_ptr(), status.data_ptr(),
+                                             _ptr(norms), _ptr(track), _ptr(lmin), _ptr(resid), sweeps,
+                                             _ptr(deflate), rank, _ptr(deflated), _ptr(lo_planes), _ptr(lo_inv),
+                                             _ptr(hi_planes), _ptr(hi_inv), workspace.data_ptr(), workspace.numel(),
+                                             _stream()), "toner_inv_roots_planes")
     return root_lo, root_hi, fro2_lo, status
 
 
