@@ -110,7 +110,8 @@ def capture_recomputed(xs, attn_out, xmid, gs, us, w1, w2, bufs, at: torch.Tenso
             jobs.append(_job(COPY, attn_out[l], None, b_o))
             jobs.append(_job(RMSNORM, xmid[l], w2[l], b_mlp))
             jobs.append(_job(SILU_MUL, gs[l], us[l], b_down))
-        return jobs
+        # the longest rows first: blocks are handed out in this order, and the last ones should be short
+        return sorted(jobs, key=lambda job: -job[5] * (3 if job[6] == SILU_MUL else 2))
 
     key = ("recomputed", tuple(t.data_ptr() for col in cols for t in col), _signature(xs[0]), _signature(gs[0]),
            _signature(bufs[0]), _signature(bufs[3]), w1[0].dtype)

@@ -28,7 +28,8 @@ __device__ __forceinline__ Bf16x8 load8(const __nv_bfloat16* p) {
   return r;
 }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const Bf16x8& r) {
-  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&r);
+  // (streaming: nobody reads a row again before the statistic at the end of the step)
+  __stcs(reinterpret_cast<uint4*>(p), *reinterpret_cast<const uint4*>(&r));
 }
 
 constexpr int kCaptureWarps = 8;  // rows per block

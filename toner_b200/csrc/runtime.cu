@@ -267,10 +267,11 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
       best = {c.bn, c.pair, splits, splits > 1 ? split_part_bytes(d, c.bn, c.pair, splits) + split_count_bytes(d, c.bn, c.pair) : 0};
     }
   }
-  if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !d.c && !inter && kb >= ctx->gemm_wide_kb) {
+  if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !inter && kb >= ctx->gemm_wide_kb) {
     // The wide tile takes in 48 KB per k-block for twice the work of 32 KB, but its epilogue is only half hidden and its
     // waves are coarser.  Estimates of both, in k-blocks of the pair tile (measured wide / pair: 12 x 3072^3 x 3 planes
-    // symmetric 0.94, 2 x 4096^3 0.86, 12 x 768 x 3072 x 3072 0.89, 18 x 2048^3 0.99; one plane, or with C, above 1).
+    // symmetric 0.94, 2 x 4096^3 0.86, 12 x 768 x 3072 x 3072 0.89, 18 x 2048^3 0.99; one plane, under the power limit: 8192^3
+    // 0.86, 24 x 2048^2 x 5632 0.92, 6 x 5632^3 symmetric with C 0.95; below 80 k-blocks above 1).
     auto waves = [&](int bn) {
       const long long t = gemm_tiles(d, bn, true), w = ctx->gemm_sms / 2;
       return (double)((t + w - 1) / w);

@@ -519,6 +519,10 @@ class FastTonerCore:
             by_shape: Dict[Tuple[int, ...], List[str]] = {}
             for role in part["roles"]:
                 by_shape.setdefault(self.roles[role]["matrix"], []).append(role)
+            for role in part["roles"]:    # (tables of new gradient addresses are uploaded ahead of the lanes)
+                group = self.roles[role]["group"]
+                if group is not None:
+                    group.grad_ptrs([p.grad for p in group.weights])
             self.lanes.run([(i, lambda scratch, names=names: self._update_shape(names, scratch))
                             for i, names in enumerate(by_shape.values())])
             if self.world > 1:   # this part's changes travel while the next part is computed

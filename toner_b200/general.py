@@ -247,6 +247,12 @@ class _TonerGeneral(Optimizer):
                 if not self.state[p].get("statistics_ready", False):
                     raise RuntimeError("Call update_statistics() with this step's input second moments before step()")
 
+    def _update_all(self, work, update) -> None:
+        """`update(group, bucket, scratch)` for every active bucket, on its lane."""
+        for _, bucket in work:       # (tables of new gradient addresses are uploaded ahead of the lanes)
+            bucket.group.grad_ptrs([p.grad for p in bucket.params])
+        self._lanes.run([(bucket.lane, lambda scratch, g=group, b=bucket: update(g, b, scratch)) for group, bucket in work])
+
     def _consume_statistics(self) -> None:
         for group in self.param_groups:
             for p in group["params"]:
@@ -341,7 +347,7 @@ class MuonT(_TonerGeneral):
             core.apply_group_delta(bucket.group, bucket.delta)
 
         if work:
-            self._lanes.run([(bucket.lane, lambda scratch, g=group, b=bucket: update(g, b, scratch)) for group, bucket in work])
+            self._update_all(work, update)
             for _, bucket in work:
                 for i, p in enumerate(bucket.params):
                     self.state[p]["momentum_buffer"] = bucket.group.m[i]
@@ -416,7 +422,7 @@ class AdamT(_TonerGeneral):
                 st["step"] = t
                 st["exp_avg"], st["exp_avg_sq"] = bucket.group.m[i], bucket.group.v[i]
         if work:
-            self._lanes.run([(bucket.lane, lambda scratch, g=group, b=bucket: update(g, b, scratch)) for group, bucket in work])
+            self._update_all(work, update)
             self._health.arm("the previous step's update")
         self._consume_statistics()
         return loss
