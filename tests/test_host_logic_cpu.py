@@ -197,3 +197,14 @@ def test_finishing_polynomial_holds_its_tolerance():
             q = np.polyval(c[::-1], r)
             assert np.abs(q * (1 - r) ** (1.0 / p) - 1).max() < 3.2e-6, (p, lower)
             assert (np.abs(c) * hi ** np.arange(len(c))).sum() <= 2.5 + 1e-9
+
+
+def test_lanes_are_bounded_by_the_scratch_they_add():
+    from toner_b200.core import Lanes
+    cpu = torch.device("cpu")
+    large = Lanes(cpu, [6 << 30, 5 << 30, 1 << 20])       # 5 GiB beside the largest: one lane, as before
+    assert not large.streams and [large.of(i) for i in range(3)] == [0, 0, 0]
+    ran = []
+    large.run([(i, lambda scratch, i=i: ran.append((i, scratch is large.scratch[0]))) for i in range(3)])
+    assert ran == [(0, True), (1, True), (2, True)]
+    assert not Lanes(cpu, [1 << 20]).streams and not Lanes(cpu, []).streams
