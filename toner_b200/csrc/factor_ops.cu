@@ -155,9 +155,10 @@ static bool finish_fit(int p, double lo, double hi, int m, double tail, FitSampl
 // q(r) of degree m >= 4 in floor(m / 2) + (m odd) products instead of Horner's m - 1: repeated division by
 // y = r^2 + beta r leaves q = (..(w y + l_1(r)) y + ..) y + l_k(r) with linear l_i, which cost no product (they enter it in
 // FP32).  beta is chosen so that the innermost quotient is affine in y itself: top y + top0 (m even), or r (top y + top0) +
-// by_r_const (m odd).  About as accurate as Horner's: what one product's single planes (11 bits) lose is relative to
-// |y| |w| = 0.015 here, |r| |w| = 0.007 there (p = 8, |r| = 0.3) -- 1e-6 of the result, against the chain's 2e-5.  With m = 7
-// on 32 statistics of width 2048 two products of six go, 360 us each.
+// by_r_const (m odd).  What a product's single planes (11 bits) lose is relative to |y| |w| here, to |r| |w| there; for p = 4
+// and 8 the difference drowns in the chain's error (roots of width 2048: 0.87 to 1.04 of what Horner and plane-by-plane
+// products gave), for p = 1 and 2, whose coefficients fall more slowly, it added up to a third: those keep Horner's rule.
+// With m = 7 on 32 statistics of width 2048 two products of six go, 360 us each.
 struct QuadraticSteps {
   double beta = 0.0, top = 0.0, top0 = 0.0, by_r_const = 0.0;
   bool by_r = false;
@@ -1645,7 +1646,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
           const float s_w = plane_scale(1.0), s_f = plane_scale(2.0);
           QuadraticSteps fast;
-          if (interleave && quadratic_steps(fin, fast)) {
+          if (interleave && p >= 4 && quadratic_steps(fin, fast)) {
             // Steps of Y = R^2 + beta R (see quadratic_steps): the product that makes Y writes its planes and those of W, an
             // affine function of Y, at once.
             __half* const Yp = Pb[1];
