@@ -152,38 +152,36 @@ static bool finish_fit(int p, double lo, double hi, int m, double tail, FitSampl
   return true;
 }
 
-// q(r) of degree m >= 4 in floor(m / 2) + (m odd) products instead of Horner's m - 1: repeated division by
-// y = r^2 + beta r leaves q = (..(w y + l_1(r)) y + ..) y + l_k(r) with linear l_i, which cost no product (they enter it in
-// FP32).  beta is chosen so that the innermost quotient is affine in y itself: top y + top0 (m even), or r (top y + top0) +
-// by_r_const (m odd).  What a product's single planes (11 bits) lose is relative to |y| |w| here, to |r| |w| there; for p = 4
-// and 8 the difference drowns in the chain's error (roots of width 2048: 0.87 to 1.04 of what Horner and plane-by-plane
-// products gave), for p = 1 and 2, whose coefficients fall more slowly, it added up to a third: those keep Horner's rule.
-// With m = 7 on 32 statistics of width 2048 two products of six go, 360 us each.
+// q(r) of degree m in half of Horner's m - 1 products, and about one: repeated division of an even-degree polynomial by
+// y = r (r + beta) leaves (..(w y + l_1(r)) y + ..) y + l_k(r) with linear l_i, which cost no product (they enter it in FP32);
+// beta is chosen so that the innermost quotient is affine in y itself, top y + top0.  m = 6: q itself, three products for five.
+// m odd: q = c_0 + c_1 r + r v(r) with v of degree m - 1 divided so (m = 7: four products for six).  What the single planes
+// (11 bits) of the products lose -- every operand's rounding, carried through, over the eigenvalues of the benchmark's and of
+// equally spaced spectra -- is 0.5 to 0.97 of Horner's for m = 6 and 0.86 to 0.98 for m = 7; q itself divided with m = 7, or m
+// = 4, reaches 1.7: near r = 0, where most eigenvalues are, an error must fall with r^2 as Horner's does.  m = 5: 0.97 to 1.01
+// from p = 8 on, 1.05 below, where it keeps Horner's rule.  32 statistics of width 2048, m = 7: two products of 350 us each go.
 struct QuadraticSteps {
-  double beta = 0.0, top = 0.0, top0 = 0.0, by_r_const = 0.0;
-  bool by_r = false;
+  double beta = 0.0, top = 0.0, top0 = 0.0;
+  bool by_r = false;                            // a last step by r (m odd)
   std::vector<std::pair<double, double>> lin;   // (linear, constant) of every division, the outermost first
 };
-static bool quadratic_steps(const FinishPoly& fin, QuadraticSteps& out) {
+static bool quadratic_steps(const FinishPoly& fin, int p, QuadraticSteps& out) {
   const int m = fin.order;
-  if (m < 4 || !(fin.c[m] > 0.0)) return false;
-  const double beta = fin.c[m - 1] / ((m / 2) * fin.c[m]);
-  if (!(beta > 0.0 && beta < 2.0)) return false;   // (a fit whose leading coefficients are no longer those of a series)
-  out.beta = beta;
+  if (m < 5 || (m == 5 && p < 8)) return false;
+  out.by_r = (m & 1) != 0;
+  int deg = out.by_r ? m - 1 : m;
   double q[kMaxFinishOrder + 1];
-  for (int j = 0; j <= m; ++j) q[j] = fin.c[j];
-  int deg = m;
-  const int stop = (m & 1) ? 3 : 2;
-  while (deg > stop) {
+  for (int j = 0; j <= deg; ++j) q[j] = !out.by_r ? fin.c[j] : (j == 0 ? 0.0 : fin.c[j + 1]);
+  const double beta = q[deg - 1] / ((deg / 2) * q[deg]);
+  if (!(q[deg] > 0.0 && std::fabs(beta) < 1.0)) return false;
+  out.beta = beta;
+  for (; deg > 2; deg -= 2) {
     for (int j = deg; j >= 2; --j) q[j - 1] -= beta * q[j];   // q[j] is now the quotient's coefficient of r^(j-2)
     out.lin.emplace_back(q[1], q[0]);
     for (int j = 0; j <= deg - 2; ++j) q[j] = q[j + 2];
-    deg -= 2;
   }
-  out.by_r = (m & 1) != 0;
-  out.top = q[deg];
-  out.top0 = out.by_r ? q[1] : q[0];
-  out.by_r_const = out.by_r ? q[0] : 0.0;
+  out.top = q[2];
+  out.top0 = q[0];
   return true;
 }
 
@@ -1623,6 +1621,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       return launch_gemm(g, stream);
     };
     int rc = 0;
+    // the finish in steps of Y; its planes of R + beta I go where the powers of T leave room (p = 1 has no such buffer)
+    QuadraticSteps fast;
+    const bool shorten = interleave && log2p > 0 && quadratic_steps(fin, p, fast);
+    __half* const shifted_planes = Pb[log2p & 1];
     __half* root_planes = nullptr;   // of A^{-1/p}, root_step matrices between hi and lo
     int root_step = 0;
     const float s_root = root_plane_scale(root_bound);
@@ -1645,11 +1647,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
           const float s_w = plane_scale(1.0), s_f = plane_scale(2.0);
-          QuadraticSteps fast;
-          if (interleave && p >= 4 && quadratic_steps(fin, fast)) {
-            // Steps of Y = R^2 + beta R (see quadratic_steps): the product that makes Y writes its planes and those of W, an
-            // affine function of Y, at once.
-            __half* const Yp = Pb[1];
+          if (shorten) {
+            // Steps of Y = R (R + beta I), see quadratic_steps: the product that makes Y writes its planes and those of W, an
+            // affine function of Y, at once.  (shifted_planes are those of -(R + beta I).)
+            __half* const Yp = Pb[(log2p & 1) ^ 1];
             const float s_y = plane_scale(1.0 + std::fabs(fast.beta));
             int left = (int)fast.lin.size() + (fast.by_r ? 1 : 0);   // products after this one; the last writes Mb[1]
             auto target = [&]() { return Mb[(left & 1) ^ 1]; };
@@ -1657,11 +1658,11 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             double bound = std::fabs(fast.top) * (1.0 + std::fabs(fast.beta)) + std::fabs(fast.top0);
             Out y;
             y.segs = 1;
-            y.c = A32; y.beta = (float)-fast.beta;
-            y.s0 = Yp; y.s0_scale = s_y; y.s0_a = (float)fast.beta;
+            y.gain = -1.0;
+            y.s0 = Yp; y.s0_scale = s_y;
             y.s1 = target(); y.s1_scale = scale(bound);
-            y.s1_a = (float)(fast.top * fast.beta + fast.top0); y.s1_b = (float)fast.top;
-            rc = sym_product(Tcur, s_t, Tcur, s_t, y, 0);
+            y.s1_a = (float)fast.top0; y.s1_b = (float)fast.top;
+            rc = sym_product(Tcur, s_t, shifted_planes, s_m, y, 0);
             if (rc) return rc;
             const __half* wcur = y.s1;
             float s_cur = y.s1_scale;
@@ -1680,12 +1681,12 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
               s_cur = w.s1_scale;
               return err;
             };
-            if (fast.by_r) {
-              rc = step(Tcur, s_t, 0.0, fast.by_r_const);
-              if (rc) return rc;
-            }
             for (auto it2 = fast.lin.rbegin(); it2 != fast.lin.rend(); ++it2) {
               rc = step(Yp, s_y, it2->first, it2->second);
+              if (rc) return rc;
+            }
+            if (fast.by_r) {
+              rc = step(Tcur, s_t, fin.c[1], fin.c[0]);
               if (rc) return rc;
             }
           } else {
@@ -1770,6 +1771,11 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           o.s1_a = 1.f;
           o.s1_b = -1.f;
           o.maxres = resid;
+          if (shorten) {
+            o.s0 = shifted_planes;
+            o.s0_scale = s_m;
+            o.s0_a = (float)-(1.0 + fast.beta);
+          }
         } else {
           o.s0 = Mb[mi ^ 1];
           o.s0_scale = s_m;
