@@ -12,14 +12,13 @@
  *   - numerical / device conditions are reported through int status words in device memory
  *   - the library never allocates caller-visible memory: scratch is a caller-provided workspace whose
  *     size comes from the matching *_workspace_bytes query.  (The per-device context keeps one small
- *     private arena for TMA tensor maps, created on first use.)
- *   - streams and the tensor-map arena: the first product that reads an operand (address, shape, strides)
- *     encodes its TMA tensor maps on the host and uploads them with an asynchronous copy on that call's
- *     stream; later products find them by that key.  A product launched on ANOTHER stream before the upload
- *     has finished is made to wait for it (an event recorded after the copy), so any stream may be passed
- *     to any call.  The arena holds 32768 maps; when it is full the library synchronises the device once
- *     and starts over (not allowed during stream capture: a captured region should reuse operand addresses,
- *     which costs no new map)
+ *     private arena for the TMA tensor maps of listed operands, created on first use.)
+ *   - tensor maps: a product's TMA tensor maps are encoded on the host and travel with the launch.  Only operands given
+ *     as a LIST of separately allocated matrices need theirs in device memory: the arena, filled by an asynchronous copy on
+ *     the stream of the first such product and found by (address, shape, strides) afterwards; a product on another stream
+ *     is ordered behind that copy by an event, so any stream may be passed to any call.  The arena holds 32768 maps; when
+ *     it is full the library synchronises the device once and starts over (not allowed during stream capture: a captured
+ *     region should reuse operand addresses, which costs no new map)
  *   - matrices are row-major FP32 unless said otherwise; "stack" means `batch` equally shaped matrices
  *     stored back to back
  *   - there is no CPU fallback: without a CUDA device every compute entry point fails

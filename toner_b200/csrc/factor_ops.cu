@@ -1264,10 +1264,10 @@ static size_t per_statistic_bytes(int n) {
   return align_up((size_t)n * n * 4, 256) * 8;
 }
 static size_t small_bytes(int chunk, int n) {
-  // twenty per-statistic scalars, four blocks of eight scalars per statistic (Ritz values, residuals, deflation
+  // nineteen per-statistic scalars, four blocks of eight scalars per statistic (Ritz values, residuals, deflation
   // coefficients, root corrections), the reduction scratch, and two blocks of eight n-vectors per statistic
   // (block power iteration: V and A V)
-  return align_up((size_t)chunk * 4, 256) * 20 + 4 * align_up((size_t)chunk * 32, 256) +
+  return align_up((size_t)chunk * 4, 256) * 19 + 4 * align_up((size_t)chunk * 32, 256) +
          align_up(sumsq_scratch_bytes(chunk), 256) + 2 * align_up((size_t)chunk * 8 * n * 4, 256);
 }
 
@@ -1466,9 +1466,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float* rest_top = small(16);
     int* rest_idx = reinterpret_cast<int*>(small(17));
     float* e_top = small(18);
-    float* rest_trace = small(19);
+    float* rest_trace = small(10);
     const size_t sm8 = align_up((size_t)kc * 32, 256);
-    char* wp = w + sm * 20;
+    char* wp = w + sm * 19;
     float* th8 = reinterpret_cast<float*>(wp); wp += sm8;     // Ritz values, residuals, deflation coefficients and
     float* res8 = reinterpret_cast<float*>(wp); wp += sm8;    // root corrections of the block deflation: eight per statistic
     float* coef8 = reinterpret_cast<float*>(wp); wp += sm8;
@@ -1478,7 +1478,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float* pv = reinterpret_cast<float*>(wp);
     float* py = reinterpret_cast<float*>(wp + vec);
     float* dv = deflate ? deflate + (long long)k0 * kMaxDeflate * n : nullptr;
-    TONER_CUDA(cudaMemsetAsync(w, 0, sm * 20 + 4 * sm8, stream));
+    TONER_CUDA(cudaMemsetAsync(w, 0, sm * 19 + 4 * sm8, stream));
 
     const float* C = ema + (long long)k0 * nn;
     const int t32 = (n + 31) / 32;
