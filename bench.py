@@ -170,14 +170,14 @@ def step_flops(w: Workload, root_gemms_d: int, root_gemms_f: int, ns_steps: int 
 def product_counts(core, optimizer: str):
     """Products per statistic of the factor engine as it ran last: X T and the log2(p) + 1 products of the M update per
     Newton step (no X product in the first step, no M update in the last), the squarings for the stronger power --
-    each three FP16 plane passes -- plus the single-pass products of the finishing series (its order - 1)."""
+    each three FP16 plane passes -- plus the single-pass products of the finishing polynomial."""
     out = {}
     for name, g in core.groups.items():
         f = g.factors
         log2p = f.p.bit_length() - 1
         split = (f.iterations - 1) * (log2p + 2) + (f.q.bit_length() - 1)
         out[name] = {"newton_steps": f.iterations, "finish_order": f.finish_order, "split": split,
-                     "single": f.finish_order - 1}
+                     "single": f.finish_products}
     return out
 
 
@@ -504,8 +504,8 @@ def run_general(args, w: Workload) -> None:
     ff = next(b.factors for b in buckets if b.factors.n == w.mlp)
     log2p = fd.p.bit_length() - 1
     # the general interface factors one statistic per parameter (q, k, v each their own): 5 hidden-width, 1 MLP-width
-    per_d = (fd.iterations - 1) * (log2p + 2) + fd.finish_order - 1
-    per_f = (ff.iterations - 1) * (log2p + 2) + ff.finish_order - 1
+    per_d = (fd.iterations - 1) * (log2p + 2) + fd.finish_products
+    per_f = (ff.iterations - 1) * (log2p + 2) + ff.finish_products
     L, h, m = w.layers, w.hidden, w.mlp
     fl = {"syrk": w.rows * L * (5 * h * (h + 1) + m * (m + 1)), "ns": 0,
           "precond": sum(L * 5 * 2 * r * c * c for r, c in w.shapes),

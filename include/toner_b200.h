@@ -223,7 +223,7 @@ int toner_split16(const float* x, const float* const* x_list, int32_t batch, int
  * per accumulator).  The last of the `iters` steps applies a polynomial q(R) ~ (I - R)^(-1/p), R = I - M, to X
  * alone: the Chebyshev interpolant of (1 - r)^(-1/p) on [-0.02, 1.15 e + 1e-3] of the smallest degree with relative
  * error below 3e-6, e being the bound on R the schedule guarantees (toner_inv_roots_finish_order_for,
- * toner_inv_roots_schedule); its degree - 1 products are single passes over FP16 planes of R.
+ * toner_inv_roots_schedule), evaluated by single passes over FP16 planes of R (toner_inv_roots_finish_products_for).
  * `iters` <= 0 selects toner_inv_roots_iterations(n, damping, p), which depends only on
  * its arguments (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632, damping 1e-3): the count with the fewest
  * plane passes, Newton steps and series together.
@@ -237,6 +237,8 @@ int toner_inv_roots_iterations(int32_t n, float damping, int32_t p);
 int toner_inv_roots_iterations_for(float lower, int32_t p);   /* the count for a given spectrum lower bound */
 /* degree of the finishing polynomial for that bound and count (iters <= 0: the default count); 0 on bad arguments */
 int toner_inv_roots_finish_order_for(float lower, int32_t p, int32_t iters);
+/* How many single-pass products evaluate that polynomial (plane_order: 1 for calls with track_sweeps + 512). */
+int toner_inv_roots_finish_products_for(float lower, int32_t p, int32_t iters, int32_t plane_order);
 /* The whole schedule the engine runs for a spectrum lower bound (host only, no device needed): returns the step count
  * (iters <= 0: the default), and writes the (a_k, b_k) of its count - 1 Newton steps (ab_out: pairs of doubles, as many
  * as ab_capacity holds), the degree of the finishing polynomial (order_out), its coefficients c_0 .. c_degree in powers

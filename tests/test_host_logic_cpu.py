@@ -208,3 +208,19 @@ def test_lanes_are_bounded_by_the_scratch_they_add():
     large.run([(i, lambda scratch, i=i: ran.append((i, scratch is large.scratch[0]))) for i in range(3)])
     assert ran == [(0, True), (1, True), (2, True)]
     assert not Lanes(cpu, [1 << 20]).streams and not Lanes(cpu, []).streams
+
+
+@pytest.mark.parametrize("p", [2, 4, 8, 16])
+def test_products_of_the_finish(p):
+    """Degree 6 takes three products, odd degrees from 5 (from 7 below p = 8) half of Horner's and one, the rest Horner's."""
+    from toner_b200 import ops
+    seen = set()
+    for lower in (0.4, 0.2, 0.15, 0.1, 0.05, 0.03, 0.02, 0.0104, 0.0084):
+        m = ops.inv_roots_finish_order(768, 1e-3, p, lower)
+        short = m == 6 or m == 7 or (m == 5 and p >= 8)
+        want = m // 2 + (m & 1) if short else m - 1
+        assert ops.inv_roots_finish_products(768, 1e-3, p, lower) == want
+        assert ops.inv_roots_finish_products(768, 1e-3, p, 1e-4, interleave=False) == \
+            ops.inv_roots_finish_order(768, 1e-3, p, 1e-4) - 1
+        seen.add(m)
+    assert seen & {6, 7}

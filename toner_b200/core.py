@@ -207,6 +207,12 @@ class FactorSet:
         """Degree of the last factorisation's finishing polynomial."""
         return ops.inv_roots_finish_order(self.n, self.damping, self.p, self._lower_used) if self.k else 0
 
+    @property
+    def finish_products(self) -> int:
+        """Single-pass products of the last factorisation's finish."""
+        return (ops.inv_roots_finish_products(self.n, self.damping, self.p, self._lower_used, interleave=self.interleave)
+                if self.k else 0)
+
     # -- which stored root serves a given strength
     def _is_hi(self, strength: float) -> bool:
         return self.q > 1 and strength == max(self.inner_strength, self.outer_strength)

@@ -312,10 +312,17 @@ def inv_roots_iterations_for(lower: float, p: int) -> int:
 
 
 def inv_roots_finish_order(n: int, damping: float, p: int, lower: float = 0.0, iters: int = 0) -> int:
-    """Degree of the polynomial that finishes the iteration (its degree - 1 products are single passes); `lower` = 0
+    """Degree of the polynomial that finishes the iteration (inv_roots_finish_products); `lower` = 0
     means the bound damping / (n (1 + damping)) that always holds."""
     worst = damping / (n * (1.0 + damping))
     return _lib.load().toner_inv_roots_finish_order_for(max(lower, worst), p, iters)
+
+
+def inv_roots_finish_products(n: int, damping: float, p: int, lower: float = 0.0, iters: int = 0,
+                              interleave: bool = True) -> int:
+    """Single-pass products that evaluate the finishing polynomial."""
+    worst = damping / (n * (1.0 + damping))
+    return _lib.load().toner_inv_roots_finish_products_for(max(lower, worst), p, iters, int(not interleave))
 
 
 def inv_roots_schedule(lower: float, p: int, iters: int = 0) -> dict:

@@ -144,7 +144,7 @@ def bench_roots(a):
     log2p, log2q = int(math.log2(a.p)), int(math.log2(a.q))
     order = ops.inv_roots_finish_order(a.n, 1e-3, a.p)
     split = (iters - 1) * (log2p + 2) + log2q     # X T and T^p M per step (no X product first, no M last), squarings
-    single = order - 1                            # Horner steps of the finishing series
+    single = ops.inv_roots_finish_products(a.n, 1e-3, a.p)   # of the finishing polynomial
     flops = a.k * (split + single) * 2 * a.n ** 3
     return report("inv_roots", {"k": a.k, "n": a.n, "p": a.p, "q": a.q, "cond": a.cond}, ms, best, flops=flops,
                   extra={"iterations": iters, "finish_order": order, "damping": 1e-3, "split_products": split,
@@ -170,7 +170,7 @@ def bench_roots_tracked(a):
     ms, best = timed(fn, 1, a.reps, False)
     log2p, log2q = int(math.log2(a.p)), int(math.log2(a.q))
     split = (f.iterations - 1) * (log2p + 2) + log2q
-    single = f.finish_order - 1
+    single = f.finish_products
     flops = a.k * (split + single) * 2 * a.n ** 3
     return report("inv_roots_tracked", {"k": a.k, "n": a.n, "p": a.p, "q": a.q, "cond": a.cond}, ms, best, flops=flops,
                   extra={"iterations": f.iterations, "finish_order": f.finish_order, "split_products": split,
