@@ -233,6 +233,43 @@ __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restr
   }
 }
 
+// The same partial sums, a warp each: it plays the eight warps of the kernel above in turn, so the additions and their order
+// are the same.  For matrices of which a block's share is at most four accesses a thread: 296 blocks a matrix then spend
+// their time starting and reducing (32 matrices of 512 x 512: 21 us, now 11; 48 of 768 x 768: 44, now 33).
+constexpr long long kSumsqWarpShare = 1024;   // 16-byte accesses of a partial sum
+__global__ void __launch_bounds__(256) sumsq_partial_warp_kernel(const float* __restrict__ x, long long total4, long long bs,
+                                                                 float* __restrict__ partial) {
+  ptx::pdl_begin();
+  const int b = blockIdx.y, lane = threadIdx.x & 31;
+  const int part = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const float4* X4 = reinterpret_cast<const float4*>(x + (long long)b * bs);
+  const long long per = (total4 + kSumsqBlocks - 1) / kSumsqBlocks;
+  const long long lo = per * part, hi = (lo + per < total4) ? lo + per : total4;
+  float s0[8], s1[8], s2[8], s3[8];
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s0[w] = s1[w] = s2[w] = s3[w] = 0.f;
+  for (long long i0 = lo + lane; i0 < hi; i0 += 256) {
+    float4 v[8];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v[w] = i0 + 32 * w < hi ? X4[i0 + 32 * w] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {   // (a zero beyond the end changes no sum)
+      s0[w] = fmaf(v[w].x, v[w].x, s0[w]); s1[w] = fmaf(v[w].y, v[w].y, s1[w]);
+      s2[w] = fmaf(v[w].z, v[w].z, s2[w]); s3[w] = fmaf(v[w].w, v[w].w, s3[w]);
+    }
+  }
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    float s = (s0[w] + s1[w]) + (s2[w] + s3[w]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    t += s;
+  }
+  if (lane == 0) partial[(long long)b * kSumsqBlocks + part] = t;
+}
+static_assert(kSumsqBlocks % 8 == 0, "eight partial sums a block");
+
 __global__ void __launch_bounds__(32) sumsq_final_kernel(const float* __restrict__ partial, float* __restrict__ out) {
   ptx::pdl_begin();
   const float t = sumsq_total(partial + (long long)blockIdx.x * kSumsqBlocks, threadIdx.x);
@@ -243,7 +280,12 @@ size_t sumsq_scratch_bytes(int batch) { return (size_t)batch * kSumsqBlocks * si
 
 int sumsq_det(const float* x, int batch, int rows, int cols, long long ld, long long bs, float* scratch, float* out,
               cudaStream_t stream) {
-  TONER_LAUNCH(sumsq_partial_kernel, dim3(kSumsqBlocks, batch), 256, stream, x, rows, cols, ld, bs, scratch);
+  const long long total = (long long)rows * cols;
+  if (ld == cols && total % 4 == 0 && total / 4 <= kSumsqWarpShare * kSumsqBlocks && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
+      (bs % 4 == 0 || batch == 1))
+    TONER_LAUNCH(sumsq_partial_warp_kernel, dim3(kSumsqBlocks / 8, batch), 256, stream, x, total / 4, bs, scratch);
+  else
+    TONER_LAUNCH(sumsq_partial_kernel, dim3(kSumsqBlocks, batch), 256, stream, x, rows, cols, ld, bs, scratch);
   if (out) TONER_LAUNCH(sumsq_final_kernel, batch, 32, stream, scratch, out);
   TONER_CUDA(cudaGetLastError());
   return 0;
