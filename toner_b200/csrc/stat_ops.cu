@@ -101,8 +101,12 @@ __global__ void __launch_bounds__(256) maxabs_kernel(const float* __restrict__ x
     const int c4 = cols / 4;
     const long long total4 = (long long)rows * c4;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
-      const int r = (int)(i / c4), c = (int)(i - (long long)r * c4) * 4;
-      const float4 q = *reinterpret_cast<const float4*>(X + (long long)r * ld + c);
+      int r = 0, c = -4;
+      if (ld != cols || aff_a != 0.f) {
+        r = (int)(i / c4);
+        c = (int)(i - (long long)r * c4) * 4;
+      }
+      const float4 q = ld == cols ? reinterpret_cast<const float4*>(X)[i] : *reinterpret_cast<const float4*>(X + (long long)r * ld + c);
       const float v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) m = fmaxf(m, fabsf(fmaf(aff_b, v[e], (c + e) == r ? aff_a : 0.f)));
@@ -143,8 +147,15 @@ __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ 
   if (vec) {
     const long long total4 = per / 4;
     const int c4 = cols / 4;
+    // (the planes have no gaps; rows and columns matter only to a gapped source and to a multiple of the identity: two 64-bit
+    // divisions an access otherwise)
+    const bool flat = ld == cols;
     auto split4 = [&](long long i, const float4 q) {
-      const int r = (int)(i / c4), c = (int)(i - (long long)r * c4) * 4;
+      int r = 0, c = -4;
+      if (aff_a != 0.f) {
+        r = (int)(i / c4);
+        c = (int)(i - (long long)r * c4) * 4;
+      }
       const float v[4] = {q.x, q.y, q.z, q.w};
       __half h[4], l[4];
 #pragma unroll
@@ -153,10 +164,11 @@ __global__ void __launch_bounds__(256) split16_kernel(const float* __restrict__ 
         h[e] = __float2half_rn(w);
         l[e] = __float2half_rn(w - __half2float(h[e]));
       }
-      *reinterpret_cast<uint2*>(hi + (long long)r * cols + c) = *reinterpret_cast<uint2*>(h);
-      if (!hi_only) *reinterpret_cast<uint2*>(lo + (long long)r * cols + c) = *reinterpret_cast<uint2*>(l);
+      *reinterpret_cast<uint2*>(hi + 4 * i) = *reinterpret_cast<uint2*>(h);
+      if (!hi_only) *reinterpret_cast<uint2*>(lo + 4 * i) = *reinterpret_cast<uint2*>(l);
     };
     auto load4 = [&](long long i) {
+      if (flat) return reinterpret_cast<const float4*>(X)[i];
       const int r = (int)(i / c4), c = (int)(i - (long long)r * c4) * 4;
       return *reinterpret_cast<const float4*>(X + (long long)r * ld + c);
     };

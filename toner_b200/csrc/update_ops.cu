@@ -13,6 +13,10 @@ static int ew_grid(long long elems4, int num_sms) {
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// Blocks for a kernel that does something besides its accesses in every block (a sum to finish, a maximum to hand in): four
+// 16-byte accesses a thread.  With one, 48 matrices of 768 x 768 were 27 000 blocks that mostly started and reduced.
+static int ew_grid4(long long elems4, int num_sms) { return ew_grid((elems4 + 3) / 4, num_sms); }
+
 // ------------------------------------------------------------------ Newton-Schulz helpers
 // x = u / (||u|| + eps), written as FP32 and as BF16 (the operand the products read); ||u||^2 as the partial sums that
 // sumsq_det left (each block adds them up itself: 1.2 KB from L2, against a launch of its own)
@@ -31,9 +35,8 @@ __global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__
   const float4* U = reinterpret_cast<const float4*>(u + (long long)b * per);
   float4* X = reinterpret_cast<float4*>(x + (long long)b * per);
   uint2* XB = reinterpret_cast<uint2*>(xb + (long long)b * per);
-  const long long n4 = per / 4;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    float4 v = U[i];
+  const long long n4 = per / 4, step = (long long)gridDim.x * blockDim.x;
+  auto scaled = [&](long long i, float4 v) {
     v.x *= f; v.y *= f; v.z *= f; v.w *= f;
     X[i] = v;
     __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), c = __floats2bfloat162_rn(v.z, v.w);
@@ -41,7 +44,13 @@ __global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__
     o.x = *reinterpret_cast<uint32_t*>(&a);
     o.y = *reinterpret_cast<uint32_t*>(&c);
     XB[i] = o;
+  };
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 3 * step < n4; i += 4 * step) {   // four loads in flight (u and x may be one array: a thread's own elements)
+    const float4 v0 = U[i], v1 = U[i + step], v2 = U[i + 2 * step], v3 = U[i + 3 * step];
+    scaled(i, v0); scaled(i + step, v1); scaled(i + 2 * step, v2); scaled(i + 3 * step, v3);
   }
+  for (; i < n4; i += step) scaled(i, U[i]);
 }
 
 // ------------------------------------------------------------------ MuonT momentum
@@ -110,14 +119,19 @@ __global__ void __launch_bounds__(256) adamt_m_kernel(const float* const* __rest
   const long long n4 = per / 4;
   const float w = 1.f - b1;
   float gx = 0.f, mx = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const float4 g = G[i];
-    float4 mm = M[i];
+  auto advance = [&](long long i, const float4 g, float4 mm) {
     mm.x = mm.x * b1 + g.x * w; mm.y = mm.y * b1 + g.y * w; mm.z = mm.z * b1 + g.z * w; mm.w = mm.w * b1 + g.w * w;
     M[i] = mm;
     gx = fmaxf(fmaxf(fmaxf(gx, fabsf(g.x)), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w)));
     mx = fmaxf(fmaxf(fmaxf(mx, fabsf(mm.x)), fabsf(mm.y)), fmaxf(fabsf(mm.z), fabsf(mm.w)));
+  };
+  const long long step = (long long)gridDim.x * blockDim.x;
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + step < n4; i += 2 * step) {
+    const float4 g0 = G[i], g1 = G[i + step], m0 = M[i], m1 = M[i + step];
+    advance(i, g0, m0); advance(i + step, g1, m1);
   }
+  if (i < n4) advance(i, G[i], M[i]);
   if (g_max) {
     block_atomic_max(gx, g_max + b);
     __syncthreads();
@@ -137,18 +151,22 @@ __global__ void __launch_bounds__(256) adamt_ratio_kernel(const float* __restric
   const long long n4 = per / 4;
   const float w = 1.f - b2;
   float mx = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const float4 tt = T[i];
-    float4 vv = V[i];
+  auto divide = [&](long long i, const float4 tt, float4 vv, float4 nn) {
     vv.x = vv.x * b2 + tt.x * tt.x * w; vv.y = vv.y * b2 + tt.y * tt.y * w;
     vv.z = vv.z * b2 + tt.z * tt.z * w; vv.w = vv.w * b2 + tt.w * tt.w * w;
     V[i] = vv;
-    float4 nn = N[i];
     nn.x = nn.x / (sqrtf(vv.x / bc2) + eps); nn.y = nn.y / (sqrtf(vv.y / bc2) + eps);
     nn.z = nn.z / (sqrtf(vv.z / bc2) + eps); nn.w = nn.w / (sqrtf(vv.w / bc2) + eps);
     N[i] = nn;
     mx = fmaxf(fmaxf(fmaxf(mx, fabsf(nn.x)), fabsf(nn.y)), fmaxf(fabsf(nn.z), fabsf(nn.w)));
+  };
+  const long long step = (long long)gridDim.x * blockDim.x;
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + step < n4; i += 2 * step) {
+    const float4 t0 = T[i], t1 = T[i + step], v0 = V[i], v1 = V[i + step], n0 = N[i], n1 = N[i + step];
+    divide(i, t0, v0, n0); divide(i + step, t1, v1, n1);
   }
+  if (i < n4) divide(i, T[i], V[i], N[i]);
   if (maxabs) block_atomic_max(mx, maxabs + b);
 }
 
@@ -288,7 +306,7 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
 
   int rc = sumsq_det(u, batch, m, n, n, mn, partial, nullptr, stream);
   if (rc) return rc;
-  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid(mn / 4, ctx->num_sms), batch), 256, stream, u, partial, eps, mn, x_out, xb[0]);
+  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid4(mn / 4, ctx->num_sms), batch), 256, stream, u, partial, eps, mn, x_out, xb[0]);
   TONER_CUDA(cudaGetLastError());
 
   const float ca = 3.4445f, cb = -4.7750f, cc = 2.0315f;  // src/toner/linalg.py:9
@@ -375,7 +393,7 @@ int toner_muont_momentum(const float* const* grad_ptrs, float* m, float* u, int3
   if (int rc = check_stack("muont_momentum", per)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (maxabs) TONER_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(uint32_t) * count, stream));
-  TONER_LAUNCH(muont_momentum_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, stream, grad_ptrs, m, u, per, mu, nesterov, maxabs);
+  TONER_LAUNCH(muont_momentum_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), count), 256, stream, grad_ptrs, m, u, per, mu, nesterov, maxabs);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -402,7 +420,7 @@ int toner_adamt_first_moment(const float* const* grad_ptrs, float* m, int32_t co
   if (!ctx) return kErrCuda;
   if (!grad_ptrs || !m || count <= 0) return fail(kErrArg, "adamt_first_moment: bad arguments");
   if (int rc = check_stack("adamt_first_moment", per)) return rc;
-  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), grad_ptrs, m, per, beta1, nullptr, nullptr);
+  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), count), 256, static_cast<cudaStream_t>(stream), grad_ptrs, m, per, beta1, nullptr, nullptr);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -415,7 +433,7 @@ int toner_adamt_ratio(const float* t, float* v, float* num, int32_t count, int64
   if (int rc = check_stack("adamt_ratio", per)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (maxabs) TONER_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(uint32_t) * count, stream));
-  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid(per / 4, ctx->num_sms), count), 256, stream, t, v, num, per, beta2, bc2, eps, maxabs);
+  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), count), 256, stream, t, v, num, per, beta2, bc2, eps, maxabs);
   TONER_CUDA(cudaGetLastError());
   return 0;
 }
@@ -545,13 +563,13 @@ int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay,
   uint32_t* const max2 = g->maxabs + 2 * g->count;
   TONER_CUDA(cudaMemsetAsync(max0, 0, sizeof(uint32_t) * 3 * g->count, stream));
   // one pass over the gradient: m <- b1 m + (1 - b1) g, max |g|, max |m|
-  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->grads, g->m, per, beta1, max0, max1);
+  TONER_LAUNCH(adamt_m_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), g->count), 256, stream, g->grads, g->m, per, beta1, max0, max1);
   int rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->grads), max0, nullptr, nullptr, false, false, stream);
   if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // t = g R
   if (!rc) rc = split_stack(*g, g->m, nullptr, max1, nullptr, nullptr, false, false, stream);
   if (!rc) rc = right_product(*g, false, g->work2, false, 1.f / bc1, nullptr, nullptr, nullptr, stream);         // (m / bc1) R
   if (rc) return rc;
-  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid(per / 4, ctx->num_sms), g->count), 256, stream, g->work, g->v, g->work2, per, beta2, bc2,
+  TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), g->count), 256, stream, g->work, g->v, g->work2, per, beta2, bc2,
                eps, max2);                                                                                       // U, in work2
   rc = sumsq_det(g->work2, g->count, g->rows, g->cols, g->cols, per, g->ss_scratch, ss0, stream);
   if (!rc) rc = split_stack(*g, g->work2, nullptr, max2, nullptr, nullptr, false, false, stream);
