@@ -224,3 +224,17 @@ def test_products_of_the_finish(p):
             ops.inv_roots_finish_order(768, 1e-3, p, 1e-4) - 1
         seen.add(m)
     assert seen & {6, 7}
+
+
+def test_the_plane_order_keeps_horners_finish_at_every_bound():
+    """A caller that asks for the plane-by-plane order of additions gets it whatever the spectrum: Horner's m - 1 products."""
+    from toner_b200 import ops
+    for p in (2, 4, 8):
+        for lower in (1e-6, 1e-4, 4e-3, 6e-3, 0.02, 0.05, 0.1, 0.2, 0.4):
+            assert ops.inv_roots_finish_products(768, 1e-3, p, lower, interleave=False) == \
+                ops.inv_roots_finish_order(768, 1e-3, p, lower) - 1, (p, lower)
+
+
+def test_only_adamt_keeps_the_plane_order():
+    from toner_b200 import core
+    assert core.may_reorder("muont") and not core.may_reorder("adamt")

@@ -1,0 +1,60 @@
+"""AdamT's products keep the plane-by-plane order of additions at every lower bound of the spectrum, in both of its
+optimizers: where an element of the preconditioned gradient nearly vanishes, another order gives another weight."""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DAMPING = 1e-3
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    from toner_b200 import ops as _ops
+    return _ops
+
+
+@pytest.mark.parametrize("lower", [1e-3, 6e-3, 0.03, 0.1])
+@pytest.mark.parametrize("p,q", [(8, 4), (4, 1)])
+def test_the_roots_of_a_statistic_do_not_depend_on_its_batch(ops, lower, p, q):
+    """Alone a statistic of width 512 is factored on single-CTA tiles, in a stack of 48 on pair tiles, which interleave plane
+    products where they may.  Plane by plane an element's additions come in one order on any tile: the bits are the same."""
+    n, k = 512, 48
+    g = torch.Generator(device="cuda").manual_seed(int(1e4 * lower) + p)
+    basis, _ = torch.linalg.qr(torch.randn(n, n, device="cuda", generator=g))
+    ema = torch.empty(k, n, n, device="cuda")
+    for i in range(k):
+        lam = 1.0 + 0.5 * torch.rand(n, device="cuda", generator=g)
+        c = (basis * lam) @ basis.T
+        ema[i] = 0.5 * (c + c.T)
+    lo, hi, fro2, st = ops.inv_roots(ema, DAMPING, p, q, lower=lower, lower_is_estimate=True, track_sweeps=12, track_restart=True,
+                                     track=torch.zeros(k, n, device="cuda"), lmin=torch.empty(k, device="cuda"), interleave=False)
+    for i in (0, k - 1):
+        one = ops.inv_roots(ema[i:i + 1].contiguous(), DAMPING, p, q, lower=lower, lower_is_estimate=True, track_sweeps=12,
+                            track_restart=True, track=torch.zeros(1, n, device="cuda"), lmin=torch.empty(1, device="cuda"),
+                            interleave=False)
+        assert torch.equal(one[0][0], lo[i]) and torch.equal(one[2][0], fro2[i])
+        assert q == 1 or torch.equal(one[1][0], hi[i])
+    ops.assert_healthy()
+    assert st.tolist() == [0] * k
+
+
+@pytest.mark.parametrize("kind", ["adamt", "muont"])
+def test_the_layer_sharded_engine_keeps_the_order_for_adamt(ops, kind):
+    from toner_b200.fast.engine import FastTonerCore
+    hid, mlp, layers, rows = 64, 128, 1, 96
+    shapes = dict(q=(hid, hid), k=(hid, hid), v=(hid, hid), attn_proj=(hid, hid), fc=(mlp, hid), mlp_proj=(hid, mlp))
+    named = {f"body.blocks.{i}.{role}.weight": torch.nn.Parameter(torch.randn(*s, device="cuda") * 0.02)
+             for i in range(layers) for role, s in shapes.items()}
+    blocks = [types.SimpleNamespace(input_rows_attn=torch.empty(rows, 1, dtype=torch.bfloat16)) for _ in range(layers)]
+    args = types.SimpleNamespace(toner_decay=0.95, toner_split=kind == "muont", toner_alpha=0.25, toner_alpha_in=0.5,
+                                 toner_alpha_out=0.125, wd=0.1, beta1=0.9, beta2=0.95, eps=1e-15, muon_momentum=0.95,
+                                 muon_nesterov=True, muon_ns_steps=2, muon_eps=1e-5, muon_ns_mode="tpu")
+    core = FastTonerCore.from_blocks(blocks, named, kind, hid=hid, mlp=mlp, rows_total=rows, args=args, world=1, rank=0,
+                                     device=torch.device("cuda", 0))
+    for g in core.groups.values():
+        assert g.factors.interleave == (kind == "muont")

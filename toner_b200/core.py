@@ -97,6 +97,16 @@ class Lanes:
                 current.wait_stream(self.streams[lane - 1])
 
 
+def may_reorder(kind: str) -> bool:
+    """Whether the split products of an optimizer ("adamt" or "muont") may take their plane products k-block by k-block.
+
+    AdamT divides (m / bc1) R by the square root of v, which comes from (g R)^2: two products that round on their own.  Where
+    an element of g R is as small as that rounding their ratio is noise over noise, of any size and either sign, so another
+    order of additions -- no less accurate -- gives other weights.  AdamT's products, those of its factors among them, keep
+    the plane-by-plane order and so their bits; the polar factor of MuonT smooths such differences."""
+    return kind != "adamt"
+
+
 def root_orders(strength_a: float, strength_b: float) -> Tuple[int, int]:
     """Map two inverse-power strengths to (p, q): the weaker is A^(-1/p), the stronger A^(-q/p).
 

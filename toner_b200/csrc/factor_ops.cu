@@ -165,10 +165,6 @@ struct QuadraticSteps {
   bool by_r = false;                            // a last step by r (m odd)
   std::vector<std::pair<double, double>> lin;   // (linear, constant) of every division, the outermost first
 };
-// Whether a factorisation may depart from the plane-by-plane order of additions, in its products and in its finish: unless
-// the caller asked for that order and the spectrum is wide enough for it to be seen (chain_length()'s first threshold).
-static bool reorders(bool plane_order, double lower) { return !plane_order || lower >= 5e-3; }
-
 static bool quadratic_steps(const FinishPoly& fin, int p, QuadraticSteps& out) {
   const int m = fin.order;
   if (m < 5 || (m == 5 && p < 8)) return false;
@@ -1317,7 +1313,7 @@ int toner_inv_roots_finish_products_for(float lower, int32_t p, int32_t iters, i
   const toner::Schedule& s = toner::schedule_for((double)lower, p, iters);
   if (s.iters < 2) return 0;
   toner::QuadraticSteps q;
-  if (!toner::reorders(plane_order != 0, lower) || p == 1 || !toner::quadratic_steps(s.fin, p, q)) return s.fin.order - 1;
+  if (plane_order || p == 1 || !toner::quadratic_steps(s.fin, p, q)) return s.fin.order - 1;
   return 1 + (int)q.lin.size() + (q.by_r ? 1 : 0);
 }
 
@@ -1591,8 +1587,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     }
     }
 
-    // plane products interleaved (toner_gemm_desc::interleave), and the finish in its short form
-    const bool interleave = reorders((track_sweeps & 512) != 0, l0);
+    // plane products interleaved (toner_gemm_desc::interleave), and the finish in its short form: unless the caller asked for
+    // the plane-by-plane order of additions
+    const bool interleave = (track_sweeps & 512) == 0;
 
     // D = (A planes) * (B planes)^T / (sa * sb): symmetric result, FP32-accurate; outputs as requested
     struct Out {

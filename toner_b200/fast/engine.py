@@ -94,7 +94,7 @@ class StatGroup:
 
     def __init__(self, name: str, keys: List[Tuple[int, str]], n: int, rows: int, counts: Sequence[int], rank: int,
                  world: int, device: torch.device, strengths: Tuple[float, float], damping: float,
-                 scratch: core.Scratch) -> None:
+                 scratch: core.Scratch, interleave: bool) -> None:
         """`counts[r]` statistics are owned by rank r, in key order (contiguous layer blocks; ranks may own different
         numbers of layers, a rank may own none)."""
         self.name, self.keys, self.n, self.rows = name, keys, n, rows
@@ -107,7 +107,7 @@ class StatGroup:
         self.tri = n * (n + 1) // 2
         # one stacked row buffer: statistic s of this rank's tokens is rows_buf[s]
         self.rows_buf = torch.empty(self.k_all, rows, n, device=device, dtype=torch.bfloat16)
-        self.factors = core.FactorSet(per_rank, n, device, strengths, damping, scratch)
+        self.factors = core.FactorSet(per_rank, n, device, strengths, damping, scratch, interleave=interleave)
         self.partial: Optional[torch.Tensor] = None   # (chunks, world, cs, tri) packed partial Grams (world > 1)
         self.summed: Optional[torch.Tensor] = None    # (per, tri) summed Grams of the owned statistics
         self.chunk_stats = per_rank
@@ -170,13 +170,14 @@ class FastTonerCore:
                                                 for c, n in ((len(KINDS_D), hid), (1, mlp))], priority=-1)
         strengths = (float(args.inner_strength), float(args.outer_strength))
         damping = float(getattr(args, "damping", 1e-3))
+        interleave = core.may_reorder(kind)
         self.groups = {
             "d": StatGroup("d", [(i, k) for i in range(layers) for k in KINDS_D], hid, row_capacity,
                            [len(KINDS_D) * c for c in self.layer_counts], rank, world, device, strengths, damping,
-                           self.factor_lanes.scratch[0]),
+                           self.factor_lanes.scratch[0], interleave),
             "f": StatGroup("f", [(i, "down") for i in range(layers)], mlp, row_capacity, list(self.layer_counts), rank,
                            world, device, strengths, damping,
-                           self.factor_lanes.scratch[self.factor_lanes.of(1)]),
+                           self.factor_lanes.scratch[self.factor_lanes.of(1)], interleave),
         }
         self.weight = 0.0
         # matrices by role; the owned layers of a role form one MatrixGroup

@@ -70,9 +70,8 @@ class _Bucket:
                  lane: int, scratch: core.Scratch) -> None:
         self.params, self.lane = params, lane
         n = params[0].shape[1]
-        # AdamT divides by its second moments, which in the first steps turns the sign of a gradient element near zero into a
-        # full step: there the factors keep the order of additions they have had (plane by plane), bit for bit.
-        self.factors = core.FactorSet(len(params), n, params[0].device, strengths, damping, scratch, interleave=kind != "adamt")
+        self.factors = core.FactorSet(len(params), n, params[0].device, strengths, damping, scratch,
+                                      interleave=core.may_reorder(kind))
         self.group = core.MatrixGroup(params, self.factors, 0, 1, kind)
         self.delta = torch.empty_like(self.group.m)
         self.index = {p: i for i, p in enumerate(params)}
