@@ -277,7 +277,8 @@ int toner_inv_roots_ex(const float* ema, int32_t k, int32_t n, float damping, in
  *                  `track_sweeps` power-iteration steps on the highest inverse power (A^(-q/p)), where that eigenvalue
  *                  is the dominant one however small it is next to lambda_max(A); track_sweeps + 256 starts from a
  *                  fixed vector instead of the buffer's content (first call, or after the statistics were replaced);
- *                  track_sweeps + 512 keeps the plane-by-plane order of additions in every product (interleave = 0).
+ *                  track_sweeps + 512 keeps the plane-by-plane order of additions in every product (interleave = 0),
+ *                  Horner's finish, and the block iteration's small factorisations one rotation or division at a time.
  *   lmin_out       (DEVICE, optional, k floats) the estimate of lambda_min(A_b) that comes with it: a Rayleigh quotient,
  *                  so it errs on the high side (by 5-25 % after 8 sweeps from scratch, less once tracking).
  *   lower, lower_is_estimate

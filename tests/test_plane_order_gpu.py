@@ -1,8 +1,10 @@
 """AdamT's products keep the plane-by-plane order of additions at every lower bound of the spectrum, in both of its
 optimizers: where an element of the preconditioned gradient nearly vanishes, another order gives another weight."""
 
+import hashlib
 import types
 
+import numpy as np
 import pytest
 import torch
 
@@ -58,3 +60,50 @@ def test_the_layer_sharded_engine_keeps_the_order_for_adamt(ops, kind):
                                      device=torch.device("cuda", 0))
     for g in core.groups.values():
         assert g.factors.interleave == (kind == "muont")
+
+
+def _noise(shape, seed):
+    """Integers of a bell-shaped distribution, the same everywhere."""
+    i = np.arange(int(np.prod(shape)), dtype=np.uint64) + np.uint64(seed << 32)
+    out = np.zeros(i.shape, dtype=np.int64)
+    for _ in range(4):
+        i = (i ^ (i >> np.uint64(31))) * np.uint64(0x9E3779B97F4A7C15)
+        out += (i >> np.uint64(58)).astype(np.int64) - 32
+    return out.reshape(shape)
+
+
+# SHA-256 of (root_lo, fro2_lo) after each of five calls, from the engine before its small factorisations (Jacobi, Cholesky) and
+# products could take another order: the strengths are equal, so there is one root.
+_BITS = {
+    (3, 264, 1200, 2, 0): ["4de1a504d3f86bfd", "d450f43f976dc89d", "dc09d693aa93dfdb", "ea193d79780b8382", "3e797a4ade6a9ffc"],
+    (2, 264, 1200, 1, 2): ["a30e5a31030530f6", "6994e893ca393110", "ecefb17d25191efe", "a15433bf34014236", "5c93a26fb3926303"],
+    (12, 512, 3000, 1, 0): ["a36bfd1ff76892f5", "d55f184a3cf8aa66", "338d4674d2d9c609", "aaa1260a90f7bdac", "cbf178ed872b76f5"],
+}
+
+
+@pytest.mark.parametrize("k,n,rows,mean,spikes", list(_BITS))
+def test_factors_keep_their_bits(ops, k, n, rows, mean, spikes):
+    """Statistics of integer rows (their Grams are exact) with a dominant mean and outlier directions: the calls go from the
+    cold block iteration and the bound that always holds to the warm one, estimated bounds and the norm estimate."""
+    from toner_b200 import core
+    c = np.empty((k, n, n), dtype=np.float32)
+    for b in range(k):
+        x = _noise((rows, n), 7 * b + n) + mean * _noise((1, n), 1000 + b)
+        for s in range(spikes):
+            x = x + _noise((rows, 1), 50 + s + b) * _noise((1, n), 90 + s) // 16
+        x = x.astype(np.float64)
+        c[b] = (x.T @ x / rows).astype(np.float32)
+    c = torch.from_numpy(c).cuda()
+    f = core.FactorSet(k, n, torch.device("cuda"), (0.25, 0.25), DAMPING, interleave=False)
+    got = []
+    for _ in range(5):
+        f.ema.copy_(c)
+        f.compute()
+        assert f.finish() == 0
+        h = hashlib.sha256()
+        for t in (f.root_lo, f.fro2_lo):
+            h.update(t.cpu().numpy().tobytes())
+        got.append(h.hexdigest()[:16])
+    ops.assert_healthy()
+    assert f.repairs == 0 and f.lower_is_estimate
+    assert got == _BITS[k, n, rows, mean, spikes]

@@ -701,9 +701,11 @@ __device__ __forceinline__ int pair_index(int i, int j) { return i * (i + 1) / 2
 // Cholesky-QR of the r vectors held in Y (r x n, vector-major): G = Y Y^T = L L^T (FP64), V = L^-1 Y.  `gram` holds G's
 // lower triangle (pair_index order) on entry.  A vector that is (numerically) a combination of the earlier ones comes out as
 // zero; its slot is seeded afresh by the next call.  L's columns are formed one after the other by the lanes of one warp (row
-// i of a column by lane i); the diagonal of `L` holds its reciprocal (zero for a dropped vector).
+// i of a column by lane i); the diagonal of `L` holds its reciprocal (zero for a dropped vector), the diagonal itself where
+// `divide` asks for divisions by it (see ritz_kernel).
 template <int R>
-__device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, const double* gram, double (*L)[kMaxDeflate]) {
+__device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, const double* gram, double (*L)[kMaxDeflate],
+                                        bool divide) {
   if (threadIdx.x < 32) {
     const int i = threadIdx.x;
     double row[R];
@@ -717,9 +719,16 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
       // lane j holds the pivot
       const double pivot = __shfl_sync(0xffffffffu, sum, j);
       const double floor = j < r ? 1e-24 * gram[pair_index(j, j)] : 0.0;
-      const double inv = (j < r && pivot > floor && pivot > 0.0) ? rsqrt(pivot) : 0.0;
-      row[j] = i == j ? pivot * inv : sum * inv;
-      if (on) L[i][j] = i == j ? inv : row[j];
+      const bool kept = j < r && pivot > floor && pivot > 0.0;
+      if (divide) {
+        const double diag = kept ? sqrt(pivot) : 0.0;
+        row[j] = i == j ? diag : (kept ? sum / diag : 0.0);
+        if (on) L[i][j] = row[j];
+      } else {
+        const double inv = kept ? rsqrt(pivot) : 0.0;
+        row[j] = i == j ? pivot * inv : sum * inv;
+        if (on) L[i][j] = i == j ? inv : row[j];
+      }
     }
   }
   __syncthreads();
@@ -732,7 +741,7 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
 #pragma unroll
         for (int i = 0; i < R; ++i)
           if (i < j) sum -= L[j][i] * out[i];
-        out[j] = sum * L[j][j];
+        out[j] = !divide ? sum * L[j][j] : (L[j][j] > 0.0 ? sum / L[j][j] : 0.0);
       } else {
         out[j] = 0.0;
       }
@@ -792,10 +801,48 @@ __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) 
   }
 }
 
+// The same with one rotation after the other, row by row of the upper triangle, and rounded as a single thread doing so would
+// (lane k takes column / row k; every lane adds up the same sums in the same order).
+__device__ void jacobi_in_order(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate], int r) {
+  const int k = threadIdx.x & 7;
+  const bool on = threadIdx.x < r;
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    double off = 0.0, diag = 0.0;
+    for (int pp = 0; pp < r; ++pp)
+      for (int qq = pp + 1; qq < r; ++qq) off += H[pp][qq] * H[pp][qq];
+    for (int pp = 0; pp < r; ++pp) diag += H[pp][pp] * H[pp][pp];
+    if (!(off > 1e-30 * diag)) break;
+    for (int pp = 0; pp < r; ++pp) {
+      for (int qq = pp + 1; qq < r; ++qq) {
+        const double apq = H[pp][qq];
+        if (apq == 0.0) continue;
+        const double tau = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
+        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+        const double cs = 1.0 / sqrt(1.0 + t * t), sn = t * cs;
+        __syncwarp();   // every lane has the rotation before an entry changes
+        if (on) {
+          const double hp = H[k][pp], hq = H[k][qq], qp = Q[k][pp], qv = Q[k][qq];
+          H[k][pp] = cs * hp - sn * hq;
+          H[k][qq] = sn * hp + cs * hq;
+          Q[k][pp] = cs * qp - sn * qv;
+          Q[k][qq] = sn * qp + cs * qv;
+        }
+        __syncwarp();
+        if (on) {
+          const double hp = H[pp][k], hq = H[qq][k];
+          H[pp][k] = cs * hp - sn * hq;
+          H[qq][k] = sn * hp + cs * hq;
+        }
+        __syncwarp();
+      }
+    }
+  }
+}
+
 // start vectors: the caller's vectors (warm), or r different fixed +-1 patterns (cold, and for a slot that holds
 // nothing yet because the rank grew since the last call), orthonormalised
 template <int R>
-__global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v, int n, int r, int vstride, int cold) {
+__global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v, int n, int r, int vstride, int cold, int in_order) {
   ptx::pdl_begin();
   __shared__ double red[8];
   constexpr int kPairs = R * (R + 1) / 2;
@@ -825,7 +872,7 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
       for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += x[i] * x[j];
   }
   block_sum_many<kPairs>(acc, part, gram);
-  cholesky_orthonormalise<R>(V, V, n, r, gram, L);
+  cholesky_orthonormalise<R>(V, V, n, r, gram, L, in_order != 0);
 }
 
 // Rayleigh-Ritz on span(V) with Y = A V (V orthonormal): H = V Y^T, H = Q diag(theta) Q^T (Jacobi, FP64), V <- Q^T V,
@@ -833,9 +880,12 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
 // then replaced by the orthonormalised Y (one more step of the power iteration).  Three passes over the two blocks of
 // vectors; every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
 // vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2; now 17.
+// in_order: a caller that keeps its order of additions (the plane-by-plane products) has the small factorisations keep theirs
+// too: Jacobi's rotations one after the other and divisions by Cholesky's diagonal.  The vectors are no better for it, but a
+// deflated eigenvalue hundreds of times the rest turns their last bits into 1e-5 of what remains.
 template <int R>
 __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float* __restrict__ y, int n, int r, int vstride,
-                                                   int last, float* __restrict__ theta, float* __restrict__ res) {
+                                                   int last, float* __restrict__ theta, float* __restrict__ res, int in_order) {
   ptx::pdl_begin();
   constexpr int kPairs = R * (R + 1) / 2, kSums = R * R > kPairs + R ? R * R : kPairs + R, kMost = kMaxDeflate;
   __shared__ double part[8 * kSums], sums[kSums];
@@ -868,7 +918,8 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    jacobi_warp(H, Q);
+    if (in_order) jacobi_in_order(H, Q, r);
+    else jacobi_warp(H, Q);
     // descending order: lane i's place is the number of values before it; the columns of Q follow
     const int i = threadIdx.x & 7;
     const double mine = H[i][i];
@@ -939,7 +990,7 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
     theta[b * kMost + threadIdx.x] = (float)l;
     res[b * kMost + threadIdx.x] = l > 0.0 ? (float)(sqrt(sums[kPairs + threadIdx.x]) / l) : INFINITY;
   }
-  if (!last) cholesky_orthonormalise<R>(Y, V, n, r, sums, L);
+  if (!last) cholesky_orthonormalise<R>(Y, V, n, r, sums, L, in_order != 0);
 }
 
 // Which of the r Ritz pairs are deflated: in descending order, as long as each has converged and stands above eight
@@ -1497,13 +1548,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       // dominant directions: block power iteration with Rayleigh-Ritz on the caller's vectors (eight sweeps from fixed
       // vectors -- the first three or four only find the subspace --, four from last call's), then deflate those that
       // converged and stand above the rest
-      const int sweeps = defl_cold ? 8 : 4;
+      const int sweeps = defl_cold ? 8 : 4, in_order = (track_sweeps & 512) ? 1 : 0;
       auto iterate = [&](auto width) -> int {   // (R as a type: every kernel of the iteration is specialised for it)
         constexpr int R = decltype(width)::value;
-        TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0);
+        TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0, in_order);
         for (int sw = 0; sw < sweeps; ++sw) {
           TONER_LAUNCH(block_gemv_kernel<R>, dim3((n + kBlockGemvRows - 1) / kBlockGemvRows, kc), 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
-          TONER_LAUNCH(ritz_kernel<R>, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8);
+          TONER_LAUNCH(ritz_kernel<R>, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order);
         }
         return 0;
       };
