@@ -435,8 +435,9 @@ int toner_muont_input(const toner_matrix_group* group, float mu, int32_t nestero
  * (optional, used without weight decay): max |P| per matrix as FP32 bits */
 int toner_muont_delta(const toner_matrix_group* group, const uint32_t* polar_maxabs, float lr, float weight_decay, float scale,
                       float* delta, void* stream);
-/* moments, ratio and shaped decay of AdamT: delta = -(c1 W R) R - lr ||U||_F U R / ||U R||_F */
-int toner_adamt_delta(const toner_matrix_group* group, float lr, float weight_decay, float beta1, float beta2, float bc1, float bc2,
+/* moments, ratio and shaped decay of AdamT: delta = -(c1 W R) R - lr ||U||_F U R / ||U R||_F.  bc1 = 1 - beta1^t is a double: its
+ * reciprocal scales the first moment's product and is rounded to FP32 once. */
+int toner_adamt_delta(const toner_matrix_group* group, float lr, float weight_decay, float beta1, float beta2, double bc1, float bc2,
                       float eps, float* delta, void* stream);
 
 /* Lists of `count` separately allocated matrices of `numel` FP32 elements (a multiple of 4, 16-byte aligned), HOST arrays of

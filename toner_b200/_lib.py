@@ -123,7 +123,7 @@ SIGNATURES = {
     "toner_apply_scaled": (C.c_int, [_vp, _vp, _i32, _i64, _f32, _f32, _vp]),
     "toner_muont_input": (C.c_int, [C.POINTER(MatrixGroup), _f32, _i32, _vp]),
     "toner_muont_delta": (C.c_int, [C.POINTER(MatrixGroup), _vp, _f32, _f32, _f32, _vp, _vp]),
-    "toner_adamt_delta": (C.c_int, [C.POINTER(MatrixGroup), _f32, _f32, _f32, _f32, _f32, _f32, _f32, _vp, _vp]),
+    "toner_adamt_delta": (C.c_int, [C.POINTER(MatrixGroup), _f32, _f32, _f32, _f32, C.c_double, _f32, _f32, _vp, _vp]),
     "toner_list_finite": (C.c_int, [C.POINTER(_vp), _i32, _i64, _vp, _vp]),
     "toner_list_axpby": (C.c_int, [C.POINTER(_vp), C.POINTER(_vp), _i32, _i64, _f32, _f32, _vp]),
     "toner_split16": (C.c_int, [_vp, _vp, _i32, _i32, _i32, _i64, _i64, _f32, _f32, _vp, _vp, _vp, _vp, _vp]),

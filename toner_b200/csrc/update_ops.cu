@@ -548,7 +548,7 @@ int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs,
   return right_product(*g, true, delta, false, -1.f, nullptr, nullptr, nullptr, stream);
 }
 
-int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay, float beta1, float beta2, float bc1, float bc2,
+int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay, float beta1, float beta2, double bc1, float bc2,
                       float eps, float* delta, void* stream_) {
   if (int rc = check_group("adamt_delta", g)) return rc;
   if (!delta || !g->v || !g->work2 || !g->ss || !g->ss_scratch || !g->inner_planes || !g->outer_fro2)
@@ -567,7 +567,7 @@ int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay,
   int rc = split_stack(*g, nullptr, const_cast<const float* const*>(g->grads), max0, nullptr, nullptr, false, false, stream);
   if (!rc) rc = right_product(*g, false, g->work, false, 1.f, nullptr, nullptr, nullptr, stream);                // t = g R
   if (!rc) rc = split_stack(*g, g->m, nullptr, max1, nullptr, nullptr, false, false, stream);
-  if (!rc) rc = right_product(*g, false, g->work2, false, 1.f / bc1, nullptr, nullptr, nullptr, stream);         // (m / bc1) R
+  if (!rc) rc = right_product(*g, false, g->work2, false, (float)(1.0 / bc1), nullptr, nullptr, nullptr, stream);       // (m / bc1) R
   if (rc) return rc;
   TONER_LAUNCH(adamt_ratio_kernel, dim3(ew_grid4(per / 4, ctx->num_sms), g->count), 256, stream, g->work, g->v, g->work2, per, beta2, bc2,
                eps, max2);                                                                                       // U, in work2
