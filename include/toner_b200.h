@@ -126,6 +126,8 @@ typedef struct toner_gemm_desc {
                                k-block, which saves a third of the operand traffic; the additions into the accumulator
                                then come in that order instead of plane by plane (no less accurate: chains become
                                shorter to make up for the cross products in them) */
+  int32_t split_chains;     /* 1: split_ws divides a tile's accumulation among exactly as many CTAs as it has chains, if at all:
+                               the chains are then added in their order and the result keeps its bits */
 } toner_gemm_desc;
 
 int toner_gemm(const toner_gemm_desc* desc, void* stream);
@@ -153,7 +155,9 @@ int toner_syrk_upper(const void* const* x_list, const void* x_base, int64_t x_ba
 
 /* The same with scratch: few statistics over many rows (one 2048-wide statistic is 36 tiles of 256 x 256) then have each
  * tile's rows divided among several CTAs.  toner_syrk_workspace_bytes gives the scratch that helps (0: none does);
- * `workspace` may be NULL.  The parts are added in a fixed order: the same call gives the same bits. */
+ * `workspace` may be NULL.  The parts are added in a fixed order: the same call gives the same bits, but not those of
+ * toner_syrk_upper, unless TONER_SYRK_KEEP_ORDER is added to the mode: rows are then divided only chain by chain (4096 rows). */
+#define TONER_SYRK_KEEP_ORDER 16
 size_t toner_syrk_workspace_bytes(int32_t k, int32_t rows, int32_t n);
 int toner_syrk_upper_ws(const void* const* x_list, const void* x_base, int64_t x_batch_stride, int32_t k, int32_t rows,
                         int32_t n, int64_t ld, float* out, int32_t mode, float beta, float gamma, void* workspace,

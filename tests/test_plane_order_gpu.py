@@ -45,10 +45,8 @@ def test_the_roots_of_a_statistic_do_not_depend_on_its_batch(ops, lower, p, q):
     assert st.tolist() == [0] * k
 
 
-@pytest.mark.parametrize("kind", ["adamt", "muont"])
-def test_the_layer_sharded_engine_keeps_the_order_for_adamt(ops, kind):
+def _engine(kind, hid, mlp, layers, rows):
     from toner_b200.fast.engine import FastTonerCore
-    hid, mlp, layers, rows = 64, 128, 1, 96
     shapes = dict(q=(hid, hid), k=(hid, hid), v=(hid, hid), attn_proj=(hid, hid), fc=(mlp, hid), mlp_proj=(hid, mlp))
     named = {f"body.blocks.{i}.{role}.weight": torch.nn.Parameter(torch.randn(*s, device="cuda") * 0.02)
              for i in range(layers) for role, s in shapes.items()}
@@ -56,9 +54,13 @@ def test_the_layer_sharded_engine_keeps_the_order_for_adamt(ops, kind):
     args = types.SimpleNamespace(toner_decay=0.95, toner_split=kind == "muont", toner_alpha=0.25, toner_alpha_in=0.5,
                                  toner_alpha_out=0.125, wd=0.1, beta1=0.9, beta2=0.95, eps=1e-15, muon_momentum=0.95,
                                  muon_nesterov=True, muon_ns_steps=2, muon_eps=1e-5, muon_ns_mode="tpu")
-    core = FastTonerCore.from_blocks(blocks, named, kind, hid=hid, mlp=mlp, rows_total=rows, args=args, world=1, rank=0,
+    return FastTonerCore.from_blocks(blocks, named, kind, hid=hid, mlp=mlp, rows_total=rows, args=args, world=1, rank=0,
                                      device=torch.device("cuda", 0))
-    for g in core.groups.values():
+
+
+@pytest.mark.parametrize("kind", ["adamt", "muont"])
+def test_the_layer_sharded_engine_keeps_the_order_for_adamt(ops, kind):
+    for g in _engine(kind, 64, 128, 1, 96).groups.values():
         assert g.factors.interleave == (kind == "muont")
 
 
@@ -107,3 +109,56 @@ def test_factors_keep_their_bits(ops, k, n, rows, mean, spikes):
     ops.assert_healthy()
     assert f.repairs == 0 and f.lower_is_estimate
     assert got == _BITS[k, n, rows, mean, spikes]
+
+
+def _undivided(ops, x):
+    """Grams of a (k, rows, n) stack, every tile's rows on one CTA (pair): the entry point without scratch."""
+    from toner_b200 import _lib
+    k, rows, n = x.shape
+    out = torch.zeros(k, n, n, device="cuda")
+    _lib.check(_lib.load().toner_syrk_upper(None, x.data_ptr(), x.stride(0), k, rows, n, x.stride(1), out.data_ptr(),
+                                            ops.EMA_FULL, 0.0, 1.0, ops._stream()), "toner_syrk_upper")
+    return out
+
+
+@pytest.mark.parametrize("k,n,rows", [(1, 72, 200), (2, 328, 2170), (4, 1064, 3208), (1, 264, 4096), (1, 264, 4097), (1, 768, 8192),
+                                      (1, 520, 12289), (9, 512, 48036)])
+def test_rows_are_divided_only_where_the_sum_keeps_its_bits(ops, k, n, rows):
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(k, rows, n, device="cuda", generator=g).to(torch.bfloat16)
+    want = _undivided(ops, x)
+    out = torch.full_like(want, float("nan"))
+    ops.syrk_upper(x, out, ops.EMA_FULL, 0.0, 1.0, keep_order=True)
+    assert torch.equal(out, want)
+    packed = torch.empty(k, n * (n + 1) // 2, device="cuda")
+    ops.syrk_upper(list(x.unbind(0)), packed, ops.PACKED, keep_order=True)
+    r, c = torch.triu_indices(n, n, device="cuda")
+    assert torch.equal(packed, want[:, r, c])
+
+
+def test_activation_statistics_keep_the_bits_of_undivided_sums(ops):
+    import toner_b200
+    layers = {str(i): torch.nn.Linear(328, 16, bias=False).cuda().to(torch.bfloat16) for i in range(2)}
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(2, 2170, 328, device="cuda", generator=g).to(torch.bfloat16)
+    stats, got = toner_b200.ActivationStatistics(layers, distributed=False), {}
+    with stats.capture(), torch.no_grad():
+        for layer, rows in zip(layers.values(), x):
+            layer(rows)
+    stats.commit(types.SimpleNamespace(update_statistics=got.update))
+    stats.close()
+    for layer, sums in zip(layers.values(), _undivided(ops, x)):
+        assert torch.equal(got[layer.weight], sums * (1.0 / 2170))
+
+
+def test_the_layer_sharded_engine_divides_no_chain_for_adamt(ops):
+    core = _engine("adamt", 512, 1024, 1, 3000)
+    want = []
+    for g in core.groups.values():
+        g.rows_buf.normal_(generator=torch.Generator(device="cuda").manual_seed(g.n))
+        want.append(_undivided(ops, g.rows_buf))
+    core._stats()
+    torch.cuda.synchronize()
+    gamma = (1 - core.decay) / core.rows_total
+    for g, sums in zip(core.groups.values(), want):
+        assert torch.equal(g.factors.ema, sums * gamma)

@@ -56,7 +56,7 @@ class GemmDesc(C.Structure):
         ("maxres", C.c_void_p),
         ("upper_d", C.c_int32),
         ("split_ws", C.c_void_p), ("split_ws_bytes", C.c_int64),
-        ("split0_aff_a", C.c_float), ("interleave", C.c_int32),
+        ("split0_aff_a", C.c_float), ("interleave", C.c_int32), ("split_chains", C.c_int32),
     ]
 
 

@@ -103,7 +103,8 @@ def may_reorder(kind: str) -> bool:
     AdamT divides (m / bc1) R by the square root of v, which comes from (g R)^2: two products that round on their own.  Where
     an element of g R is as small as that rounding their ratio is noise over noise, of any size and either sign, so another
     order of additions -- no less accurate -- gives other weights.  AdamT's products, those of its factors among them, keep
-    the plane-by-plane order and so their bits; the polar factor of MuonT smooths such differences."""
+    the plane-by-plane order and so their bits, and its statistics that of their rows; the polar factor of MuonT smooths
+    such differences."""
     return kind != "adamt"
 
 

@@ -251,8 +251,8 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
     const double busy = main + blocks * 8 * block_smem;
     double cost = main + epi + (waves - 1) * (busy > epi ? busy : epi);
     int splits = 1;
-    if (d.split_ws && d.segs == 1) {
-      for (int s = 2; s <= 32 && s <= chains && tiles * s <= workers; ++s) {
+    if (d.split_ws && d.segs == 1 && !(d.split_chains && d.promote <= 0)) {
+      for (int s = d.split_chains && chains > 2 ? chains : 2; s <= 32 && s <= chains && tiles * s <= workers; ++s) {
         const size_t need = split_part_bytes(d, c.bn, c.pair, s) + split_count_bytes(d, c.bn, c.pair);
         if (need > (size_t)d.split_ws_bytes) break;
         const double parts = 4000.0 + blocks * (800.0 + 400.0 * s);   // writing and adding the parts, the extra memset

@@ -440,8 +440,12 @@ int toner_syrk_upper_ws(const void* const* x_list, const void* x_base, int64_t x
   if ((!x_list && !x_base) || !out) return fail(kErrArg, "syrk: null pointer");
   if (k <= 0 || rows <= 0 || n <= 0) return fail(kErrArg, "syrk: sizes must be positive");
   if (n % 8 != 0 || ld % 8 != 0) return fail(kErrArg, "syrk: n and ld must be multiples of 8");
-  if (mode < 0 || mode > 2) return fail(kErrArg, "syrk: mode must be 0 (PACKED), 1 (PACKED_ACC) or 2 (EMA_FULL)");
+  const bool keep_order = (mode & TONER_SYRK_KEEP_ORDER) != 0;
+  mode &= ~TONER_SYRK_KEEP_ORDER;
+  if (mode < 0 || mode > 2)
+    return fail(kErrArg, "syrk: mode must be 0 (PACKED), 1 (PACKED_ACC) or 2 (EMA_FULL), plus 16 to keep the order of additions");
   toner_gemm_desc d = syrk_desc(k, rows, n);
+  d.split_chains = keep_order ? 1 : 0;
   d.split_ws = workspace;
   d.split_ws_bytes = (int64_t)workspace_bytes;
   toner_operand op = {};

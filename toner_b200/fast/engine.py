@@ -171,6 +171,7 @@ class FastTonerCore:
         strengths = (float(args.inner_strength), float(args.outer_strength))
         damping = float(getattr(args, "damping", 1e-3))
         interleave = core.may_reorder(kind)
+        self.keep_order = not interleave
         self.groups = {
             "d": StatGroup("d", [(i, k) for i in range(layers) for k in KINDS_D], hid, row_capacity,
                            [len(KINDS_D) * c for c in self.layer_counts], rank, world, device, strengths, damping,
@@ -357,7 +358,7 @@ class FastTonerCore:
     def _partial_grams(self, g: "StatGroup", c: int) -> None:
         """Packed Grams of statistic chunk c from the rows now in the buffers, added to earlier pieces of the step."""
         mode = ops.PACKED_ACC if self.pieces_done else ops.PACKED
-        ops.syrk_upper(g.chunk_lists[c], g.partial[c].view(-1, g.tri), mode)
+        ops.syrk_upper(g.chunk_lists[c], g.partial[c].view(-1, g.tri), mode, keep_order=self.keep_order)
 
     def _reduce_to_owners(self, g: "StatGroup", c: int):
         """Sum chunk c's partial Grams over the ranks at the owners (asynchronous; returns the NCCL work)."""
@@ -402,7 +403,7 @@ class FastTonerCore:
             raise RuntimeError(f"{self.pieces_done + 1} of the step's {self.row_pieces} row pieces were captured")
         if self.world == 1 and self.row_pieces == 1:
             self.factor_lanes.run([   # SYRK with the EMA fused
-                (i, lambda _, g=g: ops.syrk_upper(g.rows_buf, g.factors.ema, ops.EMA_FULL, b, gamma))
+                (i, lambda _, g=g: ops.syrk_upper(g.rows_buf, g.factors.ema, ops.EMA_FULL, b, gamma, self.keep_order))
                 for i, g in enumerate(self.groups.values())])
         elif self.world == 1:
             for g in self.groups.values():
@@ -447,7 +448,7 @@ class FastTonerCore:
             g = self.groups[name]
             self.side.wait_event(event)
             if self.world == 1:
-                ops.syrk_upper(g.rows_buf[lo:hi], g.factors.ema[lo:hi], ops.EMA_FULL, b, gamma)
+                ops.syrk_upper(g.rows_buf[lo:hi], g.factors.ema[lo:hi], ops.EMA_FULL, b, gamma, self.keep_order)
             if hi != g.k_all:
                 continue
             if self.world > 1:   # all of the group's rows are in: partial Grams, sums at the owners, EMA

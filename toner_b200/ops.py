@@ -15,6 +15,7 @@ from . import _lib
 from ._lib import GemmDesc, Operand, check
 
 PACKED, PACKED_ACC, EMA_FULL = 0, 1, 2
+KEEP_ORDER = 16
 PROMOTE_ACCURATE = 2  # k-blocks per tensor-core accumulation chain in FP32-accurate products
 _FMT = {torch.float16: 0, torch.bfloat16: 1}
 
@@ -209,11 +210,15 @@ def _syrk_scratch(lib, k: int, rows: int, n: int, out: torch.Tensor):
     return (torch.empty(need, device=out.device, dtype=torch.uint8) if need else None), need
 
 
-def syrk_upper(x, out: torch.Tensor, mode: int = PACKED, beta: float = 0.0, gamma: float = 1.0) -> None:
+def syrk_upper(x, out: torch.Tensor, mode: int = PACKED, beta: float = 0.0, gamma: float = 1.0,
+               keep_order: bool = False) -> None:
     """Upper-triangle X^T X of BF16 row buffers (toner_syrk_upper).
 
-    ``x`` is a (k, rows, n) stack or a list of k separately allocated (rows, n) buffers."""
+    ``x`` is a (k, rows, n) stack or a list of k separately allocated (rows, n) buffers.  ``keep_order``: rows are divided
+    among CTAs only where the sum keeps its bits (whole chains of 4096 rows)."""
     lib = _lib.load()
+    if keep_order:
+        mode |= KEEP_ORDER
     if isinstance(x, torch.Tensor):
         _need_cuda(x, out)
         if x.dtype != torch.bfloat16 or x.ndim != 3 or x.stride(2) != 1:
