@@ -238,3 +238,51 @@ def test_the_plane_order_keeps_horners_finish_at_every_bound():
 def test_only_adamt_keeps_the_plane_order():
     from toner_b200 import core
     assert core.may_reorder("muont") and not core.may_reorder("adamt")
+
+
+class _FakeStream:
+    """What Lanes asks of a stream; nothing runs on it."""
+
+    def __init__(self, *args, **kw):
+        pass
+
+    def record_event(self):
+        return object()
+
+    def wait_event(self, event):
+        pass
+
+    def wait_stream(self, other):
+        pass
+
+
+def test_a_lanes_outgrown_buffer_is_not_handed_to_another_lane(monkeypatch):
+    """Five pieces on three lanes, the second piece of lane 1 larger than its first: the first one's workspace, on which lane
+    1 still works, must not go back to the memory pool before the lanes have been joined."""
+    import contextlib
+    import weakref
+    from toner_b200 import core
+    home = _FakeStream()
+    monkeypatch.setattr(torch.cuda, "Stream", _FakeStream)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: home)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    cpu = torch.device("cpu")
+    lanes = core.Lanes(cpu, [64] * 5)
+    assert len(lanes.streams) == 2
+    seen, alive = {}, []
+
+    def job(i, nbytes):
+        def run(scratch):
+            buf = scratch.bytes_like("ns", nbytes, cpu)
+            assert buf.numel() >= nbytes
+            seen[i] = weakref.ref(buf)
+            if 1 in seen:
+                alive.append(seen[1]() is not None)
+        return i, run
+
+    lanes.run([job(0, 64), job(1, 64), job(2, 64), job(3, 64), job(4, 128)])
+    assert len(alive) == 5 and all(alive)
+    assert seen[1]() is None and seen[4]() is not None       # given back afterwards; the larger one is kept
+    assert all(s.home is None for s in lanes.scratch)
+    lanes.scratch[1].bytes_like("ns", 256, cpu)              # outside a run nothing else is beside it: given back at once
+    assert seen[4]() is None

@@ -31,9 +31,12 @@ class Scratch:
 
     def __init__(self) -> None:
         self._buffers: Dict[Tuple, torch.Tensor] = {}
-        # The stream whose memory pool buffers come from, where another one is current (see Lanes: work on a lane begins after
-        # this stream's and is waited for by it, so the pool's order of reuse holds).
+        # While Lanes.run() is under way: the stream whose memory pool buffers come from, which is not the one they are used on.
+        # The lanes begin after this stream's work and are waited for by it, so the pool's order of reuse holds between runs;
+        # inside one it does not -- what a lane hands back another could be given while the lane still works on it --, so
+        # buffers that have been outgrown are kept until the lanes have been joined.
         self.home: Optional[torch.cuda.Stream] = None
+        self._outgrown: List[torch.Tensor] = []
 
     def _empty(self, shape, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
         if self.home is None:
@@ -54,9 +57,16 @@ class Scratch:
         key = (name, "bytes", str(device))
         buf = self._buffers.get(key)
         if buf is None or buf.numel() < nbytes:
+            if buf is not None and self.home is not None:
+                self._outgrown.append(buf)
             buf = self._empty(nbytes, torch.uint8, device)
             self._buffers[key] = buf
         return buf
+
+    def joined(self) -> None:
+        """The home stream is ordered behind everything that has used this scratch."""
+        self.home = None
+        self._outgrown.clear()
 
 
 class Lanes:
@@ -95,6 +105,8 @@ class Lanes:
         finally:
             for lane in others:
                 current.wait_stream(self.streams[lane - 1])
+            for scratch in self.scratch:
+                scratch.joined()
 
 
 def may_reorder(kind: str) -> bool:
