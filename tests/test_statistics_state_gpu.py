@@ -1,0 +1,67 @@
+"""What ActivationStatistics keeps between its calls: sums after a refused commit, row buffers, streams and process groups."""
+
+import types
+
+import pytest
+import torch
+
+from oracle import toner_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tb():
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    import toner_b200
+    return toner_b200
+
+
+def _layers(widths):
+    return {f"l{i}": torch.nn.Linear(n, 16, bias=False).cuda().to(torch.bfloat16) for i, n in enumerate(widths)}
+
+
+def _forward(stats, layers, rows):
+    with stats.capture(), torch.no_grad():
+        for layer, x in zip(layers.values(), rows):
+            layer(x)
+
+
+def _rows(layers, count, gen, batch=0):
+    """(count, n) rows of every layer, or (batch, count, n) sequences."""
+    shape = (batch, count) if batch else (count,)
+    return [torch.randn(*shape, layer.in_features, device="cuda", generator=gen).to(torch.bfloat16) for layer in layers.values()]
+
+
+@pytest.mark.parametrize("batch", [0, 2])     # rows summed in the hook, and sampled rows summed when the capture ends
+def test_a_refused_commit_can_be_made_again(tb, batch):
+    layers = _layers([64, 64, 40])
+    stats = tb.ActivationStatistics(layers, head=1000, stride=1, distributed=False)
+    opt = tb.MuonT([l.weight.data.float().requires_grad_() for l in layers.values()])
+    owned = dict(zip((l.weight for l in layers.values()), opt.param_groups[0]["params"]))
+    got = {}
+
+    def update(means):
+        got.clear()
+        got.update(means)
+        opt.update_statistics({owned[w]: m for w, m in means.items()})
+
+    target, gen = types.SimpleNamespace(update_statistics=update), torch.Generator(device="cuda").manual_seed(2)
+    first = _rows(layers, 96, gen, batch)
+    _forward(stats, layers, first)
+    stats.commit(target)
+    second, third = _rows(layers, 80, gen, batch), _rows(layers, 48, gen, batch)
+    _forward(stats, layers, second)
+    with pytest.raises(RuntimeError, match="already updated"):
+        stats.commit(target)                      # the first statistics have not been used yet
+    for p in opt.param_groups[0]["params"]:
+        p.grad = torch.zeros_like(p)
+    opt.step()
+    _forward(stats, layers, third)                # more rows on top of those that are pending
+    stats.commit(target)
+    stats.close()
+    for layer, a, b in zip(layers.values(), second, third):
+        n = layer.in_features
+        x = torch.cat([a.reshape(-1, n), b.reshape(-1, n)]).float().cpu()
+        assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
