@@ -65,3 +65,29 @@ def test_a_refused_commit_can_be_made_again(tb, batch):
         n = layer.in_features
         x = torch.cat([a.reshape(-1, n), b.reshape(-1, n)]).float().cpu()
         assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
+
+
+def test_row_buffers_are_bounded_where_row_counts_vary(tb, monkeypatch):
+    """A new sequence length with every microbatch: what is kept of a width stays below the limit, within a capture and over
+    many, and no row is lost when a buffer makes room."""
+    limit = 3 * 2 * 40 * 64 * 2            # three buffers of 40 rows for two 64-wide layers
+    monkeypatch.setattr(tb.ActivationStatistics, "_ROWS_KEPT", limit)
+    layers = _layers([64, 64, 40])
+    stats, got = tb.ActivationStatistics(layers, head=1000, stride=1, distributed=False), {}
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    seen = [[] for _ in layers]
+    for lengths in ((20,), (21, 33), (40, 12, 40), (70,), (25,), (26, 27, 28, 20)):
+        with stats.capture(), torch.no_grad():
+            for length in lengths:         # several lengths within one capture
+                for j, (layer, x) in enumerate(zip(layers.values(), _rows(layers, length, gen, batch=1))):
+                    layer(x)
+                    seen[j].append(x.reshape(-1, layer.in_features).float().cpu())
+                for n in (64, 40):
+                    assert sum(b.numel() * 2 for key, b in stats._rows.items() if key[0] == n) <= limit
+    stats.commit(types.SimpleNamespace(update_statistics=got.update))
+    for layer, rows in zip(layers.values(), seen):
+        x = torch.cat(rows)
+        assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
+    assert stats._rows
+    stats.close()
+    assert not stats._rows
