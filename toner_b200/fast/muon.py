@@ -74,7 +74,7 @@ class Muon(torch.optim.Optimizer):
             if self._lanes is None:
                 self._lanes = core.Lanes(next(iter(by_shape.values()))[0].device,
                                          [ops.ns_polar_workspace_bytes(len(ms), *shape) for shape, ms in by_shape.items()])
-            jobs = []
+            jobs, held = [], []
             for shape, members in by_shape.items():
                 st = self._stack(gi, shape, members)
                 grads = [p.grad if self.precond is None else self.precond(p, p.grad) for p in members]
@@ -82,7 +82,7 @@ class Muon(torch.optim.Optimizer):
                 key = tuple(x.data_ptr() for x in grads)
                 if st["grad_key"] != key:
                     st["grad_ptrs"], st["grad_key"] = ops.pointer_table(grads), key
-                st["grads"] = grads      # (a converted copy lives until the next step's)
+                held.append(grads)       # (converted copies live until the lanes have been joined)
                 jobs.append(lambda scratch, st=st, shape=shape: self._step_shape(g, shape, st, scratch))
             # (collectives keep one order on every rank)
             self._lanes.run([(i if self.dist is None else 0, job) for i, job in enumerate(jobs)])
