@@ -35,3 +35,14 @@ def test_gradients_are_not_kept(muon):
     opt.zero_grad(set_to_none=True)
     assert all(ref() is None for ref in seen)
     assert before - torch.cuda.memory_allocated() == sum(p.numel() * 4 for p in params)
+
+
+@pytest.mark.parametrize("shapes", [[(512, 512)] * 4, [(256, 512), (512, 256), (512, 512), (512, 1024)]])
+def test_workspaces_are_given_back(muon, shapes):
+    params = _params(*shapes)
+    before = torch.cuda.memory_allocated()
+    opt = muon(params, lr=0.02, distributed=False)
+    opt.step()
+    size = sum(p.numel() * 4 for p in params)
+    assert torch.cuda.memory_allocated() - before <= 2 * size + (64 << 10)     # momentum and direction, tables of addresses
+    del opt

@@ -63,6 +63,10 @@ class Scratch:
             self._buffers[key] = buf
         return buf
 
+    def give_back(self) -> None:
+        """Hand every buffer back to the memory pool (between runs)."""
+        self._buffers.clear()
+
     def joined(self) -> None:
         """The home stream is ordered behind everything that has used this scratch."""
         self.home = None

@@ -86,6 +86,8 @@ class Muon(torch.optim.Optimizer):
                 jobs.append(lambda scratch, st=st, shape=shape: self._step_shape(g, shape, st, scratch))
             # (collectives keep one order on every rank)
             self._lanes.run([(i if self.dist is None else 0, job) for i, job in enumerate(jobs)])
+            for scratch in self._lanes.scratch:     # (workspaces are larger than the state: not held between steps)
+                scratch.give_back()
         return None
 
     def _step_shape(self, g: dict, shape: Tuple[int, int], st: dict, scratch: core.Scratch) -> None:
