@@ -79,8 +79,10 @@ class Lanes:
     them.  Work that runs side by side shares no scratch, so the pieces' scratch (`scratch_bytes`, one number a piece) adds
     up where it was the largest alone before: above 4 GiB more there is one lane -- and problems that large fill the GPU."""
 
+    MOST_ADDED = 4 << 30
+
     def __init__(self, device: torch.device, scratch_bytes: Sequence[int], priority: int = 0) -> None:
-        lanes = min(3, len(scratch_bytes)) if sum(scratch_bytes) - max(scratch_bytes, default=0) <= 4 << 30 else 1
+        lanes = min(3, len(scratch_bytes)) if sum(scratch_bytes) - max(scratch_bytes, default=0) <= self.MOST_ADDED else 1
         self.streams = [torch.cuda.Stream(device=device, priority=priority) for _ in range(lanes - 1)]
         self.scratch = [Scratch() for _ in range(max(lanes, 1))]
 

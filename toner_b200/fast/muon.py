@@ -36,7 +36,8 @@ class Muon(torch.optim.Optimizer):
                              and dist.get_world_size() > 1) else None
         self.precond = None   # optional (p, grad) -> preconditioned gradient, as in the reference
         self._stacks: Dict[Tuple[int, Tuple[int, int]], dict] = {}
-        self._lanes = None   # streams the shapes run on side by side (created at the first step)
+        # parameter group -> the workspaces of its shapes, and the streams they run on side by side
+        self._lanes: Dict[int, Tuple[Tuple[int, ...], core.Lanes]] = {}
 
     def _stack(self, gi: int, shape: Tuple[int, int], members: List[torch.nn.Parameter]) -> dict:
         """Momentum buffers of one shape live in one (count, rows, cols) stack; state[p]['momentum_buffer'] are views."""
@@ -71,9 +72,10 @@ class Muon(torch.optim.Optimizer):
                 by_shape.setdefault(tuple(p.shape), []).append(p)
             if not by_shape:
                 continue
-            if self._lanes is None:
-                self._lanes = core.Lanes(next(iter(by_shape.values()))[0].device,
-                                         [ops.ns_polar_workspace_bytes(len(ms), *shape) for shape, ms in by_shape.items()])
+            need = tuple(ops.ns_polar_workspace_bytes(len(ms), *shape) for shape, ms in by_shape.items())
+            if self._lanes.get(gi, (None,))[0] != need:      # (more or other parameters have gradients)
+                self._lanes[gi] = need, core.Lanes(next(iter(by_shape.values()))[0].device, need)
+            lanes = self._lanes[gi][1]
             jobs, held = [], []
             for shape, members in by_shape.items():
                 st = self._stack(gi, shape, members)
@@ -85,8 +87,8 @@ class Muon(torch.optim.Optimizer):
                 held.append(grads)       # (converted copies live until the lanes have been joined)
                 jobs.append(lambda scratch, st=st, shape=shape: self._step_shape(g, shape, st, scratch))
             # (collectives keep one order on every rank)
-            self._lanes.run([(i if self.dist is None else 0, job) for i, job in enumerate(jobs)])
-            for scratch in self._lanes.scratch:     # (workspaces are larger than the state: not held between steps)
+            lanes.run([(i if self.dist is None else 0, job) for i, job in enumerate(jobs)])
+            for scratch in lanes.scratch:     # (workspaces are larger than the state: not held between steps)
                 scratch.give_back()
         return None
 
