@@ -52,7 +52,7 @@ def test_every_group_has_the_lanes_its_workspaces_allow(muon, monkeypatch):
     """Two small shapes in the first group, two large ones in the second, and a large one whose gradient comes later in the
     first: the limit holds for each, and a group of one shape keeps another group from no lane."""
     from toner_b200 import core
-    monkeypatch.setattr(core.Lanes, "MOST_ADDED", 4 << 20)
+    monkeypatch.setattr(core.Lanes, "MOST_ADDED", 3 << 20)
     small, large = [(64, 64), (64, 136)], [(512, 512), (512, 1024)]
     first, second = _params(*small, (512, 512), (512, 520)), _params(*large)
     late = first[2:]
