@@ -91,3 +91,31 @@ def test_row_buffers_are_bounded_where_row_counts_vary(tb, monkeypatch):
     assert stats._rows
     stats.close()
     assert not stats._rows
+
+
+@pytest.mark.parametrize("batch", [0, 3])
+def test_layers_on_another_stream(tb, batch):
+    """The second layer runs on a side stream, behind a delay, and its input is overwritten there right after; what ends the
+    capture and the commit runs on the main stream, which does not wait for the side stream."""
+    layers = _layers([64, 64, 64])
+    stats, got = tb.ActivationStatistics(layers, head=1000, stride=1, distributed=False), {}
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    rows, side = _rows(layers, 48, gen, batch), torch.cuda.Stream()
+    buf = torch.zeros_like(rows[1])
+    side.wait_stream(torch.cuda.current_stream())
+    with stats.capture(), torch.no_grad():
+        for i, (layer, x) in enumerate(zip(layers.values(), rows)):
+            with torch.cuda.stream(side if i == 1 else torch.cuda.current_stream()):
+                if i == 1:
+                    torch.cuda._sleep(20_000_000)
+                    buf.copy_(x)
+                    layer(buf)
+                    buf.zero_()
+                else:
+                    layer(x)
+    stats.commit(types.SimpleNamespace(update_statistics=got.update))
+    stats.close()
+    for layer, x in zip(layers.values(), rows):
+        x = x.reshape(-1, 64).float().cpu()
+        assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
+    torch.cuda.synchronize()
