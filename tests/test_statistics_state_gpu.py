@@ -1,5 +1,7 @@
 """What ActivationStatistics keeps between its calls: sums after a refused commit, row buffers, streams and process groups."""
 
+import threading
+import time
 import types
 
 import pytest
@@ -119,3 +121,29 @@ def test_layers_on_another_stream(tb, batch):
         x = x.reshape(-1, 64).float().cpu()
         assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
     torch.cuda.synchronize()
+
+
+def test_layers_in_several_threads(tb):
+    """Two layers of one width in two threads: neither takes the other's place among the sums."""
+
+    class Slow(dict):
+        def get(self, *args):
+            value = super().get(*args)
+            time.sleep(0.05)               # another thread may run between the look and the store
+            return value
+
+    layers = _layers([64, 64])
+    stats, got = tb.ActivationStatistics(layers, distributed=False), {}
+    rows = _rows(layers, 48, torch.Generator(device="cuda").manual_seed(9))
+    stats._slots = Slow()
+    with stats.capture(), torch.no_grad():
+        threads = [threading.Thread(target=lambda l=layer, x=x: l(x)) for layer, x in zip(layers.values(), rows)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    stats.commit(types.SimpleNamespace(update_statistics=got.update))
+    stats.close()
+    for layer, x in zip(layers.values(), rows):
+        x = x.float().cpu()
+        assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
