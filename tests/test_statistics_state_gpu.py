@@ -147,3 +147,29 @@ def test_layers_in_several_threads(tb):
     for layer, x in zip(layers.values(), rows):
         x = x.float().cpu()
         assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
+
+
+@pytest.mark.parametrize("when", ["before commit", "between captures", "gone"])
+def test_a_process_group_that_comes_or_goes(tb, monkeypatch, when):
+    """Sums may be begun before a process group is initialised, or go on after one has been destroyed."""
+    from toner_b200 import statistics
+    there = [when == "gone"]
+    monkeypatch.setattr(statistics.dist, "is_initialized", lambda: there[0])
+    monkeypatch.setattr(statistics.dist, "all_reduce", lambda *a, **kw: None)     # (a group of one process)
+    layers = _layers([64, 64, 40])
+    stats, got = tb.ActivationStatistics(layers, head=1000, stride=1), {}
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    seen = [[] for _ in layers]
+    for step, batch in enumerate((2, 0, 2, 0)):
+        rows = _rows(layers, 30 + step, gen, batch)
+        _forward(stats, layers, rows)
+        for j, x in enumerate(rows):
+            seen[j].append(x.reshape(-1, x.shape[-1]).float().cpu())
+        if step == 1 and when != "before commit":
+            there[0] = not there[0]
+    there[0] = when != "gone"
+    stats.commit(types.SimpleNamespace(update_statistics=got.update))
+    for layer, rows in zip(layers.values(), seen):
+        x = torch.cat(rows)
+        assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
+    stats.close()
