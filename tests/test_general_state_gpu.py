@@ -1,0 +1,40 @@
+"""State of the general optimizers in unusual but legal circumstances: empty parameter groups, a step that is refused."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tb():
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    import toner_b200
+    return toner_b200
+
+
+def _params(*shapes):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    params = [torch.nn.Parameter(torch.randn(*s, device="cuda", generator=g) * 0.02) for s in shapes]
+    for p in params:
+        p.grad = torch.randn(*p.shape, device="cuda", generator=g) * 1e-3
+    return params
+
+
+def _statistics(params):
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rows = [torch.randn(300, p.shape[1], device="cuda", generator=g) for p in params]
+    return {p: x.T @ x / 300 for p, x in zip(params, rows)}
+
+
+@pytest.mark.parametrize("kind", ["MuonT", "AdamT"])
+def test_a_first_group_without_parameters(tb, kind):
+    results = []
+    for groups in (lambda p: [{"params": []}, {"params": p}], lambda p: [{"params": p}]):
+        params = _params((64, 72), (72, 64))
+        opt = getattr(tb, kind)(groups(params), lr=1e-3)
+        opt.update_statistics(_statistics(params))
+        opt.step()
+        results.append([p.detach().clone() for p in params])
+    assert all(torch.equal(a, b) for a, b in zip(*results))

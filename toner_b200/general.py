@@ -124,13 +124,15 @@ class _TonerGeneral(Optimizer):
             self._health = ops.Health()
         stacked: Dict[Tuple[int, Tuple[int, int]], List[Tensor]] = {}
         for gi, group in enumerate(self.param_groups):
-            core.root_orders(*self._strengths(group))
             for p in group["params"]:
                 if not p.is_contiguous():
                     raise ValueError("toner_b200 needs contiguous weights")
                 stacked.setdefault((gi, tuple(p.shape)), []).append(p)
+        for gi, _ in stacked:
+            core.root_orders(*self._strengths(self.param_groups[gi]))
         muont = self._kind == "muont"
-        self._lanes = core.Lanes(self.param_groups[0]["params"][0].device, [
+        device = next((ps[0].device for ps in stacked.values()), None)     # (any group may be empty)
+        self._lanes = core.Lanes(device, [
             ops.inv_roots_workspace_bytes(len(ps), shape[1]) + (ops.ns_polar_workspace_bytes(len(ps), *shape) if muont else 0)
             for (_, shape), ps in stacked.items()])
         for gi, group in enumerate(self.param_groups):
