@@ -38,3 +38,20 @@ def test_a_first_group_without_parameters(tb, kind):
         opt.step()
         results.append([p.detach().clone() for p in params])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_a_refused_adamt_step_counts_for_nobody(tb):
+    """Two parameters of one shape that have taken different numbers of steps are refused; those of the shape before them must
+    not count a step that changed no weight."""
+    first, second = _params((64, 72)), _params((72, 64), (72, 64))
+    params = first + second
+    opt = tb.AdamT(params, lr=1e-3)
+    opt.update_statistics(_statistics(params))
+    opt.step()
+    weights = [p.detach().clone() for p in params]
+    opt.state[second[0]]["step"] = 5
+    opt.update_statistics(_statistics(params))
+    with pytest.raises(RuntimeError, match="same number of steps"):
+        opt.step()
+    assert [opt.state[p]["step"] for p in params] == [1, 5, 1]
+    assert all(torch.equal(p, w) for p, w in zip(params, weights))

@@ -413,10 +413,10 @@ class AdamT(_TonerGeneral):
                                    weight_decay=group["weight_decay"], betas=tuple(group["betas"]), eps=group["eps"], t=t)
             core.apply_group_delta(bucket.group, bucket.delta)
 
-        for _, bucket in work:
-            steps = {self.state[p].get("step", 0) for p in bucket.params}
-            if len(steps) != 1:
-                raise RuntimeError("parameters stacked together must have taken the same number of steps")
+        taken = [{self.state[p].get("step", 0) for p in bucket.params} for _, bucket in work]
+        if any(len(steps) != 1 for steps in taken):      # (before any of them counts this one)
+            raise RuntimeError("parameters stacked together must have taken the same number of steps")
+        for (_, bucket), steps in zip(work, taken):
             t = steps.pop() + 1
             for i, p in enumerate(bucket.params):
                 st = self.state[p]
