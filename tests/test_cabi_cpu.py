@@ -55,3 +55,37 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
         assert "no CPU or PyTorch fallback" in str(e)
     else:
         raise AssertionError("loading a missing library must raise")
+
+
+def test_fused_entry_points_refuse_bad_arguments_before_they_touch_the_device():
+    """What a kernel would turn into a fault is an argument error (1) on the host, whether there is a device or not.  The
+    addresses are made up: nothing may be launched."""
+    from toner_b200 import _lib
+    lib, at = _lib.load(), 1 << 20
+    group = _lib.MatrixGroup()
+    for name, _ in _lib.MatrixGroup._fields_[:18]:
+        setattr(group, name, at)
+    group.count, group.rows, group.cols, group.factors, group.first, group.step = 2, 16, 16, 3, 1, 1
+
+    every = {"muont_input", "muont_delta", "adamt_delta"}
+    for field, value, refuse in (("grads", None, {"muont_input", "adamt_delta"}), ("weights", None, {"muont_delta", "adamt_delta"}),
+                                 ("inner_inv", None, {"muont_input", "adamt_delta"}), ("outer_inv", None, {"muont_delta", "adamt_delta"}),
+                                 ("outer_planes", None, {"muont_delta", "adamt_delta"}), ("first", 2, every), ("first", -1, every),
+                                 ("step", 2, every), ("m", at + 4, every), ("work", at + 8, every), ("planes", at + 2, every)):
+        bad = type(group).from_buffer_copy(group)
+        setattr(bad, field, value)
+        p = ctypes.byref(bad)
+        if "muont_input" in refuse:
+            assert lib.toner_muont_input(p, 0.9, 1, None) == 1, field
+        if "muont_delta" in refuse:
+            assert lib.toner_muont_delta(p, None, 0.1, 0.1, 1.0, at, None) == 1, field
+        if "adamt_delta" in refuse:
+            assert lib.toner_adamt_delta(p, 0.1, 0.1, 0.9, 0.9, 0.1, 0.1, 1e-8, at, None) == 1, field
+    pointers = lambda *a: (ctypes.c_void_p * len(a))(*a)  # noqa: E731
+    assert lib.toner_list_axpby(pointers(at, at), pointers(at, None), 2, 16, 0.5, 0.5, None) == 1
+    assert lib.toner_list_axpby(pointers(at, at), pointers(at, at + 4), 2, 16, 0.5, 0.5, None) == 1
+    assert lib.toner_list_finite(pointers(at, None), 2, 16, at, None) == 1
+    assert lib.toner_syrk_upper_ws(None, at, 0, 1, 4096, 64, 64, at, 2, 0.0, 1.0, at + 4, 1 << 20, None) == 1
+    planes = lambda lo, hi: lib.toner_inv_roots_planes(  # noqa: E731
+        at, 1, 64, 1e-3, 4, 2, 0, 0.0, 0, at, at, at, at, None, None, None, None, 0, None, 0, None, lo, at, hi, at, at, 1 << 30, None)
+    assert planes(at + 8, at) == 1 and planes(at, at + 2) == 1

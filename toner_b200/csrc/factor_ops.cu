@@ -1428,13 +1428,15 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
                            void* lo_planes, float* lo_inv, void* hi_planes, float* hi_inv,
                            void* workspace, size_t workspace_bytes, void* stream_) {
   using namespace toner;
-  Context* ctx = context();
-  if (!ctx) return kErrCuda;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!ema || !root_lo || !workspace) return fail(kErrArg, "inv_roots: null pointer");
   if (k <= 0 || n <= 0) return fail(kErrArg, "inv_roots: sizes must be positive");
   if (!lo_planes != !lo_inv || !hi_planes != !hi_inv || (hi_planes && q == 1))
     return fail(kErrArg, "inv_roots: planes come with their inverse scales, the second root's only where there is one");
+  if ((reinterpret_cast<uintptr_t>(lo_planes) | reinterpret_cast<uintptr_t>(hi_planes)) & 15u)
+    return fail(kErrArg, "inv_roots: operand planes must be 16-byte aligned");
+  Context* ctx = context();
+  if (!ctx) return kErrCuda;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (n % 8 != 0) return fail(kErrUnsupported, "inv_roots: n must be a multiple of 8");
   if (!(damping > 0.f)) return fail(kErrArg, "inv_roots: damping must be positive");
   if (p < 1 || p > 32 || (p & (p - 1))) return fail(kErrUnsupported, "inv_roots: root order p must be a power of two <= 32");

@@ -300,6 +300,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   if (d.packed && (!d.tri || d.mirror || d.d16)) return fail(kErrArg, "gemm: packed output is upper-triangle FP32 only");
   if (!d.d && !d.d16 && !d.split0 && !d.split1) return fail(kErrArg, "gemm: no output");
   if (d.packed && (d.split0 || d.split1)) return fail(kErrArg, "gemm: operand planes cannot be packed");
+  if (reinterpret_cast<uintptr_t>(d.split_ws) & 15u) return fail(kErrArg, "gemm: split_ws must be 16-byte aligned");
   if (d.fmt != 0 && d.fmt != 1) return fail(kErrArg, "gemm: fmt must be 0 (FP16) or 1 (BF16)");
 
   int bn = d.tile_n, splits = 1;

@@ -440,6 +440,7 @@ int toner_syrk_upper_ws(const void* const* x_list, const void* x_base, int64_t x
   if ((!x_list && !x_base) || !out) return fail(kErrArg, "syrk: null pointer");
   if (k <= 0 || rows <= 0 || n <= 0) return fail(kErrArg, "syrk: sizes must be positive");
   if (n % 8 != 0 || ld % 8 != 0) return fail(kErrArg, "syrk: n and ld must be multiples of 8");
+  if (reinterpret_cast<uintptr_t>(workspace) & 15u) return fail(kErrArg, "syrk: the workspace must be 16-byte aligned");
   const bool keep_order = (mode & TONER_SYRK_KEEP_ORDER) != 0;
   mode &= ~TONER_SYRK_KEEP_ORDER;
   if (mode < 0 || mode > 2)
@@ -530,9 +531,12 @@ int toner_unpack_ema(const float* packed, float* ema, int32_t k, int32_t n, floa
 static int list_call(const float* const* src, float* const* dst, int32_t count, int64_t numel, float beta, float gamma, int32_t* flag,
                      void* stream_) {
   using namespace toner;
+  if (!src || count <= 0 || numel <= 0 || numel % 4) return fail(kErrArg, "matrix list: the size must be a positive multiple of 4");
+  for (int i = 0; i < count; ++i)
+    if (!src[i] || (dst && !dst[i]) || (reinterpret_cast<uintptr_t>(src[i]) & 15u) || (dst && (reinterpret_cast<uintptr_t>(dst[i]) & 15u)))
+      return fail(kErrArg, "matrix list: pointers must be set and 16-byte aligned");
   Context* ctx = context();
   if (!ctx) return kErrCuda;
-  if (!src || count <= 0 || numel <= 0 || numel % 4) return fail(kErrArg, "matrix list: the size must be a positive multiple of 4");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   for (int first = 0; first < count; first += kListMax) {
     PointerList list;
@@ -540,8 +544,6 @@ static int list_call(const float* const* src, float* const* dst, int32_t count, 
     for (int i = 0; i < here; ++i) {
       list.src[i] = src[first + i];
       list.dst[i] = dst ? dst[first + i] : nullptr;
-      if (!list.src[i] || (reinterpret_cast<uintptr_t>(list.src[i]) & 15u) || (reinterpret_cast<uintptr_t>(list.dst[i]) & 15u))
-        return fail(kErrArg, "matrix list: pointers must be set and 16-byte aligned");
     }
     const int bx = blocks_for(numel / 4, 256 * 4, 8 * ctx->num_sms / (here < 8 ? here : 8) + 1);
     if (dst) TONER_LAUNCH(list_axpby_kernel, dim3(bx, here), 256, stream, list, numel / 4, beta, gamma);

@@ -500,13 +500,22 @@ static int right_product(const toner_matrix_group& g, bool outer, float* d, bool
   return launch_gemm(q, stream);
 }
 
-static int check_group(const char* what, const toner_matrix_group* g) {
-  if (!context()) return kErrCuda;
+// Everything is looked at before the first launch: the moments must not advance in a call that then fails.
+static int check_group(const char* what, const toner_matrix_group* g, bool grads, bool weights, bool inner, bool outer,
+                       const float* delta) {
   if (!g || g->count <= 0 || g->rows <= 0 || g->cols <= 0 || g->factors <= 0 || !g->m || !g->work || !g->planes || !g->inv ||
       !g->maxabs || !g->c1 || !g->c2)
     return fail(kErrArg, std::string(what) + ": bad matrix group");
+  if ((grads && !g->grads) || (weights && !g->weights) || (inner && (!g->inner_planes || !g->inner_inv)) ||
+      (outer && (!g->outer_planes || !g->outer_inv)))
+    return fail(kErrArg, std::string(what) + ": null pointer in the matrix group");
+  if (g->first < 0 || g->step < 0 || (long long)g->first + (long long)(g->count - 1) * g->step >= g->factors)
+    return fail(kErrArg, std::string(what) + ": the group's statistics lie outside the factors");
+  for (const void* p : {(const void*)g->m, (const void*)g->v, (const void*)g->work, (const void*)g->work2, (const void*)g->planes,
+                        (const void*)delta})
+    if (reinterpret_cast<uintptr_t>(p) & 15u) return fail(kErrArg, std::string(what) + ": stacks must be 16-byte aligned");
   if (g->rows % 8 || g->cols % 8) return fail(kErrUnsupported, std::string(what) + ": matrix dimensions must be multiples of 8");
-  return 0;
+  return context() ? 0 : kErrCuda;
 }
 
 static int split_stack(const toner_matrix_group& g, const float* x, const float* const* list, const uint32_t* maxabs, uint32_t* scratch,
@@ -516,7 +525,7 @@ static int split_stack(const toner_matrix_group& g, const float* x, const float*
 }
 
 int toner_muont_input(const toner_matrix_group* g, float mu, int32_t nesterov, void* stream_) {
-  if (int rc = check_group("muont_input", g)) return rc;
+  if (int rc = check_group("muont_input", g, true, false, g && g->inner_planes, false, nullptr)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   int rc = toner_muont_momentum(g->grads, g->m, g->work, g->count, (int64_t)g->rows * g->cols, mu, nesterov, g->maxabs, stream);
   if (rc || !g->inner_planes) return rc;
@@ -527,8 +536,8 @@ int toner_muont_input(const toner_matrix_group* g, float mu, int32_t nesterov, v
 
 int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs, float lr, float weight_decay, float scale,
                       float* delta, void* stream_) {
-  if (int rc = check_group("muont_delta", g)) return rc;
-  if (!delta || !g->outer_planes || !g->outer_fro2) return fail(kErrArg, "muont_delta: null pointer");
+  if (!delta || !g || !g->outer_fro2) return fail(kErrArg, "muont_delta: null pointer");
+  if (int rc = check_group("muont_delta", g, false, weight_decay != 0.f, false, true, delta)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   uint32_t* const w_max = g->maxabs + g->count;       // cleared by the coefficient kernel, with the next
   uint32_t* const v_max = g->maxabs + 2 * g->count;
@@ -550,9 +559,9 @@ int toner_muont_delta(const toner_matrix_group* g, const uint32_t* polar_maxabs,
 
 int toner_adamt_delta(const toner_matrix_group* g, float lr, float weight_decay, float beta1, float beta2, double bc1, float bc2,
                       float eps, float* delta, void* stream_) {
-  if (int rc = check_group("adamt_delta", g)) return rc;
-  if (!delta || !g->v || !g->work2 || !g->ss || !g->ss_scratch || !g->inner_planes || !g->outer_fro2)
+  if (!delta || !g || !g->v || !g->work2 || !g->ss || !g->ss_scratch || !g->outer_fro2)
     return fail(kErrArg, "adamt_delta: null pointer");
+  if (int rc = check_group("adamt_delta", g, true, weight_decay != 0.f, true, weight_decay != 0.f, delta)) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   Context* ctx = context();
   const long long per = (long long)g->rows * g->cols;
