@@ -40,7 +40,7 @@ def _rows(layers, count, gen, batch=0):
 def test_a_refused_commit_can_be_made_again(tb, batch):
     layers = _layers([64, 64, 40])
     stats = tb.ActivationStatistics(layers, head=1000, stride=1, distributed=False)
-    opt = tb.MuonT([l.weight.data.float().requires_grad_() for l in layers.values()])
+    opt = tb.MuonT([l.weight.data.float().requires_grad_() for l in layers.values()], lr=1e-3)
     owned = dict(zip((l.weight for l in layers.values()), opt.param_groups[0]["params"]))
     got = {}
 

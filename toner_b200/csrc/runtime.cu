@@ -54,6 +54,16 @@ Context* context() {
     set_error("no CUDA device is current: toner_b200 has no CPU path");
     return nullptr;
   }
+  // Tensor maps are encoded by the driver on the launching thread, which has no context of its own until the runtime has
+  // made a call on it that needs one: a thread's first call may be a product.
+  static thread_local int bound = -1;
+  if (bound != dev) {
+    if (cudaSetDevice(dev) != cudaSuccess) {
+      set_error("cudaSetDevice failed");
+      return nullptr;
+    }
+    bound = dev;
+  }
   std::lock_guard<std::mutex> lock(g_mutex);
   Context& c = g_ctx[dev];
   if (c.device == dev) return &c;
