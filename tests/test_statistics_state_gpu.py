@@ -173,3 +173,21 @@ def test_a_process_group_that_comes_or_goes(tb, monkeypatch, when):
         x = torch.cat(rows)
         assert orc.rel_fro(got[layer.weight].cpu(), orc.gram(x) / x.shape[0]) < 2e-6
     stats.close()
+
+
+def test_a_layer_whose_rows_were_never_summed_is_absent(tb, monkeypatch):
+    """Its hook failed after it had been given a place among the sums, and the caller went on."""
+    from toner_b200 import ops
+    layers = _layers([64, 64])
+    stats = tb.ActivationStatistics(layers, distributed=False)
+    rows = _rows(layers, 48, torch.Generator(device="cuda").manual_seed(11))
+    real = ops.syrk_upper
+    with stats.capture(), torch.no_grad():
+        layers["l0"](rows[0])
+        monkeypatch.setattr(ops, "syrk_upper", lambda *a, **kw: (_ for _ in ()).throw(RuntimeError("refused")))
+        with pytest.raises(RuntimeError, match="refused"):
+            layers["l1"](rows[1])
+        monkeypatch.setattr(ops, "syrk_upper", real)
+    with pytest.raises(RuntimeError, match="nothing was captured for layer.*l1"):
+        stats.commit(types.SimpleNamespace(update_statistics=lambda means: pytest.fail("committed")))
+    stats.close()
