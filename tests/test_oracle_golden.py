@@ -28,10 +28,17 @@ def test_position_counts_of_the_benchmark_configurations():
 def test_input_factors(golden, tag, s_in, s_out):
     g = golden("factors.npz")
     inner, outer, decay = orc.input_factors(t(g[f"{tag}_c"]), s_in, s_out, 1e-3)
-    # same LAPACK, same arithmetic: agreement to rounding of the eigensolver
-    assert orc.rel_fro(inner, t(g[f"{tag}_inner"])) < 2e-5
-    assert orc.rel_fro(outer, t(g[f"{tag}_outer"])) < 2e-5
-    assert orc.rel_fro(decay, t(g[f"{tag}_decay"])) < 2e-5
+    # The same arithmetic on an FP32 eigensolver that rounds as the host CPU's kernels do: it decomposes A + E exactly with
+    # ||E|| about half a unit in the last place of ||A||, which moves A^-s by up to s ||E|| / lambda_min of itself; once here
+    # and once where the fixture was written.  (One host repeats the fixture to 2e-5; another differs by 0.2 to 0.27 of this
+    # bound, and both are as far from FP64.)
+    a = t(g[f"{tag}_c"]).double()
+    a = 0.5 * (a + a.T)
+    lam = torch.linalg.eigvalsh(a / a.diagonal().mean()) + 1e-3
+    bound = 2.0 ** -23 * float(lam.max() / lam.min())
+    assert orc.rel_fro(inner, t(g[f"{tag}_inner"])) < s_in * bound
+    assert orc.rel_fro(outer, t(g[f"{tag}_outer"])) < s_out * bound
+    assert orc.rel_fro(decay, t(g[f"{tag}_decay"])) < 2 * s_out * bound
     assert abs(float(decay.diagonal().mean()) - 1.0) < 1e-5
 
 
