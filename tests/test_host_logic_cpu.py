@@ -212,18 +212,19 @@ def test_lanes_are_bounded_by_the_scratch_they_add():
 
 @pytest.mark.parametrize("p", [2, 4, 8, 16])
 def test_products_of_the_finish(p):
-    """Degree 6 takes three products, odd degrees from 5 (from 7 below p = 8) half of Horner's and one, the rest Horner's."""
+    """Degree 6 takes three products from p = 4 on, odd degrees from 5 (from 7 below p = 8) half of Horner's and one, the rest
+    Horner's."""
     from toner_b200 import ops
     seen = set()
-    for lower in (0.4, 0.2, 0.15, 0.1, 0.05, 0.03, 0.02, 0.0104, 0.0084):
+    for lower in (0.4, 0.2, 0.15, 0.1, 0.0688, 0.05, 0.03, 0.02, 0.0104, 0.0084):
         m = ops.inv_roots_finish_order(768, 1e-3, p, lower)
-        short = m == 6 or m == 7 or (m == 5 and p >= 8)
+        short = m == 7 or (m == 6 and p >= 4) or (m == 5 and p >= 8)
         want = m // 2 + (m & 1) if short else m - 1
         assert ops.inv_roots_finish_products(768, 1e-3, p, lower) == want
         assert ops.inv_roots_finish_products(768, 1e-3, p, 1e-4, interleave=False) == \
             ops.inv_roots_finish_order(768, 1e-3, p, 1e-4) - 1
         seen.add(m)
-    assert seen & {6, 7}
+    assert seen & {6, 7} and (p != 8 or 8 in seen)
 
 
 def test_the_plane_order_keeps_horners_finish_at_every_bound():

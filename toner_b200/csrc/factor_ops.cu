@@ -156,10 +156,13 @@ static bool finish_fit(int p, double lo, double hi, int m, double tail, FitSampl
 // y = r (r + beta) leaves (..(w y + l_1(r)) y + ..) y + l_k(r) with linear l_i, which cost no product (they enter it in FP32);
 // beta is chosen so that the innermost quotient is affine in y itself, top y + top0.  m = 6: q itself, three products for five.
 // m odd: q = c_0 + c_1 r + r v(r) with v of degree m - 1 divided so (m = 7: four products for six).  What the single planes
-// (11 bits) of the products lose -- every operand's rounding, carried through, over the eigenvalues of the benchmark's and of
-// equally spaced spectra -- is 0.5 to 0.97 of Horner's for m = 6 and 0.86 to 0.98 for m = 7; q itself divided with m = 7, or m
-// = 4, reaches 1.7: near r = 0, where most eigenvalues are, an error must fall with r^2 as Horner's does.  m = 5: 0.97 to 1.01
-// from p = 8 on, 1.05 below, where it keeps Horner's rule.  32 statistics of width 2048, m = 7: two products of 350 us each go.
+// (11 bits) of the products lose shows in the roots as follows, short form against Horner's, error against FP64 of statistics
+// of width 768 and 1024 (Marchenko-Pastur spectra of 1.2 to 36 rows a column, log-uniform ones of condition 10 to 1e3): m = 6
+// 0.92 to 1.02 for p = 4 and 8 but up to 1.25 for p = 2, which keeps Horner's rule; m = 7 0.83 to 1.00; m = 5 1.00 from p = 8
+// on, 1.05 below, where it keeps Horner's rule too.  m = 8 (rare: p = 8, a lower bound near 5e-4, 6.5e-3, 0.069) reaches 1.18 and
+// keeps it as well, like any other even degree; q itself divided with m = 7, or m = 4, reaches 1.7: near r = 0, where most
+// eigenvalues are, an error must fall with r^2 as Horner's does.  32 statistics of width 2048, m = 7: two products of 350 us
+// each go.
 struct QuadraticSteps {
   double beta = 0.0, top = 0.0, top0 = 0.0;
   bool by_r = false;                            // a last step by r (m odd)
@@ -167,7 +170,7 @@ struct QuadraticSteps {
 };
 static bool quadratic_steps(const FinishPoly& fin, int p, QuadraticSteps& out) {
   const int m = fin.order;
-  if (m < 5 || (m == 5 && p < 8)) return false;
+  if ((m & 1) != 0 ? (m < 5 || (m == 5 && p < 8)) : (m != 6 || p < 4)) return false;
   out.by_r = (m & 1) != 0;
   int deg = out.by_r ? m - 1 : m;
   double q[kMaxFinishOrder + 1];
