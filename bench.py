@@ -133,18 +133,18 @@ class ClockSampler:
 
 
 # DRAM bytes per launch of the dominant kernel from the ncu capture summarised in profiles/gemm_tcgen05_kernel_ncu.md:
-# the factor engine's M-update product moved 564 MB (dram__bytes_read + write) for 8 statistics of 2048^2; traffic is
+# the factor engine's M-update product moved 520 MB (dram__bytes_read + write) for 8 statistics of 2048^2; traffic is
 # proportional to the operand size (every operand byte is read from DRAM once), so a launch over k statistics of
-# width n moves 564e6 * k n^2 / (8 * 2048^2).
+# width n moves 520e6 * k n^2 / (8 * 2048^2).
 def roots_traffic(k: int, n: int) -> int:
-    return int(564e6 * k * n * n / (8 * 2048 * 2048))
+    return int(520e6 * k * n * n / (8 * 2048 * 2048))
 
 
 # The update phase's largest launch is the Newton-Schulz x-update of the widest role group (x <- a x + B x: reads B and x
 # in BF16 and x in FP32, writes x in FP32 and BF16).  Its capture on 24 matrices of 2048^2 (section 5 of the same
-# summary) moved 821 + 553 MB; the traffic is proportional to the number of elements of x.
+# summary) moved 817 + 556 MB; the traffic is proportional to the number of elements of x.
 def update_traffic(count: int, m: int, n: int) -> int:
-    return int(1374e6 * count * m * n / (24 * 2048 * 2048))
+    return int(1373e6 * count * m * n / (24 * 2048 * 2048))
 
 
 def tri_fraction(n: int, bm: int = 128, bn: int = 256) -> float:

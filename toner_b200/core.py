@@ -27,7 +27,7 @@ from . import _lib, ops
 
 
 class Scratch:
-    """Named persistent device buffers.  Stable addresses keep the library's TMA tensor maps cached."""
+    """Named device buffers that outlive a call, so that a step allocates nothing."""
 
     def __init__(self) -> None:
         self._buffers: Dict[Tuple, torch.Tensor] = {}

@@ -87,9 +87,10 @@ constexpr int kPowerSteps = 6;
 // at the lower end and the allowance an estimated bound is verified with at the upper end) of the smallest degree
 // whose relative error stays below kFinishTail there.  Spreading the error over the interval takes about half
 // the degree of the binomial series, whose error sits at r = e alone (e = 0.5, p = 8: degree 6 instead of 12).
-// The powers come from m - 1 single-pass products of FP16 planes in Horner form (a third of a split-precision
-// product each; R is small, so its rounding to FP16 costs about 5e-4 c_2 e^2), which is cheaper than the log2(p) + 2
-// split-precision products of one more Newton step; the step count is the one with the fewest plane passes in total.
+// The powers come from single-pass products of FP16 planes (a third of a split-precision product each; R is small, so its
+// rounding to FP16 costs about 5e-4 c_2 e^2), m - 1 in Horner form and about half as many in steps of R (R + beta I) where
+// quadratic_steps() allows them.  Either is cheaper than the log2(p) + 2 split-precision products of one more Newton step; the
+// step count is the one with the fewest plane passes in total, Horner's counted.
 constexpr double kFinishRadius = 0.6;
 constexpr int kMaxFinishOrder = 12;
 constexpr double kFinishTail = 3e-6;

@@ -2,8 +2,9 @@
 //
 //   D[b] = alpha_b * sum_seg A_seg[b] * B_seg[b]^T   (+ beta_b * C[b])
 //
-// One persistent CTA per SM (or one CTA pair per SM pair: cta_group::2, 256 x 256 or 256 x 512 tiles), warp-specialised:
-//   warp 0      TMA producer: 128-byte-swizzled operand tiles into a shared-memory ring
+// One persistent CTA per SM (or one CTA pair per SM pair: cta_group::2, 256 x 128, 256 x 256 or 256 x 512 tiles),
+// warp-specialised:
+//   warps 0, 2  TMA producers: 128-byte-swizzled tiles of A (warp 0) and of B (warp 2) into a shared-memory ring
 //   warp 1      allocates tensor memory and issues tcgen05.mma (one thread), accumulating in TMEM
 //   warps 4..11 epilogue: tcgen05.ld the accumulator (double-buffered, so it overlaps the next chain's
 //               MMAs), sum chains in registers, apply the affine epilogue, store FP32 / 16-bit results
@@ -32,7 +33,7 @@ constexpr int kBM = 128;          // tile rows (UMMA M)
 constexpr int kBK = 64;           // 16-bit elements per k-block: one 128-byte swizzle row
 constexpr int kUmmaK = 16;        // K per tcgen05.mma for 16-bit operands
 constexpr int kMaxSegs = 3;
-constexpr int kGemmThreads = 384;      // warpgroup 0: TMA warp, MMA warp, two idle; warpgroups 1-2: epilogue
+constexpr int kGemmThreads = 384;      // warpgroup 0: A's TMA warp, MMA warp, B's TMA warp, one idle; warpgroups 1-2: epilogue
 constexpr long long kWaitCycles = 4000000000LL;  // about two seconds; a healthy wait is microseconds
 constexpr long long kDrainCycles = 2000000LL;    // per stage, after an abort: about a millisecond for copies in flight
 constexpr long long kSettleCycles = 200000LL;    // after an abort: a CTA of a pair lets copies it cannot observe land
@@ -113,7 +114,7 @@ __host__ __device__ inline int gemm_tiles_per_batch(int M, int N, int BN, int tr
 }
 
 // kPair: two CTAs of a cluster work on one 256 x BN tile (cta_group::2); each holds 128 rows of A and BN/2
-// rows of B per stage, so a stage is two thirds the size and the ring two stages deeper.
+// rows of B per stage: 32 KB for a 256 x 256 tile, where a single CTA's 128 x 256 takes 48.
 // BN = 512 (pairs only) is the wide tile: two 256-column MMAs per k-step share the A rows, which cuts the operand
 // bytes fetched per flop by a quarter (48 KB per CTA and k-block for twice the work of 32 KB).  Its accumulator
 // fills all 512 columns of tensor memory, so there is no second buffer: the epilogue of a tile overlaps the next
@@ -453,7 +454,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 }
 
 // kChained: the kernel sums several accumulation chains per tile in registers (p.promote > 0).
-// kPair: launched as clusters of two CTAs that share each 256 x BN tile (BN = 256): both load their halves of
+// kPair: launched as clusters of two CTAs that share each 256 x BN tile (BN = 128, 256 or 512): both load their halves of
 // the operands, the leader CTA's MMA thread issues cta_group::2 MMAs, each CTA's epilogue warps write the
 // 128 rows that sit in its own tensor memory.  The pair halves the operand traffic per flop of B.
 //
