@@ -129,13 +129,16 @@ struct GemmSmem {
   static constexpr int kBRows = kPair ? BN / 2 : BN;   // rows of B this CTA loads per stage
   static constexpr int kBBytes = kBRows * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  // Four stages keep the main loop fed as well as six did (BF16 4096^3 x 4 on pair tiles: 436 us with either; three stages
-  // of the 48 KB tiles); the rest of shared memory is the epilogue's, which needs several blocks per warp in flight.
+  // A stage's way round -- freed, copied into, multiplied, freed -- takes about 2700 cycles whatever its size, so it is the
+  // number of stages that keeps the main loop fed: BF16 8192^3 on 256 x 256 pair tiles 627 cycles per k-block with four, 541
+  // with five, 535 with six (its MMAs take 512).  The epilogue wants two blocks a warp in flight where it brings in C and
+  // writes two results: 32 x 768^3 Newton-Schulz update 52 us with two or three, 58 with one.  Hence five stages of 32 KB and
+  // six of 24 KB with two blocks, four of 48 KB with one.
   // (Interleaved plane products hold two stages until the three products of a k-block have been issued: six.)
-  static constexpr int kStages = kInter ? 6 : (kStageBytes > 32 * 1024 ? 3 : (kStageBytes < 32 * 1024 ? 5 : 4));
+  static constexpr int kStages = kInter ? 6 : (kStageBytes > 32 * 1024 ? 4 : (kStageBytes < 32 * 1024 ? 6 : 5));
   static constexpr int kTileBytes = kStages * kStageBytes;
   // 4 KB blocks per epilogue warp
-  static constexpr int kEpiBufs = kInter && kStageBytes == 32 * 1024 ? 1 : (kInter || kStageBytes > 32 * 1024 ? 2 : 3);
+  static constexpr int kEpiBufs = kStageBytes > 32 * 1024 || (kInter && kStageBytes == 32 * 1024) ? 1 : 2;
   static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
   static constexpr int kBarBytes = 256;
   static constexpr int kTotal = kTileBytes + kEpiBytes + kBarBytes + 1024;  // 1024: alignment slack
@@ -250,17 +253,16 @@ __device__ __forceinline__ void stage_cols_16(uint32_t buf, int lane, const uint
   }
 }
 
-// A warp's ring of staged blocks: `bufs` (at most three) of them.  Every acquired block ends in exactly one bulk group,
+// A warp's ring of staged blocks: `bufs` (one or two) of them.  Every acquired block ends in exactly one bulk group,
 // committed in the order of acquisition, so "all but the bufs - 1 newest groups have been read" frees the block acquired bufs
 // acquisitions ago.
 struct EpilogueRing {
   uint32_t base;
   int bufs;
   int next = 0;
-  __device__ __forceinline__ uint32_t acquire(int lane) {
-    if (lane == 0) {
-      if (bufs == 3) ptx::bulk_wait_read<2>();
-      else if (bufs == 2) ptx::bulk_wait_read<1>();
+  __device__ __forceinline__ uint32_t acquire() {
+    if (ptx::elect_one()) {
+      if (bufs == 2) ptx::bulk_wait_read<1>();
       else ptx::bulk_wait_read<0>();
     }
     __syncwarp();
@@ -277,20 +279,20 @@ __device__ __forceinline__ void epilogue_block(const GemmParams& p, const Epilog
                                                uint32_t held, int b, int row_first, int c0, int lane, bool whole,
                                                EpilogueSums& t) {
   auto take = [&]() {
-    const uint32_t buf = held ? held : ring.acquire(lane);
+    const uint32_t buf = held ? held : ring.acquire();
     held = 0;
     return buf;
   };
   auto send = [&](auto&& stores) {   // what the lanes staged becomes visible to the copy engine, then one lane stores it
     ptx::fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       stores();
       ptx::bulk_commit();
     }
   };
   if (whole) {
-    if (!held) held = ring.acquire(lane);
+    if (!held) held = ring.acquire();
     stage_cols_f32(held, lane, v);
     __syncwarp();
     float4 r[8];
@@ -460,16 +462,14 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 //
 // kInter: the split-precision product Ah Bh + Ah Bl + Al Bh with its three plane products interleaved k-block by k-block: a
 // stage with the lo planes of a k-block, a stage with the hi planes, three groups of MMAs over the two, so that each plane
-// comes from L2 once instead of one and a half times.  What bounds the main loop is that traffic: with all SMs running the
-// pair tiles take in 44 B per clock and SM whatever the tile (736 cycles per k-block of 256 x 256, 1100 of 256 x 512, against
-// 512 and 1024 of MMAs); interleaved, three plane products need 64 KB instead of 96 KB and 1536 cycles of MMAs.  Measured
-// plane by plane / interleaved: 12 x 3072^3 symmetric 1002 / 736 us (1.53 PFLOP/s), 6 x 5632^3 symmetric 3096 / 2145 us.
+// comes from L2 once instead of one and a half times: three plane products need 64 KB instead of 96 KB beside their 1536
+// cycles of MMAs.  Measured plane by plane / interleaved, under the power limit: 12 x 3072^3 symmetric 864 / 744 us, in chains of two
+// 876 / 825; 6 x 5632^3 symmetric 2450 / 2170 and 2555 / 2517.
 // The cross products of a k-block go into the accumulator before its hi product.  In a chained product they now share the
 // chains, which the host therefore makes shorter than c k-blocks, except c = 2 (see the MMA loop), so that no error grows:
 // against FP64 at 2048^3, chains of 2 plane by plane and interleaved 4.1e-7; of 8 plane by plane 2.4e-6, of 5 interleaved
-// 1.9e-6 (random signs 3.4e-7, 1.5e-6 and 1.4e-6); one chain 1.8e-5 and 1.5e-5.  18 x 2048^3, chains of 2: 780k cycles plane
-// by plane, 655k interleaved (and 767k in chains of one k-block, the other way to lose no more).  (GemmParams::segs is 1
-// here: the three products are one.)
+// 1.9e-6 (random signs 3.4e-7, 1.5e-6 and 1.4e-6); one chain 1.8e-5 and 1.5e-5.  (GemmParams::segs
+// is 1 here: the three products are one.)
 template <int BN, bool kChained, bool kPair = false, bool kInter = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair, kInter>;
@@ -603,10 +603,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
   ptx::reg_dec<48>();
   if (warp == 0 || warp == 2) {
     // ------------------------------------------------------------ TMA producers: warp 0 brings A, warp 2 brings B
-    // Issuing a copy holds its thread up until the copy engine takes it: one thread fills 32 KB stages every 496 cycles at
-    // best (copies alone, two of 16 KB each), two threads every 430 -- and beside the MMAs one thread needed 736.
+    // Issuing a copy holds its thread up until the copy engine takes it, hence two threads.
     const bool for_a = warp == 0;
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -631,9 +630,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         // fill the next stage with k-block k0 of planes za / zb
         auto fill = [&](int k0, int za, int zb) {
           const long long w0 = p.prof ? clock64() : 0;
-          const bool got = ptx::mbar_wait(empty_bar(stage), phase ^ 1u, kWaitCycles);
+          const bool got = ptx::mbar_wait_unless(empty_bar(stage), phase ^ 1u, kWaitCycles, abort_flag);
           if (p.prof) prof_wait += clock64() - w0;
-          if (!got || *abort_flag) {
+          if (!got) {
             report(p.status, kTimeoutProducer);
             raise_abort();
             ok = false;
@@ -721,7 +720,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (of a pair: the leader CTA only)
-    if (lane == 0 && leader) {
+    // This thread's own instructions, not memory, were what bounded the main loop (half the copies: the same time; a quarter
+    // of the MMAs: 666 cycles a k-block instead of 775): it is elected, and the flag of a role that gave up is looked at only
+    // while waiting.  8192^3 775 -> 627 cycles a k-block, 541 with five stages: 838 -> 726 us (power-capped; zeros, which draw
+    // little power, 770 -> 572 us).
+    if (leader && ptx::elect_one()) {
       const uint32_t idesc = (1u << 4) | ((uint32_t)p.fmt << 7) | ((uint32_t)p.fmt << 10) | ((uint32_t)p.a_mn << 15) |
                              ((uint32_t)p.b_mn << 16) | ((uint32_t)(BNI >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
       // K-major: 8-row groups 1024 B apart, k advances 32 B inside the swizzled row.
@@ -748,9 +751,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           const uint32_t acc_parity = (kWide ? (gchunk & 1u) : ((gchunk >> 1) & 1u)) ^ 1u;
           auto wait_drained = [&](int bar) {
             const long long w0 = p.prof ? clock64() : 0;
-            const bool got_acc = ptx::mbar_wait(tempty_bar(bar), acc_parity, kWaitCycles);
+            const bool got_acc = ptx::mbar_wait_unless(tempty_bar(bar), acc_parity, kWaitCycles, abort_flag);
             if (p.prof) prof_acc += clock64() - w0;
-            if (!got_acc || *abort_flag) {
+            if (!got_acc) {
               report(p.status, kTimeoutMma);
               raise_abort();
               ok = false;
@@ -764,9 +767,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           // wait for the operands of a stage; its shared-memory address
           auto operands = [&](int st, uint32_t ph) {
             const long long w1 = p.prof ? clock64() : 0;
-            const bool got_ops = ptx::mbar_wait(full_bar(st), ph, kWaitCycles);
+            const bool got_ops = ptx::mbar_wait_unless(full_bar(st), ph, kWaitCycles, abort_flag);
             if (p.prof) prof_ops += clock64() - w1;
-            if (!got_ops || *abort_flag) {
+            if (!got_ops) {
               report(p.status, kTimeoutMma);
               raise_abort();
               ok = false;
@@ -903,8 +906,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         const long long w0 = p.prof ? clock64() : 0;
         // every lane observes the barrier itself, so each one is ordered after the MMAs' TMEM writes
         const uint32_t parity = kWide ? (gchunk & 1u) : ((gchunk >> 1) & 1u);
-        const int waited = __all_sync(0xffffffffu, ptx::mbar_wait(tfull_bar(buf), parity, kWaitCycles) ? 1 : 0);
-        if (!waited || *abort_flag) {
+        const int waited = __all_sync(0xffffffffu, ptx::mbar_wait_unless(tfull_bar(buf), parity, kWaitCycles, abort_flag) ? 1 : 0);
+        if (!waited) {
           if (lane == 0) {
             report(p.status, kTimeoutEpilogue);
             raise_abort();
@@ -946,8 +949,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       // being formed.
       auto fetch_c = [&](int cc) {
         if (!e.use_c || cc >= cc_end || !boxed(col_first + cc * 32)) return;
-        c_buf = c_apart ? warp_bufs + (S::kEpiBufs - 1) * kEpiBlockBytes : ring.acquire(lane);
-        if (lane == 0) {
+        c_buf = c_apart ? warp_bufs + (S::kEpiBufs - 1) * kEpiBlockBytes : ring.acquire();
+        if (ptx::elect_one()) {
           ptx::mbar_expect_tx(c_bar(ew), kEpiBlockBytes);
           ptx::tma_load_3d(c_buf, &p.c_map, c_bar(ew), col_first + cc * 32, row_first, b);
         }
@@ -1082,8 +1085,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         if (boxed(c0)) {
           uint32_t held = c_buf;
           if (held) {
-            const bool got = __all_sync(0xffffffffu, ptx::mbar_wait(c_bar(ew), c_phase, kWaitCycles) ? 1 : 0);
-            if (!got || *abort_flag) {
+            const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_unless(c_bar(ew), c_phase, kWaitCycles, abort_flag) ? 1 : 0);
+            if (!got) {
               if (lane == 0) {
                 report(p.status, kTimeoutEpilogue);
                 raise_abort();
@@ -1113,7 +1116,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           }
           epilogue_block(p, e, ring, v, held, b, row_first, c0, lane, p.tri && p.mirror && c0 == row_first, sums);
         } else {
-          const uint32_t buf = ring.acquire(lane);
+          const uint32_t buf = ring.acquire();
           stage_rows_f32(buf, lane, v);
           __syncwarp();
           e.Cb = p.C ? p.C + (long long)b * p.c_bs : nullptr;
@@ -1122,7 +1125,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           e.S0b = p.S0 ? p.S0 + (long long)b * p.s_bs : nullptr;
           e.S1b = p.S1 ? p.S1 + (long long)b * p.s_bs : nullptr;
           epilogue_block_scalar(p, e, reinterpret_cast<float*>(smem + (buf - base)), row_first, c0, lane, sums);
-          if (lane == 0) ptx::bulk_commit();   // (nothing in flight: the ring counts one group per block)
+          if (ptx::elect_one()) ptx::bulk_commit();   // (nothing in flight: the ring counts one group per block)
         }
         if (!c_buf) fetch_c(cc + 1);
       }
@@ -1149,7 +1152,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         }
       }
     }
-    if (lane == 0) {
+    __syncwarp();
+    if (ptx::elect_one()) {
       if (c_buf) ptx::mbar_wait(c_bar(ew), c_phase, kDrainCycles);   // (gave up with a block of C on its way)
       ptx::bulk_wait_all();   // the stores have read shared memory and are written before the CTA ends
     }

@@ -22,6 +22,16 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// ---------------------------------------------------------------- one thread of a warp
+// True in one thread, always the same, of a converged warp.  What tcgen05, TMA and bulk-group instructions take (descriptors,
+// barriers, coordinates) sits in registers shared by the warp: behind `lane == 0` the compiler cannot know that one thread
+// is left and issues every one of them in a loop over the warp's threads, behind this it can.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one)::"memory");
+  return one != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -52,6 +62,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity)) {
     if (clock64() - t0 > limit_cycles) return false;
+  }
+  return true;
+}
+
+// The same, and also false once *stop is set; looked at only while waiting, which a thread soon does when others have stopped.
+__device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, long long limit_cycles, const volatile int* stop) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*stop || clock64() - t0 > limit_cycles) return false;
   }
   return true;
 }
