@@ -168,16 +168,13 @@ def step_flops(w: Workload, root_gemms_d: int, root_gemms_f: int, ns_steps: int 
 
 
 def product_counts(core, optimizer: str):
-    """Products per statistic of the factor engine as it ran last: X T and the log2(p) + 1 products of the M update per
-    Newton step (no X product in the first step, no M update in the last), the squarings for the stronger power --
-    each three FP16 plane passes -- plus the single-pass products of the finishing polynomial."""
+    """Products per statistic of the factor engine as it ran last: the split-precision ones -- three FP16 plane passes each --
+    and the single-pass ones (FactorSet.products)."""
     out = {}
     for name, g in core.groups.items():
         f = g.factors
-        log2p = f.p.bit_length() - 1
-        split = (f.iterations - 1) * (log2p + 2) + (f.q.bit_length() - 1)
-        out[name] = {"newton_steps": f.iterations, "finish_order": f.finish_order, "split": split,
-                     "single": f.finish_products}
+        split, single = f.products
+        out[name] = {"newton_steps": f.iterations, "finish_order": f.finish_order, "split": split, "single": single}
     return out
 
 

@@ -252,6 +252,14 @@ int toner_inv_roots_finish_products_for(float lower, int32_t p, int32_t iters, i
  * x * q(1 - mu) = lambda^(-1/p). */
 int toner_inv_roots_schedule(float lower, int32_t p, int32_t iters, double* ab_out, int32_t ab_capacity, double* coef_out,
                              int32_t coef_capacity, int32_t* order_out, double* e_out);
+/* The schedule of a call whose bound is an estimate (toner_inv_roots_tracked with lower_is_estimate and deflate, 2 q = p, no
+ * plane order) on statistics of width n: where it costs less, `steps` Newton steps as above, from the same coefficients, and then a graded finish in
+ * place of the polynomial in R: with z = zb + za mu and u = 2 z^2 - 1, sum_j (alpha_j + beta_j z) u^j = mu^(-1/p) to 3e-6 for
+ * every mu the bound allows.  Returns K, the number of products by u (0: the schedule above is used), and writes the step
+ * count, how many of the K - 1 inner products take three plane products (the last and u itself always do), and zb, za,
+ * alpha_0, beta_0, alpha_1, ... (at most 28 doubles).  Every output pointer is optional; needs no device. */
+int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps_out, int32_t* split_out, double* coef_out,
+                               int32_t coef_capacity);
 int toner_inv_roots(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
                     float* root_lo, float* root_hi, float* fro2_lo, int32_t* status, void* workspace,
                     size_t workspace_bytes, void* stream);
@@ -290,8 +298,10 @@ int toner_inv_roots_ex(const float* ema, int32_t k, int32_t n, float damping, in
  *                  A' / norm, typically margin * min_b lmin_out[b] / norm_out[b] of the previous call.  Such a bound
  *                  cannot be checked in advance; it is verified after the chain: four power-iteration steps on
  *                  R = I - M of the last M, from the tracked direction, estimate ||R||_2, and status[b] = 4 where that
- *                  exceeds what the finishing series was cut for (by 15 % + 1e-3).  The caller recomputes such a
- *                  statistic with the bound that always holds.  resid_out (DEVICE, optional, k floats) receives the
+ *                  exceeds what the finishing series was cut for (by 15 % + 1e-3).  After a graded finish
+ *                  (toner_inv_roots_graded_for) R is I - A^(-1/2) A A^(-1/2) instead, from the computed root: two steps
+ *                  from the tracked direction and from the largest Ritz vector that stayed in A', 8e-3 allowed.  The
+ *                  caller recomputes such a statistic with the bound that always holds.  resid_out (DEVICE, optional, k floats) receives the
  *                  estimate.  With lower_is_estimate = 0 the call is toner_inv_roots_ex (plus tracking).
  *   deflate, deflate_rank, deflated_out
  *                  `deflate` (DEVICE, k * 8 * n floats, kept by the caller between calls; optional): eight vector slots

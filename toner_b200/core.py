@@ -219,7 +219,8 @@ class FactorSet:
             budget = min(32 << 30, torch.cuda.get_device_properties(device).total_memory // 5)
             chunk = max(1, min(k, budget // per))
         self.workspace = self.scratch.bytes_like("inv_roots", ops.inv_roots_workspace_bytes(chunk, n), device)
-        self._lower_used = 0.0           # the bound the last call's schedule was built for
+        self._lower_used = 0.0           # the bound the last call's schedule was built for, and whether it was an estimate
+        self._used_estimate = False
         self.fallbacks = 0
         self.repairs = 0
 
@@ -241,6 +242,18 @@ class FactorSet:
         """Single-pass products of the last factorisation's finish."""
         return (ops.inv_roots_finish_products(self.n, self.damping, self.p, self._lower_used, interleave=self.interleave)
                 if self.k else 0)
+
+    @property
+    def products(self) -> Tuple[int, int]:
+        """Split-precision and single-pass products the last factorisation took per statistic (without the norm bound's)."""
+        log2p, log2q = self.p.bit_length() - 1, self.q.bit_length() - 1
+        graded = None
+        if self._used_estimate and self.interleave and 2 * self.q == self.p and self.block_deflation:
+            graded = ops.inv_roots_graded(self._lower_used, self.p, self.n)
+        if graded:
+            steps, split = graded["steps"], graded["split"]
+            return (steps * (log2p + 2) if steps else 0) + 2 + split + log2q, graded["products"] - 1 - split
+        return (self.iterations - 1) * (log2p + 2) + log2q, self.finish_products
 
     # -- which stored root serves a given strength
     def _is_hi(self, strength: float) -> bool:
@@ -294,7 +307,7 @@ class FactorSet:
                       ritz_norm=ritz, interleave=self.interleave, lo_planes=self.lo_planes, lo_inv=self.lo_inv,
                       hi_planes=self.hi_planes if self.q > 1 else None, hi_inv=self.hi_inv if self.q > 1 else None)
         self.track_restart = False
-        self._estimate_in_flight = self.lower_is_estimate
+        self._estimate_in_flight = self._used_estimate = self.lower_is_estimate
         self._lower_used = self.lower
         self._norm_hi()
         ops.factor_report(self.status, self.norms, self.lmin, self.deflated, self._host)

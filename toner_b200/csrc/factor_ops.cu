@@ -256,23 +256,114 @@ static int default_iterations(double l0, int p) {
   return best ? best : 64;
 }
 
+// The graded finish: where the spectrum of M reaches further down than a polynomial in R = I - M can follow, q(M) ~ M^(-1/p) is
+// written in Z, M mapped from [lo, hi] onto [-1, 1], and U = 2 Z^2 - I = T_2(Z):  a Chebyshev interpolant of odd degree
+// m = 2 K + 1 is  sum_j (alpha_j I + beta_j Z) U^j,  Horner's rule in U takes K products, and the coefficients fall like the
+// square of the interpolant's rate (1/6 a power and less), so only what is near the front needs both planes: U itself and
+// the last product or two, three plane products each; those before are single passes.  An M that reaches down to 0.1 takes
+// K = 7, five single passes and three split products, where another Newton step takes five split products more.  It is used
+// where the lower bound is an estimate that is verified afterwards, with no Newton step at all (Marchenko-Pastur spectra of
+// eight rows a column and more), or to save the last one.  Error of A^(-1/8) against FP64, Newton's finish / graded:
+// 768 wide, 8192 rows 6e-6 / 1.3e-6; 2048, 73216 rows 1.7e-5 / 6e-7; 1536, 3000 rows 1.3e-5 / 2.5e-6.
+constexpr int kMaxGraded = 12;    // K
+constexpr double kGradedSingle = 0.015;   // W_(j+1) at most this part of W_0: W_j is a single pass (11 bits of it, 4e-6 of W_0)
+// Allowed of I - A^(-1/2) A A^(-1/2) where a bound was an estimate (1e-3 of A^(-1/p) on one eigenvector).  Deflated directions,
+// converged to 1e-5, leave 1e-5 (lambda_1 / lambda)^(1/2) of it.
+constexpr float kGradedResidual = 8e-3f;
+constexpr double kGradedHigh = 1.02, kGradedLowCold = 0.97, kGradedLow = 0.9;   // margins for rounding (of Newton steps, if any)
+struct GradedPoly {
+  int products = 0;               // K; 0: none
+  int split = 0;                  // W_j with 1 <= j <= split are split products as well
+  double lo = 0.0;
+  double za = 0.0, zb = 0.0;      // Z = zb I + za M
+  double alpha[kMaxGraded + 1] = {}, beta[kMaxGraded + 1] = {};
+  double bound[kMaxGraded + 1] = {};   // of W_j = sum_{i >= j} (alpha_i + beta_i z) U^(i-j)
+};
+
+// (A tracked call asks for this with a new lower end every step: one expansion of the function, 64 powers, serves every
+// degree, and nothing is fitted again.)
+static GradedPoly graded_poly(int p, double lo) {
+  constexpr int kNodes = 64, kTerms = 40, kPoints = 65;
+  struct Cosines {
+    double at[kTerms][kNodes];       // T_j at the Chebyshev nodes
+    double z[kPoints];               // where the sums are bounded
+    Cosines() {
+      const double kPi = 3.14159265358979323846;
+      for (int j = 0; j < kTerms; ++j)
+        for (int k = 0; k < kNodes; ++k) at[j][k] = std::cos(j * kPi * (k + 0.5) / kNodes);
+      for (int i = 0; i < kPoints; ++i) z[i] = std::cos(kPi * i / (kPoints - 1));
+    }
+  };
+  static const Cosines cosines;
+  const double hi = kGradedHigh;
+  double f[kNodes], c[kTerms], tail = 0.0;
+  for (int k = 0; k < kNodes; ++k) f[k] = std::pow(0.5 * (hi + lo) + 0.5 * (hi - lo) * cosines.at[1][k], -1.0 / p);
+  for (int j = 0; j < kTerms; ++j) {
+    c[j] = 0.0;
+    for (int k = 0; k < kNodes; ++k) c[j] += f[k] * cosines.at[j][k];
+    c[j] *= (j == 0 ? 1.0 : 2.0) / kNodes;
+  }
+  // the smallest odd degree 2 K + 1 whose remainder stays below the bound; the function is above hi^(-1/p) everywhere
+  GradedPoly g;
+  int K = kTerms / 2;
+  const double most = kFinishTail * std::pow(hi, -1.0 / p);
+  for (; K > 2; --K) {
+    const double more = tail + (2 * K + 1 < kTerms ? std::fabs(c[2 * K + 1]) : 0.0) + (2 * K < kTerms ? std::fabs(c[2 * K]) : 0.0);
+    if (more > most) break;
+    tail = more;
+  }
+  if (K > kMaxGraded) return g;
+  // T_{2j}(z) = T_j(U),  T_{2j+1}(z) = z V_j(U) with V_0 = 1, V_1 = 2 U - 1, V_{j+1} = 2 U V_j - V_{j-1}
+  double t0[kMaxGraded + 1] = {1.0}, t1[kMaxGraded + 1] = {0.0, 1.0}, v0[kMaxGraded + 1] = {1.0}, v1[kMaxGraded + 1] = {-1.0, 2.0};
+  for (int j = 0; j <= K; ++j) {
+    for (int i = 0; i <= K; ++i) {
+      g.alpha[i] += c[2 * j] * t0[i];
+      g.beta[i] += c[2 * j + 1] * v0[i];
+    }
+    for (int i = K; i >= 0; --i) {   // (t0, t1) <- (t1, 2 U t1 - t0), and v likewise; from above, so that t1[i - 1] is still old
+      const double t2 = (i > 0 ? 2.0 * t1[i - 1] : 0.0) - t0[i], v2 = (i > 0 ? 2.0 * v1[i - 1] : 0.0) - v0[i];
+      t0[i] = t1[i];
+      v0[i] = v1[i];
+      t1[i] = t2;
+      v1[i] = v2;
+    }
+  }
+  for (int i = 0; i < kPoints; ++i) {
+    const double z = cosines.z[i], u = 2.0 * z * z - 1.0;
+    double w = 0.0;
+    for (int j = K; j >= 0; --j) {
+      w = g.alpha[j] + g.beta[j] * z + u * w;
+      g.bound[j] = std::max(g.bound[j], 1.1 * std::fabs(w));
+    }
+  }
+  while (g.split < K && g.bound[std::min(g.split + 2, K)] > kGradedSingle * g.bound[0]) ++g.split;
+  if (g.split > K - 2 || !(std::fabs(g.beta[K]) > 1e-12)) return GradedPoly();   // (W_K has one plane)
+  g.products = K;
+  g.lo = lo;
+  g.za = 2.0 / (hi - lo);
+  g.zb = -(hi + lo) / (hi - lo);
+  return g;
+}
+
 // Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
 // Working it out takes tens of microseconds of host time and is asked for several times per factorisation (the call itself,
 // the step count and the degree it states), so a thread keeps the last few.
 struct Schedule {
   double l0 = 0.0;
-  int p = 0, asked = 0;   // asked: the caller's step count, 0 = the one with the fewest plane passes
+  int p = 0, asked = 0;   // asked: the caller's step count, 0 = the one with the fewest plane passes; -n: graded
+                          // finishes considered as well, for statistics of width n
   int iters = 0;
   std::vector<NewtonStep> steps;
   double l_last = 0.0;    // lower bound of the spectrum of the last M, i.e. after iters - 1 updates
   FinishPoly fin;
+  GradedPoly graded;      // graded.products > 0: this finish, after iters - 1 updates of M (steps holds them; none: iters == 1)
 };
 
-static const Schedule& schedule_for(double l0, int p, int iters) {
+static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0) {
   constexpr int kKept = 8;
   static thread_local Schedule kept[kKept];
   static thread_local int oldest = 0;
-  if (iters < 0) iters = 0;
+  iters = iters > 0 ? iters : -grade_n;
   for (const Schedule& s : kept)
     if (s.p == p && s.l0 == l0 && s.asked == iters) return s;
   Schedule& s = kept[oldest];
@@ -285,6 +376,39 @@ static const Schedule& schedule_for(double l0, int p, int iters) {
     s.steps = newton_schedule(l0, p, s.iters, nullptr);
     newton_schedule(l0, p, s.iters - 1, &s.l_last);
     s.fin = finish_poly_or_best(p, 1.0 - s.l_last);
+  }
+  s.graded = GradedPoly();
+  if (iters < 0) {
+    const int n = grade_n;
+    // Costs in split products.  A single pass takes 0.43 of one at width 3072, 0.5 at 2048, 0.77 at 768, where writing the results
+    // is most of it (interleaved products in batches; C and operand planes as the finish has them); the final squarings, in short
+    // chains after a graded finish, a tenth more at 3072 and a third at 768.  k updates of M are k (log2 p + 1) split products and
+    // k - 1 products with X; Newton's finish ends in one with X, the graded one in two, and in one where there is no X yet.
+    int log2p = 0;
+    while ((1 << log2p) < p) ++log2p;
+    const double single = 0.35 + 320.0 / n, squarings = (log2p - 1) * (0.05 + 250.0 / n);
+    QuadraticSteps q;
+    double best = (s.iters - 1) * (log2p + 2) +
+                  single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
+    for (int k = 0; k < s.iters; ++k) {
+      double l = l0;
+      if (k) newton_schedule(l0, p, k, &l);
+      const double front = (k ? k * (log2p + 2) + 2 : 2) + squarings;
+      if (front + single >= best) break;
+      const GradedPoly g = graded_poly(p, (k ? kGradedLow : kGradedLowCold) * l);
+      if (!g.products) continue;
+      const double cost = front + g.split + single * (g.products - 1 - g.split);
+      if (cost < best) {
+        best = cost;
+        s.graded = g;
+        s.iters = k + 1;      // (the loop's bound shrinks with it: more steps only cost more)
+      }
+    }
+    if (s.graded.products) {
+      s.l_last = l0;
+      s.steps = newton_schedule(l0, p, s.iters, nullptr);
+      if (s.iters > 1) newton_schedule(l0, p, s.iters - 1, &s.l_last);
+    }
   }
   s.p = p;
   return s;
@@ -351,13 +475,15 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 // that the single-pass squarings of the norm bound read).
 // With defl_v the input is A and the deflation A' = A + sum_j coef[j] v_j v_j^T is applied on the way (the terms of
 // rankr_update_kernel, in its order), so that A' is never written.
+// With m32 (the graded finish with no Newton step) M_0 is written there in FP32, and its planes -- the hi plane alone -- are
+// those of M_0 + m_diag I.
 __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restrict__ a32, int n, int batch,
                                                           const float* __restrict__ sumsq, float a, float b, float s_m,
                                                           float s_t, __half* __restrict__ m_planes,
                                                           __half* __restrict__ t_planes,
                                                           const float* __restrict__ defl_v,
                                                           const float* __restrict__ defl_coef, int defl_r,
-                                                          int vstride) {
+                                                          int vstride, float* __restrict__ m32 = nullptr, float m_diag = 0.f) {
   ptx::pdl_begin();
   const int bi = blockIdx.y;
   float cf[8];
@@ -398,9 +524,10 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
       *reinterpret_cast<uint2*>(mh + i * 4) = *reinterpret_cast<uint2*>(h);
       continue;
     }
+    if (m32) *reinterpret_cast<float4*>(m32 + bi * nn + i * 4) = make_float4(m[0], m[1], m[2], m[3]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float x = m[e] * s_m;
+      const float x = ((c + e) == r ? m[e] + m_diag : m[e]) * s_m;
       h[e] = __float2half_rn(x);
       l[e] = __float2half_rn(x - __half2float(h[e]));
       const float t = (((c + e) == r ? a : 0.f) - b * m[e]) * s_t;
@@ -408,7 +535,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
       k[e] = __float2half_rn(t - __half2float(g[e]));
     }
     *reinterpret_cast<uint2*>(mh + i * 4) = *reinterpret_cast<uint2*>(h);
-    *reinterpret_cast<uint2*>(ml + i * 4) = *reinterpret_cast<uint2*>(l);
+    if (!m32) *reinterpret_cast<uint2*>(ml + i * 4) = *reinterpret_cast<uint2*>(l);
     *reinterpret_cast<uint2*>(th + i * 4) = *reinterpret_cast<uint2*>(g);
     *reinterpret_cast<uint2*>(tl + i * 4) = *reinterpret_cast<uint2*>(k);
   }
@@ -1116,11 +1243,13 @@ __global__ void __launch_bounds__(256) root_finish_kernel(float* __restrict__ a,
                                                           const float* __restrict__ coef, int n, int r, int vstride, int cstride,
                                                           float s, __half* __restrict__ planes, int lo_step,
                                                           float* __restrict__ inv, float s2, float* __restrict__ inv2,
-                                                          float* __restrict__ partial) {
+                                                          float* __restrict__ partial, const float* __restrict__ diag_scale,
+                                                          float diag) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
   float cf[kMaxDeflate];
-  bool any = false;
+  const float dg = diag_scale ? diag * diag_scale[b] : 0.f;   // added to the diagonal
+  bool any = dg != 0.f;
 #pragma unroll
   for (int j = 0; j < kMaxDeflate; ++j) {
     cf[j] = j < r ? coef[b * cstride + j] : 0.f;
@@ -1141,6 +1270,12 @@ __global__ void __launch_bounds__(256) root_finish_kernel(float* __restrict__ a,
   auto finished = [&](unsigned i, float4 x) {
     if (any) {
       const unsigned row = i / n4, c = (i - row * n4) * 4;
+      if (row - c < 4u) {
+        if (row == c) x.x += dg;
+        else if (row == c + 1) x.y += dg;
+        else if (row == c + 2) x.z += dg;
+        else x.w += dg;
+      }
 #pragma unroll
       for (int j = 0; j < kMaxDeflate; ++j) {
         if (cf[j] != 0.f) {
@@ -1250,20 +1385,39 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
   __syncthreads();
   const double inv = tot[2] > 0.0 ? 1.0 / sqrt(tot[2]) : 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (float)(((double)V[i] - (double)Y[i]) * inv);
-  if (threadIdx.x == 0) e[b] = tot[1] > 0.0 ? (float)(1.0 - tot[0] / tot[1]) : 0.f;
+  if (threadIdx.x == 0) e[b] = tot[1] == 0.0 ? 0.f : (float)(1.0 - tot[0] / tot[1]);   // (NaN stays NaN)
 }
 
 // status 4 where the distance of the last M from the identity, estimated by power iteration on I - M, exceeds what the
 // schedule was built for: the caller's estimate of the spectrum's lower end was too high for this statistic.
 __global__ void verify_kernel(const float* __restrict__ e_est, const float* __restrict__ e_top, float e_allowed,
-                              int* __restrict__ status, float* __restrict__ e_out, int k) {
+                              int* __restrict__ status, float* __restrict__ e_out, int k, int both_signs) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
-  float e = e_est[b];
-  if (e_top) e = isfinite(e_top[b]) ? fmaxf(e, e_top[b]) : e_top[b];
+  float e = both_signs ? fabsf(e_est[b]) : e_est[b];
+  if (e_top) e = isfinite(e_top[b]) ? fmaxf(e, both_signs ? fabsf(e_top[b]) : e_top[b]) : e_top[b];
   if (e_out) e_out[b] = e;
   if (status && status[b] == 0 && (!isfinite(e) || e > e_allowed)) status[b] = 4;
+}
+
+// y_j <- y_j - sum_i coef[b][i] (v_i . x_j) v_i for the two vectors of statistic b: with y = A' x this makes A x of it,
+// A = A' - sum_i coef[i] v_i v_i^T.
+__global__ void __launch_bounds__(256) undeflate_kernel(float* __restrict__ y, const float* __restrict__ x,
+                                                        const float* __restrict__ v, const float* __restrict__ coef, int n, int r,
+                                                        int vstride) {
+  ptx::pdl_begin();
+  __shared__ double red[8];
+  const int b = blockIdx.x;
+  const float* X = x + ((long long)b * 2 + blockIdx.y) * n;
+  float* Y = y + ((long long)b * 2 + blockIdx.y) * n;
+  for (int i = 0; i < r; ++i) {
+    const float c = coef[b * kMaxDeflate + i];
+    if (c == 0.f) continue;
+    const float* V = v + ((long long)b * vstride + i) * n;
+    const float dot = (float)(c * block_dot(V, X, n, red));
+    for (int j = threadIdx.x; j < n; j += blockDim.x) Y[j] = fmaf(-dot, V[j], Y[j]);
+  }
 }
 
 // lmin[b] = theta^(-power): the smallest eigenvalue of A from the largest eigenvalue theta (a Rayleigh quotient, so a
@@ -1390,6 +1544,25 @@ int toner_inv_roots_schedule(float lower, int32_t p, int32_t iters, double* ab_o
   return s.iters;
 }
 
+int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps_out, int32_t* split_out, double* coef_out,
+                               int32_t coef_capacity) {
+  if (!(lower > 0.f) || !(lower < 1.f) || p < 2 || n <= 0) return 0;
+  const toner::Schedule& s = toner::schedule_for((double)lower, p, 0, n);
+  const toner::GradedPoly& g = s.graded;
+  if (!g.products) return 0;
+  if (steps_out) *steps_out = s.iters - 1;
+  if (split_out) *split_out = g.split;
+  if (coef_out) {
+    if (coef_capacity > 0) coef_out[0] = g.zb;
+    if (coef_capacity > 1) coef_out[1] = g.za;
+    for (int j = 0; j <= g.products && 2 * j + 3 < coef_capacity; ++j) {
+      coef_out[2 * j + 2] = g.alpha[j];
+      coef_out[2 * j + 3] = g.beta[j];
+    }
+  }
+  return g.products;
+}
+
 int toner_factor_report(const int32_t* status, const float* norms, const float* lmin, const int32_t* deflated, int32_t k,
                         int32_t* host_out, void* stream) {
   using namespace toner;
@@ -1466,9 +1639,12 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
                          "(both are verified together after the chain)");
   // > 0: certified bound, checked against damping / norm per statistic; < 0: estimate, verified after the chain
   const float lower_used = l0 > l_worst ? (estimated ? -(float)l0 : (float)l0) : 0.f;
-  const Schedule plan = schedule_for(l0, p, iters);
+  // (verifying the estimate after a graded finish takes A^(-1/2) and the deflated vectors)
+  const bool may_grade = estimated && iters <= 0 && (track_sweeps & 512) == 0 && p > 1 && 2 * q == p && defl_r > 0;
+  const Schedule plan = schedule_for(l0, p, iters, may_grade ? n : 0);
   iters = plan.iters;
-  if (iters < 2) return fail(kErrArg, "inv_roots: at least two iterations are required");
+  const GradedPoly& graded = plan.graded;
+  if (iters < 2 && !graded.products) return fail(kErrArg, "inv_roots: at least two iterations are required");
   const std::vector<NewtonStep>& sched = plan.steps;
   const double l_last = plan.l_last;
   const FinishPoly& fin = plan.fin;
@@ -1589,15 +1765,25 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       int rc0 = sumsq_det(A32, kc, n, n, n, nn, partials, sumsq_a, stream);
       if (rc0) return rc0;
     }
-    float s_t = plane_scale(sched[0].a);
+    // What the engine starts from: planes of M_0 and of T_0 = a I - b M_0; for a graded finish with no Newton step those of Z
+    // in T_0's place, and M_0 in FP32 with the hi plane of M_0 + g I, of which W_K is a multiple
+    const bool cold_finish = graded.products > 0 && iters == 1;
+    const double top_gain = graded.products ? graded.beta[graded.products] * graded.za : 1.0;
+    const double top_diag =
+        graded.products ? (graded.alpha[graded.products] + graded.beta[graded.products] * graded.zb) / top_gain : 0.0;
+    float* const m32 = cold_finish ? reinterpret_cast<float*>(Xb[0]) : nullptr;
+    const float s_z = plane_scale(1.2), s_top = plane_scale(1.1 * (1.0 + std::fabs(top_diag)));
+    const float init_a = cold_finish ? (float)graded.zb : (float)sched[0].a, init_b = cold_finish ? (float)-graded.za : (float)sched[0].b;
+    const float init_sm = cold_finish ? s_top : s_m, init_diag = cold_finish ? (float)top_diag : 0.f;
+    float s_t = cold_finish ? s_z : plane_scale(sched[0].a);
     if (ritz_norm) {
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate, m32, init_diag);
       TONER_CUDA(cudaGetLastError());
     } else {
-    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0);
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f);
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -1639,7 +1825,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
       TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, (float)sched[0].a, (float)sched[0].b, s_m, s_t, Mb[0], Xb[1], nullptr, nullptr, 0, 0);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], Xb[1], nullptr, nullptr, 0, 0, m32, init_diag);
       TONER_CUDA(cudaGetLastError());
     }
     }
@@ -1658,6 +1844,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       unsigned int* maxres = nullptr;
       int lo_step = 0;              // s0: matrices between its hi and lo planes (0: the chunk's)
       const float* c = nullptr; float beta = 0.f;  // result = gain * product + beta * c (c symmetric, FP32)
+      const float* beta_v = nullptr;               // per-statistic factors of beta
       double gain = 1.0;
       int segs = 3;                                // 1: hi planes only (a single pass)
     };
@@ -1674,7 +1861,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g.m = n; g.n = n; g.k = n; g.batch = kc; g.segs = o.segs; g.fmt = 0;
       g.tri = 1; g.mirror = 1;
       g.alpha = (float)(o.gain / ((double)sa * (double)sb));
-      g.c = o.c; g.ldc = n; g.c_bs = nn; g.beta = o.beta;
+      g.c = o.c; g.ldc = n; g.c_bs = nn; g.beta = o.beta; g.beta_v = o.beta_v;
       g.alpha_a = o.alpha_a;
       g.alpha_b = o.alpha_b;
       g.d = o.d; g.ldd = n; g.d_bs = nn;
@@ -1689,7 +1876,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     int rc = 0;
     // the finish in steps of Y; its planes of R + beta I go where the powers of T leave room (p = 1 has no such buffer)
     QuadraticSteps fast;
-    const bool shorten = interleave && log2p > 0 && quadratic_steps(fin, p, fast);
+    const bool shorten = interleave && log2p > 0 && !graded.products && quadratic_steps(fin, p, fast);
     __half* const shifted_planes = Pb[log2p & 1];
     __half* root_planes = nullptr;   // of A^{-1/p}, root_step matrices between hi and lo
     int root_step = 0;
@@ -1702,18 +1889,74 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     double x_bound = sched[0].a;
     int xi = 0, mi = 0, ti = 1;   // ti: which T buffer was written last
 
+    // The graded finish starts from planes of Z (in zp), M in FP32 (m_last) and planes of M + g I (top)
+    const __half* zp = Xb[1];
+    const float* m_last = m32;
+    __half* const top = cold_finish ? Mb[0] : Pb[log2p & 1];
+    const float* root_diag_scale = nullptr;
+    float root_diag = 0.f;
     for (int it = 0; it < iters; ++it) {
       const bool last = (it == iters - 1);
-      if (it > 0) {
+      if (it > 0 || last) {
         x_bound = std::min(x_bound * sched[it].a, x_cap);
         if (last) {
+          // U = 2 Z^2 - I; with no Newton step the distance of Z^2 from I, which has no entry above 1, is what a non-finite or
+          // divergent statistic is told by
+          __half* const up = Pb[(log2p & 1) ^ 1];
+          const float s_u = plane_scale(2.0);
+          if (graded.products) {
+            Out u;
+            u.s1 = up; u.s1_scale = s_u;
+            u.s1_a = -1.f; u.s1_b = 2.f;
+            if (cold_finish) u.maxres = resid;
+            rc = sym_product(zp, s_t, zp, s_t, u, chain_length(graded.lo));
+            if (rc) return rc;
+          }
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, 0.5f, damping, lower_used);
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded.products ? (cold_finish ? 1.5f : 1.f) : 0.5f, damping, lower_used);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
-          const float s_w = plane_scale(1.0), s_f = plane_scale(2.0);
-          if (shorten) {
+          const float s_w = plane_scale(1.0);
+          float s_f = plane_scale(2.0);
+          const __half* poly = Mb[1];      // planes of what X is multiplied by
+          if (graded.products) {
+            // W_j = alpha_j I + beta_j Z + U W_(j+1); the FP32 M brings in Z.  W_1 keeps both planes for the last product.
+            const int K = graded.products;
+            __half* const spare[2] = {Mb[1], cold_finish ? Pb[log2p & 1] : Mb[0]};   // (top is read by the first product)
+            const __half* wcur = top;
+            float s_cur = s_top;
+            double gain = top_gain;
+            for (int j = K - 1; j >= 1; --j) {
+              Out w;
+              w.segs = j <= graded.split ? 3 : 1;
+              w.gain = gain;
+              w.c = m_last; w.beta = (float)(graded.beta[j] * graded.za);
+              w.s1 = spare[j & 1]; w.s1_scale = plane_scale(graded.bound[j]);
+              w.s1_a = (float)(graded.alpha[j] + graded.beta[j] * graded.zb); w.s1_b = 1.f;
+              rc = sym_product(up, s_u, wcur, s_cur, w, 0);
+              if (rc) return rc;
+              wcur = w.s1;
+              s_cur = w.s1_scale;
+              gain = 1.0;
+            }
+            const double front = graded.alpha[0] + graded.beta[0] * graded.zb;
+            Out f;
+            f.gain = gain;
+            f.c = m_last; f.beta = (float)(graded.beta[0] * graded.za);
+            if (cold_finish) {     // the root itself, up to `front` on the diagonal, which root_finish_kernel adds
+              f.d = root_lo + (long long)k0 * nn;
+              f.alpha_a = f.beta_v = scale_lo;
+              root_diag_scale = scale_lo;
+              root_diag = (float)front;
+            } else {
+              f.s1 = spare[0]; f.s1_scale = s_f = plane_scale(graded.bound[0]);
+              f.s1_a = (float)front; f.s1_b = 1.f;
+              poly = f.s1;
+            }
+            rc = sym_product(up, s_u, wcur, s_cur, f, kPromoteX);
+            if (rc) return rc;
+          } else if (shorten) {
             // Steps of Y = R (R + beta I), see quadratic_steps: the product that makes Y writes its planes and those of W, an
             // affine function of Y, at once.  (shifted_planes are those of -(R + beta I).)
             __half* const Yp = Pb[(log2p & 1) ^ 1];
@@ -1778,11 +2021,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             }
           }
           float* R = root_lo + (long long)k0 * nn;
-          Out o;
-          o.d = R;
-          o.alpha_a = scale_lo;
-          rc = sym_product(Xcur, s_x, Mb[1], s_f, o, kPromoteX);
-          if (rc) return rc;
+          if (!cold_finish) {
+            Out o;
+            o.d = R;
+            o.alpha_a = scale_lo;
+            rc = sym_product(Xcur, s_x, poly, s_f, o, kPromoteX);
+            if (rc) return rc;
+          }
           // put the deflated directions back: A^{-1/p} = A'^{-1/p} + (lambda_1^{-1/p} - c^{-1/p}) v v^T; with that the root's
           // norm and its operand planes, for the squarings below and for the caller
           if (lo_planes) {
@@ -1793,7 +2038,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           }
           TONER_LAUNCH(root_finish_kernel, dim3(kSumsqBlocks, kc), 256, stream, R, defl_r > 0 ? dv : pv, defl_r > 0 ? corr8 : corr, n,
                        defl_r > 0 ? defl_r : 1, defl_r > 0 ? kMaxDeflate : 1, defl_r > 0 ? kMaxDeflate : 1, s_root, root_planes,
-                       root_step ? root_step : kc, lo_planes ? lo_inv + k0 : inv_r, s_hi, hi_inv ? hi_inv + k0 : nullptr, partials);
+                       root_step ? root_step : kc, lo_planes ? lo_inv + k0 : inv_r, s_hi, hi_inv ? hi_inv + k0 : nullptr, partials, root_diag_scale, root_diag);
           TONER_LAUNCH(root_norm_kernel, kc, 32, stream, partials, fro_tmp);
           TONER_CUDA(cudaGetLastError());
           break;
@@ -1826,11 +2071,23 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         s_pw = o.s0_scale;
       }
       {
-        const float na = (float)sched[it + 1].a, nb = (float)sched[it + 1].b;
+        const bool to_finish = it == iters - 2;
+        const float na = to_finish ? 0.f : (float)sched[it + 1].a, nb = to_finish ? 0.f : (float)sched[it + 1].b;
         const int tn = (log2p == 0) ? (ti ^ 1) : 0;  // with p == 1 the product reads T itself
         Out o;
         o.s1 = Tb[tn];
-        if (it == iters - 2) {
+        if (to_finish && graded.products) {
+          // the last M: in FP32 (beside the X in use; A is still wanted), as planes of Z and of M + g I
+          m_last = reinterpret_cast<float*>(Xb[xi]);
+          o.d = reinterpret_cast<float*>(Xb[xi]);
+          o.s1_scale = s_z;
+          o.s1_a = (float)graded.zb;
+          o.s1_b = (float)graded.za;
+          o.maxres = resid;
+          o.s0 = top;
+          o.s0_scale = s_top;
+          o.s0_a = (float)top_diag;
+        } else if (to_finish) {
           // the last M: kept in FP32 with planes of R = I - M for the finishing series, and its distance from I
           o.d = A32;
           o.s1_scale = s_m;
@@ -1853,7 +2110,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         if (rc) return rc;
         mi ^= 1;
         ti = tn;
-        Tcur = Tb[tn];
+        Tcur = zp = Tb[tn];
         s_t = o.s1_scale;
       }
     }
@@ -1885,7 +2142,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           o.s0 = Pb[pi];
           o.s0_scale = plane_scale(bound);
         }
-        rc = sym_product(Xcur, s_x, Xcur, s_x, o, kPromoteX, first ? root_step : 0);
+        // (one chain's truncation, 2e-5 at depth 2048 and twice that after the second squaring, made up for part of the
+        // Newton chain's; A^(-1/p) from a graded finish is ten times closer than that)
+        rc = sym_product(Xcur, s_x, Xcur, s_x, o, graded.products ? kPromoteAccurate : kPromoteX, first ? root_step : 0);
         if (rc) return rc;
         Xcur = Pb[pi];
         s_x = o.s0_scale;
@@ -1901,7 +2160,25 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         // and they are the dominant eigenvalues of R = I - M of the last M (kept in FP32): four power-iteration steps
         // on R from the tracked direction (the eigenvector of the smallest eigenvalue, as of the previous call) find
         // them.  The allowance: the assumed distance with 15 % and the noise floor of the estimate.
-        if (ritz_norm) {
+        if (graded.products) {
+          // After a graded finish the roots themselves are looked at: R = I - A^(-1/2) A A^(-1/2), which is 8 times (p times) the
+          // relative error of A^(-1/p) on every eigenvector, of either sign, 1e-4 at most where the interpolant holds and large
+          // where an eigenvalue lies outside the interval.  One step from the tracked direction and from the largest Ritz vector
+          // that stayed in A' leaves next to nothing but such eigenvectors; the quotients of the second step tell.
+          const float* root = (q > 1 ? root_hi : root_lo) + (long long)k0 * nn;
+          float* const py2 = py + (long long)kc * 2 * n;
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate);
+          const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
+          for (int sw = 0; sw < 2; ++sw) {
+            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, root, pv, py, n, 2, 2);
+            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, py, py2, n, 2, 2);
+            if (!ritz_norm) {
+              TONER_LAUNCH(undeflate_kernel, dim3(kc, 2), 256, stream, py2, py, dv, coef8, n, defl_r, kMaxDeflate);
+            }
+            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, root, py2, py, n, 2, 2);
+            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est));
+          }
+        } else if (ritz_norm) {
           // The norm was an estimate too.  Eigenvalues of M_0 above 1 (the estimate was too low for them) come out of
           // the first Newton step BELOW the lower bound the schedule continues from -- T = a I - b M is small there --
           // and lag the same way; they belong to the top of A', so the same four steps from the largest Ritz vector
@@ -1920,7 +2197,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             TONER_LAUNCH(power_shift_kernel, kc, 256, stream, pv, py, n, e_est, 1, 0);
           }
         }
-        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm ? e_top : nullptr, (float)(1.15 * (1.0 - l_last) + 1e-3), status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc);
+        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm || graded.products ? e_top : nullptr, graded.products ? kGradedResidual : (float)(1.15 * (1.0 - l_last) + 1e-3), status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc, graded.products ? 1 : 0);
         TONER_CUDA(cudaGetLastError());
       }
       const int sweeps = track_sweeps & 63;

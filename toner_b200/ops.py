@@ -344,6 +344,18 @@ def inv_roots_schedule(lower: float, p: int, iters: int = 0) -> dict:
             "coefficients": [coef[j] for j in range(order.value + 1)], "distance": e.value}
 
 
+def inv_roots_graded(lower: float, p: int, n: int) -> Optional[dict]:
+    """The schedule of a call on statistics of width n whose bound is an estimate (toner_inv_roots_graded_for; needs no device), where it ends in a
+    graded finish: {"steps": Newton steps, "products": K, "split": inner split products, "z": (zb, za),
+    "coefficients": [(alpha_j, beta_j), ...]}, else None."""
+    steps, split, coef = C.c_int32(0), C.c_int32(0), (C.c_double * 32)()
+    k = _lib.load().toner_inv_roots_graded_for(lower, p, n, C.byref(steps), C.byref(split), coef, 32)
+    if k <= 0:
+        return None
+    return {"steps": steps.value, "products": k, "split": split.value, "z": (coef[0], coef[1]),
+            "coefficients": [(coef[2 * j + 2], coef[2 * j + 3]) for j in range(k + 1)]}
+
+
 def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: int = 0,
               root_lo: Optional[torch.Tensor] = None, root_hi: Optional[torch.Tensor] = None,
               fro2_lo: Optional[torch.Tensor] = None, status: Optional[torch.Tensor] = None,

@@ -168,9 +168,7 @@ def bench_roots_tracked(a):
         f.finish()
 
     ms, best = timed(fn, 1, a.reps, False)
-    log2p, log2q = int(math.log2(a.p)), int(math.log2(a.q))
-    split = (f.iterations - 1) * (log2p + 2) + log2q
-    single = f.finish_products
+    split, single = f.products
     flops = a.k * (split + single) * 2 * a.n ** 3
     return report("inv_roots_tracked", {"k": a.k, "n": a.n, "p": a.p, "q": a.q, "cond": a.cond}, ms, best, flops=flops,
                   extra={"iterations": f.iterations, "finish_order": f.finish_order, "split_products": split,
