@@ -227,10 +227,11 @@ static bool may_interleave(const toner_gemm_desc& d) {
 
 // Which tile, and among how many units a tile's accumulation is divided (only where the caller gave scratch for it).  An
 // estimate of the launch in SM cycles decides, from what was measured on the kernel:
-//   * the main loop is bound by shared memory (128 B per clock: operands written by TMA and read by the MMAs), 512 cycles
-//     per 64-deep k-block of 256 x 256 on a pair and of 128 x 128 on one CTA, 384 of 256 x 128 on a pair and of 128 x 64,
-//     768 of 128 x 256;
-//   * interleaved plane products bring two thirds of the operands: 256 x 256 stays bound by its MMAs, 256 x 128 takes 500;
+//   * a 64-deep k-block takes 512 cycles of 256 x 256 on a pair and of 128 x 128 on one CTA, 384 of 256 x 128 on a pair and of
+//     128 x 64, 768 of 128 x 256 -- what their copies take; deep products are faster by a quarter on the small tiles, which they
+//     do not use;
+//   * interleaved plane products bring two thirds of the operands: 256 x 256 stays bound by its MMAs, 256 x 128 takes 320 (one
+//     product of 768 14.6 us plane by plane on 128 x 64, 13.8 interleaved on 256 x 128; twelve 25.5 on 256 x 256, 24.5);
 //   * a 32 x 32 block of the epilogue takes a warp 900 cycles plus 450 per box moved, and its boxes take shared memory away
 //     from the main loop of the next tile;
 //   * tiles of one wave run side by side, and the epilogue of one tile beside the main loop of the next.
@@ -242,7 +243,7 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
     bool pair;
     double per_kb, per_kb_inter;
   };
-  static const Config configs[] = {{256, true, 512, 512}, {128, true, 384, 500}, {256, false, 768, 768}, {128, false, 512, 512}, {64, false, 384, 384}};
+  static const Config configs[] = {{256, true, 512, 512}, {128, true, 384, 320}, {256, false, 768, 768}, {128, false, 512, 512}, {64, false, 384, 384}};
   const bool inter = may_interleave(d);
   const bool mirror = d.tri && d.mirror;
   const double boxes = (d.c ? 1.2 : 0.0) + (d.d ? (mirror && !d.upper_d ? 2.0 : 1.0) : 0.0) + (d.d16 ? (mirror ? 1.6 : 1.0) : 0.0) +
@@ -278,16 +279,17 @@ static TileChoice choose_tile(const Context* ctx, const toner_gemm_desc& d) {
     }
   }
   if (best.bn == 256 && best.pair && best.splits == 1 && d.promote <= 0 && !inter && kb >= ctx->gemm_wide_kb) {
-    // The wide tile takes in 48 KB per k-block for twice the work of 32 KB, but its epilogue is only half hidden and its
-    // waves are coarser.  Estimates of both, in k-blocks of the pair tile (measured wide / pair: 12 x 3072^3 x 3 planes
-    // symmetric 0.94, 2 x 4096^3 0.86, 12 x 768 x 3072 x 3072 0.89, 18 x 2048^3 0.99; one plane, under the power limit: 8192^3
-    // 0.86, 24 x 2048^2 x 5632 0.92, 6 x 5632^3 symmetric with C 0.95; below 80 k-blocks above 1).
+    // The wide tile takes in 48 KB per k-block for twice the work of 32 KB and draws less power for it, but its epilogue is only
+    // half hidden and its waves are coarser, and symmetric results have more of it below the diagonal.  Estimates of both, in
+    // k-blocks of the pair tile; a k-block takes 1.72 (few waves) to 2 of those (measured wide / pair, three planes symmetric:
+    // 2 x 4096^3 0.86, 12 x 3072^3 1.07, 18 x 2048^3 1.10, 6 x 5632^3 1.03, 32 x 512^3 1.15; one plane: 8192^3 0.96, 2 x 4096^3
+    // symmetric 0.89, 6 x 5632^3 symmetric with C 1.14).
     auto waves = [&](int bn) {
       const long long t = gemm_tiles(d, bn, true), w = ctx->gemm_sms / 2;
       return (double)((t + w - 1) / w);
     };
-    const double epi = 8 * block * 0.6 / 736.0;
-    if (waves(512) * (kb * 1.5 + epi) < 0.97 * waves(256) * kb) best.bn = 512;
+    const double epi = 8 * block * 0.6 / 541.0;
+    if (waves(512) * (kb * 1.8 + epi) < 0.97 * waves(256) * kb) best.bn = 512;
   }
   return best;
 }
