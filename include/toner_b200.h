@@ -353,6 +353,10 @@ int toner_factor_report(const int32_t* status, const float* norms, const float* 
 size_t toner_ns_polar_workspace_bytes(int32_t batch, int32_t m, int32_t n);
 int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t steps, float eps, float* x_out,
                    uint32_t* maxabs_out, void* workspace, size_t workspace_bytes, void* stream);
+/* The same; beside = 1: other work of the caller's runs on the GPU at the same time (another stream).  The products are then
+ * launched one by one, where an iteration alone has them all in one launch that keeps its SMs to the end. */
+int toner_ns_polar_beside(const float* u, int32_t batch, int32_t m, int32_t n, int32_t steps, float eps, float* x_out,
+                          uint32_t* maxabs_out, int32_t beside, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------ elementwise update kernels
  * Stacks are `count` matrices of `per` elements each (per a multiple of 4); gradient and weight tensors

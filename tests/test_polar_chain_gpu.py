@@ -1,0 +1,65 @@
+"""The polar iteration's products in one launch (up to a short side of 1536) against the same products launched one by one: the
+same operands, roundings and order of additions per element, so the same bits."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def one_by_one(ops, u, steps, eps=1e-5):
+    batch, m, n = u.shape
+    wide, a = m <= n, min(m, n)
+    norm = ops.sumsq(u).sqrt()
+    x = u * (1.0 / (norm + eps)).view(-1, 1, 1)
+    cur = x.to(torch.bfloat16)
+    gram, gram_b = torch.empty(batch, a, a, device="cuda"), torch.empty(batch, a, a, device="cuda", dtype=torch.bfloat16)
+    poly = torch.empty_like(gram_b)
+    for _ in range(steps):
+        op = ops.operand(cur, mn_major=not wide)
+        ops.gemm(op, op, m=a, n=a, k=max(m, n), batch=batch, fmt=1, tri=True, mirror=True, d=gram, d16=gram_b)
+        g = ops.operand(gram_b)
+        ops.gemm(g, g, m=a, n=a, k=a, batch=batch, fmt=1, tri=True, mirror=True, c=gram, d16=poly, alpha=2.0315, beta=-4.7750)
+        b, c, nxt = ops.operand(poly), ops.operand(cur, mn_major=wide), torch.empty_like(cur)
+        left, right = (b, c) if wide else (c, b)
+        ops.gemm(left, right, m=m, n=n, k=a, batch=batch, fmt=1, c=x, d=x, d16=nxt, beta=3.4445)
+        cur = nxt
+    return x
+
+
+@pytest.mark.parametrize("batch,m,n", [
+    (1, 8, 8), (3, 8, 24), (2, 64, 64), (1, 128, 72), (5, 136, 256), (2, 256, 264), (4, 264, 256), (1, 520, 1288), (7, 768, 768),
+    (40, 256, 512), (3, 1000, 680), (2, 2304, 768), (1, 1536, 1536), (2, 1544, 1536), (1, 1544, 1544), (9, 768, 2304)])
+@pytest.mark.parametrize("steps", [1, 2, 9])
+def test_same_bits_as_single_products(batch, m, n, steps):
+    from toner_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(batch + m + n + steps)
+    u = torch.randn(batch, m, n, device="cuda", generator=gen) * 0.1
+    want = one_by_one(ops, u, steps)
+    top = torch.full((batch,), 7, device="cuda", dtype=torch.int32)
+    got = ops.ns_polar(u, steps, maxabs=top)
+    ops.assert_healthy()
+    assert torch.equal(got, want), float((got - want).abs().max())
+    assert torch.equal(top.view(torch.float32), want.abs().amax(dim=(1, 2)))
+    again = ops.ns_polar(u, steps, beside=True)       # the products launched one by one by the library itself
+    assert torch.equal(got, again)
+
+
+def test_chains_side_by_side_on_streams():
+    """Several chains at once, each holding a part of the GPU: none waits for a tile that nobody runs."""
+    from toner_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    us = [torch.randn(b, m, n, device="cuda", generator=gen) for b, m, n in ((6, 768, 768), (3, 1536, 512), (1, 768, 768), (12, 256, 768))]
+    want = [ops.ns_polar(u, 6) for u in us]
+    outs = [torch.empty_like(u) for u in us]
+    spaces = [torch.empty(ops.ns_polar_workspace_bytes(*u.shape), device="cuda", dtype=torch.uint8) for u in us]
+    streams = [torch.cuda.Stream() for _ in us]
+    torch.cuda.synchronize()
+    for _ in range(8):
+        for u, out, ws, stream in zip(us, outs, spaces, streams):
+            with torch.cuda.stream(stream):
+                ops.ns_polar(u, 6, out=out, workspace=ws)
+    torch.cuda.synchronize()
+    ops.assert_healthy()
+    for out, ref in zip(outs, want):
+        assert torch.equal(out, ref)

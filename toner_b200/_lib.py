@@ -105,6 +105,7 @@ SIGNATURES = {
                                          _vp, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "toner_factor_report": (C.c_int, [_vp, _vp, _vp, _vp, _i32, _vp, _vp]),
     "toner_ns_polar_workspace_bytes": (C.c_size_t, [_i32, _i32, _i32]),
+    "toner_ns_polar_beside": (C.c_int, [_vp, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _i32, _vp, _sz, _vp]),
     "toner_ns_polar": (C.c_int, [_vp, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _vp, _sz, _vp]),
     "toner_sumsq_scratch_bytes": (C.c_size_t, [_i32]),
     "toner_sumsq": (C.c_int, [_vp, _i32, _i32, _i32, _i64, _i64, _vp, _vp, _vp]),

@@ -36,6 +36,7 @@ class Scratch:
         # inside one it does not -- what a lane hands back another could be given while the lane still works on it --, so
         # buffers that have been outgrown are kept until the lanes have been joined.
         self.home: Optional[torch.cuda.Stream] = None
+        self.beside = False     # other lanes are at work at the same time
         self._outgrown: List[torch.Tensor] = []
 
     def _empty(self, shape, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
@@ -69,7 +70,7 @@ class Scratch:
 
     def joined(self) -> None:
         """The home stream is ordered behind everything that has used this scratch."""
-        self.home = None
+        self.home, self.beside = None, False
         self._outgrown.clear()
 
 
@@ -100,6 +101,8 @@ class Lanes:
             current = torch.cuda.current_stream()
             ready = current.record_event()
         try:
+            for lane in by_lane:
+                self.scratch[lane].beside = len(by_lane) > 1
             for lane in others:
                 self.scratch[lane].home = current
                 with torch.cuda.stream(self.streams[lane - 1]):
@@ -517,7 +520,7 @@ def muont_group_delta(group: MatrixGroup, grads: Sequence[torch.Tensor], delta: 
     work = muont_ns_input(group, grads, scratch, momentum=momentum, nesterov=nesterov)
     maxabs = scratch.get("maxabs_polar", (count,), torch.int32, dev)
     ns_ws = scratch.bytes_like("ns", ops.ns_polar_workspace_bytes(count, m, n), dev)
-    ops.ns_polar(work, ns_steps, ns_eps, out=work, maxabs=maxabs, workspace=ns_ws)
+    ops.ns_polar(work, ns_steps, ns_eps, out=work, maxabs=maxabs, workspace=ns_ws, beside=scratch.beside)
     muont_delta_from_polar(group, work, delta, scratch, lr=lr, weight_decay=weight_decay, polar_maxabs=maxabs)
 
 
@@ -541,7 +544,7 @@ def muont_groups_delta(groups: Sequence[MatrixGroup], grads: Sequence[Sequence[t
     for g, gr, w in zip(groups, grads, slices):
         muont_ns_input(g, gr, scratch, momentum=momentum, nesterov=nesterov, work=w)
     ns_ws = scratch.bytes_like("ns", ops.ns_polar_workspace_bytes(total, m, n), dev)
-    ops.ns_polar(merged, ns_steps, ns_eps, out=merged, maxabs=maxabs, workspace=ns_ws)
+    ops.ns_polar(merged, ns_steps, ns_eps, out=merged, maxabs=maxabs, workspace=ns_ws, beside=scratch.beside)
     for j, (g, w, d) in enumerate(zip(groups, slices, deltas)):
         muont_delta_from_polar(g, w, d, scratch, lr=lr, weight_decay=weight_decay,
                                polar_maxabs=maxabs[j * count:(j + 1) * count], work=w)

@@ -140,7 +140,7 @@ struct GemmSmem {
   // 4 KB blocks per epilogue warp
   static constexpr int kEpiBufs = kStageBytes > 32 * 1024 || (kInter && kStageBytes == 32 * 1024) ? 1 : 2;
   static constexpr int kEpiBytes = 8 * kEpiBufs * kEpiBlockBytes;
-  static constexpr int kBarBytes = 256;
+  static constexpr int kBarBytes = 320;
   static constexpr int kTotal = kTileBytes + kEpiBytes + kBarBytes + 1024;  // 1024: alignment slack
   static constexpr int kTmemCols = kWide ? 512 : 2 * BN;
 };

@@ -56,6 +56,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// The same, ordered after what another CTA of the cluster released.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Wait with a wall-clock bound (cycles).  Returns false when the bound ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long limit_cycles) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -67,10 +79,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 }
 
 // The same, and also false once *stop is set; looked at only while waiting, which a thread soon does when others have stopped.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait_unless(uint32_t bar, uint32_t parity, long long limit_cycles, const volatile int* stop) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto done = [&]() { return kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+  if (done()) return true;
   const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
+  while (!done()) {
     if (*stop || clock64() - t0 > limit_cycles) return false;
   }
   return true;
@@ -91,6 +105,18 @@ __device__ __forceinline__ void reg_inc() {
 // ---------------------------------------------------------------- proxies / fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+// (all state spaces) orders what this thread has seen before the asynchronous copies it issues next, and the other way round
+__device__ __forceinline__ void fence_proxy_async() {
+  asm volatile("fence.proxy.async;" ::: "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release_gpu(unsigned int* p, unsigned int v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void fence_tensormap_acquire(const void* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
@@ -195,6 +221,10 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v
 // Arrive on an mbarrier that may live in the peer CTA (address from mapa).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same, releasing what this thread wrote or read before to the CTA that waits.
+__device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // 3-D tiled load into this CTA's shared memory whose completion is signalled on an mbarrier of the pair's
 // leader CTA (address from mapa).  One destination CTA per copy.

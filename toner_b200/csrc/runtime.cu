@@ -1,6 +1,9 @@
 // Per-device context, TMA tensor-map cache and the GEMM launcher.
 #include "runtime.cuh"
 
+#include "polar_chain.cuh"
+
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -106,6 +109,9 @@ Context* context() {
   allow(gemm_tcgen05_kernel<128, true, true, true>, GemmSmem<128, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, false, true, true>, GemmSmem<256, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, true, true, true>, GemmSmem<256, true, true>::kTotal);
+  allow(polar_chain_kernel<256, true>, GemmSmem<256, true>::kTotal);
+  allow(polar_chain_kernel<128, true>, GemmSmem<128, true>::kTotal);
+  allow(polar_chain_kernel<64, false>, GemmSmem<64>::kTotal);
   allow(gemm_tcgen05_kernel<512, false, true>, GemmSmem<512, true>::kTotal);
   if (!ok) {
     set_error("the GEMM kernels' shared memory was refused");
@@ -303,43 +309,8 @@ size_t gemm_split_bytes(const toner_gemm_desc& desc) {
   return choose_tile(ctx, d).ws_bytes;
 }
 
-int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
-  Context* ctx = context();
-  if (!ctx) return kErrCuda;
-  if (d.m <= 0 || d.n <= 0 || d.k <= 0 || d.batch <= 0) return fail(kErrArg, "gemm: sizes must be positive");
-  if (d.segs < 1 || d.segs > kMaxSegs) return fail(kErrArg, "gemm: segs must be 1..3");
-  if (d.tri && d.m != d.n) return fail(kErrArg, "gemm: a symmetric result needs m == n");
-  if (d.packed && (!d.tri || d.mirror || d.d16)) return fail(kErrArg, "gemm: packed output is upper-triangle FP32 only");
-  if (!d.d && !d.d16 && !d.split0 && !d.split1) return fail(kErrArg, "gemm: no output");
-  if (d.packed && (d.split0 || d.split1)) return fail(kErrArg, "gemm: operand planes cannot be packed");
-  if (reinterpret_cast<uintptr_t>(d.split_ws) & 15u) return fail(kErrArg, "gemm: split_ws must be 16-byte aligned");
-  if (d.fmt != 0 && d.fmt != 1) return fail(kErrArg, "gemm: fmt must be 0 (FP16) or 1 (BF16)");
-
-  int bn = d.tile_n, splits = 1;
-  bool pair = false;
-  if (bn == 0) {
-    const TileChoice t = choose_tile(ctx, d);
-    bn = t.bn;
-    pair = t.pair;
-    splits = t.splits;
-  } else if (bn == 512) {
-    bn = 256;
-    pair = true;
-  } else if (bn == -128) {
-    bn = 128;
-    pair = true;
-  } else if (bn == 1024) {
-    if (d.promote > 0) return fail(kErrArg, "gemm: the wide tile has no chained accumulation");
-    bn = 512;
-    pair = true;
-  }
-  if (!(bn == 64 && !pair) && bn != 128 && bn != 256 && !(bn == 512 && pair))
-    return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
-                         "(256 x 512 on a pair)");
-
-  const bool inter = pair && bn <= 256 && may_interleave(d);
-
-  GemmParams p;
+// The kernel's parameters for one product on a given tile.
+static int gemm_params(Context* ctx, const toner_gemm_desc& d, int bn, bool pair, int splits, bool inter, cudaStream_t stream, GemmParams& p) {
   std::memset(&p, 0, sizeof(p));
   // a pair's CTA loads half a tile's rows of B, at most 128 at a time; MN-major operands always come in 64 x 64 boxes
   auto operand_map = [&](const toner_operand& op, int box_rows, CUtensorMap* map, const CUtensorMap** maps) {
@@ -401,6 +372,46 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   }
   p.status = ctx->status_dev;
   p.prof = ctx->prof_dev;
+  return 0;
+}
+
+int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
+  Context* ctx = context();
+  if (!ctx) return kErrCuda;
+  if (d.m <= 0 || d.n <= 0 || d.k <= 0 || d.batch <= 0) return fail(kErrArg, "gemm: sizes must be positive");
+  if (d.segs < 1 || d.segs > kMaxSegs) return fail(kErrArg, "gemm: segs must be 1..3");
+  if (d.tri && d.m != d.n) return fail(kErrArg, "gemm: a symmetric result needs m == n");
+  if (d.packed && (!d.tri || d.mirror || d.d16)) return fail(kErrArg, "gemm: packed output is upper-triangle FP32 only");
+  if (!d.d && !d.d16 && !d.split0 && !d.split1) return fail(kErrArg, "gemm: no output");
+  if (d.packed && (d.split0 || d.split1)) return fail(kErrArg, "gemm: operand planes cannot be packed");
+  if (reinterpret_cast<uintptr_t>(d.split_ws) & 15u) return fail(kErrArg, "gemm: split_ws must be 16-byte aligned");
+  if (d.fmt != 0 && d.fmt != 1) return fail(kErrArg, "gemm: fmt must be 0 (FP16) or 1 (BF16)");
+
+  int bn = d.tile_n, splits = 1;
+  bool pair = false;
+  if (bn == 0) {
+    const TileChoice t = choose_tile(ctx, d);
+    bn = t.bn;
+    pair = t.pair;
+    splits = t.splits;
+  } else if (bn == 512) {
+    bn = 256;
+    pair = true;
+  } else if (bn == -128) {
+    bn = 128;
+    pair = true;
+  } else if (bn == 1024) {
+    if (d.promote > 0) return fail(kErrArg, "gemm: the wide tile has no chained accumulation");
+    bn = 512;
+    pair = true;
+  }
+  if (!(bn == 64 && !pair) && bn != 128 && bn != 256 && !(bn == 512 && pair))
+    return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
+                         "(256 x 512 on a pair)");
+
+  const bool inter = pair && bn <= 256 && may_interleave(d);
+  GemmParams p;
+  if (int rc = gemm_params(ctx, d, bn, pair, splits, inter, stream, p)) return rc;
 
   const long long total = gemm_tiles(d, bn, pair) * splits;
   if (total > 0x7fffffffLL) return fail(kErrArg, "gemm: too many tiles");
@@ -431,6 +442,67 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   else if (chained) TONER_GEMM(64, true, false);
   else TONER_GEMM(64, false, false);
 #undef TONER_GEMM
+  return 0;
+}
+
+int launch_polar_chain(const toner_gemm_desc (&ops)[6], int steps, unsigned int* claim, unsigned int* done, cudaStream_t stream,
+                       bool* taken) {
+  *taken = false;
+  Context* ctx = context();
+  if (!ctx) return kErrCuda;
+  // Deeper products hide their ends behind their own tiles, and a few large matrices have nothing to overlap (launched / chained:
+  // 24 x 2048^2 8384 / 8424 us, 2 x 2048 x 8192 2084 / 2214, one 2048^2 618 / 795).  One matrix alone gains little a step, and
+  // the launch costs ten microseconds more of host time (768^2, called alone, five steps 131 / 143 us, ten 254 / 254).
+  constexpr int kChainDepth = 1536, kChainSteps = 8;
+  if (ops[2].k > kChainDepth || (ops[0].batch == 1 && steps < kChainSteps)) return 0;
+  struct Config {
+    int bn;
+    bool pair;
+    double per_kb;
+  };
+  // As in choose_tile, but a product's last wave is filled by the next product's tiles: what counts is the time of a tile, times
+  // the tiles a worker gets, and that of a whole tile, first copy to last store, where a product has fewer tiles than workers.
+  static const Config configs[] = {{256, true, 541}, {128, true, 400}, {64, false, 384}};
+  const Config* best = nullptr;
+  double best_cost = 0.0;
+  for (const Config& c : configs) {
+    double cost = 0.0;
+    for (int i : {0, 2, 3}) {
+      const toner_gemm_desc& d = ops[i];
+      const double boxes = (d.c ? 1.2 : 0.0) + (d.d ? 1.0 : 0.0) + (d.d16 ? (d.tri ? 1.6 : 1.0) : 0.0);
+      const double main = (d.k + kBK - 1) / kBK * c.per_kb, epi = c.bn / 64 * (300.0 + 850.0 * boxes);
+      const double tiles = (double)gemm_tiles(d, c.bn, c.pair) / (c.pair ? ctx->gemm_sms / 2 : ctx->gemm_sms);
+      const double each = std::max(main, epi) + 0.25 * std::min(main, epi);   // (they share the SM's paths to L2)
+      cost += std::max(tiles * each, main + epi + 4000.0);
+    }
+    if (!best || cost < best_cost) {
+      best = &c;
+      best_cost = cost;
+    }
+  }
+  PolarChain p;
+  std::memset(&p, 0, sizeof(p));
+  for (int i = 0; i < 6; ++i) {
+    if (int rc = gemm_params(ctx, ops[i], best->bn, best->pair, 1, false, stream, p.op[i])) return rc;
+    if (!p.op[i].tma_ok) return 0;
+  }
+  p.steps = steps;
+  p.batch = ops[0].batch;
+  const int workers = best->pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
+  long long widest = 0;
+  for (int i = 0; i < 3; ++i) {
+    const toner_gemm_desc& d = ops[i + (i > 0)];
+    p.tiles[i] = gemm_tiles_per_batch(d.m, d.n, best->bn, d.tri, best->pair ? 2 * kBM : kBM);
+    widest = std::max(widest, (long long)p.tiles[i] * p.batch);
+  }
+  if (widest * 3 * steps > 0x3fffffffLL) return 0;   // (unit numbers and done[] have 32 bits)
+  p.claim = claim;
+  p.done = done;
+  const int grid = (int)(widest < workers ? widest : workers) * (best->pair ? 2 : 1);
+  if (best->bn == 256) TONER_CUDA(launch(polar_chain_kernel<256, true>, grid, kChainThreads, GemmSmem<256, true>::kTotal, stream, 2, p));
+  else if (best->bn == 128) TONER_CUDA(launch(polar_chain_kernel<128, true>, grid, kChainThreads, GemmSmem<128, true>::kTotal, stream, 2, p));
+  else TONER_CUDA(launch(polar_chain_kernel<64, false>, grid, kChainThreads, GemmSmem<64>::kTotal, stream, 0, p));
+  *taken = true;
   return 0;
 }
 

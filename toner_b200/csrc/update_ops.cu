@@ -19,12 +19,19 @@ static int ew_grid4(long long elems4, int num_sms) { return ew_grid((elems4 + 3)
 
 // ------------------------------------------------------------------ Newton-Schulz helpers
 // x = u / (||u|| + eps), written as FP32 and as BF16 (the operand the products read); ||u||^2 as the partial sums that
-// sumsq_det left (each block adds them up itself: 1.2 KB from L2, against a launch of its own)
+// sumsq_det left (each block adds them up itself: 1.2 KB from L2, against a launch of its own).  On the way: the counters of
+// the products that follow, and the maxima the last of them finds, start at zero.
 __global__ void __launch_bounds__(256) ns_scale_kernel(const float* __restrict__ u, const float* __restrict__ partial,
                                                        float eps, long long per, float* __restrict__ x,
-                                                       __nv_bfloat16* __restrict__ xb) {
+                                                       __nv_bfloat16* __restrict__ xb, unsigned int* __restrict__ counters,
+                                                       unsigned int* __restrict__ maxabs) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    counters[b + 1] = 0;
+    if (b == 0) counters[0] = 0;
+    if (maxabs) maxabs[b] = 0;
+  }
   __shared__ float norm;
   if (threadIdx.x < 32) {
     const float t = sumsq_total(partial + (long long)b * kSumsqBlocks, threadIdx.x);
@@ -277,14 +284,19 @@ size_t toner_ns_polar_workspace_bytes(int32_t batch, int32_t m, int32_t n) {
   if (batch <= 0 || m <= 0 || n <= 0) return 0;
   const size_t a = (size_t)(m < n ? m : n);
   const size_t mn = (size_t)m * n;
-  return align_up(sumsq_scratch_bytes(batch), 256) +
+  return align_up(sumsq_scratch_bytes(batch), 256) + align_up((size_t)(batch + 1) * 4, 256) +
          2 * align_up(mn * 2 * batch, 256) +                 // two BF16 copies of X (read one, write the other)
          align_up(a * a * 4 * batch, 256) +                  // Gram, FP32
          2 * align_up(a * a * 2 * batch, 256);               // Gram and polynomial, BF16
 }
 
 int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t steps, float eps, float* x_out,
-                   uint32_t* maxabs_out, void* workspace, size_t workspace_bytes, void* stream_) {
+                   uint32_t* maxabs_out, void* workspace, size_t workspace_bytes, void* stream) {
+  return toner_ns_polar_beside(u, batch, m, n, steps, eps, x_out, maxabs_out, 0, workspace, workspace_bytes, stream);
+}
+
+int toner_ns_polar_beside(const float* u, int32_t batch, int32_t m, int32_t n, int32_t steps, float eps, float* x_out,
+                          uint32_t* maxabs_out, int32_t beside, void* workspace, size_t workspace_bytes, void* stream_) {
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -298,6 +310,7 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
   char* w = static_cast<char*>(workspace);
   float* partial = reinterpret_cast<float*>(w); w += align_up(sumsq_scratch_bytes(batch), 256);
   __nv_bfloat16* xb[2];
+  unsigned int* counters = reinterpret_cast<unsigned int*>(w); w += align_up((size_t)(batch + 1) * 4, 256);
   xb[0] = reinterpret_cast<__nv_bfloat16*>(w); w += align_up((size_t)mn * 2 * batch, 256);
   xb[1] = reinterpret_cast<__nv_bfloat16*>(w); w += align_up((size_t)mn * 2 * batch, 256);
   float* gram = reinterpret_cast<float*>(w); w += align_up((size_t)aa * 4 * batch, 256);
@@ -306,7 +319,7 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
 
   int rc = sumsq_det(u, batch, m, n, n, mn, partial, nullptr, stream);
   if (rc) return rc;
-  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid4(mn / 4, ctx->num_sms), batch), 256, stream, u, partial, eps, mn, x_out, xb[0]);
+  TONER_LAUNCH(ns_scale_kernel, dim3(ew_grid4(mn / 4, ctx->num_sms), batch), 256, stream, u, partial, eps, mn, x_out, xb[0], counters, maxabs_out);
   TONER_CUDA(cudaGetLastError());
 
   const float ca = 3.4445f, cb = -4.7750f, cc = 2.0315f;  // src/toner/linalg.py:9
@@ -317,57 +330,60 @@ int toner_ns_polar(const float* u, int32_t batch, int32_t m, int32_t n, int32_t 
     op.mn_major = mn_major; op.z_step = 1;
     return op;
   };
-  for (int s = 0; s < steps; ++s) {
-    const __nv_bfloat16* cur = xb[s & 1];
-    __nv_bfloat16* nxt = xb[(s + 1) & 1];
-    const bool last = (s == steps - 1);
-    {  // A = x x^T on the short side (symmetric): FP32 and BF16 copies
-      toner_gemm_desc g = {};
-      g.a = op16(cur, m, n, wide ? 0 : 1);
-      g.b = g.a;
-      g.m = a; g.n = a; g.k = wide ? n : m; g.batch = batch; g.segs = 1; g.fmt = 1;
-      g.tri = 1; g.mirror = 1; g.alpha = 1.f;
-      g.upper_d = 1;  // the FP32 Gram is read back only as the upper-triangle C of the polynomial product below
-      g.d = gram; g.ldd = a; g.d_bs = aa;
-      g.d16 = gram_b; g.ld16 = a; g.d16_bs = aa; g.d16_fmt = 1;
-      rc = launch_gemm(g, stream);
-      if (rc) return rc;
+  // A = x x^T on the short side (symmetric): FP32 and BF16 copies
+  auto gram_of = [&](const __nv_bfloat16* cur) {
+    toner_gemm_desc g = {};
+    g.a = op16(cur, m, n, wide ? 0 : 1);
+    g.b = g.a;
+    g.m = a; g.n = a; g.k = wide ? n : m; g.batch = batch; g.segs = 1; g.fmt = 1;
+    g.tri = 1; g.mirror = 1; g.alpha = 1.f;
+    g.upper_d = 1;  // the FP32 Gram is read back only as the upper-triangle C of the polynomial product below
+    g.d = gram; g.ldd = a; g.d_bs = aa;
+    g.d16 = gram_b; g.ld16 = a; g.d16_bs = aa; g.d16_fmt = 1;
+    return g;
+  };
+  // B = b A + c A A, rounded to BF16 for the next product
+  auto polynomial = [&]() {
+    toner_gemm_desc g = {};
+    g.a = op16(gram_b, a, a, 0);
+    g.b = g.a;
+    g.m = a; g.n = a; g.k = a; g.batch = batch; g.segs = 1; g.fmt = 1;
+    g.tri = 1; g.mirror = 1; g.alpha = cc; g.beta = cb;
+    g.c = gram; g.ldc = a; g.c_bs = aa;
+    g.d16 = poly_b; g.ld16 = a; g.d16_bs = aa; g.d16_fmt = 1;
+    return g;
+  };
+  // x <- a x + B x  (wide)   or   x <- a x + x B  (tall); nxt: the BF16 copy for the next step
+  auto update = [&](const __nv_bfloat16* cur, __nv_bfloat16* nxt) {
+    toner_gemm_desc g = {};
+    if (wide) {
+      g.a = op16(poly_b, a, a, 0);
+      g.b = op16(cur, m, n, 1);  // B operand indexed [n_index][k]: x stored (k, n_index) is its transposed view
+    } else {
+      g.a = op16(cur, m, n, 0);
+      g.b = op16(poly_b, a, a, 0);  // symmetric: B^T = B
     }
-    {  // B = b A + c A A, rounded to BF16 for the next product
-      toner_gemm_desc g = {};
-      g.a = op16(gram_b, a, a, 0);
-      g.b = g.a;
-      g.m = a; g.n = a; g.k = a; g.batch = batch; g.segs = 1; g.fmt = 1;
-      g.tri = 1; g.mirror = 1; g.alpha = cc; g.beta = cb;
-      g.c = gram; g.ldc = a; g.c_bs = aa;
-      g.d16 = poly_b; g.ld16 = a; g.d16_bs = aa; g.d16_fmt = 1;
-      rc = launch_gemm(g, stream);
-      if (rc) return rc;
+    g.m = m; g.n = n; g.k = a; g.batch = batch; g.segs = 1; g.fmt = 1;
+    g.alpha = 1.f; g.beta = ca;
+    g.c = x_out; g.ldc = n; g.c_bs = mn;
+    g.d = x_out; g.ldd = n; g.d_bs = mn;
+    if (nxt) {
+      g.d16 = nxt; g.ld16 = n; g.d16_bs = mn; g.d16_fmt = 1;
+    } else {
+      g.maxabs = maxabs_out;
     }
-    {  // x <- a x + B x  (wide)   or   x <- a x + x B  (tall)
-      toner_gemm_desc g = {};
-      if (wide) {
-        g.a = op16(poly_b, a, a, 0);
-        g.b = op16(cur, m, n, 1);  // B operand indexed [n_index][k]: x stored (k, n_index) is its transposed view
-      } else {
-        g.a = op16(cur, m, n, 0);
-        g.b = op16(poly_b, a, a, 0);  // symmetric: B^T = B
-      }
-      g.m = m; g.n = n; g.k = a; g.batch = batch; g.segs = 1; g.fmt = 1;
-      g.alpha = 1.f; g.beta = ca;
-      g.c = x_out; g.ldc = n; g.c_bs = mn;
-      g.d = x_out; g.ldd = n; g.d_bs = mn;
-      if (!last) {
-        g.d16 = nxt; g.ld16 = n; g.d16_bs = mn; g.d16_fmt = 1;
-      } else if (maxabs_out) {
-        TONER_CUDA(cudaMemsetAsync(maxabs_out, 0, sizeof(uint32_t) * batch, stream));
-        g.maxabs = maxabs_out;
-      }
-      rc = launch_gemm(g, stream);
-      if (rc) return rc;
-    }
+    return g;
+  };
+  const toner_gemm_desc ops[6] = {gram_of(xb[0]), gram_of(xb[1]), polynomial(), update(xb[0], xb[1]), update(xb[1], xb[0]),
+                                  update(xb[(steps - 1) & 1], nullptr)};
+  bool taken = false;
+  rc = beside ? 0 : launch_polar_chain(ops, steps, counters, counters + 1, stream, &taken);
+  for (int s = 0; s < steps && !taken && !rc; ++s) {
+    rc = launch_gemm(ops[s & 1], stream);
+    if (!rc) rc = launch_gemm(ops[2], stream);
+    if (!rc) rc = launch_gemm(s + 1 < steps ? ops[3 + (s & 1)] : ops[5], stream);
   }
-  return 0;
+  return rc;
 }
 
 int toner_sumsq(const float* x, int32_t batch, int32_t rows, int32_t cols, int64_t ld, int64_t bs, float* scratch,

@@ -99,7 +99,7 @@ class Muon(torch.optim.Optimizer):
         count = st["buf"].shape[0]
         if self.dist is None:
             ws = scratch.bytes_like("ns", ops.ns_polar_workspace_bytes(count, *shape), u.device)
-            o = ops.ns_polar(u, g["ns_steps"], g["eps"], out=st["u"], workspace=ws)
+            o = ops.ns_polar(u, g["ns_steps"], g["eps"], out=st["u"], workspace=ws, beside=scratch.beside)
         else:   # rank r takes matrices r, r + W, ...; padded to equal shares for the all-gather
             world, rank = self.dist.get_world_size(), self.dist.get_rank()
             per = -(-count // world)

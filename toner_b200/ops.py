@@ -429,8 +429,9 @@ def ns_polar_workspace_bytes(batch: int, m: int, n: int) -> int:
 
 
 def ns_polar(u: torch.Tensor, steps: int = 10, eps: float = 1e-5, *, out: Optional[torch.Tensor] = None,
-             maxabs: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Newton-Schulz polar iteration with BF16 operands / FP32 accumulation on a (batch, m, n) stack."""
+             maxabs: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None, beside: bool = False) -> torch.Tensor:
+    """Newton-Schulz polar iteration with BF16 operands / FP32 accumulation on a (batch, m, n) stack.  `beside`: other work of
+    the caller's is on the GPU at the same time (toner_ns_polar_beside)."""
     _need_cuda(u)
     if u.ndim == 2:
         u = u.unsqueeze(0)
@@ -442,8 +443,8 @@ def ns_polar(u: torch.Tensor, steps: int = 10, eps: float = 1e-5, *, out: Option
     need = ns_polar_workspace_bytes(batch, m, n)
     if workspace is None:
         workspace = torch.empty(need, device=u.device, dtype=torch.uint8)
-    check(_lib.load().toner_ns_polar(u.data_ptr(), batch, m, n, steps, eps, out.data_ptr(), _ptr(maxabs),
-                                     workspace.data_ptr(), workspace.numel(), _stream()), "toner_ns_polar")
+    check(_lib.load().toner_ns_polar_beside(u.data_ptr(), batch, m, n, steps, eps, out.data_ptr(), _ptr(maxabs), int(beside),
+                                            workspace.data_ptr(), workspace.numel(), _stream()), "toner_ns_polar")
     return out
 
 
