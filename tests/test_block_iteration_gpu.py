@@ -1,0 +1,46 @@
+"""The passes over a statistic that its block iteration makes -- damping, products with 1 to 8 vectors -- at widths around the edges of
+their tiles (64 columns, 16 or 32 rows, slices of 256 columns): the vectors found are eigenvectors and the roots are right."""
+
+import pytest
+import torch
+
+from oracle import toner_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DAMPING = 1e-3
+
+
+@pytest.mark.parametrize("n", [16, 56, 64, 72, 248, 256, 264, 520, 1032])
+@pytest.mark.parametrize("rank", [1, 3, 5, 8])
+def test_vectors_and_roots_at_the_edges(n, rank):
+    from toner_b200 import ops
+    k, strong = 3, max(1, rank - 2)
+    gen = torch.Generator().manual_seed(10 * n + rank)
+    stats = []
+    for _ in range(k):
+        q, _ = torch.linalg.qr(torch.randn(n, n, generator=gen, dtype=torch.float64))
+        lam = 1.0 + torch.rand(n, generator=gen, dtype=torch.float64)
+        lam[:strong] = 40.0 * n * 1.7 ** torch.arange(strong, dtype=torch.float64)   # (far above the rest, whatever n)
+        c = (q * lam) @ q.T
+        stats.append((0.5 * (c + c.T)).float())
+    ema = torch.stack(stats).cuda()
+    ema[1] += torch.triu(torch.full((n, n), 1e-4, device="cuda"), 1) - torch.tril(torch.full((n, n), 1e-4, device="cuda"), -1)
+    vectors, count = torch.zeros(k, 8, n, device="cuda"), torch.zeros(k, device="cuda", dtype=torch.int32)
+    track = torch.zeros(k, n, device="cuda")
+    for first in (True, False):
+        lo, hi, _, st = ops.inv_roots(ema, DAMPING, 8, 4, track=track, track_sweeps=8, track_restart=first, deflate=vectors,
+                                      deflate_rank=rank, deflate_restart=first, deflated=count)
+    ops.assert_healthy()
+    assert st.tolist() == [0] * k
+    for b in range(k):
+        c = ema[b].double().cpu()
+        c = 0.5 * (c + c.T)                       # (the second statistic has an antisymmetric part, which does not count)
+        a = c / c.diagonal().mean() + DAMPING * torch.eye(n, dtype=torch.float64)
+        v = vectors[b, :rank].double().cpu()
+        assert torch.allclose(v @ v.T, torch.eye(rank, dtype=torch.float64), atol=2e-6)
+        for j in range(count[b].item() & 255):    # what was deflated has a residual below 1e-5
+            av = a @ v[j]
+            theta = (v[j] @ av).item()
+            assert (av - theta * v[j]).norm().item() < 2e-5 * theta
+        assert orc.rel_fro(lo[b].cpu(), orc.inverse_root_truth(c.float(), 0.125, DAMPING)) < 1e-4
+        assert orc.rel_fro(hi[b].cpu(), orc.inverse_root_truth(c.float(), 0.5, DAMPING)) < 4e-4

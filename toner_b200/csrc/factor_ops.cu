@@ -434,37 +434,59 @@ __global__ void __launch_bounds__(256) trace_kernel(const float* __restrict__ c,
 }
 
 // A = sym(C) / max(trace/n, 1e-30) + damping I, written to `a`.
-// 32x32 tile pairs so that C and C^T are both read along rows.
+// 64 x 64 tile pairs, so that C and C^T are both read along rows, by 16-byte accesses with the whole pair (32 KB a block) on its
+// way at once; blocks are numbered over the tiles of the upper triangle.  HBM bounds it: 32 statistics of width 2048 and 96 of 512
+// 366 -> 227 us (with 32 x 32 tiles, 4-byte accesses and a block per tile of the square).
+constexpr int kDampTile = 64;
 __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, float* __restrict__ a, int n, float damping,
                                                    const float* __restrict__ trace) {
   ptx::pdl_begin();
-  const int ti = blockIdx.y, tj = blockIdx.x;
-  if (ti > tj) return;
-  __shared__ float up[32][33], lo[32][33];
-  const long long b = blockIdx.z;
+  __shared__ float up[kDampTile][kDampTile + 1], lo[kDampTile][kDampTile + 1];
+  int ti = 0, rest = blockIdx.x;
+  for (int row = (n + kDampTile - 1) / kDampTile; rest >= row; --row) {
+    rest -= row;
+    ++ti;
+  }
+  const int tj = ti + rest;
+  const long long b = blockIdx.y;
   const float* C = c + b * (long long)n * n;
   float* A = a + b * (long long)n * n;
   const float inv = 1.f / fmaxf(trace[b] / n, 1e-30f);
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int tx = (threadIdx.x & 15) * 4, ty = threadIdx.x >> 4;   // 16 bytes of a row, 16 rows at a time
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 u[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int lr = ty + 8 * i;
-    const int r = ti * 32 + lr, cc = tj * 32 + tx;
-    up[lr][tx] = (r < n && cc < n) ? C[(long long)r * n + cc] : 0.f;
-    const int r2 = tj * 32 + lr, c2 = ti * 32 + tx;
-    lo[lr][tx] = (r2 < n && c2 < n) ? C[(long long)r2 * n + c2] : 0.f;
+    const int lr = ty + 16 * i, r = ti * kDampTile + lr, cc = tj * kDampTile + tx;
+    const int r2 = tj * kDampTile + lr, c2 = ti * kDampTile + tx;
+    u[i] = (r < n && cc < n) ? *reinterpret_cast<const float4*>(C + (long long)r * n + cc) : zero;    // (n is a multiple of 8)
+    l[i] = (r2 < n && c2 < n) ? *reinterpret_cast<const float4*>(C + (long long)r2 * n + c2) : zero;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int lr = ty + 16 * i;
+    up[lr][tx] = u[i].x; up[lr][tx + 1] = u[i].y; up[lr][tx + 2] = u[i].z; up[lr][tx + 3] = u[i].w;
+    lo[lr][tx] = l[i].x; lo[lr][tx + 1] = l[i].y; lo[lr][tx + 2] = l[i].z; lo[lr][tx + 3] = l[i].w;
   }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int lr = ty + 8 * i;
+    const int lr = ty + 16 * i;
     {
-      const int r = ti * 32 + lr, cc = tj * 32 + tx;
-      if (r < n && cc < n) A[(long long)r * n + cc] = 0.5f * (up[lr][tx] + lo[tx][lr]) * inv + (r == cc ? damping : 0.f);
+      const int r = ti * kDampTile + lr, cc = tj * kDampTile + tx;
+      const float v[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = 0.5f * (v[e] + lo[tx + e][lr]) * inv + (r == cc + e ? damping : 0.f);
+      if (r < n && cc < n) *reinterpret_cast<float4*>(A + (long long)r * n + cc) = make_float4(o[0], o[1], o[2], o[3]);
     }
     if (ti != tj) {
-      const int r = tj * 32 + lr, cc = ti * 32 + tx;
-      if (r < n && cc < n) A[(long long)r * n + cc] = 0.5f * (lo[lr][tx] + up[tx][lr]) * inv;
+      const int r = tj * kDampTile + lr, cc = ti * kDampTile + tx;
+      const float v[4] = {l[i].x, l[i].y, l[i].z, l[i].w};
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = 0.5f * (v[e] + up[tx + e][lr]) * inv;
+      if (r < n && cc < n) *reinterpret_cast<float4*>(A + (long long)r * n + cc) = make_float4(o[0], o[1], o[2], o[3]);
     }
   }
 }
@@ -684,77 +706,93 @@ __global__ void __launch_bounds__(256) rank1_update_kernel(float* __restrict__ a
 // Vectors are stored vector-major: v[(b * vstride + j) * n + c].
 constexpr int kMaxDeflate = 8;  // (init_planes_kernel keeps that many coefficients in registers)
 
-// Y_j = A v_j, j < R: one pass over A.  A block takes 32 rows (four per warp) and walks the columns 256 at a time; the
+// Y_j = A v_j, j < R: one pass over A.  A block takes 32 rows (four per warp; 16 and two from six vectors on) and walks the columns 256 at a time; the
 // 256-column slice of the vectors is staged in shared memory once per block, so the vectors are read from L2 once per
 // 32 rows instead of once per row pair (that traffic, not the pass over A, bounded the first version of this kernel).
 // The products of four slices (32 per lane) are summed in FP32 before they join the FP64 sums: conversions and FP64
 // additions run at a fraction of the FP32 rate, and with one per eight products they, not the pass over A, set the
 // pace.  R (the number of vectors, rounded up to even) is a template argument so that absent vectors cost nothing.
-// With eight vectors the sums alone are 96 registers and few warps fit: the next slice, of A in registers and of the
-// vectors in the other half of shared memory, is fetched while this one is multiplied (12 statistics of width 3072, eight
-// vectors: 262 -> 158 us a pass; two vectors 94 -> 75, at HBM's rate 69).
-constexpr int kBlockGemvRows = 32;
+// What bounds the rest is how much of A is on its way: slices come by asynchronous copies into shared memory, two (three for the
+// wide blocks of vectors) ahead of the one being multiplied, with two blocks on an SM 128 KB.  With the next slice in registers it was
+// 64 KB, and 32 with the one block that eight vectors' sums for four rows leave room for, hence two rows a warp there: 32
+// statistics of width 2048 and 96 of 512, four vectors, 104 -> 70 us a pass, two vectors 79 -> 60; eight vectors on 12 of
+// width 1280 and four of 3328 128 -> 102.
 template <int R>
-__global__ void __launch_bounds__(256, R <= 4 ? 2 : 1) block_gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
-                                                         float* __restrict__ y, int n, int r, int vstride) {
+struct BlockGemv {
+  static constexpr int kWarpRows = R <= 4 ? 4 : 2;
+  static constexpr int kRows = 8 * kWarpRows;
+  static constexpr int kStages = R <= 4 ? 3 : 4;
+  static constexpr int kStageFloat4 = (kRows + R) * 64;   // 256 columns of the block's rows and of the vectors
+  static constexpr int kBytes = kStages * kStageFloat4 * 16;
+};
+template <int R>
+__global__ void __launch_bounds__(256, 2) block_gemv_kernel(const float* __restrict__ a, const float* __restrict__ v,
+                                                            float* __restrict__ y, int n, int r, int vstride) {
   ptx::pdl_begin();
-  __shared__ float4 sv[2][R][64];
+  using B = BlockGemv<R>;
+  constexpr int kWarpRows = B::kWarpRows;
+  extern __shared__ float4 gemv_smem[];
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = blockIdx.x * kBlockGemvRows + warp * 4;
+  const int row0 = blockIdx.x * B::kRows + warp * kWarpRows;
   const float* V = v + (long long)b * vstride * n;
   const float* A = a + (long long)b * n * n;
-  double acc[4][R];
-  float part[4][R];
+  double acc[kWarpRows][R];
+  float part[kWarpRows][R];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < kWarpRows; ++i)
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       acc[i][j] = 0.0;
       part[i][j] = 0.f;
     }
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  constexpr int kShare = (R * 64 + 255) / 256;   // elements of a vector slice a thread brings in
-  float4 vn[kShare], p0[4], p1[4];
-  auto fetch = [&](int c0) {
+  // slice `k`, 256 columns: a warp's rows, two 16-byte pieces a lane and row; zeros outside the matrix
+  auto fetch = [&](int k) {
+    float4* const stage = gemv_smem + (k % B::kStages) * B::kStageFloat4;
+    const int c0 = k * 256;
+    if (c0 < n) {
 #pragma unroll
-    for (int q = 0; q < kShare; ++q) {
-      const int i = threadIdx.x + 256 * q, j = i >> 6, col = c0 + (i & 63) * 4;
-      vn[q] = (j < r && col < n) ? *reinterpret_cast<const float4*>(V + (long long)j * n + col) : zero;
-    }
-    const int ca = c0 + lane * 4, cb = ca + 128;
+      for (int q = 0; q < (R * 64 + 255) / 256; ++q) {
+        const int i = threadIdx.x + 256 * q, j = i >> 6, col = c0 + (i & 63) * 4;
+        if (i < R * 64) {
+          const bool in = j < r && col < n;
+          ptx::cp_async16(ptx::smem_u32(stage + B::kRows * 64 + i), in ? V + (long long)j * n + col : V, in);
+        }
+      }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = row0 + i;
-      const float* Ar = A + (long long)row * n;
-      p0[i] = (row < n && ca < n) ? *reinterpret_cast<const float4*>(Ar + ca) : zero;
-      p1[i] = (row < n && cb < n) ? *reinterpret_cast<const float4*>(Ar + cb) : zero;
+      for (int i = 0; i < kWarpRows; ++i) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int col = c0 + (lane + 32 * h) * 4;
+          const bool in = row0 + i < n && col < n;
+          ptx::cp_async16(ptx::smem_u32(stage + (warp * kWarpRows + i) * 64 + lane + 32 * h),
+                          in ? A + (long long)(row0 + i) * n + col : A, in);
+        }
+      }
     }
+    ptx::cp_async_commit();
   };
-  fetch(0);
+#pragma unroll
+  for (int k = 0; k < B::kStages - 1; ++k) fetch(k);
   int slice = 0;
   for (int c0 = 0; c0 < n; c0 += 256, ++slice) {
-    float4 (&now)[R][64] = sv[slice & 1];   // (last read two slices ago, before the barrier of the slice between)
+    ptx::cp_async_wait<B::kStages - 2>();
+    __syncthreads();                     // the slice is there for everyone, and the stage filled next has been read by everyone
+    fetch(slice + B::kStages - 1);
+    const float4* const stage = gemv_smem + (slice % B::kStages) * B::kStageFloat4;
+    float4 a0[kWarpRows], a1[kWarpRows];
 #pragma unroll
-    for (int q = 0; q < kShare; ++q) {
-      const int i = threadIdx.x + 256 * q;
-      if (i < R * 64) now[i >> 6][i & 63] = vn[q];
+    for (int i = 0; i < kWarpRows; ++i) {
+      a0[i] = stage[(warp * kWarpRows + i) * 64 + lane];
+      a1[i] = stage[(warp * kWarpRows + i) * 64 + lane + 32];
     }
-    float4 a0[4], a1[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a0[i] = p0[i];
-      a1[i] = p1[i];
-    }
-    __syncthreads();
-    if (c0 + 256 < n) fetch(c0 + 256);
-    // a lane's eight columns of a vector are read from shared memory once for the warp's four rows (read per row, the
+    // a lane's eight columns of a vector are read from shared memory once for the warp's rows (read per row, the
     // shared-memory traffic is R times the traffic of A and sets the pace from four vectors on)
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const float4 x0 = now[j][lane], x1 = now[j][lane + 32];
+      const float4 x0 = stage[(B::kRows + j) * 64 + lane], x1 = stage[(B::kRows + j) * 64 + lane + 32];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < kWarpRows; ++i) {
         const float s0 = fmaf(a0[i].x, x0.x, fmaf(a0[i].y, x0.y, fmaf(a0[i].z, x0.z, a0[i].w * x0.w)));
         const float s1 = fmaf(a1[i].x, x1.x, fmaf(a1[i].y, x1.y, fmaf(a1[i].z, x1.z, a1[i].w * x1.w)));
         part[i][j] += s0 + s1;
@@ -762,7 +800,7 @@ __global__ void __launch_bounds__(256, R <= 4 ? 2 : 1) block_gemv_kernel(const f
     }
     if ((slice & 3) == 3) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < kWarpRows; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
           acc[i][j] += (double)part[i][j];
@@ -771,7 +809,7 @@ __global__ void __launch_bounds__(256, R <= 4 ? 2 : 1) block_gemv_kernel(const f
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kWarpRows; ++i) {
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       double t = acc[i][j] + (double)part[i][j];
@@ -780,6 +818,18 @@ __global__ void __launch_bounds__(256, R <= 4 ? 2 : 1) block_gemv_kernel(const f
       if (lane == 0 && j < r && row0 + i < n) y[((long long)b * vstride + j) * n + row0 + i] = (float)t;
     }
   }
+}
+template <int R>
+static cudaError_t launch_block_gemv(int k, cudaStream_t stream, const float* a, const float* v, float* y, int n, int r, int vstride) {
+  return launch(block_gemv_kernel<R>, dim3((n + BlockGemv<R>::kRows - 1) / BlockGemv<R>::kRows, k), 256, BlockGemv<R>::kBytes, stream, 0,
+                a, v, y, n, r, vstride);
+}
+bool allow_factor_kernels() {
+  auto allow = [](auto kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+  };
+  return allow(block_gemv_kernel<2>, BlockGemv<2>::kBytes) && allow(block_gemv_kernel<4>, BlockGemv<4>::kBytes) &&
+         allow(block_gemv_kernel<6>, BlockGemv<6>::kBytes) && allow(block_gemv_kernel<8>, BlockGemv<8>::kBytes);
 }
 
 // Sum over the block of one double per thread; every thread gets the total.  256 threads.
@@ -1723,9 +1773,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     TONER_CUDA(cudaMemsetAsync(w, 0, sm * 19 + 4 * sm8, stream));
 
     const float* C = ema + (long long)k0 * nn;
-    const int t32 = (n + 31) / 32;
+    const int damp_tiles = (n + kDampTile - 1) / kDampTile;
     TONER_LAUNCH(trace_kernel, kc, 256, stream, C, n, trace);
-    TONER_LAUNCH(damp_kernel, dim3(t32, t32, kc), 256, stream, C, A32, n, damping, trace);
+    TONER_LAUNCH(damp_kernel, dim3(damp_tiles * (damp_tiles + 1) / 2, kc), 256, stream, C, A32, n, damping, trace);
     if (defl_r > 0) {
       // dominant directions: block power iteration with Rayleigh-Ritz on the caller's vectors (eight sweeps from fixed
       // vectors -- the first three or four only find the subspace --, four from last call's), then deflate those that
@@ -1735,7 +1785,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         constexpr int R = decltype(width)::value;
         TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0, in_order);
         for (int sw = 0; sw < sweeps; ++sw) {
-          TONER_LAUNCH(block_gemv_kernel<R>, dim3((n + kBlockGemvRows - 1) / kBlockGemvRows, kc), 256, stream, A32, dv, py, n, defl_r, kMaxDeflate);
+          TONER_CUDA(launch_block_gemv<R>(kc, stream, A32, dv, py, n, defl_r, kMaxDeflate));
           TONER_LAUNCH(ritz_kernel<R>, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order);
         }
         return 0;
@@ -2168,14 +2218,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           const float* root = (q > 1 ? root_hi : root_lo) + (long long)k0 * nn;
           float* const py2 = py + (long long)kc * 2 * n;
           TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate);
-          const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
           for (int sw = 0; sw < 2; ++sw) {
-            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, root, pv, py, n, 2, 2);
-            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, py, py2, n, 2, 2);
+            TONER_CUDA(launch_block_gemv<2>(kc, stream, root, pv, py, n, 2, 2));
+            TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, py, py2, n, 2, 2));
             if (!ritz_norm) {
               TONER_LAUNCH(undeflate_kernel, dim3(kc, 2), 256, stream, py2, py, dv, coef8, n, defl_r, kMaxDeflate);
             }
-            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, root, py2, py, n, 2, 2);
+            TONER_CUDA(launch_block_gemv<2>(kc, stream, root, py2, py, n, 2, 2));
             TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est));
           }
         } else if (ritz_norm) {
@@ -2185,9 +2234,8 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // that stayed in A' find them.  (An eigenvalue beyond a / b, where T changes sign, makes M grow instead and
           // fails the convergence test.)  Both starting vectors go through M in one pass per step.
           TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate);
-          const dim3 bg((n + kBlockGemvRows - 1) / kBlockGemvRows, kc);
           for (int sw = 0; sw < 4; ++sw) {
-            TONER_LAUNCH(block_gemv_kernel<2>, bg, 256, stream, A32, pv, py, n, 2, 2);
+            TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, pv, py, n, 2, 2));
             TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est));
           }
         } else {

@@ -113,8 +113,8 @@ Context* context() {
   allow(polar_chain_kernel<128, true>, GemmSmem<128, true>::kTotal);
   allow(polar_chain_kernel<64, false>, GemmSmem<64>::kTotal);
   allow(gemm_tcgen05_kernel<512, false, true>, GemmSmem<512, true>::kTotal);
-  if (!ok) {
-    set_error("the GEMM kernels' shared memory was refused");
+  if (!ok || !allow_factor_kernels()) {
+    set_error("the kernels' shared memory was refused");
     return nullptr;
   }
   c.device = dev;

@@ -71,6 +71,9 @@ cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
 }
 #define TONER_LAUNCH(kernel, grid, threads, stream, ...) TONER_CUDA(launch(kernel, dim3(grid), threads, 0, stream, 0, __VA_ARGS__))
 
+// Shared-memory limits of the factor engine's kernels on the current device; false where they were refused.
+bool allow_factor_kernels();
+
 // Context of the current device (created on first use).  Returns nullptr and sets the error on failure.
 Context* context();
 
