@@ -231,7 +231,8 @@ int toner_split16(const float* x, const float* const* x_list, int32_t batch, int
  * `iters` <= 0 selects toner_inv_roots_iterations(n, damping, p), which depends only on
  * its arguments (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632, damping 1e-3): the count with the fewest
  * plane passes, Newton steps and series together.
- * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step,
+ * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step (1 before a graded finish,
+ * 1.5 of max|I - Z^2| where no Newton step precedes it),
  * 2 non-finite, 3 / 4 a caller's spectrum bound that did not hold (toner_inv_roots_ex / _tracked).  The caller decides what to do with a non-zero status (the Python host recomputes that
  * statistic with an eigendecomposition, as the reference's fallback does, src/toner/fast/engine.py:714-731).
  * Workspace: toner_inv_roots_workspace_bytes(chunk, n) lets `chunk` statistics be processed at once; a
