@@ -228,9 +228,9 @@ int toner_split16(const float* x, const float* const* x_list, int32_t batch, int
  * alone: the Chebyshev interpolant of (1 - r)^(-1/p) on [-0.02, 1.15 e + 1e-3] of the smallest degree with relative
  * error below 3e-6, e being the bound on R the schedule guarantees (toner_inv_roots_finish_order_for,
  * toner_inv_roots_schedule), evaluated by single passes over FP16 planes of R (toner_inv_roots_finish_products_for).
- * `iters` <= 0 selects toner_inv_roots_iterations(n, damping, p), which depends only on
- * its arguments (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632, damping 1e-3): the count with the fewest
- * plane passes, Newton steps and series together.
+ * `iters` <= 0 selects the schedule with the fewest plane passes, steps and finish together, which depends only on n, damping,
+ * p and the bound: toner_inv_roots_iterations(n, damping, p) linear steps (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632,
+ * damping 1e-3, the finish counted), or the fewer steps of higher degree that toner_inv_roots_steps_for states.
  * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step (before a
  * graded finish max|I - Z^2| above 1.5),
  * 2 non-finite, 3 / 4 a caller's spectrum bound that did not hold (toner_inv_roots_ex / _tracked).  The caller decides what to do with a non-zero status (the Python host recomputes that
@@ -246,7 +246,7 @@ int toner_inv_roots_iterations_for(float lower, int32_t p);   /* the count for a
 int toner_inv_roots_finish_order_for(float lower, int32_t p, int32_t iters);
 /* How many single-pass products evaluate that polynomial (plane_order: 1 for calls with track_sweeps + 512). */
 int toner_inv_roots_finish_products_for(float lower, int32_t p, int32_t iters, int32_t plane_order);
-/* The whole schedule the engine runs for a spectrum lower bound (host only, no device needed): returns the step count
+/* The whole schedule of linear steps for a spectrum lower bound (host only, no device needed): returns the step count
  * (iters <= 0: the default), and writes the (a_k, b_k) of its count - 1 Newton steps (ab_out: pairs of doubles, as many
  * as ab_capacity holds), the degree of the finishing polynomial (order_out), its coefficients c_0 .. c_degree in powers
  * of r (coef_out, as many as coef_capacity holds; at most 13), and the distance e of the last M from I it is cut for
@@ -263,6 +263,14 @@ int toner_inv_roots_schedule(float lower, int32_t p, int32_t iters, double* ab_o
  * most 28 doubles).  Every output pointer is optional; needs no device. */
 int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps_out, int32_t* split_out, double* coef_out,
                                int32_t coef_capacity);
+/* The steps of a call that asks for no step count and no plane order, on statistics of width n, where that costs less than
+ * linear ones: T of degree 1, 2 or 4 in M, levelled like the linear T (129 times the lower bound instead of 13 for two products
+ * more at degree 4, p = 8).  Returns their number (0: the schedule of toner_inv_roots_schedule is used) and writes seven doubles
+ * a step (degree, zb, za, kappa, top, lin, con: with z = zb + za mu, T is con + lin mu plus nothing, top z^2 or
+ * top (z^2 + kappa)^2), the finishing polynomial and the distance e as toner_inv_roots_schedule does, and products_out[0], [1]: the split and the single-pass
+ * products that steps and finish take.  Every output pointer is optional; needs no device. */
+int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, double* step_out, int32_t step_capacity, double* coef_out,
+                              int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out);
 int toner_inv_roots(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
                     float* root_lo, float* root_hi, float* fro2_lo, int32_t* status, void* workspace,
                     size_t workspace_bytes, void* stream);
@@ -301,7 +309,8 @@ int toner_inv_roots_ex(const float* ema, int32_t k, int32_t n, float damping, in
  *                  A' / norm, typically margin * min_b lmin_out[b] / norm_out[b] of the previous call.  Such a bound
  *                  cannot be checked in advance; it is verified after the chain: four power-iteration steps on
  *                  R = I - M of the last M, from the tracked direction, estimate ||R||_2, and status[b] = 4 where that
- *                  exceeds what the finishing series was cut for (by 15 % + 1e-3).  After a graded finish
+ *                  exceeds what the finishing series was cut for (by 15 % + 1e-3; after steps of higher degree also
+ *                  where R reaches below -0.03).  After a graded finish
  *                  (toner_inv_roots_graded_for) R is I - A^(-1/2) A A^(-1/2) instead, from the computed root, on the
  *                  complement of the deflated directions: p times the relative error of A^(-1/p).  Two steps from the
  *                  tracked direction and from the largest Ritz vector that stayed in A', each with 1 / sqrt(n) of every other

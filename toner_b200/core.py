@@ -213,6 +213,7 @@ class FactorSet:
             self.hi_planes, self.hi_inv = self.lo_planes, self.lo_inv
         self._lower_used = 0.0           # the bound the last call's schedule was built for, and whether it was an estimate
         self._used_estimate = False
+        self._ran = False
         per = ops.inv_roots_workspace_bytes(1, n)
         if k == 0:            # a rank that owns no statistic of this width (weighted ownership): nothing to factor
             self.workspace = None
@@ -236,8 +237,17 @@ class FactorSet:
         return ops.inv_roots_graded(self._lower_used, self.p, self.n)
 
     @property
+    def steps(self) -> Optional[dict]:
+        """The steps of higher degree (ops.inv_roots_steps) that the last factorisation took in place of `iterations`' linear
+        ones; None where it took those, or the graded finish."""
+        if self.k == 0 or not self._ran or not self.interleave or self.graded:
+            return None
+        return ops.inv_roots_steps(max(self._lower_used, self.damping / (self.n * (1.0 + self.damping))), self.p, self.n)
+
+    @property
     def iterations(self) -> int:
-        """Newton steps of the last factorisation, the finish counted as one (before the first: of the bound that always holds)."""
+        """Linear Newton steps for the last factorisation's bound, the finish counted as one (before the first: for the bound that
+        always holds); a graded finish counts as one.  `steps` says where fewer of a higher degree took their place."""
         if self.k == 0:
             return 0
         g = self.graded
@@ -251,7 +261,9 @@ class FactorSet:
         """Degree of the last factorisation's finishing polynomial."""
         if self.k == 0:
             return 0
-        g = self.graded
+        g, s = self.graded, self.steps
+        if s:
+            return len(s["coefficients"]) - 1
         return 2 * g["products"] + 1 if g else ops.inv_roots_finish_order(self.n, self.damping, self.p, self._lower_used)
 
     @property
@@ -259,7 +271,9 @@ class FactorSet:
         """Single-pass products of the last factorisation's finish."""
         if self.k == 0:
             return 0
-        g = self.graded
+        g, s = self.graded, self.steps
+        if s:
+            return s["products"][1]
         return (g["products"] - 1 - g["split"] if g else
                 ops.inv_roots_finish_products(self.n, self.damping, self.p, self._lower_used, interleave=self.interleave))
 
@@ -269,8 +283,10 @@ class FactorSet:
         if self.k == 0:
             return 0, 0
         log2p, log2q = self.p.bit_length() - 1, self.q.bit_length() - 1
-        g = self.graded
+        g, s = self.graded, self.steps
         split = 2 + g["split"] if g else (self.iterations - 1) * (log2p + 2)   # (graded: U, the root and the inner ones)
+        if s:
+            split = s["products"][0]
         return split + log2q, self.finish_products
 
     # -- which stored root serves a given strength
@@ -327,6 +343,7 @@ class FactorSet:
         self.track_restart = False
         self._estimate_in_flight = self._used_estimate = self.lower_is_estimate
         self._lower_used = self.lower
+        self._ran = True
         self._norm_hi()
         ops.factor_report(self.status, self.norms, self.lmin, self.deflated, self._host)
         self.status_event = torch.cuda.Event()

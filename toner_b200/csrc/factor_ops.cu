@@ -18,15 +18,13 @@
 // made it, scaled by a power of two taken from a norm bound known in advance.
 #include <cmath>
 #include <cstdlib>
+#include <unordered_map>
 #include <vector>
 
+#include "root_steps.cuh"
 #include "runtime.cuh"
 
 namespace toner {
-
-struct NewtonStep {
-  double a, b, lower;
-};
 
 // Dynamic range allowed for T^p.  The unconstrained minimax step sends the top of the spectrum (mu = 1)
 // down to the new lower bound, i.e. T = a I - b M gets an eigenvalue (a - b) << a and T^p spans
@@ -74,6 +72,20 @@ static int chain_length(double lower) {
   if (lower < 5e-2) return kPromoteLinear;
   return 0;
 }
+
+// The same after steps of higher degree.  Fewer products and these chains leave the roots 0.4 times as far from FP64 as linear
+// steps do (median of 540 calls, p = 4 and 8: Marchenko-Pastur spectra of 1.5 to 6 rows a column, log-uniform ones of condition 30
+// to 1e5, widths 264 to 2048, bounds from the one that always holds to the spectrum's end), 1.06 times in the worst; two k-blocks
+// below 5e-3: 1.6 times in the worst, below 5e-4: 1.7; eight from 5e-2 on, as the linear steps have: 1.7.  (12 products of 3072:
+// 790 us in one chain, 920 in chains of eight k-blocks, 980 of two, 1000 to 1150 of one.)
+static int steep_chain_length(double lower) {
+  if (lower < 5e-3) return 1;
+  if (lower < 0.5) return kPromoteAccurate;
+  return 0;
+}
+// Products with X, and the final squarings, which in one chain would be 8 times as far off in the worst case: their one-sided
+// truncation no longer cancels part of the iteration's.
+constexpr int kPromoteSteepX = 2, kPromoteSteepSquares = 1;
 
 // Products applied to X (and the final squarings) pass their error on linearly: one chain, about 1e-5.
 constexpr int kPromoteX = 0;
@@ -366,6 +378,76 @@ static GradedPoly graded_poly(int p, double lo, const GradedCare& care) {
   return g;
 }
 
+// Cost of a single pass in split products: 0.43 of one at width 3072, 0.5 at 2048, 0.77 at 768, where writing the results is most
+// of it (interleaved products in batches; C and operand planes as the finish has them).
+static double single_pass(int n) { return 0.35 + 320.0 / n; }
+
+// Newton steps of degree 1, 2 and 4 (root_steps.cuh) in the order that costs least.  Between steps the bound of M's spectrum is
+// rounded down to an eighth of an octave: every schedule is then a path through 256 bounds, whose steps (0.1 ms of host
+// time a bound to find) and finishing polynomials a thread keeps, and a bound that moves a little from call to call costs nothing.  Against
+// exact bounds a step loses 4 % of l' on average.
+// The last product of the finish is a split one: single passes lose 2^-12 e^2 of it, which linear steps' own errors cover and these
+// would not (p = 8, e = 0.59: A^(-1/2) 2.5 times as far off as after linear steps without, 0.94 times with it).
+constexpr int kBoundsPerOctave = 8, kBounds = 32 * kBoundsPerOctave;
+constexpr int kSteepFrom = 256;   // columns: on narrower statistics linear steps can be closer (by 2.8 times, of 8e-7, 8 wide)
+struct BoundNode {
+  bool ok[3] = {};
+  NewtonStep step[3];
+  FinishPoly fin[3];       // after that step; order 0: M is too far from I
+  int fin_products[3] = {};
+};
+static double bound_of(int j) { return std::exp2(-(double)j / kBoundsPerOctave); }
+static int bound_below(double l) { return std::max(1, (int)std::ceil(-kBoundsPerOctave * std::log2(l) - 1e-6)); }
+
+static const BoundNode& bound_node(int p, int j) {
+  static thread_local std::unordered_map<int, BoundNode> known;   // (at most kBounds for each of six p)
+  const auto found = known.find(p * kBounds + j);
+  if (found != known.end()) return found->second;
+  BoundNode& node = known[p * kBounds + j];
+  for (int i = 0; i < 3; ++i) {
+    node.ok[i] = best_step(p, bound_of(j), kStepDegrees[i], kMaxPowerRange, node.step[i]);
+    if (!node.ok[i]) continue;
+    node.fin[i] = finish_poly(p, 1.0 - node.step[i].next);
+    QuadraticSteps q;
+    if (node.fin[i].order)
+      node.fin_products[i] = quadratic_steps(node.fin[i], p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : node.fin[i].order - 1;
+  }
+  return node;
+}
+
+struct StepPlan {
+  double cost = 1e9;                // in split products, the finish and its product with X counted
+  std::vector<std::pair<int, int>> path;   // (bound, degree's index)
+};
+// Cheapest steps from bound j on; `memo` is the call's own.
+static const StepPlan& cheapest(int p, int j, double single, std::unordered_map<int, StepPlan>& memo) {
+  const auto found = memo.find(j);
+  if (found != memo.end()) return found->second;
+  StepPlan best;
+  const BoundNode& node = bound_node(p, j);
+  int log2p = 0;
+  while ((1 << log2p) < p) ++log2p;
+  for (int i = 2; i >= 0; --i) {
+    if (!node.ok[i]) continue;
+    // powers, M, the next product with X, and T's own: with a linear term it writes and reads an FP32 matrix more
+    const double own = log2p + 2 + (kStepDegrees[i] == 4 ? 2 : kStepDegrees[i] - 1) + (node.step[i].lin != 0.0 ? 0.25 : 0.0);
+    const double end = single * (node.fin_products[i] - 1) + 1.0;
+    if (node.fin[i].order && own + end < best.cost) {
+      best.cost = own + end;
+      best.path = {{j, i}};
+    }
+    const int next = bound_below(node.step[i].next);
+    if (next >= j || node.step[i].next > 0.9 || own + log2p + 2 >= best.cost) continue;
+    const StepPlan& rest = cheapest(p, next, single, memo);
+    if (own + rest.cost < best.cost) {
+      best.cost = own + rest.cost;
+      best.path = {{j, i}};
+      best.path.insert(best.path.end(), rest.path.begin(), rest.path.end());
+    }
+  }
+  return memo[j] = best;
+}
+
 // Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
 // Working it out takes tens of microseconds of host time and is asked for several times per factorisation (the call itself,
 // the step count and the degree it states), so a thread keeps the last few.
@@ -373,6 +455,8 @@ struct Schedule {
   double l0 = 0.0;
   int p = 0, asked = 0;   // asked: the caller's step count, 0 = the one with the fewest plane passes; -n: graded
                           // finishes considered as well, for statistics of width n
+  int steep_n = 0;        // > 0: steps of higher degree considered as well, for statistics of that width
+  bool steep = false;     // ... and taken: cheaper than linear ones
   int iters = 0;
   std::vector<NewtonStep> steps;
   double l_last = 0.0;    // lower bound of the spectrum of the last M, i.e. after iters - 1 updates
@@ -380,18 +464,20 @@ struct Schedule {
   GradedPoly graded;      // graded.products > 0: this finish, of M_0 itself (iters == 1)
 };
 
-static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0) {
+static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0, int steep_n = 0) {
   constexpr int kKept = 8;
   static thread_local Schedule kept[kKept];
   static thread_local int oldest = 0;
   iters = iters > 0 ? iters : -grade_n;
   for (const Schedule& s : kept)
-    if (s.p == p && s.l0 == l0 && s.asked == iters) return s;
+    if (s.p == p && s.l0 == l0 && s.asked == iters && s.steep_n == steep_n) return s;
   Schedule& s = kept[oldest];
   oldest = (oldest + 1) % kKept;
   s.p = 0;   // (not a match until it is complete)
   s.l0 = l0;
   s.asked = iters;
+  s.steep_n = steep_n;
+  s.steep = false;
   s.iters = iters > 0 ? iters : default_iterations(l0, p);
   if (s.iters >= 2) {
     s.steps = newton_schedule(l0, p, s.iters, nullptr);
@@ -401,13 +487,13 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
   s.graded = GradedPoly();
   if (iters < 0) {
     const int n = grade_n;
-    // Costs in split products.  A single pass takes 0.43 of one at width 3072, 0.5 at 2048, 0.77 at 768, where writing the results
-    // is most of it (interleaved products in batches; C and operand planes as the finish has them); the final squarings, in short
-    // chains after a graded finish, a tenth more at 3072 and a third at 768.  k updates of M are k (log2 p + 1) split products and
-    // k - 1 products with X; Newton's finish ends in one with X, the graded one makes U and the root.
+    // Costs in split products.  The final squarings, in short chains after a graded finish, take a tenth more at width 3072 and a
+    // third at 768.  k linear updates of M are k (log2 p + 1) split products and k - 1 products with X; Newton's finish ends in one
+    // with X, the graded one makes U and the root.  (Against steps of higher degree, which take fewer products, the graded finish
+    // stays where it is the cheaper one of these two: it is ten times closer to the root.)
     int log2p = 0;
     while ((1 << log2p) < p) ++log2p;
-    const double single = 0.35 + 320.0 / n, squarings = (log2p - 1) * (0.05 + 250.0 / n);
+    const double single = single_pass(n), squarings = (log2p - 1) * (0.05 + 250.0 / n);
     QuadraticSteps q;
     const double newton = (s.iters - 1) * (log2p + 2) +
                           single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
@@ -417,6 +503,27 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
       s.iters = 1;
       s.steps = newton_schedule(l0, p, 1, nullptr);
       s.l_last = l0;
+    }
+  }
+  const int first = steep_n >= kSteepFrom && iters <= 0 && !s.graded.products && p > 1 ? bound_below(l0) : kBounds;
+  if (first < kBounds) {
+    int log2p = 0;
+    while ((1 << log2p) < p) ++log2p;
+    const double single = single_pass(steep_n);
+    QuadraticSteps q;
+    const double linear = (s.iters - 1) * (log2p + 2) +
+                          single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
+    std::unordered_map<int, StepPlan> memo;
+    const StepPlan& plan = cheapest(p, first, single, memo);
+    if (!plan.path.empty() && plan.cost < linear - 0.3) {
+      s.steep = true;
+      s.steps.clear();
+      for (const auto& at : plan.path) s.steps.push_back(bound_node(p, at.first).step[at.second]);
+      const auto& end = plan.path.back();
+      s.l_last = s.steps.back().next;
+      s.fin = bound_node(p, end.first).fin[end.second];
+      s.iters = (int)s.steps.size() + 1;
+      s.steps.push_back(s.steps.back());   // (the finish multiplies by none of them)
     }
   }
   s.p = p;
@@ -512,15 +619,16 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 // that the single-pass squarings of the norm bound read).
 // With defl_v the input is A and the deflation A' = A + sum_j coef[j] v_j v_j^T is applied on the way (the terms of
 // rankr_update_kernel, in its order), so that A' is never written.
-// With m32 (the graded finish with no Newton step) M_0 is written there in FP32, and its planes -- the hi plane alone -- are
-// those of M_0 + m_diag I.
+// With m32 M_0 is written there in FP32 (the graded finish, steps with a term linear in M).  With hi_only (the graded finish) its
+// planes -- the hi plane alone -- are those of M_0 + m_diag I.
 __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restrict__ a32, int n, int batch,
                                                           const float* __restrict__ sumsq, float a, float b, float s_m,
                                                           float s_t, __half* __restrict__ m_planes,
                                                           __half* __restrict__ t_planes,
                                                           const float* __restrict__ defl_v,
                                                           const float* __restrict__ defl_coef, int defl_r,
-                                                          int vstride, float* __restrict__ m32 = nullptr, float m_diag = 0.f) {
+                                                          int vstride, float* __restrict__ m32 = nullptr, float m_diag = 0.f,
+                                                          bool hi_only = false) {
   ptx::pdl_begin();
   const int bi = blockIdx.y;
   float cf[8];
@@ -572,7 +680,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* __restric
       k[e] = __float2half_rn(t - __half2float(g[e]));
     }
     *reinterpret_cast<uint2*>(mh + i * 4) = *reinterpret_cast<uint2*>(h);
-    if (!m32) *reinterpret_cast<uint2*>(ml + i * 4) = *reinterpret_cast<uint2*>(l);
+    if (!hi_only) *reinterpret_cast<uint2*>(ml + i * 4) = *reinterpret_cast<uint2*>(l);
     *reinterpret_cast<uint2*>(th + i * 4) = *reinterpret_cast<uint2*>(g);
     *reinterpret_cast<uint2*>(tl + i * 4) = *reinterpret_cast<uint2*>(k);
   }
@@ -1485,22 +1593,28 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
 // rest_trace (a graded finish) e may have either sign, and the rounding of A's entries is allowed for as well: where one
 // eigenvalue theta_1 is far above the mean c of the rest, 2^-24 theta_1 |v_i v_j| of them, is 2^-24 theta_1 / (c sqrt(n)) of R
 // (a mean of 20 standard deviations, 1000 wide: 1e-4 to 3.5e-4 seen, 7.6e-4 allowed for).
-__global__ void verify_kernel(const float* __restrict__ e_est, const float* __restrict__ e_top, float e_allowed,
+__global__ void verify_kernel(const float* __restrict__ e_est, const float* __restrict__ e_top, float e_allowed, float e_below,
                               int* __restrict__ status, float* __restrict__ e_out, int k, const float* __restrict__ theta,
                               const float* __restrict__ rest_trace, int n) {
   ptx::pdl_begin();
   const bool both_signs = theta != nullptr;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
-  float e = both_signs ? fabsf(e_est[b]) : e_est[b];
+  // (an even T sends what lies above the norm above 1: R negative there, past what the finish was fitted to)
+  auto size = [&](float x) { return both_signs ? fabsf(x) : (x < -e_below ? 1.f - x : x); };
+  float e = size(e_est[b]);
   if (e_top && isfinite(e)) {   // (fmaxf would pass over a NaN)
-    const float t = both_signs ? fabsf(e_top[b]) : e_top[b];
+    const float t = size(e_top[b]);
     e = isfinite(t) ? fmaxf(e, t) : t;
   }
   if (e_out) e_out[b] = e;
   if (theta) e_allowed += 5.96e-8f * sqrtf((float)n) * theta[b * kMaxDeflate] / rest_trace[b];
   if (status && status[b] == 0 && (!isfinite(e) || e > e_allowed)) status[b] = 4;
 }
+
+// After steps of higher degree R may reach this far below zero: the finish is fitted to kFinishLow, and a Rayleigh quotient of
+// four power steps sits inside the spectrum.
+constexpr float kSteepBelow = 0.03f;
 
 // lmin[b] = theta^(-power): the smallest eigenvalue of A from the largest eigenvalue theta (a Rayleigh quotient, so a
 // lower estimate) of its computed inverse root A^(-1/power).
@@ -1518,9 +1632,12 @@ __global__ void lmin_from_root_kernel(const float* __restrict__ theta, float pow
 // Also the bound of the finished root's entries for its operand planes: a symmetric positive matrix has no entry above
 // its largest eigenvalue, and A >= damping I by construction, so |A^(-1/p)|_ij <= damping^(-1/p) -- known without a
 // pass over the result.
+// With `ritz` (steps of higher degree under an estimated norm: the Ritz values of A, the largest of which is finite only where A
+// is) a residual that is not finite is 2 only where A is not finite: T of degree four, raised to the p-th power, overflows where
+// the norm was far too low, as a linear T does not.
 __global__ void finish_kernel(const unsigned int* __restrict__ resid, const float* __restrict__ sumsq_a,
                               float* root_scale_lo, int* status, float* norm_out, int k, int p, float tol, float damping,
-                              float lower_used) {
+                              float lower_used, const float* __restrict__ ritz) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
@@ -1528,7 +1645,7 @@ __global__ void finish_kernel(const unsigned int* __restrict__ resid, const floa
   root_scale_lo[b] = powf(ub, -1.f / p);
   if (norm_out) norm_out[b] = ub;
   const float r = __uint_as_float(resid[b]);
-  int st = !isfinite(r) ? 2 : (r > tol ? 1 : 0);
+  int st = !isfinite(r) ? (ritz && isfinite(ritz[b * kMaxDeflate]) ? 1 : 2) : (r > tol ? 1 : 0);
   // lower_used < 0: the bound is an estimate, verified after the chain instead (verify_kernel)
   if (st == 0 && lower_used > 0.f && damping / ub < lower_used * 0.999f) st = 3;
   if (status) status[b] = st;
@@ -1645,6 +1762,32 @@ int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps
   return g.products;
 }
 
+int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, double* step_out, int32_t step_capacity, double* coef_out,
+                              int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out) {
+  if (!(lower > 0.f) || !(lower < 1.f) || p < 2 || (p & (p - 1)) || p > 32 || n <= 0) return 0;
+  const toner::Schedule& s = toner::schedule_for((double)lower, p, 0, 0, n);
+  if (!s.steep) return 0;
+  int log2p = 0, split = 0;
+  while ((1 << log2p) < p) ++log2p;
+  for (int k = 0; k < s.iters - 1; ++k) {
+    const toner::NewtonStep& st = s.steps[k];
+    split += log2p + 2 + (st.degree == 4 ? 2 : st.degree - 1);
+    if (!step_out || 7 * k + 6 >= step_capacity) continue;
+    const double out[7] = {(double)st.degree, st.zb, st.za, st.kappa, st.top, st.degree == 1 ? -st.b : st.lin, st.degree == 1 ? st.a : st.con};
+    for (int j = 0; j < 7; ++j) step_out[7 * k + j] = out[j];
+  }
+  toner::QuadraticSteps q;
+  if (coef_out)
+    for (int j = 0; j <= s.fin.order && j < coef_capacity; ++j) coef_out[j] = s.fin.c[j];
+  if (order_out) *order_out = s.fin.order;
+  if (products_out) {
+    products_out[0] = split + 1;
+    products_out[1] = toner::quadratic_steps(s.fin, p, q) ? (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 2;
+  }
+  if (e_out) *e_out = 1.0 - s.l_last;
+  return s.iters - 1;
+}
+
 int toner_factor_report(const int32_t* status, const float* norms, const float* lmin, const int32_t* deflated, int32_t k,
                         int32_t* host_out, void* stream) {
   using namespace toner;
@@ -1729,7 +1872,8 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
   // (verifying the estimate after a graded finish takes A^(-1/2) and the deflated vectors)
   const bool may_grade = estimated && iters <= 0 && (track_sweeps & 512) == 0 && p > 1 && 2 * q == p && defl_r > 0 &&
                          (reinterpret_cast<uintptr_t>(root_hi) & 15u) == 0;
-  const Schedule plan = schedule_for(l0, p, iters, may_grade ? n : 0);
+  // (steps of higher degree: other roundings, so not where the plane-by-plane order is asked for, nor where the count is)
+  const Schedule plan = schedule_for(l0, p, iters, may_grade ? n : 0, iters <= 0 && (track_sweeps & 512) == 0 ? n : 0);
   iters = plan.iters;
   const GradedPoly& graded = plan.graded;
   if (iters < 2 && !graded.products) return fail(kErrArg, "inv_roots: at least two iterations are required");
@@ -1860,19 +2004,22 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     const double top_gain = graded.products ? graded.beta[graded.products] * graded.za : 1.0;
     const double top_diag =
         graded.products ? (graded.alpha[graded.products] + graded.beta[graded.products] * graded.zb) / top_gain : 0.0;
-    float* const m32 = graded_finish ? reinterpret_cast<float*>(Xb[0]) : nullptr;
+    const bool first_z = graded_finish || sched[0].degree > 1;   // planes of Z instead of T_0's
+    float* const m32 = graded_finish || sched[0].lin != 0.0 ? reinterpret_cast<float*>(Xb[0]) : nullptr;   // M_0
+    __half* const first_planes = first_z && !graded_finish ? Tb[0] : Xb[1];
     const float s_z = plane_scale(1.2), s_top = plane_scale(1.1 * (1.0 + std::fabs(top_diag)));
-    const float init_a = graded_finish ? (float)graded.zb : (float)sched[0].a, init_b = graded_finish ? (float)-graded.za : (float)sched[0].b;
+    const float init_a = (float)(graded_finish ? graded.zb : first_z ? sched[0].zb : sched[0].a);
+    const float init_b = (float)(graded_finish ? -graded.za : first_z ? -sched[0].za : sched[0].b);
     const float init_sm = graded_finish ? s_top : s_m, init_diag = graded_finish ? (float)top_diag : 0.f;
-    float s_t = graded_finish ? s_z : plane_scale(sched[0].a);
+    float s_t = first_z ? s_z : plane_scale(sched[0].a);
     if (ritz_norm) {
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], Xb[1], dv, coef8, defl_r, kMaxDeflate, m32, init_diag);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, kMaxDeflate, m32, init_diag, graded_finish);
       TONER_CUDA(cudaGetLastError());
     } else {
-    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f);
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false);
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -1914,7 +2061,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
       TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], Xb[1], nullptr, nullptr, 0, 0, m32, init_diag);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, nullptr, nullptr, 0, 0, m32, init_diag, graded_finish);
       TONER_CUDA(cudaGetLastError());
     }
     }
@@ -1936,6 +2083,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       const float* beta_v = nullptr;               // per-statistic factors of beta
       double gain = 1.0;
       int segs = 3;                                // 1: hi planes only (a single pass)
+      bool upper_d = false;                        // d is read as a product's C alone, which takes its upper triangle
     };
     // (in_step: matrices between the hi and lo planes of the operands; 0: the chunk's)
     auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote, int in_step = 0) -> int {
@@ -1953,7 +2101,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g.c = o.c; g.ldc = n; g.c_bs = nn; g.beta = o.beta; g.beta_v = o.beta_v;
       g.alpha_a = o.alpha_a;
       g.alpha_b = o.alpha_b;
-      g.d = o.d; g.ldd = n; g.d_bs = nn;
+      g.d = o.d; g.ldd = n; g.d_bs = nn; g.upper_d = o.upper_d ? 1 : 0;
       g.split0 = o.s0; g.split0_scale = o.s0_scale; g.split0_aff_a = o.s0_a;
       g.split1 = o.s1; g.split1_scale = o.s1_scale; g.split1_aff_a = o.s1_a; g.split1_aff_b = o.s1_b;
       g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)(o.lo_step ? o.lo_step : kc) * nn;
@@ -1973,7 +2121,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     const float s_hi = root_plane_scale(1.01 * std::pow((double)damping, -(double)q / p));
     // X_1 = T_0, read by both chains until the first product with X; the next T goes to T's own buffer
     const __half* Xcur = Xb[1];
-    const __half* Tcur = Xb[1];
+    const __half* Tcur = first_planes;   // (before a step of higher degree has formed T, planes of Z)
     float s_x = s_t;
     double x_bound = sched[0].a;
     int xi = 0, mi = 0, ti = 1;   // ti: which T buffer was written last
@@ -1982,6 +2130,36 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float root_diag = 0.f;
     for (int it = 0; it < iters; ++it) {
       const bool last = (it == iters - 1);
+      if (!last && sched[it].degree > 1) {
+        // T from planes of Z (Tcur), see root_steps.cuh: its square, of degree four the square of that, shifted.  T_0 is X_1 as well.
+        // The errors of these products matter as those of the powers of T do.
+        const NewtonStep& st = sched[it];
+        const int chain = steep_chain_length(st.lower);
+        const __half* from = Tcur;
+        float s_from = s_t;
+        if (st.degree == 4) {
+          Out y;
+          y.s0 = Pb[1]; y.s0_scale = plane_scale(1.1 + std::fabs(st.kappa));
+          y.s0_a = (float)st.kappa;
+          rc = sym_product(from, s_from, from, s_from, y, chain);
+          if (rc) return rc;
+          from = y.s0;
+          s_from = y.s0_scale;
+        }
+        Out t;
+        t.gain = st.top;
+        t.s0 = it == 0 ? Xb[1] : (st.degree == 4 ? Tb[0] : Pb[1]);
+        t.s0_scale = plane_scale(st.a);
+        t.s0_a = (float)st.con;
+        if (st.lin != 0.0) {
+          t.c = it == 0 ? m32 : A32; t.beta = (float)st.lin;
+        }
+        rc = sym_product(from, s_from, from, s_from, t, chain);
+        if (rc) return rc;
+        Tcur = t.s0;
+        s_t = t.s0_scale;
+        if (it == 0) s_x = s_t;
+      }
       if (it > 0 || last) {
         x_bound = std::min(x_bound * sched[it].a, x_cap);
         if (last) {
@@ -1999,7 +2177,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             if (rc) return rc;
           }
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : 0.5f, damping, lower_used);
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : (plan.steep ? 0.65f : 0.5f), damping, lower_used, plan.steep && ritz_norm ? th8 : nullptr);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
@@ -2045,7 +2223,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             auto scale = [&](double bound) { return left == 0 ? s_f : plane_scale(std::max(1.0, bound)); };
             double bound = std::fabs(fast.top) * (1.0 + std::fabs(fast.beta)) + std::fabs(fast.top0);
             Out y;
-            y.segs = 1;
+            y.segs = plan.steep && left == 0 ? 3 : 1;
             y.gain = -1.0;
             y.s0 = Yp; y.s0_scale = s_y;
             y.s1 = target(); y.s1_scale = scale(bound);
@@ -2058,7 +2236,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
               --left;
               bound = (1.0 + std::fabs(fast.beta)) * bound + std::fabs(linear) + std::fabs(constant);
               Out w;
-              w.segs = 1;
+              w.segs = plan.steep && left == 0 ? 3 : 1;
               if (linear != 0.0) {
                 w.c = A32; w.beta = (float)-linear;
               }
@@ -2085,7 +2263,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             for (int j = order - 1; j >= 1; --j) {
               const double aj = fin.c[j];
               Out w;
-              w.segs = 1;
+              w.segs = plan.steep && j == 1 ? 3 : 1;
               w.gain = gain;
               w.c = A32; w.beta = (float)-aj;
               w.s1 = Mb[j & 1];
@@ -2103,7 +2281,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             Out o;
             o.d = R;
             o.alpha_a = scale_lo;
-            rc = sym_product(Xcur, s_x, Mb[1], s_f, o, kPromoteX);
+            rc = sym_product(Xcur, s_x, Mb[1], s_f, o, plan.steep ? kPromoteSteepX : kPromoteX);
             if (rc) return rc;
           }
           // put the deflated directions back: A^{-1/p} = A'^{-1/p} + (lambda_1^{-1/p} - c^{-1/p}) v v^T; with that the root's
@@ -2124,7 +2302,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         Out o;
         o.s0 = Xb[xi];
         o.s0_scale = plane_scale(x_bound);
-        rc = sym_product(Xcur, s_x, Tcur, s_t, o, kPromoteX);
+        rc = sym_product(Xcur, s_x, Tcur, s_t, o, plan.steep ? kPromoteSteepX : kPromoteX);
         if (rc) return rc;
         Xcur = Xb[xi];
         s_x = o.s0_scale;
@@ -2134,7 +2312,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       // grows with the length of the accumulation chain and, unlike rounding noise, does not average out over
       // the sum; a relative error e of M matters as e / (smallest eigenvalue of M), so the chains are kept
       // short while the spectrum's lower bound is small and lengthened as it approaches 1.
-      const int chain = chain_length(sched[it].lower);
+      const int chain = plan.steep ? steep_chain_length(sched[it].lower) : chain_length(sched[it].lower);
       const __half* pw = Tcur;
       float s_pw = s_t;
       double pw_bound = sched[it].a;
@@ -2168,9 +2346,19 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         } else {
           o.s0 = Mb[mi ^ 1];
           o.s0_scale = s_m;
-          o.s1_scale = plane_scale(na);
-          o.s1_a = na;
-          o.s1_b = -nb;
+          if (sched[it + 1].degree > 1) {   // planes of the next Z, and M in FP32 where T has a term linear in it
+            if (sched[it + 1].lin != 0.0) {
+              o.d = A32;
+              o.upper_d = true;
+            }
+            o.s1_scale = s_z;
+            o.s1_a = (float)sched[it + 1].zb;
+            o.s1_b = (float)sched[it + 1].za;
+          } else {
+            o.s1_scale = plane_scale(na);
+            o.s1_a = na;
+            o.s1_b = -nb;
+          }
         }
         rc = sym_product(pw, s_pw, Mb[mi], s_m, o, chain);
         if (rc) return rc;
@@ -2212,7 +2400,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         // Newton chain's.  A^(-1/p) from a graded finish is ten times closer than that; two squarings in chains of two k-blocks
         // leave 3.5e-6 of A^(-1/2) whatever the width, of one k-block 2e-6, in the same time: 24 statistics of 2048, condition 2
         // and 5, 5570 and 6125 / 5620 and 6080 us a call.)
-        rc = sym_product(Xcur, s_x, Xcur, s_x, o, graded_finish ? 1 : kPromoteX, first ? root_step : 0);
+        rc = sym_product(Xcur, s_x, Xcur, s_x, o, graded_finish ? 1 : plan.steep ? kPromoteSteepSquares : kPromoteX, first ? root_step : 0);
         if (rc) return rc;
         Xcur = Pb[pi];
         s_x = o.s0_scale;
@@ -2264,7 +2452,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             TONER_LAUNCH(power_shift_kernel, kc, 256, stream, pv, py, n, e_est, 1, 0, nullptr, nullptr, 0, 0);
           }
         }
-        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm || graded_finish ? e_top : nullptr, graded_finish ? (float)(kGradedResidual + p * kGradedTail) : (float)(1.15 * (1.0 - l_last) + 1e-3), status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc, graded_finish ? th8 : nullptr, rest_trace, n);
+        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm || graded_finish ? e_top : nullptr, graded_finish ? (float)(kGradedResidual + p * kGradedTail) : (float)(1.15 * (1.0 - l_last) + 1e-3), plan.steep ? kSteepBelow : INFINITY, status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc, graded_finish ? th8 : nullptr, rest_trace, n);
         TONER_CUDA(cudaGetLastError());
       }
       const int sweeps = track_sweeps & 63;

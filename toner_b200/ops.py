@@ -331,7 +331,7 @@ def inv_roots_finish_products(n: int, damping: float, p: int, lower: float = 0.0
 
 
 def inv_roots_schedule(lower: float, p: int, iters: int = 0) -> dict:
-    """The whole schedule the engine runs for a spectrum lower bound (toner_inv_roots_schedule; needs no device):
+    """The whole schedule of linear steps for a spectrum lower bound (toner_inv_roots_schedule; needs no device):
     {"iterations", "steps": [(a_k, b_k), ...], "coefficients": [c_0, ...] of the finishing polynomial in powers of
     r = 1 - mu, "distance": e}."""
     ab = (C.c_double * 128)()
@@ -342,6 +342,19 @@ def inv_roots_schedule(lower: float, p: int, iters: int = 0) -> dict:
         raise ValueError("inv_roots_schedule: lower must lie inside (0, 1), p >= 1, iters 0 or >= 2")
     return {"iterations": count, "steps": [(ab[2 * k], ab[2 * k + 1]) for k in range(count - 1)],
             "coefficients": [coef[j] for j in range(order.value + 1)], "distance": e.value}
+
+
+def inv_roots_steps(lower: float, p: int, n: int) -> Optional[dict]:
+    """The schedule of a call on statistics of width n that takes steps of higher degree (toner_inv_roots_steps_for; needs no
+    device): {"steps": [(degree, zb, za, kappa, top, lin, con)], "coefficients": of the finishing polynomial, "distance": e,
+    "products": (split, single passes)}; None where linear steps are used."""
+    steps, coef = (C.c_double * 128)(), (C.c_double * 16)()
+    order, products, e = C.c_int32(0), (C.c_int32 * 2)(), C.c_double(0.0)
+    count = _lib.load().toner_inv_roots_steps_for(lower, p, n, steps, 128, coef, 16, C.byref(order), products, C.byref(e))
+    if count <= 0:
+        return None
+    return {"steps": [(int(steps[7 * k]), *steps[7 * k + 1:7 * k + 7]) for k in range(count)],
+            "coefficients": coef[:order.value + 1], "distance": e.value, "products": (products[0], products[1])}
 
 
 def inv_roots_graded(lower: float, p: int, n: int) -> Optional[dict]:
