@@ -268,9 +268,12 @@ int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps
  * more at degree 4, p = 8).  Returns their number (0: the schedule of toner_inv_roots_schedule is used) and writes seven doubles
  * a step (degree, zb, za, kappa, top, lin, con: with z = zb + za mu, T is con + lin mu plus nothing, top z^2 or
  * top (z^2 + kappa)^2), the finishing polynomial and the distance e as toner_inv_roots_schedule does, and products_out[0], [1]: the split and the single-pass
- * products that steps and finish take.  Every output pointer is optional; needs no device. */
-int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, double* step_out, int32_t step_capacity, double* coef_out,
-                              int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out);
+ * products that steps and finish take.  kind: the bound is an estimate (0), certified (1), the one that always holds (2).  late_out > 0 (kind
+ * 2): a statistic whose norm, on the device, puts its spectrum above this starts with the second step.  Every output pointer is
+ * optional; needs no device. */
+int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, int32_t kind, double* step_out, int32_t step_capacity,
+                              double* coef_out, int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out,
+                              double* late_out);
 int toner_inv_roots(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
                     float* root_lo, float* root_hi, float* fro2_lo, int32_t* status, void* workspace,
                     size_t workspace_bytes, void* stream);

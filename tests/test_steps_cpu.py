@@ -4,33 +4,56 @@ import numpy as np
 import pytest
 
 
+def _take(s, lam, steps, p):
+    """Scalars lam through these steps of schedule s and its finish."""
+    x, mu = np.ones_like(lam), lam.copy()
+    for degree, zb, za, kappa, top, lin, con in steps:
+        z = zb + za * mu
+        t = con + lin * mu + top * {1: 0.0, 2: z ** 2, 4: (z ** 2 + kappa) ** 2}[degree]
+        assert t.min() > 0 and (t.max() / t.min()) ** p < 1.05e3
+        x, mu = x * t, mu * t ** p
+        assert mu.max() < 1.0 + 1e-6, (p, lam[0], mu.max())
+    assert 1.0 - mu.min() <= s["distance"] + 1e-9, (p, lam[0])
+    q = np.polyval(np.array(s["coefficients"])[::-1], 1.0 - mu)
+    assert np.abs(x * q * lam ** (1.0 / p) - 1.0).max() < 5e-6, (p, lam[0])
+
+
+@pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("n", [264, 768, 3072])
 @pytest.mark.parametrize("p", [2, 4, 8, 16, 32])
-def test_the_stated_steps_take_every_eigenvalue_to_its_root(p, n):
+def test_the_stated_steps_take_every_eigenvalue_to_its_root(p, n, kind):
     """x = 1, mu = lambda; t = T(mu), x *= t, mu *= t^p per step; then x q(1 - mu) must be lambda^(-1/p) for every lambda the
     bound allows.  mu stays at 1 or below, ends within the stated distance of 1, T^p
     keeps the dynamic range its operand planes resolve (1e3, the grid's miss beside it), and products are saved."""
     from toner_b200 import ops
     used = 0
     for lower in np.geomspace(1.5e-7, 0.3, 60):
-        s = ops.inv_roots_steps(float(lower), p, n)
+        s = ops.inv_roots_steps(float(lower), p, n, kind)
         if s is None:
             continue
         used += 1
+        assert s["late"] == 0.0
         lam = np.unique(np.concatenate([np.geomspace(float(np.float32(lower)), 1.0, 4001), np.linspace(float(np.float32(lower)), 1.0, 4001)]))
-        x, mu = np.ones_like(lam), lam.copy()
-        for degree, zb, za, kappa, top, lin, con in s["steps"]:
-            z = zb + za * mu
-            t = con + lin * mu + top * {1: 0.0, 2: z ** 2, 4: (z ** 2 + kappa) ** 2}[degree]
-            assert t.min() > 0 and (t.max() / t.min()) ** p < 1.05e3
-            x, mu = x * t, mu * t ** p
-            assert mu.max() < 1.0 + 1e-6, (p, lower, mu.max())
-        assert 1.0 - mu.min() <= s["distance"] + 1e-9, (p, lower)
-        q = np.polyval(np.array(s["coefficients"])[::-1], 1.0 - mu)
-        assert np.abs(x * q * lam ** (1.0 / p) - 1.0).max() < 5e-6, (p, lower)
+        _take(s, lam, s["steps"], p)
         # fewer products than the linear steps for the same bound, single passes by what they take
         linear = (ops.inv_roots_iterations_for(float(lower), p) - 1) * (p.bit_length() + 1)
         single = ops.inv_roots_finish_products(n, 1e-3, p, float(lower))
         weight = 0.35 + 320.0 / n
         assert s["products"][0] + weight * s["products"][1] < linear + weight * single
     assert used >= 30, used
+
+
+@pytest.mark.parametrize("n", [256, 512, 776, 2048, 5632, 16384])
+@pytest.mark.parametrize("p", [2, 4, 8, 16, 32])
+def test_the_bound_that_always_holds_with_and_without_its_first_step(p, n):
+    """All steps for a spectrum down to damping / n, the steps from the second on for one down to the stated bound, which a norm of
+    16 puts every spectrum above where one step of degree four gets that far."""
+    from toner_b200 import ops
+    worst = 1e-3 / (n * 1.001)
+    s = ops.inv_roots_steps(worst, p, n, 2)
+    lam = lambda low: np.unique(np.concatenate([np.geomspace(low, 1.0, 4001), np.linspace(low, 1.0, 4001)]))
+    _take(s, lam(float(np.float32(worst))), s["steps"], p)
+    if s["late"]:
+        assert s["steps"][1][0] > 1 and s["late"] <= 1e-3 / 16
+        _take(s, lam(s["late"]), s["steps"][1:], p)
+    assert s["late"] > 0 or p not in (4, 8) or n == 16384     # (not where the second step would be a linear one)

@@ -93,3 +93,38 @@ def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops):
             assert float((lo.double() - want).norm() / want.norm()) < 2e-5
         else:
             assert all(s in (1, 4) or x <= 1.08 for s, x in zip(st.tolist(), reach)), (st.tolist(), reach)
+
+
+@pytest.mark.parametrize("p,q", [(4, 1), (8, 4)])
+@pytest.mark.parametrize("n", [264, 1032])
+def test_a_first_step_left_out_by_some_statistics(ops, p, q, n):
+    """The bound that always holds: statistics of a small norm start with the second step, those of a large one (two directions of one
+    size, which are not deflated) with the first.  Each comes out as beside others of its kind, and as close to FP64 as linear steps
+    bring it."""
+    small = _statistics(n, 300.0)
+    spikes = _statistics(n, 30.0, 1)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    d, _ = torch.linalg.qr(torch.randn(n, 2, device="cuda", generator=g))
+    spikes = spikes + (d @ d.T) * spikes.diagonal(dim1=1, dim2=2).sum(1)[:, None, None]
+    stats = torch.cat([small[:1], spikes, small[1:]]).contiguous()
+    late = ops.inv_roots_steps(DAMPING / (n * 1.001), p, n, 2)["late"]
+    norms = torch.zeros(3, device="cuda")
+    lo, hi, _, st = ops.inv_roots(stats, DAMPING, p, q, norms=norms)
+    ops.assert_healthy()
+    assert st.tolist() == [0, 0, 0]
+    starts_late = [DAMPING / x > late for x in norms.tolist()]
+    assert late > 0 and starts_late == [True, False, True], (late, norms.tolist())
+    a = stats.double()
+    a = a / a.diagonal(dim1=1, dim2=2).mean(1)[:, None, None] + DAMPING * torch.eye(n, device="cuda", dtype=torch.float64)
+    lam, vec = torch.linalg.eigh(a)
+    linear = ops.inv_roots(stats, DAMPING, p, q, interleave=False)
+    for root, plain, s in ((lo, linear[0], 1.0 / p), (hi, linear[1], q / p)):
+        if root is None:
+            continue
+        want = (vec * lam.pow(-s)[:, None, :]) @ vec.mT
+        got, ref = [(x.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1) for x in (root, plain)]
+        # (the middle one's spectrum starts at 3e-6, below 2^-22 of T^p's range of 1e3: up to 1.4 times the linear steps' error)
+        assert (got <= torch.tensor([1.2, 1.6, 1.2], device="cuda") * ref + 1e-6 * q).all(), (got.tolist(), ref.tolist())
+    for b in range(3):
+        own = ops.inv_roots(stats[b:b + 1].expand(3, n, n).contiguous(), DAMPING, p, q)     # (of one tile choice: three as well)
+        assert torch.equal(own[0][b], lo[b]) and (hi is None or torch.equal(own[1][b], hi[b]))

@@ -242,7 +242,9 @@ class FactorSet:
         ones; None where it took those, or the graded finish."""
         if self.k == 0 or not self._ran or not self.interleave or self.graded:
             return None
-        return ops.inv_roots_steps(max(self._lower_used, self.damping / (self.n * (1.0 + self.damping))), self.p, self.n)
+        worst = self.damping / (self.n * (1.0 + self.damping))
+        kind = 2 if self._lower_used <= worst else (0 if self._used_estimate else 1)
+        return ops.inv_roots_steps(max(self._lower_used, worst), self.p, self.n, kind)
 
     @property
     def iterations(self) -> int:

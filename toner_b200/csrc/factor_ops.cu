@@ -219,10 +219,10 @@ static bool finish_usable(const FinishPoly& f, double hi) {
   return true;
 }
 
-static FinishPoly finish_poly(int p, double e) {
+static FinishPoly finish_poly(int p, double e, double grow = kFinishGrow, double radius = kFinishRadius) {
   FinishPoly f;
-  if (!(e < kFinishRadius)) return f;
-  const double hi = kFinishGrow * e + kFinishPad;
+  if (!(e < radius)) return f;
+  const double hi = grow * e + kFinishPad;
   FitSamples samples;
   for (int m = 2; m <= kMaxFinishOrder; ++m) {
     if (finish_fit(p, kFinishLow, hi, m, kFinishTail, samples, f.c)) {
@@ -389,12 +389,15 @@ static double single_pass(int n) { return 0.35 + 320.0 / n; }
 // The last product of the finish is a split one: single passes lose 2^-12 e^2 of it, which linear steps' own errors cover and these
 // would not (p = 8, e = 0.59: A^(-1/2) 2.5 times as far off as after linear steps without, 0.94 times with it).
 constexpr int kBoundsPerOctave = 8, kBounds = 32 * kBoundsPerOctave;
+// A certified bound needs no margin for an estimate's allowance, only for rounding (M_0's planes resolve 2^-25: 4e-4 of the smallest
+// eigenvalue at a norm of 16, damping 1e-3), and so may end further from I.
+constexpr double kCertifiedGrow = 1.04, kCertifiedRadius = 0.66;
 constexpr int kSteepFrom = 256;   // columns: on narrower statistics linear steps can be closer (by 2.8 times, of 8e-7, 8 wide)
 struct BoundNode {
   bool ok[3] = {};
   NewtonStep step[3];
-  FinishPoly fin[3];       // after that step; order 0: M is too far from I
-  int fin_products[3] = {};
+  FinishPoly fin[2][3];       // after that step, under an estimated and a certified bound; order 0: M is too far from I
+  int fin_products[2][3] = {};
 };
 static double bound_of(int j) { return std::exp2(-(double)j / kBoundsPerOctave); }
 static int bound_below(double l) { return std::max(1, (int)std::ceil(-kBoundsPerOctave * std::log2(l) - 1e-6)); }
@@ -407,10 +410,12 @@ static const BoundNode& bound_node(int p, int j) {
   for (int i = 0; i < 3; ++i) {
     node.ok[i] = best_step(p, bound_of(j), kStepDegrees[i], kMaxPowerRange, node.step[i]);
     if (!node.ok[i]) continue;
-    node.fin[i] = finish_poly(p, 1.0 - node.step[i].next);
-    QuadraticSteps q;
-    if (node.fin[i].order)
-      node.fin_products[i] = quadratic_steps(node.fin[i], p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : node.fin[i].order - 1;
+    for (int c = 0; c < 2; ++c) {
+      FinishPoly& fin = node.fin[c][i];
+      fin = c ? finish_poly(p, 1.0 - node.step[i].next, kCertifiedGrow, kCertifiedRadius) : finish_poly(p, 1.0 - node.step[i].next);
+      QuadraticSteps q;
+      if (fin.order) node.fin_products[c][i] = quadratic_steps(fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : fin.order - 1;
+    }
   }
   return node;
 }
@@ -419,8 +424,10 @@ struct StepPlan {
   double cost = 1e9;                // in split products, the finish and its product with X counted
   std::vector<std::pair<int, int>> path;   // (bound, degree's index)
 };
+// T's own products; with a linear term it writes and reads an FP32 matrix more
+static double own_products(const NewtonStep& s) { return (s.degree == 4 ? 2 : s.degree - 1) + (s.lin != 0.0 ? 0.25 : 0.0); }
 // Cheapest steps from bound j on; `memo` is the call's own.
-static const StepPlan& cheapest(int p, int j, double single, std::unordered_map<int, StepPlan>& memo) {
+static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo) {
   const auto found = memo.find(j);
   if (found != memo.end()) return found->second;
   StepPlan best;
@@ -429,16 +436,15 @@ static const StepPlan& cheapest(int p, int j, double single, std::unordered_map<
   while ((1 << log2p) < p) ++log2p;
   for (int i = 2; i >= 0; --i) {
     if (!node.ok[i]) continue;
-    // powers, M, the next product with X, and T's own: with a linear term it writes and reads an FP32 matrix more
-    const double own = log2p + 2 + (kStepDegrees[i] == 4 ? 2 : kStepDegrees[i] - 1) + (node.step[i].lin != 0.0 ? 0.25 : 0.0);
-    const double end = single * (node.fin_products[i] - 1) + 1.0;
-    if (node.fin[i].order && own + end < best.cost) {
+    const double own = log2p + 2 + own_products(node.step[i]);   // (powers, M, the next product with X)
+    const double end = single * (node.fin_products[certified][i] - 1) + 1.0;
+    if (node.fin[certified][i].order && own + end < best.cost) {
       best.cost = own + end;
       best.path = {{j, i}};
     }
     const int next = bound_below(node.step[i].next);
     if (next >= j || node.step[i].next > 0.9 || own + log2p + 2 >= best.cost) continue;
-    const StepPlan& rest = cheapest(p, next, single, memo);
+    const StepPlan& rest = cheapest(p, next, certified, single, memo);
     if (own + rest.cost < best.cost) {
       best.cost = own + rest.cost;
       best.path = {{j, i}};
@@ -456,7 +462,9 @@ struct Schedule {
   int p = 0, asked = 0;   // asked: the caller's step count, 0 = the one with the fewest plane passes; -n: graded
                           // finishes considered as well, for statistics of width n
   int steep_n = 0;        // > 0: steps of higher degree considered as well, for statistics of that width
+  int kind = 0;           // for these: the bound is an estimate (0), certified (1), the one that always holds (2)
   bool steep = false;     // ... and taken: cheaper than linear ones
+  double late = 0.0;      // > 0: a statistic whose spectrum is above this starts with the second step
   int iters = 0;
   std::vector<NewtonStep> steps;
   double l_last = 0.0;    // lower bound of the spectrum of the last M, i.e. after iters - 1 updates
@@ -464,20 +472,23 @@ struct Schedule {
   GradedPoly graded;      // graded.products > 0: this finish, of M_0 itself (iters == 1)
 };
 
-static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0, int steep_n = 0) {
+static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0, int steep_n = 0,
+                                    int kind = 0) {
   constexpr int kKept = 8;
   static thread_local Schedule kept[kKept];
   static thread_local int oldest = 0;
   iters = iters > 0 ? iters : -grade_n;
   for (const Schedule& s : kept)
-    if (s.p == p && s.l0 == l0 && s.asked == iters && s.steep_n == steep_n) return s;
+    if (s.p == p && s.l0 == l0 && s.asked == iters && s.steep_n == steep_n && s.kind == kind) return s;
   Schedule& s = kept[oldest];
   oldest = (oldest + 1) % kKept;
   s.p = 0;   // (not a match until it is complete)
   s.l0 = l0;
   s.asked = iters;
   s.steep_n = steep_n;
+  s.kind = kind;
   s.steep = false;
+  s.late = 0.0;
   s.iters = iters > 0 ? iters : default_iterations(l0, p);
   if (s.iters >= 2) {
     s.steps = newton_schedule(l0, p, s.iters, nullptr);
@@ -514,14 +525,36 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
     const double linear = (s.iters - 1) * (log2p + 2) +
                           single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
     std::unordered_map<int, StepPlan> memo;
-    const StepPlan& plan = cheapest(p, first, single, memo);
-    if (!plan.path.empty() && plan.cost < linear - 0.3) {
+    StepPlan plan = cheapest(p, first, kind > 0, single, memo);
+    if (kind == 2) {
+      // The bound that always holds, damping / n, is a norm of n; statistics have one of 5 to 15, which the device knows before the
+      // first product.  So the first step goes from this bound to that of a norm of 16, damping / 16, or as far as it gets, and is
+      // left out for every statistic whose norm allows it; the others follow as they would from there.
+      const BoundNode& node = bound_node(p, first);
+      const int norm16 = bound_below(l0 * steep_n / 16.0);
+      for (int i = 1; i < 3 && norm16 < first - 2 * kBoundsPerOctave; ++i) {
+        if (!node.ok[i]) continue;
+        const int from = std::max(norm16, bound_below(node.step[i].next));
+        if (from > norm16 && i < 2) continue;   // (degree four gets further)
+        const StepPlan& rest = cheapest(p, from, true, single, memo);
+        if (rest.path.empty() || rest.path[0].second == 0) break;   // (a first T of degree one is no product's result)
+        const double all = log2p + 2 + own_products(node.step[i]) + rest.cost;
+        if (rest.cost < 0.9 * plan.cost && all < linear) {
+          s.late = bound_of(from);
+          plan.cost = all;
+          plan.path = {{first, i}};
+          plan.path.insert(plan.path.end(), rest.path.begin(), rest.path.end());
+        }
+        break;
+      }
+    }
+    if (!plan.path.empty() && (s.late > 0.0 || plan.cost < linear - 0.3)) {
       s.steep = true;
       s.steps.clear();
       for (const auto& at : plan.path) s.steps.push_back(bound_node(p, at.first).step[at.second]);
       const auto& end = plan.path.back();
       s.l_last = s.steps.back().next;
-      s.fin = bound_node(p, end.first).fin[end.second];
+      s.fin = bound_node(p, end.first).fin[kind > 0][end.second];
       s.iters = (int)s.steps.size() + 1;
       s.steps.push_back(s.steps.back());   // (the finish multiplies by none of them)
     }
@@ -621,16 +654,30 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 // rankr_update_kernel, in its order), so that A' is never written.
 // With m32 M_0 is written there in FP32 (the graded finish, steps with a term linear in M).  With hi_only (the graded finish) its
 // planes -- the hi plane alone -- are those of M_0 + m_diag I.
-__global__ void __launch_bounds__(256) init_planes_kernel(const float* __restrict__ a32, int n, int batch,
+// late (per statistic, optional): where it is not zero the iteration starts with the second step, whose operands l gives.
+struct InitLate {
+  float a, b;
+  __half* m_planes;
+  __half* t_planes;
+  float* m32;
+};
+__global__ void __launch_bounds__(256) init_planes_kernel(const float* a32, int n, int batch,
                                                           const float* __restrict__ sumsq, float a, float b, float s_m,
                                                           float s_t, __half* __restrict__ m_planes,
                                                           __half* __restrict__ t_planes,
                                                           const float* __restrict__ defl_v,
                                                           const float* __restrict__ defl_coef, int defl_r,
-                                                          int vstride, float* __restrict__ m32 = nullptr, float m_diag = 0.f,
-                                                          bool hi_only = false) {
+                                                          int vstride, float* m32, float m_diag, bool hi_only,
+                                                          const int* __restrict__ late, InitLate second) {
   ptx::pdl_begin();
   const int bi = blockIdx.y;
+  if (late && late[bi]) {   // (second.m32 may be a32 itself: every element is read before it is written, by one thread)
+    a = second.a;
+    b = second.b;
+    m_planes = second.m_planes;
+    t_planes = second.t_planes;
+    m32 = second.m32;
+  }
   float cf[8];
   bool any = false;
 #pragma unroll
@@ -1505,8 +1552,9 @@ __global__ void __launch_bounds__(32) root_norm_kernel(const float* __restrict__
 // With P = A' / ||A'||_F:  lambda_max(P) <= ||P^(2^j)||_F^(1 / 2^j) = (sum lambda^(2^(j+1)))^(1 / 2^(j+1))  for every j, and
 // the bound tightens with j (for a flat spectrum it is n^(-1/2) times n^(1/4), n^(1/8), n^(1/16) for j = 1, 2, 3).
 // bound^2 <- bound^2 * t^2 with t the smallest of the three, 3 % above it for the single-pass products' rounding.
+// late (optional): 1 where the norm puts the spectrum's lower end, damping / norm at least, above late_from.
 __global__ void tighten_bound_kernel(float* __restrict__ bound2, const float* __restrict__ ss2, const float* __restrict__ ss4,
-                                     const float* __restrict__ ss8, int k) {
+                                     const float* __restrict__ ss8, int k, int* __restrict__ late, float late_from, float damping) {
   ptx::pdl_begin();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= k) return;
@@ -1522,6 +1570,7 @@ __global__ void tighten_bound_kernel(float* __restrict__ bound2, const float* __
     if (isfinite(t8) && t8 > 0.f) t = fminf(t, 1.03f * t8);
   }
   if (t < 1.f) bound2[b] *= t * t;
+  if (late) late[b] = damping > late_from * sqrtf(bound2[b]) ? 1 : 0;   // (not for a NaN)
 }
 
 // x <- x - sum_i (v_i . x) v_i over the deflated directions v_i of one statistic (coef[i] != 0).  By a block of 256 threads.
@@ -1672,10 +1721,10 @@ static size_t per_statistic_bytes(int n) {
   return align_up((size_t)n * n * 4, 256) * 8;
 }
 static size_t small_bytes(int chunk, int n) {
-  // nineteen per-statistic scalars, four blocks of eight scalars per statistic (Ritz values, residuals, deflation
+  // twenty per-statistic scalars, four blocks of eight scalars per statistic (Ritz values, residuals, deflation
   // coefficients, root corrections), the reduction scratch, and two blocks of eight n-vectors per statistic
   // (block power iteration: V and A V)
-  return align_up((size_t)chunk * 4, 256) * 19 + 4 * align_up((size_t)chunk * 32, 256) +
+  return align_up((size_t)chunk * 4, 256) * 20 + 4 * align_up((size_t)chunk * 32, 256) +
          align_up(sumsq_scratch_bytes(chunk), 256) + 2 * align_up((size_t)chunk * 8 * n * 4, 256);
 }
 
@@ -1762,11 +1811,13 @@ int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps
   return g.products;
 }
 
-int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, double* step_out, int32_t step_capacity, double* coef_out,
-                              int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out) {
-  if (!(lower > 0.f) || !(lower < 1.f) || p < 2 || (p & (p - 1)) || p > 32 || n <= 0) return 0;
-  const toner::Schedule& s = toner::schedule_for((double)lower, p, 0, 0, n);
+int toner_inv_roots_steps_for(float lower, int32_t p, int32_t n, int32_t kind, double* step_out, int32_t step_capacity,
+                              double* coef_out, int32_t coef_capacity, int32_t* order_out, int32_t* products_out, double* e_out,
+                              double* late_out) {
+  if (!(lower > 0.f) || !(lower < 1.f) || p < 2 || (p & (p - 1)) || p > 32 || n <= 0 || kind < 0 || kind > 2) return 0;
+  const toner::Schedule& s = toner::schedule_for((double)lower, p, 0, 0, n, kind);
   if (!s.steep) return 0;
+  if (late_out) *late_out = s.late;
   int log2p = 0, split = 0;
   while ((1 << log2p) < p) ++log2p;
   for (int k = 0; k < s.iters - 1; ++k) {
@@ -1873,7 +1924,8 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
   const bool may_grade = estimated && iters <= 0 && (track_sweeps & 512) == 0 && p > 1 && 2 * q == p && defl_r > 0 &&
                          (reinterpret_cast<uintptr_t>(root_hi) & 15u) == 0;
   // (steps of higher degree: other roundings, so not where the plane-by-plane order is asked for, nor where the count is)
-  const Schedule plan = schedule_for(l0, p, iters, may_grade ? n : 0, iters <= 0 && (track_sweeps & 512) == 0 ? n : 0);
+  const Schedule plan = schedule_for(l0, p, iters, may_grade ? n : 0, iters <= 0 && (track_sweeps & 512) == 0 ? n : 0,
+                                     estimated ? 0 : (l0 > l_worst ? 1 : 2));
   iters = plan.iters;
   const GradedPoly& graded = plan.graded;
   if (iters < 2 && !graded.products) return fail(kErrArg, "inv_roots: at least two iterations are required");
@@ -1942,7 +1994,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float* e_top = small(18);
     float* rest_trace = small(10);
     const size_t sm8 = align_up((size_t)kc * 32, 256);
-    char* wp = w + sm * 19;
+    char* wp = w + sm * 20;
     float* th8 = reinterpret_cast<float*>(wp); wp += sm8;     // Ritz values, residuals, deflation coefficients and
     float* res8 = reinterpret_cast<float*>(wp); wp += sm8;    // root corrections of the block deflation: eight per statistic
     float* coef8 = reinterpret_cast<float*>(wp); wp += sm8;
@@ -1952,7 +2004,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float* pv = reinterpret_cast<float*>(wp);
     float* py = reinterpret_cast<float*>(wp + vec);
     float* dv = deflate ? deflate + (long long)k0 * kMaxDeflate * n : nullptr;
-    TONER_CUDA(cudaMemsetAsync(w, 0, sm * 19 + 4 * sm8, stream));
+    TONER_CUDA(cudaMemsetAsync(w, 0, sm * 20 + 4 * sm8, stream));
 
     const float* C = ema + (long long)k0 * nn;
     const int damp_tiles = (n + kDampTile - 1) / kDampTile;
@@ -2012,14 +2064,19 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     const float init_b = (float)(graded_finish ? -graded.za : first_z ? -sched[0].za : sched[0].b);
     const float init_sm = graded_finish ? s_top : s_m, init_diag = graded_finish ? (float)top_diag : 0.f;
     float s_t = first_z ? s_z : plane_scale(sched[0].a);
+    // Statistics that start with the second step: M_0 where the first one leaves M, planes of the second Z, and the first step's
+    // products left out; T_1 is their X_2 (the product with X is left out too).
+    int* const late = plan.late > 0.0 ? reinterpret_cast<int*>(small(19)) : nullptr;
+    InitLate second = {};
+    if (late) second = {(float)sched[1].zb, (float)-sched[1].za, Mb[1], Tb[0], sched[1].lin != 0.0 ? A32 : nullptr};
     if (ritz_norm) {
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, kMaxDeflate, m32, init_diag, graded_finish);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, kMaxDeflate, m32, init_diag, graded_finish, nullptr, InitLate());
       TONER_CUDA(cudaGetLastError());
     } else {
-    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false);
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false, nullptr, InitLate());
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -2060,8 +2117,8 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       if (rc1) return rc1;
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
-      TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, nullptr, nullptr, 0, 0, m32, init_diag, graded_finish);
+      TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc, late, (float)(1.0001 * plan.late), damping);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, nullptr, nullptr, 0, 0, m32, init_diag, graded_finish, late, second);
       TONER_CUDA(cudaGetLastError());
     }
     }
@@ -2086,7 +2143,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       bool upper_d = false;                        // d is read as a product's C alone, which takes its upper triangle
     };
     // (in_step: matrices between the hi and lo planes of the operands; 0: the chunk's)
-    auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote, int in_step = 0) -> int {
+    auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote, int in_step = 0, const int* skip = nullptr) -> int {
       toner_gemm_desc g = {};
       toner_operand op = {};
       const int lo = in_step ? in_step : kc;
@@ -2108,7 +2165,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g.maxres = o.maxres;
       g.promote = promote;
       g.interleave = interleave ? 1 : 0;
-      return launch_gemm(g, stream);
+      return launch_gemm(g, stream, skip);
     };
     int rc = 0;
     // the finish in steps of Y; its planes of R + beta I go where the powers of T leave room (p = 1 has no such buffer)
@@ -2130,6 +2187,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     float root_diag = 0.f;
     for (int it = 0; it < iters; ++it) {
       const bool last = (it == iters - 1);
+      const int* const skip = it == 0 ? late : nullptr;
       if (!last && sched[it].degree > 1) {
         // T from planes of Z (Tcur), see root_steps.cuh: its square, of degree four the square of that, shifted.  T_0 is X_1 as well.
         // The errors of these products matter as those of the powers of T do.
@@ -2141,7 +2199,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           Out y;
           y.s0 = Pb[1]; y.s0_scale = plane_scale(1.1 + std::fabs(st.kappa));
           y.s0_a = (float)st.kappa;
-          rc = sym_product(from, s_from, from, s_from, y, chain);
+          rc = sym_product(from, s_from, from, s_from, y, chain, 0, skip);
           if (rc) return rc;
           from = y.s0;
           s_from = y.s0_scale;
@@ -2154,7 +2212,11 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         if (st.lin != 0.0) {
           t.c = it == 0 ? m32 : A32; t.beta = (float)st.lin;
         }
-        rc = sym_product(from, s_from, from, s_from, t, chain);
+        if (it == 1 && late) {
+          t.s1 = Xb[xi]; t.s1_scale = plane_scale(std::min(x_bound * st.a, x_cap));
+          t.s1_a = (float)st.con; t.s1_b = 1.f;
+        }
+        rc = sym_product(from, s_from, from, s_from, t, chain, 0, skip);
         if (rc) return rc;
         Tcur = t.s0;
         s_t = t.s0_scale;
@@ -2177,7 +2239,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             if (rc) return rc;
           }
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : (plan.steep ? 0.65f : 0.5f), damping, lower_used, plan.steep && ritz_norm ? th8 : nullptr);
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : (plan.steep ? 0.7f : 0.5f), damping, lower_used, plan.steep && ritz_norm ? th8 : nullptr);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
@@ -2302,7 +2364,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         Out o;
         o.s0 = Xb[xi];
         o.s0_scale = plane_scale(x_bound);
-        rc = sym_product(Xcur, s_x, Tcur, s_t, o, plan.steep ? kPromoteSteepX : kPromoteX);
+        rc = sym_product(Xcur, s_x, Tcur, s_t, o, plan.steep ? kPromoteSteepX : kPromoteX, 0, it == 1 ? late : nullptr);
         if (rc) return rc;
         Xcur = Xb[xi];
         s_x = o.s0_scale;
@@ -2321,7 +2383,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         Out o;
         o.s0 = Pb[j & 1];
         o.s0_scale = plane_scale(pw_bound);
-        rc = sym_product(pw, s_pw, pw, s_pw, o, chain);
+        rc = sym_product(pw, s_pw, pw, s_pw, o, chain, 0, skip);
         if (rc) return rc;
         pw = o.s0;
         s_pw = o.s0_scale;
@@ -2360,7 +2422,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             o.s1_b = -nb;
           }
         }
-        rc = sym_product(pw, s_pw, Mb[mi], s_m, o, chain);
+        rc = sym_product(pw, s_pw, Mb[mi], s_m, o, chain, 0, skip);
         if (rc) return rc;
         mi ^= 1;
         ti = tn;

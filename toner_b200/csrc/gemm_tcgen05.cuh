@@ -91,6 +91,7 @@ struct GemmParams {
   __half* S1;
   long long s_ld, s_bs, s_plane;
   float s0_scale, s0_aff_a, s1_scale, s1_aff_a, s1_aff_b;
+  const int* skip;   // optional, per batch: not zero where the product is left out (its outputs keep what they hold)
   int* status;  // set non-zero if a bounded wait ran out
   unsigned long long* prof;  // optional: eight cycle counters summed over CTAs (see toner_gemm_phase_cycles)
   // 32 x 32 boxes of C and of the outputs, (columns, rows, batch): FP32 with 128-byte, 16-bit with 64-byte swizzle
@@ -570,6 +571,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     }
     return w;
   };
+  // (every role asks alike: what is left out is left out by all of them)
+  auto left_out = [&](int b) { return p.skip != nullptr && p.skip[b] != 0; };
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::kStages; ++s) {
       ptx::mbar_init(full_bar(s), 1);
@@ -615,6 +618,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         const Unit w = unit_of(u);
         int b, tm, tn;
         tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
+        if (left_out(b)) continue;
         const CUtensorMap* amap = &p.a_map;
         const CUtensorMap* bmap = &p.b_map;
         if (p.a_maps) {
@@ -743,6 +747,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       const long long prof_t0 = p.prof ? clock64() : 0;
       for (int u = unit; u < total_units && ok; u += units) {
         const Unit w = unit_of(u);
+        if (left_out(w.tile / tiles_per_batch)) continue;
         for (int ch = w.ch_lo; ch < w.ch_hi && ok; ++ch, ++gchunk) {
           int kb_begin = w.kb_lo, kb_end = w.kb_hi;
           if (p.promote > 0) chunk_range(ch, kb_begin, kb_end);
@@ -898,6 +903,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       const Unit w = unit_of(u);
       int b, tm, tn;
       tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
+      if (left_out(b)) continue;
       const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN;  // this CTA's 128 rows of the tile
       const int row_first = m0 + lane_group * 32;
       const int col_first = n0 + half * (BN / 2);

@@ -375,7 +375,7 @@ static int gemm_params(Context* ctx, const toner_gemm_desc& d, int bn, bool pair
   return 0;
 }
 
-int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
+int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const int* skip) {
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   if (d.m <= 0 || d.n <= 0 || d.k <= 0 || d.batch <= 0) return fail(kErrArg, "gemm: sizes must be positive");
@@ -412,6 +412,7 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream) {
   const bool inter = pair && bn <= 256 && may_interleave(d);
   GemmParams p;
   if (int rc = gemm_params(ctx, d, bn, pair, splits, inter, stream, p)) return rc;
+  p.skip = skip;
 
   const long long total = gemm_tiles(d, bn, pair) * splits;
   if (total > 0x7fffffffLL) return fail(kErrArg, "gemm: too many tiles");

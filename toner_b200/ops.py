@@ -344,17 +344,20 @@ def inv_roots_schedule(lower: float, p: int, iters: int = 0) -> dict:
             "coefficients": [coef[j] for j in range(order.value + 1)], "distance": e.value}
 
 
-def inv_roots_steps(lower: float, p: int, n: int) -> Optional[dict]:
+def inv_roots_steps(lower: float, p: int, n: int, kind: int = 0) -> Optional[dict]:
     """The schedule of a call on statistics of width n that takes steps of higher degree (toner_inv_roots_steps_for; needs no
     device): {"steps": [(degree, zb, za, kappa, top, lin, con)], "coefficients": of the finishing polynomial, "distance": e,
-    "products": (split, single passes)}; None where linear steps are used."""
+    "products": (split, single passes), "late": the bound from which a statistic starts with the second step, 0: none}; None
+    where linear steps are used.  kind: the bound is an estimate (0), certified (1), the one that always holds (2)."""
     steps, coef = (C.c_double * 128)(), (C.c_double * 16)()
-    order, products, e = C.c_int32(0), (C.c_int32 * 2)(), C.c_double(0.0)
-    count = _lib.load().toner_inv_roots_steps_for(lower, p, n, steps, 128, coef, 16, C.byref(order), products, C.byref(e))
+    order, products, e, late = C.c_int32(0), (C.c_int32 * 2)(), C.c_double(0.0), C.c_double(0.0)
+    count = _lib.load().toner_inv_roots_steps_for(lower, p, n, kind, steps, 128, coef, 16, C.byref(order), products, C.byref(e),
+                                                  C.byref(late))
     if count <= 0:
         return None
     return {"steps": [(int(steps[7 * k]), *steps[7 * k + 1:7 * k + 7]) for k in range(count)],
-            "coefficients": coef[:order.value + 1], "distance": e.value, "products": (products[0], products[1])}
+            "coefficients": coef[:order.value + 1], "distance": e.value, "products": (products[0], products[1]),
+            "late": late.value}
 
 
 def inv_roots_graded(lower: float, p: int, n: int) -> Optional[dict]:
