@@ -188,10 +188,10 @@ class FactorSet:
         self.lmin = torch.zeros(k, device=device, dtype=torch.float32)
         self.lmin_host = self._host[2 * k:3 * k].view(torch.float32)
         self.track_restart = True        # the vectors hold nothing yet (or the statistics were replaced)
-        # Dominant directions (outlier features): eight vector slots per statistic, found by block power iteration and
-        # deflated where they stand out.  The block is two vectors wider than the number of directions that looked like
+        # Dominant directions (outlier features): twelve vector slots per statistic (eight where the plane order is kept, and with it
+        # the bits), found by block power iteration and deflated where they stand out.  The block is two vectors wider than the number of directions that looked like
         # outliers last time (a block wider than the group of outliers is what makes close outliers converge).
-        self.deflate = torch.zeros(k, 8, n, device=device, dtype=torch.float32)
+        self.deflate = torch.zeros(k, 12 if interleave else 8, n, device=device, dtype=torch.float32)
         self.deflated = torch.zeros(k, device=device, dtype=torch.int32)
         self.deflated_host = self._host[3 * k:4 * k]
         self.deflate_rank = 4
@@ -395,7 +395,7 @@ class FactorSet:
         worst = self.damping / (self.n * (1.0 + self.damping))
         if self.tracking and self.block_deflation:
             candidates = int((host[3 * k:4 * k] >> 8).max())
-            self.deflate_rank = max(2, min(8, candidates + 2))
+            self.deflate_rank = max(2, min(self.deflate.shape[1], candidates + 2))
         self.lower, self.lower_is_estimate = 0.0, False
         if getattr(self, "_estimate_in_flight", False) and any(c in (1, 4) for c in codes):
             self.estimate_backoff = 8     # (a gross overestimate already fails the convergence test, status 1)

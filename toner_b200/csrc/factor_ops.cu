@@ -563,6 +563,9 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
   return s;
 }
 
+// Directions that are deflated at most: four numbers a statistic and direction (Ritz value, residual, coefficients) lie this far apart.
+constexpr int kMaxDeflate = 12;
+
 // ------------------------------------------------------------------ elementwise helpers
 __global__ void __launch_bounds__(256) trace_kernel(const float* __restrict__ c, int n, float* __restrict__ trace) {
   ptx::pdl_begin();
@@ -678,11 +681,11 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* a32, int 
     t_planes = second.t_planes;
     m32 = second.m32;
   }
-  float cf[8];
+  float cf[kMaxDeflate];
   bool any = false;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    cf[j] = (defl_v != nullptr && j < defl_r) ? defl_coef[bi * 8 + j] : 0.f;
+  for (int j = 0; j < kMaxDeflate; ++j) {
+    cf[j] = (defl_v != nullptr && j < defl_r) ? defl_coef[bi * kMaxDeflate + j] : 0.f;
     any = any || cf[j] != 0.f;
   }
   const float* DV = defl_v ? defl_v + (long long)bi * vstride * n : nullptr;
@@ -699,7 +702,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* a32, int 
     float4 v = A[i];
     if (any) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < kMaxDeflate; ++j) {
         if (cf[j] != 0.f) {
           const float vr = DV[(long long)j * n + r];
           const float4 vc = *reinterpret_cast<const float4*>(DV + (long long)j * n + c);
@@ -874,7 +877,8 @@ __global__ void __launch_bounds__(256) rank1_update_kernel(float* __restrict__ a
 // statistic per sweep, whatever r is, and converges with the ratio of the (r+1)-th eigenvalue to the wanted one, so
 // close pairs among the dominant ones do not slow it down; the vectors are kept by the caller between calls.
 // Vectors are stored vector-major: v[(b * vstride + j) * n + c].
-constexpr int kMaxDeflate = 8;  // (init_planes_kernel keeps that many coefficients in registers)
+// Eight slots a statistic, or twelve.
+constexpr int kSlots = 8, kMoreSlots = kMaxDeflate;
 
 // Y_j = A v_j, j < R: one pass over A.  A block takes 32 rows (four per warp; 16 and two from six vectors on) and walks the columns 256 at a time; the
 // 256-column slice of the vectors is staged in shared memory once per block, so the vectors are read from L2 once per
@@ -892,7 +896,7 @@ template <int R>
 struct BlockGemv {
   static constexpr int kWarpRows = R <= 4 ? 4 : 2;
   static constexpr int kRows = 8 * kWarpRows;
-  static constexpr int kStages = R <= 4 ? 3 : 4;
+  static constexpr int kStages = R <= 4 || R > 10 ? 3 : 4;
   static constexpr int kStageFloat4 = (kRows + R) * 64;   // 256 columns of the block's rows and of the vectors
   static constexpr int kBytes = kStages * kStageFloat4 * 16;
 };
@@ -1000,7 +1004,8 @@ bool allow_factor_kernels() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
   };
   return allow(block_gemv_kernel<2>, BlockGemv<2>::kBytes) && allow(block_gemv_kernel<4>, BlockGemv<4>::kBytes) &&
-         allow(block_gemv_kernel<6>, BlockGemv<6>::kBytes) && allow(block_gemv_kernel<8>, BlockGemv<8>::kBytes);
+         allow(block_gemv_kernel<6>, BlockGemv<6>::kBytes) && allow(block_gemv_kernel<8>, BlockGemv<8>::kBytes) &&
+         allow(block_gemv_kernel<10>, BlockGemv<10>::kBytes) && allow(block_gemv_kernel<12>, BlockGemv<12>::kBytes);
 }
 
 // Sum over the block of one double per thread; every thread gets the total.  256 threads.
@@ -1050,14 +1055,14 @@ __device__ __forceinline__ void block_sum_many(double (&acc)[K], double* part, d
 // entry (i, j), j <= i, of a symmetric matrix's lower triangle
 __device__ __forceinline__ int pair_index(int i, int j) { return i * (i + 1) / 2 + j; }
 
-// Cholesky-QR of the r vectors held in Y (r x n, vector-major): G = Y Y^T = L L^T (FP64), V = L^-1 Y.  `gram` holds G's
+// Cholesky-QR of the r vectors held in Y (r x n, vector-major; a thread's columns from `first` on): G = Y Y^T = L L^T (FP64), V = L^-1 Y.  `gram` holds G's
 // lower triangle (pair_index order) on entry.  A vector that is (numerically) a combination of the earlier ones comes out as
 // zero; its slot is seeded afresh by the next call.  L's columns are formed one after the other by the lanes of one warp (row
 // i of a column by lane i); the diagonal of `L` holds its reciprocal (zero for a dropped vector), the diagonal itself where
 // `divide` asks for divisions by it (see ritz_kernel).
 template <int R>
 __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, const double* gram, double (*L)[kMaxDeflate],
-                                        bool divide) {
+                                        bool divide, int first, int step) {
   if (threadIdx.x < 32) {
     const int i = threadIdx.x;
     double row[R];
@@ -1084,7 +1089,7 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
     }
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+  for (int c = first; c < n; c += step) {
     double out[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
@@ -1105,17 +1110,19 @@ __device__ void cholesky_orthonormalise(const float* Y, float* V, int n, int r, 
   __syncthreads();
 }
 
-// Eigenpairs of the symmetric r x r matrix H (shared memory, FP64) by Jacobi rotations, H and Q of size kMaxDeflate with
-// zeros beyond r.  One warp: each of the seven rounds of a sweep rotates four disjoint pairs at once (round-robin order), eight
-// lanes a pair, one matrix index each.  A single thread doing the rotations one by one took 20 us of a 23 us launch at r = 4
-// and most of 160 us at r = 8.
+// Eigenpairs of the symmetric r x r matrix H (shared memory, FP64) by Jacobi rotations, zeros from r to R (even).  One warp: each of
+// the R - 1 rounds of a sweep rotates R / 2 disjoint pairs at once (round-robin order), the lanes of a pair taking its rows and
+// columns in turn.  A single thread doing the rotations one by one took 20 us of a 23 us launch at r = 4 and most of 160 us at r = 8;
+// eight seats whatever R, seven rounds for three at R = 4.
+template <int R>
 __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) {
-  static_assert(kMaxDeflate == 8, "four pairs of eight lanes");
-  const int lane = threadIdx.x, pair = lane >> 3, k = lane & 7;
+  constexpr int kPairs = R / 2, kLanes = 32 / kPairs;
+  const int lane = threadIdx.x, pair = lane / kLanes, k0 = lane % kLanes;
+  const bool on = pair < kPairs;
   for (int sweep = 0; sweep < 12; ++sweep) {
     double off = 0.0, diag = 0.0;
-    for (int e = lane; e < 64; e += 32) {
-      const int i = e >> 3, j = e & 7;
+    for (int e = lane; e < R * R; e += 32) {
+      const int i = e / R, j = e - i * R;
       const double h = H[i][j];
       if (i == j) diag += h * h;
       else if (j > i) off += h * h;
@@ -1125,29 +1132,37 @@ __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) 
       off += __shfl_xor_sync(0xffffffffu, off, o);
       diag += __shfl_xor_sync(0xffffffffu, diag, o);
     }
-    if (!(off > 1e-30 * diag)) break;   // off-diagonal part below FP64 rounding of the diagonal: converged
-    for (int round = 0; round < 7; ++round) {
-      // seat 7 stays, the others rotate: pair 0 = (7, round), pair i = (round + i, round - i) mod 7
-      int a = pair == 0 ? 7 : (round + pair) % 7, b = pair == 0 ? round : (round + 7 - pair) % 7;
-      const int pp = min(a, b), qq = max(a, b);
-      const double apq = H[pp][qq];
+    if (!(off > 1e-28 * diag)) break;   // off-diagonal part 1e-14 of the largest: far below what FP32 vectors hold
+    for (int round = 0; round < R - 1; ++round) {
+      // the last seat stays, the others rotate
+      const int a = pair == 0 ? R - 1 : (round + pair) % (R - 1), b = pair == 0 ? round : (round + R - 1 - pair) % (R - 1);
+      const int pp = on ? min(a, b) : 0, qq = on ? max(a, b) : 0;
+      const double apq = on ? H[pp][qq] : 0.0;
       double cs = 1.0, sn = 0.0;
-      if (apq != 0.0) {
+      if (on && apq != 0.0) {
         const double tau = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
         const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
         cs = rsqrt(1.0 + t * t);
         sn = t * cs;
       }
       __syncwarp();   // every pair has its rotation before any entry changes
-      const double hp = H[k][pp], hq = H[k][qq], qp = Q[k][pp], qv = Q[k][qq];   // columns pp, qq of H and Q
-      H[k][pp] = cs * hp - sn * hq;
-      H[k][qq] = sn * hp + cs * hq;
-      Q[k][pp] = cs * qp - sn * qv;
-      Q[k][qq] = sn * qp + cs * qv;
+      if (on) {
+        for (int k = k0; k < R; k += kLanes) {
+          const double hp = H[k][pp], hq = H[k][qq], qp = Q[k][pp], qv = Q[k][qq];   // columns pp, qq of H and Q
+          H[k][pp] = cs * hp - sn * hq;
+          H[k][qq] = sn * hp + cs * hq;
+          Q[k][pp] = cs * qp - sn * qv;
+          Q[k][qq] = sn * qp + cs * qv;
+        }
+      }
       __syncwarp();
-      const double rp = H[pp][k], rq = H[qq][k];                                 // rows pp, qq of H
-      H[pp][k] = cs * rp - sn * rq;
-      H[qq][k] = sn * rp + cs * rq;
+      if (on) {
+        for (int k = k0; k < R; k += kLanes) {
+          const double rp = H[pp][k], rq = H[qq][k];                                 // rows pp, qq of H
+          H[pp][k] = cs * rp - sn * rq;
+          H[qq][k] = sn * rp + cs * rq;
+        }
+      }
       __syncwarp();
     }
   }
@@ -1224,80 +1239,131 @@ __global__ void __launch_bounds__(256) block_start_kernel(float* __restrict__ v,
       for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += x[i] * x[j];
   }
   block_sum_many<kPairs>(acc, part, gram);
-  cholesky_orthonormalise<R>(V, V, n, r, gram, L, in_order != 0);
+  cholesky_orthonormalise<R>(V, V, n, r, gram, L, in_order != 0, threadIdx.x, blockDim.x);
+}
+
+// Sums over a cluster's CTAs, as block_sum_many's over one block: `mine` is K doubles of shared memory that the others read.
+template <int K>
+__device__ __forceinline__ void cluster_sum_many(double (&acc)[K], double* part, double* mine, double* out, int ctas) {
+  block_sum_many<K>(acc, part, ctas > 1 ? mine : out);
+  if (ctas > 1) {
+    ptx::cluster_sync();   // every CTA's sums are there
+    if (threadIdx.x < K) {
+      double t = 0.0;
+      for (int rank = 0; rank < ctas; ++rank) t += ptx::ld_cluster_f64(ptx::mapa(ptx::smem_u32(mine + threadIdx.x), rank));
+      out[threadIdx.x] = t;
+    }
+    ptx::cluster_sync();   // ... and have been read
+  }
 }
 
 // Rayleigh-Ritz on span(V) with Y = A V (V orthonormal): H = V Y^T, H = Q diag(theta) Q^T (Jacobi, FP64), V <- Q^T V,
 // Y <- Q^T Y (Ritz vectors, descending theta), res_j = ||Y_j - theta_j V_j|| / |theta_j|.  Unless this is the last sweep, V is
-// then replaced by the orthonormalised Y (one more step of the power iteration).  Three passes over the two blocks of
-// vectors; every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
+// then replaced by the orthonormalised Y - sigma V, one more step of the power iteration on A - sigma I: with sigma = 0.8 c, c the
+// mean of the eigenvalues that do not stand out, what lies below 1.6 c shrinks as if it were 0.8 c (a bulk up to 1.8 under a
+// direction of 10: by 0.11 a sweep where A itself gives 0.18; four sweeps then reach the residual that deflation asks for, with
+// which the fifth direction of spiked:4 was left in one call of four).
+// Three passes over the two blocks of vectors (five from ten vectors on, whose sums are taken for half of the rows at a time);
+// every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
 // vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2; now 17.
-// in_order: a caller that keeps its order of additions (the plane-by-plane products) has the small factorisations keep theirs
-// too: Jacobi's rotations one after the other and divisions by Cholesky's diagonal.  The vectors are no better for it, but a
-// deflated eigenvalue hundreds of times the rest turns their last bits into 1e-5 of what remains.
+// A cluster shares a statistic's columns (a few statistics are a few blocks on 148 SMs, and a pass of one block over 3328 columns is
+// thirteen round trips to L2): every CTA factors the small matrix for itself, from the same sums.
+// in_order (one CTA, no sigma): a caller that keeps its order of additions (the plane-by-plane products) has the small
+// factorisations keep theirs too: Jacobi's rotations one after the other and divisions by Cholesky's diagonal.  The vectors are no
+// better for it, but a deflated eigenvalue hundreds of times the rest turns their last bits into 1e-5 of what remains.
 template <int R>
 __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float* __restrict__ y, int n, int r, int vstride,
-                                                   int last, float* __restrict__ theta, float* __restrict__ res, int in_order) {
+                                                   int last, float* __restrict__ theta, float* __restrict__ res, int in_order,
+                                                   float trace) {
   ptx::pdl_begin();
-  constexpr int kPairs = R * (R + 1) / 2, kSums = R * R > kPairs + R ? R * R : kPairs + R, kMost = kMaxDeflate;
-  __shared__ double part[8 * kSums], sums[kSums];
-  __shared__ double H[kMost][kMost], Q[kMost][kMost], lam[kMost], L[kMost][kMost];
-  const int b = blockIdx.x;
+  constexpr int kPairs = R * (R + 1) / 2, kMost = kMaxDeflate;
+  constexpr bool kHalves = R > 8;
+  constexpr int kRows = kHalves ? R / 2 : R;                            // of the rows whose sums are taken at a time
+  constexpr int kFirst = kRows * R, kSecond = kHalves ? kRows * R + kRows : kPairs + R;
+  constexpr int kSums = kFirst > kSecond ? kFirst : kSecond;
+  __shared__ double part[8 * kSums], mine[kSums], sums[kSums], gram[kPairs], resid[R];
+  __shared__ double H[kMost][kMost], Q[kMost][kMost], lam[kMost], L[kMost][kMost], shift;
+  const int ctas = (int)ptx::cluster_nctarank(), rank = (int)ptx::cluster_ctarank();
+  const int b = blockIdx.y;
+  const int first = rank * blockDim.x + threadIdx.x, step = ctas * blockDim.x;
   float* V = v + (long long)b * vstride * n;
   float* Y = y + (long long)b * vstride * n;
-  {
-    double acc[R * R];
+  for (int e = threadIdx.x; e < kMost * kMost; e += blockDim.x) {
+    const int i = e / kMost, j = e - i * kMost;
+    H[i][j] = 0.0;
+    Q[i][j] = i == j ? 1.0 : 0.0;
+  }
+  // V Y^T, kept in L until it is whole
 #pragma unroll
-    for (int i = 0; i < R * R; ++i) acc[i] = 0.0;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
-      double vv[R], yy[R];
+  for (int half = 0; half < R / kRows; ++half) {
+    double acc[kFirst];
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        vv[i] = i < r ? (double)V[(long long)i * n + c] : 0.0;
-        yy[i] = i < r ? (double)Y[(long long)i * n + c] : 0.0;
-      }
+    for (int i = 0; i < kFirst; ++i) acc[i] = 0.0;
+    for (int c = first; c < n; c += step) {
+      double vv[kRows], yy[R];
 #pragma unroll
-      for (int i = 0; i < R; ++i)
+      for (int i = 0; i < kRows; ++i) vv[i] = half * kRows + i < r ? (double)V[(long long)(half * kRows + i) * n + c] : 0.0;
+#pragma unroll
+      for (int i = 0; i < R; ++i) yy[i] = i < r ? (double)Y[(long long)i * n + c] : 0.0;
+#pragma unroll
+      for (int i = 0; i < kRows; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) acc[i * R + j] += vv[i] * yy[j];
     }
-    block_sum_many<R * R>(acc, part, sums);
+    cluster_sum_many<kFirst>(acc, part, mine, sums, ctas);
+    for (int e = threadIdx.x; e < kFirst; e += blockDim.x) L[half * kRows + e / R][e % R] = sums[e];
+    __syncthreads();
   }
-  if (threadIdx.x < 64) {
-    const int i = threadIdx.x >> 3, j = threadIdx.x & 7;
-    H[i][j] = (i < r && j < r) ? 0.5 * (sums[i * R + j] + sums[j * R + i]) : 0.0;
-    Q[i][j] = i == j ? 1.0 : 0.0;
+  for (int e = threadIdx.x; e < R * R; e += blockDim.x) {
+    const int i = e / R, j = e % R;
+    if (i < r && j < r) H[i][j] = 0.5 * (L[i][j] + L[j][i]);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
     if (in_order) jacobi_in_order(H, Q, r);
-    else jacobi_warp(H, Q);
+    else jacobi_warp<R>(H, Q);
     // descending order: lane i's place is the number of values before it; the columns of Q follow
-    const int i = threadIdx.x & 7;
-    const double mine = H[i][i];
+    const int i = threadIdx.x % kMost;
+    const double own = H[i][i];
     int place = 0;
     for (int j = 0; j < r; ++j) {
       const double o = H[j][j];
-      if (o > mine || (o == mine && j < i)) ++place;
+      if (o > own || (o == own && j < i)) ++place;
     }
     double col[kMost];
 #pragma unroll
     for (int k = 0; k < kMost; ++k) col[k] = Q[k][i];
     __syncwarp();
     if (threadIdx.x < r) {
-      lam[place] = mine;
+      lam[place] = own;
 #pragma unroll
       for (int k = 0; k < kMost; ++k) Q[k][place] = col[k];
     }
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      // the mean of what does not stand above eight times it, as block_decide_kernel has it
+      double sum = 0.0;
+      int m = 0;
+      for (; m < r && n - (m + 1) > 0; ++m) {
+        const double rest = ((double)trace - sum - lam[m]) / (double)(n - (m + 1));
+        if (!(rest > 0.0 && lam[m] > 8.0 * rest)) break;
+        sum += lam[m];
+      }
+      const double rest = ((double)trace - sum) / (double)(n - m);
+      shift = in_order || last || !(rest > 0.0) ? 0.0 : 0.8 * rest;
+    }
   }
   __syncthreads();
+  const double sigma = shift;
   {
     // rotate both blocks (new vector j = sum_i Q[i][j] old vector i); on the way: the squared residuals and the Gram
     // matrix of the rotated Y (for its orthonormalisation)
-    double acc[kPairs + R];
+    double acc[kHalves ? 1 : kSecond];
+    if constexpr (!kHalves) {
 #pragma unroll
-    for (int i = 0; i < kPairs + R; ++i) acc[i] = 0.0;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+      for (int i = 0; i < kSecond; ++i) acc[i] = 0.0;
+    }
+    for (int c = first; c < n; c += step) {
       double vv[R], yy[R], nv[R], ny[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) {
@@ -1316,33 +1382,79 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
             }
           }
           // what is stored is what later passes read: round before the sums
-          const float fv = (float)sv, fy = (float)sy;
+          const float fv = (float)sv;
+          sv = fv;
+          if (sigma != 0.0) sy -= sigma * sv;
+          const float fy = (float)sy;
           V[(long long)j * n + c] = fv;
           Y[(long long)j * n + c] = fy;
-          sv = fv;
           sy = fy;
         }
         nv[j] = sv;
         ny[j] = sy;
       }
+      if constexpr (!kHalves) {
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        if (i < r) {
+        for (int i = 0; i < R; ++i) {
+          if (i < r) {
 #pragma unroll
-          for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += ny[i] * ny[j];
-          const double d = ny[i] - lam[i] * nv[i];
-          acc[kPairs + i] += d * d;
+            for (int j = 0; j <= i; ++j) acc[i * (i + 1) / 2 + j] += ny[i] * ny[j];
+            const double d = ny[i] - (lam[i] - sigma) * nv[i];
+            acc[kPairs + i] += d * d;
+          }
         }
       }
     }
-    block_sum_many<kPairs + R>(acc, part, sums);
+    if constexpr (!kHalves) {
+      cluster_sum_many<kSecond>(acc, part, mine, sums, ctas);
+      for (int e = threadIdx.x; e < kPairs + R; e += blockDim.x) (e < kPairs ? gram[e] : resid[e - kPairs]) = sums[e];
+    }
   }
-  if (threadIdx.x < r) {
+  if constexpr (kHalves) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      double acc[kSecond];
+#pragma unroll
+      for (int i = 0; i < kSecond; ++i) acc[i] = 0.0;
+      for (int c = first; c < n; c += step) {   // (columns this thread has just written)
+        double ny[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) ny[i] = i < r ? (double)Y[(long long)i * n + c] : 0.0;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+          const int row = half * kRows + i;
+          if (row < r) {
+#pragma unroll
+            for (int j = 0; j < R; ++j) acc[i * R + j] += ny[half * kRows + i] * ny[j];
+            const double d = ny[half * kRows + i] - (lam[row] - sigma) * (double)V[(long long)row * n + c];
+            acc[kRows * R + i] += d * d;
+          }
+        }
+      }
+      cluster_sum_many<kSecond>(acc, part, mine, sums, ctas);
+      for (int e = threadIdx.x; e < kRows * R; e += blockDim.x) {
+        const int i = half * kRows + e / R, j = e % R;
+        if (j <= i) gram[pair_index(i, j)] = sums[e];
+      }
+      if (threadIdx.x < kRows) resid[half * kRows + threadIdx.x] = sums[kRows * R + threadIdx.x];
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  if (rank == 0 && threadIdx.x < r) {
     const double l = lam[threadIdx.x];
     theta[b * kMost + threadIdx.x] = (float)l;
-    res[b * kMost + threadIdx.x] = l > 0.0 ? (float)(sqrt(sums[kPairs + threadIdx.x]) / l) : INFINITY;
+    res[b * kMost + threadIdx.x] = l > 0.0 ? (float)(sqrt(resid[threadIdx.x]) / l) : INFINITY;
   }
-  if (!last) cholesky_orthonormalise<R>(Y, V, n, r, sums, L, in_order != 0);
+  if (!last) cholesky_orthonormalise<R>(Y, V, n, r, gram, L, in_order != 0, first, step);
+}
+// CTAs that share a statistic: as many as have two hundred columns each, eight at most.
+static int ritz_ctas(int n) { return n >= 2048 ? 8 : n >= 1024 ? 4 : n >= 512 ? 2 : 1; }
+template <int R>
+static cudaError_t launch_ritz(int k, cudaStream_t stream, float* v, float* y, int n, int r, int vstride, int last, float* theta, float* res,
+                               int in_order, float trace) {
+  const int ctas = in_order ? 1 : ritz_ctas(n);
+  return launch(ritz_kernel<R>, dim3(ctas, k), 256, 0, stream, ctas > 1 ? ctas : 0, v, y, n, r, vstride, last, theta, res, in_order, trace);
 }
 
 // Which of the r Ritz pairs are deflated: in descending order, as long as each has converged and stands above eight
@@ -1721,11 +1833,11 @@ static size_t per_statistic_bytes(int n) {
   return align_up((size_t)n * n * 4, 256) * 8;
 }
 static size_t small_bytes(int chunk, int n) {
-  // twenty per-statistic scalars, four blocks of eight scalars per statistic (Ritz values, residuals, deflation
-  // coefficients, root corrections), the reduction scratch, and two blocks of eight n-vectors per statistic
+  // twenty per-statistic scalars, four blocks of kMaxDeflate scalars per statistic (Ritz values, residuals, deflation
+  // coefficients, root corrections), the reduction scratch, and two blocks of as many n-vectors per statistic
   // (block power iteration: V and A V)
-  return align_up((size_t)chunk * 4, 256) * 20 + 4 * align_up((size_t)chunk * 32, 256) +
-         align_up(sumsq_scratch_bytes(chunk), 256) + 2 * align_up((size_t)chunk * 8 * n * 4, 256);
+  return align_up((size_t)chunk * 4, 256) * 20 + 4 * align_up((size_t)chunk * kMaxDeflate * 4, 256) +
+         align_up(sumsq_scratch_bytes(chunk), 256) + 2 * align_up((size_t)chunk * kMaxDeflate * n * 4, 256);
 }
 
 // Largest power of two s with s * bound <= 2^14: FP16 planes of s * x then stay a factor four below overflow
@@ -1911,10 +2023,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     return fail(kErrArg, "inv_roots: track_sweeps is 0..63, plus 256 to start afresh, plus 512 for plane-by-plane products");
   const int defl_r = deflate ? (deflate_rank & 15) : 0;      // directions the block iteration looks for (0: one, the old way)
   const bool defl_cold = deflate && (deflate_rank & 256);
+  const int slots = (deflate_rank & 1024) ? kMoreSlots : kSlots;
   const bool ritz_norm = deflate && (deflate_rank & 512);   // norm from the block iteration instead of three squarings
-  if (deflate && (defl_r < 1 || defl_r > kMaxDeflate || (deflate_rank & ~(15 | 256 | 512))))
+  if (deflate && (defl_r < 1 || defl_r > slots || (deflate_rank & ~(15 | 256 | 512 | 1024))))
     return fail(kErrArg, "inv_roots: deflate_rank is 1..8, plus 256 to start from fixed vectors, plus 512 to take the "
-                         "norm from the block iteration");
+                         "norm from the block iteration; 1..12 with 1024, twelve slots a statistic");
+  if (deflate && defl_r > kSlots && (track_sweeps & 512))
+    return fail(kErrUnsupported, "inv_roots: calls in plane order look for eight directions at most");
   if (ritz_norm && (defl_cold || !estimated))
     return fail(kErrArg, "inv_roots: the norm estimate needs vectors from an earlier call and an estimated lower bound "
                          "(both are verified together after the chain)");
@@ -1993,17 +2108,17 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     int* rest_idx = reinterpret_cast<int*>(small(17));
     float* e_top = small(18);
     float* rest_trace = small(10);
-    const size_t sm8 = align_up((size_t)kc * 32, 256);
+    const size_t sm8 = align_up((size_t)kc * kMaxDeflate * 4, 256);
     char* wp = w + sm * 20;
     float* th8 = reinterpret_cast<float*>(wp); wp += sm8;     // Ritz values, residuals, deflation coefficients and
-    float* res8 = reinterpret_cast<float*>(wp); wp += sm8;    // root corrections of the block deflation: eight per statistic
+    float* res8 = reinterpret_cast<float*>(wp); wp += sm8;    // root corrections of the block deflation
     float* coef8 = reinterpret_cast<float*>(wp); wp += sm8;
     float* corr8 = reinterpret_cast<float*>(wp); wp += sm8;
     float* partials = reinterpret_cast<float*>(wp); wp += align_up(sumsq_scratch_bytes(kc), 256);
-    const size_t vec = align_up((size_t)kc * 8 * n * 4, 256);
+    const size_t vec = align_up((size_t)kc * kMaxDeflate * n * 4, 256);
     float* pv = reinterpret_cast<float*>(wp);
     float* py = reinterpret_cast<float*>(wp + vec);
-    float* dv = deflate ? deflate + (long long)k0 * kMaxDeflate * n : nullptr;
+    float* dv = deflate ? deflate + (long long)k0 * slots * n : nullptr;
     TONER_CUDA(cudaMemsetAsync(w, 0, sm * 20 + 4 * sm8, stream));
 
     const float* C = ema + (long long)k0 * nn;
@@ -2018,10 +2133,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       const int sweeps = defl_cold ? 8 : 4, in_order = (track_sweeps & 512) ? 1 : 0;
       auto iterate = [&](auto width) -> int {   // (R as a type: every kernel of the iteration is specialised for it)
         constexpr int R = decltype(width)::value;
-        TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, kMaxDeflate, defl_cold ? 1 : 0, in_order);
+        TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, slots, defl_cold ? 1 : 0, in_order);
         for (int sw = 0; sw < sweeps; ++sw) {
-          TONER_CUDA(launch_block_gemv<R>(kc, stream, A32, dv, py, n, defl_r, kMaxDeflate));
-          TONER_LAUNCH(ritz_kernel<R>, kc, 256, stream, dv, py, n, defl_r, kMaxDeflate, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order);
+          TONER_CUDA(launch_block_gemv<R>(kc, stream, A32, dv, py, n, defl_r, slots));
+          TONER_CUDA(launch_ritz<R>(kc, stream, dv, py, n, defl_r, slots, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order, (float)((double)n * (1.0 + (double)damping))));
         }
         return 0;
       };
@@ -2029,11 +2144,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       if (defl_r <= 2) rcd = iterate(std::integral_constant<int, 2>());
       else if (defl_r <= 4) rcd = iterate(std::integral_constant<int, 4>());
       else if (defl_r <= 6) rcd = iterate(std::integral_constant<int, 6>());
-      else rcd = iterate(std::integral_constant<int, 8>());
+      else if (defl_r <= 8) rcd = iterate(std::integral_constant<int, 8>());
+      else if (defl_r <= 10) rcd = iterate(std::integral_constant<int, 10>());
+      else rcd = iterate(std::integral_constant<int, 12>());
       if (rcd) return rcd;
       TONER_LAUNCH(block_decide_kernel, (kc + 127) / 128, 128, stream, th8, res8, kc, n, defl_r, damping, p, ritz_norm ? defl_r - 1 : defl_r, coef8, corr8, deflated_out ? deflated_out + k0 : nullptr, rest_top, rest_idx, rest_trace);
       if (!ritz_norm) {   // (with the norm estimate the deflation is applied where the operand planes are formed)
-        TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, dv, coef8, n, defl_r, kMaxDeflate);
+        TONER_LAUNCH(rankr_update_kernel, dim3(ew_blocks, kc), 256, stream, A32, dv, coef8, n, defl_r, slots);
       }
     } else {
       // dominant direction: six power-iteration steps, then deflate where they converged
@@ -2073,7 +2190,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, kMaxDeflate, m32, init_diag, graded_finish, nullptr, InitLate());
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, slots, m32, init_diag, graded_finish, nullptr, InitLate());
       TONER_CUDA(cudaGetLastError());
     } else {
     TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false, nullptr, InitLate());
@@ -2355,7 +2472,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             root_planes = Xb[xi];
           }
           TONER_LAUNCH(root_finish_kernel, dim3(kSumsqBlocks, kc), 256, stream, R, defl_r > 0 ? dv : pv, defl_r > 0 ? corr8 : corr, n,
-                       defl_r > 0 ? defl_r : 1, defl_r > 0 ? kMaxDeflate : 1, defl_r > 0 ? kMaxDeflate : 1, s_root, root_planes,
+                       defl_r > 0 ? defl_r : 1, defl_r > 0 ? slots : 1, defl_r > 0 ? kMaxDeflate : 1, s_root, root_planes,
                        root_step ? root_step : kc, lo_planes ? lo_inv + k0 : inv_r, s_hi, hi_inv ? hi_inv + k0 : nullptr, partials, root_diag_scale, root_diag);
           TONER_LAUNCH(root_norm_kernel, kc, 32, stream, partials, fro_tmp);
           TONER_CUDA(cudaGetLastError());
@@ -2488,13 +2605,13 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // deviations, where the root it leaves is as good as any.
           const float* root = (q > 1 ? root_hi : root_lo) + (long long)k0 * nn;
           float* const py2 = py + (long long)kc * 2 * n;
-          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate, 1.f);
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 1.f);
           for (int sw = 0; sw < 2; ++sw) {
             TONER_CUDA(launch_block_gemv<2>(kc, stream, root, pv, py, n, 2, 2));
-            TONER_LAUNCH(project_kernel, dim3(kc, 2), 256, stream, py, dv, coef8, n, defl_r, kMaxDeflate);
+            TONER_LAUNCH(project_kernel, dim3(kc, 2), 256, stream, py, dv, coef8, n, defl_r, slots);
             TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, py, py2, n, 2, 2));
             TONER_CUDA(launch_block_gemv<2>(kc, stream, root, py2, py, n, 2, 2));
-            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), dv, coef8, defl_r, kMaxDeflate);
+            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), dv, coef8, defl_r, slots);
           }
         } else if (ritz_norm) {
           // The norm was an estimate too.  Eigenvalues of M_0 above 1 (the estimate was too low for them) come out of
@@ -2502,7 +2619,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // and lag the same way; they belong to the top of A', so the same four steps from the largest Ritz vector
           // that stayed in A' find them.  (An eigenvalue beyond a / b, where T changes sign, makes M grow instead and
           // fails the convergence test.)  Both starting vectors go through M in one pass per step.
-          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, kMaxDeflate, 0.f);
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 0.f);
           for (int sw = 0; sw < 4; ++sw) {
             TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, pv, py, n, 2, 2));
             TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), nullptr, nullptr, 0, 0);

@@ -389,7 +389,7 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     holds); ``norms`` (k,) receives the bound of lambda_max(A'_b) the engine normalised by, from which the next call's
     bound can be derived.  ``track`` (k, n), ``lmin`` (k,), ``track_sweeps``, ``track_restart``, ``lower_is_estimate``,
     ``resid`` (k,): tracking of the smallest eigenvalue between calls and a bound that is an estimate, verified after
-    the chain; ``deflate`` (k, 8, n), ``deflate_rank``, ``deflate_restart``, ``deflated`` (k,) int32: several dominant
+    the chain; ``deflate`` (k, 8, n) or (k, 12, n), ``deflate_rank``, ``deflate_restart``, ``deflated`` (k,) int32: several dominant
     directions found by block power iteration and deflated (see the header); ``ritz_norm``: take the norm from that
     iteration's largest remaining Ritz value instead of three squarings (an estimate, verified with ``lower``);
     ``interleave`` = False: plane products one after the other (see the header); ``lo_planes`` (2, k, n, n) FP16 with
@@ -418,9 +418,11 @@ def inv_roots(ema: torch.Tensor, damping: float, p: int, q: int = 1, *, iters: i
     if track is not None and (track.shape != (k, n) or track.dtype != torch.float32 or not track.is_contiguous()):
         raise ValueError("the tracking vectors are a contiguous FP32 (k, n) tensor")
     sweeps = (int(track_sweeps) & 63) | (256 if track_restart else 0) | (0 if interleave else 512)
-    if deflate is not None and (deflate.shape != (k, 8, n) or deflate.dtype != torch.float32 or not deflate.is_contiguous()):
-        raise ValueError("the deflation vectors are a contiguous FP32 (k, 8, n) tensor")
-    rank = (int(deflate_rank) & 15) | (256 if deflate_restart else 0) | (512 if ritz_norm else 0)
+    if deflate is not None and (deflate.shape not in ((k, 8, n), (k, 12, n)) or deflate.dtype != torch.float32
+                                or not deflate.is_contiguous()):
+        raise ValueError("the deflation vectors are a contiguous FP32 (k, 8, n) or (k, 12, n) tensor")
+    rank = ((int(deflate_rank) & 15) | (256 if deflate_restart else 0) | (512 if ritz_norm else 0)
+            | (1024 if deflate is not None and deflate.shape[1] == 12 else 0))
     for t in (lo_planes, hi_planes):
         if t is not None and (t.shape != (2, k, n, n) or t.dtype != torch.float16 or not t.is_contiguous()):
             raise ValueError("operand planes are a contiguous FP16 (2, k, n, n) tensor")
