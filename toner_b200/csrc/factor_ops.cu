@@ -1026,22 +1026,40 @@ __device__ __forceinline__ double block_dot(const float* x, const float* y, int 
   return block_sum(s, red);
 }
 
+// Sums over the warp of K doubles per lane: at every step of the butterfly a lane keeps the half of its values that its bit of the
+// lane index names and hands over the other, so that K + 31 shuffles do what 5 K did (the same pairs are added, and so the bits).
+// Value i ends up with the lanes whose bits, the highest first, are those of i's place in the halvings; store(i, sum) is called by one.
+template <int kHalf, int kBit, int P>
+__device__ __forceinline__ void warp_fold(double (&v)[P], int lane, int& at) {
+  const bool upper = (lane & kBit) != 0;
+#pragma unroll
+  for (int i = 0; i < kHalf; ++i) {
+    const double keep = upper ? v[i + kHalf] : v[i], give = upper ? v[i] : v[i + kHalf];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, kBit);
+  }
+  at += upper ? kHalf : 0;
+  if constexpr (kBit > 1) warp_fold<kHalf / 2, kBit / 2>(v, lane, at);
+}
+template <int K, typename Store>
+__device__ __forceinline__ void warp_sum_many(const double (&acc)[K], Store store) {
+  constexpr int kPadded = (K + 31) / 32 * 32;
+  const int lane = threadIdx.x & 31;
+  double v[kPadded];
+#pragma unroll
+  for (int i = 0; i < kPadded; ++i) v[i] = i < K ? acc[i] : 0.0;
+  int at = 0;
+  warp_fold<kPadded / 2, 16>(v, lane, at);
+#pragma unroll
+  for (int i = 0; i < kPadded / 32; ++i)
+    if (at + i < K) store(at + i, v[i]);
+}
+
 // Sums over the block of K doubles per thread (256 threads): out[i] holds the total of acc[i] afterwards (shared
 // memory, valid for every thread after the call).  `part` is 8 * K doubles of shared scratch.
 template <int K>
-__device__ __forceinline__ void block_sum_many(double (&acc)[K], double* part, double* out) {
-#pragma unroll
-  for (int i = 0; i < K; ++i) {
-    double x = acc[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    acc[i] = x;
-  }
+__device__ __forceinline__ void block_sum_many(const double (&acc)[K], double* part, double* out) {
   __syncthreads();  // earlier readers of part / out are done
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int i = 0; i < K; ++i) part[(threadIdx.x >> 5) * K + i] = acc[i];
-  }
+  warp_sum_many<K>(acc, [&](int i, double x) { part[(threadIdx.x >> 5) * K + i] = x; });
   __syncthreads();
   if (threadIdx.x < K) {
     double t = 0.0;
@@ -1139,9 +1157,12 @@ __device__ void jacobi_warp(double (*H)[kMaxDeflate], double (*Q)[kMaxDeflate]) 
       const int pp = on ? min(a, b) : 0, qq = on ? max(a, b) : 0;
       const double apq = on ? H[pp][qq] : 0.0;
       double cs = 1.0, sn = 0.0;
-      if (on && apq != 0.0) {
-        const double tau = (H[qq][qq] - H[pp][pp]) / (2.0 * apq);
-        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+      // (The angle in FP32, which leaves 1e-7 of the entry for the next sweep; the rotation itself is orthogonal to FP64.  FP64
+      // divisions and a square root were half of a round's time.)
+      const float twice = 2.f * (float)apq;
+      if (on && twice != 0.f) {
+        const float tau = (float)(H[qq][qq] - H[pp][pp]) / twice;
+        const double t = (double)((tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(1.f + tau * tau)));
         cs = rsqrt(1.0 + t * t);
         sn = t * cs;
       }
@@ -1265,7 +1286,7 @@ __device__ __forceinline__ void cluster_sum_many(double (&acc)[K], double* part,
 // which the fifth direction of spiked:4 was left in one call of four).
 // Three passes over the two blocks of vectors (five from ten vectors on, whose sums are taken for half of the rows at a time);
 // every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
-// vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2; now 17.
+// vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2, with r's 17.
 // A cluster shares a statistic's columns (a few statistics are a few blocks on 148 SMs, and a pass of one block over 3328 columns is
 // thirteen round trips to L2): every CTA factors the small matrix for itself, from the same sums.
 // in_order (one CTA, no sigma): a caller that keeps its order of additions (the plane-by-plane products) has the small
@@ -1448,8 +1469,10 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
   }
   if (!last) cholesky_orthonormalise<R>(Y, V, n, r, gram, L, in_order != 0, first, step);
 }
-// CTAs that share a statistic: as many as have two hundred columns each, eight at most.
-static int ritz_ctas(int n) { return n >= 2048 ? 8 : n >= 1024 ? 4 : n >= 512 ? 2 : 1; }
+// CTAs that share a statistic.  A launch, four statistics of width 768 / 1280 / 3328 / 5632 without a gap in their spectrum, us:  r = 4
+// 15 / 19 / 34 / 52 by one, 13 / 13 / 16 / 23 by eight;  r = 8  42 / 50 / 94 / 171, 31 / 31 / 37 / 49;  r = 11  107 / 129 / 235 / 434,
+// 79 / 80 / 92 / 117.  (Before the sums were folded and the angles taken in FP32, by one: r = 4  17 / 20 / 31 / 61, r = 8  43 / 53 / 91 / 182.)
+static int ritz_ctas(int n) { return n >= 1024 ? 8 : n >= 512 ? 4 : 1; }
 template <int R>
 static cudaError_t launch_ritz(int k, cudaStream_t stream, float* v, float* y, int n, int r, int vstride, int last, float* theta, float* res,
                                int in_order, float trace) {
