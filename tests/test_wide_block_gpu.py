@@ -52,7 +52,7 @@ def test_more_outliers_than_eight(monkeypatch):
     from toner_b200 import core, ops
     from toner_b200.synthetic import fill_rows_spectrum
     n, rows, k = 768, 10001, 2
-    f = core.FactorSet(k, n, torch.device("cuda"), (0.5, 0.125), DAMPING)
+    f = core.FactorSet(k, n, torch.device("cuda"), (0.5, 0.125), DAMPING, slots=12)
     buf = torch.empty(k, rows, n, device="cuda", dtype=torch.bfloat16)
     seen = []
     for step in range(10):
@@ -72,7 +72,7 @@ def test_more_outliers_than_eight(monkeypatch):
 
 def test_plane_order_has_eight_directions():
     from toner_b200 import core, ops
-    f = core.FactorSet(1, 64, torch.device("cuda"), (0.25, 0.25), DAMPING, interleave=False)
+    f = core.FactorSet(1, 64, torch.device("cuda"), (0.25, 0.25), DAMPING, interleave=False, slots=12)
     assert f.deflate.shape[1] == 8
     ema = torch.eye(64, device="cuda").unsqueeze(0)
     with pytest.raises(RuntimeError):

@@ -155,7 +155,7 @@ class FactorSet:
     of the outer factor."""
 
     def __init__(self, k: int, n: int, device: torch.device, strengths: Tuple[float, float], damping: float,
-                 scratch: Optional[Scratch] = None, chunk: Optional[int] = None, interleave: bool = True) -> None:
+                 scratch: Optional[Scratch] = None, chunk: Optional[int] = None, interleave: bool = True, slots: int = 8) -> None:
         if n % 8:
             raise ValueError("statistic width must be a multiple of 8 (TMA row pitch of the 16-bit operands)")
         self.k, self.n, self.device, self.damping = k, n, device, float(damping)
@@ -188,10 +188,10 @@ class FactorSet:
         self.lmin = torch.zeros(k, device=device, dtype=torch.float32)
         self.lmin_host = self._host[2 * k:3 * k].view(torch.float32)
         self.track_restart = True        # the vectors hold nothing yet (or the statistics were replaced)
-        # Dominant directions (outlier features): twelve vector slots per statistic (eight where the plane order is kept, and with it
-        # the bits), found by block power iteration and deflated where they stand out.  The block is two vectors wider than the number of directions that looked like
+        # Dominant directions (outlier features): `slots` vector slots per statistic, eight or twelve (eight where the plane order is
+        # kept, and with it the bits), found by block power iteration and deflated where they stand out.  The block is two vectors wider than the number of directions that looked like
         # outliers last time (a block wider than the group of outliers is what makes close outliers converge).
-        self.deflate = torch.zeros(k, 12 if interleave else 8, n, device=device, dtype=torch.float32)
+        self.deflate = torch.zeros(k, slots if interleave else 8, n, device=device, dtype=torch.float32)
         self.deflated = torch.zeros(k, device=device, dtype=torch.int32)
         self.deflated_host = self._host[3 * k:4 * k]
         self.deflate_rank = 4

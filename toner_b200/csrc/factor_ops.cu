@@ -90,6 +90,8 @@ constexpr int kPromoteSteepX = 2, kPromoteSteepSquares = 1;
 // Products applied to X (and the final squarings) pass their error on linearly: one chain, about 1e-5.
 constexpr int kPromoteX = 0;
 
+constexpr long long kHalfFrom = 4 << 20;   // elements of a stack of statistics from which operand planes are stored by half
+
 // power-iteration steps spent on the dominant direction (each one pass over the statistic)
 constexpr int kPowerSteps = 6;
 
@@ -657,6 +659,7 @@ __global__ void __launch_bounds__(256) damp_kernel(const float* __restrict__ c, 
 // rankr_update_kernel, in its order), so that A' is never written.
 // With m32 M_0 is written there in FP32 (the graded finish, steps with a term linear in M).  With hi_only (the graded finish) its
 // planes -- the hi plane alone -- are those of M_0 + m_diag I.
+// half: of every output only the blocks of 256 x 256 on and above the diagonal are written (and of A read).
 // late (per statistic, optional): where it is not zero the iteration starts with the second step, whose operands l gives.
 struct InitLate {
   float a, b;
@@ -671,7 +674,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* a32, int 
                                                           const float* __restrict__ defl_v,
                                                           const float* __restrict__ defl_coef, int defl_r,
                                                           int vstride, float* m32, float m_diag, bool hi_only,
-                                                          const int* __restrict__ late, InitLate second) {
+                                                          const int* __restrict__ late, InitLate second, bool half) {
   ptx::pdl_begin();
   const int bi = blockIdx.y;
   if (late && late[bi]) {   // (second.m32 may be a32 itself: every element is read before it is written, by one thread)
@@ -699,6 +702,7 @@ __global__ void __launch_bounds__(256) init_planes_kernel(const float* a32, int 
   const int n4 = n / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nn / 4; i += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(i / n4), c = (int)(i - (long long)r * n4) * 4;
+    if (half && (c >> kHalfShift) < (r >> kHalfShift)) continue;
     float4 v = A[i];
     if (any) {
 #pragma unroll
@@ -2193,6 +2197,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     // What the engine starts from: planes of M_0 and of T_0 = a I - b M_0; for a graded finish those of Z
     // in T_0's place, and M_0 in FP32 with the hi plane of M_0 + g I, of which W_K is a multiple
     const bool graded_finish = graded.products > 0;
+    // Operand planes between products are stored by half: writing the mirror images took 4 to 10 % of a product (12 x 3072 in chains
+    // of two, one / two pairs of planes: 948 -> 906 and 1055 -> 958 us; 36 x 768 81 -> 76 and 98 -> 90; a product of the finish, with C,
+    // 12 x 3072 390 -> 348).  On the few matrices of a small step a map more per operand costs the host what it saves.
+    const bool half = (long long)kc * nn >= kHalfFrom;
     const double top_gain = graded.products ? graded.beta[graded.products] * graded.za : 1.0;
     const double top_diag =
         graded.products ? (graded.alpha[graded.products] + graded.beta[graded.products] * graded.zb) / top_gain : 0.0;
@@ -2213,10 +2221,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       // Neither A' nor its Frobenius norm is formed: the norm is the estimate (capped by the trace), and the planes of
       // M_0 and T_0 are made from A with the deflation applied on the way.
       TONER_LAUNCH(ritz_norm_kernel, (kc + 127) / 128, 128, stream, sumsq_a, rest_top, rest_trace, kc);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, slots, m32, init_diag, graded_finish, nullptr, InitLate());
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, dv, coef8, defl_r, slots, m32, init_diag, graded_finish, nullptr, InitLate(), half);
       TONER_CUDA(cudaGetLastError());
     } else {
-    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false, nullptr, InitLate());
+    TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, 0.f, 0.f, s_m, s_t, Mb[0], nullptr, nullptr, nullptr, 0, 0, nullptr, 0.f, false, nullptr, InitLate(), half);
     TONER_CUDA(cudaGetLastError());
     {
       // A tighter bound of the largest eigenvalue than ||A'||_F: with P = A' / ||A'||_F, lambda_max(P) <= ||P^2||_F^(1/2)
@@ -2237,7 +2245,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g.alpha = (float)(1.0 / ((double)s_m * (double)s_m));
       g.d = P2; g.ldd = n; g.d_bs = nn;
       g.split0 = Pb[1]; g.split0_scale = s_w; g.split_ld = n; g.split_bs = nn; g.split_plane = (long long)kc * nn;
-      int rc1 = launch_gemm(g, stream);
+      GemmMore planes;
+      planes.half_in = planes.half_out = half;
+      int rc1 = launch_gemm(g, stream, planes);
       if (rc1) return rc1;
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss2, stream);
       if (rc1) return rc1;
@@ -2246,19 +2256,19 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g4.a.base = Pb[1]; g4.b.base = Pb[1];
       g4.alpha = (float)(1.0 / ((double)s_w * (double)s_w));
       g4.d = P4; g4.split0 = Mb[1];
-      rc1 = launch_gemm(g4, stream);
+      rc1 = launch_gemm(g4, stream, planes);
       if (rc1) return rc1;
       rc1 = sumsq_det(P4, kc, n, n, n, nn, partials, ss4, stream);
       if (rc1) return rc1;
       toner_gemm_desc g8 = g4;
       g8.a.base = Mb[1]; g8.b.base = Mb[1];
       g8.d = P2; g8.split0 = nullptr;
-      rc1 = launch_gemm(g8, stream);
+      rc1 = launch_gemm(g8, stream, planes);
       if (rc1) return rc1;
       rc1 = sumsq_det(P2, kc, n, n, n, nn, partials, ss8, stream);
       if (rc1) return rc1;
       TONER_LAUNCH(tighten_bound_kernel, (kc + 127) / 128, 128, stream, sumsq_a, ss2, ss4, ss8, kc, late, (float)(1.0001 * plan.late), damping);
-      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, nullptr, nullptr, 0, 0, m32, init_diag, graded_finish, late, second);
+      TONER_LAUNCH(init_planes_kernel, dim3(ew_blocks, kc), 256, stream, A32, n, kc, sumsq_a, init_a, init_b, init_sm, s_t, Mb[0], first_planes, nullptr, nullptr, 0, 0, m32, init_diag, graded_finish, late, second, half);
       TONER_CUDA(cudaGetLastError());
     }
     }
@@ -2281,6 +2291,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       double gain = 1.0;
       int segs = 3;                                // 1: hi planes only (a single pass)
       bool upper_d = false;                        // d is read as a product's C alone, which takes its upper triangle
+      bool whole_in = false, whole_out = false;    // operands, planes of the result that are stored whole
     };
     // (in_step: matrices between the hi and lo planes of the operands; 0: the chunk's)
     auto sym_product = [&](const __half* ap, float sa, const __half* bp, float sb, const Out& o, int promote, int in_step = 0, const int* skip = nullptr) -> int {
@@ -2305,7 +2316,11 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       g.maxres = o.maxres;
       g.promote = promote;
       g.interleave = interleave ? 1 : 0;
-      return launch_gemm(g, stream, skip);
+      GemmMore more;
+      more.skip = skip;
+      more.half_in = half && !o.whole_in;
+      more.half_out = half && !o.whole_out;
+      return launch_gemm(g, stream, more);
     };
     int rc = 0;
     // the finish in steps of Y; its planes of R + beta I go where the powers of T leave room (p = 1 has no such buffer)
@@ -2586,8 +2601,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         Out o;
         if (first) {
           o.alpha_a = o.alpha_b = lo_planes ? lo_inv + k0 : inv_r;
+          o.whole_in = true;   // (root_finish_kernel's planes)
         }
         if (have == q) {
+          o.whole_out = true;
           o.d = root_hi + (long long)k0 * nn;
           if (hi_planes) {
             o.s0 = static_cast<__half*>(hi_planes) + (long long)k0 * nn;

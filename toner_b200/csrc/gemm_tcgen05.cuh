@@ -91,12 +91,18 @@ struct GemmParams {
   __half* S1;
   long long s_ld, s_bs, s_plane;
   float s0_scale, s0_aff_a, s1_scale, s1_aff_a, s1_aff_b;
+  // Symmetric matrices of which only the 256 x 256 blocks on and above the diagonal are stored, these whole.  Both operands (kernels
+  // with kHalf): a k-block left of an operand's rows' own block is read from its mirror image, MN-major, through the *_turned maps
+  // (64 x 64 boxes).  half_out: the operand planes S0 and S1.
+  int half_out;
   const int* skip;   // optional, per batch: not zero where the product is left out (its outputs keep what they hold)
   int* status;  // set non-zero if a bounded wait ran out
   unsigned long long* prof;  // optional: eight cycle counters summed over CTAs (see toner_gemm_phase_cycles)
   // 32 x 32 boxes of C and of the outputs, (columns, rows, batch): FP32 with 128-byte, 16-bit with 64-byte swizzle
   CUtensorMap c_map, d_map, h_map, s0_map, s1_map;
+  CUtensorMap a_turned, b_turned;
 };
+constexpr int kHalfShift = 8;   // log2 of the blocks of half-stored matrices: tiles of every size lie in one of them
 
 __host__ __device__ inline long long packed_off(long long r, long long c, long long n) {
   return r * n - r * (r + 1) / 2 + c;
@@ -373,7 +379,7 @@ __device__ __forceinline__ void epilogue_block(const GemmParams& p, const Epilog
       ptx::tma_store_3d(map, buf, c0, row_first, b);
       ptx::tma_store_3d(map, buf + kEpiBlockBytes / 2, c0, row_first, b + p.s_lo_z);
     });
-    if (image) {
+    if (image && !(p.half_out && (c0 >> kHalfShift) != (row_first >> kHalfShift))) {
       const uint32_t tb = take();
       stage_cols_16(tb, lane, hi);
       stage_cols_16(tb + kEpiBlockBytes / 2, lane, lo);
@@ -471,7 +477,7 @@ __device__ __forceinline__ void epilogue_block_scalar(const GemmParams& p, const
 // against FP64 at 2048^3, chains of 2 plane by plane and interleaved 4.1e-7; of 8 plane by plane 2.4e-6, of 5 interleaved
 // 1.9e-6 (random signs 3.4e-7, 1.5e-6 and 1.4e-6); one chain 1.8e-5 and 1.5e-5.  (GemmParams::segs
 // is 1 here: the three products are one.)
-template <int BN, bool kChained, bool kPair = false, bool kInter = false>
+template <int BN, bool kChained, bool kPair = false, bool kInter = false, bool kHalf = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, kPair, kInter>;
   static_assert(!kInter || (kPair && BN <= 256), "interleaved plane products: 256 x 256 or 256 x 128 on pairs");
@@ -619,21 +625,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
         int b, tm, tn;
         tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
         if (left_out(b)) continue;
-        const CUtensorMap* amap = &p.a_map;
-        const CUtensorMap* bmap = &p.b_map;
-        if (p.a_maps) {
-          amap = p.a_maps + b;
-          ptx::fence_tensormap_acquire(amap);
-        }
-        if (p.b_maps) {
-          bmap = p.b_maps + b;
-          ptx::fence_tensormap_acquire(bmap);
+        const CUtensorMap* map = for_a ? &p.a_map : &p.b_map;
+        if (for_a ? p.a_maps != nullptr : p.b_maps != nullptr) {
+          map = (for_a ? p.a_maps : p.b_maps) + b;
+          ptx::fence_tensormap_acquire(map);
         }
         // a pair splits the tile's rows (A) and its columns (B) between its two CTAs
-        // (of a wide tile each CTA holds 128 columns of either 256-column half: n0 is its share of the first half)
-        const int m0 = tm * TM + (int)cta_rank * kBM, n0 = tn * BN + (int)cta_rank * (kWide ? BNI / 2 : S::kBRows);
-        // fill the next stage with k-block k0 of planes za / zb
-        auto fill = [&](int k0, int za, int zb) {
+        // (of a wide tile each CTA holds 128 columns of either 256-column half: r0 is its share of the first half)
+        const int r0 = for_a ? tm * TM + (int)cta_rank * kBM : tn * BN + (int)cta_rank * (kWide ? BNI / 2 : S::kBRows);
+        // fill this operand's part of the next stage with k-block k0 of plane z
+        auto fill = [&](int k0, int z) {
           const long long w0 = p.prof ? clock64() : 0;
           const bool got = ptx::mbar_wait_unless(empty_bar(stage), phase ^ 1u, kWaitCycles, abort_flag);
           if (p.prof) prof_wait += clock64() - w0;
@@ -643,47 +644,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
             ok = false;
             return;
           }
-          const uint32_t sa = base + stage * S::kStageBytes;
-          const uint32_t sb = sa + S::kABytes;
+          const uint32_t dst = base + stage * S::kStageBytes + (for_a ? 0 : S::kABytes);
+          uint32_t bar = full_bar(stage);
           if constexpr (kPair) {
             // Both CTAs' copies report to the leader's barrier, which expects the bytes of the whole pair.
-            const uint32_t lbar = ptx::mapa(full_bar(stage), 0);
-            if (for_a) {
-              if (leader) ptx::mbar_expect_tx(full_bar(stage), 2 * S::kStageBytes);
-              if (p.a_mn) {
-#pragma unroll
-                for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d_pair(sa + s * 8192, amap, lbar, m0 + s * 64, k0, za);
-              } else {
-                ptx::tma_load_3d_pair(sa, amap, lbar, k0, m0, za);
-              }
-            } else if constexpr (kWide) {
-              if (p.b_mn) {
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                  ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + (s >> 1) * BNI + (s & 1) * 64, k0, zb);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 2; ++j) ptx::tma_load_3d_pair(sb + j * 16384, bmap, lbar, k0, n0 + j * BNI, zb);
-              }
-            } else if (p.b_mn) {
-#pragma unroll
-              for (int s = 0; s < S::kBRows / 64; ++s) ptx::tma_load_3d_pair(sb + s * 8192, bmap, lbar, n0 + s * 64, k0, zb);
-            } else {
-              ptx::tma_load_3d_pair(sb, bmap, lbar, k0, n0, zb);
-            }
+            if (for_a && leader) ptx::mbar_expect_tx(bar, 2 * S::kStageBytes);
+            bar = ptx::mapa(bar, 0);
           } else if (for_a) {
-            ptx::mbar_expect_tx(full_bar(stage), S::kStageBytes);
-            if (p.a_mn) {
-#pragma unroll
-              for (int s = 0; s < kBM / 64; ++s) ptx::tma_load_3d(sa + s * 8192, amap, full_bar(stage), m0 + s * 64, k0, za);
+            ptx::mbar_expect_tx(bar, S::kStageBytes);
+          }
+          auto copy = [&](uint32_t to, const CUtensorMap* from, int x, int y) {
+            if constexpr (kPair) ptx::tma_load_3d_pair(to, from, bar, x, y, z);
+            else ptx::tma_load_3d(to, from, bar, x, y, z);
+          };
+          // `slabs` times 64 rows from r on: stored MN-major, the mirror image of a half-stored operand's, or K-major
+          auto rows = [&](uint32_t to, int r, int slabs) {
+            const bool image = kHalf && (k0 >> kHalfShift) < (r >> kHalfShift);
+            if (image || (for_a ? p.a_mn : p.b_mn)) {
+              const CUtensorMap* const from = image ? (for_a ? &p.a_turned : &p.b_turned) : map;
+              for (int s = 0; s < slabs; ++s) copy(to + s * 8192, from, r + s * 64, k0);
             } else {
-              ptx::tma_load_3d(sa, amap, full_bar(stage), k0, m0, za);
+              copy(to, map, k0, r);
             }
-          } else if (p.b_mn) {
-#pragma unroll
-            for (int s = 0; s < BN / 64; ++s) ptx::tma_load_3d(sb + s * 8192, bmap, full_bar(stage), n0 + s * 64, k0, zb);
+          };
+          if constexpr (kWide) {
+            rows(dst, r0, 2);
+            if (!for_a) rows(dst + 16384, r0 + BNI, 2);
           } else {
-            ptx::tma_load_3d(sb, bmap, full_bar(stage), k0, n0, zb);
+            rows(dst, r0, for_a ? kBM / 64 : (kPair ? S::kBRows : BN) / 64);
           }
           if (++stage == S::kStages) {
             stage = 0;
@@ -691,18 +679,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           }
         };
         if constexpr (kInter) {
-          const int za = b * p.a_z_stride, zb = b * p.b_z_stride;
+          const int z = b * (for_a ? p.a_z_stride : p.b_z_stride);
+          const int z_lo = z + (for_a ? p.a_seg_z[2] : p.b_seg_z[1]), z_hi = z + (for_a ? p.a_seg_z[0] : p.b_seg_z[0]);
           for (int kb = w.kb_lo; kb < w.kb_hi && ok; ++kb) {
-            fill(kb * kBK, za + p.a_seg_z[2], zb + p.b_seg_z[1]);
-            if (ok) fill(kb * kBK, za + p.a_seg_z[0], zb + p.b_seg_z[0]);
+            fill(kb * kBK, z_lo);
+            if (ok) fill(kb * kBK, z_hi);
           }
         } else {
           for (int kb = w.kb_lo; kb < w.kb_hi && ok;) {
             const int si = kb / kb_per_seg, seg_end = min(w.kb_hi, (si + 1) * kb_per_seg);
             const int seg = rest_first ? (si + 1 == p.segs ? 0 : si + 1) : si;
-            const int za = b * p.a_z_stride + p.a_seg_z[seg];
-            const int zb = b * p.b_z_stride + p.b_seg_z[seg];
-            for (; kb < seg_end && ok; ++kb) fill((kb - si * kb_per_seg) * kBK, za, zb);
+            const int z = for_a ? b * p.a_z_stride + p.a_seg_z[seg] : b * p.b_z_stride + p.b_seg_z[seg];
+            for (; kb < seg_end && ok; ++kb) fill((kb - si * kb_per_seg) * kBK, z);
           }
         }
       }
@@ -730,15 +718,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
     // while waiting.  8192^3 775 -> 627 cycles a k-block, 541 with five stages: 838 -> 726 us (power-capped; zeros, which draw
     // little power, 770 -> 572 us).
     if (leader && ptx::elect_one()) {
-      const uint32_t idesc = (1u << 4) | ((uint32_t)p.fmt << 7) | ((uint32_t)p.fmt << 10) | ((uint32_t)p.a_mn << 15) |
-                             ((uint32_t)p.b_mn << 16) | ((uint32_t)(BNI >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+      const uint32_t idesc_k = (1u << 4) | ((uint32_t)p.fmt << 7) | ((uint32_t)p.fmt << 10) | ((uint32_t)(BNI >> 3) << 17) |
+                               ((uint32_t)(TM >> 4) << 24);
       // K-major: 8-row groups 1024 B apart, k advances 32 B inside the swizzled row.
       // MN-major: 64-element slabs 8192 B apart (LBO), 8-k-row groups 1024 B apart (SBO), k advances 16 rows = 2048 B.
       // The descriptor's upper word (8-row groups 1024 B apart, version, 128-byte swizzle) never changes; the lower
       // word is the address in 16-byte units plus the leading-dimension offset, so a k-step is an addition.
       const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-      const uint32_t a_lo_const = ((p.a_mn ? 8192u : 16u) >> 4) << 16, b_lo_const = ((p.b_mn ? 8192u : 16u) >> 4) << 16;
-      const uint32_t a_step16 = (p.a_mn ? 2048u : 32u) >> 4, b_step16 = (p.b_mn ? 2048u : 32u) >> 4;
+      // Which operands of a k-block are MN-major (of a wide tile, the halves of B): those that are stored so, and of half-stored ones
+      // the mirror images.  What follows from it is kept, not worked out for every k-block: that cost Newton-Schulz 1.4 %.
+      uint32_t a_lo_const, a_step16, b_lo_const[kWide ? 2 : 1], b_step16[kWide ? 2 : 1], idesc[kWide ? 2 : 1];
+      auto orient = [&](bool a_mn, bool b_mn, int j) {
+        a_lo_const = (a_mn ? 512u : 1u) << 16;
+        a_step16 = a_mn ? 128u : 2u;
+        b_lo_const[j] = (b_mn ? 512u : 1u) << 16;
+        b_step16[j] = b_mn ? 128u : 2u;
+        idesc[j] = idesc_k | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
+      };
+#pragma unroll
+      for (int j = 0; j < (kWide ? 2 : 1); ++j) orient(p.a_mn != 0, p.b_mn != 0, j);
       int stage = 0;
       uint32_t phase = 0;
       uint32_t gchunk = 0;  // accumulator hand-offs so far; buffer = gchunk & 1
@@ -748,6 +746,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
       for (int u = unit; u < total_units && ok; u += units) {
         const Unit w = unit_of(u);
         if (left_out(w.tile / tiles_per_batch)) continue;
+        int a_block = 0, b_block = 0;   // blocks of half-stored operands that the tile's rows of A and of B lie in
+        if constexpr (kHalf) {
+          int b, tm, tn;
+          tile_coord(p, BN, TM, w.tile, tiles_per_batch, tiles_n, b, tm, tn);
+          a_block = (tm * TM) >> kHalfShift;
+          b_block = (tn * BN) >> kHalfShift;
+        }
+        auto turn = [&](int kb) {   // (k-blocks in processing order: every segment goes through all of them)
+          if (!kHalf) return;
+          if (!kInter) {
+            if (kb >= kb_per_seg) kb -= kb_per_seg;
+            if (kb >= kb_per_seg) kb -= kb_per_seg;
+          }
+          const int block = (kb * kBK) >> kHalfShift;
+#pragma unroll
+          for (int j = 0; j < (kWide ? 2 : 1); ++j) orient(block < a_block, block < b_block + j, j);
+        };
         for (int ch = w.ch_lo; ch < w.ch_hi && ok; ++ch, ++gchunk) {
           int kb_begin = w.kb_lo, kb_end = w.kb_hi;
           if (p.promote > 0) chunk_range(ch, kb_begin, kb_end);
@@ -786,13 +801,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
           // the MMAs of one k-block (columns from 256 * j on), A from stage address sa, B from sb
           auto multiply = [&](uint32_t sa, uint32_t sb, int j, uint32_t fresh) {
             const uint32_t a_lo = ((sa & 0x3FFFFu) >> 4) | a_lo_const;
-            const uint32_t b_lo = (((sb + S::kABytes) & 0x3FFFFu) >> 4) | b_lo_const;
+            const uint32_t b_lo = (((sb + S::kABytes) & 0x3FFFFu) >> 4) | b_lo_const[j];
 #pragma unroll
             for (int k = 0; k < kBK / kUmmaK; ++k) {
               const uint64_t da = ((uint64_t)desc_hi << 32) | (a_lo + k * a_step16);
-              const uint64_t db = ((uint64_t)desc_hi << 32) | (b_lo + j * ((BNI / 2) * kBK * 2 / 16) + k * b_step16);
-              if constexpr (kPair) ptx::mma_f16_pair(d_tmem + j * BNI, da, db, idesc, k != 0 ? 1u : fresh);
-              else ptx::mma_f16(d_tmem, da, db, idesc, k != 0 ? 1u : fresh);
+              const uint64_t db = ((uint64_t)desc_hi << 32) | (b_lo + j * ((BNI / 2) * kBK * 2 / 16) + k * b_step16[j]);
+              if constexpr (kPair) ptx::mma_f16_pair(d_tmem + j * BNI, da, db, idesc[j], k != 0 ? 1u : fresh);
+              else ptx::mma_f16(d_tmem, da, db, idesc[j], k != 0 ? 1u : fresh);
             }
           };
           auto release_stage = [&](int st) {  // frees the stage (in both CTAs of a pair) once the MMAs so far have read it
@@ -826,6 +841,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
               int s_lo, s_hi, s_lo1, s_hi1 = 0;
               const uint32_t lo = next_operands(s_lo), hi = ok ? next_operands(s_hi) : 0u;
               if (!ok) break;
+              turn(kb);   // (two k-blocks from an even one on lie in one block of 256)
               multiply(hi, lo, 0, kb != kb_begin ? 1u : 0u);   // Ah Bl
               multiply(lo, hi, 0, 1u);                         // Al Bh
               release_stage(s_lo);
@@ -851,6 +867,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
               int st;
               const uint32_t at = next_operands(st);
               if (!ok) break;
+              turn(kb);
               multiply(at, at, 0, fresh);
               if constexpr (kWide) {
                 if (kb == kb_begin && !wait_drained(1)) break;

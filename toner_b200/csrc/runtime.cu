@@ -101,6 +101,15 @@ Context* context() {
   allow(gemm_tcgen05_kernel<128, true>, GemmSmem<128>::kTotal);
   allow(gemm_tcgen05_kernel<256, false>, GemmSmem<256>::kTotal);
   allow(gemm_tcgen05_kernel<256, true>, GemmSmem<256>::kTotal);
+  allow(gemm_tcgen05_kernel<128, false, true, false, true>, GemmSmem<128, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, true, true, false, true>, GemmSmem<128, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, false, true, false, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, true, true, false, true>, GemmSmem<256, true>::kTotal);
+  allow(gemm_tcgen05_kernel<512, false, true, false, true>, GemmSmem<512, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, false, true, true, true>, GemmSmem<128, true, true>::kTotal);
+  allow(gemm_tcgen05_kernel<128, true, true, true, true>, GemmSmem<128, true, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, false, true, true, true>, GemmSmem<256, true, true>::kTotal);
+  allow(gemm_tcgen05_kernel<256, true, true, true, true>, GemmSmem<256, true, true>::kTotal);
   allow(gemm_tcgen05_kernel<128, false, true>, GemmSmem<128, true>::kTotal);
   allow(gemm_tcgen05_kernel<128, true, true>, GemmSmem<128, true>::kTotal);
   allow(gemm_tcgen05_kernel<256, false, true>, GemmSmem<256, true>::kTotal);
@@ -375,7 +384,7 @@ static int gemm_params(Context* ctx, const toner_gemm_desc& d, int bn, bool pair
   return 0;
 }
 
-int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const int* skip) {
+int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const GemmMore& more) {
   Context* ctx = context();
   if (!ctx) return kErrCuda;
   if (d.m <= 0 || d.n <= 0 || d.k <= 0 || d.batch <= 0) return fail(kErrArg, "gemm: sizes must be positive");
@@ -409,18 +418,33 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const int* skip) 
     return fail(kErrArg, "gemm: tile_n must be 0, 64, 128, 256, -128 (256 x 128 on a CTA pair), 512 (256 x 256 on a pair) or 1024 "
                          "(256 x 512 on a pair)");
 
+  if (more.half_in && !pair) {   // (large stacks: pair tiles, of which alone there are kernels for it)
+    bn = 128;
+    pair = true;
+    splits = 1;
+  }
   const bool inter = pair && bn <= 256 && may_interleave(d);
   GemmParams p;
   if (int rc = gemm_params(ctx, d, bn, pair, splits, inter, stream, p)) return rc;
-  p.skip = skip;
+  p.skip = more.skip;
+  p.half_out = more.half_out ? 1 : 0;
+  if (more.half_in) {
+    if (d.a.list || d.b.list || d.a.mn_major || d.b.mn_major) return fail(kErrArg, "gemm: half-stored operands are K-major stacks");
+    int rc = encode_one(&p.a_turned, d.a.base, d.a.rows, d.a.cols, d.a.ld, d.a.z_stride, d.a.nz, 64);
+    if (rc) return rc;
+    if (d.b.base == d.a.base) p.b_turned = p.a_turned;
+    else rc = encode_one(&p.b_turned, d.b.base, d.b.rows, d.b.cols, d.b.ld, d.b.z_stride, d.b.nz, 64);
+    if (rc) return rc;
+  }
 
   const long long total = gemm_tiles(d, bn, pair) * splits;
   if (total > 0x7fffffffLL) return fail(kErrArg, "gemm: too many tiles");
   const bool chained = p.promote > 0;
   const int workers = pair ? ctx->gemm_sms / 2 : ctx->gemm_sms;
   const int grid = (int)(total < workers ? total : workers) * (pair ? 2 : 1);
-#define TONER_INTER(BN, CHAINED)                                                                                           \
-  TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, true, true>, grid, kGemmThreads, GemmSmem<BN, true, true>::kTotal, stream, 2, p))
+#define TONER_INTER(BN, CHAINED)                                                                                                        \
+  TONER_CUDA(launch(more.half_in ? gemm_tcgen05_kernel<BN, CHAINED, true, true, true> : gemm_tcgen05_kernel<BN, CHAINED, true, true>, grid, \
+                    kGemmThreads, GemmSmem<BN, true, true>::kTotal, stream, 2, p))
   if (inter) {
     if (bn == 256 && chained) TONER_INTER(256, true);
     else if (bn == 256) TONER_INTER(256, false);
@@ -429,8 +453,9 @@ int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const int* skip) 
     return 0;
   }
 #undef TONER_INTER
-#define TONER_GEMM(BN, CHAINED, PAIR)                                                                                       \
-  TONER_CUDA(launch(gemm_tcgen05_kernel<BN, CHAINED, PAIR>, grid, kGemmThreads, GemmSmem<BN, PAIR>::kTotal, stream, PAIR ? 2 : 0, p))
+#define TONER_GEMM(BN, CHAINED, PAIR)                                                                                                  \
+  TONER_CUDA(launch(PAIR && more.half_in ? gemm_tcgen05_kernel<BN, CHAINED, PAIR, false, PAIR> : gemm_tcgen05_kernel<BN, CHAINED, PAIR>, \
+                    grid, kGemmThreads, GemmSmem<BN, PAIR>::kTotal, stream, PAIR ? 2 : 0, p))
   if (pair && bn == 512) TONER_GEMM(512, false, true);
   else if (pair && bn == 256 && chained) TONER_GEMM(256, true, true);
   else if (pair && bn == 256) TONER_GEMM(256, false, true);

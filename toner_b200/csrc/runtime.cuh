@@ -82,8 +82,13 @@ Context* context();
 // operands always use 64 x 64 boxes.
 int get_maps(Context* ctx, const toner_operand& op, int batch, int box_rows, cudaStream_t stream, const CUtensorMap** out);
 
-// skip: optional, per batch (device memory): the product is left out where it is not zero.
-int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const int* skip = nullptr);
+// skip: optional, per batch (device memory): the product is left out where it is not zero.  half_in, half_out: both operands, and
+// the operand planes of the result, are symmetric matrices of which only the 256 x 256 blocks on and above the diagonal are stored.
+struct GemmMore {
+  const int* skip = nullptr;
+  bool half_in = false, half_out = false;
+};
+int launch_gemm(const toner_gemm_desc& d, cudaStream_t stream, const GemmMore& more = GemmMore());
 // The products of a whole polar iteration (Gram of either operand copy, polynomial, update either way and the last one) in one
 // launch; claim and done[batch] are zero when it starts.  in_step: the host has launches of its own to make meanwhile.
 // *taken = false: not done, the products are to be launched one by one.

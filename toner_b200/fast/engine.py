@@ -107,7 +107,7 @@ class StatGroup:
         self.tri = n * (n + 1) // 2
         # one stacked row buffer: statistic s of this rank's tokens is rows_buf[s]
         self.rows_buf = torch.empty(self.k_all, rows, n, device=device, dtype=torch.bfloat16)
-        self.factors = core.FactorSet(per_rank, n, device, strengths, damping, scratch, interleave=interleave)
+        self.factors = core.FactorSet(per_rank, n, device, strengths, damping, scratch, interleave=interleave, slots=12)
         self.partial: Optional[torch.Tensor] = None   # (chunks, world, cs, tri) packed partial Grams (world > 1)
         self.summed: Optional[torch.Tensor] = None    # (per, tri) summed Grams of the owned statistics
         self.chunk_stats = per_rank

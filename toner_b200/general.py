@@ -71,7 +71,7 @@ class _Bucket:
         self.params, self.lane = params, lane
         n = params[0].shape[1]
         self.factors = core.FactorSet(len(params), n, params[0].device, strengths, damping, scratch,
-                                      interleave=core.may_reorder(kind))
+                                      interleave=core.may_reorder(kind), slots=12)
         self.group = core.MatrixGroup(params, self.factors, 0, 1, kind)
         self.delta = torch.empty_like(self.group.m)
         self.index = {p: i for i, p in enumerate(params)}
