@@ -658,20 +658,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tcgen05_kernel(const __g
             else ptx::tma_load_3d(to, from, bar, x, y, z);
           };
           // `slabs` times 64 rows from r on: stored MN-major, the mirror image of a half-stored operand's, or K-major
-          auto rows = [&](uint32_t to, int r, int slabs) {
+          auto rows = [&](uint32_t to, int r, auto slabs) {
             const bool image = kHalf && (k0 >> kHalfShift) < (r >> kHalfShift);
             if (image || (for_a ? p.a_mn : p.b_mn)) {
               const CUtensorMap* const from = image ? (for_a ? &p.a_turned : &p.b_turned) : map;
-              for (int s = 0; s < slabs; ++s) copy(to + s * 8192, from, r + s * 64, k0);
+#pragma unroll
+              for (int s = 0; s < decltype(slabs)::value; ++s) copy(to + s * 8192, from, r + s * 64, k0);
             } else {
               copy(to, map, k0, r);
             }
           };
-          if constexpr (kWide) {
-            rows(dst, r0, 2);
-            if (!for_a) rows(dst + 16384, r0 + BNI, 2);
+          constexpr std::integral_constant<int, kBM / 64> kOfA;
+          constexpr std::integral_constant<int, (kWide ? 128 : kPair ? S::kBRows : BN) / 64> kOfB;
+          if (for_a) {
+            rows(dst, r0, kOfA);
           } else {
-            rows(dst, r0, for_a ? kBM / 64 : (kPair ? S::kBRows : BN) / 64);
+            rows(dst, r0, kOfB);
+            if constexpr (kWide) rows(dst + 16384, r0 + BNI, kOfB);
           }
           if (++stage == S::kStages) {
             stage = 0;
