@@ -10,7 +10,7 @@ def _take(s, lam, steps, p):
     for degree, zb, za, kappa, top, lin, con in steps:
         z = zb + za * mu
         t = con + lin * mu + top * {1: 0.0, 2: z ** 2, 4: (z ** 2 + kappa) ** 2}[degree]
-        assert t.min() > 0 and (t.max() / t.min()) ** p < 1.05e3
+        assert t.min() > 0 and (t.max() / t.min()) ** p < 1.05 * (1e3 if degree == 1 else min(400.0, 6.25 * p * p))
         x, mu = x * t, mu * t ** p
         assert mu.max() < 1.0 + 1e-6, (p, lam[0], mu.max())
     assert 1.0 - mu.min() <= s["distance"] + 1e-9, (p, lam[0])
@@ -20,11 +20,11 @@ def _take(s, lam, steps, p):
 
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("n", [264, 768, 3072])
-@pytest.mark.parametrize("p", [2, 4, 8, 16, 32])
+@pytest.mark.parametrize("p", [4, 8, 16, 32])
 def test_the_stated_steps_take_every_eigenvalue_to_its_root(p, n, kind):
     """x = 1, mu = lambda; t = T(mu), x *= t, mu *= t^p per step; then x q(1 - mu) must be lambda^(-1/p) for every lambda the
     bound allows.  mu stays at 1 or below, ends within the stated distance of 1, T^p
-    keeps the dynamic range its operand planes resolve (1e3, the grid's miss beside it), and products are saved."""
+    keeps the dynamic range its products may have (5 % for what the grid misses), and products are saved."""
     from toner_b200 import ops
     used = 0
     for lower in np.geomspace(1.5e-7, 0.3, 60):
@@ -44,7 +44,7 @@ def test_the_stated_steps_take_every_eigenvalue_to_its_root(p, n, kind):
 
 
 @pytest.mark.parametrize("n", [256, 512, 776, 2048, 5632, 16384])
-@pytest.mark.parametrize("p", [2, 4, 8, 16, 32])
+@pytest.mark.parametrize("p", [4, 8, 16, 32])
 def test_the_bound_that_always_holds_with_and_without_its_first_step(p, n):
     """All steps for a spectrum down to damping / n, the steps from the second on for one down to the stated bound, which a norm of
     16 puts every spectrum above where one step of degree four gets that far."""
@@ -57,3 +57,9 @@ def test_the_bound_that_always_holds_with_and_without_its_first_step(p, n):
         assert s["steps"][1][0] > 1 and s["late"] <= 1e-3 / 16
         _take(s, lam(s["late"]), s["steps"][1:], p)
     assert s["late"] > 0 or p not in (4, 8) or n == 16384     # (not where the second step would be a linear one)
+
+
+def test_square_roots_and_narrow_statistics_keep_linear_steps():
+    from toner_b200 import ops
+    for lower in np.geomspace(1.5e-7, 0.3, 60):
+        assert all(ops.inv_roots_steps(float(lower), p, n, kind) is None for p, n in ((1, 768), (2, 768), (8, 248)) for kind in range(3))

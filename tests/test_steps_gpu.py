@@ -28,7 +28,7 @@ def _statistics(n, cond, k=2):
 @pytest.mark.parametrize("p,q", [(2, 1), (4, 1), (8, 4), (8, 1), (16, 8), (32, 2)])
 def test_every_path_of_steps(ops, p, q, n):
     """Bounds from the one that always holds to the spectrum's own end take schedules of every degree, first and later, with
-    every kind of finish.  Linear steps are what calls in plane order take, and all calls below 256 columns.  Measured, the errors
+    every kind of finish.  Linear steps are what calls in plane order take, all calls below 256 columns and square roots.  Measured, the errors
     are 0.4 times theirs in the median and 1.2 times in the worst (p = 16); 1e-6 q for the operand planes' rounding,
     2^-22 of norms up to four times the root's, the q-th power of it."""
     stats = _statistics(n, 300.0)
@@ -61,7 +61,37 @@ def test_every_path_of_steps(ops, p, q, n):
         half = len(errors) // 2
         for got, linear in zip(errors[:half], errors[half:]):
             assert got <= 1.2 * linear + 1e-6 * q, (k, degrees, got, linear)
-    assert not first if n < 256 else (4 in first and later), (first, later)
+    assert not first if n < 256 or p < 4 else (4 in first and later), (first, later)
+
+
+@pytest.mark.parametrize("p,q", [(4, 1), (8, 4), (16, 8)])
+@pytest.mark.parametrize("n,rows", [(256, 0.1), (512, 0.17), (768, 0.9), (1280, 0.5)])
+def test_directions_the_statistic_is_large_in(ops, p, q, n, rows):
+    """Fewer rows than columns, the bound that always holds, the norm's and the spectrum's own: errors weighted by the statistic
+    (what a gradient of such activations sees), which the small eigenvalues' share of the Frobenius norm hides.  Measured 0.3 to
+    0.6 of the linear steps' in the mean and 1.02 in the worst (p = 8); 1.2 for another draw's rounding."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(2, int(n * rows), n, device="cuda", generator=g) + 0.3 * torch.randn(2, 1, n, device="cuda", generator=g)
+    c = x.mT @ x
+    c = (0.5 * (c + c.mT)).contiguous()
+    a = c.double() / c.double().diagonal(dim1=1, dim2=2).mean(1)[:, None, None]
+    lam, vec = torch.linalg.eigh(a + DAMPING * torch.eye(n, device="cuda", dtype=torch.float64))
+    norms = torch.zeros(2, device="cuda")
+    ops.inv_roots(c, DAMPING, p, q, norms=norms)
+    for lower in (0.0, 0.6 * DAMPING / float(norms.max()), 0.5 * float((lam[:, 0] / norms.double()).min())):
+        weighted = []
+        for interleave in (True, False):
+            lo, hi, _, st = ops.inv_roots(c, DAMPING, p, q, lower=lower, interleave=interleave)
+            ops.assert_healthy()
+            assert st.tolist() == [0, 0]
+            for root, s in ((lo, 1.0 / p), (hi, q / p)):
+                if root is not None:
+                    want = (vec * lam.pow(-s)[:, None, :]) @ vec.mT
+                    d = root.double() - want
+                    of = lambda m: (m @ a @ m).diagonal(dim1=1, dim2=2).sum(1)
+                    weighted.append(float((of(d) / of(want)).max().sqrt()))
+        half = len(weighted) // 2
+        assert all(got <= 1.2 * linear for got, linear in zip(weighted[:half], weighted[half:])), (lower, weighted)
 
 
 def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops):

@@ -394,6 +394,16 @@ constexpr int kBoundsPerOctave = 8, kBounds = 32 * kBoundsPerOctave;
 // A certified bound needs no margin for an estimate's allowance, only for rounding (M_0's planes resolve 2^-25: 4e-4 of the smallest
 // eigenvalue at a norm of 16, damping 1e-3), and so may end further from I.
 constexpr double kCertifiedGrow = 1.04, kCertifiedRadius = 0.66;
+// Products with T^p lose 2^-22 of its largest eigenvalue.  Where T is smallest, on the large eigenvalues of M, that is as much more
+// of T^p as its range, and it mixes their eigenvectors with those of the small ones: errors that the Frobenius norm of an inverse
+// root hardly shows and its norm weighted by the statistic itself does.  So weighted, A^(-q/p) was 1.55 times as far off as after
+// linear steps in the worst (p = 8; 1.9 for p = 4, 4.4 for p = 2) with a range of 1e3, of 135 calls: rank-deficient statistics of 0.1 to
+// 0.9 rows a column, full ones of 1.5 and 4, log-uniform ones of condition 1e2 to 1e6, 256 to 2048 wide, three bounds each.  With
+// these 1.02, 0.58 and 0.84, and 0.6, 0.3 and 0.45 in the mean (p = 8, 4, 16); l' is a sixth smaller.  Narrower still for p = 8: 0.94 with
+// 300, but a fourth step where nothing is known (roots of four 2048 columns wide 2.38 -> 3.44 ms; with 1e3 2.34).  Square roots keep linear
+// steps: rank-deficient statistics' were 1.18 times as far off with 50.
+static double step_range(int p) { return std::min(400.0, 6.25 * p * p); }
+constexpr int kSteepFromPower = 4;
 constexpr int kSteepFrom = 256;   // columns: on narrower statistics linear steps can be closer (by 2.8 times, of 8e-7, 8 wide)
 struct BoundNode {
   bool ok[3] = {};
@@ -410,7 +420,7 @@ static const BoundNode& bound_node(int p, int j) {
   if (found != known.end()) return found->second;
   BoundNode& node = known[p * kBounds + j];
   for (int i = 0; i < 3; ++i) {
-    node.ok[i] = best_step(p, bound_of(j), kStepDegrees[i], kMaxPowerRange, node.step[i]);
+    node.ok[i] = best_step(p, bound_of(j), kStepDegrees[i], i ? step_range(p) : kMaxPowerRange, node.step[i]);
     if (!node.ok[i]) continue;
     for (int c = 0; c < 2; ++c) {
       FinishPoly& fin = node.fin[c][i];
@@ -428,15 +438,14 @@ struct StepPlan {
 };
 // T's own products; with a linear term it writes and reads an FP32 matrix more
 static double own_products(const NewtonStep& s) { return (s.degree == 4 ? 2 : s.degree - 1) + (s.lin != 0.0 ? 0.25 : 0.0); }
-// Cheapest steps from bound j on; `memo` is the call's own.
-static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo) {
-  const auto found = memo.find(j);
-  if (found != memo.end()) return found->second;
+static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo);
+// Cheapest steps from bound j on, the first of degree two or four unless `any`; `memo` is the call's own.
+static StepPlan cheapest_first(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool any) {
   StepPlan best;
   const BoundNode& node = bound_node(p, j);
   int log2p = 0;
   while ((1 << log2p) < p) ++log2p;
-  for (int i = 2; i >= 0; --i) {
+  for (int i = 2; i >= (any ? 0 : 1); --i) {
     if (!node.ok[i]) continue;
     const double own = log2p + 2 + own_products(node.step[i]);   // (powers, M, the next product with X)
     const double end = single * (node.fin_products[certified][i] - 1) + 1.0;
@@ -453,7 +462,12 @@ static const StepPlan& cheapest(int p, int j, bool certified, double single, std
       best.path.insert(best.path.end(), rest.path.begin(), rest.path.end());
     }
   }
-  return memo[j] = best;
+  return best;
+}
+static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo) {
+  const auto found = memo.find(j);
+  if (found != memo.end()) return found->second;
+  return memo[j] = cheapest_first(p, j, certified, single, memo, true);
 }
 
 // Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
@@ -518,7 +532,7 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
       s.l_last = l0;
     }
   }
-  const int first = steep_n >= kSteepFrom && iters <= 0 && !s.graded.products && p > 1 ? bound_below(l0) : kBounds;
+  const int first = steep_n >= kSteepFrom && iters <= 0 && !s.graded.products && p >= kSteepFromPower ? bound_below(l0) : kBounds;
   if (first < kBounds) {
     int log2p = 0;
     while ((1 << log2p) < p) ++log2p;
@@ -538,8 +552,8 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
         if (!node.ok[i]) continue;
         const int from = std::max(norm16, bound_below(node.step[i].next));
         if (from > norm16 && i < 2) continue;   // (degree four gets further)
-        const StepPlan& rest = cheapest(p, from, true, single, memo);
-        if (rest.path.empty() || rest.path[0].second == 0) break;   // (a first T of degree one is no product's result)
+        const StepPlan rest = cheapest_first(p, from, true, single, memo, false);   // (a first T of degree one is no product's result)
+        if (rest.path.empty()) break;
         const double all = log2p + 2 + own_products(node.step[i]) + rest.cost;
         if (rest.cost < 0.9 * plan.cost && all < linear) {
           s.late = bound_of(from);

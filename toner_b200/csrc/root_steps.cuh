@@ -1,12 +1,12 @@
 // Newton steps of higher degree (host only): T = q(M) of degree 1, 2 or 4 in the coupled iteration X <- X T, M <- T^p M.
 //
 // A step takes the spectrum of M from [l, 1] to [l', 1].  With the best linear T l' is 13 l at most (p = 8) and the step takes
-// log2 p + 2 products; a T of degree two costs one product more and reaches 38 l, one of degree four two more and 129 l: the
-// logarithm gained per product is 0.52, 0.61 and 0.69, and the steps next to I gain likewise (l = 0.013: one step of degree four
+// log2 p + 2 products; a T of degree two costs one product more and reaches 34 l, one of degree four two more and 110 l: the
+// logarithm gained per product is 0.51, 0.59 and 0.67, and the steps next to I gain likewise (l = 0.013: one step of degree four
 // where it took two linear ones).
 //
 // The q for which l' is largest:  maximise r subject to  r g(mu) <= q(mu) <= mu^(-1/p)  on [l, kStepHigh], with  g = mu^(-1/p)
-// or, where that is more, the cap on the dynamic range of T^p (kMaxPowerRange); l' = r^p.  This is a linear Chebyshev problem: at
+// or, where that is more, the cap on the dynamic range of T^p (max_range); l' = r^p.  This is a linear Chebyshev problem: at
 // the best q the two bounds are touched in turn at degree + 2 points, found by Remez' exchange on a grid.
 //
 // q is formed as  top z^2 + con  or  top (z^2 + kappa)^2 + lin mu + con  with z = zb + za mu: a square is a product of one pair of
