@@ -2211,10 +2211,15 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     // What the engine starts from: planes of M_0 and of T_0 = a I - b M_0; for a graded finish those of Z
     // in T_0's place, and M_0 in FP32 with the hi plane of M_0 + g I, of which W_K is a multiple
     const bool graded_finish = graded.products > 0;
+    // plane products interleaved (toner_gemm_desc::interleave), and the finish in its short form: unless the caller asked for
+    // the plane-by-plane order of additions
+    const bool interleave = (track_sweeps & 512) == 0;
     // Operand planes between products are stored by half: writing the mirror images took 4 to 10 % of a product (12 x 3072 in chains
     // of two, one / two pairs of planes: 948 -> 906 and 1055 -> 958 us; 36 x 768 81 -> 76 and 98 -> 90; a product of the finish, with C,
     // 12 x 3072 390 -> 348).  On the few matrices of a small step a map more per operand costs the host what it saves.
-    const bool half = (long long)kc * nn >= kHalfFrom;
+    // (Half storage takes tiles of CTA pairs.  Interleaved linear steps in long chains follow the tile, and below 512 columns others are
+    // taken: square roots of 64 x 264 were 2.45e-5 off on pairs and 2.08e-5 on theirs.)
+    const bool half = (long long)kc * nn >= kHalfFrom && (n >= 512 || !interleave || plan.steep || graded_finish);
     const double top_gain = graded.products ? graded.beta[graded.products] * graded.za : 1.0;
     const double top_diag =
         graded.products ? (graded.alpha[graded.products] + graded.beta[graded.products] * graded.zb) / top_gain : 0.0;
@@ -2286,10 +2291,6 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
       TONER_CUDA(cudaGetLastError());
     }
     }
-
-    // plane products interleaved (toner_gemm_desc::interleave), and the finish in its short form: unless the caller asked for
-    // the plane-by-plane order of additions
-    const bool interleave = (track_sweeps & 512) == 0;
 
     // D = (A planes) * (B planes)^T / (sa * sb): symmetric result, FP32-accurate; outputs as requested
     struct Out {
