@@ -174,7 +174,8 @@ def product_counts(core, optimizer: str):
     for name, g in core.groups.items():
         f = g.factors
         split, single = f.products
-        out[name] = {"newton_steps": f.iterations, "finish_order": f.finish_order, "graded": f.graded is not None, "split": split,
+        higher = f.steps   # steps of degree two and four, where they took the place of linear ones
+        out[name] = {"newton_steps": len(higher["steps"]) + 1 if higher else f.iterations, "finish_order": f.finish_order, "graded": f.graded is not None, "split": split,
                      "single": single}
     return out
 

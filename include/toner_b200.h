@@ -231,8 +231,8 @@ int toner_split16(const float* x, const float* const* x_list, int32_t batch, int
  * `iters` <= 0 selects the schedule with the fewest plane passes, steps and finish together, which depends only on n, damping,
  * p and the bound: toner_inv_roots_iterations(n, damping, p) linear steps (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632,
  * damping 1e-3, the finish counted), or the fewer steps of higher degree that toner_inv_roots_steps_for states.
- * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step (before a
- * graded finish max|I - Z^2| above 1.5),
+ * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step (0.7 after
+ * steps of higher degree; before a graded finish max|I - Z^2| above 1.5),
  * 2 non-finite, 3 / 4 a caller's spectrum bound that did not hold (toner_inv_roots_ex / _tracked).  The caller decides what to do with a non-zero status (the Python host recomputes that
  * statistic with an eigendecomposition, as the reference's fallback does, src/toner/fast/engine.py:714-731).
  * `ema` may start anywhere; root_lo, the workspace, `deflate` and, where a direction is tracked, `track` and root_hi start on
@@ -264,8 +264,8 @@ int toner_inv_roots_schedule(float lower, int32_t p, int32_t iters, double* ab_o
 int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps_out, int32_t* split_out, double* coef_out,
                                int32_t coef_capacity);
 /* The steps of a call that asks for no step count and no plane order, on statistics of width n, where that costs less than
- * linear ones: T of degree 1, 2 or 4 in M, levelled like the linear T (129 times the lower bound instead of 13 for two products
- * more at degree 4, p = 8).  Returns their number (0: the schedule of toner_inv_roots_schedule is used) and writes seven doubles
+ * linear ones (p >= 4, n >= 256): T of degree 1, 2 or 4 in M, levelled like the linear T (110 times the lower bound instead of 13
+ * for two products more at degree 4, p = 8).  Returns their number (0: the schedule of toner_inv_roots_schedule is used) and writes seven doubles
  * a step (degree, zb, za, kappa, top, lin, con: with z = zb + za mu, T is con + lin mu plus nothing, top z^2 or
  * top (z^2 + kappa)^2), the finishing polynomial and the distance e as toner_inv_roots_schedule does, and products_out[0], [1]: the split and the single-pass
  * products that steps and finish take.  kind: the bound is an estimate (0), certified (1), the one that always holds (2).  late_out > 0 (kind

@@ -153,8 +153,7 @@ def test_a_first_step_left_out_by_some_statistics(ops, p, q, n):
             continue
         want = (vec * lam.pow(-s)[:, None, :]) @ vec.mT
         got, ref = [(x.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1) for x in (root, plain)]
-        # (the middle one's spectrum starts at 3e-6, below 2^-22 of T^p's range of 1e3: up to 1.4 times the linear steps' error)
-        assert (got <= torch.tensor([1.2, 1.6, 1.2], device="cuda") * ref + 1e-6 * q).all(), (got.tolist(), ref.tolist())
+        assert (got <= 1.2 * ref + 1e-6 * q).all(), (got.tolist(), ref.tolist())
     for b in range(3):
         own = ops.inv_roots(stats[b:b + 1].expand(3, n, n).contiguous(), DAMPING, p, q)     # (of one tile choice: three as well)
         assert torch.equal(own[0][b], lo[b]) and (hi is None or torch.equal(own[1][b], hi[b]))

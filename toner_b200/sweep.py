@@ -139,16 +139,24 @@ def bench_roots(a):
     ws = torch.empty(ops.inv_roots_workspace_bytes(a.k, a.n), device="cuda", dtype=torch.uint8)
     lo = torch.empty_like(c)
     hi = torch.empty_like(c) if a.q > 1 else None
-    fn = lambda: ops.inv_roots(c, 1e-3, a.p, a.q, root_lo=lo, root_hi=hi, workspace=ws)
+    norms = torch.empty(a.k, device="cuda")
+    fn = lambda: ops.inv_roots(c, 1e-3, a.p, a.q, root_lo=lo, root_hi=hi, workspace=ws, norms=norms)
     ms, best = timed(fn, a.warmup, a.reps, False)
     log2p, log2q = int(math.log2(a.p)), int(math.log2(a.q))
     order = ops.inv_roots_finish_order(a.n, 1e-3, a.p)
     split = (iters - 1) * (log2p + 2) + log2q     # X T and T^p M per step (no X product first, no M last), squarings
     single = ops.inv_roots_finish_products(a.n, 1e-3, a.p)   # of the finishing polynomial
-    flops = a.k * (split + single) * 2 * a.n ** 3
+    left_out = 0
+    steps = ops.inv_roots_steps(1e-3 / (a.n * (1 + 1e-3)), a.p, a.n, 2)
+    if steps:             # steps of higher degree; statistics that start with the second leave out T_0, T_0^p M and X_1 T_1
+        split, single = steps["products"][0] + log2q, steps["products"][1]
+        order = len(steps["coefficients"]) - 1
+        if steps["late"]:
+            left_out = int((1e-3 / norms > steps["late"]).sum()) * (log2p + (4 if steps["steps"][0][0] == 4 else 3))
+    flops = (a.k * (split + single) - left_out) * 2 * a.n ** 3
     return report("inv_roots", {"k": a.k, "n": a.n, "p": a.p, "q": a.q, "cond": a.cond}, ms, best, flops=flops,
-                  extra={"iterations": iters, "finish_order": order, "damping": 1e-3, "split_products": split,
-                         "single_pass_products": single,
+                  extra={"iterations": len(steps["steps"]) + 1 if steps else iters, "finish_order": order, "damping": 1e-3,
+                         "split_products": split, "left_out": left_out, "single_pass_products": single,
                          "note": "dense count 2 n^3 per product; a split product runs 3 FP16 plane passes, a "
                                  "single-pass one 1, over the tiles meeting the upper triangle"})
 
