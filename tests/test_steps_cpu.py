@@ -59,6 +59,47 @@ def test_the_bound_that_always_holds_with_and_without_its_first_step(p, n):
     assert s["late"] > 0 or p not in (4, 8) or n == 16384     # (not where the second step would be a linear one)
 
 
+def _turned(steps, coefficients, distance, p, mu0):
+    """Of norms that are too low by these factors (the top of M_0's spectrum), those after which the checks of an estimated bound (the
+    convergence test's 0.7, the distance with its allowance, 0.03 below zero) see nothing and the root is wrong."""
+    x, mu = np.ones_like(mu0), mu0.copy()
+    with np.errstate(over="ignore", invalid="ignore"):
+        for degree, zb, za, kappa, top, lin, con in steps:
+            z = zb + za * mu
+            t = con + lin * mu + top * {1: 0.0, 2: z ** 2, 4: (z ** 2 + kappa) ** 2}[degree]
+            x, mu = x * t, mu * t ** p
+        r = 1.0 - mu
+        seen = ~np.isfinite(r) | (np.abs(r) > 0.7) | (r > 1.15 * distance + 1e-3) | (r < -0.03)
+        right = np.abs(x * np.polyval(np.array(coefficients)[::-1], r) * mu0 ** (1.0 / p) - 1.0) < 1e-4
+    return mu0[~seen & ~right]
+
+
+@pytest.mark.parametrize("n", [264, 768, 3072])
+@pytest.mark.parametrize("p", [4, 8, 16, 32])
+def test_a_norm_that_is_too_low_is_seen_or_does_no_harm(p, n):
+    """Under an estimated bound the norm is an estimate too, and M_0 may reach above 1.  A schedule with steps of higher degree lets
+    through no wrong root that the linear steps for the same bound would not, nothing at all up to a reach of 1.3 for p = 4 and 2
+    from p = 8 on: after a step of even degree no linear T follows, whose sign could turn."""
+    from toner_b200 import ops
+    reach = np.linspace(1.0, 4.0, 30001)
+    used = 0
+    for lower in np.geomspace(1.5e-7, 0.3, 200):
+        s = ops.inv_roots_steps(float(lower), p, n, 0)
+        if s is None:
+            continue
+        used += 1
+        degrees = [step[0] for step in s["steps"]]
+        assert degrees == sorted(degrees, key=lambda d: d > 1), degrees
+        wrong = _turned(s["steps"], s["coefficients"], s["distance"], p, reach)
+        assert not (wrong < (1.3 if p == 4 else 2.0)).any(), (lower, degrees, wrong.min())
+        if wrong.size:
+            linear = ops.inv_roots_schedule(float(lower), p)
+            of_linear = _turned([(1, 0.0, 0.0, 0.0, 0.0, -b, a) for a, b in linear["steps"]], linear["coefficients"],
+                                linear["distance"], p, reach)
+            assert of_linear.size and of_linear.min() <= wrong.min() + 1e-3, (lower, degrees, wrong.min())
+    assert used >= 100, used
+
+
 def test_square_roots_and_narrow_statistics_keep_linear_steps():
     from toner_b200 import ops
     for lower in np.geomspace(1.5e-7, 0.3, 60):

@@ -438,14 +438,19 @@ struct StepPlan {
 };
 // T's own products; with a linear term it writes and reads an FP32 matrix more
 static double own_products(const NewtonStep& s) { return (s.degree == 4 ? 2 : s.degree - 1) + (s.lin != 0.0 ? 0.25 : 0.0); }
-static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo);
-// Cheapest steps from bound j on, the first of degree two or four unless `any`; `memo` is the call's own.
-static StepPlan cheapest_first(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool any) {
+static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear);
+// Cheapest steps from bound j on, the first of degree two or four unless `linear`; `memo` is the call's own.
+// Where the bound is an estimate so may the norm be, and M_0 may reach above 1.  A T of degree two or four sends what lies there
+// further up, to where a linear T is negative; T^p is not, so M could come back to I with the sign of X turned and no check to see it
+// (p = 8: degrees 4, 1 from a reach of 1.12).  So after a step of even degree, whose T is positive everywhere, only such steps follow:
+// 0.5 split products more for 4 bounds in 400 at p = 4, none at p = 8 to 32.  Linear steps before them leave what linear ones alone leave
+// (verified vectors below).
+static StepPlan cheapest_first(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear) {
   StepPlan best;
   const BoundNode& node = bound_node(p, j);
   int log2p = 0;
   while ((1 << log2p) < p) ++log2p;
-  for (int i = 2; i >= (any ? 0 : 1); --i) {
+  for (int i = 2; i >= (linear ? 0 : 1); --i) {
     if (!node.ok[i]) continue;
     const double own = log2p + 2 + own_products(node.step[i]);   // (powers, M, the next product with X)
     const double end = single * (node.fin_products[certified][i] - 1) + 1.0;
@@ -455,7 +460,7 @@ static StepPlan cheapest_first(int p, int j, bool certified, double single, std:
     }
     const int next = bound_below(node.step[i].next);
     if (next >= j || node.step[i].next > 0.9 || own + log2p + 2 >= best.cost) continue;
-    const StepPlan& rest = cheapest(p, next, certified, single, memo);
+    const StepPlan& rest = cheapest(p, next, certified, single, memo, certified || i == 0);
     if (own + rest.cost < best.cost) {
       best.cost = own + rest.cost;
       best.path = {{j, i}};
@@ -464,10 +469,11 @@ static StepPlan cheapest_first(int p, int j, bool certified, double single, std:
   }
   return best;
 }
-static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo) {
-  const auto found = memo.find(j);
+static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear) {
+  const int key = linear ? j : -j;
+  const auto found = memo.find(key);
   if (found != memo.end()) return found->second;
-  return memo[j] = cheapest_first(p, j, certified, single, memo, true);
+  return memo[key] = cheapest_first(p, j, certified, single, memo, linear);
 }
 
 // Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
@@ -541,7 +547,7 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
     const double linear = (s.iters - 1) * (log2p + 2) +
                           single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
     std::unordered_map<int, StepPlan> memo;
-    StepPlan plan = cheapest(p, first, kind > 0, single, memo);
+    StepPlan plan = cheapest(p, first, kind > 0, single, memo, true);
     if (kind == 2) {
       // The bound that always holds, damping / n, is a norm of n; statistics have one of 5 to 15, which the device knows before the
       // first product.  So the first step goes from this bound to that of a norm of 16, damping / 16, or as far as it gets, and is
@@ -2670,10 +2676,12 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           }
         } else if (ritz_norm) {
           // The norm was an estimate too.  Eigenvalues of M_0 above 1 (the estimate was too low for them) come out of
-          // the first Newton step BELOW the lower bound the schedule continues from -- T = a I - b M is small there --
-          // and lag the same way; they belong to the top of A', so the same four steps from the largest Ritz vector
-          // that stayed in A' find them.  (An eigenvalue beyond a / b, where T changes sign, makes M grow instead and
-          // fails the convergence test.)  Both starting vectors go through M in one pass per step.
+          // a linear first step BELOW the lower bound the schedule continues from -- T = a I - b M is small there --
+          // and lag the same way, out of steps of higher degree ABOVE 1; they belong to the top of A', so the same four steps from the largest Ritz vector
+          // that stayed in A' find them.  (What lies beyond a / b, where a linear T is negative, lags or grows too, but for
+          // bands a few 1e-3 wide that come back to I with the sign of X turned: of linear schedules at a reach of 1.03 or
+          // more for p = 2, 1.24 for p = 4, 1.95 for p = 8, none up to 3.4 for 16 and 32; the norm is 1.4 times the Ritz
+          // value, so that has to be as much more too low.)  Both starting vectors go through M in one pass per step.
           TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 0.f);
           for (int sw = 0; sw < 4; ++sw) {
             TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, pv, py, n, 2, 2));
