@@ -231,8 +231,8 @@ int toner_split16(const float* x, const float* const* x_list, int32_t batch, int
  * `iters` <= 0 selects the schedule with the fewest plane passes, steps and finish together, which depends only on n, damping,
  * p and the bound: toner_inv_roots_iterations(n, damping, p) linear steps (8 for p = 8, 8 for p = 4, 10 for p = 2 at n = 5632,
  * damping 1e-3, the finish counted), or the fewer steps of higher degree that toner_inv_roots_steps_for states.
- * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| above 0.5 before the last step (0.7 after
- * steps of higher degree; before a graded finish max|I - Z^2| above 1.5),
+ * status[b] (DEVICE, optional): 0 converged, 1 residual max|I - M| before the last step above what the finish is fitted to
+ * (0.5 to 0.7, with the bound's schedule; before a graded finish max|I - Z^2| above 1.5),
  * 2 non-finite, 3 / 4 a caller's spectrum bound that did not hold (toner_inv_roots_ex / _tracked).  The caller decides what to do with a non-zero status (the Python host recomputes that
  * statistic with an eigendecomposition, as the reference's fallback does, src/toner/fast/engine.py:714-731).
  * `ema` may start anywhere; root_lo, the workspace, `deflate` and, where a direction is tracked, `track` and root_hi start on

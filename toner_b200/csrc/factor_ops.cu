@@ -113,7 +113,12 @@ constexpr double kFinishLow = -0.02, kFinishGrow = 1.15, kFinishPad = 1e-3;
 struct FinishPoly {
   int order = 0;                       // 0: no degree up to the cap reaches the bound at this distance
   double c[kMaxFinishOrder + 1] = {};  // q(r) = sum_j c[j] r^j
+  double reach = 0.0;                  // upper end of the interval it is fitted to (0: not fitted)
 };
+// Entries of I - M above this before the finish: not converged.  No entry of a symmetric matrix exceeds its norm, and up to where the
+// finish is fitted to, the schedule's e with its margin, the root is right; a hundredth more for rounding.  At least 0.5, which M that
+// diverges goes far beyond.  (0.5 whatever e flagged right roots: 768 columns in plane order, p = 4, nothing known, end at e = 0.527.)
+static float converged_within(const FinishPoly& f) { return (float)std::max(0.5, f.reach + 0.01); }
 
 // (1 - r)^(1/p) at the points where a fit is checked; a point is evaluated when a fit first gets that far.
 struct FitSamples {
@@ -229,7 +234,8 @@ static FinishPoly finish_poly(int p, double e, double grow = kFinishGrow, double
   for (int m = 2; m <= kMaxFinishOrder; ++m) {
     if (finish_fit(p, kFinishLow, hi, m, kFinishTail, samples, f.c)) {
       f.order = m;
-      if (!finish_usable(f, hi)) f.order = 0;
+      if (!finish_usable(f, hi)) return FinishPoly();
+      f.reach = hi;
       return f;
     }
   }
@@ -2415,7 +2421,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
             if (rc) return rc;
           }
           // fold ||A||_F^{-1/p} into the product; the distance of M from I was gathered when M was produced
-          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : (plan.steep ? 0.7f : 0.5f), damping, lower_used, plan.steep && ritz_norm ? th8 : nullptr);
+          TONER_LAUNCH(finish_kernel, (kc + 127) / 128, 128, stream, resid, sumsq_a, scale_lo, status ? status + k0 : nullptr, norm_out ? norm_out + k0 : nullptr, kc, p, graded_finish ? 1.5f : converged_within(fin), damping, lower_used, plan.steep && ritz_norm ? th8 : nullptr);
           TONER_CUDA(cudaGetLastError());
           // Tcur holds planes of R = I - M and A32 the FP32 M (both from the last update of M).  q(R), one plane per product,
           // into Mb[1]; the terms linear in M enter in FP32 as beta * c.
