@@ -1313,7 +1313,11 @@ __device__ __forceinline__ void cluster_sum_many(double (&acc)[K], double* part,
 // then replaced by the orthonormalised Y - sigma V, one more step of the power iteration on A - sigma I: with sigma = 0.8 c, c the
 // mean of the eigenvalues that do not stand out, what lies below 1.6 c shrinks as if it were 0.8 c (a bulk up to 1.8 under a
 // direction of 10: by 0.11 a sweep where A itself gives 0.18; four sweeps then reach the residual that deflation asks for, with
-// which the fifth direction of spiked:4 was left in one call of four).
+// which the fifth direction of spiked:4 was left in one call of four).  Where no trace is given sigma is 0: the last step takes A itself,
+// which leaves nothing of the smallest eigenvalues' directions in V, where their inverse roots are largest; after a shifted one the Ritz
+// rotation took that from the block's other vectors and rounded the top vector once more (4.3e-8 off for 3.5e-8; A^(-1/2) weighted by the
+// statistic, columns that decay exponentially: 1.08 times as far off as without shifts in the mean of 40 calls and 1.31 in the worst,
+// now 0.93 and 1.02).
 // Three passes over the two blocks of vectors (five from ten vectors on, whose sums are taken for half of the rows at a time);
 // every reduction is taken for all pairs at once.  R: r rounded up to even, as in block_gemv_kernel -- with eight
 // vectors' sums (64 and 44 doubles to reduce) whatever r, a launch took 42 us on 12 statistics of width 3072 and r = 2, with r's 17.
@@ -2189,7 +2193,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         TONER_LAUNCH(block_start_kernel<R>, kc, 256, stream, dv, n, defl_r, slots, defl_cold ? 1 : 0, in_order);
         for (int sw = 0; sw < sweeps; ++sw) {
           TONER_CUDA(launch_block_gemv<R>(kc, stream, A32, dv, py, n, defl_r, slots));
-          TONER_CUDA(launch_ritz<R>(kc, stream, dv, py, n, defl_r, slots, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order, (float)((double)n * (1.0 + (double)damping))));
+          // (the last step of the power iteration is one on A itself, see ritz_kernel)
+          const float trace = sw < sweeps - 2 ? (float)((double)n * (1.0 + (double)damping)) : 0.f;
+          TONER_CUDA(launch_ritz<R>(kc, stream, dv, py, n, defl_r, slots, sw == sweeps - 1 ? 1 : 0, th8, res8, in_order, trace));
         }
         return 0;
       };
