@@ -1,7 +1,13 @@
 """Steps of higher degree (toner_inv_roots_steps_for): scalars through the stated schedule, over all bounds (no device)."""
 
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "toner_b200", "csrc")
 
 
 def _take(s, lam, steps, p):
@@ -104,3 +110,39 @@ def test_square_roots_and_narrow_statistics_keep_linear_steps():
     from toner_b200 import ops
     for lower in np.geomspace(1.5e-7, 0.3, 60):
         assert all(ops.inv_roots_steps(float(lower), p, n, kind) is None for p, n in ((1, 768), (2, 768), (8, 248)) for kind in range(3))
+
+
+BOUNDS = r"""
+#include "root_steps.cuh"
+#include <cstdio>
+int main() {
+  using namespace toner;
+  int steps = 0;
+  for (int p : {4, 8, 16, 32})
+    for (int j = 1; j < 256; ++j)
+      for (int degree : {2, 4}) {
+        NewtonStep s;
+        if (!best_step(p, std::exp2(-j / 8.0), degree, std::min(400.0, 6.25 * p * p), s)) continue;
+        double z_most = 0.0, y_most = 0.0;
+        for (int i = 0; i <= 2000; ++i) {
+          const double z = s.zb + s.za * kStepHigh * i / 2000;
+          z_most = std::max(z_most, std::fabs(z));
+          y_most = std::max(y_most, std::fabs(z * z + s.kappa));
+        }
+        const bool holds = z_most <= s.most_z && y_most <= s.most_y && s.most_z < 1.001 * z_most && s.most_y < 1.001 * y_most;
+        if (!holds) return std::printf("p %d bound %d degree %d: %g %g, %g %g", p, j, degree, z_most, s.most_z, y_most, s.most_y), 1;
+        ++steps;
+      }
+  return std::printf("%d", steps), 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_operand_planes_are_scaled_for_all_that_z_and_its_square_reach(tmp_path):
+    """Every step that can be planned states the largest |z| and |z^2 + kappa| on [0, 1.06]: what their FP16 planes are scaled for, a
+    factor four below overflow.  (Constants of 1.2 and 1.1 + |kappa| were up to 3.9 and 3.5 times too small.)"""
+    (tmp_path / "bounds.cpp").write_text(BOUNDS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, str(tmp_path / "bounds.cpp"), "-o", str(tmp_path / "bounds")], check=True)
+    out = subprocess.run([str(tmp_path / "bounds")], capture_output=True, text=True)
+    assert out.returncode == 0 and int(out.stdout) > 1500, out.stdout

@@ -2244,7 +2244,9 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     const bool first_z = graded_finish || sched[0].degree > 1;   // planes of Z instead of T_0's
     float* const m32 = graded_finish || sched[0].lin != 0.0 ? reinterpret_cast<float*>(Xb[0]) : nullptr;   // M_0
     __half* const first_planes = first_z && !graded_finish ? Tb[0] : Xb[1];
-    const float s_z = plane_scale(1.2), s_top = plane_scale(1.1 * (1.0 + std::fabs(top_diag)));
+    double most_z = graded_finish ? 1.2 : 0.0;   // (one scale for all steps: statistics that start late have the second Z in the first one's planes)
+    for (int i = 0; !graded_finish && i < iters - 1; ++i) most_z = std::max(most_z, sched[i].most_z);
+    const float s_z = plane_scale(most_z > 0.0 ? most_z : 1.0), s_top = plane_scale(1.1 * (1.0 + std::fabs(top_diag)));
     const float init_a = (float)(graded_finish ? graded.zb : first_z ? sched[0].zb : sched[0].a);
     const float init_b = (float)(graded_finish ? -graded.za : first_z ? -sched[0].za : sched[0].b);
     const float init_sm = graded_finish ? s_top : s_m, init_diag = graded_finish ? (float)top_diag : 0.f;
@@ -2385,7 +2387,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         float s_from = s_t;
         if (st.degree == 4) {
           Out y;
-          y.s0 = Pb[1]; y.s0_scale = plane_scale(1.1 + std::fabs(st.kappa));
+          y.s0 = Pb[1]; y.s0_scale = plane_scale(st.most_y);
           y.s0_a = (float)st.kappa;
           rc = sym_product(from, s_from, from, s_from, y, chain, 0, skip);
           if (rc) return rc;

@@ -31,6 +31,7 @@ struct NewtonStep {
   int degree = 1;
   double za = 0.0, zb = 0.0, kappa = 0.0, top = 0.0, lin = 0.0, con = 0.0;
   double next = 0.0;     // lower end of the spectrum of T^p M
+  double most_z = 0.0, most_y = 0.0;   // bounds of |z| and |z^2 + kappa| on [0, kStepHigh], which their operand planes are scaled for
   double at(double mu) const {
     if (degree == 1) return a - b * mu;
     const double z = zb + za * mu, y = degree == 2 ? z : z * z + kappa;
@@ -143,6 +144,9 @@ inline bool scale_step(int p, NewtonStep& s) {
     s.a = 1.01 * largest * scale;
   }
   s.next = std::pow(least * scale * (1.0 - kMargin), p);
+  const double z0 = std::fabs(s.zb), z1 = std::fabs(s.zb + s.za * kStepHigh);   // (z is linear: largest at an end; z^2 least at 0)
+  s.most_z = std::max(z0, z1);
+  s.most_y = std::max(std::fabs(s.kappa), std::fabs(s.most_z * s.most_z + s.kappa));
   return true;
 }
 
