@@ -2235,9 +2235,11 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     // Operand planes between products are stored by half: writing the mirror images took 4 to 10 % of a product (12 x 3072 in chains
     // of two, one / two pairs of planes: 948 -> 906 and 1055 -> 958 us; 36 x 768 81 -> 76 and 98 -> 90; a product of the finish, with C,
     // 12 x 3072 390 -> 348).  On the few matrices of a small step a map more per operand costs the host what it saves.
-    // (Half storage takes tiles of CTA pairs.  Interleaved linear steps in long chains follow the tile, and below 512 columns others are
-    // taken: square roots of 64 x 264 were 2.45e-5 off on pairs and 2.08e-5 on theirs.)
-    const bool half = (long long)kc * nn >= kHalfFrom && (n >= 512 || !interleave || plan.steep || graded_finish);
+    // Half storage takes tiles of CTA pairs, and narrow statistics are faster on others: whole over half, a call on 4 Mi / 12 Mi elements,
+    // 0.60 at 64 columns, 0.74 at 128, 0.96 / 0.80 at 256, 0.87 / 0.91 at 264, 0.83 at 320, 0.98 / 0.91 at 384, 1.00 / 1.04 at 440, 1.03 at 504, 1.04 /
+    // 1.06 at 512, 1.01 / 0.98 at 576, 1.04 / 1.09 at 768.  (Interleaved linear steps in long chains also round by the tile: square roots of
+    // 64 x 264 were 2.45e-5 off on pairs and 2.08e-5 on theirs.)
+    const bool half = (long long)kc * nn >= kHalfFrom && n >= (plan.steep || graded_finish || !interleave ? 440 : 512);
     const double top_gain = graded.products ? graded.beta[graded.products] * graded.za : 1.0;
     const double top_diag =
         graded.products ? (graded.alpha[graded.products] + graded.beta[graded.products] * graded.zb) / top_gain : 0.0;
