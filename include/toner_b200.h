@@ -337,8 +337,10 @@ int toner_inv_roots_ex(const float* ema, int32_t k, int32_t n, float damping, in
  * iteration that was NOT deflated, never above ||A'||_F.  That value errs low, by up to a fifth at the dense edge of
  * a bulk, once its vector is a few calls old (the caller's business: a fresh slot's value sits near the mean
  * eigenvalue).  An eigenvalue of
- * A' / norm above 1 comes out of the first Newton step below the lower bound and lags like one below `lower`; the
- * verification looks for it with four more steps from that Ritz vector, status 4 as above. */
+ * A' / norm above 1 comes out of a linear first step below the lower bound and lags like one below `lower`; the
+ * verification looks for it with four more steps from that Ritz vector, status 4 as above.  Steps of higher degree send it above 1
+ * (past 1.06 of the norm, up to which they forgive it): four steps on (1 - e / 2) I - M from that Ritz vector's residual look for it, and a root
+ * may then hold NaNs, status 1. */
 int toner_inv_roots_tracked(const float* ema, int32_t k, int32_t n, float damping, int32_t p, int32_t q, int32_t iters,
                             float lower, int32_t lower_is_estimate, float* root_lo, float* root_hi, float* fro2_lo,
                             int32_t* status, float* norm_out, float* track, float* lmin_out, float* resid_out,

@@ -94,35 +94,52 @@ def test_directions_the_statistic_is_large_in(ops, p, q, n, rows):
         assert all(got <= 1.2 * linear for got, linear in zip(weighted[:half], weighted[half:])), (lower, weighted)
 
 
-def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops):
-    """The norm as an estimate 5 % too low: a T of even degree is levelled up to 1.06 and the roots are right; 20 % too low sends M
-    past 1, and the statistic is flagged."""
-    n, p, q = 384, 8, 4
-    stats = _statistics(n, 60.0)
+def _hidden_top(n, low, reach, share):
+    """Two statistics whose largest eigenvalue is 1.4 reach times the next, a block of one vector that is the next one's eigenvector but
+    for `share` of the top's -- four sweeps gain a factor of ten at most, so the norm comes out near 1.4 times the next -- and A."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, _ = torch.linalg.qr(torch.randn(n, n, device="cuda", generator=g, dtype=torch.float64))
+    lam = low * torch.exp(torch.rand(2, n, device="cuda", generator=g, dtype=torch.float64) * torch.tensor(1.5 / low).log())
+    lam[:, 0], lam[:, -2], lam[:, -1] = low, 1.6, 1.6 * 1.4 * reach
+    c = ((q * lam[:, None, :]) @ q.T).float()
+    stats = (0.5 * (c + c.mT)).contiguous()
     a = stats.double()
     a = a / a.diagonal(dim1=1, dim2=2).mean(1)[:, None, None] + DAMPING * torch.eye(n, device="cuda", dtype=torch.float64)
     lam, vec = torch.linalg.eigh(a)
-    for low, right in ((1.05, True), (1.2, False)):
-        # the norm is 1.4 times the largest Ritz value that is not deflated: vectors of the block that mix the top with a
-        # direction further down, at the angle which gives that value
-        theta = lam[:, -1] / (1.4 * low)
-        c2 = (theta - lam[:, 0]) / (lam[:, -1] - lam[:, 0])
-        vectors = torch.zeros(2, 8, n, device="cuda")
-        vectors[:, 0] = (c2.sqrt()[:, None] * vec[:, :, -1] + (1 - c2).sqrt()[:, None] * vec[:, :, 0]).float()
-        lower = 0.5 * float((lam[:, 0] / lam[:, -1]).min())
-        assert ops.inv_roots_steps(lower, p, n) is not None and ops.inv_roots_graded(lower, p, n) is None
+    block = torch.zeros(2, 8, n, device="cuda")
+    block[:, 0] = (vec[:, :, -2] + share * vec[:, :, -1]).float()
+    return stats, lam, vec, block
+
+
+@pytest.mark.parametrize("share", [0.003, 0.03])
+@pytest.mark.parametrize("low", [1e-4, 1e-3, 1e-2, 0.05, 0.15])
+@pytest.mark.parametrize("p,q", [(8, 4), (4, 1), (16, 8)])
+def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops, p, q, low, share):
+    """The norm as an estimate is too low for a direction the block holds next to nothing of.  Up to a reach of 1.06 T is levelled and
+    the roots are right (2e-5 of FP64 from a lower bound of 5e-5); beyond, the statistic is flagged or its root is right all the same."""
+    n = 384
+    flagged = 0
+    for reach in (1.02, 1.05, 1.1, 1.15, 1.2, 1.3, 1.5, 2.0):
+        stats, lam, vec, block = _hidden_top(n, low, reach, share)
+        lower = 0.5 * float((lam[:, 0] / (1.4 * lam[:, -2])).min())
+        steps = ops.inv_roots_steps(lower, p, n)
+        if steps is None:      # (linear steps forgive more, and flag where they do not)
+            continue
+        assert ops.inv_roots_graded(lower, p, n) is None or 2 * q != p
         norms = torch.zeros(2, device="cuda")
         lo, _, _, st = ops.inv_roots(stats, DAMPING, p, q, lower=lower, lower_is_estimate=True, norms=norms,
                                      track=vec[:, :, 0].float().contiguous(), lmin=torch.empty(2, device="cuda"), track_sweeps=4,
-                                     deflate=vectors, deflate_rank=1, ritz_norm=True)
+                                     deflate=block, deflate_rank=1, ritz_norm=True)
         ops.assert_healthy()
-        reach = (lam[:, -1] / norms.double()).tolist()
-        if right and all(x <= 1.06 for x in reach):
-            assert st.tolist() == [0, 0]
-            want = (vec * lam.pow(-1.0 / p)[:, None, :]) @ vec.mT
-            assert float((lo.double() - want).norm() / want.norm()) < 2e-5
-        else:
-            assert all(s in (1, 4) or x <= 1.08 for s, x in zip(st.tolist(), reach)), (st.tolist(), reach)
+        reached = (lam[:, -1] / norms.double()).tolist()
+        assert all(x <= 1.06 for x in reached) if reach < 1.06 else share > 0.01 or all(x > 1.08 for x in reached), reached
+        want = (vec * lam.pow(-1.0 / p)[:, None, :]) @ vec.mT
+        error = ((lo.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).tolist()
+        for s, e, x in zip(st.tolist(), error, reached):
+            assert s in (1, 4) or e < 1e-4, (low, reach, x, s, e)
+            assert x > 1.06 or s == 0, (low, reach, x, s, e)
+            flagged += s != 0
+    assert flagged > 0 or steps is None
 
 
 @pytest.mark.parametrize("p,q", [(4, 1), (8, 4)])

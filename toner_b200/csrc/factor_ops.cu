@@ -1578,18 +1578,23 @@ __global__ void ritz_norm_kernel(float* __restrict__ bound2, const float* __rest
 
 // out[b][0] = first[b] (the tracked direction), out[b][1] = the Ritz vector rest_idx[b] of statistic b (zero where there
 // is none): the two starting vectors of the verification, side by side for the two-vector passes.  `spread` > 0 adds fixed signs
-// of norm `spread` to both: a share of about 1 / sqrt(n) of every direction.
+// of norm `spread` to both: a share of about 1 / sqrt(n) of every direction.  With y = A v the second vector is that Ritz vector's
+// residual y - theta v.
 __global__ void __launch_bounds__(256) pick_vector_kernel(const float* __restrict__ first, const float* __restrict__ v,
                                                           const int* __restrict__ idx, float* __restrict__ out, int n,
-                                                          int vstride, float spread) {
+                                                          int vstride, float spread, const float* __restrict__ y,
+                                                          const float* __restrict__ theta) {
   ptx::pdl_begin();
   const int b = blockIdx.y;
   const int j = idx[b];
+  const float value = y && j >= 0 ? theta[b * kMaxDeflate + j] : 0.f;
   const float amount = spread * rsqrtf((float)n);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const unsigned h = (unsigned)i * (unsigned)i * 2654435761u;   // (signs of two quadratic sequences)
     const float s0 = (h >> 31) ? amount : -amount, s1 = ((h + (unsigned)i * 1013904223u) >> 31) ? amount : -amount;
-    const float x0 = first[(long long)b * n + i], x1 = j >= 0 ? v[((long long)b * vstride + j) * n + i] : 0.f;
+    const float x0 = first[(long long)b * n + i];
+    float x1 = j >= 0 ? v[((long long)b * vstride + j) * n + i] : 0.f;
+    if (y && j >= 0) x1 = y[((long long)b * vstride + j) * n + i] - value * x1;
     out[((long long)b * 2) * n + i] = spread > 0.f ? x0 + s0 : x0;
     out[((long long)b * 2 + 1) * n + i] = spread > 0.f ? x1 + s1 : x1;
   }
@@ -1764,12 +1769,14 @@ __global__ void __launch_bounds__(256) project_kernel(float* __restrict__ x, con
 // the incoming v, 1 - v.y / v.v (0 where v is zero: nothing is known).
 // Vector j = blockIdx.y of statistic b sits at (b * vs + j) * n; its quotient goes to e[j * e_stride + b].
 // With defl_v the new v is kept orthogonal to the deflated directions.
+// The step of vector 1 is one on (1 - shift) I - M, and lowest[b] (optional, zero at first) keeps the least of its quotients.
 __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v, const float* __restrict__ y, int n,
                                                           float* __restrict__ e, int vs, long long e_stride,
                                                           const float* __restrict__ defl_v, const float* __restrict__ defl_coef,
-                                                          int defl_r, int vstride) {
+                                                          int defl_r, int vstride, float shift, float* __restrict__ lowest) {
   ptx::pdl_begin();
   const int b = blockIdx.x;
+  const double keep = blockIdx.y == 1 ? 1.0 - (double)shift : 1.0;
   float* V = v + ((long long)b * vs + blockIdx.y) * n;
   const float* Y = y + ((long long)b * vs + blockIdx.y) * n;
   e += (long long)blockIdx.y * e_stride;
@@ -1777,7 +1784,7 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
   __shared__ double tot[3];
   double vy = 0.0, vv = 0.0, tt = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double yi = Y[i], vi = V[i], d = vi - yi;
+    const double yi = Y[i], vi = V[i], d = keep * vi - yi;
     vy += vi * yi;
     vv += vi * vi;
     tt += d * d;
@@ -1801,8 +1808,12 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
   }
   __syncthreads();
   const double inv = tot[2] > 0.0 ? 1.0 / sqrt(tot[2]) : 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (float)(((double)V[i] - (double)Y[i]) * inv);
-  if (threadIdx.x == 0) e[b] = tot[1] == 0.0 ? 0.f : (float)(1.0 - tot[0] / tot[1]);   // (NaN stays NaN)
+  for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (float)((keep * (double)V[i] - (double)Y[i]) * inv);
+  if (threadIdx.x == 0) {
+    const float quotient = tot[1] == 0.0 ? 0.f : (float)(1.0 - tot[0] / tot[1]);   // (NaN stays NaN)
+    e[b] = quotient;
+    if (lowest && blockIdx.y == 1) lowest[b] = fminf(lowest[b], quotient);
+  }
   if (defl_v) project_out(V, defl_v + (long long)b * vstride * n, defl_coef + b * kMaxDeflate, n, defl_r, red[0]);
 }
 
@@ -1813,7 +1824,7 @@ __global__ void __launch_bounds__(256) power_shift_kernel(float* __restrict__ v,
 // (a mean of 20 standard deviations, 1000 wide: 1e-4 to 3.5e-4 seen, 7.6e-4 allowed for).
 __global__ void verify_kernel(const float* __restrict__ e_est, const float* __restrict__ e_top, float e_allowed, float e_below,
                               int* __restrict__ status, float* __restrict__ e_out, int k, const float* __restrict__ theta,
-                              const float* __restrict__ rest_trace, int n) {
+                              const float* __restrict__ rest_trace, int n, const float* __restrict__ lowest) {
   ptx::pdl_begin();
   const bool both_signs = theta != nullptr;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1824,6 +1835,7 @@ __global__ void verify_kernel(const float* __restrict__ e_est, const float* __re
   if (e_top && isfinite(e)) {   // (fmaxf would pass over a NaN)
     const float t = size(e_top[b]);
     e = isfinite(t) ? fmaxf(e, t) : t;
+    if (lowest && isfinite(e)) e = fmaxf(e, size(lowest[b]));
   }
   if (e_out) e_out[b] = e;
   if (theta) e_allowed += 5.96e-8f * sqrtf((float)n) * theta[b * kMaxDeflate] / rest_trace[b];
@@ -2165,6 +2177,7 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
     int* rest_idx = reinterpret_cast<int*>(small(17));
     float* e_top = small(18);
     float* rest_trace = small(10);
+    float* const lowest = plan.steep && ritz_norm ? small(19) : nullptr;   // (`late` is for calls that certify the norm)
     const size_t sm8 = align_up((size_t)kc * kMaxDeflate * 4, 256);
     char* wp = w + sm * 20;
     float* th8 = reinterpret_cast<float*>(wp); wp += sm8;     // Ritz values, residuals, deflation coefficients and
@@ -2682,35 +2695,40 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
           // deviations, where the root it leaves is as good as any.
           const float* root = (q > 1 ? root_hi : root_lo) + (long long)k0 * nn;
           float* const py2 = py + (long long)kc * 2 * n;
-          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 1.f);
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 1.f, nullptr, nullptr);
           for (int sw = 0; sw < 2; ++sw) {
             TONER_CUDA(launch_block_gemv<2>(kc, stream, root, pv, py, n, 2, 2));
             TONER_LAUNCH(project_kernel, dim3(kc, 2), 256, stream, py, dv, coef8, n, defl_r, slots);
             TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, py, py2, n, 2, 2));
             TONER_CUDA(launch_block_gemv<2>(kc, stream, root, py2, py, n, 2, 2));
-            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), dv, coef8, defl_r, slots);
+            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), dv, coef8, defl_r, slots, 0.f, nullptr);
           }
         } else if (ritz_norm) {
           // The norm was an estimate too.  Eigenvalues of M_0 above 1 (the estimate was too low for them) come out of
-          // a linear first step BELOW the lower bound the schedule continues from -- T = a I - b M is small there --
-          // and lag the same way, out of steps of higher degree ABOVE 1; they belong to the top of A', so the same four steps from the largest Ritz vector
-          // that stayed in A' find them.  (What lies beyond a / b, where a linear T is negative, lags or grows too, but for
-          // bands a few 1e-3 wide that come back to I with the sign of X turned: of linear schedules at a reach of 1.03 or
-          // more for p = 2, 1.24 for p = 4, 1.95 for p = 8, none up to 3.4 for 16 and 32; the norm is 1.4 times the Ritz
-          // value, so that has to be as much more too low.)  Both starting vectors go through M in one pass per step.
-          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 0.f);
+          // linear steps BELOW the lower bound the schedule continues from -- T = a I - b M is small there -- and lag the same way;
+          // they belong to the top of A', so the same four steps from the largest Ritz vector that stayed in A' find them.  (What lies
+          // beyond a / b, where T is negative, lags or grows too, but for bands a few 1e-3 wide that come back to I with the sign of
+          // X turned: at a reach of 1.03 or more for p = 2, 1.24 for p = 4, 1.95 for p = 8, none up to 3.4 for 16 and 32; the norm
+          // is 1.4 times the Ritz value, so that has to be as much more too low.)  Both starting vectors go through M in one pass
+          // per step.
+          // Steps of higher degree send them ABOVE 1, where R is negative and small at first beside what it may be on the other side
+          // (degree 2 from l = 0.034: R = -0.3 for a reach of 1.2, 0.54 for the lower end).  Steps on R lose such a direction; those on
+          // (1 - e / 2) I - M gain it.  And they start from the Ritz vector's residual, which holds what the block has not found yet,
+          // the largest eigenvalues first.  (From the Ritz vector itself, on R: A^(-1/8) 6e-2 off, unflagged, where 0.3 % of it were
+          // a direction 1.68 times as large.)
+          TONER_LAUNCH(pick_vector_kernel, dim3(8, kc), 256, stream, vt, dv, rest_idx, pv, n, slots, 0.f, lowest ? py : nullptr, th8);
           for (int sw = 0; sw < 4; ++sw) {
             TONER_CUDA(launch_block_gemv<2>(kc, stream, A32, pv, py, n, 2, 2));
-            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), nullptr, nullptr, 0, 0);
+            TONER_LAUNCH(power_shift_kernel, dim3(kc, 2), 256, stream, pv, py, n, e_est, 2, (long long)(e_top - e_est), nullptr, nullptr, 0, 0, lowest ? (float)(0.5 * (1.0 - l_last)) : 0.f, lowest);
           }
         } else {
           TONER_CUDA(cudaMemcpyAsync(pv, vt, sizeof(float) * (size_t)kc * n, cudaMemcpyDeviceToDevice, stream));
           for (int sw = 0; sw < 4; ++sw) {
             TONER_LAUNCH(gemv_kernel, dim3((n + 7) / 8, kc), 256, stream, A32, pv, py, n);
-            TONER_LAUNCH(power_shift_kernel, kc, 256, stream, pv, py, n, e_est, 1, 0, nullptr, nullptr, 0, 0);
+            TONER_LAUNCH(power_shift_kernel, kc, 256, stream, pv, py, n, e_est, 1, 0, nullptr, nullptr, 0, 0, 0.f, nullptr);
           }
         }
-        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm || graded_finish ? e_top : nullptr, graded_finish ? (float)(kGradedResidual + p * kGradedTail) : (float)(1.15 * (1.0 - l_last) + 1e-3), plan.steep ? kSteepBelow : INFINITY, status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc, graded_finish ? th8 : nullptr, rest_trace, n);
+        TONER_LAUNCH(verify_kernel, (kc + 127) / 128, 128, stream, e_est, ritz_norm || graded_finish ? e_top : nullptr, graded_finish ? (float)(kGradedResidual + p * kGradedTail) : (float)(1.15 * (1.0 - l_last) + 1e-3), plan.steep ? kSteepBelow : INFINITY, status ? status + k0 : nullptr, resid_out ? resid_out + k0 : nullptr, kc, graded_finish ? th8 : nullptr, rest_trace, n, lowest);
         TONER_CUDA(cudaGetLastError());
       }
       const int sweeps = track_sweeps & 63;
