@@ -142,6 +142,43 @@ def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops, p, 
     assert flagged > 0 or steps is None
 
 
+def test_an_overflow_is_the_calls_alone():
+    """A norm far too low overflows steps of higher degree although A is finite: status 1, the call is repaired, and the tracked
+    vectors stay what they were, so that estimates are used again after the usual eight calls.  A that is not finite is status 2."""
+    from toner_b200 import core, ops
+    n = 384
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, _ = torch.linalg.qr(torch.randn(n, n, device="cuda", generator=g, dtype=torch.float64))
+
+    def statistic(top):
+        lam = torch.linspace(1e-3, 1.5, n, device="cuda", dtype=torch.float64)
+        lam[-1], lam[-2] = 1.6, 1.6 * top
+        c = ((q * lam) @ q.T).float()
+        return (0.5 * (c + c.T)).expand(2, n, n).contiguous()
+
+    f = core.FactorSet(2, n, torch.device("cuda"), (0.5, 0.125), DAMPING, slots=12)
+    used = []
+    for call in range(18):
+        f.ema.copy_(statistic(0.9 if call < 6 else 2.1))
+        if call == 6:          # the block knows every large direction but the one that is now the largest
+            for j in range(f.deflate.shape[1]):
+                f.deflate[:, j] = q[:, n - 1 if j == 0 else n - 2 - j].float()
+        f.compute()
+        torch.cuda.synchronize()
+        used.append(f._used_estimate)
+        assert f.status.tolist() == ([1, 1] if call == 6 else [0, 0]), (call, f.status.tolist())
+        assert torch.isfinite(f.root_lo).all().item() == (call != 6)
+        f.finish()
+        assert torch.isfinite(f.track).all() and torch.isfinite(f.root_lo).all()
+    assert used[6] and f.repairs == 2 and f.fallbacks == 0 and all(used[-3:]), used
+    bad = statistic(2.1)
+    bad[1, 5, 5] = float("inf")
+    _, _, _, st = ops.inv_roots(bad, DAMPING, 8, 4, lower=1e-4, lower_is_estimate=True, track=torch.ones(2, n, device="cuda"),
+                                lmin=torch.empty(2, device="cuda"), track_sweeps=4, deflate=f.deflate[:, :8].contiguous(), deflate_rank=4, ritz_norm=True)
+    ops.assert_healthy()
+    assert st.tolist()[1] == 2, st.tolist()
+
+
 @pytest.mark.parametrize("p,q", [(4, 1), (8, 4)])
 @pytest.mark.parametrize("n", [264, 1032])
 def test_a_first_step_left_out_by_some_statistics(ops, p, q, n):

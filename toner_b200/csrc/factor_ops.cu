@@ -857,7 +857,10 @@ __global__ void __launch_bounds__(256) power_norm_kernel(float* __restrict__ v, 
   block_sum3(rr, 0.0, 0.0);
   rr = tot[0];
   const double inv = yy > 0.0 ? 1.0 / sqrt(yy) : 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (float)(Y[i] * inv);
+  // (Y of a root that overflowed -- a norm taken too low, status 1 -- says nothing: V, which the next call starts from, stays)
+  if (isfinite(yy)) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (float)(Y[i] * inv);
+  }
   if (threadIdx.x == 0) {
     lam[b] = (float)l;
     res[b] = (l > 0.0 && vv > 0.0) ? (float)(sqrt(rr) / (l * sqrt(vv))) : INFINITY;
