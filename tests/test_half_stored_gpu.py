@@ -13,7 +13,7 @@ def _give_back():
     torch.cuda.empty_cache()     # (gigabytes, of which later tests that count memory would be handed pieces)
 
 
-@pytest.mark.parametrize("n,k", [(264, 64), (520, 16), (768, 8), (1000, 5), (1288, 3), (2056, 1)])
+@pytest.mark.parametrize("n,k", [(264, 64), (520, 16), (768, 8), (1000, 5), (1288, 3), (2040, 2)])
 @pytest.mark.parametrize("p,q", [(8, 4), (4, 1), (2, 1)])
 def test_the_same_roots_as_from_whole_planes(n, k, p, q):
     """A workspace for a few statistics makes the call go through them in chunks below the size from which planes are stored by half.
@@ -23,9 +23,8 @@ def test_the_same_roots_as_from_whole_planes(n, k, p, q):
     directions and, for 2 q = p, the graded finish."""
     from toner_b200 import ops
     assert k * n * n >= 4 << 20
-    few = max(1, ((4 << 20) - 1) // (n * n))
-    if few * n * n >= 4 << 20:
-        pytest.skip("one statistic is a large stack")
+    few = ((4 << 20) - 1) // (n * n)
+    assert few >= 1
     g = torch.Generator(device="cuda").manual_seed(n)
     x = torch.randn(k, 3 * n, n, device="cuda", generator=g)
     x[:, :, 0] *= 30.0
@@ -62,6 +61,38 @@ def test_the_same_roots_as_from_whole_planes(n, k, p, q):
                 errors = [float(((r.double() - w).flatten(1).norm(dim=1) / w.flatten(1).norm(dim=1)).mean()) for r in (whole, half)]
                 assert errors[1] <= 1.01 * errors[0] + 2e-8, (call, errors)
             lower = 0.5 * float((states[0]["lmin"] / states[0]["norms"]).min())
+
+
+@pytest.mark.parametrize("n", [2048, 2056, 3072])
+@pytest.mark.parametrize("p,q", [(8, 4), (4, 1)])
+def test_widths_of_which_one_statistic_is_a_large_stack(n, p, q):
+    """From 2048 columns on there is no call on whole planes to compare with, but a block read from the wrong place is of the root's own
+    size.  The limit: truncation is 1.2e-7 a k-block of 64 in one chain, in each of the linear steps' products with X and as much again
+    for the powers of T; q times that for the root's q-th power."""
+    from toner_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(2, 2 * n, n, device="cuda", generator=g)
+    x[:, :, 0] *= 30.0
+    ema = x.mT @ x / (2 * n)
+    ema = (0.5 * (ema + ema.mT)).contiguous()
+    del x
+    a = ema.double()
+    a = a / a.diagonal(dim1=1, dim2=2).mean(1)[:, None, None] + DAMPING * torch.eye(n, device="cuda", dtype=torch.float64)
+    lam, vec = torch.linalg.eigh(a)
+    lower = 0.5 * float((lam[:, 0] / lam[:, -2]).min())
+    limit = 2 * ops.inv_roots_iterations(n, DAMPING, p) * (n / 64) * 1.2e-7
+    for interleave in (False, True):
+        for bound in (0.0, lower):
+            lo, hi, _, st = ops.inv_roots(ema, DAMPING, p, q, lower=bound, lower_is_estimate=bound > 0, interleave=interleave,
+                                          track=torch.zeros(2, n, device="cuda"), lmin=torch.zeros(2, device="cuda"), track_sweeps=8,
+                                          track_restart=True, deflate=torch.zeros(2, 8, n, device="cuda"), deflate_rank=3, deflate_restart=True)
+            ops.assert_healthy()
+            assert st.tolist() == [0, 0]
+            for root, s, most in ((lo, 1.0 / p, limit), (hi, q / p, q * limit)):
+                if root is not None:
+                    want = (vec * lam.pow(-s)[:, None, :]) @ vec.mT
+                    assert torch.equal(root, root.mT)
+                    assert float(((root.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)).max()) < most
 
 
 @pytest.mark.parametrize("n,k,p,q", [(128, 260, 8, 4), (264, 64, 2, 1), (264, 64, 8, 4), (432, 24, 4, 1)])

@@ -180,9 +180,9 @@ def test_an_overflow_is_the_calls_alone():
 
 
 @pytest.mark.parametrize("p,q", [(4, 1), (8, 4)])
-@pytest.mark.parametrize("n", [264, 1032])
+@pytest.mark.parametrize("n", [264, 1032, 1288, 2056])
 def test_a_first_step_left_out_by_some_statistics(ops, p, q, n):
-    """The bound that always holds: statistics of a small norm start with the second step, those of a large one (two directions of one
+    """(From 1288 columns on with planes stored by half.)  The bound that always holds: statistics of a small norm start with the second step, those of a large one (two directions of one
     size, which are not deflated) with the first.  Each comes out as beside others of its kind, and as close to FP64 as linear steps
     bring it."""
     small = _statistics(n, 300.0)
