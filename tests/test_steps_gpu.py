@@ -126,6 +126,8 @@ def test_a_norm_above_which_the_spectrum_reaches_is_forgiven_or_flagged(ops, p, 
         if steps is None:      # (linear steps forgive more, and flag where they do not)
             continue
         assert ops.inv_roots_graded(lower, p, n) is None or 2 * q != p
+        if steps["steps"][0][0] == 1 and reach > 1.3:     # (where a linear T is negative: as after linear steps alone)
+            continue
         norms = torch.zeros(2, device="cuda")
         lo, _, _, st = ops.inv_roots(stats, DAMPING, p, q, lower=lower, lower_is_estimate=True, norms=norms,
                                      track=vec[:, :, 0].float().contiguous(), lmin=torch.empty(2, device="cuda"), track_sweeps=4,

@@ -390,6 +390,21 @@ static GradedPoly graded_poly(int p, double lo, const GradedCare& care) {
 // of it (interleaved products in batches; C and operand planes as the finish has them).
 static double single_pass(int n) { return 0.35 + 320.0 / n; }
 
+// What steps of higher degree are weighed with against linear ones: times in products of one chain of accumulations.  Products in
+// chains of 8 / 2 / 1 k-blocks took 1.15 / 1.28 / 1.4 of one (widths 512 to 3072, 1 to 48 statistics: 1.02 to 1.37, 1.15 to 1.55, 1.15 to 1.8), less
+// below 640 columns, where a launch is most of it (1.05 / 1.1 / 1.12 at 264), a single pass at most 0.85, the FP32 matrix of a linear
+// term 0.15: 1080 calls, each with steps and with linear ones, 1 to 2 % off by these.
+struct StepCosts {
+  double single, chained[3];   // (of chains of 8, of 2, of 1)
+  explicit StepCosts(int n) : single(std::min(0.85, single_pass(n))) {
+    const double wide = std::min(1.0, n / 640.0);
+    chained[0] = 1.0 + 0.15 * wide;
+    chained[1] = 1.0 + 0.28 * wide;
+    chained[2] = 1.0 + 0.4 * wide;
+  }
+  double product(int chain) const { return chain == 0 ? 1.0 : chain == 1 ? chained[2] : chain == 2 ? chained[1] : chained[0]; }
+};
+
 // Newton steps of degree 1, 2 and 4 (root_steps.cuh) in the order that costs least.  Between steps the bound of M's spectrum is
 // rounded down to an eighth of an octave: every schedule is then a path through 256 bounds, whose steps (0.1 ms of host
 // time a bound to find) and finishing polynomials a thread keeps, and a bound that moves a little from call to call costs nothing.  Against
@@ -442,31 +457,35 @@ struct StepPlan {
   double cost = 1e9;                // in split products, the finish and its product with X counted
   std::vector<std::pair<int, int>> path;   // (bound, degree's index)
 };
-// T's own products; with a linear term it writes and reads an FP32 matrix more
-static double own_products(const NewtonStep& s) { return (s.degree == 4 ? 2 : s.degree - 1) + (s.lin != 0.0 ? 0.25 : 0.0); }
-static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear);
+// A step from bound j on: T's own products, its powers and M, and the next product with X; with a linear term an FP32 matrix is written
+// and read more.
+static double step_cost(const NewtonStep& s, int j, int log2p, const StepCosts& costs) {
+  return (log2p + 1 + (s.degree == 4 ? 2 : s.degree - 1)) * costs.product(steep_chain_length(bound_of(j))) + (s.lin != 0.0 ? 0.15 : 0.0) +
+         costs.product(kPromoteSteepX);
+}
+static const StepPlan& cheapest(int p, int j, bool certified, const StepCosts& costs, std::unordered_map<int, StepPlan>& memo, bool linear);
 // Cheapest steps from bound j on, the first of degree two or four unless `linear`; `memo` is the call's own.
 // Where the bound is an estimate so may the norm be, and M_0 may reach above 1.  A T of degree two or four sends what lies there
 // further up, to where a linear T is negative; T^p is not, so M could come back to I with the sign of X turned and no check to see it
 // (p = 8: degrees 4, 1 from a reach of 1.12).  So after a step of even degree, whose T is positive everywhere, only such steps follow:
 // 0.5 split products more for 4 bounds in 400 at p = 4, none at p = 8 to 32.  Linear steps before them leave what linear ones alone leave
 // (verified vectors below).
-static StepPlan cheapest_first(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear) {
+static StepPlan cheapest_first(int p, int j, bool certified, const StepCosts& costs, std::unordered_map<int, StepPlan>& memo, bool linear) {
   StepPlan best;
   const BoundNode& node = bound_node(p, j);
   int log2p = 0;
   while ((1 << log2p) < p) ++log2p;
   for (int i = 2; i >= (linear ? 0 : 1); --i) {
     if (!node.ok[i]) continue;
-    const double own = log2p + 2 + own_products(node.step[i]);   // (powers, M, the next product with X)
-    const double end = single * (node.fin_products[certified][i] - 1) + 1.0;
+    const double own = step_cost(node.step[i], j, log2p, costs);
+    const double end = costs.single * (node.fin_products[certified][i] - 1) + 1.0;
     if (node.fin[certified][i].order && own + end < best.cost) {
       best.cost = own + end;
       best.path = {{j, i}};
     }
     const int next = bound_below(node.step[i].next);
     if (next >= j || node.step[i].next > 0.9 || own + log2p + 2 >= best.cost) continue;
-    const StepPlan& rest = cheapest(p, next, certified, single, memo, certified || i == 0);
+    const StepPlan& rest = cheapest(p, next, certified, costs, memo, certified || i == 0);
     if (own + rest.cost < best.cost) {
       best.cost = own + rest.cost;
       best.path = {{j, i}};
@@ -475,11 +494,11 @@ static StepPlan cheapest_first(int p, int j, bool certified, double single, std:
   }
   return best;
 }
-static const StepPlan& cheapest(int p, int j, bool certified, double single, std::unordered_map<int, StepPlan>& memo, bool linear) {
+static const StepPlan& cheapest(int p, int j, bool certified, const StepCosts& costs, std::unordered_map<int, StepPlan>& memo, bool linear) {
   const int key = linear ? j : -j;
   const auto found = memo.find(key);
   if (found != memo.end()) return found->second;
-  return memo[key] = cheapest_first(p, j, certified, single, memo, linear);
+  return memo[key] = cheapest_first(p, j, certified, costs, memo, linear);
 }
 
 // Everything a call runs for a lower bound l0: the steps, the distance of the last M from I, the finishing polynomial.
@@ -548,15 +567,18 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
   if (first < kBounds) {
     int log2p = 0;
     while ((1 << log2p) < p) ++log2p;
-    const double single = single_pass(steep_n);
+    const StepCosts costs(steep_n);
     QuadraticSteps q;
-    const double linear = (s.iters - 1) * (log2p + 2) +
-                          single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
+    double linear = costs.single * (quadratic_steps(s.fin, p, q) ? 1 + (int)q.lin.size() + (q.by_r ? 1 : 0) : s.fin.order - 1);
+    for (int k = 0; k < s.iters - 1; ++k) linear += (log2p + 1) * costs.product(chain_length(s.steps[k].lower)) + 1.0;
+    // (the squarings that follow, of 2 q = p: in one chain after linear steps)
+    const double squarings = (p > 4 ? log2p - 1 : 0) * (costs.product(kPromoteSteepSquares) - 1.0);
     std::unordered_map<int, StepPlan> memo;
-    StepPlan plan = cheapest(p, first, kind > 0, single, memo, true);
+    StepPlan plan = cheapest(p, first, kind > 0, costs, memo, true);
     if (kind == 2) {
-      // The bound that always holds, damping / n, is a norm of n; statistics have one of 5 to 15, which the device knows before the
-      // first product.  So the first step goes from this bound to that of a norm of 16, damping / 16, or as far as it gets, and is
+      // The bound that always holds, damping / n, is a norm of n; statistics have one of 1.4 to 16 (rows of synthetic.py, 512 to 5632
+      // columns, up to four outliers deflated; 24 where 752 rows of 3072 columns are log-uniform to 1e6; more outliers than the block
+      // holds leave hundreds), which the device knows before the first product.  So the first step goes from this bound to that of a norm of 16, damping / 16, or as far as it gets, and is
       // left out for every statistic whose norm allows it; the others follow as they would from there.
       const BoundNode& node = bound_node(p, first);
       const int norm16 = bound_below(l0 * steep_n / 16.0);
@@ -564,10 +586,12 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
         if (!node.ok[i]) continue;
         const int from = std::max(norm16, bound_below(node.step[i].next));
         if (from > norm16 && i < 2) continue;   // (degree four gets further)
-        const StepPlan rest = cheapest_first(p, from, true, single, memo, false);   // (a first T of degree one is no product's result)
+        const StepPlan rest = cheapest_first(p, from, true, costs, memo, false);   // (a first T of degree one is no product's result)
         if (rest.path.empty()) break;
-        const double all = log2p + 2 + own_products(node.step[i]) + rest.cost;
-        if (rest.cost < 0.9 * plan.cost && all < linear) {
+        // (What is left out is launched all the same, hence a tenth less at least.  Statistics of which none starts late pay for all: 0.80 to
+        // 0.99 of the linear steps' time with norms of 95 to 1025, 264 to 3072 wide, p = 4 to 16, those that do 0.60 to 0.83; hence 5 % more allowed.)
+        const double all = step_cost(node.step[i], first, log2p, costs) + rest.cost;
+        if (rest.cost < 0.9 * plan.cost && all + squarings < 1.05 * linear) {
           s.late = bound_of(from);
           plan.cost = all;
           plan.path = {{first, i}};
@@ -576,7 +600,9 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
         break;
       }
     }
-    if (!plan.path.empty() && (s.late > 0.0 || plan.cost < linear - 0.3)) {
+    // (Of 739 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 46 then took more than 1 % longer than with linear
+    // steps, 10 % at most, where a last wave is nearly empty: 12 x 1280, 1 x 3072.  By product counts, 0.3 fewer wanted, 188 of 951 did, 19 % at most.)
+    if (!plan.path.empty() && (s.late > 0.0 || plan.cost + squarings < linear)) {
       s.steep = true;
       s.steps.clear();
       for (const auto& at : plan.path) s.steps.push_back(bound_node(p, at.first).step[at.second]);
@@ -2709,11 +2735,10 @@ int toner_inv_roots_planes(const float* ema, int32_t k, int32_t n, float damping
         } else if (ritz_norm) {
           // The norm was an estimate too.  Eigenvalues of M_0 above 1 (the estimate was too low for them) come out of
           // linear steps BELOW the lower bound the schedule continues from -- T = a I - b M is small there -- and lag the same way;
-          // they belong to the top of A', so the same four steps from the largest Ritz vector that stayed in A' find them.  (What lies
-          // beyond a / b, where T is negative, lags or grows too, but for bands a few 1e-3 wide that come back to I with the sign of
-          // X turned: at a reach of 1.03 or more for p = 2, 1.24 for p = 4, 1.95 for p = 8, none up to 3.4 for 16 and 32; the norm
-          // is 1.4 times the Ritz value, so that has to be as much more too low.)  Both starting vectors go through M in one pass
-          // per step.
+          // they belong to the top of A', so the same four steps from the largest Ritz vector that stayed in A' find them.  Both
+          // starting vectors go through M in one pass per step.  (What lies beyond a / b, where T is negative, may come back to I with the
+          // sign of X turned, which nothing here sees: from a reach of 1.03 on for p = 2, 1.24 for p = 4, 1.95 for p = 8, none up to 3.4
+          // for 16 and 32.  The norm is 1.4 times the Ritz value, so that has to be as much more too low.)
           // Steps of higher degree send them ABOVE 1, where R is negative and small at first beside what it may be on the other side
           // (degree 2 from l = 0.034: R = -0.3 for a reach of 1.2, 0.54 for the lower end).  Steps on R lose such a direction; those on
           // (1 - e / 2) I - M gain it.  And they start from the Ritz vector's residual, which holds what the block has not found yet,
