@@ -46,6 +46,31 @@ def test_vectors_and_roots_with_twelve_slots(n, rank):
             assert float((root[b].double() - want).norm() / want.norm()) < most
 
 
+@pytest.mark.parametrize("n,rank", [(512, 4), (512, 9), (1032, 4), (1032, 12)])
+def test_clusters_by_the_number_of_statistics(n, rank):
+    """Of few statistics a cluster of four or eight takes the columns of each, of many (96 blocks, 192 up to four vectors) a smaller one or a
+    single block: the vectors of a stack's first statistics are those of calls on fewer (2e-6: FP32, 30 times the rest and 1.5 apart)."""
+    from toner_b200 import ops
+    k, strong = 100, max(1, rank - 2)
+    g = torch.Generator(device="cuda").manual_seed(n + rank)
+    q, _ = torch.linalg.qr(torch.randn(n, n, device="cuda", generator=g, dtype=torch.float64))
+    lam = 0.5 + torch.rand(n, device="cuda", generator=g, dtype=torch.float64)
+    lam[:strong] = 30.0 * 1.5 ** torch.arange(strong, device="cuda", dtype=torch.float64)
+    c = ((q * lam) @ q.T).float()
+    ema = (0.5 * (c + c.T)).expand(k, n, n).contiguous()
+    first = None
+    for count in (2, 13, 25, 30, 49, 100):      # eight (from 1024 columns) or four, then half of it, ...
+        vectors, found = torch.zeros(count, 12, n, device="cuda"), torch.zeros(count, device="cuda", dtype=torch.int32)
+        ops.inv_roots(ema[:count], DAMPING, 8, 4, lower=1e-3, track=torch.zeros(count, n, device="cuda"), track_sweeps=1, track_restart=True,
+                      deflate=vectors, deflate_rank=rank, deflate_restart=True, deflated=found)
+        ops.assert_healthy()
+        assert ((found & 255) == strong).all()
+        v = vectors[:, :strong]
+        assert torch.equal(v, v[:1].expand_as(v))
+        first = v[0] if first is None else first
+        assert float((v[0] - first * torch.sign((v[0] * first).sum(1, keepdim=True))).norm(dim=1).max()) < 2e-6
+
+
 def test_more_outliers_than_eight(monkeypatch):
     """Rows with eight outlier directions and a mean, as the benchmark's spiked:8: all nine are found and deflated, no estimate of
     the spectrum fails, and what is left takes the graded finish."""

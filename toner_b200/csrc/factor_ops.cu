@@ -1535,11 +1535,19 @@ __global__ void __launch_bounds__(256) ritz_kernel(float* __restrict__ v, float*
 // CTAs that share a statistic.  A launch, four statistics of width 768 / 1280 / 3328 / 5632 without a gap in their spectrum, us:  r = 4
 // 15 / 19 / 34 / 52 by one, 13 / 13 / 16 / 23 by eight;  r = 8  42 / 50 / 94 / 171, 31 / 31 / 37 / 49;  r = 11  107 / 129 / 235 / 434,
 // 79 / 80 / 92 / 117.  (Before the sums were folded and the angles taken in FP32, by one: r = 4  17 / 20 / 31 / 61, r = 8  43 / 53 / 91 / 182.)
-static int ritz_ctas(int n) { return n >= 1024 ? 8 : n >= 512 ? 4 : 1; }
+// By one / two / four / eight, us:  384 columns, 12 statistics, r = 8  36 / 32 / 28 / 28, 264 and 24 of them 32 / 30 / 31 / 55;  512, 24, r = 4
+// 15.5 / 15.3 / 15.5 / 15.6;  768, 12, r = 4  22 / 16 / 15 / 14;  1024, 4, r = 4  58 / 56 / 43 / 33;  2048, 12, r = 8  78 / 56 / 43 / 36.
+// No more blocks than find a place at once: the wide kernels (r > 4) take an SM each, and clusters fill the GPU's groups of SMs unevenly.
+// r = 8, 768 columns:  24 statistics 43 / 37 / 32 / 56, 36  43 / 38 / 59 / 82, 96  44 / 70 / 86 / 188;  r = 4:  48  21 / 21 / 18 / 29, 96  21 / 20 / 30 / 51.
+static int ritz_ctas(int n, int k, int width) {
+  int ctas = n >= 1024 ? 8 : n >= 512 ? 4 : 1;
+  while (ctas > 1 && (long long)k * ctas > (width > 4 ? 96 : 192)) ctas /= 2;
+  return ctas;
+}
 template <int R>
 static cudaError_t launch_ritz(int k, cudaStream_t stream, float* v, float* y, int n, int r, int vstride, int last, float* theta, float* res,
                                int in_order, float trace) {
-  const int ctas = in_order ? 1 : ritz_ctas(n);
+  const int ctas = in_order ? 1 : ritz_ctas(n, k, R);
   return launch(ritz_kernel<R>, dim3(ctas, k), 256, 0, stream, ctas > 1 ? ctas : 0, v, y, n, r, vstride, last, theta, res, in_order, trace);
 }
 
