@@ -391,16 +391,16 @@ static GradedPoly graded_poly(int p, double lo, const GradedCare& care) {
 static double single_pass(int n) { return 0.35 + 320.0 / n; }
 
 // What steps of higher degree are weighed with against linear ones: times in products of one chain of accumulations.  Products in
-// chains of 8 / 2 / 1 k-blocks took 1.15 / 1.28 / 1.4 of one (widths 512 to 3072, 1 to 48 statistics: 1.02 to 1.37, 1.15 to 1.55, 1.15 to 1.8), less
-// below 640 columns, where a launch is most of it (1.05 / 1.1 / 1.12 at 264), a single pass at most 0.85, the FP32 matrix of a linear
-// term 0.15: 1080 calls, each with steps and with linear ones, 1 to 2 % off by these.
+// chains of 8 / 2 / 1 k-blocks take 1.15 / 1.3 / 1.42 of one around 1000 columns (1.14 to 1.22, 1.18 to 1.43, 1.15 to 1.7 with 4 to 36 statistics),
+// less below 640, where a launch is most of it (1.05 / 1.1 / 1.12 at 264), and on wide statistics (1.10 / 1.24 / 1.34 at 2048, 1.05 / 1.19 / 1.25 at 3072), a single
+// pass at most 0.85, the FP32 matrix of a linear term 0.15: 1080 calls, each with steps and with linear ones.
 struct StepCosts {
   double single, chained[3];   // (of chains of 8, of 2, of 1)
   explicit StepCosts(int n) : single(std::min(0.85, single_pass(n))) {
-    const double wide = std::min(1.0, n / 640.0);
-    chained[0] = 1.0 + 0.15 * wide;
-    chained[1] = 1.0 + 0.28 * wide;
-    chained[2] = 1.0 + 0.4 * wide;
+    const double share = std::min(1.0, n / 640.0) * std::min(1.0, std::sqrt(1280.0 / n));
+    chained[0] = 1.0 + 0.15 * share;
+    chained[1] = 1.0 + 0.3 * share;
+    chained[2] = 1.0 + 0.42 * share;
   }
   double product(int chain) const { return chain == 0 ? 1.0 : chain == 1 ? chained[2] : chain == 2 ? chained[1] : chained[0]; }
 };
@@ -600,9 +600,10 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
         break;
       }
     }
-    // (Of 739 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 46 then took more than 1 % longer than with linear
-    // steps, 10 % at most, where a last wave is nearly empty: 12 x 1280, 1 x 3072.  By product counts, 0.3 fewer wanted, 188 of 951 did, 19 % at most.)
-    if (!plan.path.empty() && (s.late > 0.0 || plan.cost + squarings < linear)) {
+    // (Of 714 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 41 then took more than 1 % longer than with linear
+    // steps: a single statistic of 3072 columns, whose 78 tiles are two waves, by 16 % at most, the others by 7 %.  By product counts, 0.3
+    // fewer wanted, 188 of 951 did, by 19 %.)
+    if (!plan.path.empty() && (s.late > 0.0 || plan.cost + squarings < 0.98 * linear)) {
       s.steep = true;
       s.steps.clear();
       for (const auto& at : plan.path) s.steps.push_back(bound_node(p, at.first).step[at.second]);
