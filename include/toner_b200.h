@@ -266,8 +266,8 @@ int toner_inv_roots_graded_for(float lower, int32_t p, int32_t n, int32_t* steps
 /* The steps of a call that asks for no step count and no plane order, on statistics of width n, where that costs less than
  * linear ones (p >= 4, n >= 256): T of degree 1, 2 or 4 in M, levelled like the linear T (110 times the lower bound instead of 13
  * for two products more at degree 4, p = 8).  Returns their number (0: the schedule of toner_inv_roots_schedule is used) and writes seven doubles
- * a step (degree, zb, za, kappa, top, lin, con: with z = zb + za mu, T is con + lin mu plus nothing, top z^2 or
- * top (z^2 + kappa)^2), the finishing polynomial and the distance e as toner_inv_roots_schedule does, and products_out[0], [1]: the split and the single-pass
+ * a step (degree, zb, za, kappa, top, lin, con: with z = zb + za mu, T is con + lin mu for degree 1, con + top z^2 for degree 2 and
+ * con + lin mu + top (z^2 + kappa)^2 for degree 4), the finishing polynomial and the distance e as toner_inv_roots_schedule does, and products_out[0], [1]: the split and the single-pass
  * products that steps and finish take.  kind: the bound is an estimate (0), certified (1), the one that always holds (2).  late_out > 0 (kind
  * 2): a statistic whose norm, on the device, puts its spectrum above this starts with the second step.  Every output pointer is
  * optional; needs no device. */

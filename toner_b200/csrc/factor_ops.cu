@@ -73,11 +73,11 @@ static int chain_length(double lower) {
   return 0;
 }
 
-// The same after steps of higher degree.  Fewer products and these chains leave the roots 0.4 times as far from FP64 as linear
-// steps do (median of 540 calls, p = 4 and 8: Marchenko-Pastur spectra of 1.5 to 6 rows a column, log-uniform ones of condition 30
-// to 1e5, widths 264 to 2048, bounds from the one that always holds to the spectrum's end), 1.06 times in the worst; two k-blocks
-// below 5e-3: 1.6 times in the worst, below 5e-4: 1.7; eight from 5e-2 on, as the linear steps have: 1.7.  (12 products of 3072:
-// 790 us in one chain, 920 in chains of eight k-blocks, 980 of two, 1000 to 1150 of one.)
+// The same after steps of higher degree.  Fewer products and these chains leave the roots 0.30 to 0.46 times as far from FP64 as linear
+// steps do (means of 466 calls, p = 4, 8, 16: rows of 0.1 to 6 a column, log-uniform spectra of condition 30 to 1e6, widths 264 to 2048, bounds
+// from the one that always holds to the spectrum's end), 0.97 times in the worst.  Without the rank-deficient ones, of 540 calls: 0.4 in the median
+// and 1.06 in the worst; two k-blocks below 5e-3: 1.6 times in the worst, below 5e-4: 1.7; eight from 5e-2 on, as the linear steps have: 1.7.
+// (12 products of 3072: 790 us in one chain, 920 in chains of eight k-blocks, 980 of two, 1000 to 1150 of one.)
 static int steep_chain_length(double lower) {
   if (lower < 5e-3) return 1;
   if (lower < 0.5) return kPromoteAccurate;
@@ -601,7 +601,7 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
       }
     }
     // (Of 714 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 41 then took more than 1 % longer than with linear
-    // steps: a single statistic of 3072 columns, whose 78 tiles are two waves, by 16 % at most, the others by 7 %.  By product counts, 0.3
+    // steps: 25 times a single statistic of 3072 columns, whose 78 tiles are two waves, by 16 % at most, the others by 7 %.  By product counts, 0.3
     // fewer wanted, 188 of 951 did, by 19 %.)
     if (!plan.path.empty() && (s.late > 0.0 || plan.cost + squarings < 0.98 * linear)) {
       s.steep = true;
