@@ -74,7 +74,7 @@ static int chain_length(double lower) {
 }
 
 // The same after steps of higher degree.  Fewer products and these chains leave the roots 0.30 to 0.46 times as far from FP64 as linear
-// steps do (means of 466 calls, p = 4, 8, 16: rows of 0.1 to 6 a column, log-uniform spectra of condition 30 to 1e6, widths 264 to 2048, bounds
+// steps do (means of 467 calls, p = 4, 8, 16: rows of 0.1 to 6 a column, log-uniform spectra of condition 30 to 1e6, widths 264 to 2048, bounds
 // from the one that always holds to the spectrum's end), 0.97 times in the worst.  Without the rank-deficient ones, of 540 calls: 0.4 in the median
 // and 1.06 in the worst; two k-blocks below 5e-3: 1.6 times in the worst, below 5e-4: 1.7; eight from 5e-2 on, as the linear steps have: 1.7.
 // (12 products of 3072: 790 us in one chain, 920 in chains of eight k-blocks, 980 of two, 1000 to 1150 of one.)
@@ -392,12 +392,12 @@ static double single_pass(int n) { return 0.35 + 320.0 / n; }
 
 // What steps of higher degree are weighed with against linear ones: times in products of one chain of accumulations.  Products in
 // chains of 8 / 2 / 1 k-blocks take 1.15 / 1.3 / 1.42 of one around 1000 columns (1.14 to 1.22, 1.18 to 1.43, 1.15 to 1.7 with 4 to 36 statistics),
-// less below 640, where a launch is most of it (1.05 / 1.1 / 1.12 at 264), and on wide statistics (1.10 / 1.24 / 1.34 at 2048, 1.05 / 1.19 / 1.25 at 3072), a single
+// less below 800, where a launch is ever more of it (1.05 / 1.1 / 1.11 at 264), and on wide statistics (1.10 / 1.24 / 1.34 at 2048, 1.05 / 1.19 / 1.25 at 3072), a single
 // pass at most 0.85, the FP32 matrix of a linear term 0.15: 1080 calls, each with steps and with linear ones.
 struct StepCosts {
   double single, chained[3];   // (of chains of 8, of 2, of 1)
   explicit StepCosts(int n) : single(std::min(0.85, single_pass(n))) {
-    const double share = std::min(1.0, n / 640.0) * std::min(1.0, std::sqrt(1280.0 / n));
+    const double share = std::min(1.0, n / 800.0) * std::min(1.0, std::sqrt(1280.0 / n));
     chained[0] = 1.0 + 0.15 * share;
     chained[1] = 1.0 + 0.3 * share;
     chained[2] = 1.0 + 0.42 * share;
@@ -600,7 +600,7 @@ static const Schedule& schedule_for(double l0, int p, int iters, int grade_n = 0
         break;
       }
     }
-    // (Of 714 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 41 then took more than 1 % longer than with linear
+    // (Of 731 such calls -- p = 4, 8, 16, widths 264 to 3072, bounds from 5e-5 to 0.3 -- 44 then took more than 1 % longer than with linear
     // steps: 25 times a single statistic of 3072 columns, whose 78 tiles are two waves, by 16 % at most, the others by 7 %.  By product counts, 0.3
     // fewer wanted, 188 of 951 did, by 19 %.)
     if (!plan.path.empty() && (s.late > 0.0 || plan.cost + squarings < 0.98 * linear)) {
